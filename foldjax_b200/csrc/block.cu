@@ -15,51 +15,10 @@
 #include <cuda_bf16.h>
 
 #include "host.cuh"
+#include "single.cuh"
 
 namespace b200 {
 namespace {
-
-// ---- single-track float32 helpers (rows of c_s channels; N x 384 values: tiny next to z)
-// One warp per row: LN with bf16 scale/bias, float32 statistics (_common.py:15-26 with a
-// float32 input: no intermediate rounding).
-__global__ void ln_rows_kernel(const float* __restrict__ x, int rows, int c, const __nv_bfloat16* __restrict__ scale,
-                               const __nv_bfloat16* __restrict__ bias, float eps, float* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= rows) return;
-  const float* src = x + static_cast<long long>(row) * c;
-  float s = 0.f;
-  for (int i = lane; i < c; i += 32) s += src[i];
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  const float mean = s / c;
-  float q = 0.f;
-  for (int i = lane; i < c; i += 32) {
-    const float v = src[i] - mean;
-    q += v * v;
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
-  const float rstd = 1.0f / sqrtf(q / c + eps);
-  float* dst = out + static_cast<long long>(row) * c;
-  for (int i = lane; i < c; i += 32)
-    dst[i] = (src[i] - mean) * rstd * __bfloat162float(scale[i]) + __bfloat162float(bias[i]);
-}
-
-// h = silu(a) * b, elementwise (transition.py:108)
-__global__ void swiglu_kernel(const float* __restrict__ a, const float* __restrict__ b, long long total,
-                              float* __restrict__ h) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const float v = a[i];
-  h[i] = v / (1.0f + expf(-v)) * b[i];
-}
-
-__global__ void add_kernel(const float* __restrict__ a, const float* __restrict__ b, long long total,
-                           float* __restrict__ out) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < total) out[i] = a[i] + b[i];
-}
 
 // dst[pair][:] = mask[pair] != 0 ? src[pair][:] : 0 for 128-channel bf16 pairs, one thread per
 // 16-byte chunk. With src == dst only the dropped pairs are written. The pair gate of
@@ -73,12 +32,6 @@ __global__ void gate_pairs_kernel(const uint4* __restrict__ src, uint4* __restri
     dst[idx] = make_uint4(0u, 0u, 0u, 0u);
   else if (src != dst)
     dst[idx] = src[idx];
-}
-
-// s[row][:] = 0 where mask[row] == 0 (the single-track gate of the same block)
-__global__ void gate_rows_kernel(float* __restrict__ s, const float* __restrict__ mask, int rows, int c) {
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx < static_cast<long long>(rows) * c && mask[idx / c] == 0.f) s[idx] = 0.f;
 }
 
 __global__ void fill_kernel(float* __restrict__ p, long long total, float v) {
@@ -98,7 +51,7 @@ struct Offsets {
 };
 
 struct Plan {
-  size_t w, sub, sub_bytes, sn, upd, h1, h2, hs, ones, total;
+  size_t w, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
 };
 
 Plan plan(int n, int c_s, int heads_s, int hidden_z, int hidden_s, bool single) {
@@ -106,18 +59,19 @@ Plan plan(int n, int c_s, int heads_s, int hidden_z, int hidden_s, bool single) 
   Offsets o;
   p.w = o.take(static_cast<size_t>(n) * n * 128 * 2);
   size_t sub = b200tri_trimul_workspace_bytes(n);
-  const size_t cand[3] = {b200tri_triatt_workspace_bytes(n), b200tri_pair_transition_workspace_bytes(hidden_z),
-                          single ? b200tri_attention_pair_bias_workspace_bytes(n, c_s, heads_s) : 0};
+  const size_t cand[2] = {b200tri_triatt_workspace_bytes(n), b200tri_pair_transition_workspace_bytes(hidden_z)};
   for (size_t c : cand) sub = c > sub ? c : sub;
   p.sub_bytes = sub;
   p.sub = o.take(sub);
   if (single) {
-    const size_t act = static_cast<size_t>(n) * c_s * 4, hid = static_cast<size_t>(n) * hidden_s * 4;
-    p.sn = o.take(act);
-    p.upd = o.take(act);
-    p.h1 = o.take(hid);
-    p.h2 = o.take(hid);
-    p.hs = o.take(hid);
+    const size_t act = static_cast<size_t>(n) * c_s;
+    p.sn = o.take(act * 2 * 3);
+    p.partial = o.take(act * 4 * SINGLE_MAX_SPLITS);
+    p.h = o.take(static_cast<size_t>(n) * round_up(hidden_s, 8) * 2 * 3);
+    p.att = o.take(single_attention_work(n, c_s, heads_s).total);
+    p.fc[0] = o.take(tma_weight_bytes(c_s, hidden_s));
+    p.fc[1] = o.take(tma_weight_bytes(c_s, hidden_s));
+    p.fc[2] = o.take(tma_weight_bytes(hidden_s, c_s));
     p.ones = o.take(static_cast<size_t>(n) * 4);
   }
   p.total = o.total();
@@ -199,6 +153,9 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
                "pairformer: the single track needs s_out, c_s and heads_s");
   const b200tri_pairformer_block_params& first = a->params[0];
   const int hidden_z = first.transition_z.hidden, hidden_s = single ? first.transition_s.hidden : 0;
+  B200_REQUIRE(!single || (a->heads_s <= 16 && a->c_s == a->heads_s * 24), B200TRI_ERR_UNSUPPORTED,
+               "pairformer: the single track is built for up to 16 heads of width 24 (got c_s %d, %d heads)", a->c_s,
+               a->heads_s);
   B200_REQUIRE(hidden_z > 0 && (!single || hidden_s > 0), B200TRI_ERR_INVALID, "pairformer: transition widths missing");
   const Plan pl = plan(a->n, a->c_s, a->heads_s, hidden_z, hidden_s, single);
   B200_REQUIRE(a->workspace && a->workspace_bytes >= pl.total, B200TRI_ERR_WORKSPACE,
@@ -209,7 +166,6 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   uint8_t* ws = static_cast<uint8_t*>(a->workspace);
   void* w = ws + pl.w;
   const int n = a->n, c_s = a->c_s;
-  const long long act = static_cast<long long>(n) * c_s;
   const float* token_mask = a->mask;
   if (single && !token_mask) {
     float* ones = reinterpret_cast<float*>(ws + pl.ones);
@@ -220,19 +176,12 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   }
 
   const void* z_cur = a->z_in;
-  const float* s_cur = a->s_in;
   const long long pairs = static_cast<long long>(n) * n;
   const bool gate = a->pair_gate != 0 && a->pair_mask != nullptr;
   auto gate_pairs = [&](const void* src, void* dst) -> int {
     count_launch();
     gate_pairs_kernel<<<static_cast<unsigned>((pairs * 16 + 255) / 256), 256, 0, stream>>>(
         static_cast<const uint4*>(src), static_cast<uint4*>(dst), a->pair_mask, pairs);
-    B200_CUDA_OK(cudaGetLastError());
-    return B200TRI_OK;
-  };
-  auto gate_rows = [&](float* sv) -> int {
-    count_launch();
-    gate_rows_kernel<<<static_cast<unsigned>((act + 255) / 256), 256, 0, stream>>>(sv, token_mask, n, c_s);
     B200_CUDA_OK(cudaGetLastError());
     return B200TRI_OK;
   };
@@ -324,17 +273,22 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     z_cur = a->z_out;
     if (!single) continue;
 
-    // ---- single track, float32
-    float* sn = reinterpret_cast<float*>(ws + pl.sn);
-    float* upd = reinterpret_cast<float*>(ws + pl.upd);
-    float* h1 = reinterpret_cast<float*>(ws + pl.h1);
-    float* h2 = reinterpret_cast<float*>(ws + pl.h2);
-    float* hs = reinterpret_cast<float*>(ws + pl.hs);
-    count_launch();
-    ln_rows_kernel<<<(n * 32 + 255) / 256, 256, 0, stream>>>(
-        s_cur, n, c_s, static_cast<const __nv_bfloat16*>(P.pre_norm_s_scale),
-        static_cast<const __nv_bfloat16*>(P.pre_norm_s_bias), a->eps, sn);
-    B200_CUDA_OK(cudaGetLastError());
+    // ---- single track, float32: s += attention(LN(s), z), s += transition(s), each sum taken
+    // by the row kernel that also normalises the rows for the product behind it
+    __nv_bfloat16* sn = reinterpret_cast<__nv_bfloat16*>(ws + pl.sn);
+    float* partial = reinterpret_cast<float*>(ws + pl.partial);
+    __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(ws + pl.h);
+    RowArgs row = {};
+    row.rows = n;
+    row.c = c_s;
+    row.eps = a->eps;
+    if (layer == 0) {
+      row.base = a->s_in;
+      row.scale = P.pre_norm_s_scale;
+      row.bias = P.pre_norm_s_bias;
+      row.pieces = sn;
+      if ((rc = launch_row_norm(row, stream, true))) return rc;
+    }
     b200tri_attention_pair_bias_args t = {};
     t.n = n;
     t.c_s = c_s;
@@ -342,8 +296,6 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     t.heads = a->heads_s;
     t.eps = a->eps;
     t.inf = a->att_inf;
-    t.s = sn;
-    t.k_in = sn;
     t.z = a->z_out;
     t.mask = token_mask;
     t.proj_q = P.attention.proj_q;
@@ -355,30 +307,37 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     t.proj_z_norm_bias = P.attention.proj_z_norm_bias;
     t.proj_z = P.attention.proj_z;
     t.proj_o = P.attention.proj_o;
-    t.out = upd;
-    t.workspace = ws + pl.sub;
-    t.workspace_bytes = pl.sub_bytes;
-    if ((rc = b200tri_attention_pair_bias(&t, stream_))) return rc;
-    count_launch();
-    add_kernel<<<static_cast<unsigned>((act + 255) / 256), 256, 0, stream>>>(s_cur, upd, act, a->s_out);
-    B200_CUDA_OK(cudaGetLastError());
-    if (gate && (rc = gate_rows(a->s_out))) return rc;
+    int splits = 1;
+    if ((rc = single_attention(&t, sn, sn, ws + pl.att, partial, &splits, stream))) return rc;
+    row.base = layer == 0 ? a->s_in : a->s_out;
+    row.partial = partial;
+    row.splits = splits;
+    row.row_mask = gate ? token_mask : nullptr;
+    row.scale = P.transition_s.norm_scale;
+    row.bias = P.transition_s.norm_bias;
+    row.sum_out = a->s_out;
+    row.pieces = sn;
+    if ((rc = launch_row_norm(row, stream, true))) return rc;
     // transition_s: LN -> fc1 | fc2 -> silu(fc1) * fc2 -> fc3, added to s (transition.py:99-112)
     const int hid = P.transition_s.hidden;
-    count_launch(2);
-    ln_rows_kernel<<<(n * 32 + 255) / 256, 256, 0, stream>>>(
-        a->s_out, n, c_s, static_cast<const __nv_bfloat16*>(P.transition_s.norm_scale),
-        static_cast<const __nv_bfloat16*>(P.transition_s.norm_bias), a->eps, sn);
-    B200_CUDA_OK(cudaGetLastError());
-    if ((rc = launch_linear_f32(sn, nullptr, P.transition_s.fc1, nullptr, n, c_s, hid, 0, nullptr, h1, stream))) return rc;
-    if ((rc = launch_linear_f32(sn, nullptr, P.transition_s.fc2, nullptr, n, c_s, hid, 0, nullptr, h2, stream))) return rc;
-    const long long hact = static_cast<long long>(n) * hid;
-    swiglu_kernel<<<static_cast<unsigned>((hact + 255) / 256), 256, 0, stream>>>(h1, h2, hact, hs);
-    B200_CUDA_OK(cudaGetLastError());
-    if ((rc = launch_linear_f32(hs, nullptr, P.transition_s.fc3, nullptr, n, hid, c_s, 0, a->s_out, a->s_out, stream)))
+    const long long hp = round_up(hid, 8);
+    if ((rc = launch_swiglu(sn, n, c_s, P.transition_s.fc1, P.transition_s.fc2, hid, ws + pl.fc[0], ws + pl.fc[1], h, hp,
+                            stream, true)))
       return rc;
-    if (gate && (rc = gate_rows(a->s_out))) return rc;
-    s_cur = a->s_out;
+    if ((rc = launch_linear_partial(h, hp, n, hid, P.transition_s.fc3, c_s, ws + pl.fc[2], partial, &splits, stream, true)))
+      return rc;
+    row.base = a->s_out;
+    row.splits = splits;
+    const bool last = layer + 1 == a->n_blocks;
+    if (!last) {
+      const b200tri_pairformer_block_params next =
+          a->stacked ? unstack(first, layer + 1, c_s, a->heads_s) : a->params[layer + 1];
+      row.scale = next.pre_norm_s_scale;
+      row.bias = next.pre_norm_s_bias;
+    } else {
+      row.pieces = nullptr;
+    }
+    if ((rc = launch_row_norm(row, stream, true))) return rc;
   }
   return B200TRI_OK;
 }

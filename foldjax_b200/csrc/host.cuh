@@ -79,6 +79,28 @@ struct SmReserve {
 // from several host threads (one per device under XLA).
 int ensure_smem_limit(const void* kernel, int bytes);
 
+void count_launch(int n = 1);
+
+// Launches a kernel, counted. `pdl` lets it start before its predecessor in the stream has
+// drained (programmatic dependent launch): only for a kernel that calls pdl_wait() before it
+// touches anything the predecessor reads or writes.
+template <typename... KArgs, typename... Args>
+int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  count_launch();
+  B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+  return B200TRI_OK;
+}
+
 // The two module-level ops for every shape / element type outside the tensor-core
 // specialisation (generic.cu): other channel and head counts, float32 trunks.
 size_t trimul_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t c_hidden, int32_t dtype);
@@ -86,15 +108,9 @@ size_t triatt_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t heads, int
 int trimul_forward_generic(const b200tri_trimul_args* a, int c_z, int c_hidden, cudaStream_t stream);
 int triatt_forward_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream);
 
-// out[M][N] = (x * gate?) @ w (+ bias) (sigmoid?) (+ res): fp32 activations, bf16 weights [K][N]
-// (single_attention.cu; the single track's projections and transition use it).
-int launch_linear_f32(const float* x, const float* gate, const void* w, const void* bias, int M, int K, int N,
-                      int sigmoid, const float* res, float* out, cudaStream_t stream);
-
 // Launch accounting and optional per-kernel event timing.
 enum KernelId { K_TRIMUL_PROJECT = 0, K_TRIMUL_CONTRACT, K_TRIMUL_FINISH, K_TRIATT_PROJECT, K_TRIATT_CORE,
                 K_TRIATT_FINISH, K_PAIR_TRANSITION, K_PAIR_BIAS, K_CP_EXCHANGE, K_CP_READY, K_CP_COPY, K_COUNT };
-void count_launch(int n = 1);
 bool timing_enabled();
 struct TimedLaunch {  // brackets the launches made during its lifetime
   int id;

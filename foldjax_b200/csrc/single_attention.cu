@@ -17,6 +17,7 @@
 // fp32 pipes: at 16 heads x 24 channels it is far too small to be worth tensor-core
 // tiles, and its operands are fp32.
 #include "host.cuh"
+#include "single.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -130,66 +131,181 @@ pair_bias_kernel(const __nv_bfloat16* __restrict__ z, long long n_pairs, int n, 
   }
 }
 
-// ------------------------------------------------------------------ linear
-// out[M][N] = act(x[M][K] @ W[K][N] (+ b[N])) with fp32 x, bf16 W and b, fp32 out;
-// optional elementwise gate on the input rows: x <- x * gate (the reference's g * out
-// in front of the output projection). 64 x 64 tiles, 4 x 4 outputs per thread.
-__global__ void __launch_bounds__(256)
-linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ gate, const __nv_bfloat16* __restrict__ w,
-                  const __nv_bfloat16* __restrict__ b, int M, int K, int N, int sigmoid, float* __restrict__ out,
-                  const float* __restrict__ res = nullptr) {
-  __shared__ float xs[16][64 + 1];
-  __shared__ float ws[16][64];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int idx = threadIdx.x; idx < 64 * 16; idx += 256) {
-      const int r = idx >> 4, c = idx & 15;
-      const int m = m0 + r, k = k0 + c;
-      float v = 0.f;
-      if (m < M && k < K) {
-        v = x[static_cast<long long>(m) * K + k];
-        if (gate) v *= gate[static_cast<long long>(m) * K + k];
-      }
-      xs[c][r] = v;
+// ------------------------------------------------------------------ row kernels
+// See launch_row_norm. One warp per row, the row in registers (up to 12 values per lane).
+constexpr int ROW_VALUES = MAX_HEADS * HD / 32;
+__global__ void __launch_bounds__(128) row_norm_kernel(const RowArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (row >= a.rows) return;
+  const long long off = static_cast<long long>(row) * a.c;
+  const bool keep = a.row_mask == nullptr || a.row_mask[row] != 0.f;
+  float v[ROW_VALUES];
+  float s = 0.f;
+#pragma unroll
+  for (int e = 0; e < ROW_VALUES; ++e) {
+    const int i = lane + 32 * e;
+    v[e] = 0.f;
+    if (i >= a.c || !keep) continue;
+    if (a.partial) {
+      float u = 0.f;
+      for (int p = 0; p < a.splits; ++p) u += a.partial[static_cast<long long>(p) * a.rows * a.c + off + i];
+      v[e] = u;
     }
-    for (int idx = threadIdx.x; idx < 16 * 64; idx += 256) {
-      const int r = idx >> 6, c = idx & 63;
-      const int k = k0 + r, nn = n0 + c;
-      ws[r][c] = (k < K && nn < N) ? __bfloat162float(w[static_cast<long long>(k) * N + nn]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float a[4], bb[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        a[e] = xs[k][ty * 4 + e];
-        bb[e] = ws[k][tx * 4 + e];
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r], bb[c], acc[r][c]);
-    }
-    __syncthreads();
+    if (a.base) v[e] = a.base[off + i] + v[e];
+    s += v[e];
   }
+  if (a.sum_out) {
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int m = m0 + ty * 4 + r;
-    if (m >= M) continue;
+    for (int e = 0; e < ROW_VALUES; ++e)
+      if (lane + 32 * e < a.c) a.sum_out[off + lane + 32 * e] = v[e];
+  }
+  if (!a.pieces) return;
+  if (a.scale) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int nn = n0 + tx * 4 + c;
-      if (nn >= N) continue;
-      float v = acc[r][c] + (b ? __bfloat162float(b[nn]) : 0.f);
-      if (sigmoid) v = 1.0f / (1.0f + expf(-v));
-      if (res) v += res[static_cast<long long>(m) * N + nn];
-      out[static_cast<long long>(m) * N + nn] = v;
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const float mean = s / a.c;
+    float q = 0.f;
+#pragma unroll
+    for (int e = 0; e < ROW_VALUES; ++e)
+      if (lane + 32 * e < a.c) q += (v[e] - mean) * (v[e] - mean);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
+    const float rstd = 1.0f / sqrtf(q / a.c + a.eps);
+    const __nv_bfloat16* scale = static_cast<const __nv_bfloat16*>(a.scale);
+    const __nv_bfloat16* bias = static_cast<const __nv_bfloat16*>(a.bias);
+#pragma unroll
+    for (int e = 0; e < ROW_VALUES; ++e) {
+      const int i = lane + 32 * e;
+      if (i < a.c) v[e] = (v[e] - mean) * rstd * __bfloat162float(scale[i]) + __bfloat162float(bias[i]);
     }
+  }
+  const long long plane = static_cast<long long>(a.rows) * a.c;
+#pragma unroll
+  for (int e = 0; e < ROW_VALUES; ++e) {
+    const int i = lane + 32 * e;
+    if (i >= a.c) continue;
+    __nv_bfloat16* dst = a.pieces + off + i;
+    split3(v[e], dst[0], dst[plane], dst[2 * plane]);
   }
 }
+
+// dst[k][ld] = src[k][n], padding columns zero: weights TMA cannot read as they are.
+__global__ void pad_weight_kernel(const __nv_bfloat16* __restrict__ src, int k, int n, int ld,
+                                  __nv_bfloat16* __restrict__ dst) {
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= static_cast<long long>(k) * ld) return;
+  const int r = static_cast<int>(idx / ld), c = static_cast<int>(idx % ld);
+  dst[idx] = c < n ? src[static_cast<long long>(r) * n + c] : __float2bfloat16_rn(0.f);
+}
+
+// ---------------------------------------------------------------- product policies
+// float32 activations (three pieces) x bf16 weights as stored. The old CUDA-core kernel took
+// 116 us for 128 x 384 x 384 (six blocks on the whole chip, 24 dependent k steps of scalar
+// loads); the products of a block are 0.6-15 GFLOP, so what bounds them at every size is
+// latency: many small tiles, K split until the tiles cover the SMs.
+//
+// [q | k | v | g] in one launch: column tiles of 64 walk the four weights in turn.
+struct QkvgPolicy {
+  static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
+  static constexpr bool B_MN = true;
+  struct Params {
+    int rows, c, tiles_per_w, first_w;
+    const __nv_bfloat16* q_bias;
+    float* out[4];
+  };
+  static __device__ int b_map(int, int n_tile, int, const Params& p) { return p.first_w + n_tile / p.tiles_per_w; }
+  static __device__ int b_col(int, int n_tile, int, const Params& p) { return n_tile % p.tiles_per_w * BN; }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvgPolicy>& acc, int quarter,
+                                  int half, int lane) {
+    float r[32];
+    acc.load(0, half * 32, r);
+    const int row = m_tile * GEMM_BM + quarter * 32 + lane;
+    const int which = p.first_w + n_tile / p.tiles_per_w, c0 = n_tile % p.tiles_per_w * BN + half * 32;
+    if (row >= p.rows) return;
+    float* dst = p.out[which] + static_cast<long long>(row) * p.c + c0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      float v[4];
+      if (c0 + 4 * q >= p.c) break;  // c is a multiple of 8
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[e] = r[4 * q + e];
+        if (which == 0) v[e] += __bfloat162float(p.q_bias[c0 + 4 * q + e]);
+        if (which == 3) v[e] = 1.0f / (1.0f + expf(-v[e]));
+      }
+      *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+};
+
+// float32 partial sums, one plane per K split.
+struct PartialPolicy {
+  static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
+  static constexpr bool B_MN = true;
+  struct Params {
+    int rows, n;
+    float* out;
+  };
+  static __device__ int b_map(int, int, int, const Params&) { return 0; }
+  static __device__ int b_col(int, int n_tile, int, const Params&) { return n_tile * BN; }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int split, const Accum<PartialPolicy>& acc,
+                                  int quarter, int half, int lane) {
+    float r[32];
+    acc.load(0, half * 32, r);
+    const int row = m_tile * GEMM_BM + quarter * 32 + lane, c0 = n_tile * BN + half * 32;
+    if (row >= p.rows) return;
+    float* dst = p.out + (static_cast<long long>(split) * p.rows + row) * p.n + c0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (c0 + 4 * q < p.n)
+        *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+  }
+};
+
+// 64 columns of x @ fc1 beside the same 64 of x @ fc2; silu(a) * b leaves as pieces
+// (transition.py:108).
+struct SwigluPolicy {
+  static constexpr int BN = 128, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
+  static constexpr bool B_MN = true;
+  struct Params {
+    int rows, hidden;
+    long long pitch;  // of a piece's rows
+    __nv_bfloat16* h;
+  };
+  static __device__ int b_map(int, int, int grp, const Params&) { return grp; }
+  static __device__ int b_col(int, int n_tile, int, const Params&) { return n_tile * 64; }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<SwigluPolicy>& acc, int quarter,
+                                  int half, int lane) {
+    float a[32], b[32];
+    acc.load(0, half * 32, a);
+    acc.load(0, 64 + half * 32, b);
+    const int row = m_tile * GEMM_BM + quarter * 32 + lane, c0 = n_tile * 64 + half * 32;
+    if (row >= p.rows) return;
+    __nv_bfloat16* dst = p.h + static_cast<long long>(row) * p.pitch + c0;
+    const long long plane = static_cast<long long>(p.rows) * p.pitch;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (c0 + 8 * q >= p.pitch) break;  // the pitch is a multiple of 8; padding columns come out as zero
+      uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float av = a[8 * q + 2 * e + u];
+          v[u] = av / (1.0f + expf(-av)) * b[8 * q + 2 * e + u];
+        }
+        split3x2(v[0], v[1], hi[e], mid[e], lo[e]);
+      }
+      *reinterpret_cast<uint4*>(dst + 8 * q) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(dst + plane + 8 * q) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+      *reinterpret_cast<uint4*>(dst + 2 * plane + 8 * q) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+};
 
 // --------------------------------------------------------- token attention
 // One thread per (query i, head h); keys in tiles of 32 staged in shared memory.
@@ -200,8 +316,8 @@ constexpr int TK = 32;  // keys per tile
 
 __global__ void __launch_bounds__(TQ)
 token_attention_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                       const float* __restrict__ bias, const float* __restrict__ mask, int n, int n_keys, int ld,
-                       int c_s, float inf, float* __restrict__ out) {
+                       const float* __restrict__ gate, const float* __restrict__ bias, const float* __restrict__ mask, int n,
+                       int n_keys, int ld, int c_s, float inf, __nv_bfloat16* __restrict__ out) {
   __shared__ float ks[TK][HD], vs[TK][HD], ms[TK];
   const int h = blockIdx.y;
   const int i = blockIdx.x * TQ + threadIdx.x;
@@ -254,29 +370,177 @@ token_attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
   }
   if (live) {
     const float inv = 1.0f / l_run;
+    const long long off = static_cast<long long>(i) * c_s + h * HD, plane = static_cast<long long>(n) * c_s;
 #pragma unroll
-    for (int d = 0; d < HD; ++d) out[static_cast<long long>(i) * c_s + h * HD + d] = acc[d] * inv;
+    for (int d = 0; d < HD; ++d) {  // gated, as the pieces the output projection reads
+      __nv_bfloat16* dst = out + off + d;
+      split3(acc[d] * inv * gate[off + d], dst[0], dst[plane], dst[2 * plane]);
+    }
   }
 }
 
 }  // namespace
 
-int launch_linear_f32(const float* x, const float* gate, const void* w, const void* bias, int M, int K, int N,
-                      int sigmoid, const float* res, float* out, cudaStream_t stream) {
-  const dim3 grid((N + 63) / 64, (M + 63) / 64);
+int launch_row_norm(const RowArgs& a, cudaStream_t stream, bool pdl) {
+  return launch(row_norm_kernel, dim3((a.rows + 3) / 4), dim3(128), 0, stream, pdl, a);
+}
+
+// Enough splits that the tiles cover the SMs, at least two k steps each, none of them empty.
+int single_splits(int tiles, int kb) {
+  int s = 148 / (tiles > 0 ? tiles : 1);
+  s = s > kb / 2 ? kb / 2 : s;
+  s = s > SINGLE_MAX_SPLITS ? SINGLE_MAX_SPLITS : s;
+  if (s <= 1) return 1;
+  const int per = (kb + s - 1) / s;
+  return (kb + per - 1) / per;
+}
+
+size_t tma_weight_bytes(int k, int n) { return static_cast<size_t>(k) * round_up(n, 8) * 2; }
+
+int tma_weight(const void* w, int k, int n, void* scratch, cudaStream_t stream, const void** out, long long* pitch) {
+  *out = w;
+  *pitch = n;
+  if (n % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) return B200TRI_OK;
+  *out = scratch;
+  *pitch = round_up(n, 8);
+  const long long total = static_cast<long long>(k) * *pitch;
+  return launch(pad_weight_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, stream, false,
+                static_cast<const __nv_bfloat16*>(w), k, n, static_cast<int>(*pitch), static_cast<__nv_bfloat16*>(scratch));
+}
+
+static int kblocks(int k) { return (k + GEMM_BK - 1) / GEMM_BK; }
+static int mtiles(int rows) { return (rows + GEMM_BM - 1) / GEMM_BM; }
+
+int launch_linear_partial(const __nv_bfloat16* pieces, long long pitch, int rows, int k, const void* w, int n,
+                          void* w_scratch, float* partial, int* splits, cudaStream_t stream, bool pdl) {
+  const void* wp;
+  long long wpitch;
+  int rc = tma_weight(w, k, n, w_scratch, stream, &wp, &wpitch);
+  if (rc) return rc;
+  GemmMaps maps = {};
+  if ((rc = gemm_map_kmajor(&maps.a[0], pieces, 3, rows, k, pitch, GEMM_BM))) return rc;
+  if ((rc = gemm_map_mnmajor(&maps.b[0], wp, k, n, wpitch))) return rc;
+  GemmShape g = {mtiles(rows), (n + PartialPolicy::BN - 1) / PartialPolicy::BN, 1, {kblocks(k), 0}, nullptr};
+  g.splits = single_splits(g.m_tiles * g.n_tiles, g.kb[0]);
+  *splits = g.splits;
+  return launch_piece_gemm<PartialPolicy>(maps, g, {rows, n, partial}, stream, pdl && wp == w);
+}
+
+int launch_swiglu(const __nv_bfloat16* pieces, int rows, int k, const void* fc1, const void* fc2, int hidden,
+                  void* w1_scratch, void* w2_scratch, __nv_bfloat16* h, long long pitch, cudaStream_t stream, bool pdl) {
+  const void *w1, *w2;
+  long long p1, p2;
+  int rc = tma_weight(fc1, k, hidden, w1_scratch, stream, &w1, &p1);
+  if (rc || (rc = tma_weight(fc2, k, hidden, w2_scratch, stream, &w2, &p2))) return rc;
+  GemmMaps maps = {};
+  if ((rc = gemm_map_kmajor(&maps.a[0], pieces, 3, rows, k, k, GEMM_BM))) return rc;
+  if ((rc = gemm_map_mnmajor(&maps.b[0], w1, k, hidden, p1))) return rc;
+  if ((rc = gemm_map_mnmajor(&maps.b[1], w2, k, hidden, p2))) return rc;
+  const GemmShape g = {mtiles(rows), (hidden + 63) / 64, 1, {kblocks(k), 0}, nullptr};
+  return launch_piece_gemm<SwigluPolicy>(maps, g, {rows, hidden, pitch, h}, stream, pdl && w1 == fc1 && w2 == fc2);
+}
+
+SingleAttentionWork single_attention_work(int n, int c_s, int heads) {
+  SingleAttentionWork w;
+  Carver c(nullptr);
+  const size_t act = static_cast<size_t>(n) * c_s;
+  auto take = [&](size_t bytes) {
+    c.take<uint8_t>(bytes);
+    return c.off - bytes;
+  };
+  w.q = take(act * 4);
+  w.k = take(act * 4);
+  w.v = take(act * 4);
+  w.g = take(act * 4);
+  w.bias = take(static_cast<size_t>(heads) * n * round_up(n, 4) * 4);
+  w.ao = take(act * 2 * 3);
+  for (size_t& off : w.w) off = take(tma_weight_bytes(c_s, c_s));
+  w.total = c.total();
+  return w;
+}
+
+int single_attention(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk,
+                     uint8_t* work, float* partial, int* splits, cudaStream_t stream) {
+  const int n = a->n, c_s = a->c_s, heads = a->heads, ld = round_up(n, 4);
+  const SingleAttentionWork off = single_attention_work(n, c_s, heads);
+  float* out[4] = {reinterpret_cast<float*>(work + off.q), reinterpret_cast<float*>(work + off.k),
+                   reinterpret_cast<float*>(work + off.v), reinterpret_cast<float*>(work + off.g)};
+  float* bias = reinterpret_cast<float*>(work + off.bias);
+  __nv_bfloat16* ao = reinterpret_cast<__nv_bfloat16*>(work + off.ao);
+  auto bf = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
+
+  // q, k, v, g. With separate key-side rows: k, v from those in a launch of their own
+  // (weights in the order q, g | k, v then).
+  const bool same = xq == xk;
+  const void* w_same[4] = {a->proj_q, a->proj_k, a->proj_v, a->proj_g};
+  GemmMaps maps = {};
+  bool direct = true;
+  int rc;
+  for (int i = 0; i < 4; ++i) {
+    const void* wp;
+    long long pitch;
+    if ((rc = tma_weight(w_same[i], c_s, c_s, work + off.w[i], stream, &wp, &pitch))) return rc;
+    if ((rc = gemm_map_mnmajor(&maps.b[i], wp, c_s, c_s, pitch))) return rc;
+    direct = direct && wp == w_same[i];
+  }
+  const int per_w = (c_s + QkvgPolicy::BN - 1) / QkvgPolicy::BN;
+  QkvgPolicy::Params ep = {n, c_s, per_w, 0, bf(a->proj_q_bias), {out[0], out[1], out[2], out[3]}};
+  // (first weight, weight count) of each launch
+  const int runs_same[1][2] = {{0, 4}}, runs_split[3][2] = {{0, 1}, {1, 2}, {3, 1}};
+  const int n_runs = same ? 1 : 3;
+  for (int r = 0; r < n_runs; ++r) {
+    const int* run = same ? runs_same[r] : runs_split[r];
+    if ((rc = gemm_map_kmajor(&maps.a[0], !same && r == 1 ? xk : xq, 3, n, c_s, c_s, GEMM_BM))) return rc;
+    ep.first_w = run[0];
+    const GemmShape g = {mtiles(n), per_w * run[1], 1, {kblocks(c_s), 0}, nullptr};
+    if ((rc = launch_piece_gemm<QkvgPolicy>(maps, g, ep, stream, direct && same))) return rc;
+  }
+  {
+    TimedLaunch timed(K_PAIR_BIAS, stream);
+    const long long n_pairs = static_cast<long long>(n) * n;
+    const long long tiles = (n_pairs + 127) / 128;
+    const long long blocks = tiles < 16LL * sm_count() ? tiles : 16LL * sm_count();
+    count_launch();
+    pair_bias_kernel<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(bf(a->z), n_pairs, n, ld, heads,
+                                                                       bf(a->proj_z_norm_scale), bf(a->proj_z_norm_bias),
+                                                                       bf(a->proj_z), a->eps, bias);
+    B200_CUDA_OK(cudaGetLastError());
+  }
   count_launch();
-  linear_f32_kernel<<<grid, 256, 0, stream>>>(x, gate, static_cast<const __nv_bfloat16*>(w),
-                                              static_cast<const __nv_bfloat16*>(bias), M, K, N, sigmoid, out, res);
+  token_attention_kernel<<<dim3((n + TQ - 1) / TQ, heads), TQ, 0, stream>>>(
+      out[0], out[1], out[2], out[3], bias, static_cast<const float*>(a->mask), n, n, ld, c_s, a->inf, ao);
   B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
+  return launch_linear_partial(ao, c_s, n, c_s, a->proj_o, c_s, work + off.w[4], partial, splits, stream, false);
 }
 
 }  // namespace b200
 
+// Standalone entry: the pieces of s (and of k_in), the attention, the sum of its partials.
+namespace {
+struct StandalonePlan {
+  size_t xq, xk, partial, work, total;
+};
+StandalonePlan standalone_plan(int n, int c_s, int heads) {
+  using namespace b200;
+  StandalonePlan p;
+  Carver c(nullptr);
+  const size_t act = static_cast<size_t>(n) * c_s;
+  auto take = [&](size_t bytes) {
+    c.take<uint8_t>(bytes);
+    return c.off - bytes;
+  };
+  p.xq = take(act * 2 * 3);
+  p.xk = take(act * 2 * 3);
+  p.partial = take(act * 4 * SINGLE_MAX_SPLITS);
+  p.work = take(single_attention_work(n, c_s, heads).total);
+  p.total = c.total();
+  return p;
+}
+}  // namespace
+
 extern "C" size_t b200tri_attention_pair_bias_workspace_bytes(int32_t n, int32_t c_s, int32_t heads) {
   if (n <= 0 || c_s <= 0 || heads <= 0) return 0;
-  const size_t ld = static_cast<size_t>(b200::round_up(n, 4));
-  return (5 * static_cast<size_t>(n) * c_s + static_cast<size_t>(heads) * n * ld) * sizeof(float) + 8 * 1024;
+  return standalone_plan(n, c_s, heads).total + 1024;  // the workspace may start anywhere: aligned up inside
 }
 
 extern "C" int b200tri_attention_pair_bias(const b200tri_attention_pair_bias_args* a, b200tri_stream_t stream_) {
@@ -295,37 +559,30 @@ extern "C" int b200tri_attention_pair_bias(const b200tri_attention_pair_bias_arg
   const size_t need = b200tri_attention_pair_bias_workspace_bytes(a->n, a->c_s, a->heads);
   B200_REQUIRE(a->workspace && a->workspace_bytes >= need, B200TRI_ERR_WORKSPACE,
                "attention pair bias: workspace of %zu bytes needed", need);
-  const int n = a->n, c_s = a->c_s, heads = a->heads;
-  const int ld = round_up(n, 4);
-  Carver ws(a->workspace);
-  const size_t act = static_cast<size_t>(n) * c_s;
-  float* q = ws.take<float>(act);
-  float* g = ws.take<float>(act);
-  float* k = ws.take<float>(act);
-  float* v = ws.take<float>(act);
-  float* ao = ws.take<float>(act);
-  float* bias = ws.take<float>(static_cast<size_t>(heads) * n * ld);
-  const float* s = static_cast<const float*>(a->s);
-  const float* k_in = a->k_in ? static_cast<const float*>(a->k_in) : s;
-  auto bf = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  const dim3 lin_grid((c_s + 63) / 64, (n + 63) / 64);
-  count_launch(7);
-  linear_f32_kernel<<<lin_grid, 256, 0, stream>>>(s, nullptr, bf(a->proj_q), bf(a->proj_q_bias), n, c_s, c_s, 0, q);
-  linear_f32_kernel<<<lin_grid, 256, 0, stream>>>(s, nullptr, bf(a->proj_g), nullptr, n, c_s, c_s, 1, g);
-  linear_f32_kernel<<<lin_grid, 256, 0, stream>>>(k_in, nullptr, bf(a->proj_k), nullptr, n, c_s, c_s, 0, k);
-  linear_f32_kernel<<<lin_grid, 256, 0, stream>>>(k_in, nullptr, bf(a->proj_v), nullptr, n, c_s, c_s, 0, v);
-  {
-    TimedLaunch timed(K_PAIR_BIAS, stream);
-    const long long n_pairs = static_cast<long long>(n) * n;
-    const long long tiles = (n_pairs + 127) / 128;
-    const long long blocks = tiles < 16LL * sm_count() ? tiles : 16LL * sm_count();
-    pair_bias_kernel<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(bf(a->z), n_pairs, n, ld, heads,
-                                                                       bf(a->proj_z_norm_scale), bf(a->proj_z_norm_bias),
-                                                                       bf(a->proj_z), a->eps, bias);
+  const StandalonePlan pl = standalone_plan(a->n, a->c_s, a->heads);
+  uint8_t* ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(a->workspace) + 1023) & ~uintptr_t(1023));
+  __nv_bfloat16* xq = reinterpret_cast<__nv_bfloat16*>(ws + pl.xq);
+  __nv_bfloat16* xk = xq;
+  float* partial = reinterpret_cast<float*>(ws + pl.partial);
+  RowArgs row = {};
+  row.rows = a->n;
+  row.c = a->c_s;
+  row.base = static_cast<const float*>(a->s);
+  row.pieces = xq;
+  int rc = launch_row_norm(row, stream, false);
+  if (rc) return rc;
+  if (a->k_in && a->k_in != a->s) {
+    xk = reinterpret_cast<__nv_bfloat16*>(ws + pl.xk);
+    row.base = static_cast<const float*>(a->k_in);
+    row.pieces = xk;
+    if ((rc = launch_row_norm(row, stream, false))) return rc;
   }
-  token_attention_kernel<<<dim3((n + TQ - 1) / TQ, heads), TQ, 0, stream>>>(q, k, v, bias, static_cast<const float*>(a->mask),
-                                                                          n, n, ld, c_s, a->inf, ao);
-  linear_f32_kernel<<<lin_grid, 256, 0, stream>>>(ao, g, bf(a->proj_o), nullptr, n, c_s, c_s, 0, static_cast<float*>(a->out));
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
+  int splits = 1;
+  if ((rc = single_attention(a, xq, xk, ws + pl.work, partial, &splits, stream))) return rc;
+  row.base = nullptr;
+  row.partial = partial;
+  row.splits = splits;
+  row.pieces = nullptr;
+  row.sum_out = static_cast<float*>(a->out);
+  return launch_row_norm(row, stream, true);
 }

@@ -241,6 +241,21 @@ __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t saddr, uint32_t ro
   d |= swz << 61;
   return d;
 }
+// The same for an MN-major tile under the 128-byte swizzle: smem row = one k, 128 B = 64
+// consecutive M (or N) elements, eight k rows per atom. `group_bytes` separates successive
+// groups of 64 M/N elements; atoms along K follow one another every 1024 bytes, so stepping
+// K by 16 advances the start address by 2048. A linear kernel stored [in][out] is loaded by
+// TMA straight into this form: no transposed copy of a weight is ever made.
+__device__ __forceinline__ uint64_t umma_desc_mnmajor(uint32_t saddr, uint32_t group_bytes) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>((group_bytes >> 4) & 0x3FFFu) << 16;
+  d |= static_cast<uint64_t>((1024u >> 4) & 0x3FFFu) << 32;
+  d |= 1ull << 46;
+  d |= 2ull << 61;
+  return d;
+}
+constexpr uint32_t UMMA_A_MN = 1u << 15, UMMA_B_MN = 1u << 16;  // instruction descriptor: operand is MN-major
 // Step the descriptor along K by `bytes` inside the swizzled row.
 __device__ __forceinline__ uint64_t umma_desc_advance(uint64_t d, uint32_t bytes) { return d + (bytes >> 4); }
 
@@ -353,6 +368,13 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk) {
   return row * 128u + (((chunk ^ row) & 7u) << 4);
 }
+
+// Programmatic dependent launch. A kernel launched with the attribute may start while its
+// predecessor in the stream still runs; pdl_wait() returns once that predecessor has finished
+// and its writes are visible. pdl_trigger() lets the successor be scheduled as soon as every
+// CTA of this grid has got there. Both do nothing in a plain launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Named barrier among `nthreads` threads (id 1..15; 0 is __syncthreads()).
 __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t nthreads) {

@@ -1,0 +1,62 @@
+"""The block's float32 single track (split-bf16 products on the tensor cores) at the sizes where
+its tiles end: rows around 128, few heads, hidden widths that are no multiple of 8 or 64 (the
+padded weight copy), weights TMA cannot read in place, and K split over several partial sums.
+
+Given the pair tensor the block produced, the single track is recomputed in float64 on the same
+bf16 weights. Tolerance 2e-4, the reference test's own for this op
+(tests/models/boltz2/test_attention_checkpoint_parity.py:47-52); float32 sums over at most 1536
+products of order one stay below 1536 * 2^-24 = 1e-4 of their scale."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import triangle_oracle as orc
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _params(rng, heads, hidden):
+    c_s = 24 * heads
+    params = orc.random_pairformer_params(rng, c_s=c_s, heads_s=heads, std=0.05, ln_noise=0.1)
+    w = lambda *shape: (rng.standard_normal(shape) * 0.05).astype(np.float32)
+    params["transition_s"] = {"norm": params["transition_s"]["norm"], "fc1": {"kernel": w(c_s, hidden)},
+                              "fc2": {"kernel": w(c_s, hidden)}, "fc3": {"kernel": w(hidden, c_s)}}
+    return orc.round_params(params, "bfloat16")
+
+
+def _misaligned(t):
+    """The same values 2 bytes off a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    buf[1:] = t.reshape(-1)
+    return buf[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("n,heads,hidden,shift", [(1, 1, 8, False), (127, 4, 100, False), (129, 16, 1536, False),
+                                                  (128, 16, 1537, True), (260, 3, 64, False), (40, 16, 36, True)])
+def test_single_track_against_float64(cuda_device, n, heads, hidden, shift):
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.pairformer import pairformer_forward
+
+    rng = np.random.default_rng(n + hidden)
+    params = _params(rng, heads, hidden)
+    z = orc.round_bf16(rng.standard_normal((1, n, n, 128)).astype(np.float32))
+    s = rng.standard_normal((1, n, 24 * heads)).astype(np.float32)
+    mask = (rng.random((1, n)) < 0.9).astype(np.float32)
+    mask[0, 0] = 1.0
+    pd = dev.params_to_device(params)
+    if shift:
+        for group, names in (("attention", ("proj_q", "proj_k", "proj_v", "proj_g", "proj_o")),
+                             ("transition_s", ("fc1", "fc2", "fc3"))):
+            for name in names:
+                pd[group][name]["kernel"] = _misaligned(pd[group][name]["kernel"])
+    s_got, z_got = pairformer_forward([pd], torch.from_numpy(s).cuda(), dev.to_device(z, torch.bfloat16),
+                                      torch.from_numpy(mask).cuda(), torch.ones(1, n, n, device="cuda"))
+    _lib.device_status()
+    s_got, z_got = s_got.cpu().numpy(), z_got.float().cpu().numpy()
+    sn = orc.layer_norm(s, params["pre_norm_s"]["scale"], params["pre_norm_s"]["bias"], 1e-5)
+    ref = s + orc.attention_pair_bias(params["attention"], sn, z_got, mask, k_in=sn, dtype="float64")
+    ref = ref + orc.transition(params["transition_s"], ref, dtype="float64")
+    np.testing.assert_allclose(s_got, ref, rtol=2e-4, atol=2e-4)
