@@ -185,6 +185,7 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     B200_CUDA_OK(cudaGetLastError());
     return B200TRI_OK;
   };
+  PdlChain chain(false);
   for (int layer = 0; layer < a->n_blocks; ++layer) {
     const b200tri_pairformer_block_params P =
         a->stacked ? unstack(first, layer, c_s, a->heads_s) : a->params[layer];
@@ -246,6 +247,7 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
         t.workspace_bytes = pl.sub_bytes;
         if ((rc = b200tri_triatt_forward(&t, stream_))) return rc;
       }
+      chain.set();
       if (gate && (rc = gate_pairs(dst, dst))) return rc;
       z_cur = dst;
     }

@@ -101,6 +101,38 @@ int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
   return B200TRI_OK;
 }
 
+// While one of these lives, the library's launches on this host thread are chained: the kernel
+// before the next one in the stream was launched by the same call. A chained kernel may start
+// early (launch with pdl) and may read the caller's weights before pdl_wait(): every kernel of
+// the library triggers its successor only after its own pdl_wait(), so whatever wrote the
+// weights has finished by then.
+struct PdlChain {
+  bool before;
+  explicit PdlChain(bool on = true);
+  void set();
+  ~PdlChain();
+};
+bool pdl_chained();
+
+// A weight as TMA needs it: `w` itself when it is 16-byte aligned, else a copy in `scratch`.
+int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stream, const void** out);
+
+// Tensor map over a [k][n] bf16 linear kernel as stored (row pitch n), read in boxes of 64
+// columns x `box_k` rows: MN-major operand tiles under the 128-byte swizzle.
+int make_weight_map(CUtensorMap* out, const void* w, int k, int n, int box_k);
+
+// The mask-bias rows of the attention core, written by the projection stage of the same call.
+struct MaskBiasOut {
+  const float* mask;  // null = all ones
+  long long ms_outer, ms_inner;
+  float inf;
+  float* out;  // [n_outer][ld]
+  int ld;
+};
+int att_project_launch(const b200tri_triatt_project_args* a, const MaskBiasOut* mb, cudaStream_t stream);
+// The core with its mask-bias rows already in the workspace.
+int att_core_launch_premasked(const b200tri_triatt_core_args* a, cudaStream_t stream);
+
 // The two module-level ops for every shape / element type outside the tensor-core
 // specialisation (generic.cu): other channel and head counts, float32 trunks.
 size_t trimul_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t c_hidden, int32_t dtype);

@@ -13,6 +13,12 @@ namespace b200 {
 
 constexpr int SLAB_BYTES = 128 * 128;  // 128 rows x 64 bf16
 
+// Channel pair `i` of a bf16 layer-norm parameter, packed (any alignment).
+__device__ __forceinline__ uint32_t ln_param_pair(const void* p, int i) {
+  const unsigned short* h = static_cast<const unsigned short*>(p) + 2 * i;
+  return static_cast<uint32_t>(h[0]) | (static_cast<uint32_t>(h[1]) << 16);
+}
+
 // v[0..7] = slab 0 chunks, v[8..15] = slab 1 chunks (16 bytes = 8 channels each).
 __device__ __forceinline__ void ln_load_row(const uint8_t* tile, int row, uint4 (&v)[16]) {
 #pragma unroll

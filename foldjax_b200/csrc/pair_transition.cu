@@ -47,8 +47,8 @@ constexpr int NWORK = 4;  // activation warpgroups
 constexpr int THREADS = 64 + 128 + NWORK * 128;
 
 struct Smem {
-  uint8_t w12[WSTAGES][2 * SLAB_BYTES];  // rows 0-63: W1 chunk, 64-127: W2 chunk; [128][128 in] as two K slabs
-  uint8_t w3[WSTAGES][SLAB_BYTES];       // [128 out][64 hidden]
+  uint8_t w12[WSTAGES][2 * SLAB_BYTES];  // fc1 and fc2 of the chunk: [128 in][64 hidden] each, MN-major
+  uint8_t w3[WSTAGES][SLAB_BYTES];       // fc3 of the chunk: two boxes [64 hidden][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
   uint8_t h[SLAB_BYTES];                 // [128 pairs][64 hidden]
   uint32_t gamma2[64], beta2[64];
@@ -61,7 +61,8 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 struct Params {
   long long rows, total_tiles;
   int nchunks;         // hidden / 64
-  const uint32_t* ln;  // gamma, beta: 2 x 64 words
+  const void* gamma;
+  const void* beta;
   const __nv_bfloat16* residual;
   const float* row_mask;
   __nv_bfloat16* out;
@@ -78,8 +79,9 @@ __device__ __forceinline__ uint32_t swiglu_bf16x2(float a0, float a1, float b0, 
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
-pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w12,
-                       const __grid_constant__ CUtensorMap tm_w3, const Params p) {
+pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1,
+                       const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_w3,
+                       const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -90,7 +92,8 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   }
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_x);
-    tma_prefetch_desc(&tm_w12);
+    tma_prefetch_desc(&tm_w1);
+    tma_prefetch_desc(&tm_w2);
     tma_prefetch_desc(&tm_w3);
     for (int s = 0; s < WSTAGES; ++s) {
       mbar_init(&sm.w_full[s], 1);
@@ -115,9 +118,11 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = p.ln[threadIdx.x - 64];
-    sm.beta2[threadIdx.x - 64] = p.ln[64 + threadIdx.x - 64];
+    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
+    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
   }
   tc_fence_before();
   __syncthreads();
@@ -155,14 +160,15 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
         const uint32_t ph = static_cast<uint32_t>((n / WSTAGES) & 1);
         if (!mbar_wait(&sm.w_empty[ws], ph ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.w_full[ws], 3 * SLAB_BYTES);
-        tma_load_2d(sm.w12[ws], &tm_w12, &sm.w_full[ws], 0, c * 128);
-        tma_load_2d(sm.w12[ws] + SLAB_BYTES, &tm_w12, &sm.w_full[ws], 64, c * 128);
-        tma_load_2d(sm.w3[ws], &tm_w3, &sm.w_full[ws], c * HC, 0);
+        tma_load_2d(sm.w12[ws], &tm_w1, &sm.w_full[ws], c * HC, 0);
+        tma_load_2d(sm.w12[ws] + SLAB_BYTES, &tm_w2, &sm.w_full[ws], c * HC, 0);
+        tma_load_2d(sm.w3[ws], &tm_w3, &sm.w_full[ws], 0, c * HC);
+        tma_load_2d(sm.w3[ws] + SLAB_BYTES / 2, &tm_w3, &sm.w_full[ws], 64, c * HC);
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
       for (long long n = 0; n <= total_n; ++n) {
         if (n < total_n) {  // first product of chunk step n
           const long long it = n / nchunks;
@@ -174,14 +180,12 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
           if (!mbar_wait(&sm.w_full[ws], static_cast<uint32_t>((n / WSTAGES) & 1), p.status, ST_TIMEOUT_MMA)) break;
           if (!mbar_wait(&sm.d1_empty[d], static_cast<uint32_t>(((n >> 1) & 1) ^ 1), p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
+          const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w12[ws]), SLAB_BYTES);
 #pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.x[xs]) + s * SLAB_BYTES, 128);
-            const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.w12[ws]) + s * SLAB_BYTES, 128);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_ss(tmem_base + d * 128, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
-                           (s | k) != 0);
+          for (int k = 0; k < 8; ++k) {
+            const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.x[xs]) + (k >> 2) * SLAB_BYTES, 128);
+            umma_bf16_ss(tmem_base + d * 128, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc,
+                         k != 0);
           }
           umma_commit(&sm.d1_full[d]);
           if (c == nchunks - 1) umma_commit(&sm.x_empty[xs]);  // every first product of the tile has been issued
@@ -196,10 +200,10 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
           if (!mbar_wait(&sm.h_full, static_cast<uint32_t>(m & 1), p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
           const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.h), 128);
-          const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.w3[ws]), 128);
+          const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w3[ws]), SLAB_BYTES / 2);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem_base + 256 + tb * 128, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32),
+            umma_bf16_ss(tmem_base + 256 + tb * 128, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 2048),
                          idesc, (c | k) != 0);
           umma_commit(&sm.w_empty[ws]);  // covers both products that read this stage
           umma_commit(&sm.h_empty);
@@ -314,31 +318,6 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-// Weight repacking (every call; a few microseconds). The reference stores linear
-// kernels as [in, out]; the tensor core wants K-major rows.
-// w12[(c * 128 + r) * 128 + k] = r < 64 ? fc1[k][c * 64 + r] : fc2[k][c * 64 + r - 64]
-__global__ void pack_w12_kernel(const __nv_bfloat16* __restrict__ fc1, const __nv_bfloat16* __restrict__ fc2, int hidden,
-                                __nv_bfloat16* __restrict__ dst) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 2 * hidden * 128) return;
-  const int k = idx & 127, rr = idx >> 7;
-  const int c = rr >> 7, r = rr & 127;
-  const __nv_bfloat16* src = r < HC ? fc1 : fc2;
-  dst[idx] = src[static_cast<long long>(k) * hidden + c * HC + (r & (HC - 1))];
-}
-// w3[o * hidden + h] = fc3[h][o]
-__global__ void pack_w3_kernel(const __nv_bfloat16* __restrict__ fc3, int hidden, __nv_bfloat16* __restrict__ dst) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= hidden * 128) return;
-  const int h = idx % hidden, o = idx / hidden;
-  dst[idx] = fc3[static_cast<long long>(h) * 128 + o];
-}
-__global__ void pack_ln_kernel(const uint32_t* __restrict__ scale, const uint32_t* __restrict__ bias,
-                               uint32_t* __restrict__ dst) {
-  const int idx = threadIdx.x;
-  dst[idx] = idx < 64 ? scale[idx] : bias[idx - 64];
-}
-
 }  // namespace
 }  // namespace b200
 
@@ -367,22 +346,17 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
   int* status = device_status_word();
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "pair transition: no current CUDA device");
 
+  // the weights are read in place; the workspace is only for one that is not 16-byte aligned
   Carver ws(a->workspace);
-  __nv_bfloat16* w12 = ws.take<__nv_bfloat16>(static_cast<size_t>(2) * a->hidden * 128);
-  __nv_bfloat16* w3 = ws.take<__nv_bfloat16>(static_cast<size_t>(a->hidden) * 128);
-  uint32_t* ln = ws.take<uint32_t>(128, 256);
-  {
-    const int total = 2 * a->hidden * 128;
-    count_launch(3);
-    pack_w12_kernel<<<(total + 255) / 256, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(a->fc1),
-                                                            static_cast<const __nv_bfloat16*>(a->fc2), a->hidden, w12);
-    pack_w3_kernel<<<(a->hidden * 128 + 255) / 256, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(a->fc3), a->hidden, w3);
-    pack_ln_kernel<<<1, 128, 0, stream>>>(static_cast<const uint32_t*>(a->norm_scale),
-                                          static_cast<const uint32_t*>(a->norm_bias), ln);
-    B200_CUDA_OK(cudaGetLastError());
+  const size_t w_elems = static_cast<size_t>(a->hidden) * 128;
+  const void* const w_in[3] = {a->fc1, a->fc2, a->fc3};
+  const void* w[3];
+  for (int i = 0; i < 3; ++i) {
+    const int rc = aligned_weight(w_in[i], w_elems * 2, ws.take<__nv_bfloat16>(w_elems), stream, &w[i]);
+    if (rc) return rc;
   }
 
-  CUtensorMap tm_x, tm_w12, tm_w3;
+  CUtensorMap tm_x, tm_w1, tm_w2, tm_w3;
   {
     const uint64_t dims[2] = {128, (uint64_t)a->rows};
     const uint64_t str[1] = {256};
@@ -391,24 +365,16 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
     if (rc) return rc;
   }
   {
-    const uint64_t dims[2] = {128, (uint64_t)2 * a->hidden};
-    const uint64_t str[1] = {256};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w12, w12, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
-    if (rc) return rc;
-  }
-  {
-    const uint64_t dims[2] = {(uint64_t)a->hidden, 128};
-    const uint64_t str[1] = {(uint64_t)a->hidden * 2};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w3, w3, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
-    if (rc) return rc;
+    int rc = make_weight_map(&tm_w1, w[0], 128, a->hidden, 128);
+    if (rc || (rc = make_weight_map(&tm_w2, w[1], 128, a->hidden, 128))) return rc;
+    if ((rc = make_weight_map(&tm_w3, w[2], a->hidden, 128, HC))) return rc;
   }
   Params p;
   p.rows = a->rows;
   p.total_tiles = (a->rows + 127) / 128;
   p.nchunks = a->hidden / HC;
-  p.ln = ln;
+  p.gamma = a->norm_scale;
+  p.beta = a->norm_bias;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
   p.row_mask = a->row_mask;
   p.out = static_cast<__nv_bfloat16*>(a->out);
@@ -422,9 +388,7 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_PAIR_TRANSITION, stream);
-    count_launch();
-    pair_transition_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_x, tm_w12, tm_w3, p);
+    return launch(pair_transition_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x,
+                  tm_w1, tm_w2, tm_w3, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }

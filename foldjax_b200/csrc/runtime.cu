@@ -68,6 +68,28 @@ int sm_count() {
   return n - t_sm_reserve > 8 ? n - t_sm_reserve : n;
 }
 
+static thread_local bool t_pdl_chain = false;
+
+PdlChain::PdlChain(bool on) : before(t_pdl_chain) { t_pdl_chain = before || on; }
+void PdlChain::set() { t_pdl_chain = true; }
+PdlChain::~PdlChain() { t_pdl_chain = before; }
+bool pdl_chained() { return t_pdl_chain; }
+
+int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stream, const void** out) {
+  *out = w;
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) return B200TRI_OK;
+  *out = scratch;
+  B200_CUDA_OK(cudaMemcpyAsync(scratch, w, bytes, cudaMemcpyDeviceToDevice, stream));
+  return B200TRI_OK;
+}
+
+int make_weight_map(CUtensorMap* out, const void* w, int k, int n, int box_k) {
+  const uint64_t dims[2] = {static_cast<uint64_t>(n), static_cast<uint64_t>(k)};
+  const uint64_t str[1] = {static_cast<uint64_t>(n) * 2};
+  const uint32_t box[2] = {64, static_cast<uint32_t>(box_k)};
+  return make_tmap(out, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
+}
+
 int ensure_smem_limit(const void* kernel, int bytes) {
   static std::mutex mu;
   static std::vector<std::pair<const void*, int>> done;

@@ -363,6 +363,14 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// Mask bias of one key: inf * (mask - 1), or the caller's additive bias as it is. A value at or
+// below MASKED_SCORE replaces the score (see the attention core). fmaxf drops a NaN operand, so a
+// NaN bias would silently become "keep": it is mapped to "drop".
+constexpr float MASKED_SCORE = -30000.0f;
+__device__ __forceinline__ float mask_bias(float m, float inf, bool additive) {
+  const float b = additive ? m : inf * (m - 1.0f);
+  return (b == b) ? fmaxf(b, MASKED_SCORE) : MASKED_SCORE;
+}
 // Byte offset of (row, 16-byte chunk) inside a K-major tile with 128-byte rows
 // under the 128-byte swizzle (the layout TMA writes and tcgen05.mma reads).
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk) {

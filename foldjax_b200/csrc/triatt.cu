@@ -115,8 +115,16 @@ extern "C" int b200tri_triatt_forward(const b200tri_triatt_args* a, b200tri_stre
   pa.bias_head_stride = n * pl.ld;
   pa.workspace = ws + pl.off_proj;
   pa.workspace_bytes = b200tri_triatt_project_workspace_bytes();
-  int rc = b200tri_triatt_project(&pa, stream);
+  // (the projection also writes the core's mask-bias rows: one launch less)
+  const MaskBiasOut mb = {a->mask,
+                          a->starting ? n : 1,
+                          a->starting ? 1 : n,
+                          a->inf,
+                          reinterpret_cast<float*>(ws + pl.off_core),
+                          round_up(a->n, 64)};
+  int rc = att_project_launch(&pa, &mb, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
+  PdlChain chain;
 
   b200tri_triatt_core_args ca = {};
   ca.n_i = ca.n_j = ca.n_k = a->n;
@@ -136,7 +144,7 @@ extern "C" int b200tri_triatt_forward(const b200tri_triatt_args* a, b200tri_stre
   ca.o = ws + pl.off_o;
   ca.workspace = ws + pl.off_core;
   ca.workspace_bytes = b200tri_triatt_core_workspace_bytes(a->n, a->n);
-  rc = b200tri_triatt_core(&ca, stream);
+  rc = att_core_launch_premasked(&ca, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
 
   b200tri_triatt_finish_args fa = {};

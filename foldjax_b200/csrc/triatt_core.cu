@@ -90,7 +90,7 @@ constexpr float EXP_MAGIC = 12582912.0f;  // 1.5 * 2^23: adding it leaves round(
 // has the same two effects (zero weight beside any valid key, uniform without one)
 // while keeping the softmax offset small enough for a single fp32 fma per
 // exponent. Smaller mask biases (soft masks) are added as they are.
-constexpr float MASKED_SCORE = -30000.0f;
+// (MASKED_SCORE and the rule itself: mask_bias() in tc.cuh)
 
 struct Smem {
   uint8_t q[NWG][Q_BYTES];
@@ -224,6 +224,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
   const uint32_t tmem_base = sm.tmem_base;
   const int items_per_head = p.groups * p.tiles_j;
 
@@ -634,10 +636,7 @@ __global__ void mask_bias_kernel(const float* __restrict__ mask, long long ms_i,
   const int i = static_cast<int>(idx / ld), k = static_cast<int>(idx % ld);
   float v = -INFINITY;
   if (k < n_k && mask) {
-    const float m = mask[i * ms_i + k * ms_k];
-    // fmaxf drops a NaN operand, so a NaN bias would silently become "keep": map it to "drop"
-    const float b = additive ? m : inf * (m - 1.0f);
-    v = (b == b) ? fmaxf(b, MASKED_SCORE) : MASKED_SCORE;
+    v = mask_bias(mask[i * ms_i + k * ms_k], inf, additive);
   } else if (k < n_k) {
     v = 0.0f;
   }
@@ -660,11 +659,16 @@ extern "C" size_t b200tri_triatt_core_multi_workspace_bytes(int32_t n_i, int32_t
 namespace {
 // `may_time` = false keeps the launch free of event creation whatever the timing switch
 // says at that moment (the allocation-free entry point relies on it).
-int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time);
+int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time,
+                bool premasked = false);
 }  // namespace
 
 extern "C" int b200tri_triatt_core(const b200tri_triatt_core_args* a, b200tri_stream_t stream) {
   return core_launch(a, 1, stream, true);
+}
+
+int b200::att_core_launch_premasked(const b200tri_triatt_core_args* a, cudaStream_t stream) {
+  return core_launch(a, 1, reinterpret_cast<b200tri_stream_t>(stream), true, true);
 }
 
 extern "C" int b200tri_triatt_core_multi(const b200tri_triatt_core_args* tiles, int32_t n_tiles,
@@ -673,7 +677,8 @@ extern "C" int b200tri_triatt_core_multi(const b200tri_triatt_core_args* tiles, 
 }
 
 namespace {
-int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time) {
+int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time,
+                bool premasked) {
   using namespace b200;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   B200_REQUIRE(tiles != nullptr, B200TRI_ERR_INVALID, "att core: null args");
@@ -708,7 +713,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
                      ti->bias_ld >= a->n_k,
                  B200TRI_ERR_INVALID, "att core: pitches must be multiples of 8 elements and cover n_k");
     float* mb = reinterpret_cast<float*>(static_cast<uint8_t*>(a->workspace) + need_one * t);
-    {
+    if (!premasked) {
       const long long total = static_cast<long long>(a->n_i) * ldm;
       count_launch();
       mask_bias_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(
@@ -783,11 +788,8 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   const long long grid = p.total_items < sm_count() ? p.total_items : sm_count();
   {
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
-    count_launch();
-    att_core_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_q, tm, p);
+    return launch(att_core_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tm, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }
 }  // namespace
 

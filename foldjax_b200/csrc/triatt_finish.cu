@@ -20,7 +20,6 @@
 // Bound: HBM (read x and o, write out: 3 * n*n*128*2 bytes; + residual).
 #include "host.cuh"
 #include "ln.cuh"
-#include "pack.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -39,7 +38,7 @@ constexpr int EPI_THREAD0 = 192;  // first thread of the epilogue warps
 #endif
 
 struct Smem {
-  uint8_t w[4 * SLAB_BYTES];  // Wg^T (2 slabs), Wo^T (2 slabs)
+  uint8_t w[4 * SLAB_BYTES];  // Wg, Wo: two boxes [128 in][64 out] each, MN-major
   uint8_t x[STAGES][TILE_BYTES];
   uint8_t o[STAGES][TILE_BYTES];
 #if B200_AFIN_TMASTORE
@@ -55,7 +54,9 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 struct Params {
   int n_outer, n_inner, tiles_inner;
   long long total_tiles;
-  const uint32_t* ln;  // gamma, beta: 2 x 64 words
+  const void* gamma;
+  const void* beta;
+  bool early_weights;  // the weights may be read before pdl_wait()
   const __nv_bfloat16* residual;
   __nv_bfloat16* out;
   long long os_outer, os_inner;
@@ -65,8 +66,8 @@ struct Params {
 
 __global__ void __launch_bounds__(THREADS, 1)
 att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_o,
-                  const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_out,
-                  const Params p) {
+                  const __grid_constant__ CUtensorMap tm_wg, const __grid_constant__ CUtensorMap tm_wo,
+                  const __grid_constant__ CUtensorMap tm_out, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -78,7 +79,8 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_x);
     tma_prefetch_desc(&tm_o);
-    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_wg);
+    tma_prefetch_desc(&tm_wo);
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.in_full[s], 1);
@@ -98,21 +100,27 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
+  if (!p.early_weights) pdl_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = p.ln[threadIdx.x - 64];
-    sm.beta2[threadIdx.x - 64] = p.ln[64 + threadIdx.x - 64];
+    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
+    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
+  }
+  if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
+    mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
+    for (int g = 0; g < 2; ++g)
+      for (int s = 0; s < 2; ++s)
+        tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, g ? &tm_wo : &tm_wg, &sm.w_full, s * 64, 0);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
   // TMEM: buffer a (= tile parity): G at a*256, OUT at a*256 + 128.
+  if (p.early_weights) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
-      for (int g = 0; g < 2; ++g)
-        for (int s = 0; s < 2; ++s) tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, &tm_w, &sm.w_full, s * 64, g * 128);
       int stage = 0;
       uint32_t phase = 0;
       for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
@@ -132,19 +140,16 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       // Two products per tile; the second of tile t is issued after the first of
       // tile t+1, mirroring the order in which the gating warps deliver operands.
       auto product = [&](uint32_t d_tmem, uint32_t a_smem, int wgroup) {
+        const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w + wgroup * 2 * SLAB_BYTES), SLAB_BYTES);
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const uint64_t adesc = umma_desc_kmajor(a_smem + s * SLAB_BYTES, 128);
-          const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.w + (wgroup * 2 + s) * SLAB_BYTES), 128);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(d_tmem, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
-                         (s | k) != 0);
+        for (int k = 0; k < 8; ++k) {
+          const uint64_t adesc = umma_desc_kmajor(a_smem + (k >> 2) * SLAB_BYTES, 128);
+          umma_bf16_ss(d_tmem, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc, k != 0);
         }
       };
       long long n_my = 0;
@@ -327,15 +332,16 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
   int* status = device_status_word();
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "att finish: no current CUDA device");
 
+  // the weights are read in place; the workspace is only for one that is not 16-byte aligned
   Carver ws(a->workspace);
-  __nv_bfloat16* wpk = ws.take<__nv_bfloat16>(256 * 128);
-  uint32_t* ln = ws.take<uint32_t>(128, 256);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_g), 128, 0, 128, wpk, stream);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_o), 128, 0, 128, wpk + 128 * 128, stream);
-  pack_copy_words(a->norm_scale, ln, 64, stream);
-  pack_copy_words(a->norm_bias, ln + 64, 64, stream);
-
-  CUtensorMap tm_x, tm_o, tm_w, tm_out;
+  const void *w_g, *w_o;
+  {
+    void* s0 = ws.take<__nv_bfloat16>(128 * 128);
+    void* s1 = ws.take<__nv_bfloat16>(128 * 128);
+    int rc = aligned_weight(a->w_g, 128 * 128 * 2, s0, stream, &w_g);
+    if (rc || (rc = aligned_weight(a->w_o, 128 * 128 * 2, s1, stream, &w_o))) return rc;
+  }
+  CUtensorMap tm_x, tm_o, tm_wg, tm_wo, tm_out;
   {  // the result through the caller's strides (the ending node lands transposed back in place)
     const uint64_t dims[3] = {128, (uint64_t)a->n_inner, (uint64_t)a->n_outer};
     const uint64_t str[2] = {(uint64_t)a->os_inner * 2, (uint64_t)a->os_outer * 2};
@@ -358,18 +364,17 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
     if (rc) return rc;
   }
   {
-    const uint64_t dims[2] = {128, 256};
-    const uint64_t str[1] = {256};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w, wpk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
-    if (rc) return rc;
+    int rc = make_weight_map(&tm_wg, w_g, 128, 128, 128);
+    if (rc || (rc = make_weight_map(&tm_wo, w_o, 128, 128, 128))) return rc;
   }
   Params p;
   p.n_outer = a->n_outer;
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
   p.total_tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
-  p.ln = ln;
+  p.gamma = a->norm_scale;
+  p.beta = a->norm_bias;
+  p.early_weights = pdl_chained() && w_g == a->w_g && w_o == a->w_o;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
   p.out = static_cast<__nv_bfloat16*>(a->out);
   p.os_outer = a->os_outer;
@@ -384,9 +389,7 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_TRIATT_FINISH, stream);
-    count_launch();
-    att_finish_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_x, tm_o, tm_w, tm_out, p);
+    return launch(att_finish_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_o,
+                  tm_wg, tm_wo, tm_out, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }

@@ -34,7 +34,6 @@
 
 #include "host.cuh"
 #include "ln.cuh"
-#include "pack.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -53,7 +52,8 @@ constexpr int XSTAGES = 2;
 constexpr int XSTAGES = 3;
 #endif
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
-constexpr int W_BYTES = 8 * SLAB_BYTES;  // rows 0..255 [Wq|Wk], 256..383 Wv, 384..399 Wb, rest zero
+constexpr int W_BYTES = 6 * SLAB_BYTES;  // Wq, Wk, Wv: two boxes [128 in][64 out] each, MN-major
+constexpr int WB_SLAB = 16 * 128;        // Wb, K-major: [16 heads (4 used)][64 in], two slabs
 constexpr int LN_WARPS = 8;  // two threads per pair
 constexpr int THREADS = 64 + LN_WARPS * 32 + 128;
 constexpr int EPI_THREAD0 = 64 + LN_WARPS * 32;  // first thread of the epilogue warps
@@ -62,6 +62,7 @@ enum { G_QK = 0, G_B = 1, G_V = 2 };
 
 struct Smem {
   uint8_t w[W_BYTES];
+  uint8_t wb[2 * WB_SLAB];
   uint8_t x[XSTAGES][TILE_BYTES];
 #if B200_APROJ_TMASTORE
   uint8_t out[TILE_BYTES];  // staging of one 32 KiB output tile (q, then k, then vT)
@@ -76,8 +77,11 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 struct Params {
   int n_outer, n_inner, tiles_inner;
   long long total_tiles;
-  const uint32_t* gamma2;
-  const uint32_t* beta2;
+  const void* gamma;
+  const void* beta;
+  const __nv_bfloat16* w_bias;  // [128][4]
+  bool early_weights;           // the weights may be read before pdl_wait()
+  MaskBiasOut mb;               // mb.out null: no mask-bias rows wanted
   __nv_bfloat16* q;
   __nv_bfloat16* k;
   __half* vt;
@@ -90,7 +94,8 @@ struct Params {
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
-att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_wq,
+                   const __grid_constant__ CUtensorMap tm_wk, const __grid_constant__ CUtensorMap tm_wv,
                    const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_vt,
                    const Params p) {
@@ -104,7 +109,9 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   }
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_x);
-    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_wq);
+    tma_prefetch_desc(&tm_wk);
+    tma_prefetch_desc(&tm_wv);
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < XSTAGES; ++s) {
       mbar_init(&sm.x_full[s], 1);
@@ -121,20 +128,32 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
+  if (!p.early_weights) pdl_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = p.gamma2[threadIdx.x - 64];
-    sm.beta2[threadIdx.x - 64] = p.beta2[threadIdx.x - 64];
+    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
+    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
+  }
+  for (int idx = threadIdx.x; idx < 2 * 16 * 64; idx += THREADS) {  // (slab, head, channel of the slab)
+    const int slab = idx >> 10, row = (idx >> 6) & 15, c = idx & 63;
+    const __nv_bfloat16 v = row < 4 ? p.w_bias[(slab * 64 + c) * 4 + row] : __float2bfloat16_rn(0.f);
+    *reinterpret_cast<__nv_bfloat16*>(sm.wb + slab * WB_SLAB + sw128_offset(row, c >> 3) + (c & 7) * 2) = v;
+  }
+  fence_proxy_async();
+  if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
+    mbar_expect_tx(&sm.w_full, W_BYTES);
+    for (int g = 0; g < 3; ++g)
+      for (int s = 0; s < 2; ++s)
+        tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, g == 0 ? &tm_wq : g == 1 ? &tm_wk : &tm_wv, &sm.w_full, s * 64, 0);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  if (p.early_weights) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&sm.w_full, W_BYTES);
-      for (int g = 0; g < 4; ++g)
-        for (int s = 0; s < 2; ++s) tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, &tm_w, &sm.w_full, s * 64, g * 128);
       int stage = 0;
       uint32_t phase = 0;
       for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
@@ -152,9 +171,9 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 256);
+      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128) | UMMA_B_MN;
       constexpr uint32_t idesc_b = umma_idesc_bf16(128, 16);
-      constexpr uint32_t idesc_v = umma_idesc_bf16(128, 128);
+      constexpr uint32_t idesc_v = umma_idesc_bf16(128, 128) | UMMA_A_MN;
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
@@ -163,46 +182,40 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         tc_fence_after();
         const uint32_t xs = smem_u32(sm.x[stage]);
         const uint32_t ws = smem_u32(sm.w);
-        // [q|k]: A = xn (rows = pairs), B = weight rows 0..255 (slabs 0..3: rows 0-127 s0,s1; rows 128-255 s0,s1)
+        // [q|k]: A = xn (rows = pairs), B = Wq, Wk
         if (!mbar_wait(&sm.acc_empty[G_QK], (it & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
 #pragma unroll
-        for (int half = 0; half < 2; ++half)  // N = 256 as two N = 128 halves (weight groups 0 and 1)
+        for (int half = 0; half < 2; ++half) {
+          const uint64_t bdesc = umma_desc_mnmajor(ws + half * 2 * SLAB_BYTES, SLAB_BYTES);
 #pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint64_t adesc = umma_desc_kmajor(xs + s * SLAB_BYTES, 128);
-            const uint64_t bdesc = umma_desc_kmajor(ws + (half * 2 + s) * SLAB_BYTES, 128);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_ss(tmem_base + TM_QK + half * 128, umma_desc_advance(adesc, k * 32),
-                           umma_desc_advance(bdesc, k * 32), idesc_v, (s | k) != 0);
-          }
+          for (int k = 0; k < 8; ++k)
+            umma_bf16_ss(tmem_base + TM_QK + half * 128,
+                         umma_desc_advance(umma_desc_kmajor(xs + (k >> 2) * SLAB_BYTES, 128), (k & 3) * 32),
+                         umma_desc_advance(bdesc, k * 2048), idesc_qk, k != 0);
+        }
         umma_commit(&sm.acc_full[G_QK]);
-        // bias: A = xn, B = weight rows 384..399 (group 3), N = 16
+        // bias: A = xn, B = Wb, N = 16
         if (!mbar_wait(&sm.acc_empty[G_B], (it & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
           const uint64_t adesc = umma_desc_kmajor(xs + s * SLAB_BYTES, 128);
-          const uint64_t bdesc = umma_desc_kmajor(ws + (3 * 2 + s) * SLAB_BYTES, 128);
+          const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.wb) + s * WB_SLAB, 128);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             umma_bf16_ss(tmem_base + TM_B, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32),
                          idesc_b, (s | k) != 0);
         }
         umma_commit(&sm.acc_full[G_B]);
-        // vT: A = Wv (rows = channels, group 2), B = xn (rows = pairs)
+        // vT: A = Wv (rows = channels), B = xn (rows = pairs)
         if (!mbar_wait(&sm.acc_empty[G_V], (it & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
+        const uint64_t vdesc = umma_desc_mnmajor(ws + 4 * SLAB_BYTES, SLAB_BYTES);
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const uint64_t adesc = umma_desc_kmajor(ws + (2 * 2 + s) * SLAB_BYTES, 128);
-          const uint64_t bdesc = umma_desc_kmajor(xs + s * SLAB_BYTES, 128);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16_ss(tmem_base + TM_V, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32),
-                         idesc_v, (s | k) != 0);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ss(tmem_base + TM_V, umma_desc_advance(vdesc, k * 2048),
+                       umma_desc_advance(umma_desc_kmajor(xs + (k >> 2) * SLAB_BYTES, 128), (k & 3) * 32), idesc_v, k != 0);
         umma_commit(&sm.acc_full[G_V]);
         umma_commit(&sm.x_empty[stage]);
         if (++stage == XSTAGES) {
@@ -210,13 +223,20 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
           phase ^= 1;
         }
       }
-      (void)idesc_qk;
     }
   } else if (warp < 2 + LN_WARPS) {
     const int r = (warp - 2) * 16 + (lane & 15);  // pair of the tile; lanes l and l ^ 16 share it
     int stage = 0;
     uint32_t phase = 0;
     for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+      if (p.mb.out && lane < 16) {  // the core's mask-bias row of these pairs, pitch padding included
+        const int o = static_cast<int>(tile / p.tiles_inner), t = static_cast<int>(tile % p.tiles_inner) * 128 + r;
+        if (t < p.mb.ld)
+          p.mb.out[static_cast<long long>(o) * p.mb.ld + t] =
+              t >= p.n_inner ? -INFINITY
+              : p.mb.mask    ? mask_bias(p.mb.mask[o * p.mb.ms_outer + t * p.mb.ms_inner], p.mb.inf, false)
+                             : 0.0f;
+      }
       if (!mbar_wait(&sm.x_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
       ln_row_two_threads(sm.x[stage], r, lane >> 4, sm.gamma2, sm.beta2, p.eps);
       fence_proxy_async();
@@ -425,9 +445,11 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 
 extern "C" size_t b200tri_triatt_project_workspace_bytes(void) { return 512 * 128 * 2 + 1024; }
 
-extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200tri_stream_t stream_) {
-  using namespace b200;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200tri_stream_t stream) {
+  return b200::att_project_launch(a, nullptr, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b200::att_project_launch(const b200tri_triatt_project_args* a, const MaskBiasOut* mb, cudaStream_t stream) {
   B200_REQUIRE(a != nullptr, B200TRI_ERR_INVALID, "att project: null args");
   B200_REQUIRE(a->x && a->q && a->k && a->vt && a->bias && a->norm_scale && a->norm_bias && a->w_q && a->w_k &&
                    a->w_v && a->w_bias,
@@ -445,19 +467,17 @@ extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200
   int* status = device_status_word();
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "att project: no current CUDA device");
 
+  // the weights are read in place; the workspace is only for one that is not 16-byte aligned
   Carver ws(a->workspace);
-  __nv_bfloat16* wpk = ws.take<__nv_bfloat16>(512 * 128);
-  uint32_t* gamma2 = ws.take<uint32_t>(64, 256);
-  uint32_t* beta2 = ws.take<uint32_t>(64, 256);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_q), 128, 0, 128, wpk, stream);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_k), 128, 0, 128, wpk + 128 * 128, stream);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_v), 128, 0, 128, wpk + 256 * 128, stream);
-  pack_zero(wpk + 384 * 128, 128 * 128, stream);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->w_bias), 4, 0, 4, wpk + 384 * 128, stream);
-  pack_copy_words(a->norm_scale, gamma2, 64, stream);
-  pack_copy_words(a->norm_bias, beta2, 64, stream);
-
-  CUtensorMap tm_x, tm_w, tm_q, tm_k, tm_vt;
+  const void* const w_in[3] = {a->w_q, a->w_k, a->w_v};
+  const void* w[3];
+  bool in_place = true;
+  for (int i = 0; i < 3; ++i) {
+    const int rc = aligned_weight(w_in[i], 128 * 128 * 2, ws.take<__nv_bfloat16>(128 * 128), stream, &w[i]);
+    if (rc) return rc;
+    in_place = in_place && w[i] == w_in[i];
+  }
+  CUtensorMap tm_x, tm_w[3], tm_q, tm_k, tm_vt;
   {  // q and k [n_outer][n_inner][128], written as tiles of [128 pairs][64 channels]
     const uint64_t dims[3] = {128, (uint64_t)a->n_inner, (uint64_t)a->n_outer};
     const uint64_t str[2] = {256, (uint64_t)a->n_inner * 256};
@@ -481,11 +501,8 @@ extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200
     int rc = make_tmap(&tm_x, a->x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
   }
-  {
-    const uint64_t dims[2] = {128, 512};
-    const uint64_t str[1] = {256};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w, wpk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
+  for (int i = 0; i < 3; ++i) {
+    const int rc = make_weight_map(&tm_w[i], w[i], 128, 128, 128);
     if (rc) return rc;
   }
   Params p;
@@ -493,8 +510,11 @@ extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
   p.total_tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
-  p.gamma2 = gamma2;
-  p.beta2 = beta2;
+  p.gamma = a->norm_scale;
+  p.beta = a->norm_bias;
+  p.w_bias = static_cast<const __nv_bfloat16*>(a->w_bias);
+  p.early_weights = pdl_chained() && in_place;
+  p.mb = mb ? *mb : MaskBiasOut{};
   p.q = static_cast<__nv_bfloat16*>(a->q);
   p.k = static_cast<__nv_bfloat16*>(a->k);
   p.vt = static_cast<__half*>(a->vt);
@@ -512,9 +532,7 @@ extern "C" int b200tri_triatt_project(const b200tri_triatt_project_args* a, b200
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_TRIATT_PROJECT, stream);
-    count_launch();
-    att_project_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_x, tm_w, tm_q, tm_k, tm_vt, p);
+    return launch(att_project_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x,
+                  tm_w[0], tm_w[1], tm_w[2], tm_q, tm_k, tm_vt, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }

@@ -127,6 +127,7 @@ extern "C" int b200tri_trimul_forward(const b200tri_trimul_args* a, b200tri_stre
   pa.workspace_bytes = b200tri_trimul_project_workspace_bytes();
   int rc = b200tri_trimul_project(&pa, stream);
   if (rc) return rc;
+  PdlChain chain;
 
   b200tri_trimul_contract_args ca = {};
   ca.n_i = ca.n_j = ca.n_k = a->n;

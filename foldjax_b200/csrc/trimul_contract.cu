@@ -73,6 +73,8 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
   const uint32_t tmem_base = tmem_base_s;
 
   const int k_iters = p.n_src * p.kb_per_src;
@@ -319,10 +321,7 @@ extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b2
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_CONTRACT, reinterpret_cast<cudaStream_t>(stream));
-    count_launch();
-    contract_kernel<<<static_cast<unsigned>(grid), THREADS, SMEM_BYTES, reinterpret_cast<cudaStream_t>(stream)>>>(
-      tm_a, tm_b, p);
+    return launch(contract_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES,
+                  reinterpret_cast<cudaStream_t>(stream), true, tm_a, tm_b, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }

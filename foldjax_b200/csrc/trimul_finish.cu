@@ -20,7 +20,6 @@
 // Bound: HBM (read t and x, write out: 3 * n_i*n_j*128*2 bytes; + residual).
 #include "host.cuh"
 #include "ln.cuh"
-#include "pack.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -39,7 +38,7 @@ constexpr int EPI_THREAD0 = 192;  // first thread of the epilogue warps
 #endif
 
 struct Smem {
-  uint8_t w[4 * SLAB_BYTES];  // g_out^T (2 slabs), p_out^T (2 slabs)
+  uint8_t w[4 * SLAB_BYTES];  // g_out, p_out: two boxes [128 in][64 out] each, MN-major
   uint8_t x[STAGES][TILE_BYTES];
   uint8_t t[STAGES][TILE_BYTES];
 #if B200_FIN_TMASTORE
@@ -54,7 +53,8 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 struct FinishParams {
   int n_i, n_j, tiles_j;
   long long total_tiles;
-  const uint32_t* ln;  // gamma_in, beta_in, gamma_out, beta_out: 4 x 64 words
+  const void* ln[4];    // gamma_in, beta_in, gamma_out, beta_out
+  bool early_weights;   // the weights may be read before pdl_wait()
   const __nv_bfloat16* residual;
   __nv_bfloat16* out;
   long long os_i, os_j;
@@ -65,8 +65,8 @@ struct FinishParams {
 
 __global__ void __launch_bounds__(THREADS, 1)
 finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_t,
-              const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_out,
-              const FinishParams p) {
+              const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_p,
+              const __grid_constant__ CUtensorMap tm_out, const FinishParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -79,7 +79,8 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_x);
     tma_prefetch_desc(&tm_t);
-    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_g);
+    tma_prefetch_desc(&tm_p);
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.in_full[s], 1);
@@ -97,23 +98,29 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
+  if (!p.early_weights) pdl_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
     const int q = threadIdx.x - 64;
-    sm.gamma_in[q] = p.ln[q];
-    sm.beta_in[q] = p.ln[64 + q];
-    sm.gamma_out[q] = p.ln[128 + q];
-    sm.beta_out[q] = p.ln[192 + q];
+    sm.gamma_in[q] = ln_param_pair(p.ln[0], q);
+    sm.beta_in[q] = ln_param_pair(p.ln[1], q);
+    sm.gamma_out[q] = ln_param_pair(p.ln[2], q);
+    sm.beta_out[q] = ln_param_pair(p.ln[3], q);
+  }
+  if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
+    mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
+    for (int g = 0; g < 2; ++g)
+      for (int s = 0; s < 2; ++s)
+        tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, g ? &tm_p : &tm_g, &sm.w_full, s * 64, 0);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  if (p.early_weights) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
-      for (int g = 0; g < 2; ++g)
-        for (int s = 0; s < 2; ++s) tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, &tm_w, &sm.w_full, s * 64, g * 128);
       int stage = 0;
       uint32_t phase = 0;
       for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
@@ -132,7 +139,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
@@ -145,14 +152,11 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         for (int g = 0; g < 2; ++g) {
           const uint32_t d_tmem = tmem_base + acc * 256 + g * 128;
           const uint32_t in = smem_u32(g == 0 ? sm.x[stage] : sm.t[stage]);
+          const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w + g * 2 * SLAB_BYTES), SLAB_BYTES);
 #pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint64_t adesc = umma_desc_kmajor(in + s * SLAB_BYTES, 128);
-            const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.w + (g * 2 + s) * SLAB_BYTES), 128);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_ss(d_tmem, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
-                           (s | k) != 0);
+          for (int k = 0; k < 8; ++k) {
+            const uint64_t adesc = umma_desc_kmajor(in + (k >> 2) * SLAB_BYTES, 128);
+            umma_bf16_ss(d_tmem, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc, k != 0);
           }
         }
         umma_commit(&sm.in_empty[stage]);
@@ -300,17 +304,16 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
   int* status = device_status_word();
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "finish: no current CUDA device");
 
+  // the weights are read in place; the workspace is only for one that is not 16-byte aligned
   Carver ws(a->workspace);
-  __nv_bfloat16* wpk = ws.take<__nv_bfloat16>(256 * 128);
-  uint32_t* ln = ws.take<uint32_t>(256, 256);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->g_out), 128, 0, 128, wpk, stream);
-  pack_transpose(static_cast<const __nv_bfloat16*>(a->p_out), 128, 0, 128, wpk + 128 * 128, stream);
-  pack_copy_words(a->norm_in_scale, ln, 64, stream);
-  pack_copy_words(a->norm_in_bias, ln + 64, 64, stream);
-  pack_copy_words(a->norm_out_scale, ln + 128, 64, stream);
-  pack_copy_words(a->norm_out_bias, ln + 192, 64, stream);
-
-  CUtensorMap tm_x, tm_t, tm_w, tm_out;
+  const void *w_g, *w_p;
+  {
+    void* s0 = ws.take<__nv_bfloat16>(128 * 128);
+    void* s1 = ws.take<__nv_bfloat16>(128 * 128);
+    int rc = aligned_weight(a->g_out, 128 * 128 * 2, s0, stream, &w_g);
+    if (rc || (rc = aligned_weight(a->p_out, 128 * 128 * 2, s1, stream, &w_p))) return rc;
+  }
+  CUtensorMap tm_x, tm_t, tm_g, tm_p, tm_out;
   {
     const uint64_t dims[3] = {128, (uint64_t)a->n_j, (uint64_t)a->n_i};
     const uint64_t str[2] = {(uint64_t)a->os_j * 2, (uint64_t)a->os_i * 2};
@@ -339,18 +342,19 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
     if (rc) return rc;
   }
   {
-    const uint64_t dims[2] = {128, 256};
-    const uint64_t str[1] = {256};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w, wpk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
-    if (rc) return rc;
+    int rc = make_weight_map(&tm_g, w_g, 128, 128, 128);
+    if (rc || (rc = make_weight_map(&tm_p, w_p, 128, 128, 128))) return rc;
   }
   FinishParams p;
   p.n_i = a->n_i;
   p.n_j = a->n_j;
   p.tiles_j = (a->n_j + 127) / 128;
   p.total_tiles = static_cast<long long>(p.tiles_j) * a->n_i;
-  p.ln = ln;
+  p.ln[0] = a->norm_in_scale;
+  p.ln[1] = a->norm_in_bias;
+  p.ln[2] = a->norm_out_scale;
+  p.ln[3] = a->norm_out_bias;
+  p.early_weights = pdl_chained() && w_g == a->g_out && w_p == a->p_out;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
   p.out = static_cast<__nv_bfloat16*>(a->out);
   p.os_i = a->os_i;
@@ -366,9 +370,7 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_FINISH, stream);
-    count_launch();
-    finish_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_x, tm_t, tm_w, tm_out, p);
+    return launch(finish_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_t,
+                  tm_g, tm_p, tm_out, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }

@@ -23,7 +23,6 @@
 // Bound: HBM (read x once, write a and b once: 3 * n*n*128*2 bytes).
 #include "host.cuh"
 #include "ln.cuh"
-#include "pack.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -38,7 +37,7 @@ constexpr int LN_WARPS = 8;  // two threads per pair
 constexpr int THREADS = 64 + LN_WARPS * 32 + 128;
 
 struct Smem {
-  uint8_t w[W_BYTES];
+  uint8_t w[W_BYTES];  // group g (p_a, g_a, p_b, g_b): two boxes [128 in][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
   __nv_bfloat16 mask[MASK_SLOTS][128];  // mask.astype(bf16), as the reference casts it
   uint32_t gamma2[64];
@@ -53,8 +52,9 @@ struct ProjParams {
   long long total_tiles;
   const float* mask;
   long long ms_outer, ms_inner;
-  const uint32_t* gamma2;
-  const uint32_t* beta2;
+  const void* gamma;
+  const void* beta;
+  bool early_weights;  // the weights may be read before pdl_wait()
   __nv_bfloat16* a;
   __nv_bfloat16* b;
   long long ld, chan_stride, block_stride;
@@ -64,8 +64,8 @@ struct ProjParams {
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
-project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
-               const ProjParams p) {
+project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_p,
+               const __grid_constant__ CUtensorMap tm_g, const ProjParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -77,7 +77,8 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_x);
-    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_p);
+    tma_prefetch_desc(&tm_g);
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < XSTAGES; ++s) {
       mbar_init(&sm.x_full[s], 1);
@@ -94,20 +95,26 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
+  if (!p.early_weights) pdl_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = p.gamma2[threadIdx.x - 64];
-    sm.beta2[threadIdx.x - 64] = p.beta2[threadIdx.x - 64];
+    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
+    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
+  }
+  if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
+    mbar_expect_tx(&sm.w_full, W_BYTES);
+    for (int g = 0; g < 4; ++g)
+      for (int s = 0; s < 2; ++s)
+        tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, (g & 1) ? &tm_g : &tm_p, &sm.w_full, (g >> 1) * 128 + s * 64, 0);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  if (p.early_weights) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     if (elect_one()) {
-      mbar_expect_tx(&sm.w_full, W_BYTES);
-      for (int g = 0; g < 4; ++g)
-        for (int s = 0; s < 2; ++s) tma_load_2d(sm.w + (g * 2 + s) * SLAB_BYTES, &tm_w, &sm.w_full, s * 64, g * 128);
       int stage = 0;
       uint32_t phase = 0;
       for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
@@ -125,7 +132,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
+      constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_A_MN;
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
@@ -142,14 +149,11 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           for (int g = 0; g < 2; ++g) {
             const int group = half * 2 + g;
             const uint32_t d_tmem = tmem_base + group * 128;
+            const uint64_t wdesc = umma_desc_mnmajor(smem_u32(sm.w + group * 2 * SLAB_BYTES), SLAB_BYTES);
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-              const uint64_t wdesc = umma_desc_kmajor(smem_u32(sm.w + (group * 2 + s) * SLAB_BYTES), 128);
-              const uint64_t xdesc = umma_desc_kmajor(xs + s * SLAB_BYTES, 128);
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                umma_bf16_ss(d_tmem, umma_desc_advance(wdesc, k * 32), umma_desc_advance(xdesc, k * 32), idesc,
-                             (s | k) != 0);
+            for (int k = 0; k < 8; ++k) {
+              const uint64_t xdesc = umma_desc_kmajor(xs + (k >> 2) * SLAB_BYTES, 128);
+              umma_bf16_ss(d_tmem, umma_desc_advance(wdesc, k * 2048), umma_desc_advance(xdesc, (k & 3) * 32), idesc, k != 0);
             }
           }
           umma_commit(&sm.acc_full[half]);
@@ -257,7 +261,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 }  // namespace b200
 
 extern "C" size_t b200tri_trimul_project_workspace_bytes(void) {
-  return 512 * 128 * 2 + 1024;  // packed weights + layer-norm parameters
+  return 512 * 128 * 2 + 1024;  // copies of weights that are not 16-byte aligned
 }
 
 extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200tri_stream_t stream_) {
@@ -278,21 +282,17 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
   int* status = device_status_word();
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "project: no current CUDA device");
 
+  // the weights are read in place; the workspace is only for one that is not 16-byte aligned
+  const bool chained = pdl_chained();
   Carver ws(a->workspace);
-  __nv_bfloat16* wpk = ws.take<__nv_bfloat16>(512 * 128);
-  uint32_t* gamma2 = ws.take<uint32_t>(64, 256);
-  uint32_t* beta2 = ws.take<uint32_t>(64, 256);
-  // Row groups of the packed weight: p_a, g_a, p_b, g_b (a = first 128 channels).
-  const __nv_bfloat16* p_in = static_cast<const __nv_bfloat16*>(a->p_in);
-  const __nv_bfloat16* g_in = static_cast<const __nv_bfloat16*>(a->g_in);
-  pack_transpose(p_in, 256, 0, 128, wpk + 0 * 128 * 128, stream);
-  pack_transpose(g_in, 256, 0, 128, wpk + 1 * 128 * 128, stream);
-  pack_transpose(p_in, 256, 128, 128, wpk + 2 * 128 * 128, stream);
-  pack_transpose(g_in, 256, 128, 128, wpk + 3 * 128 * 128, stream);
-  pack_copy_words(a->norm_in_scale, gamma2, 64, stream);
-  pack_copy_words(a->norm_in_bias, beta2, 64, stream);
-
-  CUtensorMap tm_x, tm_w;
+  const void *w_p, *w_g;
+  {
+    void* s0 = ws.take<__nv_bfloat16>(128 * 256);
+    void* s1 = ws.take<__nv_bfloat16>(128 * 256);
+    int rc = aligned_weight(a->p_in, 128 * 256 * 2, s0, stream, &w_p);
+    if (rc || (rc = aligned_weight(a->g_in, 128 * 256 * 2, s1, stream, &w_g))) return rc;
+  }
+  CUtensorMap tm_x, tm_p, tm_g;
   {
     const uint64_t dims[3] = {128, (uint64_t)a->n_inner, (uint64_t)a->n_outer};
     const uint64_t str[2] = {(uint64_t)a->xs_inner * 2, (uint64_t)a->xs_outer * 2};
@@ -301,11 +301,8 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
     if (rc) return rc;
   }
   {
-    const uint64_t dims[2] = {128, 512};
-    const uint64_t str[1] = {256};
-    const uint32_t box[2] = {64, 128};
-    int rc = make_tmap(&tm_w, wpk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
-    if (rc) return rc;
+    int rc = make_weight_map(&tm_p, w_p, 128, 256, 128);
+    if (rc || (rc = make_weight_map(&tm_g, w_g, 128, 256, 128))) return rc;
   }
   ProjParams p;
   p.n_outer = a->n_outer;
@@ -315,8 +312,9 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
   p.mask = a->mask;
   p.ms_outer = a->ms_outer;
   p.ms_inner = a->ms_inner;
-  p.gamma2 = gamma2;
-  p.beta2 = beta2;
+  p.gamma = a->norm_in_scale;
+  p.beta = a->norm_in_bias;
+  p.early_weights = chained && w_p == a->p_in && w_g == a->g_in;
   p.a = static_cast<__nv_bfloat16*>(a->a);
   p.b = static_cast<__nv_bfloat16*>(a->b);
   p.ld = a->ld;
@@ -333,9 +331,7 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_PROJECT, stream);
-    count_launch();
-    project_kernel<<<static_cast<unsigned>(grid), THREADS, sizeof(Smem), stream>>>(tm_x, tm_w, p);
+    return launch(project_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_p,
+                  tm_g, p);
   }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
 }
