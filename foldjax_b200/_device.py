@@ -36,6 +36,15 @@ def workspace(nbytes: int, tag: str = "default") -> torch.Tensor:
     return buf
 
 
+# Batch items share a launch as far as this much scratch memory carries them.
+BATCH_WORKSPACE = 2 << 30
+
+
+def batch_bytes(one: int, batch: int) -> int:
+    """Workspace of a batched call: ``one`` item's bytes times the items that run together."""
+    return one * max(1, min(batch, BATCH_WORKSPACE // max(one, 1)))
+
+
 def aligned_ptr(buf: torch.Tensor, align: int = 1024) -> int:
     p = buf.data_ptr()
     return (p + align - 1) // align * align

@@ -38,7 +38,7 @@ class TrimulArgs(C.Structure):
         ("p_out", C.c_void_p), ("g_out", C.c_void_p),
         ("residual", C.c_void_p), ("out", C.c_void_p),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("dtype", C.c_int32),
-        ("c_z", C.c_int32), ("c_hidden", C.c_int32),
+        ("c_z", C.c_int32), ("c_hidden", C.c_int32), ("batch", C.c_int32),
     ]
 
 
@@ -92,6 +92,7 @@ class TriattArgs(C.Structure):
         ("w_q", C.c_void_p), ("w_k", C.c_void_p), ("w_v", C.c_void_p), ("w_g", C.c_void_p), ("w_o", C.c_void_p),
         ("residual", C.c_void_p), ("out", C.c_void_p),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("dtype", C.c_int32), ("c_z", C.c_int32),
+        ("batch", C.c_int32),
     ]
 
 

@@ -1,0 +1,581 @@
+// Attention core in float32 arithmetic on the tensor cores: the triangle attention of a float32
+// trunk and of bf16 trunks of any head shape (rows i of the pair tensor share the bias), and
+// the single track's token attention (one row, 16 heads of width 24).
+//
+//   S = (q . k) * scale + mask_bias + bias        o = softmax(S) . v
+//
+// q, k, v arrive as IN bf16 pieces each (gemm.cuh): three when they are float32, one when the
+// trunk is bf16. The probabilities are split into three pieces by the thread that computes
+// them, so P.V is as exact as a float32 product. The piece products of one result are issued
+// smallest first into one float32 accumulator, so that only the leading one is summed at full
+// magnitude. Everything in between is float32 as in the reference (_attention_block,
+// src/foldjax/models/boltz2/models/triangle/triangle_attention.py:428-455;
+// _attention_qblock, primitives/attention.py:124-140): softmax in float32. With float32 operands
+// the running numerator stays in registers (P.V of a step starts from zero and is added by the
+// thread, which also makes the rescale a register fma). With bf16 operands it accumulates in TMEM
+// and is rescaled only when the maximum grew by more than RESCALE; the bias is bf16 too then and is
+// added by the tensor core, as in triatt_core.cu (S = bias . I + q . k).
+//
+// One CTA per SM, persistent; an item is (head, NWG rows, 128 queries), or with one row (head,
+// NWG tiles of 128 queries), walked in steps of 64 keys:
+//   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
+//   warpgroups  softmax, one thread per query
+// Bound: issue slots. A score costs about 2 instructions of exponential, 4.5 of split and 2-4
+// others, most of them packed two to an instruction; 52 % of the slots were busy with two softmax
+// warpgroups. With bf16 operands a third one fits, because there the probabilities overwrite
+// the scores in TMEM (OVERLAY): the scores of the next step then wait for this step's P.V, which
+// the other two warpgroups hide.
+#include "att_split.cuh"
+#include "gemm.cuh"
+#include "tc.cuh"
+
+namespace b200 {
+
+namespace {
+
+constexpr int KT = 64;
+constexpr float RESCALE = 5.5f;  // probabilities stay below e^5.5
+
+template <int HDP, int IN, bool TOKEN>
+struct Cfg {
+  static constexpr bool OVERLAY = IN == 1;
+  static constexpr int NWG = HDP == 32 ? (IN == 1 ? 3 : 2) : (IN == 1 ? 2 : 1);
+  static constexpr int KV = TOKEN ? 1 : NWG;  // rows whose keys a step loads
+  static constexpr int NB = TOKEN ? NWG : 1;  // bias tiles of a step
+  static constexpr int STAGES = IN == 1 ? 3 : 2;
+  static constexpr int THREADS = 128 + NWG * 128;
+  static constexpr int Q_BYTES = 128 * HDP * 2, K_BYTES = KT * HDP * 2, V_BYTES = HDP * 128;
+  static constexpr int BIAS_BYTES = 128 * KT * (IN == 1 ? 2 : 4);
+  static constexpr uint32_t TM_S = 0, TM_P = OVERLAY ? 0 : 64, TM_O = TM_P + 96, TM_WG = TM_O + HDP;
+  static_assert(NWG * TM_WG <= 512, "tensor memory budget");
+  // three warpgroups: registers move from the control warpgroup (512 x 128 = 128 x 80 + 384 x 144)
+  static constexpr bool SHIFT_REGS = NWG == 3;
+  static constexpr uint32_t STAGE_TX = KV * IN * (K_BYTES + V_BYTES) + NB * BIAS_BYTES + KV * KT * 4;
+};
+
+template <int HDP, int IN, bool TOKEN>
+struct Smem {
+  using C = Cfg<HDP, IN, TOKEN>;
+  uint8_t q[C::NWG][IN][C::Q_BYTES];
+  uint8_t k[C::STAGES][C::KV][IN][C::K_BYTES];
+  uint8_t v[C::STAGES][C::KV][IN][C::V_BYTES];
+  // float32: two boxes of 32 keys, [128 queries][32 floats]; bf16: [128 queries][64]
+  uint8_t bias[C::STAGES][C::NB][C::BIAS_BYTES];
+  uint8_t ident[IN == 1 ? KT * 128 : 128];  // 64 x 64 bf16 identity
+  alignas(128) float mb[C::STAGES][C::KV][KT];
+  uint64_t q_full, q_empty, st_full[C::STAGES], st_empty[C::STAGES], s_full[C::NWG], s_free[C::NWG], p_full[C::NWG],
+      pv_done[C::NWG];
+  uint32_t tmem_base;
+};
+
+struct Maps {
+  CUtensorMap q, k, v, b, m;
+};
+
+struct Params {
+  int n_i, n, heads, head_dim;
+  int groups, tiles_j, steps;
+  uint32_t total_items;
+  float scale;
+  void* o;                   // [rows][n][heads * head_dim], float32, or bf16 with bf16 operands
+  const float* gate;         // one row: the output is o * gate as pieces
+  __nv_bfloat16* pieces;     // [3][n][heads * head_dim]
+  int* status;
+};
+
+// e^(s - m) for two scores, m at least their maximum so far. The difference comes first, so the
+// error of 2^t is about 2^-23 |t| of a weight 2^-|t|: never above 2^-24 of the largest weight.
+__device__ __forceinline__ float2 exp_below(float2 s, float2 minus_m) {
+  const float2 t = __fmul2_rn(__fadd2_rn(s, minus_m), make_float2(1.44269504f, 1.44269504f));
+  return make_float2(fast_exp2(t.x), fast_exp2(t.y));
+}
+// split3x2 with packed subtractions
+__device__ __forceinline__ void split3f2(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const float2 minus = make_float2(-1.0f, -1.0f);
+  hi = pack_bf16x2(v.x, v.y);
+  const float2 r = __ffma2_rn(make_float2(bf16_lo(hi), bf16_hi(hi)), minus, v);
+  mid = pack_bf16x2(r.x, r.y);
+  const float2 q = __ffma2_rn(make_float2(bf16_lo(mid), bf16_hi(mid)), minus, r);
+  lo = pack_bf16x2(q.x, q.y);
+}
+
+template <int HDP, int IN, bool TOKEN>
+__global__ void __launch_bounds__(Cfg<HDP, IN, TOKEN>::THREADS, 1)
+att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
+  using C = Cfg<HDP, IN, TOKEN>;
+  using TQ = Terms<IN, IN>;  // q . k
+  using TP = Terms<3, IN>;   // P . v
+  constexpr int NWG = C::NWG, STAGES = C::STAGES;
+  static_assert(sizeof(Smem<HDP, IN, TOKEN>) <= 232448, "shared memory budget");
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  Smem<HDP, IN, TOKEN>& sm = *reinterpret_cast<Smem<HDP, IN, TOKEN>*>(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((smem_u32(smem_raw) & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
+    return;
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm.q);
+    tma_prefetch_desc(&tm.k);
+    tma_prefetch_desc(&tm.v);
+    tma_prefetch_desc(&tm.b);
+    mbar_init(&sm.q_full, 1);
+    mbar_init(&sm.q_empty, 1);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&sm.st_full[s], 1);
+      mbar_init(&sm.st_empty[s], 1 + NWG * 4);
+    }
+    for (int g = 0; g < NWG; ++g) {
+      mbar_init(&sm.s_full[g], 1);
+      mbar_init(&sm.s_free[g], 128);
+      mbar_init(&sm.p_full[g], 128);
+      mbar_init(&sm.pv_done[g], 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&sm.tmem_base, 512);
+    tmem_relinquish();
+  }
+  if (IN == 1) {  // the identity, K-major under the 128-byte swizzle
+    for (int idx = threadIdx.x; idx < KT * 32; idx += C::THREADS) {
+      const int r = idx / 32, w = idx % 32;
+      const int e0 = ((w >> 2) ^ (r & 7)) * 8 + (w & 3) * 2;  // logical element of the word's low half
+      reinterpret_cast<uint32_t*>(sm.ident)[idx] = e0 == r ? 0x00003F80u : e0 + 1 == r ? 0x3F800000u : 0u;
+    }
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t tmem_base = sm.tmem_base;
+  const uint32_t items_per_head = p.groups * p.tiles_j;
+  // item -> head, batch item, row inside it and first query of warpgroup 0; the others follow at
+  // successive rows, or (one row) at successive tiles of 128 queries
+  auto locate = [&](uint32_t item, int& b, int& h, int& i, int& j0) {
+    const uint32_t bh = item / items_per_head, rem = item - bh * items_per_head;
+    b = bh / p.heads;
+    h = bh - b * p.heads;
+    const uint32_t grp = rem / p.tiles_j, tile = rem - grp * p.tiles_j;
+    i = grp * NWG;  // (one group of rows in the one-row form)
+    j0 = tile * (TOKEN ? NWG * 128 : 128);
+  };
+
+  if (C::SHIFT_REGS && warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0, item_it = 0;
+      bool alive = true;
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+        if (!mbar_wait(&sm.q_empty, (item_it & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        mbar_expect_tx(&sm.q_full, NWG * IN * C::Q_BYTES);
+        int b, h, i, j0;
+        locate(item, b, h, i, j0);
+        const int row = b * p.n_i + i;
+        for (int g = 0; g < NWG; ++g)
+          for (int pc = 0; pc < IN; ++pc)
+            tma_load_5d(sm.q[g][pc], &tm.q, &sm.q_full, 0, h, TOKEN ? j0 + g * 128 : j0, TOKEN ? row : row + g, pc);
+        for (int t = 0; t < p.steps; ++t) {
+          if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
+            alive = false;
+            break;
+          }
+          const int k0 = t * KT;
+          mbar_expect_tx(&sm.st_full[stage], C::STAGE_TX);
+#pragma unroll 1
+          for (int g = 0; g < C::KV; ++g) {
+#pragma unroll 1
+            for (int pc = 0; pc < IN; ++pc) {
+              tma_load_5d(sm.k[stage][g][pc], &tm.k, &sm.st_full[stage], 0, h, k0, row + g, pc);
+              tma_load_5d(sm.v[stage][g][pc], &tm.v, &sm.st_full[stage], k0, 0, h, row + g, pc);
+            }
+            tma_load_2d(sm.mb[stage][g], &tm.m, &sm.st_full[stage], k0, row + g);
+          }
+          for (int g = 0; g < C::NB; ++g) {
+            for (int half = 0; half < (IN == 1 ? 1 : 2); ++half)
+              tma_load_4d(sm.bias[stage][g] + half * 16384, &tm.b, &sm.st_full[stage], k0 + half * 32, j0 + g * 128, h, b);
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, KT);
+      int stage = 0;
+      uint32_t phase = 0, item_it = 0, g = 0;
+      bool alive = true;
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+        if (!mbar_wait(&sm.q_full, item_it & 1, p.status, ST_TIMEOUT_MMA)) break;
+        for (int t = 0; t < p.steps && alive; ++t, ++g) {
+          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
+            alive = false;
+            break;
+          }
+          for (int wg = 0; wg < NWG; ++wg) {
+            // the scores' columns are free once they have been read, or (overlaid) once P.V is through
+            if (!mbar_wait(C::OVERLAY ? &sm.pv_done[wg] : &sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
+              alive = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem_base + wg * C::TM_WG + C::TM_S;
+            if (IN == 1) {
+              const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[stage][0]), 128);
+              const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
+#pragma unroll
+              for (int kk = 0; kk < KT / 16; ++kk)
+                umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
+            }
+#pragma unroll
+            for (int term = 0; term < TQ::N; ++term) {
+              const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[wg][TQ::a(term)]), HDP * 2);
+              const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.k[stage][TOKEN ? 0 : wg][TQ::b(term)]), HDP * 2);
+#pragma unroll
+              for (int kk = 0; kk < HDP / 16; ++kk)
+                umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc,
+                             IN == 1 || (term | kk) != 0);
+            }
+            umma_commit(&sm.s_full[wg]);
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (alive) umma_commit(&sm.q_empty);
+      }
+    }
+  } else if (warp == 2) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, HDP);
+      int stage = 0;
+      uint32_t phase = 0, g = 0;
+      bool alive = true;
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
+        for (int t = 0; t < p.steps && alive; ++t, ++g) {
+          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
+            alive = false;
+            break;
+          }
+          for (int wg = 0; wg < NWG; ++wg) {
+            if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
+              alive = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t base = tmem_base + wg * C::TM_WG;
+#pragma unroll
+            for (int term = 0; term < TP::N; ++term) {
+              const uint64_t vdesc = umma_desc_kmajor(smem_u32(sm.v[stage][TOKEN ? 0 : wg][TP::b(term)]), 128);
+#pragma unroll
+              for (int kk = 0; kk < KT / 16; ++kk)
+                umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
+                             idesc, (C::OVERLAY && t > 0) || (term | kk) != 0);
+            }
+            umma_commit(&sm.pv_done[wg]);
+          }
+          if (!alive) break;
+          umma_commit(&sm.st_empty[stage]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    if (C::SHIFT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    const int wg = (warp - 4) >> 2, quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    const uint32_t t_wg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + wg * C::TM_WG;
+    int stage = 0;
+    uint32_t phase = 0, g = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
+      float m_run = -INFINITY, l_run = 0.f, alpha = 0.f;
+      float o[C::OVERLAY ? 1 : HDP];
+#pragma unroll
+      for (int d = 0; d < (C::OVERLAY ? 1 : HDP); ++d) o[d] = 0.f;
+      auto take_pv = [&] {  // o = o * (rescale of the step P.V belongs to) + P.V
+#pragma unroll
+        for (int part = 0; part < HDP / 16; ++part) {
+          uint32_t r[16];
+          tmem_ld16(t_wg + C::TM_O + part * 16, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            float& acc = o[C::OVERLAY ? 0 : part * 16 + e];
+            acc = fmaf(acc, alpha, __uint_as_float(r[e]));
+          }
+        }
+      };
+      for (int t = 0; t < p.steps; ++t, ++g) {
+        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) ||
+            !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+          alive = false;
+          break;
+        }
+        // (overlaid scores can only have been formed after the previous P.V: no wait, but its order)
+        if (C::OVERLAY && !mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+          alive = false;
+          break;
+        }
+        tc_fence_after();
+        __syncwarp();
+        float2 s[KT / 2];
+        {
+          uint32_t r0[32], r1[32];
+          tmem_ld32(t_wg + C::TM_S, r0);
+          tmem_ld32(t_wg + C::TM_S + 32, r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            s[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
+            s[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+          }
+        }
+        tc_fence_before();
+        if (!C::OVERLAY) mbar_arrive(&sm.s_free[wg]);
+        const float* mrow = sm.mb[stage][TOKEN ? 0 : wg];
+        const bool masked = __any_sync(0xffffffffu, mrow[lane] != 0.f || mrow[lane + 32] != 0.f);
+        if (IN == 1) {  // the bias is in already
+          if (masked)
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
+              s[2 * c] = __fadd2_rn(s[2 * c], make_float2(m4.x, m4.y));
+              s[2 * c + 1] = __fadd2_rn(s[2 * c + 1], make_float2(m4.z, m4.w));
+              if ((c & 1) == 1) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
+            }
+        } else {  // the reference's order of the two sums
+          const uint8_t* brow = sm.bias[stage][TOKEN ? wg : 0];
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * 16384 + sw128_offset(row, c & 7));
+            const float2 b2[2] = {make_float2(b4.x, b4.y), make_float2(b4.z, b4.w)};
+            float2 m2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            if ((c & 1) == 1) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
+            if (masked) {
+              const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
+              m2[0] = make_float2(m4.x, m4.y);
+              m2[1] = make_float2(m4.z, m4.w);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              float2& x = s[2 * c + u];
+              x = TOKEN ? __fadd2_rn(__ffma2_rn(x, make_float2(p.scale, p.scale), b2[u]), m2[u])
+                        : __fadd2_rn(__fadd2_rn(x, m2[u]), b2[u]);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
+        float mxa = m_run, mxb = s[0].x;
+#pragma unroll
+        for (int e = 0; e < KT / 2; e += 2) {
+          mxa = fmax3(mxa, s[e].x, s[e].y);
+          mxb = fmax3(mxb, s[e + 1].x, s[e + 1].y);
+        }
+        float mx = fmaxf(mxa, mxb);  // (with the running maximum in it)
+        if (C::OVERLAY) {  // keep the offset unless the maximum grew a lot
+          const bool need = mx - m_run > RESCALE;  // true on the first step
+          if (!need) mx = m_run;
+          if (__any_sync(0xffffffffu, need) && t > 0) {
+            const float scale = fast_exp2((m_run - mx) * 1.44269504f);
+#pragma unroll
+            for (int part = 0; part < HDP / 16; ++part) {
+              uint32_t r[16];
+              tmem_ld16(t_wg + C::TM_O + part * 16, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * scale);
+              tmem_st16(t_wg + C::TM_O + part * 16, r);
+            }
+          }
+        }
+        const float alpha_new = fast_exp2((m_run - mx) * 1.44269504f);  // 0 on the first step
+        m_run = mx;
+        float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int e = 0; e < KT / 2; ++e) {
+          s[e] = exp_below(s[e], make_float2(-mx, -mx));
+          l2[e & 1] = __fadd2_rn(l2[e & 1], s[e]);
+        }
+        l_run = fmaf(l_run, alpha_new, (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));
+        if (!C::OVERLAY) {  // the previous step's P.V: its result is taken, then P may be overwritten
+          if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+            alive = false;
+            break;
+          }
+          tc_fence_after();
+          if (t > 0) take_pv();
+        }
+        alpha = alpha_new;
+#pragma unroll
+        for (int oct = 0; oct < 4; ++oct) {  // 16 keys at a time: few live registers
+          uint32_t pc[3][8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) split3f2(s[oct * 8 + e], pc[0][e], pc[1][e], pc[2][e]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) tmem_st8(t_wg + C::TM_P + q * 32 + oct * 8, pc[q]);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&sm.p_full[wg]);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      if (!alive) break;
+      if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) break;
+      tc_fence_after();
+      __syncwarp();
+      if (!C::OVERLAY) take_pv();
+      int b, h, i, j0;
+      locate(item, b, h, i, j0);
+      if (TOKEN)
+        j0 += wg * 128;
+      else
+        i += wg;
+      const int j = j0 + row;
+      const bool live = i < p.n_i && j < p.n;
+      const long long off = ((static_cast<long long>(b * p.n_i + i) * p.n + j) * p.heads + h) * p.head_dim;
+      const float inv = 1.0f / l_run;
+      if (C::OVERLAY) {
+#pragma unroll
+        for (int part = 0; part < HDP / 16; ++part) {
+          uint32_t r[16];
+          tmem_ld16(t_wg + C::TM_O + part * 16, r);
+          tmem_ld_wait();
+          if (!live) continue;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack_bf16x2(__uint_as_float(r[8 * q + 2 * e]) * inv, __uint_as_float(r[8 * q + 2 * e + 1]) * inv);
+            if (part * 16 + q * 8 < p.head_dim)
+              *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.o) + off + part * 16 + q * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+      tc_fence_before();
+      if constexpr (!C::OVERLAY && TOKEN) {
+        const long long plane = static_cast<long long>(p.n) * p.heads * p.head_dim;
+#pragma unroll
+        for (int d = 0; d < HDP; d += 8) {
+          if (!live || d >= p.head_dim) break;
+          uint32_t w[3][4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            split3x2(o[d + 2 * e] * inv * p.gate[off + d + 2 * e], o[d + 2 * e + 1] * inv * p.gate[off + d + 2 * e + 1], w[0][e],
+                     w[1][e], w[2][e]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            *reinterpret_cast<uint4*>(p.pieces + q * plane + off + d) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+        }
+      } else if constexpr (!C::OVERLAY) {
+#pragma unroll
+        for (int d = 0; d < HDP; d += 4)
+          if (live && d < p.head_dim)
+            *reinterpret_cast<float4*>(static_cast<float*>(p.o) + off + d) =
+                make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
+      }
+    }
+  }
+
+  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
+template <int HDP, int IN, bool TOKEN>
+int launch_cfg(const Maps& tm, Params p, cudaStream_t stream) {
+  using C = Cfg<HDP, IN, TOKEN>;
+  const int tiles = (p.n + 127) / 128;
+  p.groups = TOKEN ? 1 : (p.n_i + C::NWG - 1) / C::NWG;
+  p.tiles_j = TOKEN ? (tiles + C::NWG - 1) / C::NWG : tiles;
+  const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
+  B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "float32 attention: too many tiles");
+  p.total_items = static_cast<uint32_t>(items);
+  const int rc =
+      ensure_smem_limit(reinterpret_cast<const void*>(att_split_kernel<HDP, IN, TOKEN>), (int)sizeof(Smem<HDP, IN, TOKEN>));
+  if (rc) return rc;
+  const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
+  return launch(att_split_kernel<HDP, IN, TOKEN>, dim3(grid), dim3(C::THREADS),
+                sizeof(Smem<HDP, IN, TOKEN>), stream, true, tm, p);
+}
+
+}  // namespace
+
+int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
+  B200_REQUIRE(a.head_dim % 8 == 0 && a.head_dim >= 8 && a.head_dim <= 64, B200TRI_ERR_UNSUPPORTED,
+               "float32 attention: head widths are multiples of 8 up to 64 (got %d)", a.head_dim);
+  const bool token = a.pieces != nullptr;
+  B200_REQUIRE(!token || (!a.bf16 && a.batch == 1 && a.n_i == 1 && a.head_dim <= 32), B200TRI_ERR_INVALID,
+               "float32 attention: the gated form takes one row of heads up to 32 wide");
+  const uint32_t hdp = a.head_dim <= 32 ? 32 : 64;
+  const Swz qk_swz = hdp == 32 ? Swz::B64 : Swz::B128;
+  const uint64_t hd = a.head_dim, heads = a.heads, width = hd * heads, n = a.n;
+  const uint64_t rows = static_cast<uint64_t>(a.n_i) * a.batch, in = a.bf16 ? 1 : 3;
+  Maps tm;
+  int rc;
+  {
+    const uint64_t dims[5] = {hd, heads, n, rows, in};
+    const uint64_t str[4] = {hd * 2, width * 2, n * width * 2, rows * n * width * 2};
+    const uint32_t box_q[5] = {hdp, 1, 128, 1, 1}, box_k[5] = {hdp, 1, KT, 1, 1};
+    if ((rc = make_tmap(&tm.q, a.q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box_q, qk_swz))) return rc;
+    if ((rc = make_tmap(&tm.k, a.k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box_k, qk_swz))) return rc;
+  }
+  {
+    const uint64_t ld = a.v_ld;
+    const uint64_t dims[5] = {n, hd, heads, rows, in};
+    const uint64_t str[4] = {ld * 2, hd * ld * 2, width * ld * 2, rows * width * ld * 2};
+    const uint32_t box[5] = {KT, hdp, 1, 1, 1};
+    if ((rc = make_tmap(&tm.v, a.vt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box, Swz::B128))) return rc;
+  }
+  {
+    const uint64_t ld = a.bias_ld, size = a.bf16 ? 2 : 4;
+    const uint64_t dims[4] = {n, n, heads, static_cast<uint64_t>(a.batch)};
+    const uint64_t str[3] = {ld * size, n * ld * size, heads * n * ld * size};
+    const uint32_t box[4] = {a.bf16 ? 64u : 32u, 128, 1, 1};
+    if ((rc = make_tmap(&tm.b, a.bias, a.bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dims, str,
+                        box, Swz::B128)))
+      return rc;
+  }
+  {
+    const uint64_t ld = a.mask_ld;
+    const uint64_t dims[2] = {ld, rows};
+    const uint64_t str[1] = {ld * 4};
+    const uint32_t box[2] = {KT, 1};
+    if ((rc = make_tmap(&tm.m, a.mask_bias, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, dims, str, box, Swz::None))) return rc;
+  }
+  Params p = {};
+  p.n_i = a.n_i;
+  p.n = a.n;
+  p.heads = a.heads;
+  p.head_dim = a.head_dim;
+  p.steps = (a.n + KT - 1) / KT;
+  p.total_items = static_cast<uint32_t>(a.batch) * a.heads;
+  p.scale = a.scale;
+  p.o = a.o;
+  p.gate = a.gate;
+  p.pieces = a.pieces;
+  p.status = device_status_word();
+  B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "float32 attention: no current CUDA device");
+  if (token) return launch_cfg<32, 3, true>(tm, p, stream);
+  if (a.bf16) return hdp == 32 ? launch_cfg<32, 1, false>(tm, p, stream) : launch_cfg<64, 1, false>(tm, p, stream);
+  return hdp == 32 ? launch_cfg<32, 3, false>(tm, p, stream) : launch_cfg<64, 3, false>(tm, p, stream);
+}
+
+}  // namespace b200

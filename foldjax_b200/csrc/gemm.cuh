@@ -12,11 +12,14 @@
 // have an accumulator of their own, where that half ulp is 2^-8 smaller, and the leading term
 // alternates between NMAIN accumulators; the epilogue adds them in float32.
 //
-// piece_gemm_kernel: persistent, one CTA per SM, tiles of 128 x BN.
-//   warp 0       TMA producer: per k step of 64 every piece of A [128][64] (K-major) and of B,
-//                either K-major [BN][64] or MN-major [64][BN] (weights as stored, [in][out])
+// piece_gemm_kernel: persistent, tiles of 128 x BN.
+//   warp 0       TMA producer: per k step of 64 every piece of A [128][64] and of B [BN][64],
+//                each K-major (activations) or MN-major (weights as stored, [in][out])
 //   warp 1       MMA issuer
-//   warps 4-11   epilogue (policy code), two warps per TMEM lane quarter
+//   warps 4-     epilogue (policy code): EPI warps, EPI / 4 per TMEM lane quarter, each with its
+//                share of the columns, 16 at a time
+// The epilogues (conversions, gates, scattered stores) are latency-bound: a policy asks for two
+// CTAs per SM where its tile fits twice, or for more epilogue warps where it does not.
 // A tile has one or two segments (two products with operands of their own, in neighbouring
 // TMEM columns), and its accumulators are double-buffered where they fit, so that the epilogue
 // of one tile overlaps the products of the next. With few tiles K is split: each split writes its own partial.
@@ -28,8 +31,6 @@ namespace b200 {
 
 constexpr int GEMM_BM = 128, GEMM_BK = 64;
 constexpr int GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;  // one piece of one k step
-constexpr int GEMM_EPI_WARPS = 8;
-constexpr int GEMM_THREADS = 128 + GEMM_EPI_WARPS * 32;
 
 // v = hi + mid + lo
 __device__ __forceinline__ void split3(float v, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_bfloat16& lo) {
@@ -77,11 +78,11 @@ struct GemmShape {
 };
 
 // What a policy P provides:
-//   BN, PA, PB, NSEG, NMAIN, B_MN              shape constants
-//   struct Params                              epilogue arguments
-//   b_map(seg, n_tile, g, params), b_col(...)  which B map and column group g (64 wide, MN-major)
-//                                              or row block (K-major, g = 0) of a tile reads
-//   epilogue(params, m_tile, n_tile, split, accumulators, quarter, half, lane)
+//   BN, PA, PB, NSEG, NMAIN, A_MN, B_MN, M_FAST   shape constants (M_FAST: successive tiles walk m)
+//   EPI, CTAS                                     epilogue warps, CTAs per SM
+//   struct Params                                 arguments
+//   load_a / load_b(maps, params, seg, k, tile, piece, dst, bar)  one piece of one k step
+//   epilogue(params, m_tile, n_tile, split, accumulators, quarter, col0, col1, lane)   columns [col0, col1)
 template <class P>
 constexpr int gemm_acc_count() {  // accumulators of one segment
   return P::NMAIN + (P::PA * P::PB > 1 ? 1 : 0);
@@ -91,26 +92,32 @@ constexpr int gemm_acc_count() {  // accumulators of one segment
 template <class P>
 struct Accum {
   uint32_t base;  // TMEM address of the warp's lanes, first column of the tile
-  int used;       // leading-term accumulators that were written
-  // 32 columns starting at `col` of segment `seg`, one TMEM lane per thread
-  __device__ __forceinline__ void load(int seg, int col, float (&v)[32]) const {
+  int used[P::NSEG];  // k steps of each segment: only so many leading-term accumulators were written
+  // 16 columns starting at `col` of segment `seg`, one TMEM lane per thread
+  __device__ __forceinline__ void load(int seg, int col, float (&v)[16]) const {
     constexpr int NACC = gemm_acc_count<P>();
-    uint32_t r[32];
+    __syncwarp();  // (the callers' guards may have split the warp; TMEM loads are warp-wide)
+    uint32_t r[NACC][16];
     const uint32_t t = base + seg * (NACC * P::BN) + col;
-    tmem_ld32(t, r);
+#pragma unroll
+    for (int m = 0; m < NACC; ++m) tmem_ld16(t + m * P::BN, r[m]);
     tmem_ld_wait();
 #pragma unroll
-    for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+    for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[0][e]);
 #pragma unroll
     for (int m = 1; m < NACC; ++m) {
-      if (m < P::NMAIN && m >= used) continue;
-      tmem_ld32(t + m * P::BN, r);
-      tmem_ld_wait();
+      if (m < P::NMAIN && m >= used[seg]) continue;
 #pragma unroll
-      for (int e = 0; e < 32; ++e) v[e] += __uint_as_float(r[e]);
+      for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(r[m][e]);
     }
   }
 };
+
+// MN-major operand piece: `groups` boxes of 64 columns from `col` on, 64 rows of k.
+__device__ __forceinline__ void gemm_load_mn(const CUtensorMap* m, uint8_t* dst, uint64_t* bar, int groups, int col, int k,
+                                             int piece) {
+  for (int g = 0; g < groups; ++g) tma_load_3d(dst + g * 8192, m, bar, col + g * 64, k, piece);
+}
 
 template <class P>
 constexpr int gemm_stage_bytes() {
@@ -118,7 +125,12 @@ constexpr int gemm_stage_bytes() {
 }
 template <class P>
 constexpr int gemm_stages() {
-  return (220 * 1024) / gemm_stage_bytes<P>() > 6 ? 6 : (220 * 1024) / gemm_stage_bytes<P>();
+  constexpr int fit = (P::CTAS == 1 ? 220 : 110) * 1024 / gemm_stage_bytes<P>();
+  return fit > 6 ? 6 : fit;
+}
+template <class P>
+constexpr int gemm_threads() {
+  return 128 + P::EPI * 32;
 }
 template <class P>
 constexpr int gemm_smem_bytes() {
@@ -126,14 +138,14 @@ constexpr int gemm_smem_bytes() {
 }
 
 template <class P>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(gemm_threads<P>(), P::CTAS)
 piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, const typename P::Params ep) {
   constexpr int STAGES = gemm_stages<P>(), STAGE_BYTES = gemm_stage_bytes<P>();
   constexpr int SEG = gemm_acc_count<P>() * P::BN;  // accumulator columns of one segment
   constexpr int ACC = P::NSEG * SEG;                // and of one tile
-  constexpr uint32_t NBUF = 2 * ACC <= 512 ? 2 : 1;
+  constexpr uint32_t NBUF = 2 * ACC <= 512 / P::CTAS ? 2 : 1;
   constexpr int USED = NBUF * ACC, TMEM_COLS = USED <= 64 ? 64 : USED <= 128 ? 128 : USED <= 256 ? 256 : 512;
-  static_assert(ACC <= 512 && STAGES >= 2, "tile does not fit");
+  static_assert(NBUF * ACC <= 512 / P::CTAS && STAGES >= 2, "tile does not fit");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -149,7 +161,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
     }
     for (int b = 0; b < 2; ++b) {  // (one is spare without double buffering)
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], GEMM_EPI_WARPS);
+      mbar_init(&acc_empty[b], P::EPI);
     }
     fence_barrier_init();
   }
@@ -163,17 +175,28 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
   pdl_wait();
   pdl_trigger();
   const uint32_t tmem_base = tmem_base_s;
-  const long long total = static_cast<long long>(g.m_tiles) * g.n_tiles * g.splits;
+  // (32-bit tile arithmetic: a 64-bit division costs a role several hundred cycles per tile)
+  const uint32_t total = static_cast<uint32_t>(g.m_tiles) * g.n_tiles * g.splits;
+  auto locate = [&](uint32_t tile, int& split, int& m_tile, int& n_tile) {
+    split = 0;
+    if (g.splits > 1) {
+      split = static_cast<int>(tile % g.splits);
+      tile /= g.splits;
+    }
+    const uint32_t fast = P::M_FAST ? g.m_tiles : g.n_tiles;
+    const int hi = static_cast<int>(tile / fast), lo = static_cast<int>(tile - hi * fast);
+    m_tile = P::M_FAST ? lo : hi;
+    n_tile = P::M_FAST ? hi : lo;
+  };
 
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
-      for (long long tile = blockIdx.x; tile < total && alive; tile += gridDim.x) {
-        const int split = static_cast<int>(tile % g.splits);
-        const int n_tile = static_cast<int>((tile / g.splits) % g.n_tiles);
-        const int m_tile = static_cast<int>(tile / g.splits / g.n_tiles);
+      for (uint32_t tile = blockIdx.x; tile < total && alive; tile += gridDim.x) {
+        int split, m_tile, n_tile;
+        locate(tile, split, m_tile, n_tile);
         for (int seg = 0; seg < P::NSEG && alive; ++seg) {
           const int per = (g.kb[seg] + g.splits - 1) / g.splits;
           const int k1 = min(g.kb[seg], (split + 1) * per);
@@ -186,17 +209,9 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
             uint8_t* sb = sa + P::PA * GEMM_A_BYTES;
             mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
             for (int pc = 0; pc < P::PA; ++pc)
-              tma_load_3d(sa + pc * GEMM_A_BYTES, &maps.a[seg], &full_bar[stage], kb * GEMM_BK, m_tile * GEMM_BM, pc);
-            for (int pc = 0; pc < P::PB; ++pc) {
-              if (P::B_MN) {
-                for (int grp = 0; grp < P::BN / 64; ++grp)
-                  tma_load_3d(sb + pc * P::BN * 128 + grp * 8192, &maps.b[P::b_map(seg, n_tile, grp, ep)], &full_bar[stage],
-                              P::b_col(seg, n_tile, grp, ep), kb * GEMM_BK, pc);
-              } else {
-                tma_load_3d(sb + pc * P::BN * 128, &maps.b[P::b_map(seg, n_tile, 0, ep)], &full_bar[stage], kb * GEMM_BK,
-                            P::b_col(seg, n_tile, 0, ep), pc);
-              }
-            }
+              P::load_a(maps, ep, seg, kb * GEMM_BK, m_tile, pc, sa + pc * GEMM_A_BYTES, &full_bar[stage]);
+            for (int pc = 0; pc < P::PB; ++pc)
+              P::load_b(maps, ep, seg, kb * GEMM_BK, n_tile, pc, sb + pc * P::BN * 128, &full_bar[stage]);
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1;
@@ -207,13 +222,13 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, P::BN) | (P::B_MN ? UMMA_B_MN : 0u);
+      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, P::BN) | (P::A_MN ? UMMA_A_MN : 0u) | (P::B_MN ? UMMA_B_MN : 0u);
       using T = Terms<P::PA, P::PB>;
       int stage = 0;
       uint32_t phase = 0, it = 0;
       bool alive = true;
-      for (long long tile = blockIdx.x; tile < total && alive; tile += gridDim.x, ++it) {
-        const int split = static_cast<int>(tile % g.splits);
+      for (uint32_t tile = blockIdx.x; tile < total && alive; tile += gridDim.x, ++it) {
+        const int split = g.splits > 1 ? static_cast<int>(tile % g.splits) : 0;
         const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
         if (!mbar_wait(&acc_empty[buf], buf_phase ^ 1, g.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
@@ -231,7 +246,8 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
             const uint32_t sb = sa + P::PA * GEMM_A_BYTES;
 #pragma unroll
             for (int t = 0; t < T::N; ++t) {
-              const uint64_t adesc = umma_desc_kmajor(sa + T::a(t) * GEMM_A_BYTES, 128);
+              const uint64_t adesc = P::A_MN ? umma_desc_mnmajor(sa + T::a(t) * GEMM_A_BYTES, 8192)
+                                             : umma_desc_kmajor(sa + T::a(t) * GEMM_A_BYTES, 128);
               const uint64_t bdesc = P::B_MN ? umma_desc_mnmajor(sb + T::b(t) * P::BN * 128, 8192)
                                              : umma_desc_kmajor(sb + T::b(t) * P::BN * 128, 128);
               const bool lead = t == T::N - 1;
@@ -239,8 +255,8 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
               const int fresh = lead ? kb - k0 < P::NMAIN : (kb == k0 && t == 0);  // first product into it
 #pragma unroll
               for (int k = 0; k < GEMM_BK / 16; ++k)
-                umma_bf16_ss(d_tmem, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, P::B_MN ? k * 2048 : k * 32),
-                             idesc, !(fresh && k == 0));
+                umma_bf16_ss(d_tmem, umma_desc_advance(adesc, P::A_MN ? k * 2048 : k * 32),
+                             umma_desc_advance(bdesc, P::B_MN ? k * 2048 : k * 32), idesc, !(fresh && k == 0));
             }
             umma_commit(&empty_bar[stage]);
             if (++stage == STAGES) {
@@ -253,19 +269,23 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
       }
     }
   } else if (warp >= 4) {
-    const int quarter = warp & 3, half = (warp - 4) >> 2;
+    const int quarter = warp & 3, part = (warp - 4) >> 2;
+    constexpr int SHARE = P::BN / (P::EPI / 4);
     uint32_t it = 0;
-    for (long long tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
-      const int split = static_cast<int>(tile % g.splits);
-      const int n_tile = static_cast<int>((tile / g.splits) % g.n_tiles);
-      const int m_tile = static_cast<int>(tile / g.splits / g.n_tiles);
+    for (uint32_t tile = blockIdx.x; tile < total; tile += gridDim.x, ++it) {
+      int split, m_tile, n_tile;
+      locate(tile, split, m_tile, n_tile);
       const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
       if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
-      const int per = (g.kb[0] + g.splits - 1) / g.splits;
-      const Accum<P> acc = {tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC,
-                            min(g.kb[0], (split + 1) * per) - split * per};
-      P::epilogue(ep, m_tile, n_tile, split, acc, quarter, half, lane);
+      Accum<P> acc;
+      acc.base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
+#pragma unroll
+      for (int seg = 0; seg < P::NSEG; ++seg) {
+        const int per = (g.kb[seg] + g.splits - 1) / g.splits;
+        acc.used[seg] = min(g.kb[seg], (split + 1) * per) - split * per;
+      }
+      P::epilogue(ep, m_tile, n_tile, split, acc, quarter, part * SHARE, (part + 1) * SHARE, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
@@ -286,8 +306,10 @@ int launch_piece_gemm(const GemmMaps& maps, GemmShape g, const typename P::Param
   int rc = ensure_smem_limit(reinterpret_cast<const void*>(piece_gemm_kernel<P>), gemm_smem_bytes<P>());
   if (rc) return rc;
   const long long total = static_cast<long long>(g.m_tiles) * g.n_tiles * g.splits;
-  const unsigned grid = static_cast<unsigned>(total < sm_count() ? total : sm_count());
-  return launch(piece_gemm_kernel<P>, dim3(grid), dim3(GEMM_THREADS), gemm_smem_bytes<P>(), stream, pdl, maps, g, ep);
+  B200_REQUIRE(total < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "gemm: too many tiles (%lld)", total);
+  const long long slots = static_cast<long long>(P::CTAS) * sm_count();
+  const unsigned grid = static_cast<unsigned>(total < slots ? total : slots);
+  return launch(piece_gemm_kernel<P>, dim3(grid), dim3(gemm_threads<P>()), gemm_smem_bytes<P>(), stream, pdl, maps, g, ep);
 }
 
 // Activations: bf16 pieces [pieces][rows][k], row pitch `pitch` elements (a multiple of 8);
@@ -299,9 +321,9 @@ inline int gemm_map_kmajor(CUtensorMap* out, const void* base, int pieces, long 
   const uint32_t box[3] = {GEMM_BK, static_cast<uint32_t>(box_rows), 1};
   return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
 }
-// Weights as stored, [k][n] with row pitch `pitch` (a multiple of 8), read as MN-major tiles.
-inline int gemm_map_mnmajor(CUtensorMap* out, const void* base, int k, int n, long long pitch) {
-  const uint64_t dims[3] = {static_cast<uint64_t>(n), static_cast<uint64_t>(k), 1};
+// Weights as stored, [pieces][k][n] with row pitch `pitch` (a multiple of 8), read as MN-major tiles.
+inline int gemm_map_mnmajor(CUtensorMap* out, const void* base, int k, int n, long long pitch, int pieces = 1) {
+  const uint64_t dims[3] = {static_cast<uint64_t>(n), static_cast<uint64_t>(k), static_cast<uint64_t>(pieces)};
   const uint64_t str[2] = {static_cast<uint64_t>(pitch) * 2, static_cast<uint64_t>(pitch) * k * 2};
   const uint32_t box[3] = {64, GEMM_BK, 1};
   return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);

@@ -1,5 +1,5 @@
-// The two triangle ops for every shape and element type the tensor-core specialisation
-// (c_z = c_hidden = 128, 4 heads x 32, bf16) does not cover:
+// The two triangle ops for every shape and element type the fused 128-channel bf16 kernels do
+// not cover:
 //
 //  * the float32 trunk of the reference at the specialised shape (a correctness mode with a
 //    1e-4 bar: triangle_multiplication_forward's default contraction precision is float32,
@@ -10,12 +10,15 @@
 //    (src/foldjax/models/opendde/structural_refiner.py:62), other head counts and widths -
 //    in bf16 or float32.
 //
-// Structure. Layer norms, projections, gates, softmax and P.V are plain CUDA-core kernels in
-// float32 arithmetic. The triangle contraction, the one cubic step of the multiplicative
-// update, stays on the tensor cores: in bf16 the operands are the bf16 values themselves; in
-// float32 each operand is split into three bf16 pieces (hi + mid + lo carry 24 significand
-// bits) and the six products that matter - hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi - are
-// accumulated in float32 by the bf16 contraction kernel, smallest terms first.
+// Structure: every product runs on the tensor cores (gemm.cuh), with bf16 operands as they are
+// and float32 operands as three bf16 pieces; gates, masks, rounding and layout changes sit in
+// the products' epilogues, so that a multiplicative update is five launches
+//   layer norm -> [gate|value] product -> contraction -> layer norm -> output product
+// and an attention five
+//   layer norm -> q, k, v, bias product -> core -> gate product -> output product
+// (plus one that splits or pads weights where they cannot be read as stored). The layer norms
+// are CUDA-core kernels. Before, everything but the contraction ran on CUDA cores: 26.2 ms for the four
+// updates of a 256-token 384-channel refiner block, 6.9 ms for four 200-token templates.
 //
 // With a bf16 trunk every point where the reference's bf16 arrays round (after each matmul,
 // the sigmoid, each elementwise product or sum, the two steps of the layer-norm affine,
@@ -26,6 +29,8 @@
 
 #include <type_traits>
 
+#include "att_split.cuh"
+#include "gemm.cuh"
 #include "host.cuh"
 #include "tc.cuh"
 
@@ -40,327 +45,640 @@ struct Rb {
 
 __device__ __forceinline__ float sigmoid_exact(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// bf16 or float32 array -> float32 (parameters and the pair tensor of a bf16 trunk)
-__global__ void to_f32_kernel(const __nv_bfloat16* __restrict__ src, long long total, float* __restrict__ dst) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < total) dst[i] = __bfloat162float(src[i]);
+// Two neighbouring values as PIECES packed words, `plane` elements apart (dst 4-byte aligned).
+template <int PIECES>
+__device__ __forceinline__ void store_pair(__nv_bfloat16* dst, long long plane, float a, float b) {
+  if (PIECES == 1) {
+    *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(a, b);
+  } else {
+    uint32_t hi, mid, lo;
+    split3x2(a, b, hi, mid, lo);
+    *reinterpret_cast<uint32_t*>(dst) = hi;
+    *reinterpret_cast<uint32_t*>(dst + plane) = mid;
+    *reinterpret_cast<uint32_t*>(dst + 2 * plane) = lo;
+  }
+}
+// Eight neighbouring values the same way (dst 16-byte aligned).
+template <int PIECES>
+__device__ __forceinline__ void store_eight(__nv_bfloat16* dst, long long plane, const float* v) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (PIECES == 1) {
+      w[0][e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+    } else {
+      split3x2(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(dst + q * plane) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+}
+// Eight neighbouring values to the caller's tensor, with the caller's residual added (one more
+// rounding of the trunk dtype).
+template <bool BF, typename O>
+__device__ __forceinline__ void store_out(O* dst, const O* res, float* v, bool aligned) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = Rb<BF>::r(v[e]);
+  if (aligned) {
+    constexpr int W = 8 * sizeof(O) / 16;
+    uint4 raw[W];
+    O* o = reinterpret_cast<O*>(raw);
+    if (res) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) raw[w] = reinterpret_cast<const uint4*>(res)[w];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = Rb<BF>::r(static_cast<float>(o[e]) + v[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = static_cast<O>(v[e]);
+#pragma unroll
+    for (int w = 0; w < W; ++w) reinterpret_cast<uint4*>(dst)[w] = raw[w];
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) dst[e] = static_cast<O>(res ? Rb<BF>::r(static_cast<float>(res[e]) + v[e]) : v[e]);
+  }
+}
+
+// -------------------------------------------------------------------------- weights
+// dst[piece][k][ld] = pieces of src[k][n], padding columns zero: float32 weights, and bf16 ones
+// whose pitch or address TMA cannot take.
+struct WeightJob {
+  const void* src;
+  __nv_bfloat16* dst;
+  int k, n, ld;
+};
+struct WeightJobs {
+  WeightJob job[6];
+};
+template <bool BF>
+__global__ void weight_kernel(const WeightJobs jobs) {
+  pdl_wait();
+  pdl_trigger();
+  const WeightJob j = jobs.job[blockIdx.y];
+  const long long total = static_cast<long long>(j.k) * j.ld;
+  for (long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
+       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int r = static_cast<int>(idx / j.ld), c = static_cast<int>(idx % j.ld);
+    const long long at = static_cast<long long>(r) * j.n + c;
+    if (BF) {
+      j.dst[idx] = c < j.n ? static_cast<const __nv_bfloat16*>(j.src)[at] : __float2bfloat16_rn(0.f);
+    } else {
+      split3(c < j.n ? static_cast<const float*>(j.src)[at] : 0.f, j.dst[idx], j.dst[total + idx], j.dst[2 * total + idx]);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ layer norm + gather
-// xn[(o * n_inner + t)][:] = LN(x[o * xs_o + t * xs_i + :]); one warp per pair, any width c.
-// X is float or __nv_bfloat16 (the caller's pair tensor is read as it is stored).
-template <bool BF, typename X>
-__global__ void ln_gather_kernel(const X* __restrict__ x, long long xs_o, long long xs_i, int n_outer, int n_inner,
-                                 int c, const float* __restrict__ scale, const float* __restrict__ bias, float eps,
-                                 float* __restrict__ xn) {
+// xn[piece][(b, o, t)][:] = LN(x[b][o * xs_o + t * xs_i + :]). A warp takes W successive t of one
+// row, each in registers (V channel pairs per lane), so that the loads of all of them are in
+// flight together. Optionally the pair's mask bias of the attention core, mb[(b, o)][t] (the
+// pitch padding with the last pair of a row).
+// Bound: HBM / L2 traffic. The grid is (t, o, b): no divisions.
+struct LnArgs {
+  const void* x;
+  long long xs_b, xs_o, xs_i;
+  int batch, n, c;
+  const void* scale;
+  const void* bias;
+  float eps;
+  __nv_bfloat16* xn;
+  bool aligned;  // x is read two channels at a time
+  float* mb;     // or null
+  const float* mask;
+  long long ms_b, ms_o, ms_i;
+  float inf;
+  int mb_ld;
+};
+constexpr int LN_WARPS = 8;
+template <bool BF, int V, int W>
+__global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a) {
+  using X = typename std::conditional<BF, __nv_bfloat16, float>::type;
+  using X2 = typename std::conditional<BF, __nv_bfloat162, float2>::type;
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
-  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long pairs = static_cast<long long>(n_outer) * n_inner;
-  if (warp >= pairs) return;
-  const int o = static_cast<int>(warp / n_inner), t = static_cast<int>(warp % n_inner);
-  const X* src = x + o * xs_o + t * xs_i;
-  float s = 0.f;
-  for (int i = lane; i < c; i += 32) s += static_cast<float>(src[i]);
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  const float mean = s / c;
-  float q = 0.f;
-  for (int i = lane; i < c; i += 32) {
-    const float v = static_cast<float>(src[i]) - mean;
-    q += v * v;
+  const int t0 = (blockIdx.x * LN_WARPS + (threadIdx.x >> 5)) * W, o = blockIdx.y, b = blockIdx.z;
+  if (t0 >= a.n) return;
+  const int bo = b * a.n + o;
+  if (a.mb) {
+    float* row = a.mb + static_cast<long long>(bo) * a.mb_ld;
+    if (lane < W && t0 + lane < a.n)
+      row[t0 + lane] = a.mask ? fmaxf(a.inf * (a.mask[b * a.ms_b + o * a.ms_o + (t0 + lane) * a.ms_i] - 1.0f), SPLIT_MASK_MIN) : 0.f;
+    if (t0 + W >= a.n)
+      for (int e = a.n + lane; e < a.mb_ld; e += 32) row[e] = SPLIT_MASK_PAD;
   }
+  const X* src = static_cast<const X*>(a.x) + b * a.xs_b + o * a.xs_o + t0 * a.xs_i;
+  float2 v[W][V];
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
-  const float rstd = 1.0f / sqrtf(q / c + eps);
-  float* dst = xn + warp * c;
-  for (int i = lane; i < c; i += 32) {
-    const float normed = Rb<BF>::r((static_cast<float>(src[i]) - mean) * rstd);  // cast before the affine step
-    dst[i] = Rb<BF>::r(Rb<BF>::r(normed * scale[i]) + bias[i]);
-  }
-}
-
-// --------------------------------------------------------------------------- float32 GEMM
-// out[row(m)][n] = R(sum_k a[m][k] * w[k][n]) (+ res); a is [M][K] dense, w [K][N] dense.
-// Output rows are addressed as (m / rows_inner) * s_outer + (m % rows_inner) * s_inner, which
-// lets the last projection of the attention write straight through the caller's strides.
-// O is the output element type (float, or __nv_bfloat16 for the final result of a bf16 trunk).
-template <bool BF, typename O>
-__global__ void __launch_bounds__(256)
-gemm_kernel(const float* __restrict__ a, const float* __restrict__ w, long long M, int K, int N, O* __restrict__ out,
-            const O* __restrict__ res, int rows_inner, long long s_outer, long long s_inner) {
-  __shared__ float as[16][64 + 1];
-  __shared__ float ws[16][64];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const long long m0 = static_cast<long long>(blockIdx.x) * 64;  // rows on x: the pair count exceeds 65535 * 64
-  const int n0 = blockIdx.y * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int idx = threadIdx.x; idx < 64 * 16; idx += 256) {
-      const int r = idx >> 4, c = idx & 15;
-      const long long m = m0 + r;
-      as[c][r] = (m < M && k0 + c < K) ? a[m * K + k0 + c] : 0.f;
-    }
-    for (int idx = threadIdx.x; idx < 16 * 64; idx += 256) {
-      const int r = idx >> 6, c = idx & 63;
-      ws[r][c] = (k0 + r < K && n0 + c < N) ? w[static_cast<long long>(k0 + r) * N + n0 + c] : 0.f;
-    }
-    __syncthreads();
+  for (int w = 0; w < W; ++w) {
+    const X* row = src + (t0 + w < a.n ? w : 0) * a.xs_i;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        av[e] = as[k][ty * 4 + e];
-        bv[e] = ws[k][tx * 4 + e];
+    for (int e = 0; e < V; ++e) {
+      const int i = 2 * (lane + 32 * e);
+      v[w][e] = make_float2(0.f, 0.f);
+      if (i < a.c) {
+        if (a.aligned) {
+          const X2 q = *reinterpret_cast<const X2*>(row + i);
+          v[w][e] = make_float2(static_cast<float>(q.x), static_cast<float>(q.y));
+        } else {
+          v[w][e] = make_float2(static_cast<float>(row[i]), static_cast<float>(row[i + 1]));
+        }
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
     }
-    __syncthreads();
+  }
+  const float inv_c = 1.0f / a.c;
+  float s[W], q[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    s[w] = 0.f;
+#pragma unroll
+    for (int e = 0; e < V; ++e) s[w] += v[w][e].x + v[w][e].y;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-    const long long row = (m / rows_inner) * s_outer + (m % rows_inner) * s_inner;
+  for (int d = 16; d > 0; d >>= 1)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = Rb<BF>::r(acc[i][j]);
-      if (res) v = Rb<BF>::r(v + static_cast<float>(res[row + n]));  // the caller's z + update
-      out[row + n] = static_cast<O>(v);
+    for (int w = 0; w < W; ++w) s[w] += __shfl_xor_sync(0xffffffffu, s[w], d);
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    s[w] *= inv_c;
+    q[w] = 0.f;
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+      if (2 * (lane + 32 * e) < a.c) {
+        const float dx = v[w][e].x - s[w], dy = v[w][e].y - s[w];
+        q[w] = fmaf(dx, dx, fmaf(dy, dy, q[w]));
+      }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+    for (int w = 0; w < W; ++w) q[w] += __shfl_xor_sync(0xffffffffu, q[w], d);
+#pragma unroll
+  for (int w = 0; w < W; ++w) q[w] = 1.0f / sqrtf(q[w] * inv_c + a.eps);
+  const X* scale = static_cast<const X*>(a.scale);
+  const X* bias = static_cast<const X*>(a.bias);
+  const long long plane = static_cast<long long>(a.batch) * a.n * a.n * a.c;
+  __nv_bfloat16* dst = a.xn + (static_cast<long long>(bo) * a.n + t0) * a.c;
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const int i = 2 * (lane + 32 * e);
+    if (i >= a.c) continue;
+    const float g[2] = {static_cast<float>(scale[i]), static_cast<float>(scale[i + 1])};
+    const float h[2] = {static_cast<float>(bias[i]), static_cast<float>(bias[i + 1])};
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (t0 + w >= a.n) break;
+      float r[2] = {v[w][e].x, v[w][e].y};
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {  // cast before the affine step
+        const float normed = Rb<BF>::r((r[u] - s[w]) * q[w]);
+        r[u] = Rb<BF>::r(Rb<BF>::r(normed * g[u]) + h[u]);
+      }
+      store_pair<BF ? 1 : 3>(dst + w * a.c + i, plane, r[0], r[1]);
     }
   }
 }
 
-template <bool BF, typename O = float>
-int gemm(const float* a, const float* w, long long M, int K, int N, O* out, cudaStream_t stream, const O* res = nullptr,
-         int rows_inner = 0, long long s_outer = 0, long long s_inner = 0) {
-  if (rows_inner <= 0) {  // dense [M][N]
-    rows_inner = 1;
-    s_outer = N;
-    s_inner = 0;
-  }
-  dim3 grid(static_cast<unsigned>((M + 63) / 64), static_cast<unsigned>((N + 63) / 64));
-  count_launch();
-  gemm_kernel<BF, O><<<grid, 256, 0, stream>>>(a, w, M, K, N, out, res, rows_inner, s_outer, s_inner);
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
-}
-
-// ------------------------------------------------------------------- tri-mult: gate + split
-// v = R(R(R(sigmoid(g)) * p) * mask) for the 2 * c_h projected channels of a pair; the first
-// c_h are a, the rest b (triangle.py:102). Written as bf16 pieces into piece-major,
-// channel-major planes [piece][channel][o][ld] with the channel count padded to `planes` (a
-// multiple of 128: the tensor-core contraction walks 128 channels per call; padding planes
-// stay zero). One block = one row o and 32 consecutive t; shared memory turns the
-// channel-contiguous reads into t-contiguous writes, 64 channels at a time.
 template <bool BF>
-__global__ void __launch_bounds__(256)
-glu_split_kernel(const float* __restrict__ p, const float* __restrict__ g, const float* __restrict__ mask,
-                 long long ms_o, long long ms_i, int n_outer, int n_inner, int ld, int c_h, int planes, int pieces,
-                 __nv_bfloat16* __restrict__ a, __nv_bfloat16* __restrict__ b) {
-  __shared__ float tile[32][64 + 1];
-  const int o = blockIdx.y, t0 = blockIdx.x * 32;
-  const int width = 2 * c_h;
-  const long long plane = static_cast<long long>(n_outer) * ld;  // one channel
-  const long long piece = static_cast<long long>(planes) * plane;
-  for (int c0 = 0; c0 < width; c0 += 64) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * 64; idx += 256) {
-      const int tt = idx >> 6, cc = idx & 63;
-      const int t = t0 + tt, c = c0 + cc;
-      float v = 0.f;
-      if (t < n_inner && c < width) {
-        const long long pair = static_cast<long long>(o) * n_inner + t;
-        const float m = mask ? Rb<BF>::r(mask[o * ms_o + t * ms_i]) : 1.0f;
-        const float gate = Rb<BF>::r(sigmoid_exact(g[pair * width + c]));
-        v = Rb<BF>::r(Rb<BF>::r(gate * p[pair * width + c]) * m);
-      }
-      tile[tt][cc] = v;
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * 64; idx += 256) {
-      const int cc = idx >> 5, tt = idx & 31;
-      const int t = t0 + tt, c = c0 + cc;
-      if (t >= ld || c >= width) continue;
-      const float v = t < n_inner ? tile[tt][cc] : 0.f;  // pitch padding is zero: it is read as k
-      const int chan = c < c_h ? c : c - c_h;
-      __nv_bfloat16* dst = (c < c_h ? a : b) + static_cast<long long>(chan) * plane + static_cast<long long>(o) * ld + t;
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-      dst[0] = hi;
-      if (pieces == 3) {
-        const float r1 = v - __bfloat162float(hi);
-        const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-        dst[piece] = mid;
-        dst[2 * piece] = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-      }
-    }
-  }
+int launch_ln_gather(LnArgs a, cudaStream_t stream, bool pdl) {
+  a.aligned = (reinterpret_cast<uintptr_t>(a.x) & (BF ? 3 : 7)) == 0;
+  auto go = [&](auto kernel, int w) {
+    const dim3 grid((a.n + LN_WARPS * w - 1) / (LN_WARPS * w), static_cast<unsigned>(a.n), static_cast<unsigned>(a.batch));
+    return launch(kernel, grid, dim3(LN_WARPS * 32), 0, stream, pdl, a);
+  };
+  if (a.c <= 64) return go(ln_gather_kernel<BF, 1, 4>, 4);
+  if (a.c <= 128) return go(ln_gather_kernel<BF, 2, 4>, 4);
+  if (a.c <= 384) return go(ln_gather_kernel<BF, 6, 2>, 2);
+  return go(ln_gather_kernel<BF, 16, 1>, 1);
 }
 
 // ------------------------------------------------------------ tri-mult: LN of the contraction
-// tn[(i * n + j)][:] = LN_out(R(t[:, i, j])) with t channel-major float32 [planes][n][ld]; the
-// contraction is rounded to the trunk dtype before the layer norm (triangle.py:124-126).
-// One warp per pair.
+// tn[piece][(b, i, j)][:] = LN_out(t[b][:, i, j]) with t channel-major [b * c_h + channel][n][ld],
+// rounded to the trunk dtype before the layer norm (triangle.py:124-126). One block = 128 bytes
+// of neighbouring j of a row (64 in bf16, 32 in float32) with all their channels in shared
+// memory. A lane owns one word of that row - two j in bf16, one in float32 - and a warp an
+// eighth of the channels, so that the statistics are plain sums per lane (one exchange of eight
+// partial sums each) and nothing is shuffled: 40 instructions per pair where one warp per pair
+// took 209. Eight neighbouring channels leave per lane as one 16-byte store.
+constexpr int LNT_WARPS = 8;
 template <bool BF>
-__global__ void ln_channel_major_kernel(const float* __restrict__ t, int n, int ld, int c_h,
-                                        const float* __restrict__ scale, const float* __restrict__ bias, float eps,
-                                        float* __restrict__ tn) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long pairs = static_cast<long long>(n) * n;
-  if (warp >= pairs) return;
-  const int i = static_cast<int>(warp / n), j = static_cast<int>(warp % n);
-  const float* src = t + static_cast<long long>(i) * ld + j;
-  const long long plane = static_cast<long long>(n) * ld;
-  float s = 0.f;
-  for (int c = lane; c < c_h; c += 32) s += Rb<BF>::r(src[c * plane]);
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-  const float mean = s / c_h;
-  float q = 0.f;
-  for (int c = lane; c < c_h; c += 32) {
-    const float v = Rb<BF>::r(src[c * plane]) - mean;
-    q += v * v;
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
-  const float rstd = 1.0f / sqrtf(q / c_h + eps);
-  float* dst = tn + warp * c_h;
-  for (int c = lane; c < c_h; c += 32) {
-    const float normed = Rb<BF>::r((Rb<BF>::r(src[c * plane]) - mean) * rstd);
-    dst[c] = Rb<BF>::r(Rb<BF>::r(normed * scale[c]) + bias[c]);
-  }
+constexpr int lnt_j() {
+  return BF ? 64 : 32;
 }
-
-// out[i][j][c] = R(o[(i * n + j)][c] * R(sigmoid(gate[(gi * n + gj)][c]))) (+ residual), where the
-// gate rows live in the projection frame: (gi, gj) = (i, j), or (j, i) when that frame is
-// transposed.
-template <bool BF, typename O>
-__global__ void gate_out_kernel(const float* __restrict__ o, const float* __restrict__ gate, int n, int c_z,
-                                int transposed, const O* __restrict__ residual, O* __restrict__ out) {
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const long long total = static_cast<long long>(n) * n * c_z;
-  if (idx >= total) return;
-  const int c = static_cast<int>(idx % c_z);
-  const long long pair = idx / c_z;
-  const int i = static_cast<int>(pair / n), j = static_cast<int>(pair % n);
-  const long long gp = transposed ? static_cast<long long>(j) * n + i : pair;
-  float v = Rb<BF>::r(o[idx] * Rb<BF>::r(sigmoid_exact(gate[gp * c_z + c])));
-  if (residual) v = Rb<BF>::r(static_cast<float>(residual[idx]) + v);
-  out[idx] = static_cast<O>(v);
-}
-
-// in place: o[m][c] = R(o[m][c] * R(sigmoid(g[m][c])))
+inline int lnt_smem(int c_h) { return c_h * 128 + 2 * LNT_WARPS * 64 * 4; }
 template <bool BF>
-__global__ void mul_sigmoid_kernel(float* __restrict__ o, const float* __restrict__ g, long long total) {
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx < total) o[idx] = Rb<BF>::r(o[idx] * Rb<BF>::r(sigmoid_exact(g[idx])));
-}
-
-// ------------------------------------------------------------------- tri-attn: attention core
-// One block = (row o, head h, 128 queries); one thread per query; K and V of the row stream
-// through shared memory 32 keys at a time. Scores follow the reference's order and precision
-// (triangle_attention.py:449-455): (q.k + mask_bias) + tri_bias in float32, softmax in float32,
-// P.v in float32, cast to the trunk dtype. q is divided by sqrt(d), evaluated and rounded in
-// the trunk dtype, first (:399-400).
-constexpr int AQ = 128, AK = 32;
-template <bool BF, int HD>
-__global__ void __launch_bounds__(AQ)
-att_core_kernel_f32(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                    const float* __restrict__ bias, const float* __restrict__ mask, long long ms_o, long long ms_k,
-                    float inf, int n, int heads, float* __restrict__ out) {
-  __shared__ float ks[AK][HD], vs[AK][HD], mb[AK];
-  const int o = blockIdx.z, h = blockIdx.y;
-  const int j = blockIdx.x * AQ + threadIdx.x;
-  const bool live = j < n;
-  const int width = heads * HD;
-  const float q_scale = Rb<BF>::r(sqrtf(static_cast<float>(HD)));
-  float qr[HD], acc[HD];
-  const float* qrow = q + (static_cast<long long>(o) * n + (live ? j : 0)) * width + h * HD;
+__global__ void __launch_bounds__(LNT_WARPS * 32)
+ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, const void* __restrict__ scale_,
+                        const void* __restrict__ bias_, float eps, long long pairs, __nv_bfloat16* __restrict__ tn) {
+  using X = typename std::conditional<BF, __nv_bfloat16, float>::type;
+  constexpr int JT = lnt_j<BF>(), JL = JT / 32;  // j of a block, of a lane
+  extern __shared__ uint32_t tile[];             // [c_h][32 words], then the partial sums
+  float* part = reinterpret_cast<float*>(tile + c_h * 32);
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.y, b = blockIdx.z, j0 = blockIdx.x * JT;
+  const X* src = static_cast<const X*>(t_) + (static_cast<long long>(b) * c_h * n + i) * ld + j0;
+  const long long chan = static_cast<long long>(n) * ld;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // groups of eight channels, dealt to the warps in turn
+  const int groups = c_h / 8;
+  auto value = [&](uint32_t w, int u) { return BF ? (u ? bf16_hi(w) : bf16_lo(w)) : __uint_as_float(w); };
+  float s[JL] = {}, q[JL] = {};
+  for (int g = warp; g < groups; g += LNT_WARPS) {
+    uint32_t w[8];
 #pragma unroll
-  for (int d = 0; d < HD; ++d) {
-    qr[d] = Rb<BF>::r(qrow[d] / q_scale);
-    acc[d] = 0.f;
+    for (int e = 0; e < 8; ++e) w[e] = reinterpret_cast<const uint32_t*>(src + (g * 8 + e) * chan)[lane];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      tile[(g * 8 + e) * 32 + lane] = w[e];
+#pragma unroll
+      for (int u = 0; u < JL; ++u) s[u] += value(w[e], u);
+    }
   }
-  float m_run = -INFINITY, l_run = 0.f;
-  for (int k0 = 0; k0 < n; k0 += AK) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < AK * HD; idx += AQ) {
-      const int r = idx / HD, d = idx % HD;
-      const int kk = k0 + r;
-      const long long src = (static_cast<long long>(o) * n + kk) * width + h * HD + d;
-      ks[r][d] = kk < n ? k[src] : 0.f;
-      vs[r][d] = kk < n ? v[src] : 0.f;
-    }
-    if (threadIdx.x < AK) {
-      const int kk = k0 + threadIdx.x;
-      mb[threadIdx.x] = kk < n ? (mask ? inf * (mask[o * ms_o + kk * ms_k] - 1.0f) : 0.0f) : -INFINITY;
-    }
-    __syncthreads();
-    if (!live) continue;
-    float sc[AK];
-    float mx = m_run;
 #pragma unroll
-    for (int r = 0; r < AK; ++r) {
-      float s = 0.f;
+  for (int u = 0; u < JL; ++u) part[(warp * JL + u) * 32 + lane] = s[u];
+  __syncthreads();
+  const float inv_c = 1.0f / c_h;
 #pragma unroll
-      for (int d = 0; d < HD; ++d) s = fmaf(qr[d], ks[r][d], s);
-      const int kk = k0 + r;
-      const float tb = kk < n ? bias[(static_cast<long long>(j) * n + kk) * heads + h] : 0.f;
-      s = (s + mb[r]) + tb;
-      sc[r] = s;
-      mx = fmaxf(mx, s);
-    }
-    const float corr = expf(m_run - mx);  // 0 on the first tile
-    l_run *= corr;
+  for (int u = 0; u < JL; ++u) {
+    s[u] = 0.f;
 #pragma unroll
-    for (int d = 0; d < HD; ++d) acc[d] *= corr;
-#pragma unroll
-    for (int r = 0; r < AK; ++r) {
-      const float pexp = expf(sc[r] - mx);
-      l_run += pexp;
-#pragma unroll
-      for (int d = 0; d < HD; ++d) acc[d] = fmaf(pexp, vs[r][d], acc[d]);
-    }
-    m_run = mx;
+    for (int w = 0; w < LNT_WARPS; ++w) s[u] += part[(w * JL + u) * 32 + lane];
+    s[u] *= inv_c;  // the mean
   }
-  if (live) {
-    float* dst = out + (static_cast<long long>(o) * n + j) * width + h * HD;
+  for (int g = warp; g < groups; g += LNT_WARPS)
 #pragma unroll
-    for (int d = 0; d < HD; ++d) dst[d] = Rb<BF>::r(acc[d] / l_run);
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t w = tile[(g * 8 + e) * 32 + lane];  // (this thread's own words)
+#pragma unroll
+      for (int u = 0; u < JL; ++u) {
+        const float d = value(w, u) - s[u];
+        q[u] = fmaf(d, d, q[u]);
+      }
+    }
+  float* part_q = part + LNT_WARPS * JL * 32;
+#pragma unroll
+  for (int u = 0; u < JL; ++u) part_q[(warp * JL + u) * 32 + lane] = q[u];
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < JL; ++u) {
+    q[u] = 0.f;
+#pragma unroll
+    for (int w = 0; w < LNT_WARPS; ++w) q[u] += part_q[(w * JL + u) * 32 + lane];
+    q[u] = 1.0f / sqrtf(q[u] * inv_c + eps);
+  }
+  const X* scale = static_cast<const X*>(scale_);
+  const X* bias = static_cast<const X*>(bias_);
+  __nv_bfloat16* dst = tn + ((static_cast<long long>(b) * n + i) * n + j0 + lane * JL) * c_h;
+  for (int g = warp; g < groups; g += LNT_WARPS) {
+    float v[JL][8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int c = g * 8 + e;
+      const uint32_t w = tile[c * 32 + lane];
+      const float sc = static_cast<float>(scale[c]), bi = static_cast<float>(bias[c]);
+#pragma unroll
+      for (int u = 0; u < JL; ++u)
+        v[u][e] = Rb<BF>::r(Rb<BF>::r(Rb<BF>::r((value(w, u) - s[u]) * q[u]) * sc) + bi);
+    }
+#pragma unroll
+    for (int u = 0; u < JL; ++u)
+      if (j0 + lane * JL + u < n) store_eight<BF ? 1 : 3>(dst + u * c_h + g * 8, pairs * c_h, v[u]);
   }
 }
 
 template <bool BF>
-int launch_att_core(int head_dim, dim3 grid, cudaStream_t stream, const float* q, const float* k, const float* v,
-                    const float* bias, const float* mask, long long ms_o, long long ms_k, float inf, int n, int heads,
-                    float* out) {
-  count_launch();
-  switch (head_dim) {
-#define B200_CASE(HD)                                                                                      \
-  case HD:                                                                                                 \
-    att_core_kernel_f32<BF, HD><<<grid, AQ, 0, stream>>>(q, k, v, bias, mask, ms_o, ms_k, inf, n, heads, out); \
-    break;
-    B200_CASE(8)
-    B200_CASE(16)
-    B200_CASE(24)
-    B200_CASE(32)
-    B200_CASE(48)
-    B200_CASE(64)
-#undef B200_CASE
-    default:
-      set_error("triatt: head widths 8, 16, 24, 32, 48 and 64 are built (got %d)", head_dim);
-      return B200TRI_ERR_UNSUPPORTED;
-  }
-  B200_CUDA_OK(cudaGetLastError());
-  return B200TRI_OK;
+int launch_ln_channel_major(const void* t, int n, int batch, int ld, int c_h, const void* scale, const void* bias, float eps,
+                            __nv_bfloat16* tn, cudaStream_t stream) {
+  const int rc = ensure_smem_limit(reinterpret_cast<const void*>(ln_channel_major_kernel<BF>), lnt_smem(1024));
+  if (rc) return rc;
+  const dim3 grid((n + lnt_j<BF>() - 1) / lnt_j<BF>(), static_cast<unsigned>(n), static_cast<unsigned>(batch));
+  return launch(ln_channel_major_kernel<BF>, grid, dim3(LNT_WARPS * 32), lnt_smem(c_h), stream, true, t, n, ld, c_h, scale, bias,
+                eps, static_cast<long long>(batch) * n * n, tn);
 }
 
+// ------------------------------------------------------------------- product policies
+// Rows of pieces addressed as (batch, outer, inner): one box is `box` successive inner positions.
+int map_rows(CUtensorMap* out, const void* base, int k, int n, long long s_inner, long long s_outer, int batch,
+             int pieces, long long s_piece, int box) {
+  const uint64_t un = n;
+  const uint64_t dims[5] = {static_cast<uint64_t>(k), un, un, static_cast<uint64_t>(batch), static_cast<uint64_t>(pieces)};
+  const uint64_t str[4] = {static_cast<uint64_t>(s_inner) * 2, static_cast<uint64_t>(s_outer) * 2,
+                           un * un * static_cast<uint64_t>(k) * 2, static_cast<uint64_t>(s_piece) * 2};
+  const uint32_t bx[5] = {GEMM_BK, static_cast<uint32_t>(box), 1, 1, 1};
+  return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, bx, Swz::B128);
+}
+
+// Tile `tile` of rows walked `box` inner positions at a time.
+struct RowTile {
+  int b, o, t0;
+  __device__ RowTile(uint32_t tile, uint32_t n, uint32_t tiles_t, int box) {
+    const uint32_t bo = tile / tiles_t, bb = bo / n;
+    t0 = static_cast<int>(tile - bo * tiles_t) * box;
+    o = static_cast<int>(bo - bb * n);
+    b = static_cast<int>(bb);
+  }
+};
+
+// [a|b] = R(R(sigmoid(xn g)) * (xn p)) * mask, channel-major planes [piece][b * c_h + channel][o][ld].
+// Transposed product (a TMEM lane is a channel of the 2 * c_h, segment 0 the values, 1 the
+// gates), so that a thread stores runs of neighbouring pairs.
+template <int PIECES, int NM>
+struct GluPolicy {
+  static constexpr int BN = PIECES == 1 ? 128 : 64, PA = PIECES, PB = PIECES, NSEG = 2, NMAIN = NM;
+  static constexpr bool A_MN = true, B_MN = false, M_FAST = true;
+  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  struct Params {
+    int n, tiles_t, c_h, ld;
+    long long piece;  // elements between pieces of a plane set
+    const float* mask;
+    long long ms_b, ms_o, ms_i;
+    __nv_bfloat16 *a, *b;
+  };
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int seg, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.a[seg], dst, bar, 2, m_tile * GEMM_BM, k, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params& p, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    const RowTile r(n_tile, p.n, p.tiles_t, BN);
+    tma_load_5d(dst, &maps.b[0], bar, k, r.t0, r.o, r.b, piece);
+  }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<GluPolicy>& acc, int quarter,
+                                  int col0, int col1, int lane) {
+    constexpr bool BF = PIECES == 1;
+    const RowTile rt(n_tile, p.n, p.tiles_t, BN);
+    const int c = m_tile * GEMM_BM + quarter * 32 + lane;
+    const int chan = c < p.c_h ? c : c - p.c_h;
+    __nv_bfloat16* dst = (c < p.c_h ? p.a : p.b) +
+                         ((static_cast<long long>(rt.b) * p.c_h + chan) * p.n + rt.o) * p.ld + rt.t0;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      if (rt.t0 + col >= p.n) break;
+      const int t = rt.t0 + col + (lane & 15);
+      float mk = 1.0f;
+      if (p.mask && t < p.n) mk = Rb<BF>::r(p.mask[rt.b * p.ms_b + rt.o * p.ms_o + t * p.ms_i]);
+      float v[16], g[16];
+      acc.load(0, col, v);
+      acc.load(1, col, g);
+#pragma unroll
+      for (int e = 0; e < 16; e += 2) {
+        const float m0 = __shfl_sync(0xffffffffu, mk, e), m1 = __shfl_sync(0xffffffffu, mk, e + 1);
+        if (BF) {
+          const uint32_t u = bf16x2_mul(bf16x2_mul(sigmoid_bf16x2(g[e], g[e + 1]), pack_bf16x2(v[e], v[e + 1])),
+                                        pack_bf16x2(m0, m1));
+          v[e] = bf16_lo(u);
+          v[e + 1] = bf16_hi(u);
+        } else {
+          v[e] = sigmoid_exact(g[e]) * v[e] * m0;
+          v[e + 1] = sigmoid_exact(g[e + 1]) * v[e + 1] * m1;
+        }
+      }
+      if (c < 2 * p.c_h)  // (the pitch is a multiple of 64: the padding takes what lies past n)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) store_eight<PIECES>(dst + col + 8 * q, p.piece, v + 8 * q);
+    }
+  }
+};
+
+// out = R(R(tn p_out) * R(sigmoid(R(xn g_out)))) (+ residual)
+template <int PIECES, int NM, int BN_>
+struct OutGatePolicy {
+  static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 2, NMAIN = NM;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr bool BF = PIECES == 1;
+  using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
+  struct Params {
+    int n, tiles_j, c_z;
+    const O* res;
+    O* out;
+    bool aligned;
+  };
+  static __device__ void load_a(const GemmMaps& maps, const Params& p, int seg, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    const RowTile r(m_tile, p.n, p.tiles_j, GEMM_BM);
+    tma_load_5d(dst, &maps.a[seg], bar, k, r.t0, r.o, r.b, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params&, int seg, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.b[seg], dst, bar, BN / 64, n_tile * BN, k, piece);
+  }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<OutGatePolicy>& acc, int quarter,
+                                  int col0, int col1, int lane) {
+    const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
+    const int j = rt.t0 + quarter * 32 + lane;
+    const long long off = ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      const int c0 = n_tile * BN + col;
+      if (c0 >= p.c_z) break;
+      float v[16], g[16];
+      acc.load(0, col, v);
+      acc.load(1, col, g);
+      if (j >= p.n) continue;
+#pragma unroll
+      for (int e = 0; e < 16; e += 2) {
+        if (BF) {
+          const uint32_t u = bf16x2_mul(pack_bf16x2(v[e], v[e + 1]), sigmoid_bf16x2(g[e], g[e + 1]));
+          v[e] = bf16_lo(u);
+          v[e + 1] = bf16_hi(u);
+        } else {
+          v[e] *= sigmoid_exact(g[e]);
+          v[e + 1] *= sigmoid_exact(g[e + 1]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (c0 + 8 * q < p.c_z)
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+    }
+  }
+};
+
+// q / sqrt(d), k: rows [piece][pair][hd]. v: transposed, [piece][(b, o)][hd][ld]. bias: [b][head][o][ld] in the trunk dtype. Column tiles walk
+// the four weights in turn.
+template <int PIECES, int NM, int BN_>
+struct QkvbPolicy {
+  static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr bool BF = PIECES == 1;
+  struct Params {
+    int n, hd, heads, tiles_w, ld;
+    uint32_t pairs;
+    float q_scale;
+    long long row_piece, v_piece;  // elements between pieces of q / k and of v
+    __nv_bfloat16 *q, *k, *vt;
+    void* bias;
+  };
+  static __device__ int which(const Params& p, int n_tile) { return n_tile / p.tiles_w < 3 ? n_tile / p.tiles_w : 3; }
+  static __device__ void load_a(const GemmMaps& maps, const Params& p, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params& p, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    const int w = which(p, n_tile);
+    gemm_load_mn(&maps.b[w], dst, bar, BN / 64, (n_tile - w * p.tiles_w) * BN, k, piece);
+  }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvbPolicy>& acc, int quarter,
+                                  int col0, int col1, int lane) {
+    const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
+    const uint32_t bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
+    const int w = which(p, n_tile);
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      const int c0 = (n_tile - w * p.tiles_w) * BN + col;
+      if (c0 >= (w == 3 ? p.heads : p.hd)) break;
+      float v[16];
+      acc.load(0, col, v);
+      if (pair >= p.pairs) continue;
+      if (w < 2) {
+        __nv_bfloat16* dst = (w ? p.k : p.q) + static_cast<long long>(pair) * p.hd + c0;
+        if (w == 0)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] = Rb<BF>::r(v[e]) / p.q_scale;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (c0 + 8 * q < p.hd) store_eight<PIECES>(dst + 8 * q, p.row_piece, v + 8 * q);
+      } else if (w == 2) {
+        __nv_bfloat16* dst = p.vt + (static_cast<long long>(bo) * p.hd + c0) * p.ld + t;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          if (c0 + e >= p.hd) break;
+          if (BF) {
+            dst[static_cast<long long>(e) * p.ld] = __float2bfloat16_rn(v[e]);
+          } else {
+            __nv_bfloat16* d = dst + static_cast<long long>(e) * p.ld;
+            split3(v[e], d[0], d[p.v_piece], d[2 * p.v_piece]);
+          }
+        }
+      } else {
+        const long long at = (static_cast<long long>(b * p.heads + c0) * p.n + o) * p.ld + t;
+        const long long head = static_cast<long long>(p.n) * p.ld;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          if (c0 + e >= p.heads) break;
+          if (BF)
+            static_cast<__nv_bfloat16*>(p.bias)[at + e * head] = __float2bfloat16_rn(v[e]);
+          else
+            static_cast<float*>(p.bias)[at + e * head] = v[e];
+        }
+      }
+    }
+  }
+};
+
+// y = R(o * R(sigmoid(R(xn Wg)))): bf16 in place over o, float32 o -> pieces
+template <int PIECES, int NM, int BN_>
+struct GatePolicy {
+  static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr bool BF = PIECES == 1;
+  struct Params {
+    long long pairs;
+    int hd;
+    const float* o;
+    __nv_bfloat16* y;
+  };
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params&, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.b[0], dst, bar, BN / 64, n_tile * BN, k, piece);
+  }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<GatePolicy>& acc, int quarter,
+                                  int col0, int col1, int lane) {
+    const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      const int c0 = n_tile * BN + col;
+      if (c0 >= p.hd) break;
+      float g[16];
+      acc.load(0, col, g);
+      if (pair >= p.pairs) continue;
+      const long long off = pair * p.hd + c0;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (c0 + 8 * q >= p.hd) break;
+        if (BF) {
+          uint4* ptr = reinterpret_cast<uint4*>(p.y + off + 8 * q);
+          uint4 w = *ptr;
+          w.x = bf16x2_mul(w.x, sigmoid_bf16x2(g[8 * q + 0], g[8 * q + 1]));
+          w.y = bf16x2_mul(w.y, sigmoid_bf16x2(g[8 * q + 2], g[8 * q + 3]));
+          w.z = bf16x2_mul(w.z, sigmoid_bf16x2(g[8 * q + 4], g[8 * q + 5]));
+          w.w = bf16x2_mul(w.w, sigmoid_bf16x2(g[8 * q + 6], g[8 * q + 7]));
+          *ptr = w;
+        } else {
+          float v[8];
+#pragma unroll
+          for (int h4 = 0; h4 < 2; ++h4) {
+            const float4 f = *reinterpret_cast<const float4*>(p.o + off + 8 * q + 4 * h4);
+            v[4 * h4 + 0] = f.x;
+            v[4 * h4 + 1] = f.y;
+            v[4 * h4 + 2] = f.z;
+            v[4 * h4 + 3] = f.w;
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] *= sigmoid_exact(g[8 * q + e]);
+          store_eight<PIECES>(p.y + off + 8 * q, p.pairs * p.hd, v);
+        }
+      }
+    }
+  }
+};
+
+// out[b][o * s_o + t * s_i] = R(y Wo) (+ residual): the ending node lands transposed back
+template <int PIECES, int NM, int BN_>
+struct ProjOutPolicy {
+  static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr bool BF = PIECES == 1;
+  using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
+  struct Params {
+    long long pairs;
+    int n, c_z;
+    long long s_b, s_o, s_i;
+    const O* res;
+    O* out;
+    bool aligned;
+  };
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params&, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.b[0], dst, bar, BN / 64, n_tile * BN, k, piece);
+  }
+  static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<ProjOutPolicy>& acc, int quarter,
+                                  int col0, int col1, int lane) {
+    const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
+    const uint32_t bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
+    const long long off = b * p.s_b + o * p.s_o + t * p.s_i;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      const int c0 = n_tile * BN + col;
+      if (c0 >= p.c_z) break;
+      float v[16];
+      acc.load(0, col, v);
+      if (pair >= p.pairs) continue;
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (c0 + 8 * q < p.c_z)
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+    }
+  }
+};
+
+int ksteps(int k) { return (k + GEMM_BK - 1) / GEMM_BK; }
+
+// ------------------------------------------------------------------------- workspaces
 struct Offsets {
   size_t off = 0;
   size_t take(size_t bytes) {
@@ -372,215 +690,308 @@ struct Offsets {
   size_t total() const { return (off + 1023) / 1024 * 1024; }
 };
 
-int planes_for(int c_h) { return round_up(c_h, 128); }
-
 struct TrimulPlan {
-  size_t xn, p, g, ap, bp, t, tn, o, gate, params, total;
+  size_t xn, ap, bp, t, tn, w[4], total;
 };
 
-TrimulPlan trimul_plan(int n, int c_z, int c_h, bool f32) {
+TrimulPlan trimul_plan(int n, int batch, int c_z, int c_h, bool f32) {
   TrimulPlan pl;
   Offsets w;
-  const size_t pairs = static_cast<size_t>(n) * n, ld = round_up(n, 64), planes = planes_for(c_h);
-  const int pieces = f32 ? 3 : 1;
-  pl.xn = w.take(pairs * c_z * 4);
-  pl.p = w.take(pairs * 2 * c_h * 4);
-  pl.g = w.take(pairs * 2 * c_h * 4);
-  pl.ap = w.take(pieces * planes * n * ld * 2);
-  pl.bp = w.take(pieces * planes * n * ld * 2);
-  pl.t = w.take(planes * n * ld * 4);
-  pl.tn = w.take(pairs * c_h * 4);
-  pl.o = w.take(pairs * c_z * 4);
-  pl.gate = w.take(pairs * c_z * 4);
-  // float32 copies of the parameters of a bf16 trunk
-  pl.params = w.take((2 * static_cast<size_t>(c_z) + 2 * c_h + 2 * static_cast<size_t>(c_z) * 2 * c_h +
-                      static_cast<size_t>(c_h) * c_z + static_cast<size_t>(c_z) * c_z) * 4 + 8 * 1024);
+  const size_t pairs = static_cast<size_t>(batch) * n * n, ld = round_up(n, 64), pieces = f32 ? 3 : 1;
+  const size_t planes = static_cast<size_t>(batch) * c_h * n * ld;
+  pl.xn = w.take(pieces * pairs * c_z * 2);
+  pl.ap = w.take(pieces * planes * 2);
+  pl.bp = w.take(pieces * planes * 2);
+  pl.t = w.take(planes * (f32 ? 4 : 2));
+  pl.tn = w.take(pieces * pairs * c_h * 2);
+  pl.w[0] = w.take(pieces * c_z * 2 * c_h * 2);
+  pl.w[1] = w.take(pieces * c_z * 2 * c_h * 2);
+  pl.w[2] = w.take(pieces * c_h * c_z * 2);
+  pl.w[3] = w.take(pieces * c_z * c_z * 2);
   pl.total = w.total();
   return pl;
 }
 
 struct TriattPlan {
-  size_t xn, q, k, v, gate, o, bias, params, total;
+  size_t xn, q, k, vt, bias, mb, o, y, w[6], total;
 };
 
-TriattPlan triatt_plan(int n, int c_z, int heads, int head_dim) {
+TriattPlan triatt_plan(int n, int batch, int c_z, int heads, int head_dim, bool f32) {
   TriattPlan pl;
   Offsets w;
-  const size_t pairs = static_cast<size_t>(n) * n, hd = static_cast<size_t>(heads) * head_dim;
-  pl.xn = w.take(pairs * c_z * 4);
-  pl.q = w.take(pairs * hd * 4);
-  pl.k = w.take(pairs * hd * 4);
-  pl.v = w.take(pairs * hd * 4);
-  pl.gate = w.take(pairs * hd * 4);
-  pl.o = w.take(pairs * hd * 4);
-  pl.bias = w.take(pairs * heads * 4);
-  pl.params = w.take((2 * static_cast<size_t>(c_z) + static_cast<size_t>(c_z) * heads + 4 * c_z * hd + hd * c_z) * 4 +
-                     10 * 1024);
+  const size_t pairs = static_cast<size_t>(batch) * n * n, hd = static_cast<size_t>(heads) * head_dim;
+  const size_t ld = round_up(n, 64), pieces = f32 ? 3 : 1, rows = static_cast<size_t>(batch) * n;
+  pl.xn = w.take(pieces * pairs * c_z * 2);
+  pl.q = w.take(pieces * pairs * hd * 2);
+  pl.k = w.take(pieces * pairs * hd * 2);
+  pl.vt = w.take(pieces * rows * hd * ld * 2);
+  pl.bias = w.take(rows * heads * ld * (f32 ? 4 : 2));
+  pl.mb = w.take(rows * ld * 4);
+  pl.o = w.take(pairs * hd * (f32 ? 4 : 2));
+  pl.y = f32 ? w.take(pieces * pairs * hd * 2) : pl.o;
+  for (int i = 0; i < 6; ++i) pl.w[i] = w.take(pieces * c_z * (i == 3 ? static_cast<size_t>(round_up(heads, 8)) : hd) * 2);
   pl.total = w.total();
   return pl;
 }
 
-// A parameter as float32: the caller's array itself (float32 trunk), or a converted copy
-// carved from `scratch` (bf16 trunk).
-struct ParamStage {
-  uint8_t* scratch;
-  size_t off = 0;
+// Batch items one pass can take with the workspace the caller gave.
+template <class F>
+int items_per_pass(int batch, int n, size_t bytes, F total_of) {
+  int g = batch;
+  // (pair indices are 32-bit inside the kernels)
+  while (g > 1 && (total_of(g) > bytes || static_cast<long long>(g) * n * n > 4000000000ll)) --g;
+  return g;
+}
+
+// Weights of one op: read in place where TMA can, else listed for one weight_kernel launch.
+struct WeightStage {
   bool f32;
-  cudaStream_t stream;
-  int rc = B200TRI_OK;
-  const float* get(const void* p, size_t count) {
-    if (f32) return static_cast<const float*>(p);
-    off = (off + 255) / 256 * 256;
-    float* dst = reinterpret_cast<float*>(scratch + off);
-    off += count * 4;
-    count_launch();
-    to_f32_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(p), static_cast<long long>(count), dst);
-    if (cudaGetLastError() != cudaSuccess) rc = B200TRI_ERR_CUDA;
-    return dst;
+  WeightJobs jobs = {};
+  int count = 0;
+  int add(CUtensorMap* map, const void* w, int k, int n, uint8_t* scratch) {
+    const int ld = round_up(n, 8);
+    if (!f32 && n % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) return gemm_map_mnmajor(map, w, k, n, n);
+    jobs.job[count++] = {w, reinterpret_cast<__nv_bfloat16*>(scratch), k, n, ld};
+    return gemm_map_mnmajor(map, scratch, k, n, ld, f32 ? 3 : 1);
+  }
+  int run(cudaStream_t stream) {
+    if (!count) return B200TRI_OK;
+    const dim3 grid(64, static_cast<unsigned>(count));
+    return f32 ? launch(weight_kernel<false>, grid, dim3(256), 0, stream, true, jobs)
+               : launch(weight_kernel<true>, grid, dim3(256), 0, stream, true, jobs);
   }
 };
+
+bool aligned16(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
 
 template <bool BF>
 int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t stream) {
   using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
-  const int n = a->n;
-  const long long pairs = static_cast<long long>(n) * n;
-  const int ld = round_up(n, 64), planes = planes_for(c_h), pieces = BF ? 1 : 3;
-  const TrimulPlan pl = trimul_plan(n, c_z, c_h, !BF);
+  constexpr int P = BF ? 1 : 3;
+  const int n = a->n, batch = a->batch > 0 ? a->batch : 1;
+  const int group = items_per_pass(batch, n, a->workspace_bytes, [&](int g) { return trimul_plan(n, g, c_z, c_h, !BF).total; });
+  const TrimulPlan pl = trimul_plan(n, group, c_z, c_h, !BF);
   uint8_t* ws = static_cast<uint8_t*>(a->workspace);
-  float* xn = reinterpret_cast<float*>(ws + pl.xn);
-  float* p = reinterpret_cast<float*>(ws + pl.p);
-  float* g = reinterpret_cast<float*>(ws + pl.g);
-  __nv_bfloat16* ap = reinterpret_cast<__nv_bfloat16*>(ws + pl.ap);
-  __nv_bfloat16* bp = reinterpret_cast<__nv_bfloat16*>(ws + pl.bp);
-  float* t = reinterpret_cast<float*>(ws + pl.t);
-  float* tn = reinterpret_cast<float*>(ws + pl.tn);
-  float* o = reinterpret_cast<float*>(ws + pl.o);
-  float* gate = reinterpret_cast<float*>(ws + pl.gate);
-  ParamStage ps{ws + pl.params, 0, !BF, stream};
-  const float* ln_in_s = ps.get(a->norm_in_scale, c_z);
-  const float* ln_in_b = ps.get(a->norm_in_bias, c_z);
-  const float* p_in = ps.get(a->p_in, static_cast<size_t>(c_z) * 2 * c_h);
-  const float* g_in = ps.get(a->g_in, static_cast<size_t>(c_z) * 2 * c_h);
-  const float* ln_out_s = ps.get(a->norm_out_scale, c_h);
-  const float* ln_out_b = ps.get(a->norm_out_bias, c_h);
-  const float* p_out = ps.get(a->p_out, static_cast<size_t>(c_h) * c_z);
-  const float* g_out = ps.get(a->g_out, static_cast<size_t>(c_z) * c_z);
-  if (ps.rc) return ps.rc;
-  // projection frame (o, t): the outgoing update reads x[o][t], the incoming one x[t][o], so
-  // both contract over t (triangle.py:231, :239).
-  const long long xs_o = a->incoming ? c_z : static_cast<long long>(n) * c_z;
-  const long long xs_i = a->incoming ? static_cast<long long>(n) * c_z : c_z;
-  const long long ms_o = a->incoming ? 1 : n, ms_i = a->incoming ? n : 1;
-  count_launch();
-  ln_gather_kernel<BF, O><<<static_cast<unsigned>((pairs * 32 + 255) / 256), 256, 0, stream>>>(
-      static_cast<const O*>(a->x), xs_o, xs_i, n, n, c_z, ln_in_s, ln_in_b, a->eps, xn);
-  B200_CUDA_OK(cudaGetLastError());
+  auto at = [&](size_t off) { return reinterpret_cast<__nv_bfloat16*>(ws + off); };
+  GemmMaps glu = {}, fin = {};
+  WeightStage weights{!BF};
   int rc;
-  if ((rc = gemm<BF>(xn, p_in, pairs, c_z, 2 * c_h, p, stream))) return rc;
-  if ((rc = gemm<BF>(xn, g_in, pairs, c_z, 2 * c_h, g, stream))) return rc;
-  if (planes != c_h) {  // padding channel planes must read as zero
-    B200_CUDA_OK(cudaMemsetAsync(ap, 0, static_cast<size_t>(pieces) * planes * n * ld * 2, stream));
-    B200_CUDA_OK(cudaMemsetAsync(bp, 0, static_cast<size_t>(pieces) * planes * n * ld * 2, stream));
-  }
-  count_launch();
-  glu_split_kernel<BF><<<dim3(static_cast<unsigned>(ld / 32), static_cast<unsigned>(n)), 256, 0, stream>>>(
-      p, g, a->mask, ms_o, ms_i, n, n, ld, c_h, planes, pieces, ap, bp);
-  B200_CUDA_OK(cudaGetLastError());
-  // bf16 products with float32 accumulation carried from call to call (smallest terms first
-  // in float32 mode), 128 channel planes per call
-  const long long plane = static_cast<long long>(n) * ld, piece = static_cast<long long>(planes) * plane;
-  const int order3[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
-  const int n_terms = BF ? 1 : 6;
-  for (int c0 = 0; c0 < planes; c0 += 128) {
-    for (int s = 0; s < n_terms; ++s) {
-      const int pa = BF ? 0 : order3[s][0], pb = BF ? 0 : order3[s][1];
+  if ((rc = weights.add(&glu.a[0], a->p_in, c_z, 2 * c_h, ws + pl.w[0]))) return rc;
+  if ((rc = weights.add(&glu.a[1], a->g_in, c_z, 2 * c_h, ws + pl.w[1]))) return rc;
+  if ((rc = weights.add(&fin.b[0], a->p_out, c_h, c_z, ws + pl.w[2]))) return rc;
+  if ((rc = weights.add(&fin.b[1], a->g_out, c_z, c_z, ws + pl.w[3]))) return rc;
+  if ((rc = weights.run(stream))) return rc;
+  const int ld = round_up(n, 64);
+  const long long nn = static_cast<long long>(n) * n;
+  for (int b0 = 0; b0 < batch; b0 += group) {
+    const int nb = batch - b0 < group ? batch - b0 : group;
+    const long long pairs = nb * nn, plane = static_cast<long long>(n) * ld, piece = nb * c_h * plane;
+    const O* res = a->residual ? static_cast<const O*>(a->residual) + b0 * nn * c_z : nullptr;
+    O* out = static_cast<O*>(a->out) + b0 * nn * c_z;
+    const float* mask = a->mask ? a->mask + b0 * nn : nullptr;
+    // projection frame (o, t): the outgoing update reads x[o][t], the incoming one x[t][o], so
+    // both contract over t (triangle.py:231, :239)
+    LnArgs ln = {};
+    ln.x = static_cast<const O*>(a->x) + b0 * nn * c_z;
+    ln.xs_b = nn * c_z;
+    ln.xs_o = a->incoming ? c_z : static_cast<long long>(n) * c_z;
+    ln.xs_i = a->incoming ? static_cast<long long>(n) * c_z : c_z;
+    ln.batch = nb;
+    ln.n = n;
+    ln.c = c_z;
+    ln.scale = a->norm_in_scale;
+    ln.bias = a->norm_in_bias;
+    ln.eps = a->eps;
+    ln.xn = at(pl.xn);
+    if ((rc = launch_ln_gather<BF>(ln, stream, true))) return rc;
+    {
+      constexpr int BN = GluPolicy<P, 1>::BN;
+      if ((rc = map_rows(&glu.b[0], at(pl.xn), c_z, n, c_z, static_cast<long long>(n) * c_z, nb, P, pairs * c_z, BN))) return rc;
+      const int tiles_t = (n + BN - 1) / BN;
+      const GemmShape g = {(2 * c_h + GEMM_BM - 1) / GEMM_BM, nb * n * tiles_t, 1, {ksteps(c_z), ksteps(c_z)}, nullptr};
+      auto go = [&](auto policy) {
+        using Pol = decltype(policy);
+        return launch_piece_gemm<Pol>(glu, g, {n, tiles_t, c_h, ld, piece, mask, nn, a->incoming ? 1ll : n,
+                                               a->incoming ? n : 1ll, at(pl.ap), at(pl.bp)},
+                                      stream, true);
+      };
+      if constexpr (BF)
+        rc = go(GluPolicy<1, 1>{});
+      else  // (a longer K wants its leading term in more accumulators than double buffering leaves room for)
+        rc = c_z <= 128 ? go(GluPolicy<3, 1>{}) : go(GluPolicy<3, 3>{});
+      if (rc) return rc;
+    }
+    {
       b200tri_trimul_contract_args ca = {};
       ca.n_i = ca.n_j = ca.n_k = n;
       ca.n_src = 1;
-      ca.a = ap + pa * piece + c0 * plane;
-      ca.b = bp + pb * piece + c0 * plane;
+      ca.a = at(pl.ap);
+      ca.b = at(pl.bp);
       ca.a_ld = ca.b_ld = ca.out_ld = ld;
       ca.a_chan_stride = ca.b_chan_stride = ca.out_chan_stride = plane;
       ca.a_src_stride = ca.b_src_stride = piece;
-      ca.acc_in = s ? t + c0 * plane : nullptr;
-      ca.out_f32 = t + c0 * plane;
-      if ((rc = b200tri_trimul_contract(&ca, reinterpret_cast<b200tri_stream_t>(stream)))) return rc;
+      if (BF)
+        ca.out_bf16 = ws + pl.t;
+      else
+        ca.out_f32 = reinterpret_cast<float*>(ws + pl.t);
+      const ContractTerms terms = BF ? ContractTerms{} : ContractTerms{6, {2, 0, 1, 1, 0, 0}, {0, 2, 1, 0, 1, 0}};
+      if ((rc = contract_launch(&ca, nb * c_h, terms, stream))) return rc;
+    }
+    if ((rc = launch_ln_channel_major<BF>(ws + pl.t, n, nb, ld, c_h, a->norm_out_scale, a->norm_out_bias, a->eps, at(pl.tn),
+                                          stream)))
+      return rc;
+    {
+      // the gate's rows live in the projection frame: transposed for the incoming update
+      const long long r1 = a->incoming ? static_cast<long long>(n) * c_z : c_z, r2 = a->incoming ? c_z : static_cast<long long>(n) * c_z;
+      if ((rc = map_rows(&fin.a[0], at(pl.tn), c_h, n, c_h, static_cast<long long>(n) * c_h, nb, P, pairs * c_h, GEMM_BM))) return rc;
+      if ((rc = map_rows(&fin.a[1], at(pl.xn), c_z, n, r1, r2, nb, P, pairs * c_z, GEMM_BM))) return rc;
+      const int tiles_j = (n + GEMM_BM - 1) / GEMM_BM;
+      auto go = [&](auto policy) {
+        using Pol = decltype(policy);
+        const GemmShape g = {nb * n * tiles_j, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_h), ksteps(c_z)}, nullptr};
+        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res)}, stream, true);
+      };
+      if constexpr (BF)
+        rc = c_z <= 64 ? go(OutGatePolicy<1, 1, 64>{}) : go(OutGatePolicy<1, 1, 128>{});
+      else
+        rc = c_z <= 128 && c_h <= 128 ? go(OutGatePolicy<3, 1, 64>{}) : go(OutGatePolicy<3, 3, 64>{});
+      if (rc) return rc;
     }
   }
-  count_launch();
-  ln_channel_major_kernel<BF><<<static_cast<unsigned>((pairs * 32 + 255) / 256), 256, 0, stream>>>(
-      t, n, ld, c_h, ln_out_s, ln_out_b, a->eps, tn);
-  B200_CUDA_OK(cudaGetLastError());
-  if ((rc = gemm<BF>(tn, p_out, pairs, c_h, c_z, o, stream))) return rc;
-  if ((rc = gemm<BF>(xn, g_out, pairs, c_z, c_z, gate, stream))) return rc;
-  count_launch();
-  gate_out_kernel<BF, O><<<static_cast<unsigned>((pairs * c_z + 255) / 256), 256, 0, stream>>>(
-      o, gate, n, c_z, a->incoming ? 1 : 0, static_cast<const O*>(a->residual), static_cast<O*>(a->out));
-  B200_CUDA_OK(cudaGetLastError());
   return B200TRI_OK;
 }
 
 template <bool BF>
 int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
   using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
-  const int n = a->n, heads = a->heads, head_dim = a->head_dim, hd = heads * head_dim;
-  const long long pairs = static_cast<long long>(n) * n;
-  const TriattPlan pl = triatt_plan(n, c_z, heads, head_dim);
+  constexpr int P = BF ? 1 : 3;
+  const int n = a->n, heads = a->heads, head_dim = a->head_dim, hd = heads * head_dim, batch = a->batch > 0 ? a->batch : 1;
+  const int group =
+      items_per_pass(batch, n, a->workspace_bytes, [&](int g) { return triatt_plan(n, g, c_z, heads, head_dim, !BF).total; });
+  const TriattPlan pl = triatt_plan(n, group, c_z, heads, head_dim, !BF);
   uint8_t* ws = static_cast<uint8_t*>(a->workspace);
-  float* xn = reinterpret_cast<float*>(ws + pl.xn);
-  float* q = reinterpret_cast<float*>(ws + pl.q);
-  float* k = reinterpret_cast<float*>(ws + pl.k);
-  float* v = reinterpret_cast<float*>(ws + pl.v);
-  float* gate = reinterpret_cast<float*>(ws + pl.gate);
-  float* o = reinterpret_cast<float*>(ws + pl.o);
-  float* bias = reinterpret_cast<float*>(ws + pl.bias);
-  ParamStage ps{ws + pl.params, 0, !BF, stream};
-  const float* ln_s = ps.get(a->norm_scale, c_z);
-  const float* ln_b = ps.get(a->norm_bias, c_z);
-  const float* w_bias = ps.get(a->w_bias, static_cast<size_t>(c_z) * heads);
-  const float* w_q = ps.get(a->w_q, static_cast<size_t>(c_z) * hd);
-  const float* w_k = ps.get(a->w_k, static_cast<size_t>(c_z) * hd);
-  const float* w_v = ps.get(a->w_v, static_cast<size_t>(c_z) * hd);
-  const float* w_g = ps.get(a->w_g, static_cast<size_t>(c_z) * hd);
-  const float* w_o = ps.get(a->w_o, static_cast<size_t>(hd) * c_z);
-  if (ps.rc) return ps.rc;
+  auto at = [&](size_t off) { return reinterpret_cast<__nv_bfloat16*>(ws + off); };
+  GemmMaps proj = {}, gate = {}, outp = {};
+  WeightStage weights{!BF};
+  int rc;
+  if ((rc = weights.add(&proj.b[0], a->w_q, c_z, hd, ws + pl.w[0]))) return rc;
+  if ((rc = weights.add(&proj.b[1], a->w_k, c_z, hd, ws + pl.w[1]))) return rc;
+  if ((rc = weights.add(&proj.b[2], a->w_v, c_z, hd, ws + pl.w[2]))) return rc;
+  if ((rc = weights.add(&proj.b[3], a->w_bias, c_z, heads, ws + pl.w[3]))) return rc;
+  if ((rc = weights.add(&gate.b[0], a->w_g, c_z, hd, ws + pl.w[4]))) return rc;
+  if ((rc = weights.add(&outp.b[0], a->w_o, hd, c_z, ws + pl.w[5]))) return rc;
+  if ((rc = weights.run(stream))) return rc;
+  const int ld = round_up(n, 64);
+  const long long nn = static_cast<long long>(n) * n;
   // attention frame (o = row, t = position inside the row): the ending node is the starting
   // node on the transposed pair tensor and mask (triangle_attention.py:128-130, :160-161)
   const long long s_o = a->starting ? static_cast<long long>(n) * c_z : c_z;
   const long long s_i = a->starting ? c_z : static_cast<long long>(n) * c_z;
-  count_launch();
-  ln_gather_kernel<BF, O><<<static_cast<unsigned>((pairs * 32 + 255) / 256), 256, 0, stream>>>(
-      static_cast<const O*>(a->x), s_o, s_i, n, n, c_z, ln_s, ln_b, a->eps, xn);
-  B200_CUDA_OK(cudaGetLastError());
-  int rc;
-  if ((rc = gemm<BF>(xn, w_q, pairs, c_z, hd, q, stream))) return rc;
-  if ((rc = gemm<BF>(xn, w_k, pairs, c_z, hd, k, stream))) return rc;
-  if ((rc = gemm<BF>(xn, w_v, pairs, c_z, hd, v, stream))) return rc;
-  if ((rc = gemm<BF>(xn, w_g, pairs, c_z, hd, gate, stream))) return rc;
-  if ((rc = gemm<BF>(xn, w_bias, pairs, c_z, heads, bias, stream))) return rc;
-  rc = launch_att_core<BF>(head_dim, dim3(static_cast<unsigned>((n + AQ - 1) / AQ), static_cast<unsigned>(heads),
-                                          static_cast<unsigned>(n)),
-                           stream, q, k, v, bias, a->mask, a->starting ? n : 1, a->starting ? 1 : n, a->inf, n, heads, o);
-  if (rc) return rc;
-  count_launch();
-  mul_sigmoid_kernel<BF><<<static_cast<unsigned>((pairs * hd + 255) / 256), 256, 0, stream>>>(o, gate, pairs * hd);
-  B200_CUDA_OK(cudaGetLastError());
-  return gemm<BF, O>(o, w_o, pairs, hd, c_z, static_cast<O*>(a->out), stream, static_cast<const O*>(a->residual), n, s_o,
-                     s_i);
+  for (int b0 = 0; b0 < batch; b0 += group) {
+    const int nb = batch - b0 < group ? batch - b0 : group;
+    const long long pairs = nb * nn;
+    const O* res = a->residual ? static_cast<const O*>(a->residual) + b0 * nn * c_z : nullptr;
+    O* out = static_cast<O*>(a->out) + b0 * nn * c_z;
+    float* mb = reinterpret_cast<float*>(ws + pl.mb);
+    LnArgs ln = {};
+    ln.x = static_cast<const O*>(a->x) + b0 * nn * c_z;
+    ln.xs_b = nn * c_z;
+    ln.xs_o = s_o;
+    ln.xs_i = s_i;
+    ln.batch = nb;
+    ln.n = n;
+    ln.c = c_z;
+    ln.scale = a->norm_scale;
+    ln.bias = a->norm_bias;
+    ln.eps = a->eps;
+    ln.xn = at(pl.xn);
+    ln.mb = mb;
+    ln.mask = a->mask ? a->mask + b0 * nn : nullptr;
+    ln.ms_b = nn;
+    ln.ms_o = a->starting ? n : 1;
+    ln.ms_i = a->starting ? 1 : n;
+    ln.inf = a->inf;
+    ln.mb_ld = ld;
+    if ((rc = launch_ln_gather<BF>(ln, stream, true))) return rc;
+    const float root = sqrtf(static_cast<float>(head_dim));
+    const int m_tiles = static_cast<int>((pairs + GEMM_BM - 1) / GEMM_BM);
+    {
+      if ((rc = gemm_map_kmajor(&proj.a[0], at(pl.xn), P, pairs, c_z, c_z, GEMM_BM))) return rc;
+      auto go = [&](auto policy) {
+        using Pol = decltype(policy);
+        const int tiles_w = (hd + Pol::BN - 1) / Pol::BN;
+        const GemmShape g = {m_tiles, 3 * tiles_w + (heads + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
+        const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
+        return launch_piece_gemm<Pol>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, pairs * hd,
+                                                static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
+                                                ws + pl.bias},
+                                      stream, true);
+      };
+      if constexpr (BF)
+        rc = hd <= 64 ? go(QkvbPolicy<1, 1, 64>{}) : go(QkvbPolicy<1, 1, 128>{});
+      else
+        rc = go(QkvbPolicy<3, 3, 64>{});
+      if (rc) return rc;
+    }
+    {
+      AttSplitArgs s = {};
+      s.bf16 = BF;
+      s.batch = nb;
+      s.n_i = s.n = n;
+      s.heads = heads;
+      s.head_dim = head_dim;
+      s.q = at(pl.q);
+      s.k = at(pl.k);
+      s.vt = at(pl.vt);
+      s.v_ld = s.bias_ld = s.mask_ld = ld;
+      s.bias = ws + pl.bias;
+      s.mask_bias = mb;
+      s.scale = 1.0f;
+      s.o = ws + pl.o;
+      if ((rc = launch_att_split(s, stream))) return rc;
+    }
+    {
+      if ((rc = gemm_map_kmajor(&gate.a[0], at(pl.xn), P, pairs, c_z, c_z, GEMM_BM))) return rc;
+      auto go = [&](auto policy) {
+        using Pol = decltype(policy);
+        const GemmShape g = {m_tiles, (hd + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
+        return launch_piece_gemm<Pol>(gate, g, {pairs, hd, reinterpret_cast<const float*>(ws + pl.o), at(pl.y)}, stream, true);
+      };
+      if constexpr (BF)
+        rc = hd <= 64 ? go(GatePolicy<1, 1, 64>{}) : go(GatePolicy<1, 1, 128>{});
+      else
+        rc = go(GatePolicy<3, 3, 64>{});
+      if (rc) return rc;
+    }
+    {
+      if ((rc = gemm_map_kmajor(&outp.a[0], at(pl.y), P, pairs, hd, hd, GEMM_BM))) return rc;
+      auto go = [&](auto policy) {
+        using Pol = decltype(policy);
+        const GemmShape g = {m_tiles, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(hd), 0}, nullptr};
+        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res)}, stream, true);
+      };
+      if constexpr (BF)
+        rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{}) : go(ProjOutPolicy<1, 1, 128>{});
+      else
+        rc = go(ProjOutPolicy<3, 3, 64>{});
+      if (rc) return rc;
+    }
+  }
+  return B200TRI_OK;
 }
 
 }  // namespace
 
 size_t trimul_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t c_h, int32_t dtype) {
   if (n <= 0 || c_z <= 0 || c_h <= 0) return 0;
-  return trimul_plan(n, c_z, c_h, dtype == B200TRI_DTYPE_F32).total + 1024;
+  return trimul_plan(n, 1, c_z, c_h, dtype == B200TRI_DTYPE_F32).total;
 }
 
-size_t triatt_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t heads, int32_t head_dim) {
+size_t triatt_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t heads, int32_t head_dim, int32_t dtype) {
   if (n <= 0 || c_z <= 0 || heads <= 0 || head_dim <= 0) return 0;
-  return triatt_plan(n, c_z, heads, head_dim).total + 1024;
+  return triatt_plan(n, 1, c_z, heads, head_dim, dtype == B200TRI_DTYPE_F32).total;
 }
 
 int trimul_forward_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t stream) {
@@ -591,6 +1002,9 @@ int trimul_forward_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaS
 
 int triatt_forward_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
   B200_REQUIRE(a->n <= 65535, B200TRI_ERR_UNSUPPORTED, "triatt (general shapes): n up to 65535");
+  B200_REQUIRE(a->head_dim == 8 || a->head_dim == 16 || a->head_dim == 24 || a->head_dim == 32 || a->head_dim == 48 ||
+                   a->head_dim == 64,
+               B200TRI_ERR_UNSUPPORTED, "triatt: head widths 8, 16, 24, 32, 48 and 64 are built (got %d)", a->head_dim);
   return a->dtype == B200TRI_DTYPE_F32 ? triatt_generic<false>(a, c_z, stream) : triatt_generic<true>(a, c_z, stream);
 }
 

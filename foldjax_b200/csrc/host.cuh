@@ -121,6 +121,16 @@ int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stre
 // columns x `box_k` rows: MN-major operand tiles under the 128-byte swizzle.
 int make_weight_map(CUtensorMap* out, const void* w, int k, int n, int box_k);
 
+// A contraction over `channels` channel planes. `terms` (if any) replaces the sources by a list
+// of operand-plane pairs accumulated one after the other in the same float32 accumulator: the
+// piece products of split operands, smallest first, so that only the leading one is summed at
+// full magnitude.
+struct ContractTerms {
+  int n;
+  uint8_t a[8], b[8];
+};
+int contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms, cudaStream_t stream);
+
 // The mask-bias rows of the attention core, written by the projection stage of the same call.
 struct MaskBiasOut {
   const float* mask;  // null = all ones
@@ -136,7 +146,7 @@ int att_core_launch_premasked(const b200tri_triatt_core_args* a, cudaStream_t st
 // The two module-level ops for every shape / element type outside the tensor-core
 // specialisation (generic.cu): other channel and head counts, float32 trunks.
 size_t trimul_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t c_hidden, int32_t dtype);
-size_t triatt_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t heads, int32_t head_dim);
+size_t triatt_workspace_bytes_generic(int32_t n, int32_t c_z, int32_t heads, int32_t head_dim, int32_t dtype);
 int trimul_forward_generic(const b200tri_trimul_args* a, int c_z, int c_hidden, cudaStream_t stream);
 int triatt_forward_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream);
 

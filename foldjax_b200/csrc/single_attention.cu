@@ -210,24 +210,34 @@ __global__ void pad_weight_kernel(const __nv_bfloat16* __restrict__ src, int k, 
 // [q | k | v | g] in one launch: column tiles of 64 walk the four weights in turn.
 struct QkvgPolicy {
   static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
-  static constexpr bool B_MN = true;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = 8, CTAS = 1;
   struct Params {
     int rows, c, tiles_per_w, first_w;
     const __nv_bfloat16* q_bias;
     float* out[4];
   };
-  static __device__ int b_map(int, int n_tile, int, const Params& p) { return p.first_w + n_tile / p.tiles_per_w; }
-  static __device__ int b_col(int, int n_tile, int, const Params& p) { return n_tile % p.tiles_per_w * BN; }
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params& p, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.b[p.first_w + n_tile / p.tiles_per_w], dst, bar, 1, n_tile % p.tiles_per_w * BN, k, piece);
+  }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvgPolicy>& acc, int quarter,
-                                  int half, int lane) {
-    float r[32];
-    acc.load(0, half * 32, r);
+                                  int col0, int col1, int lane) {
     const int row = m_tile * GEMM_BM + quarter * 32 + lane;
-    const int which = p.first_w + n_tile / p.tiles_per_w, c0 = n_tile % p.tiles_per_w * BN + half * 32;
-    if (row >= p.rows) return;
+    const int which = p.first_w + n_tile / p.tiles_per_w;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+    float r[16];
+    acc.load(0, col, r);
+    if (row >= p.rows) continue;
+    const int c0 = n_tile % p.tiles_per_w * BN + col;
     float* dst = p.out[which] + static_cast<long long>(row) * p.c + c0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < 4; ++q) {
       float v[4];
       if (c0 + 4 * q >= p.c) break;  // c is a multiple of 8
 #pragma unroll
@@ -238,30 +248,42 @@ struct QkvgPolicy {
       }
       *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
     }
+    }
   }
 };
 
 // float32 partial sums, one plane per K split.
 struct PartialPolicy {
   static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
-  static constexpr bool B_MN = true;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = 8, CTAS = 1;
   struct Params {
     int rows, n;
     float* out;
   };
-  static __device__ int b_map(int, int, int, const Params&) { return 0; }
-  static __device__ int b_col(int, int n_tile, int, const Params&) { return n_tile * BN; }
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params&, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    gemm_load_mn(&maps.b[0], dst, bar, 1, n_tile * BN, k, piece);
+  }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int split, const Accum<PartialPolicy>& acc,
-                                  int quarter, int half, int lane) {
-    float r[32];
-    acc.load(0, half * 32, r);
-    const int row = m_tile * GEMM_BM + quarter * 32 + lane, c0 = n_tile * BN + half * 32;
-    if (row >= p.rows) return;
-    float* dst = p.out + (static_cast<long long>(split) * p.rows + row) * p.n + c0;
+                                  int quarter, int col0, int col1, int lane) {
+    const int row = m_tile * GEMM_BM + quarter * 32 + lane;
+#pragma unroll 1
+    for (int col = col0; col < col1; col += 16) {
+      float r[16];
+      acc.load(0, col, r);
+      if (row >= p.rows) continue;
+      const int c0 = n_tile * BN + col;
+      float* dst = p.out + (static_cast<long long>(split) * p.rows + row) * p.n + c0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (c0 + 4 * q < p.n)
-        *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+      for (int q = 0; q < 4; ++q)
+        if (c0 + 4 * q < p.n)
+          *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+    }
   }
 };
 
@@ -269,40 +291,51 @@ struct PartialPolicy {
 // (transition.py:108).
 struct SwigluPolicy {
   static constexpr int BN = 128, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
-  static constexpr bool B_MN = true;
+  static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
+  static constexpr int EPI = 8, CTAS = 1;
   struct Params {
     int rows, hidden;
     long long pitch;  // of a piece's rows
     __nv_bfloat16* h;
   };
-  static __device__ int b_map(int, int, int grp, const Params&) { return grp; }
-  static __device__ int b_col(int, int n_tile, int, const Params&) { return n_tile * 64; }
+  static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
+  }
+  static __device__ void load_b(const GemmMaps& maps, const Params&, int, int k, int n_tile, int piece, uint8_t* dst,
+                                uint64_t* bar) {
+    for (int w = 0; w < 2; ++w) gemm_load_mn(&maps.b[w], dst + w * 8192, bar, 1, n_tile * 64, k, piece);
+  }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<SwigluPolicy>& acc, int quarter,
-                                  int half, int lane) {
-    float a[32], b[32];
-    acc.load(0, half * 32, a);
-    acc.load(0, 64 + half * 32, b);
-    const int row = m_tile * GEMM_BM + quarter * 32 + lane, c0 = n_tile * 64 + half * 32;
-    if (row >= p.rows) return;
-    __nv_bfloat16* dst = p.h + static_cast<long long>(row) * p.pitch + c0;
+                                  int col0, int col1, int lane) {
+    const int row = m_tile * GEMM_BM + quarter * 32 + lane;
     const long long plane = static_cast<long long>(p.rows) * p.pitch;
+#pragma unroll 1
+    for (int col = col0 / 2; col < col1 / 2; col += 16) {  // this warp's share of the 64 hidden columns
+      float a[16], b[16];
+      acc.load(0, col, a);
+      acc.load(0, 64 + col, b);
+      if (row >= p.rows) continue;
+      const int c0 = n_tile * 64 + col;
+      __nv_bfloat16* dst = p.h + static_cast<long long>(row) * p.pitch + c0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (c0 + 8 * q >= p.pitch) break;  // the pitch is a multiple of 8; padding columns come out as zero
-      uint32_t hi[4], mid[4], lo[4];
+      for (int q = 0; q < 2; ++q) {
+        if (c0 + 8 * q >= p.pitch) break;  // the pitch is a multiple of 8; padding columns come out as zero
+        uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float v[2];
+        for (int e = 0; e < 4; ++e) {
+          float v[2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const float av = a[8 * q + 2 * e + u];
-          v[u] = av / (1.0f + expf(-av)) * b[8 * q + 2 * e + u];
+          for (int u = 0; u < 2; ++u) {
+            const float av = a[8 * q + 2 * e + u];
+            v[u] = av / (1.0f + expf(-av)) * b[8 * q + 2 * e + u];
+          }
+          split3x2(v[0], v[1], hi[e], mid[e], lo[e]);
         }
-        split3x2(v[0], v[1], hi[e], mid[e], lo[e]);
+        *reinterpret_cast<uint4*>(dst + 8 * q) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(dst + plane + 8 * q) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+        *reinterpret_cast<uint4*>(dst + 2 * plane + 8 * q) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
       }
-      *reinterpret_cast<uint4*>(dst + 8 * q) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(dst + plane + 8 * q) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-      *reinterpret_cast<uint4*>(dst + 2 * plane + 8 * q) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
   }
 };

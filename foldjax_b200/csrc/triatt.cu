@@ -51,7 +51,7 @@ extern "C" size_t b200tri_triatt_workspace_bytes_shape(int32_t n, int32_t dtype,
   c_z = c_z > 0 ? c_z : 128;
   if (dtype != B200TRI_DTYPE_BF16 && dtype != B200TRI_DTYPE_F32) return 0;
   if (specialised(dtype, c_z, heads, head_dim)) return b200tri_triatt_workspace_bytes(n);
-  return b200::triatt_workspace_bytes_generic(n, c_z, heads, head_dim);
+  return b200::triatt_workspace_bytes_generic(n, c_z, heads, head_dim, dtype);
 }
 
 extern "C" size_t b200tri_triatt_workspace_bytes_dtype(int32_t n, int32_t dtype) {
@@ -71,7 +71,7 @@ extern "C" int b200tri_triatt_forward(const b200tri_triatt_args* a, b200tri_stre
   B200_REQUIRE(c_z % 8 == 0 && c_z <= 1024, B200TRI_ERR_UNSUPPORTED,
                "triatt: c_z must be a multiple of 8 up to 1024 (got %d)", c_z);
   if (!specialised(a->dtype, c_z, a->heads, a->head_dim)) {
-    const size_t need = triatt_workspace_bytes_generic(a->n, c_z, a->heads, a->head_dim);
+    const size_t need = triatt_workspace_bytes_generic(a->n, c_z, a->heads, a->head_dim, a->dtype);
     B200_REQUIRE(a->workspace != nullptr && a->workspace_bytes >= need, B200TRI_ERR_WORKSPACE,
                  "triatt (general shapes): workspace of %zu bytes needed for n=%d, got %zu", need, a->n,
                  a->workspace_bytes);
@@ -80,6 +80,20 @@ extern "C" int b200tri_triatt_forward(const b200tri_triatt_args* a, b200tri_stre
     B200_REQUIRE(a->norm_scale && a->norm_bias && a->w_bias && a->w_q && a->w_k && a->w_v && a->w_g && a->w_o,
                  B200TRI_ERR_INVALID, "triatt: null parameter pointer");
     return triatt_forward_generic(a, c_z, reinterpret_cast<cudaStream_t>(stream));
+  }
+  if (a->batch > 1) {
+    b200tri_triatt_args one = *a;
+    one.batch = 1;
+    const size_t nn = static_cast<size_t>(a->n) * a->n;
+    for (int b = 0; b < a->batch; ++b) {
+      const int rc = b200tri_triatt_forward(&one, stream);
+      if (rc) return rc;
+      one.x = static_cast<const uint8_t*>(one.x) + nn * 256;
+      one.out = static_cast<uint8_t*>(one.out) + nn * 256;
+      if (one.mask) one.mask += nn;
+      if (one.residual) one.residual = static_cast<const uint8_t*>(one.residual) + nn * 256;
+    }
+    return B200TRI_OK;
   }
   const Plan pl = plan_offsets(a->n);
   B200_REQUIRE(a->workspace != nullptr && a->workspace_bytes >= pl.total, B200TRI_ERR_WORKSPACE,

@@ -88,6 +88,20 @@ extern "C" int b200tri_trimul_forward(const b200tri_trimul_args* a, b200tri_stre
                  B200TRI_ERR_INVALID, "trimul: null parameter pointer");
     return trimul_forward_generic(a, c_z, c_hidden, reinterpret_cast<cudaStream_t>(stream));
   }
+  if (a->batch > 1) {
+    b200tri_trimul_args one = *a;
+    one.batch = 1;
+    const size_t nn = static_cast<size_t>(a->n) * a->n;
+    for (int b = 0; b < a->batch; ++b) {
+      const int rc = b200tri_trimul_forward(&one, stream);
+      if (rc) return rc;
+      one.x = static_cast<const uint8_t*>(one.x) + nn * 256;
+      one.out = static_cast<uint8_t*>(one.out) + nn * 256;
+      if (one.mask) one.mask += nn;
+      if (one.residual) one.residual = static_cast<const uint8_t*>(one.residual) + nn * 256;
+    }
+    return B200TRI_OK;
+  }
   const Plan pl = plan_offsets(a->n);
   B200_REQUIRE(a->workspace != nullptr && a->workspace_bytes >= pl.total, B200TRI_ERR_WORKSPACE,
                "trimul: workspace of %zu bytes needed for n=%d, got %zu", pl.total, a->n, a->workspace_bytes);

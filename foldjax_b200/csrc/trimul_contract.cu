@@ -30,6 +30,7 @@ constexpr int THREADS = 192;
 
 struct ContractParams {
   int n_i, n_j, n_src;
+  ContractTerms terms;
   int kb_per_src;  // ceil(n_k / BK)
   int tiles_m, tiles_n;
   long long total_tiles;
@@ -98,8 +99,10 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             uint8_t* sa = smem + stage * STAGE_BYTES;
             mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
             // rows are (block, row in block): a tile starts at block row0 / rpb
-            tma_load_5d(sa, &tm_a, &full_bar[stage], kb * BK, (mi * BM) % p.a_rpb, (mi * BM) / p.a_rpb, d, s);
-            tma_load_5d(sa + A_BYTES, &tm_b, &full_bar[stage], kb * BK, (nj * BN) % p.b_rpb, (nj * BN) / p.b_rpb, d, s);
+            tma_load_5d(sa, &tm_a, &full_bar[stage], kb * BK, (mi * BM) % p.a_rpb, (mi * BM) / p.a_rpb, d,
+                        p.terms.n ? p.terms.a[s] : s);
+            tma_load_5d(sa + A_BYTES, &tm_b, &full_bar[stage], kb * BK, (nj * BN) % p.b_rpb, (nj * BN) / p.b_rpb, d,
+                        p.terms.n ? p.terms.b[s] : s);
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1;
@@ -235,7 +238,11 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 }  // namespace b200
 
 extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b200tri_stream_t stream) {
-  using namespace b200;
+  return b200::contract_launch(a, 128, b200::ContractTerms{}, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms,
+                          cudaStream_t stream) {
   B200_REQUIRE(a != nullptr, B200TRI_ERR_INVALID, "contract: null args");
   B200_REQUIRE(a->a && a->b, B200TRI_ERR_INVALID, "contract: null operand");
   B200_REQUIRE(a->out_f32 || a->out_bf16, B200TRI_ERR_INVALID, "contract: no output buffer");
@@ -276,21 +283,29 @@ extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b2
                B200TRI_ERR_INVALID, "contract: rows_per_block must divide or be a multiple of the tile rows (128 for a, 256 for b)");
   B200_REQUIRE(a->a_block_stride % 8 == 0 && a->b_block_stride % 8 == 0 && a->out_block_stride % 8 == 0,
                B200TRI_ERR_INVALID, "contract: block strides must be multiples of 8 elements");
+  int planes = a->n_src;  // planes of an operand: one per source, or one per piece
+  if (terms.n) {
+    planes = 1;
+    for (int t = 0; t < terms.n; ++t) {
+      planes = terms.a[t] >= planes ? terms.a[t] + 1 : planes;
+      planes = terms.b[t] >= planes ? terms.b[t] + 1 : planes;
+    }
+  }
   CUtensorMap tm_a, tm_b;
   {
-    const uint64_t dims[5] = {(uint64_t)a->n_k, (uint64_t)a_rows, a_blocks, 128, (uint64_t)a->n_src};
-    const uint64_t str[4] = {(uint64_t)a->a_ld * 2, (uint64_t)(a_blocks > 1 ? a->a_block_stride : a->a_chan_stride * 128) * 2,
+    const uint64_t dims[5] = {(uint64_t)a->n_k, (uint64_t)a_rows, a_blocks, (uint64_t)channels, (uint64_t)planes};
+    const uint64_t str[4] = {(uint64_t)a->a_ld * 2, (uint64_t)(a_blocks > 1 ? a->a_block_stride : a->a_chan_stride * channels) * 2,
                              (uint64_t)a->a_chan_stride * 2,
-                             (uint64_t)(a->n_src > 1 ? a->a_src_stride : a->a_chan_stride * 128) * 2};
+                             (uint64_t)(planes > 1 ? a->a_src_stride : a->a_chan_stride * channels) * 2};
     const uint32_t box[5] = {BK, a_box_r, a_box_b, 1, 1};
     int rc = make_tmap(&tm_a, a->a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box, Swz::B128);
     if (rc) return rc;
   }
   {
-    const uint64_t dims[5] = {(uint64_t)a->n_k, (uint64_t)b_rows, b_blocks, 128, (uint64_t)a->n_src};
-    const uint64_t str[4] = {(uint64_t)a->b_ld * 2, (uint64_t)(b_blocks > 1 ? a->b_block_stride : a->b_chan_stride * 128) * 2,
+    const uint64_t dims[5] = {(uint64_t)a->n_k, (uint64_t)b_rows, b_blocks, (uint64_t)channels, (uint64_t)planes};
+    const uint64_t str[4] = {(uint64_t)a->b_ld * 2, (uint64_t)(b_blocks > 1 ? a->b_block_stride : a->b_chan_stride * channels) * 2,
                              (uint64_t)a->b_chan_stride * 2,
-                             (uint64_t)(a->n_src > 1 ? a->b_src_stride : a->b_chan_stride * 128) * 2};
+                             (uint64_t)(planes > 1 ? a->b_src_stride : a->b_chan_stride * channels) * 2};
     const uint32_t box[5] = {BK, b_box_r, b_box_b, 1, 1};
     int rc = make_tmap(&tm_b, a->b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box, Swz::B128);
     if (rc) return rc;
@@ -298,11 +313,12 @@ extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b2
   ContractParams p;
   p.n_i = a->n_i;
   p.n_j = a->n_j;
-  p.n_src = a->n_src;
+  p.n_src = terms.n ? terms.n : a->n_src;
+  p.terms = terms;
   p.kb_per_src = (a->n_k + BK - 1) / BK;
   p.tiles_m = (a->n_i + BM - 1) / BM;
   p.tiles_n = (a->n_j + BN - 1) / BN;
-  p.total_tiles = 128ll * p.tiles_m * p.tiles_n;
+  p.total_tiles = static_cast<long long>(channels) * p.tiles_m * p.tiles_n;
   p.acc_in = a->acc_in;
   p.out_f32 = a->out_f32;
   p.out_bf16 = static_cast<__nv_bfloat16*>(a->out_bf16);
@@ -320,8 +336,8 @@ extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b2
   }
   const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
   {
-    TimedLaunch timed(K_TRIMUL_CONTRACT, reinterpret_cast<cudaStream_t>(stream));
-    return launch(contract_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES,
-                  reinterpret_cast<cudaStream_t>(stream), true, tm_a, tm_b, p);
+    TimedLaunch timed(K_TRIMUL_CONTRACT, stream);
+    return launch(contract_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, stream, true,
+                  tm_a, tm_b, p);
   }
 }

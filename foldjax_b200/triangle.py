@@ -141,16 +141,15 @@ def triangle_multiplication_forward(
     if c_hidden % 8 or c_hidden > 1024:
         raise ValueError(f"libb200tri takes hidden widths that are multiples of 8 up to 1024; got {c_hidden}")
     nbytes = lib.b200tri_trimul_workspace_bytes_shape(n, code, c_z, c_hidden)
+    if b > 1 and (code, c_z, c_hidden) != (_lib.DTYPE_BF16, C_Z, C_Z):
+        nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     ws = dev.workspace(nbytes, "trimul")
-    for bi in range(b):
-        args = _lib.TrimulArgs(
-            n=n, incoming=int(direction == "incoming"), eps=float(eps),
-            x=xd[bi].data_ptr(), mask=_ptr(md[bi]) if md is not None else None,
-            residual=_ptr(rd[bi]) if rd is not None else None, out=out[bi].data_ptr(),
-            workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes, dtype=code, c_z=c_z, c_hidden=c_hidden,
-            **{k: v.data_ptr() for k, v in leaves.items()},
-        )
-        _lib.check(lib.b200tri_trimul_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    args = _lib.TrimulArgs(
+        n=n, incoming=int(direction == "incoming"), eps=float(eps), x=xd.data_ptr(), mask=_ptr(md), residual=_ptr(rd),
+        out=out.data_ptr(), workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes, dtype=code, c_z=c_z, c_hidden=c_hidden,
+        batch=b, **{k: v.data_ptr() for k, v in leaves.items()},
+    )
+    _lib.check(lib.b200tri_trimul_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

@@ -99,16 +99,15 @@ def triangle_attention_forward(
     if heads * head_dim != width or head_dim not in (8, 16, 24, 32, 48, 64):
         raise ValueError(f"libb200tri takes head widths 8, 16, 24, 32, 48 and 64; got {heads} heads over {width} channels")
     nbytes = lib.b200tri_triatt_workspace_bytes_shape(n, code, c_z, heads, head_dim)
+    if b > 1 and (code, c_z, heads, head_dim) != (_lib.DTYPE_BF16, C_Z, HEADS, HEAD_DIM):
+        nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     ws = dev.workspace(nbytes, "triatt")
-    for bi in range(b):
-        args = _lib.TriattArgs(
-            n=n, starting=int(bool(starting)), heads=heads, head_dim=head_dim, inf=float(inf), eps=float(eps),
-            x=xd[bi].data_ptr(), mask=_ptr(md[bi]) if md is not None else None,
-            residual=_ptr(rd[bi]) if rd is not None else None, out=out[bi].data_ptr(),
-            workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes, dtype=code, c_z=c_z,
-            **{k: v.data_ptr() for k, v in leaves.items()},
-        )
-        _lib.check(lib.b200tri_triatt_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    args = _lib.TriattArgs(
+        n=n, starting=int(bool(starting)), heads=heads, head_dim=head_dim, inf=float(inf), eps=float(eps),
+        x=xd.data_ptr(), mask=_ptr(md), residual=_ptr(rd), out=out.data_ptr(), workspace=dev.aligned_ptr(ws),
+        workspace_bytes=nbytes, dtype=code, c_z=c_z, batch=b, **{k: v.data_ptr() for k, v in leaves.items()},
+    )
+    _lib.check(lib.b200tri_triatt_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

@@ -121,10 +121,14 @@ typedef struct {
                     parameter, of residual and of out. 0 = bf16. */
   /* Channel counts, 0 = 128: x is [n, n, c_z]; p_in / g_in [c_z, 2 * c_hidden]; norm_out
    * [c_hidden]; p_out [c_hidden, c_z]; g_out [c_z, c_z]. c_z = c_hidden = 128 in bf16 runs the
-   * tensor-core kernels end to end; any other shape (the template stacks' c_z = 64 with
-   * c_hidden = 128, the 384-channel refiner) or float32 runs the general path: CUDA-core
-   * stages around the tensor-core contraction. Multiples of 8, up to 1024. */
+   * fused kernels; any other shape (the template stacks' c_z = 64 with c_hidden = 128, the
+   * 384-channel refiner) or float32 runs the general path: unfused tensor-core products
+   * between layer-norm passes. Multiples of 8, up to 1024. */
   int32_t c_z, c_hidden;
+  /* Independent pair tensors x[batch][n, n, c_z] (mask, residual and out likewise, dense), 0 = 1.
+   * The general path takes as many items per launch as the workspace holds (the size functions
+   * give the bytes of one; a multiple holds more). */
+  int32_t batch;
 } b200tri_trimul_args;
 
 size_t b200tri_trimul_workspace_bytes(int32_t n); /* bf16, 128 channels */
@@ -259,6 +263,7 @@ typedef struct {
    * tensor-core kernels; other shapes (head widths 8, 16, 24, 32, 48, 64) or float32 run the
    * general CUDA-core path. */
   int32_t c_z;
+  int32_t batch; /* as in b200tri_trimul_args */
 } b200tri_triatt_args;
 
 size_t b200tri_triatt_workspace_bytes(int32_t n); /* bf16, c_z = 128, 4 heads x 32 */
