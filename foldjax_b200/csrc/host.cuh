@@ -141,7 +141,12 @@ struct MaskBiasOut {
 };
 int att_project_launch(const b200tri_triatt_project_args* a, const MaskBiasOut* mb, cudaStream_t stream);
 // The core with its mask-bias rows already in the workspace.
-int att_core_launch_premasked(const b200tri_triatt_core_args* a, cudaStream_t stream);
+// `strides` (null: q, k and o are [row][token][head][32]): where a token, a head and a row of q / o
+// (head_j, row_j) and of k (head_k, row_k) start, in elements and in multiples of 8.
+struct CoreStrides {
+  long long token, head_j, head_k, row_j, row_k;
+};
+int att_core_launch_premasked(const b200tri_triatt_core_args* a, const CoreStrides* strides, cudaStream_t stream);
 
 // The two module-level ops for every shape / element type outside the tensor-core
 // specialisation (generic.cu): other channel and head counts, float32 trunks.

@@ -158,7 +158,7 @@ extern "C" int b200tri_triatt_forward(const b200tri_triatt_args* a, b200tri_stre
   ca.o = ws + pl.off_o;
   ca.workspace = ws + pl.off_core;
   ca.workspace_bytes = b200tri_triatt_core_workspace_bytes(a->n, a->n);
-  rc = att_core_launch_premasked(&ca, reinterpret_cast<cudaStream_t>(stream));
+  rc = att_core_launch_premasked(&ca, nullptr, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
 
   b200tri_triatt_finish_args fa = {};

@@ -35,7 +35,15 @@
 // Bound: not the tensor pipe and not HBM. Per score the SM issues about 7 instructions (3-input
 // max, packed fma, ex2 or the cubic with its exponent insertion, clamp, half a cvt) against 128
 // tensor flops, and the MUFU unit delivers 16 exponentials per clock and SM: the kernel runs
-// at about 60 % of its issue slots with the tensor pipe under 40 % busy at head dim 32.
+// at about 60 % of its issue slots with the tensor pipe under 40 % busy at head dim 32. What a
+// step costs beyond that is registers: 64 scores per thread under the 128-register limit of 512
+// threads. So nothing that an item's end needs is kept across its steps (the position is worked
+// out again there, with 32-bit divisions) and its result is read back in halves; a warp, not a
+// thread, arrives on the barriers; the next item's queries are loaded while this one still runs.
+// Clocks per step of three rows at n = 256 / 512 / 1024 / 2048: 2970 / 2450 / 2130 / 2020 with
+// the position kept in registers, 2645 / 2315 / 2055 / 1960 so. Measured and not better: score
+// buffers in pairs, a ring of their own for K and the bias, four stages, 7 or 9 of 16 pairs on
+// the FMA pipe, results staged for a TMA store.
 #include <cuda_fp16.h>
 
 #include <mutex>
@@ -47,30 +55,11 @@ namespace b200 {
 
 namespace {
 
-#ifndef B200_NWG
-#define B200_NWG 3
-#endif
-#ifndef B200_TURNS
-#define B200_TURNS 0
-#endif
-// 1: the pair bias is added by the tensor core (S = bias . I + Q . K^T); 0: by the softmax threads.
-#ifndef B200_BIAS_MMA
-#define B200_BIAS_MMA 1
-#endif
-// Of every 16 pairs of exponentials, this many are evaluated on the FMA pipe.
-#ifndef B200_POLY
-#define B200_POLY 8
-#endif
-// 1: registers are moved from the control warpgroup to the softmax warpgroups at start-up.
-#ifndef B200_POLY_IMAD
-#define B200_POLY_IMAD 0
-#endif
-#ifndef B200_SETMAXNREG
-#define B200_SETMAXNREG 1
-#endif
-constexpr int NWG = B200_NWG;  // softmax warpgroups = rows i that share one bias tile
+constexpr int NWG = 3;  // softmax warpgroups = rows i that share one bias tile
 constexpr int KT = 64;
 constexpr int STAGES = 3;
+constexpr int POLY = 8;    // of every 16 pairs of exponentials, this many are evaluated on the FMA pipe
+constexpr int QBUF = 2;    // the next item's queries arrive while the last steps of this one run
 constexpr int THREADS = 128 + NWG * 128;  // warpgroup 0: producer, MMA issuer, 2 idle warps; then the softmax warpgroups
 constexpr int Q_BYTES = 128 * 64;    // [128 j][32 d] bf16
 constexpr int BIAS_BYTES = 128 * 128;  // [128 j][64 k] bf16
@@ -93,16 +82,13 @@ constexpr float EXP_MAGIC = 12582912.0f;  // 1.5 * 2^23: adding it leaves round(
 // (MASKED_SCORE and the rule itself: mask_bias() in tc.cuh)
 
 struct Smem {
-  uint8_t q[NWG][Q_BYTES];
+  uint8_t q[QBUF][NWG][Q_BYTES];
   uint8_t bias[STAGES][BIAS_BYTES];
-#if B200_BIAS_MMA
   uint8_t ident[KT * 128];  // 64 x 64 bf16 identity, K-major rows of 128 B under the 128-byte swizzle
-#endif
   uint8_t k[STAGES][NWG][K_BYTES];
   uint8_t v[STAGES][NWG][V_BYTES];
   float mb[STAGES][NWG][KT];
-  uint64_t q_full, q_empty, st_full[STAGES], st_empty[STAGES], s_full[NWG], s_free[NWG], p_full[NWG], pv_done[NWG];
-  uint64_t turn[NWG][4];  // whose exponentials run on each scheduler's MUFU unit
+  uint64_t q_full[QBUF], q_empty[QBUF], st_full[STAGES], st_empty[STAGES], s_full[NWG], s_free[NWG], p_full[NWG], pv_done[NWG];
   uint32_t tmem_base;
 };
 static_assert(sizeof(Smem) <= 232448, "shared memory budget");
@@ -120,8 +106,9 @@ struct Params {
   int steps_per_tile;
   int heads;
   int groups, tiles_j, steps;
-  long long total_items;
-  __nv_bfloat16* o;  // [n_i][n_j][128]
+  uint32_t total_items;
+  __nv_bfloat16* o;
+  long long o_token, o_head, o_row;  // strides of o in elements
   float* row_max;    // optional [n_i][heads][n_j]: offset m used (natural log units)
   float* row_sum;    // optional: sum of exp(S - m)
   float* acc_o;      // fp32 running numerator [n_i][n_j][128] (ring attention)
@@ -150,17 +137,8 @@ __device__ __forceinline__ float2 poly_exp2x2(float2 u, float2 log2e2, float2 ma
   float2 q = __ffma2_rn(make_float2(0.05286743f, 0.05286743f), f, make_float2(0.24215189f, 0.24215189f));
   q = __ffma2_rn(q, f, make_float2(0.69358677f, 0.69358677f));
   q = __ffma2_rn(q, f, make_float2(0.99996275f, 0.99996275f));
-#if B200_POLY_IMAD
-  // bits(q) + (bits(y) << 23) as one integer multiply-add per value (FMA pipe) instead of a
-  // shift and an add on the ALU pipe, which the maxima and clamps already load.
-  int rx, ry;
-  asm("mad.lo.s32 %0, %1, 8388608, %2;" : "=r"(rx) : "r"(__float_as_int(y.x)), "r"(__float_as_int(q.x)));
-  asm("mad.lo.s32 %0, %1, 8388608, %2;" : "=r"(ry) : "r"(__float_as_int(y.y)), "r"(__float_as_int(q.y)));
-  return make_float2(__int_as_float(rx), __int_as_float(ry));
-#else
   return make_float2(__int_as_float(__float_as_int(q.x) + (__float_as_int(y.x) << 23)),
                      __int_as_float(__float_as_int(q.y) + (__float_as_int(y.y) << 23)));
-#endif
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -179,18 +157,19 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm.v[0]);
     tma_prefetch_desc(&tm.b[0]);
     tma_prefetch_desc(&tm.m[0]);
-    mbar_init(&sm.q_full, 1);
-    mbar_init(&sm.q_empty, 1);
+    for (int b = 0; b < QBUF; ++b) {
+      mbar_init(&sm.q_full[b], 1);
+      mbar_init(&sm.q_empty[b], 1);
+    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.st_full[s], 1);
       mbar_init(&sm.st_empty[s], 1 + NWG * 4);
     }
     for (int g = 0; g < NWG; ++g) {
       mbar_init(&sm.s_full[g], 1);
-      mbar_init(&sm.s_free[g], 128);
-      mbar_init(&sm.p_full[g], 128);
+      mbar_init(&sm.s_free[g], 4);
+      mbar_init(&sm.p_full[g], 4);
       mbar_init(&sm.pv_done[g], 1);
-      for (int qr = 0; qr < 4; ++qr) mbar_init(&sm.turn[g][qr], 1);
     }
     fence_barrier_init();
   }
@@ -206,7 +185,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.v[0][0][0] + tile * V_BYTES + V_TMA_BYTES);
     dst[w] = (w < 32) ? 0x3C003C00u : 0u;  // fp16 1.0 pairs in row 32
   }
-#if B200_BIAS_MMA
   // The bias tile of a step is itself a K-major A operand ([128 queries][64 keys]); multiplied
   // by this identity it lands in the score accumulator exactly (bf16 x 1.0 in fp32), so the
   // softmax threads never touch the bias.
@@ -219,7 +197,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (e0 + 1 == row) val = 0x3F800000u;
     reinterpret_cast<uint32_t*>(sm.ident)[idx] = val;
   }
-#endif
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
@@ -227,30 +204,32 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   pdl_wait();
   pdl_trigger();
   const uint32_t tmem_base = sm.tmem_base;
-  const int items_per_head = p.groups * p.tiles_j;
+  // (32-bit divisions: 64-bit ones cost each role hundreds of cycles per item)
+  const uint32_t items_per_head = p.groups * p.tiles_j;
+  auto locate = [&](uint32_t item, int& h, int& i0, int& j0) {
+    const uint32_t head = item / items_per_head, rem = item - head * items_per_head, group = rem / p.tiles_j;
+    h = head;
+    i0 = group * NWG;
+    j0 = (rem - group * p.tiles_j) * 128;
+  };
 
-#if B200_SETMAXNREG
   // The control warpgroup needs few registers; the softmax warpgroups hold 64 scores per
   // thread and want more than the 128 an even split of the register file gives them.
-#endif
 
   if (warp < 4) {
-#if B200_SETMAXNREG
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-#endif
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0, item_it = 0;
       bool alive = true;
-      for (long long item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
-        const int h = static_cast<int>(item / items_per_head);
-        const int rem = static_cast<int>(item % items_per_head);
-        const int i0 = (rem / p.tiles_j) * NWG;
-        const int j0 = (rem % p.tiles_j) * 128;
-        if (!mbar_wait(&sm.q_empty, (item_it & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.q_full, NWG * Q_BYTES);
-        for (int g = 0; g < NWG; ++g) tma_load_3d(sm.q[g], &tm_q, &sm.q_full, h * 32, j0, i0 + g);
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+        int h, i0, j0;
+        locate(item, h, i0, j0);
+        const uint32_t qb = item_it % QBUF;
+        if (!mbar_wait(&sm.q_empty[qb], ((item_it / QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        mbar_expect_tx(&sm.q_full[qb], NWG * Q_BYTES);
+        for (int g = 0; g < NWG; ++g) tma_load_4d(sm.q[qb][g], &tm_q, &sm.q_full[qb], 0, h, j0, i0 + g);
         for (int t = 0; t < p.steps; ++t) {
           if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
             alive = false;
@@ -261,9 +240,9 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           mbar_expect_tx(&sm.st_full[stage], STAGE_TX);
           tma_load_3d(sm.bias[stage], &tm.b[tile], &sm.st_full[stage], k0, j0, h);
           for (int g = 0; g < NWG; ++g) {
-            tma_load_3d(sm.k[stage][g], &tm.k[tile], &sm.st_full[stage], h * 32, k0, i0 + g);
-            tma_load_3d(sm.v[stage][g], &tm.v[tile], &sm.st_full[stage], k0, h * 32, i0 + g);
+            tma_load_4d(sm.k[stage][g], &tm.k[tile], &sm.st_full[stage], 0, h, k0, i0 + g);
             tma_load_2d(sm.mb[stage][g], &tm.m[tile], &sm.st_full[stage], k0, i0 + g);
+            tma_load_3d(sm.v[stage][g], &tm.v[tile], &sm.st_full[stage], k0, h * 32, i0 + g);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -282,8 +261,9 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0, item_it = 0, g = 0;  // g: global step counter
       bool alive = true;
-      for (long long item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
-        if (!mbar_wait(&sm.q_full, item_it & 1, p.status, ST_TIMEOUT_MMA)) break;
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+        const uint32_t qb = item_it % QBUF;
+        if (!mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA)) break;
         for (int t = 0; t < p.steps && alive; ++t, ++g) {
           if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
             alive = false;
@@ -295,10 +275,9 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               break;
             }
             tc_fence_after();
-            const uint64_t adesc = desc_sw64(smem_u32(sm.q[wg]));
+            const uint64_t adesc = desc_sw64(smem_u32(sm.q[qb][wg]));
             const uint64_t bdesc = desc_sw64(smem_u32(sm.k[stage][wg]));
             const uint32_t d = tmem_base + wg * TM_WG + TM_S;
-#if B200_BIAS_MMA
             const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
             const uint64_t identdesc = desc_sw128(smem_u32(sm.ident));
 #pragma unroll
@@ -306,9 +285,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_qk,
                            kk != 0);
             umma_bf16_ss(d, adesc, bdesc, idesc_qk, 1);
-#else
-            umma_bf16_ss(d, adesc, bdesc, idesc_qk, 0);
-#endif
             umma_bf16_ss(d, umma_desc_advance(adesc, 32), umma_desc_advance(bdesc, 32), idesc_qk, 1);
             umma_commit(&sm.s_full[wg]);
           }
@@ -317,7 +293,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             phase ^= 1;
           }
         }
-        if (alive) umma_commit(&sm.q_empty);  // every Q.K^T of the item has been issued
+        if (alive) umma_commit(&sm.q_empty[qb]);  // every Q.K^T of the item has been issued
       }
     }
   } else if (warp == 2) {
@@ -327,7 +303,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0, g = 0;
       bool alive = true;
-      for (long long item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
+      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
         for (int t = 0; t < p.steps && alive; ++t, ++g) {
           // (already complete when P arrives; observed here so this thread's products
           // are ordered after the TMA writes of V)
@@ -360,9 +336,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   } else {
     // ------------------------------------------------------------- softmax
-#if B200_SETMAXNREG
     asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-#endif
     const int wg = (warp - 4) >> 2;
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;  // query inside the tile = TMEM lane
@@ -370,19 +344,19 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int stage = 0;
     uint32_t phase = 0, g = 0;
     bool alive = true;
-    for (long long item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
-      const int h = static_cast<int>(item / items_per_head);
-      const int rem = static_cast<int>(item % items_per_head);
-      const int i = (rem / p.tiles_j) * NWG + wg;
-      const int j = (rem % p.tiles_j) * 128 + row;
+    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
       // The softmax offset, kept in log2 units and integer-valued: exp(s - m) is evaluated as
       // 2^(s * log2e - m2). An integer m2 lets the polynomial path fold it into its range
       // reduction exactly and makes every rescale factor an exact power of two.
       float m2_used = -INFINITY;
-      const bool in_range = i < p.n_i && j < p.n_j;
-      const long long si = (static_cast<long long>(i) * p.heads + h) * p.n_j + j;
-      const long long oi = (static_cast<long long>(i) * p.n_j + j) * 128 + h * 32;
       if (p.resume) {
+        int h, i, j;
+        locate(item, h, i, j);
+        i += wg;
+        j += row;
+        const bool in_range = i < p.n_i && j < p.n_j;
+        const long long si = (static_cast<long long>(i) * p.heads + h) * p.n_j + j;
+        const long long oi = (static_cast<long long>(i) * p.n_j + j) * 128 + h * 32;
         // Continue the softmax of earlier key tiles: offset, denominator and fp32
         // numerator go back where the loop keeps them (registers and TMEM). The
         // previous item's O has been read out by this thread already, and the
@@ -423,7 +397,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // fp32 values per instruction (add/fma .f32x2), halving the softmax's ALU work.
         float2 u[KT / 2];
         {
-#if B200_BIAS_MMA
           // q.k + bias arrives from the tensor core; both halves are requested at once.
           uint32_t r0[32], r1[32];
           tmem_ld32(t_wg + TM_S, r0);
@@ -434,38 +407,9 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             u[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
             u[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
           }
-#else
-          // Two halves of 32 keys: the TMEM load of the second half and the bias
-          // fetches overlap the adds of the first, and at most one raw half is live.
-          const uint8_t* brow = sm.bias[stage];
-          uint32_t r[32];
-          uint4 b4[4];
-          tmem_ld32(t_wg + TM_S, r);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) b4[c] = *reinterpret_cast<const uint4*>(brow + sw128_offset(row, c));
-          tmem_ld_wait();
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const uint32_t w[4] = {b4[c].x, b4[c].y, b4[c].z, b4[c].w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int q = 4 * c + e;  // pair inside this half: keys 32*half + 2q, +1
-                u[16 * half + q] = __fadd2_rn(make_float2(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1])),
-                                              make_float2(bf16_lo(w[e]), bf16_hi(w[e])));
-              }
-            }
-            if (half == 0) {
-              tmem_ld32(t_wg + TM_S + 32, r);
-#pragma unroll
-              for (int c = 0; c < 4; ++c) b4[c] = *reinterpret_cast<const uint4*>(brow + sw128_offset(row, 4 + c));
-              tmem_ld_wait();
-            }
-          }
-#endif
           tc_fence_before();
-          mbar_arrive(&sm.s_free[wg]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.s_free[wg]);  // (an arrival per thread keeps the LSU busier)
         }
         const float* mrow = sm.mb[stage][wg];
         const bool masked = __any_sync(0xffffffffu, (mk0 != 0.f) || (mk1 != 0.f));
@@ -491,18 +435,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           break;
         }
         tc_fence_after();
-#if B200_TURNS
-        // The exponentials of one warp keep a scheduler's MUFU unit busy by themselves,
-        // while the rest of a step (loads, adds, maxima) needs issue slots but no MUFU.
-        // Left alone, the three warps of a scheduler drift into the same phase and the
-        // two resources are used one after the other. So the exponent phase is taken in
-        // turns: warpgroup w runs it after warpgroup w - 1 (warpgroup 0 after the last
-        // one's previous step), and the others' load/add/max work fills the issue slots.
-        if (!mbar_wait(&sm.turn[wg][quarter], wg == 0 ? ((g & 1) ^ 1) : (g & 1), p.status, ST_TIMEOUT_SOFTMAX)) {
-          alive = false;
-          break;
-        }
-#endif
         // four independent chains, so the reduction is not one 32-deep dependency
         float mxa = fmaxf(u[0].x, u[0].y), mxb = fmaxf(u[1].x, u[1].y);
         float mxc = fmaxf(u[2].x, u[2].y), mxd = fmaxf(u[3].x, u[3].y);
@@ -526,7 +458,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const bool any_need = __any_sync(0xffffffffu, need);
         // exp(u - m) = 2^(u * log2e - m2): one fma per pair feeds the MUFU unit (|m2| < 2^17, so
         // the sum is exact to the last bit of the product and cancels exactly for the keys that
-        // equal the offset). B200_POLY of every 16 pairs take the polynomial path instead: the
+        // equal the offset). POLY of every 16 pairs take the polynomial path instead: the
         // MUFU unit delivers 16 results per clock and SM and would otherwise be the one pipe
         // every exponential queues for, while the FMA pipe idles.
         // P goes to TMEM in two halves of 32 keys to keep the live registers down.
@@ -542,7 +474,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int e = 0; e < 16; ++e) {
               const float2 ue = u[16 * half + e];
               float2 ex;
-              if (((e + 1) * B200_POLY) / 16 != (e * B200_POLY) / 16) {  // spread evenly over the half
+              if (((e + 1) * POLY) / 16 != (e * POLY) / 16) {  // spread evenly over the half
                 ex = poly_exp2x2(make_float2(fmaxf(ue.x, u_min), fmaxf(ue.y, u_min)), log2e2, mm2);
               } else {
                 const float2 t2 = __ffma2_rn(ue, log2e2, nm2);
@@ -556,10 +488,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             tmem_st16(t_wg + TM_P + 16 * half, packed);
           }
         }
-#if B200_TURNS
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.turn[(wg + 1) % NWG][quarter]);
-#endif
         if ((t > 0 || p.resume) && any_need) {
           uint32_t o[32];
           tmem_ld32(t_wg + TM_O, o);
@@ -576,7 +504,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         tmem_st_wait();
         tc_fence_before();
-        mbar_arrive(&sm.p_full[wg]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.p_full[wg]);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;
@@ -586,36 +515,46 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // ---- item epilogue: O / l -> bf16 -> o[i][j][h*32 ..]
       if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) break;
       tc_fence_after();
-      uint32_t o[32], lcol[16];
-      tmem_ld32(t_wg + TM_O, o);
+      int h, i, j;
+      locate(item, h, i, j);
+      i += wg;
+      j += row;
+      const bool in_range = i < p.n_i && j < p.n_j;
+      uint32_t lcol[16];
       tmem_ld16(t_wg + TM_L, lcol);
       tmem_ld_wait();
-      tc_fence_before();
       const float l = __uint_as_float(lcol[0]);  // sum_k exp(S - m), accumulated by the P.V products
-      if (in_range) {
-        if (p.normalize) {
-          const float inv = __fdividef(1.0f, l);
-          uint4* dst = reinterpret_cast<uint4*>(p.o + oi);
+      const float inv = __fdividef(1.0f, l);
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
+      for (int part = 0; part < 2; ++part) {
+        uint32_t o[16];
+        tmem_ld16(t_wg + TM_O + part * 16, o);
+        tmem_ld_wait();
+        if (p.normalize) {
+          uint4* dst = reinterpret_cast<uint4*>(p.o + i * p.o_row + h * p.o_head + j * p.o_token + part * 16);
+#pragma unroll
+          for (int q4 = 0; q4 < 2; ++q4) {
             uint32_t w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               w[e] = pack_bf16x2(__uint_as_float(o[8 * q4 + 2 * e]) * inv, __uint_as_float(o[8 * q4 + 2 * e + 1]) * inv);
-            dst[q4] = make_uint4(w[0], w[1], w[2], w[3]);
+            if (in_range) dst[q4] = make_uint4(w[0], w[1], w[2], w[3]);
           }
-        } else {
-          float4* dst = reinterpret_cast<float4*>(p.acc_o + oi);
+        } else if (in_range) {
+          float4* dst = reinterpret_cast<float4*>(p.acc_o + (static_cast<long long>(i) * p.n_j + j) * 128 + h * 32 + part * 16);
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
-            dst[q4] = make_float4(__uint_as_float(o[4 * q4]), __uint_as_float(o[4 * q4 + 1]),
-                                  __uint_as_float(o[4 * q4 + 2]), __uint_as_float(o[4 * q4 + 3]));
-        }
-        if (p.row_max) {
-          p.row_max[si] = m2_used * LN2;  // natural-log units
-          p.row_sum[si] = l;
+          for (int q4 = 0; q4 < 4; ++q4)
+            dst[q4] = make_float4(__uint_as_float(o[4 * q4]), __uint_as_float(o[4 * q4 + 1]), __uint_as_float(o[4 * q4 + 2]),
+                                  __uint_as_float(o[4 * q4 + 3]));
         }
       }
+      if (in_range && p.row_max) {
+        const long long si = (static_cast<long long>(i) * p.heads + h) * p.n_j + j;
+        p.row_max[si] = m2_used * LN2;  // natural-log units
+        p.row_sum[si] = l;
+      }
+      __syncwarp();
+      tc_fence_before();
     }
   }
 
@@ -660,15 +599,15 @@ namespace {
 // `may_time` = false keeps the launch free of event creation whatever the timing switch
 // says at that moment (the allocation-free entry point relies on it).
 int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time,
-                bool premasked = false);
+                bool premasked = false, const b200::CoreStrides* strides = nullptr);
 }  // namespace
 
 extern "C" int b200tri_triatt_core(const b200tri_triatt_core_args* a, b200tri_stream_t stream) {
   return core_launch(a, 1, stream, true);
 }
 
-int b200::att_core_launch_premasked(const b200tri_triatt_core_args* a, cudaStream_t stream) {
-  return core_launch(a, 1, reinterpret_cast<b200tri_stream_t>(stream), true, true);
+int b200::att_core_launch_premasked(const b200tri_triatt_core_args* a, const CoreStrides* strides, cudaStream_t stream) {
+  return core_launch(a, 1, reinterpret_cast<b200tri_stream_t>(stream), true, true, strides);
 }
 
 extern "C" int b200tri_triatt_core_multi(const b200tri_triatt_core_args* tiles, int32_t n_tiles,
@@ -678,7 +617,7 @@ extern "C" int b200tri_triatt_core_multi(const b200tri_triatt_core_args* tiles, 
 
 namespace {
 int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stream_t stream_, bool may_time,
-                bool premasked) {
+                bool premasked, const b200::CoreStrides* strides) {
   using namespace b200;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   B200_REQUIRE(tiles != nullptr, B200TRI_ERR_INVALID, "att core: null args");
@@ -704,6 +643,8 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   B200_REQUIRE(status != nullptr, B200TRI_ERR_CUDA, "att core: no current CUDA device");
 
   const int ldm = round_up(a->n_k, 64);
+  // q, k and o: [row][token][head][32] unless the caller says otherwise
+  const CoreStrides st = strides ? *strides : CoreStrides{128, 32, 32, 128ll * a->n_j, 128ll * a->n_k};
   TileMaps tm;
   for (int t = 0; t < n_tiles; ++t) {
     const b200tri_triatt_core_args* ti = tiles + t;
@@ -721,10 +662,10 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
       B200_CUDA_OK(cudaGetLastError());
     }
     {
-      const uint64_t dims[3] = {128, (uint64_t)a->n_k, (uint64_t)a->n_i};
-      const uint64_t str[2] = {256, (uint64_t)a->n_k * 256};
-      const uint32_t box[3] = {32, KT, 1};
-      int rc = make_tmap(&tm.k[t], ti->k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B64);
+      const uint64_t dims[4] = {32, 4, (uint64_t)a->n_k, (uint64_t)a->n_i};
+      const uint64_t str[3] = {(uint64_t)st.head_k * 2, (uint64_t)st.token * 2, (uint64_t)st.row_k * 2};
+      const uint32_t box[4] = {32, 1, KT, 1};
+      int rc = make_tmap(&tm.k[t], ti->k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B64);
       if (rc) return rc;
     }
     {
@@ -757,10 +698,10 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   }
   CUtensorMap tm_q;
   {
-    const uint64_t dims[3] = {128, (uint64_t)a->n_j, (uint64_t)a->n_i};
-    const uint64_t str[2] = {256, (uint64_t)a->n_j * 256};
-    const uint32_t box[3] = {32, 128, 1};
-    int rc = make_tmap(&tm_q, a->q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B64);
+    const uint64_t dims[4] = {32, 4, (uint64_t)a->n_j, (uint64_t)a->n_i};
+    const uint64_t str[3] = {(uint64_t)st.head_j * 2, (uint64_t)st.token * 2, (uint64_t)st.row_j * 2};
+    const uint32_t box[4] = {32, 1, 128, 1};
+    int rc = make_tmap(&tm_q, a->q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B64);
     if (rc) return rc;
   }
   Params p;
@@ -772,7 +713,12 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   p.tiles_j = (a->n_j + 127) / 128;
   p.steps_per_tile = (a->n_k + KT - 1) / KT;
   p.steps = p.steps_per_tile * n_tiles;
-  p.total_items = static_cast<long long>(a->heads) * p.groups * p.tiles_j;
+  const long long items = static_cast<long long>(a->heads) * p.groups * p.tiles_j;
+  B200_REQUIRE(items < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "att core: too many rows times queries for one launch");
+  p.total_items = static_cast<uint32_t>(items);
+  p.o_token = st.token;
+  p.o_head = st.head_j;
+  p.o_row = st.row_j;
   p.o = static_cast<__nv_bfloat16*>(a->o);
   p.row_max = a->row_max;
   p.row_sum = a->row_sum;
@@ -785,7 +731,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_core_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_items < sm_count() ? p.total_items : sm_count();
+  const long long grid = items < sm_count() ? items : sm_count();
   {
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
     return launch(att_core_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tm, p);
