@@ -15,13 +15,22 @@ import torch
 _workspaces: dict[tuple[int, str], torch.Tensor] = {}
 
 
+_cuda_seen = False
+
+
 def require_cuda() -> None:
+    global _cuda_seen
+    if _cuda_seen:  # asking the driver again costs a small call microseconds
+        return
     if not torch.cuda.is_available():
         raise RuntimeError("foldjax_b200 needs a CUDA device (B200, sm_100a); there is no CPU fallback")
+    torch.cuda.init()
+    _cuda_seen = True
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device as a raw handle (no Stream object is built)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def workspace(nbytes: int, tag: str = "default") -> torch.Tensor:
@@ -29,7 +38,7 @@ def workspace(nbytes: int, tag: str = "default") -> torch.Tensor:
     dev = torch.cuda.current_device()
     key = (dev, tag)
     buf = _workspaces.get(key)
-    if buf is None or buf.numel() < int(nbytes) + 1024:  # callers round the pointer up by up to 1023 B
+    if buf is None or buf.numel() < nbytes + 1024:  # callers round the pointer up by up to 1023 B
         _workspaces.pop(key, None)
         buf = torch.empty(int(nbytes) + 1024, dtype=torch.uint8, device=f"cuda:{dev}")
         _workspaces[key] = buf
@@ -58,7 +67,7 @@ def check_out(out: torch.Tensor, like: torch.Tensor, name: str = "out") -> torch
         raise ValueError(f"{name} must be a torch tensor, got {type(out).__name__}")
     if out.dtype != like.dtype:
         raise ValueError(f"{name} must be {like.dtype}, got {out.dtype}")
-    if tuple(out.shape) != tuple(like.shape):
+    if out.shape != like.shape:
         raise ValueError(f"{name} shape {tuple(out.shape)} does not match the input {tuple(like.shape)}")
     if not out.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
@@ -68,7 +77,7 @@ def check_out(out: torch.Tensor, like: torch.Tensor, name: str = "out") -> torch
 
 
 def check_same_shape(t: torch.Tensor, like: torch.Tensor, name: str) -> torch.Tensor:
-    if tuple(t.shape) != tuple(like.shape):
+    if t.shape != like.shape:
         raise ValueError(f"{name} shape {tuple(t.shape)} does not match the input {tuple(like.shape)}")
     return t
 
@@ -85,8 +94,17 @@ def release_workspaces() -> None:
     _workspaces.clear()
 
 
+def ready(x: Any, dtype: torch.dtype | None) -> bool:
+    """Whether the kernels can read ``x`` as it is: a contiguous tensor of ``dtype`` on the current
+    device. Most calls bring nothing else, and a ``.to()`` that copies nothing is not free."""
+    return (isinstance(x, torch.Tensor) and x.is_cuda and (dtype is None or x.dtype is dtype) and x.is_contiguous()
+            and x.get_device() == torch._C._cuda_getDevice())
+
+
 def to_device(x: Any, dtype: torch.dtype | None = None, device: torch.device | None = None) -> torch.Tensor:
     """numpy / torch (any device) -> contiguous CUDA tensor of `dtype`."""
+    if device is None and ready(x, dtype):
+        return x
     device = device or torch.device("cuda", torch.cuda.current_device())
     if isinstance(x, np.ndarray):
         if x.dtype.name == "bfloat16":  # ml_dtypes

@@ -69,7 +69,7 @@ def attention_pair_bias_forward(
     if c_s != heads * HEAD_DIM or tuple(lv["proj_q"].shape) != (c_s, c_s) or tuple(lv["proj_z"].shape) != (C_Z, heads):
         raise ValueError(f"libb200tri is built for heads of width {HEAD_DIM} and c_z = {C_Z}; got c_s {c_s}, {heads} heads")
     out = torch.empty_like(sd)
-    nbytes = lib.b200tri_attention_pair_bias_workspace_bytes(n, c_s, heads)
+    nbytes = _lib.workspace_bytes("b200tri_attention_pair_bias_workspace_bytes", n, c_s, heads)
     ws = dev.workspace(nbytes, "attention_pair_bias")
     for bi in range(b):
         args = _lib.AttentionPairBiasArgs(
@@ -78,7 +78,7 @@ def attention_pair_bias_forward(
             out=out[bi].data_ptr(), workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes,
             **{k: v.data_ptr() for k, v in lv.items()},
         )
-        _lib.check(lib.b200tri_attention_pair_bias(C.byref(args), C.c_void_p(dev.stream_ptr())))
+        _lib.check(lib.b200tri_attention_pair_bias(C.byref(args), dev.stream_ptr()))
     if host_in:
         host = out.cpu()
         return host.numpy() if numpy_in else host

@@ -14,6 +14,7 @@ the whole stack in one call.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Any, Mapping, Sequence
 
 import numpy as np
@@ -21,7 +22,7 @@ import torch
 
 from . import _device as dev
 from . import _lib
-from .triangle import C_Z
+from .triangle import C_Z, _leaf
 
 _TRIMUL = {"norm_in_scale": ("norm_in", "scale"), "norm_in_bias": ("norm_in", "bias"), "p_in": ("p_in", "kernel"),
            "g_in": ("g_in", "kernel"), "norm_out_scale": ("norm_out", "scale"), "norm_out_bias": ("norm_out", "bias"),
@@ -38,10 +39,17 @@ _ATT = {"proj_q": ("proj_q", "kernel"), "proj_q_bias": ("proj_q", "bias"), "proj
         "proj_z": ("proj_z", "kernel"), "proj_o": ("proj_o", "kernel")}
 
 
-def _get(node: Any, path: tuple[str, ...]) -> Any:
-    for key in path:
-        node = node[key]
-    return node
+# every parameter in the order of PairformerBlockParams' fields
+_PAIR_LEAVES = ([("tri_mul_out", *p) for p in _TRIMUL.values()] + [("tri_mul_in", *p) for p in _TRIMUL.values()]
+                + [("tri_att_start", *p) for p in _TRIATT.values()] + [("tri_att_end", *p) for p in _TRIATT.values()]
+                + [("transition_z", *p) for p in _TRANS.values()])
+_SINGLE_LEAVES = ([("pre_norm_s", "scale"), ("pre_norm_s", "bias")] + [("attention", *p) for p in _ATT.values()]
+                  + [("transition_s", *p) for p in _TRANS.values()])
+_FC1_Z, _PROJ_Z, _FC1_S = (leaves.index(path) for leaves, path in (
+    (_PAIR_LEAVES, ("transition_z", "fc1", "kernel")), (_SINGLE_LEAVES, ("attention", "proj_z", "kernel")),
+    (_SINGLE_LEAVES, ("transition_s", "fc1", "kernel"))))
+# pointers, the transition's hidden width, pointers, the single transition's hidden width
+_BLOCK_LAYOUT = struct.Struct(f"@{len(_PAIR_LEAVES)}Pi{len(_SINGLE_LEAVES)}Pi4x")
 
 
 class _Packed:
@@ -49,33 +57,19 @@ class _Packed:
 
     def __init__(self, params: Mapping[str, Any], single: bool):
         self.keep: list[torch.Tensor] = []
-        self.struct = _lib.PairformerBlockParams()
-
-        def ptr(node: Any) -> int:
-            t = node if isinstance(node, torch.Tensor) and node.is_cuda and node.dtype == torch.bfloat16 else \
-                dev.to_device(node, torch.bfloat16)
-            t = t.contiguous()
-            self.keep.append(t)
-            return t.data_ptr()
-
-        def fill(dst, table, src):
-            for field_name, path in table.items():
-                setattr(dst, field_name, ptr(_get(src, path)))
-
-        fill(self.struct.tri_mul_out, _TRIMUL, params["tri_mul_out"])
-        fill(self.struct.tri_mul_in, _TRIMUL, params["tri_mul_in"])
-        fill(self.struct.tri_att_start, _TRIATT, params["tri_att_start"])
-        fill(self.struct.tri_att_end, _TRIATT, params["tri_att_end"])
-        fill(self.struct.transition_z, _TRANS, params["transition_z"])
-        self.struct.transition_z.hidden = int(np.shape(_get(params["transition_z"], ("fc1", "kernel")))[-1])
-        self.heads_s = 0
+        pair = self._leaves(params, _PAIR_LEAVES)
+        self.hidden_z, self.hidden_s, self.heads_s = pair[_FC1_Z].shape[-1], 0, 0
+        pointers = [0] * len(_SINGLE_LEAVES)
         if single:
-            self.struct.pre_norm_s_scale = ptr(params["pre_norm_s"]["scale"])
-            self.struct.pre_norm_s_bias = ptr(params["pre_norm_s"]["bias"])
-            fill(self.struct.attention, _ATT, params["attention"])
-            fill(self.struct.transition_s, _TRANS, params["transition_s"])
-            self.struct.transition_s.hidden = int(np.shape(_get(params["transition_s"], ("fc1", "kernel")))[-1])
-            self.heads_s = int(np.shape(_get(params["attention"], ("proj_z", "kernel")))[-1])
+            leaves = self._leaves(params, _SINGLE_LEAVES)
+            pointers = [t.data_ptr() for t in leaves]
+            self.heads_s, self.hidden_s = leaves[_PROJ_Z].shape[-1], leaves[_FC1_S].shape[-1]
+        self.struct = _BLOCK_LAYOUT.pack(*[t.data_ptr() for t in pair], self.hidden_z, *pointers, self.hidden_s)
+
+    def _leaves(self, params: Mapping[str, Any], paths: Sequence[tuple[str, ...]]) -> list[torch.Tensor]:
+        found = [_leaf(params, *path) for path in paths]
+        self.keep += found
+        return found
 
 
 #: what distinguishes the block of each model family at the level of this driver
@@ -138,19 +132,19 @@ def pairformer_forward(
     if single:
         sd = dev.to_device(s, torch.float32)
         sd = sd.unsqueeze(0) if sd.dim() == 2 else sd
-        if sd.dim() != 3 or tuple(sd.shape[:2]) != (b, n):
+        if sd.dim() != 3 or sd.shape[:2] != (b, n):
             raise ValueError(f"s shape {tuple(sd.shape)} does not match the pair tensor {tuple(zd.shape)}")
     pmd = None
     if pair_mask is not None:
         pmd = dev.to_device(pair_mask, torch.float32)
         pmd = pmd.unsqueeze(0) if pmd.dim() == 2 else pmd
-        if tuple(pmd.shape) != (b, n, n):
+        if pmd.shape != (b, n, n):
             raise ValueError(f"pair_mask shape {tuple(pmd.shape)} does not match the pair tensor {tuple(zd.shape)}")
     md = None
     if mask is not None:
         md = dev.to_device(mask, torch.float32)
         md = md.unsqueeze(0) if md.dim() == 1 else md
-        if tuple(md.shape) != (b, n):
+        if md.shape != (b, n):
             raise ValueError(f"mask shape {tuple(md.shape)} does not match the pair tensor {tuple(zd.shape)}")
     if gate and md is None and pmd is not None and single:
         md = torch.diagonal(pmd, dim1=-2, dim2=-1).contiguous()  # single_valid = diag(pair_valid)
@@ -162,14 +156,12 @@ def pairformer_forward(
         packed = [_Packed(p, single) for p in params]
         if blocks == 0:
             raise ValueError("pairformer_forward needs at least one block of parameters")
-    structs = (_lib.PairformerBlockParams * len(packed))(*[p.struct for p in packed])
+    structs = (_lib.PairformerBlockParams * len(packed)).from_buffer_copy(b"".join(p.struct for p in packed))
     c_s = sd.shape[2] if single else 0
     heads_s = packed[0].heads_s
     if single and c_s != heads_s * 24:
         raise ValueError(f"libb200tri is built for single-track heads of width 24; got c_s {c_s}, {heads_s} heads")
-    hidden_z = packed[0].struct.transition_z.hidden
-    hidden_s = packed[0].struct.transition_s.hidden if single else 0
-    nbytes = lib.b200tri_pairformer_workspace_bytes(n, c_s, heads_s, hidden_z, hidden_s)
+    nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s, packed[0].hidden_z, packed[0].hidden_s)
     ws = dev.workspace(nbytes, "pairformer")
     z_out = torch.empty_like(zd)
     s_out = torch.empty_like(sd) if single else None
@@ -181,7 +173,7 @@ def pairformer_forward(
             pair_mask=pmd[bi].data_ptr() if pmd is not None else None, mask=md[bi].data_ptr() if md is not None else None,
             workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes,
             pair_gate=int(gate), mask_transition=int(mask_trans), attention_first=int(bool(attention_first)))
-        _lib.check(lib.b200tri_pairformer_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
+        _lib.check(lib.b200tri_pairformer_forward(C.byref(args), dev.stream_ptr()))
     if squeeze:
         z_out = z_out[0]
         s_out = s_out[0] if single and np.ndim(s) == 2 else s_out

@@ -78,8 +78,7 @@ def transition_forward(
         "fc3": _leaf(params, "fc3", "kernel"),
     }
     hidden = leaves["fc1"].shape[-1]
-    if (tuple(leaves["fc1"].shape) != (C_Z, hidden) or tuple(leaves["fc2"].shape) != (C_Z, hidden)
-            or tuple(leaves["fc3"].shape) != (hidden, C_Z)):
+    if leaves["fc1"].shape != (C_Z, hidden) or leaves["fc2"].shape != (C_Z, hidden) or leaves["fc3"].shape != (hidden, C_Z):
         raise ValueError(
             f"transition kernels must be fc1/fc2 [{C_Z}, hidden] and fc3 [hidden, {C_Z}]; got "
             f"{tuple(leaves['fc1'].shape)}, {tuple(leaves['fc2'].shape)}, {tuple(leaves['fc3'].shape)}")
@@ -90,15 +89,13 @@ def transition_forward(
         md = dev.to_device(mask, torch.float32)
         if md.numel() != rows:
             raise ValueError(f"mask shape {tuple(md.shape)} does not give one value per row of x {tuple(xd.shape)}")
-    nbytes = lib.b200tri_pair_transition_workspace_bytes(hidden)
+    nbytes = _lib.workspace_bytes("b200tri_pair_transition_workspace_bytes", hidden)
     ws = dev.workspace(nbytes, "pair_transition")
-    args = _lib.PairTransitionArgs(
-        rows=rows, channels=C_Z, hidden=hidden, eps=float(eps),
-        x=xd.data_ptr(), residual=_ptr(rd), out=out.data_ptr(),
-        workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes, row_mask=_ptr(md),
-        **{k: v.data_ptr() for k, v in leaves.items()},
-    )
-    _lib.check(lib.b200tri_pair_transition(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    # (the leaves are in the order of the struct's fields)
+    args = _lib.pack_pair_transition(rows, C_Z, hidden, float(eps), xd.data_ptr(),
+                                     *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(),
+                                     dev.aligned_ptr(ws), nbytes, _ptr(md))
+    _lib.check(lib.b200tri_pair_transition(C.byref(args), dev.stream_ptr()))
     if host_in:
         host = out.float().cpu() if numpy_in else out.cpu()
         dev.check_device_status()

@@ -21,33 +21,50 @@ from . import _lib
 C_Z = 128  # channel width of the tensor-core specialisation (other widths run the general path)
 
 
-def _ptr(t: torch.Tensor | None) -> int | None:
-    return None if t is None else t.data_ptr()
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _check_pair(x: torch.Tensor) -> tuple[torch.Tensor, Any]:
     """-> (the pair tensor as [B, N, N, C], the caller's leading shape). A missing batch axis is
     added and leading axes beyond one are folded into B, the way the reference's fused
     wrappers do it (src/foldjax/models/_cueq.py:89-121); the second item is what to restore."""
-    lead = tuple(x.shape[:-3])
-    if x.dim() < 3 or x.shape[-2] != x.shape[-3]:
-        raise ValueError(f"expected a pair tensor [B, N, N, C], got shape {tuple(x.shape)}")
-    if x.shape[-1] % 8 or x.shape[-1] > 1024:
-        raise ValueError(f"libb200tri takes channel counts that are multiples of 8 up to 1024; got {x.shape[-1]} channels")
-    return x.reshape((-1,) + tuple(x.shape[-3:])), lead
+    shape = tuple(x.shape)
+    if len(shape) < 3 or shape[-2] != shape[-3]:
+        raise ValueError(f"expected a pair tensor [B, N, N, C], got shape {shape}")
+    if shape[-1] % 8 or shape[-1] > 1024:
+        raise ValueError(f"libb200tri takes channel counts that are multiples of 8 up to 1024; got {shape[-1]} channels")
+    return x if len(shape) == 4 else x.reshape((-1,) + shape[-3:]), shape[:-3]
 
 
 def _unfold(t: torch.Tensor, lead: tuple) -> torch.Tensor:
-    return t.reshape(tuple(lead) + tuple(t.shape[1:]))
+    return t if len(lead) == 1 else t.reshape(tuple(lead) + tuple(t.shape[1:]))
 
 
 def _leaf(params: Mapping, *path: str, dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     node: Any = params
     for key in path:
         node = node[key]
-    if not isinstance(node, torch.Tensor) or not node.is_cuda or node.dtype != dtype:
+    if not isinstance(node, torch.Tensor) or node.dtype is not dtype or not node.is_cuda:
         node = dev.to_device(node, dtype)
-    return node.contiguous()
+    return node if node.is_contiguous() else node.contiguous()
+
+
+def _check_leaves(leaves: Mapping[str, torch.Tensor], want: Mapping[str, tuple], what: str, where: str) -> None:
+    for name, shape in want.items():
+        if leaves[name].shape != shape:
+            raise ValueError(f"{what} parameter {name} has shape {tuple(leaves[name].shape)}, expected {shape} for {where}")
+
+
+def _pair_mask(mask: Any, b: int, n: int, x: Any) -> torch.Tensor | None:
+    """The pair mask of a call as float32 with b * n * n values (None = ones)."""
+    if mask is None:
+        return None
+    md = dev.to_device(mask, torch.float32)
+    shape = md.shape
+    if shape != (b, n, n) and (len(shape) < 2 or shape[-2:] != (n, n) or md.numel() != b * n * n):
+        raise ValueError(f"mask shape {tuple(shape)} does not match pair tensor {tuple(x.shape)}")
+    return md
 
 
 def resolve_dtype(x: Any, dtype: str | None) -> tuple[torch.dtype, int]:
@@ -104,16 +121,11 @@ def triangle_multiplication_forward(
     numpy_in = isinstance(x, np.ndarray)
     tdt, code = resolve_dtype(x, dtype)
     xd, lead = _check_pair(dev.to_device(x, tdt))
-    b, n, c_z = xd.shape[0], xd.shape[1], xd.shape[3]
-    md = None
-    if mask is not None:
-        md = dev.to_device(mask, torch.float32)
-        if md.dim() < 2 or tuple(md.shape[-2:]) != (n, n) or md.numel() != b * n * n:
-            raise ValueError(f"mask shape {tuple(md.shape)} does not match pair tensor {tuple(x.shape)}")
-        md = md.reshape(b, n, n)
+    b, n, _, c_z = xd.shape
+    md = _pair_mask(mask, b, n, x)
     rd = None
     if residual is not None:
-        rd, _ = _check_pair(dev.to_device(residual, tdt))
+        rd = xd if residual is x else _check_pair(dev.to_device(residual, tdt))[0]
         dev.check_same_shape(rd, xd, "residual")
     if out is None:
         out = torch.empty_like(xd)
@@ -134,22 +146,18 @@ def triangle_multiplication_forward(
     c_hidden = leaves["p_out"].shape[0]
     want = {"norm_in_scale": (c_z,), "norm_in_bias": (c_z,), "p_in": (c_z, 2 * c_hidden), "g_in": (c_z, 2 * c_hidden),
             "norm_out_scale": (c_hidden,), "norm_out_bias": (c_hidden,), "p_out": (c_hidden, c_z), "g_out": (c_z, c_z)}
-    for name, shape in want.items():
-        if tuple(leaves[name].shape) != shape:
-            raise ValueError(f"triangle multiplication parameter {name} has shape {tuple(leaves[name].shape)}, "
-                             f"expected {shape} for c_z = {c_z}, c_hidden = {c_hidden}")
+    _check_leaves(leaves, want, "triangle multiplication", f"c_z = {c_z}, c_hidden = {c_hidden}")
     if c_hidden % 8 or c_hidden > 1024:
         raise ValueError(f"libb200tri takes hidden widths that are multiples of 8 up to 1024; got {c_hidden}")
-    nbytes = lib.b200tri_trimul_workspace_bytes_shape(n, code, c_z, c_hidden)
+    nbytes = _lib.workspace_bytes("b200tri_trimul_workspace_bytes_shape", n, code, c_z, c_hidden)
     if b > 1 and (code, c_z, c_hidden) != (_lib.DTYPE_BF16, C_Z, C_Z):
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     ws = dev.workspace(nbytes, "trimul")
-    args = _lib.TrimulArgs(
-        n=n, incoming=int(direction == "incoming"), eps=float(eps), x=xd.data_ptr(), mask=_ptr(md), residual=_ptr(rd),
-        out=out.data_ptr(), workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes, dtype=code, c_z=c_z, c_hidden=c_hidden,
-        batch=b, **{k: v.data_ptr() for k, v in leaves.items()},
-    )
-    _lib.check(lib.b200tri_trimul_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    # (the leaves are in the order of the struct's fields)
+    args = _lib.pack_trimul(n, int(direction == "incoming"), float(eps), xd.data_ptr(), _ptr(md),
+                            *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
+                            nbytes, code, c_z, c_hidden, b)
+    _lib.check(lib.b200tri_trimul_forward(C.byref(args), dev.stream_ptr()))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

@@ -11,6 +11,7 @@ are accepted and ignored, as the reference's fused backends do.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from typing import Any, Mapping
 
 import numpy as np
@@ -18,7 +19,7 @@ import torch
 
 from . import _device as dev
 from . import _lib
-from .triangle import C_Z, _check_pair, _leaf, _ptr, _unfold, resolve_dtype
+from .triangle import C_Z, _check_leaves, _check_pair, _leaf, _pair_mask, _ptr, _unfold, resolve_dtype
 
 HEADS = 4
 HEAD_DIM = 32
@@ -60,16 +61,11 @@ def triangle_attention_forward(
     numpy_in = isinstance(x, np.ndarray)
     tdt, code = resolve_dtype(x, dtype)
     xd, lead = _check_pair(dev.to_device(x, tdt))
-    b, n, c_z = xd.shape[0], xd.shape[1], xd.shape[3]
-    md = None
-    if mask is not None:
-        md = dev.to_device(mask, torch.float32)
-        if md.dim() < 2 or tuple(md.shape[-2:]) != (n, n) or md.numel() != b * n * n:
-            raise ValueError(f"mask shape {tuple(md.shape)} does not match pair tensor {tuple(x.shape)}")
-        md = md.reshape(b, n, n)
+    b, n, _, c_z = xd.shape
+    md = _pair_mask(mask, b, n, x)
     rd = None
     if residual is not None:
-        rd, _ = _check_pair(dev.to_device(residual, tdt))
+        rd = xd if residual is x else _check_pair(dev.to_device(residual, tdt))[0]
         dev.check_same_shape(rd, xd, "residual")
     if out is None:
         out = torch.empty_like(xd)
@@ -92,22 +88,18 @@ def triangle_attention_forward(
     head_dim = width // max(heads, 1)
     want = {"norm_scale": (c_z,), "norm_bias": (c_z,), "w_bias": (c_z, heads), "w_q": (c_z, width), "w_k": (c_z, width),
             "w_v": (c_z, width), "w_g": (c_z, width), "w_o": (width, c_z)}
-    for name, shape in want.items():
-        if tuple(leaves[name].shape) != shape:
-            raise ValueError(f"triangle attention parameter {name} has shape {tuple(leaves[name].shape)}, expected "
-                             f"{shape} for c_z = {c_z}, {heads} heads x {head_dim}")
+    _check_leaves(leaves, want, "triangle attention", f"c_z = {c_z}, {heads} heads x {head_dim}")
     if heads * head_dim != width or head_dim not in (8, 16, 24, 32, 48, 64):
         raise ValueError(f"libb200tri takes head widths 8, 16, 24, 32, 48 and 64; got {heads} heads over {width} channels")
-    nbytes = lib.b200tri_triatt_workspace_bytes_shape(n, code, c_z, heads, head_dim)
+    nbytes = _lib.workspace_bytes("b200tri_triatt_workspace_bytes_shape", n, code, c_z, heads, head_dim)
     if b > 1 and (code, c_z, heads, head_dim) != (_lib.DTYPE_BF16, C_Z, HEADS, HEAD_DIM):
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     ws = dev.workspace(nbytes, "triatt")
-    args = _lib.TriattArgs(
-        n=n, starting=int(bool(starting)), heads=heads, head_dim=head_dim, inf=float(inf), eps=float(eps),
-        x=xd.data_ptr(), mask=_ptr(md), residual=_ptr(rd), out=out.data_ptr(), workspace=dev.aligned_ptr(ws),
-        workspace_bytes=nbytes, dtype=code, c_z=c_z, batch=b, **{k: v.data_ptr() for k, v in leaves.items()},
-    )
-    _lib.check(lib.b200tri_triatt_forward(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    # (the leaves are in the order of the struct's fields)
+    args = _lib.pack_triatt(n, int(bool(starting)), heads, head_dim, C.c_float(inf).value, float(eps), xd.data_ptr(), _ptr(md),
+                            *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
+                            nbytes, code, c_z, b)
+    _lib.check(lib.b200tri_triatt_forward(C.byref(args), dev.stream_ptr()))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()
@@ -130,49 +122,44 @@ def attention_core(q, k, v, tri_bias, mask_bias, scale: float | None = None):
     soft and hard entries can be mixed; a row with no kept key comes out as the uniform average
     over its keys, the convention of the finite -1e9 mask (triangle_attention.py:138-142), not as
     the zeros of the reference's 2-D ring (src/foldjax/models/_cp_attention.py:380-385).
-    Enqueue-only: nothing here waits for the device. The operands are re-laid out for the
-    kernel with torch copies (q,k -> [I,J,H*D], v -> [I,H*D,K] fp16, bias -> [H,J,K]); the
-    module-level forward avoids those copies by producing that layout directly.
+    Enqueue-only: nothing here waits for the device. bf16 operands are read where they are (the
+    library transposes v, builds the mask rows and, only where its rows are off TMA's 16-byte
+    grid or float32, copies the bias); other element types are converted first.
     """
     dev.require_cuda()
     lib = _lib.load()
     lead = q.shape[:-4]
-    qf = q.reshape((-1,) + tuple(q.shape[-4:]))
-    kf = k.reshape((-1,) + tuple(k.shape[-4:]))
-    vf = v.reshape((-1,) + tuple(v.shape[-4:]))
-    bf = tri_bias.reshape((-1,) + tuple(tri_bias.shape[-4:]))
-    mf = mask_bias.reshape((-1,) + tuple(mask_bias.shape[-4:]))
-    bsz, n_i, h, n_j, d = qf.shape
-    n_k = kf.shape[-2]
+    bsz = math.prod(lead)
+    n_i, h, n_j, d = q.shape[-4:]
+    n_k = k.shape[-2]
     if (h, d) != (HEADS, HEAD_DIM):
         raise ValueError(f"libb200tri is built for 4 heads x 32; got {h} x {d}")
-    if tuple(mf.shape[1:]) != (n_i, 1, 1, n_k) or tuple(bf.shape[1:]) != (1, h, n_j, n_k):
+    if mask_bias.shape[-4:] != (n_i, 1, 1, n_k) or tri_bias.shape[-4:] != (1, h, n_j, n_k):
         raise ValueError(f"mask_bias {tuple(mask_bias.shape)} / tri_bias {tuple(tri_bias.shape)} do not match "
                          f"q {tuple(q.shape)} and k {tuple(k.shape)}")
-    qf = qf.to(torch.bfloat16)
+    for name, t, count in (("k", k, bsz * n_i * h * n_k * d), ("v", v, bsz * n_i * h * n_k * d),
+                           ("tri_bias", tri_bias, bsz * h * n_j * n_k), ("mask_bias", mask_bias, bsz * n_i * n_k)):
+        if t.numel() != count:
+            raise ValueError(f"{name} shape {tuple(t.shape)} does not match q {tuple(q.shape)}")
+    qd = _operand(q, torch.bfloat16)
     if scale is not None:
-        qf = qf * torch.tensor(float(scale), dtype=torch.bfloat16, device=qf.device)  # one bf16 rounding
-    ld = (n_k + 63) // 64 * 64
-    out = torch.empty((bsz, n_i, h, n_j, d), dtype=v.dtype, device=v.device)
-    nbytes = lib.b200tri_triatt_core_workspace_bytes(n_i, n_k)
-    ws = dev.workspace(nbytes, "triatt_core")
-    for bi in range(bsz):
-        q2 = qf[bi].permute(0, 2, 1, 3).reshape(n_i, n_j, h * d).contiguous()
-        k2 = kf[bi].permute(0, 2, 1, 3).reshape(n_i, n_k, h * d).to(torch.bfloat16).contiguous()
-        v2 = torch.zeros(n_i, h * d, ld, dtype=torch.float16, device=v.device)
-        v2[:, :, :n_k] = vf[bi].permute(0, 1, 3, 2).reshape(n_i, h * d, n_k).to(torch.float16)
-        b2 = torch.zeros(h, n_j, ld, dtype=torch.bfloat16, device=v.device)
-        b2[:, :, :n_k] = bf[bi, 0].to(torch.bfloat16)
-        mb = mf[bi, :, 0, 0, :].float().contiguous()
-        o2 = torch.empty(n_i, n_j, h * d, dtype=torch.bfloat16, device=v.device)
-        args = _lib.TriattCoreArgs(
-            n_i=n_i, n_j=n_j, n_k=n_k, heads=h, head_dim=d,
-            q=q2.data_ptr(), k=k2.data_ptr(), vt=v2.data_ptr(), v_ld=ld,
-            bias=b2.data_ptr(), bias_ld=ld, bias_head_stride=n_j * ld,
-            mask=mb.data_ptr(), ms_i=n_k, ms_k=1, inf=0.0, mask_additive=1,
-            o=o2.data_ptr(), row_max=None, row_sum=None, unnormalized=0,
-            workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes,
-        )
-        _lib.check(lib.b200tri_triatt_core(C.byref(args), C.c_void_p(dev.stream_ptr())))
-        out[bi] = o2.reshape(n_i, n_j, h, d).permute(0, 2, 1, 3).to(v.dtype)
-    return out.reshape(tuple(lead) + tuple(out.shape[1:]))
+        # one bf16 rounding of q times the bf16 value of scale
+        qd = qd * torch.tensor(float(scale), dtype=torch.bfloat16).item()
+    kd = _operand(k, torch.bfloat16)
+    vd = _operand(v, v.dtype if v.dtype in (torch.bfloat16, torch.float32) else torch.float32)
+    bd = _operand(tri_bias, tri_bias.dtype if tri_bias.dtype in (torch.bfloat16, torch.float32) else torch.bfloat16)
+    md = _operand(mask_bias, torch.float32)
+    out = torch.empty(q.shape, dtype=torch.bfloat16, device=q.device)
+    nbytes = _lib.workspace_bytes("b200tri_attention_core_workspace_bytes", n_i, n_j, n_k)
+    ws = dev.workspace(nbytes, "attention_core")
+    args = _lib.pack_attention_core(bsz, n_i, n_j, n_k, h, d, int(vd.dtype is torch.float32), int(bd.dtype is torch.float32),
+                                    qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), bd.data_ptr(), md.data_ptr(),
+                                    out.data_ptr(), dev.aligned_ptr(ws), nbytes)
+    _lib.check(lib.b200tri_attention_core(C.byref(args), dev.stream_ptr()))
+    return out if v.dtype is torch.bfloat16 else out.to(v.dtype)
+
+
+def _operand(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``t`` as the library reads it: dense, of ``dtype`` and 16-byte aligned (a slice need not be)."""
+    t = t.to(dtype).contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()

@@ -344,6 +344,25 @@ typedef struct {
 size_t b200tri_triatt_core_workspace_bytes(int32_t n_i, int32_t n_k);
 int b200tri_triatt_core(const b200tri_triatt_core_args* args, b200tri_stream_t stream);
 
+/* The attention-core operator: core(q, k, v, tri_bias, mask_bias) -> out with the operands in the
+ * caller's order, q/out [batch][n_i][heads][n_j][32], k/v [batch][n_i][heads][n_k][32], bias
+ * [batch][heads][n_j][n_k], mask_bias [batch][n_i][n_k] float32 and additive; q, k, out and (unless
+ * the flags say float32) v and bias are bf16, everything dense. Replaces pallas_attention_core,
+ * src/foldjax/models/boltz2/models/triangle/triangle_attention_pallas.py:180. q, k, v and out must
+ * be 16-byte aligned; q is scaled already. */
+typedef struct {
+  int32_t batch, n_i, n_j, n_k, heads, head_dim; /* 4 heads x 32 */
+  int32_t v_f32, bias_f32;
+  const void *q, *k, *v, *bias;
+  const float* mask_bias;
+  void* out;
+  void* workspace; /* b200tri_attention_core_workspace_bytes, 1024-byte aligned */
+  size_t workspace_bytes;
+} b200tri_attention_core_args;
+
+size_t b200tri_attention_core_workspace_bytes(int32_t n_i, int32_t n_j, int32_t n_k);
+int b200tri_attention_core(const b200tri_attention_core_args* args, b200tri_stream_t stream);
+
 /* core over several key tiles in ONE launch: the same softmax walks tiles[0..n_tiles) in
  * order, each tile with its own k, vt, bias and mask buffers (the peers' tiles of a
  * context-parallel ring, which live in separate receive buffers); q, the sizes, the
