@@ -310,7 +310,9 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     t.proj_z = P.attention.proj_z;
     t.proj_o = P.attention.proj_o;
     int splits = 1;
-    if ((rc = single_attention(&t, sn, sn, ws + pl.att, partial, &splits, stream))) return rc;
+    if ((rc = single_project(&t, sn, sn, ws + pl.att, stream)) || (rc = single_pair_bias(&t, ws + pl.att, stream)) ||
+        (rc = single_attend(&t, ws + pl.att, partial, &splits, stream)))
+      return rc;
     row.base = layer == 0 ? a->s_in : a->s_out;
     row.partial = partial;
     row.splits = splits;

@@ -41,12 +41,16 @@ int launch_swiglu(const __nv_bfloat16* pieces, int rows, int k, const void* fc1,
                   void* w1_scratch, void* w2_scratch, __nv_bfloat16* h, long long pitch, cudaStream_t stream, bool pdl);
 
 struct SingleAttentionWork {  // offsets inside the attention workspace
-  size_t q, k, v, g, bias, ao, w[5], total;
+  size_t q, k, vt, g, bias, mask, ao, w[5], total;
 };
 SingleAttentionWork single_attention_work(int n, int c_s, int heads);
-// partial[splits][n][c_s] = (g * softmax(q k^T / sqrt(d) + bias(z) + mask) v) @ Wo, from the
-// pieces of the query-side and key-side rows. `work` is carved by single_attention_work.
-int single_attention(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk,
-                     uint8_t* work, float* partial, int* splits, cudaStream_t stream);
+// The attention with pair bias in three steps, `work` carved by single_attention_work:
+// q, k, v and the gate from the pieces of the query-side and key-side rows (does not read z);
+int single_project(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk, uint8_t* work,
+                   cudaStream_t stream);
+// the projected pair bias and the mask row (reads z and the token mask only);
+int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream);
+// partial[splits][n][c_s] = (g * softmax(q k^T / sqrt(d) + bias + mask) v) @ Wo.
+int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream);
 
 }  // namespace b200

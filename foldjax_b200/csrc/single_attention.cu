@@ -11,11 +11,9 @@
 // Everything here is fp32 arithmetic on fp32 s and bf16 z / weights (the trunk
 // dtype), like the reference's promoted computation.
 //
-// The only part that scales with N^2 * c_z is the pair-bias pass over z
-// (pair_bias_kernel, HBM-bound: 256 B read and 4 * heads B written per pair); the
-// token attention itself is N^2 * c_s work (14 GFLOP at N = 3072) and runs on the
-// fp32 pipes: at 16 heads x 24 channels it is far too small to be worth tensor-core
-// tiles, and its operands are fp32.
+// The pass over z is pair_bias_kernel, bound by HBM (256 B read and 4 * heads B written per pair);
+// the token attention is att_split.cu's one-row form; the products are gemm.cuh's.
+#include "att_split.cuh"
 #include "host.cuh"
 #include "single.cuh"
 #include "tc.cuh"
@@ -29,167 +27,261 @@ constexpr int MAX_HEADS = 16;
 constexpr int HD = 24;  // head width the token-attention kernel is built for
 
 // ---------------------------------------------------------------- pair bias
-// One thread per pair, 128 pairs per tile. With gamma folded into the projection,
+// Tiles of 128 pairs. With gamma folded into the projection,
 //   bias_h = rstd * (sum_c x_c W'[c][h] - mean * sum_c W'[c][h]) + sum_c beta_c W[c][h],
-// so the normalised row is never formed: one pass for the mean, one for the variance
-// (two-pass, as the reference computes it), one pass of heads FMAs per channel. The tile is
-// loaded with coalesced 16-byte loads into shared memory (16-byte chunks XOR-swizzled by the
-// pair index, so that neither the row-major stores nor the thread-per-row reads conflict)
-// and every pass reads it from there: the row never has to live in registers, and the
-// projection runs two heads per instruction (fma.f32x2).
-__global__ void __launch_bounds__(128, 4)
-pair_bias_kernel(const __nv_bfloat16* __restrict__ z, long long n_pairs, int n, int ld, int heads,
-                 const __nv_bfloat16* __restrict__ ln_scale, const __nv_bfloat16* __restrict__ ln_bias,
-                 const __nv_bfloat16* __restrict__ wz, float eps, float* __restrict__ bias) {
-  __shared__ __align__(16) float w[C_Z][MAX_HEADS];  // gamma_c * Wz[c][h]
+// so the normalised row is never formed. x is bf16 already and W' goes in as three bf16 pieces, 16
+// columns each, so one 128 x 48 x 128 product on the tensor cores is as exact as a float32 one;
+// meanwhile one thread per pair takes mean and variance (two-pass, as the reference computes
+// them) from the same shared-memory tile. On the CUDA cores the 2048 multiply-adds of a pair
+// were the bound: 200 us at n = 1024, four times what the bytes need.
+//   warps 0-3   mean, variance, result     warp 4   TMA producer     warp 5   MMA issuer
+// Two CTAs per SM: one's loads and result stores run beside the other's arithmetic.
+constexpr int PB_STAGES = 3, PB_TILE = 128 * C_Z * 2, PB_N = 3 * MAX_HEADS, PB_W = PB_N * 128;
+constexpr int PB_THREADS = 192, PB_SMEM = PB_STAGES * PB_TILE + 2 * PB_W + 1024;
+
+struct PairBiasParams {
+  uint32_t n_pairs, n;
+  int ld, heads, mask_ld;
+  bool early;  // the weights may be read before the predecessor in the stream is through
+  const __nv_bfloat16 *ln_scale, *ln_bias, *wz;
+  float eps, inf;
+  const float* mask;
+  float *bias, *mask_rows;
+  int* status;
+};
+
+__global__ void __launch_bounds__(PB_THREADS, 2) pair_bias_kernel(const __grid_constant__ CUtensorMap tm_z, const PairBiasParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* w_s = smem + PB_STAGES * PB_TILE;  // W' pieces, K-major: two halves of 64 channels x 48 rows
+  __shared__ uint64_t full_bar[PB_STAGES], empty_bar[PB_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_s;
   __shared__ float sw[MAX_HEADS], bw[MAX_HEADS];
-  __shared__ __align__(16) uint4 tile_s[128 * 16];   // 128 pairs x 16 chunks of 8 channels
-  for (int idx = threadIdx.x; idx < C_Z * MAX_HEADS; idx += blockDim.x) {
-    const int c = idx / MAX_HEADS, h = idx % MAX_HEADS;
-    w[c][h] = h < heads ? __bfloat162float(ln_scale[c]) * __bfloat162float(wz[c * heads + h]) : 0.f;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 4 && lane == 0) {
+    tma_prefetch_desc(&tm_z);
+    for (int s = 0; s < PB_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1 + 4);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 4);
+    }
+    fence_barrier_init();
   }
-  __syncthreads();
-  if (threadIdx.x < MAX_HEADS) {
-    const int h = threadIdx.x;
-    float a = 0.f, b = 0.f;
-    for (int c = 0; c < C_Z; ++c) {
-      a += w[c][h];
-      if (h < heads) b += __bfloat162float(ln_bias[c]) * __bfloat162float(wz[c * heads + h]);
-    }
-    sw[h] = a;
-    bw[h] = b;
+  if (warp == 5) {
+    tmem_alloc(&tmem_base_s, 128);
+    tmem_relinquish();
   }
+  if (!p.early) pdl_wait();
+  if (warp < 4) {  // thread = (head, 16 channels)
+    const int h = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 16;
+    float sum = 0.f, beta = 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+      float w[2] = {0.f, 0.f};
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = c0 + e + u;
+        const float raw = h < p.heads ? __bfloat162float(p.wz[c * p.heads + h]) : 0.f;
+        w[u] = __bfloat162float(p.ln_scale[c]) * raw;
+        sum += w[u];
+        beta += __bfloat162float(p.ln_bias[c]) * raw;
+      }
+      uint32_t pc[3];
+      split3x2(w[0], w[1], pc[0], pc[1], pc[2]);
+      const int k = (c0 + e) & 63;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint32_t*>(w_s + (c0 >> 6) * PB_W + sw128_offset(q * MAX_HEADS + h, k >> 3) + (k & 7) * 2) = pc[q];
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      beta += __shfl_xor_sync(0xffffffffu, beta, d);
+    }
+    if ((threadIdx.x & 7) == 0) {
+      sw[h] = sum;
+      bw[h] = beta;
+    }
+    fence_proxy_async();
+  }
+  tc_fence_before();
   __syncthreads();
-  const long long tiles = (n_pairs + 127) / 128;
-  const int p = threadIdx.x, key = p & 15;
-  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const long long base = tile * 128;
-    const long long left = n_pairs - base;  // pairs of this tile that exist (>= 1)
-    const uint4* src = reinterpret_cast<const uint4*>(z + base * C_Z);
-#pragma unroll 8
-    for (int it = 0; it < 16; ++it) {
-      const int idx = it * 128 + p;  // chunk idx of the tile: pair idx / 16, chunk idx % 16
-      const int pr = idx >> 4, ch = idx & 15;
-      const uint4 v = pr < left ? src[idx] : make_uint4(0u, 0u, 0u, 0u);
-      tile_s[pr * 16 + (ch ^ (pr & 15))] = v;
-    }
-    __syncthreads();
-    const uint4* row = tile_s + p * 16;
-    float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const uint4 v = row[c ^ key];
-      const uint32_t x4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s4[e] += bf16_lo(x4[e]) + bf16_hi(x4[e]);
-    }
-    const float mean = ((s4[0] + s4[1]) + (s4[2] + s4[3])) * (1.0f / C_Z);
-    float q4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const uint4 v = row[c ^ key];
-      const uint32_t x4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float a = bf16_lo(x4[e]) - mean, b = bf16_hi(x4[e]) - mean;
-        q4[e] = fmaf(a, a, q4[e]);
-        q4[e] = fmaf(b, b, q4[e]);
+  tc_fence_after();
+  if (p.early) pdl_wait();
+  pdl_trigger();
+  const uint32_t tmem_base = tmem_base_s;
+  const uint32_t tiles = (p.n_pairs + 127) / 128;
+
+  if (warp == 4) {
+    if (elect_one()) {
+      uint32_t it = 0;
+      for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+        const uint32_t stage = it % PB_STAGES;
+        if (!mbar_wait(&empty_bar[stage], ((it / PB_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        uint8_t* dst = smem + stage * PB_TILE;
+        mbar_expect_tx(&full_bar[stage], PB_TILE);
+        for (int half = 0; half < 2; ++half)
+          tma_load_2d(dst + half * (PB_TILE / 2), &tm_z, &full_bar[stage], half * 64, static_cast<int>(tile * 128));
       }
     }
-    const float rstd = rsqrtf(((q4[0] + q4[1]) + (q4[2] + q4[3])) * (1.0f / C_Z) + eps);
-    float2 acc[MAX_HEADS / 2];
+  } else if (warp == 5) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(128, PB_N);
+      uint32_t it = 0;
+      for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+        const uint32_t stage = it % PB_STAGES, buf = it & 1;
+        if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
+        if (!mbar_wait(&full_bar[stage], (it / PB_STAGES) & 1, p.status, ST_TIMEOUT_MMA)) break;
+        tc_fence_after();
 #pragma unroll
-    for (int h = 0; h < MAX_HEADS / 2; ++h) acc[h] = make_float2(0.f, 0.f);
-#pragma unroll 2
-    for (int c = 0; c < 16; ++c) {
-      const uint4 v = row[c ^ key];
-      const uint32_t x4[4] = {v.x, v.y, v.z, v.w};
+        for (int half = 0; half < 2; ++half) {
+          const uint64_t adesc = umma_desc_kmajor(smem_u32(smem + stage * PB_TILE + half * (PB_TILE / 2)), 128);
+          const uint64_t bdesc = umma_desc_kmajor(smem_u32(w_s + half * PB_W), 128);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int ch = 8 * c + 2 * e;  // channels ch (low half) and ch + 1 (high half)
-        const float a = bf16_lo(x4[e]), b = bf16_hi(x4[e]);
-        const float2 a2 = make_float2(a, a), b2 = make_float2(b, b);
-        const float4* wa = reinterpret_cast<const float4*>(w[ch]);
-        const float4* wb = reinterpret_cast<const float4*>(w[ch + 1]);
+          for (int k = 0; k < 4; ++k)
+            umma_bf16_ss(tmem_base + buf * 64, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
+                         (half | k) != 0);
+        }
+        umma_commit(&empty_bar[stage]);
+        umma_commit(&acc_full[buf]);
+      }
+    }
+  } else {
+    // the token attention's mask row; keys past the end get no weight
+    if (blockIdx.x == 0)
+      for (int j = threadIdx.x; j < p.mask_ld; j += 128)
+        p.mask_rows[j] = j < static_cast<int>(p.n) ? fmaxf((1.0f - p.mask[j]) * -p.inf, SPLIT_MASK_MIN) : SPLIT_MASK_PAD;
+    const int r = threadIdx.x;
+    uint32_t it = 0;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+      const uint32_t stage = it % PB_STAGES, buf = it & 1;
+      if (!mbar_wait(&full_bar[stage], (it / PB_STAGES) & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      const uint8_t* src = smem + stage * PB_TILE;
+      uint4 x[16];
+      float2 s4[4] = {};
 #pragma unroll
-        for (int h4 = 0; h4 < MAX_HEADS / 4; ++h4) {
-          const float4 fa = wa[h4], fb = wb[h4];
-          acc[2 * h4 + 0] = __ffma2_rn(b2, make_float2(fb.x, fb.y), __ffma2_rn(a2, make_float2(fa.x, fa.y), acc[2 * h4 + 0]));
-          acc[2 * h4 + 1] = __ffma2_rn(b2, make_float2(fb.z, fb.w), __ffma2_rn(a2, make_float2(fa.z, fa.w), acc[2 * h4 + 1]));
+      for (int c = 0; c < 16; ++c) {
+        x[c] = *reinterpret_cast<const uint4*>(src + (c >> 3) * (PB_TILE / 2) + sw128_offset(r, c & 7));
+        s4[0] = __fadd2_rn(s4[0], make_float2(bf16_lo(x[c].x), bf16_hi(x[c].x)));
+        s4[1] = __fadd2_rn(s4[1], make_float2(bf16_lo(x[c].y), bf16_hi(x[c].y)));
+        s4[2] = __fadd2_rn(s4[2], make_float2(bf16_lo(x[c].z), bf16_hi(x[c].z)));
+        s4[3] = __fadd2_rn(s4[3], make_float2(bf16_lo(x[c].w), bf16_hi(x[c].w)));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty_bar[stage]);
+      const float2 s2 = __fadd2_rn(__fadd2_rn(s4[0], s4[1]), __fadd2_rn(s4[2], s4[3]));
+      const float mean = (s2.x + s2.y) * (1.0f / C_Z);
+      const float2 mm = make_float2(-mean, -mean);
+      float2 q4[4] = {};
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        const uint32_t v[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 d = __fadd2_rn(make_float2(bf16_lo(v[e]), bf16_hi(v[e])), mm);
+          q4[e] = __ffma2_rn(d, d, q4[e]);
         }
       }
-    }
-    const long long pair = base + p;
-    if (pair < n_pairs) {
-      const long long i = pair / n, j = pair % n;
+      const float2 q2 = __fadd2_rn(__fadd2_rn(q4[0], q4[1]), __fadd2_rn(q4[2], q4[3]));
+      const float rstd = rsqrtf((q2.x + q2.y) * (1.0f / C_Z) + p.eps);
+      if (!mbar_wait(&acc_full[buf], (it >> 1) & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      tc_fence_after();
+      __syncwarp();
+      uint32_t hi[16], mid[16], lo[16];
+      const uint32_t t = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + buf * 64;
+      tmem_ld16(t, hi);
+      tmem_ld16(t + 16, mid);
+      tmem_ld16(t + 32, lo);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      const uint32_t pair = tile * 128 + r;
+      if (pair < p.n_pairs) {
+        const uint32_t i = pair / p.n, j = pair - i * p.n;
+        float* dst = p.bias + static_cast<size_t>(i) * p.ld + j;
+        const size_t plane = static_cast<size_t>(p.n) * p.ld;
 #pragma unroll
-      for (int h = 0; h < MAX_HEADS; ++h)
-        if (h < heads)
-          bias[(static_cast<long long>(h) * n + i) * ld + j] = rstd * ((h & 1 ? acc[h >> 1].y : acc[h >> 1].x) - mean * sw[h]) + bw[h];
+        for (int h = 0; h < MAX_HEADS; ++h)
+          if (h < p.heads) {
+            const float dot = __uint_as_float(hi[h]) + (__uint_as_float(mid[h]) + __uint_as_float(lo[h]));
+            dst[h * plane] = rstd * (dot - mean * sw[h]) + bw[h];
+          }
+      }
     }
-    __syncthreads();  // the tile is overwritten by the next round's loads
   }
+
+  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5) tmem_dealloc(tmem_base, 128);
 }
 
 // ------------------------------------------------------------------ row kernels
-// See launch_row_norm. One warp per row, the row in registers (up to 12 values per lane).
-constexpr int ROW_VALUES = MAX_HEADS * HD / 32;
-__global__ void __launch_bounds__(128) row_norm_kernel(const RowArgs a) {
+// See launch_row_norm. One block per row, four neighbouring channels per thread: every load of a
+// row (the base and up to eight partial planes) is in flight at once. With one warp per row and
+// the planes added one after the other the kernel was a chain of 96 dependent loads, 20 us.
+constexpr int ROW_THREADS = MAX_HEADS * HD / 4;
+__device__ __forceinline__ float row_sum(float v, float* scratch) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return (scratch[0] + scratch[1]) + scratch[2];
+}
+__global__ void __launch_bounds__(ROW_THREADS) row_norm_kernel(const RowArgs a) {
+  static_assert(ROW_THREADS == 96, "three warps");
+  __shared__ float scratch[2][3];
   pdl_wait();
   pdl_trigger();
-  const int lane = threadIdx.x & 31;
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= a.rows) return;
-  const long long off = static_cast<long long>(row) * a.c;
+  const int row = blockIdx.x, i = threadIdx.x * 4;
+  const bool live = i < a.c;  // c is a multiple of 8
+  const long long off = static_cast<long long>(row) * a.c + i, plane = static_cast<long long>(a.rows) * a.c;
   const bool keep = a.row_mask == nullptr || a.row_mask[row] != 0.f;
-  float v[ROW_VALUES];
-  float s = 0.f;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (live && keep) {
+    float4 part[SINGLE_MAX_SPLITS], base = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int e = 0; e < ROW_VALUES; ++e) {
-    const int i = lane + 32 * e;
-    v[e] = 0.f;
-    if (i >= a.c || !keep) continue;
-    if (a.partial) {
-      float u = 0.f;
-      for (int p = 0; p < a.splits; ++p) u += a.partial[static_cast<long long>(p) * a.rows * a.c + off + i];
-      v[e] = u;
+    for (int p = 0; p < SINGLE_MAX_SPLITS; ++p)
+      part[p] = a.partial && p < a.splits ? *reinterpret_cast<const float4*>(a.partial + p * plane + off)
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.base) base = *reinterpret_cast<const float4*>(a.base + off);
+#pragma unroll
+    for (int p = 0; p < SINGLE_MAX_SPLITS; ++p) {
+      v[0] += part[p].x;
+      v[1] += part[p].y;
+      v[2] += part[p].z;
+      v[3] += part[p].w;
     }
-    if (a.base) v[e] = a.base[off + i] + v[e];
-    s += v[e];
+    v[0] = base.x + v[0];
+    v[1] = base.y + v[1];
+    v[2] = base.z + v[2];
+    v[3] = base.w + v[3];
   }
-  if (a.sum_out) {
-#pragma unroll
-    for (int e = 0; e < ROW_VALUES; ++e)
-      if (lane + 32 * e < a.c) a.sum_out[off + lane + 32 * e] = v[e];
-  }
+  if (a.sum_out && live) *reinterpret_cast<float4*>(a.sum_out + off) = make_float4(v[0], v[1], v[2], v[3]);
   if (!a.pieces) return;
   if (a.scale) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    const float mean = s / a.c;
+    const float mean = row_sum((v[0] + v[1]) + (v[2] + v[3]), scratch[0]) / a.c;
     float q = 0.f;
 #pragma unroll
-    for (int e = 0; e < ROW_VALUES; ++e)
-      if (lane + 32 * e < a.c) q += (v[e] - mean) * (v[e] - mean);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
-    const float rstd = 1.0f / sqrtf(q / a.c + a.eps);
+    for (int e = 0; e < 4; ++e) q += live ? (v[e] - mean) * (v[e] - mean) : 0.f;
+    const float rstd = 1.0f / sqrtf(row_sum(q, scratch[1]) / a.c + a.eps);
     const __nv_bfloat16* scale = static_cast<const __nv_bfloat16*>(a.scale);
     const __nv_bfloat16* bias = static_cast<const __nv_bfloat16*>(a.bias);
 #pragma unroll
-    for (int e = 0; e < ROW_VALUES; ++e) {
-      const int i = lane + 32 * e;
-      if (i < a.c) v[e] = (v[e] - mean) * rstd * __bfloat162float(scale[i]) + __bfloat162float(bias[i]);
-    }
+    for (int e = 0; e < 4; ++e)
+      if (live) v[e] = (v[e] - mean) * rstd * __bfloat162float(scale[i + e]) + __bfloat162float(bias[i + e]);
   }
-  const long long plane = static_cast<long long>(a.rows) * a.c;
+  if (!live) return;
+  uint32_t pc[3][2];
+  split3x2(v[0], v[1], pc[0][0], pc[1][0], pc[2][0]);
+  split3x2(v[2], v[3], pc[0][1], pc[1][1], pc[2][1]);
 #pragma unroll
-  for (int e = 0; e < ROW_VALUES; ++e) {
-    const int i = lane + 32 * e;
-    if (i >= a.c) continue;
-    __nv_bfloat16* dst = a.pieces + off + i;
-    split3(v[e], dst[0], dst[plane], dst[2 * plane]);
-  }
+  for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(a.pieces + q * plane + off) = make_uint2(pc[q][0], pc[q][1]);
 }
 
 // dst[k][ld] = src[k][n], padding columns zero: weights TMA cannot read as they are.
@@ -207,15 +299,18 @@ __global__ void pad_weight_kernel(const __nv_bfloat16* __restrict__ src, int k, 
 // loads); the products of a block are 0.6-15 GFLOP, so what bounds them at every size is
 // latency: many small tiles, K split until the tiles cover the SMs.
 //
-// [q | k | v | g] in one launch: column tiles of 64 walk the four weights in turn.
+// [q | k | v | g] in one launch: column tiles of 64 walk the four weights in turn. q and k leave as
+// pieces, v as transposed pieces (both as the token attention reads them), the gate in float32.
 struct QkvgPolicy {
   static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = 8, CTAS = 1;
   struct Params {
     int rows, c, tiles_per_w, first_w;
+    long long v_ld;
     const __nv_bfloat16* q_bias;
-    float* out[4];
+    __nv_bfloat16 *q, *k, *vt;
+    float* gate;
   };
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
@@ -229,25 +324,49 @@ struct QkvgPolicy {
                                   int col0, int col1, int lane) {
     const int row = m_tile * GEMM_BM + quarter * 32 + lane;
     const int which = p.first_w + n_tile / p.tiles_per_w;
+    const long long plane = static_cast<long long>(p.rows) * p.c, off = static_cast<long long>(row) * p.c;
 #pragma unroll 1
     for (int col = col0; col < col1; col += 16) {
-    float r[16];
-    acc.load(0, col, r);
-    if (row >= p.rows) continue;
-    const int c0 = n_tile % p.tiles_per_w * BN + col;
-    float* dst = p.out[which] + static_cast<long long>(row) * p.c + c0;
+      float r[16];
+      acc.load(0, col, r);
+      const int c0 = n_tile % p.tiles_per_w * BN + col;
+      if (row >= p.rows || c0 >= p.c) continue;
+      if (which == 2) {  // one channel per store: 32 lanes are 32 neighbouring tokens
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float v[4];
-      if (c0 + 4 * q >= p.c) break;  // c is a multiple of 8
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        v[e] = r[4 * q + e];
-        if (which == 0) v[e] += __bfloat162float(p.q_bias[c0 + 4 * q + e]);
-        if (which == 3) v[e] = 1.0f / (1.0f + expf(-v[e]));
+        for (int e = 0; e < 16; ++e) {
+          if (c0 + e >= p.c) break;  // c is a multiple of 8
+          __nv_bfloat16* dst = p.vt + (c0 + e) * p.v_ld + row;
+          split3(r[e], dst[0], dst[p.c * p.v_ld], dst[2 * p.c * p.v_ld]);
+        }
+        continue;
       }
-      *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
-    }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int c8 = c0 + 8 * q;
+        if (c8 >= p.c) break;
+        float* v = r + 8 * q;
+        if (which == 3) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = 1.0f / (1.0f + expf(-v[e]));
+          float4* dst = reinterpret_cast<float4*>(p.gate + off + c8);
+          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+          continue;
+        }
+        uint32_t pc[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (which == 0) {
+            v[2 * e] += __bfloat162float(p.q_bias[c8 + 2 * e]);
+            v[2 * e + 1] += __bfloat162float(p.q_bias[c8 + 2 * e + 1]);
+          }
+          split3x2(v[2 * e], v[2 * e + 1], pc[0][e], pc[1][e], pc[2][e]);
+        }
+        __nv_bfloat16* dst = (which == 0 ? p.q : p.k) + off + c8;
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+          *reinterpret_cast<uint4*>(dst + t * plane) = make_uint4(pc[t][0], pc[t][1], pc[t][2], pc[t][3]);
+      }
     }
   }
 };
@@ -340,82 +459,10 @@ struct SwigluPolicy {
   }
 };
 
-// --------------------------------------------------------- token attention
-// One thread per (query i, head h); keys in tiles of 32 staged in shared memory.
-// Online softmax in fp32; scores = q.k / sqrt(d) + bias + (1 - mask) * -inf, added in
-// that order like the reference (attention.py:134-136).
-constexpr int TQ = 64;  // queries per block
-constexpr int TK = 32;  // keys per tile
-
-__global__ void __launch_bounds__(TQ)
-token_attention_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                       const float* __restrict__ gate, const float* __restrict__ bias, const float* __restrict__ mask, int n,
-                       int n_keys, int ld, int c_s, float inf, __nv_bfloat16* __restrict__ out) {
-  __shared__ float ks[TK][HD], vs[TK][HD], ms[TK];
-  const int h = blockIdx.y;
-  const int i = blockIdx.x * TQ + threadIdx.x;
-  const bool live = i < n;
-  const float inv_scale = 1.0f / sqrtf(static_cast<float>(HD));
-  float qr[HD], acc[HD];
-#pragma unroll
-  for (int d = 0; d < HD; ++d) {
-    qr[d] = live ? q[static_cast<long long>(i) * c_s + h * HD + d] : 0.f;
-    acc[d] = 0.f;
-  }
-  float m_run = -INFINITY, l_run = 0.f;
-  const float* brow = bias + (static_cast<long long>(h) * n + (live ? i : 0)) * ld;
-  for (int j0 = 0; j0 < n_keys; j0 += TK) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < TK * HD; idx += TQ) {
-      const int r = idx / HD, d = idx % HD;
-      const int j = j0 + r;
-      ks[r][d] = j < n_keys ? k[static_cast<long long>(j) * c_s + h * HD + d] : 0.f;
-      vs[r][d] = j < n_keys ? v[static_cast<long long>(j) * c_s + h * HD + d] : 0.f;
-    }
-    if (threadIdx.x < TK) {
-      const int j = j0 + threadIdx.x;
-      ms[threadIdx.x] = j < n_keys ? (1.0f - mask[j]) * -inf : -INFINITY;  // keys past the end: no weight
-    }
-    __syncthreads();
-    float sc[TK];
-    float mx = m_run;
-#pragma unroll
-    for (int r = 0; r < TK; ++r) {
-      float dot = 0.f;
-#pragma unroll
-      for (int d = 0; d < HD; ++d) dot = fmaf(qr[d], ks[r][d], dot);
-      const float b = (j0 + r < n_keys) ? brow[j0 + r] : 0.f;
-      sc[r] = (dot * inv_scale + b) + ms[r];
-      mx = fmaxf(mx, sc[r]);
-    }
-    const float alpha = __expf(m_run - mx);  // 0 on the first tile
-    l_run *= alpha;
-#pragma unroll
-    for (int d = 0; d < HD; ++d) acc[d] *= alpha;
-#pragma unroll
-    for (int r = 0; r < TK; ++r) {
-      const float pr = __expf(sc[r] - mx);
-      l_run += pr;
-#pragma unroll
-      for (int d = 0; d < HD; ++d) acc[d] = fmaf(pr, vs[r][d], acc[d]);
-    }
-    m_run = mx;
-  }
-  if (live) {
-    const float inv = 1.0f / l_run;
-    const long long off = static_cast<long long>(i) * c_s + h * HD, plane = static_cast<long long>(n) * c_s;
-#pragma unroll
-    for (int d = 0; d < HD; ++d) {  // gated, as the pieces the output projection reads
-      __nv_bfloat16* dst = out + off + d;
-      split3(acc[d] * inv * gate[off + d], dst[0], dst[plane], dst[2 * plane]);
-    }
-  }
-}
-
 }  // namespace
 
 int launch_row_norm(const RowArgs& a, cudaStream_t stream, bool pdl) {
-  return launch(row_norm_kernel, dim3((a.rows + 3) / 4), dim3(128), 0, stream, pdl, a);
+  return launch(row_norm_kernel, dim3(a.rows), dim3(ROW_THREADS), 0, stream, pdl, a);
 }
 
 // Enough splits that the tiles cover the SMs, at least two k steps each, none of them empty.
@@ -481,43 +528,43 @@ SingleAttentionWork single_attention_work(int n, int c_s, int heads) {
     c.take<uint8_t>(bytes);
     return c.off - bytes;
   };
-  w.q = take(act * 4);
-  w.k = take(act * 4);
-  w.v = take(act * 4);
+  w.q = take(act * 2 * 3);
+  w.k = take(act * 2 * 3);
+  w.vt = take(static_cast<size_t>(c_s) * round_up(n, 8) * 2 * 3);
   w.g = take(act * 4);
-  w.bias = take(static_cast<size_t>(heads) * n * round_up(n, 4) * 4);
+  w.bias = take(static_cast<size_t>(heads) * n * round_up(n, 8) * 4);
+  w.mask = take(static_cast<size_t>(round_up(n, 64)) * 4);
   w.ao = take(act * 2 * 3);
   for (size_t& off : w.w) off = take(tma_weight_bytes(c_s, c_s));
   w.total = c.total();
   return w;
 }
 
-int single_attention(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk,
-                     uint8_t* work, float* partial, int* splits, cudaStream_t stream) {
-  const int n = a->n, c_s = a->c_s, heads = a->heads, ld = round_up(n, 4);
-  const SingleAttentionWork off = single_attention_work(n, c_s, heads);
-  float* out[4] = {reinterpret_cast<float*>(work + off.q), reinterpret_cast<float*>(work + off.k),
-                   reinterpret_cast<float*>(work + off.v), reinterpret_cast<float*>(work + off.g)};
-  float* bias = reinterpret_cast<float*>(work + off.bias);
-  __nv_bfloat16* ao = reinterpret_cast<__nv_bfloat16*>(work + off.ao);
-  auto bf = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
+namespace {
+const __nv_bfloat16* bf(const void* p) { return static_cast<const __nv_bfloat16*>(p); }
+}  // namespace
 
-  // q, k, v, g. With separate key-side rows: k, v from those in a launch of their own
-  // (weights in the order q, g | k, v then).
+int single_project(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk, uint8_t* work,
+                   cudaStream_t stream) {
+  const int n = a->n, c_s = a->c_s;
+  const SingleAttentionWork off = single_attention_work(n, c_s, a->heads);
+  // With separate key-side rows: k, v from those in a launch of their own.
   const bool same = xq == xk;
-  const void* w_same[4] = {a->proj_q, a->proj_k, a->proj_v, a->proj_g};
+  const void* w[4] = {a->proj_q, a->proj_k, a->proj_v, a->proj_g};
   GemmMaps maps = {};
   bool direct = true;
   int rc;
   for (int i = 0; i < 4; ++i) {
     const void* wp;
     long long pitch;
-    if ((rc = tma_weight(w_same[i], c_s, c_s, work + off.w[i], stream, &wp, &pitch))) return rc;
+    if ((rc = tma_weight(w[i], c_s, c_s, work + off.w[i], stream, &wp, &pitch))) return rc;
     if ((rc = gemm_map_mnmajor(&maps.b[i], wp, c_s, c_s, pitch))) return rc;
-    direct = direct && wp == w_same[i];
+    direct = direct && wp == w[i];
   }
   const int per_w = (c_s + QkvgPolicy::BN - 1) / QkvgPolicy::BN;
-  QkvgPolicy::Params ep = {n, c_s, per_w, 0, bf(a->proj_q_bias), {out[0], out[1], out[2], out[3]}};
+  auto at = [&](size_t o) { return reinterpret_cast<__nv_bfloat16*>(work + o); };
+  QkvgPolicy::Params ep = {n,         c_s,       per_w,      0, round_up(n, 8), bf(a->proj_q_bias), at(off.q), at(off.k),
+                           at(off.vt), reinterpret_cast<float*>(work + off.g)};
   // (first weight, weight count) of each launch
   const int runs_same[1][2] = {{0, 4}}, runs_split[3][2] = {{0, 1}, {1, 2}, {3, 1}};
   const int n_runs = same ? 1 : 3;
@@ -528,22 +575,64 @@ int single_attention(const b200tri_attention_pair_bias_args* a, const __nv_bfloa
     const GemmShape g = {mtiles(n), per_w * run[1], 1, {kblocks(c_s), 0}, nullptr};
     if ((rc = launch_piece_gemm<QkvgPolicy>(maps, g, ep, stream, direct && same))) return rc;
   }
-  {
-    TimedLaunch timed(K_PAIR_BIAS, stream);
-    const long long n_pairs = static_cast<long long>(n) * n;
-    const long long tiles = (n_pairs + 127) / 128;
-    const long long blocks = tiles < 16LL * sm_count() ? tiles : 16LL * sm_count();
-    count_launch();
-    pair_bias_kernel<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(bf(a->z), n_pairs, n, ld, heads,
-                                                                       bf(a->proj_z_norm_scale), bf(a->proj_z_norm_bias),
-                                                                       bf(a->proj_z), a->eps, bias);
-    B200_CUDA_OK(cudaGetLastError());
-  }
-  count_launch();
-  token_attention_kernel<<<dim3((n + TQ - 1) / TQ, heads), TQ, 0, stream>>>(
-      out[0], out[1], out[2], out[3], bias, static_cast<const float*>(a->mask), n, n, ld, c_s, a->inf, ao);
-  B200_CUDA_OK(cudaGetLastError());
-  return launch_linear_partial(ao, c_s, n, c_s, a->proj_o, c_s, work + off.w[4], partial, splits, stream, false);
+  return B200TRI_OK;
+}
+
+int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream) {
+  const int n = a->n;
+  const SingleAttentionWork off = single_attention_work(n, a->c_s, a->heads);
+  const long long n_pairs = static_cast<long long>(n) * n;
+  B200_REQUIRE(n_pairs < (1ll << 31) - 128, B200TRI_ERR_UNSUPPORTED, "pair bias: too many tokens (%d)", n);
+  PairBiasParams p = {};
+  p.n_pairs = static_cast<uint32_t>(n_pairs);
+  p.n = n;
+  p.ld = round_up(n, 8);
+  p.heads = a->heads;
+  p.mask_ld = round_up(n, 64);
+  p.early = pdl_chained();
+  p.ln_scale = bf(a->proj_z_norm_scale);
+  p.ln_bias = bf(a->proj_z_norm_bias);
+  p.wz = bf(a->proj_z);
+  p.eps = a->eps;
+  p.inf = a->inf;
+  p.mask = static_cast<const float*>(a->mask);
+  p.bias = reinterpret_cast<float*>(work + off.bias);
+  p.mask_rows = reinterpret_cast<float*>(work + off.mask);
+  p.status = device_status_word();
+  B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "pair bias: no current CUDA device");
+  CUtensorMap tm_z;
+  const uint64_t dims[2] = {C_Z, static_cast<uint64_t>(n_pairs)};
+  const uint64_t str[1] = {C_Z * 2};
+  const uint32_t box[2] = {64, 128};
+  int rc = make_tmap(&tm_z, a->z, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
+  if (rc || (rc = ensure_smem_limit(reinterpret_cast<const void*>(pair_bias_kernel), PB_SMEM))) return rc;
+  const long long tiles = (n_pairs + 127) / 128, slots = 2ll * sm_count();
+  TimedLaunch timed(K_PAIR_BIAS, stream);
+  return launch(pair_bias_kernel, dim3(static_cast<unsigned>(tiles < slots ? tiles : slots)), dim3(PB_THREADS), PB_SMEM, stream,
+                true, tm_z, p);
+}
+
+int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream) {
+  const int n = a->n, c_s = a->c_s;
+  const SingleAttentionWork off = single_attention_work(n, c_s, a->heads);
+  AttSplitArgs s = {};
+  s.batch = s.n_i = 1;
+  s.n = n;
+  s.heads = a->heads;
+  s.head_dim = HD;
+  s.q = bf(work + off.q);
+  s.k = bf(work + off.k);
+  s.vt = bf(work + off.vt);
+  s.v_ld = s.bias_ld = round_up(n, 8);
+  s.bias = work + off.bias;
+  s.mask_bias = reinterpret_cast<float*>(work + off.mask);
+  s.mask_ld = round_up(n, 64);
+  s.scale = 1.0f / sqrtf(static_cast<float>(HD));
+  s.gate = reinterpret_cast<float*>(work + off.g);
+  s.pieces = reinterpret_cast<__nv_bfloat16*>(work + off.ao);
+  const int rc = launch_att_split(s, stream);
+  if (rc) return rc;
+  return launch_linear_partial(s.pieces, c_s, n, c_s, a->proj_o, c_s, work + off.w[4], partial, splits, stream, true);
 }
 
 }  // namespace b200
@@ -611,7 +700,9 @@ extern "C" int b200tri_attention_pair_bias(const b200tri_attention_pair_bias_arg
     if ((rc = launch_row_norm(row, stream, false))) return rc;
   }
   int splits = 1;
-  if ((rc = single_attention(a, xq, xk, ws + pl.work, partial, &splits, stream))) return rc;
+  if ((rc = single_project(a, xq, xk, ws + pl.work, stream)) || (rc = single_pair_bias(a, ws + pl.work, stream)) ||
+      (rc = single_attend(a, ws + pl.work, partial, &splits, stream)))
+    return rc;
   row.base = nullptr;
   row.partial = partial;
   row.splits = splits;
