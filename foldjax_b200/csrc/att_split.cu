@@ -500,7 +500,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
 }
 
 template <int HDP, int IN, bool TOKEN>
-int launch_cfg(const Maps& tm, Params p, cudaStream_t stream) {
+int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   using C = Cfg<HDP, IN, TOKEN>;
   const int tiles = (p.n + 127) / 128;
   p.groups = TOKEN ? 1 : (p.n_i + C::NWG - 1) / C::NWG;
@@ -513,7 +513,7 @@ int launch_cfg(const Maps& tm, Params p, cudaStream_t stream) {
   if (rc) return rc;
   const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
   return launch(att_split_kernel<HDP, IN, TOKEN>, dim3(grid), dim3(C::THREADS),
-                sizeof(Smem<HDP, IN, TOKEN>), stream, true, tm, p);
+                sizeof(Smem<HDP, IN, TOKEN>), stream, pdl, tm, p);
 }
 
 }  // namespace
@@ -573,9 +573,9 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   p.pieces = a.pieces;
   p.status = device_status_word();
   B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "float32 attention: no current CUDA device");
-  if (token) return launch_cfg<32, 3, true>(tm, p, stream);
-  if (a.bf16) return hdp == 32 ? launch_cfg<32, 1, false>(tm, p, stream) : launch_cfg<64, 1, false>(tm, p, stream);
-  return hdp == 32 ? launch_cfg<32, 3, false>(tm, p, stream) : launch_cfg<64, 3, false>(tm, p, stream);
+  if (token) return launch_cfg<32, 3, true>(tm, p, a.pdl, stream);
+  if (a.bf16) return hdp == 32 ? launch_cfg<32, 1, false>(tm, p, a.pdl, stream) : launch_cfg<64, 1, false>(tm, p, a.pdl, stream);
+  return hdp == 32 ? launch_cfg<32, 3, false>(tm, p, a.pdl, stream) : launch_cfg<64, 3, false>(tm, p, a.pdl, stream);
 }
 
 }  // namespace b200

@@ -25,6 +25,7 @@ struct AttSplitArgs {
   void* o;                             // [batch * n_i][n][heads * head_dim]
   const float* gate;                   // one-row form: [n][heads * head_dim]
   __nv_bfloat16* pieces;               // one-row form: the output, o * gate as pieces [3][n][heads * head_dim]
+  bool pdl;                            // the predecessor in the stream is a kernel of the library
 };
 int launch_att_split(const AttSplitArgs& a, cudaStream_t stream);
 

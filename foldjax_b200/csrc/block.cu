@@ -14,6 +14,8 @@
 // round trips; one call per trunk replaces the scan.
 #include <cuda_bf16.h>
 
+#include <optional>
+
 #include "host.cuh"
 #include "single.cuh"
 
@@ -185,11 +187,62 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     B200_CUDA_OK(cudaGetLastError());
     return B200TRI_OK;
   };
+  auto params_of = [&](int layer) { return a->stacked ? unstack(first, layer, c_s, a->heads_s) : a->params[layer]; };
+  int rc;
+
+  // The single track is float32: s += attention(LN(s), z), s += transition(s), each sum taken by
+  // the row kernel that also normalises the rows for the product behind it. The pair bias is its
+  // only step that reads z, so in a stack everything else of a block's single track - six
+  // launches that fill a few SMs each - runs on a side stream beside the next block's pair track,
+  // and the first block's q, k, v and gate beside its own. 48 blocks at n = 128: 9.3 -> 8.2 ms.
+  auto attention_args = [&](const b200tri_pairformer_block_params& P) {
+    b200tri_attention_pair_bias_args t = {};
+    t.n = n;
+    t.c_s = c_s;
+    t.c_z = 128;
+    t.heads = a->heads_s;
+    t.eps = a->eps;
+    t.inf = a->att_inf;
+    t.z = a->z_out;
+    t.mask = token_mask;
+    t.proj_q = P.attention.proj_q;
+    t.proj_q_bias = P.attention.proj_q_bias;
+    t.proj_k = P.attention.proj_k;
+    t.proj_v = P.attention.proj_v;
+    t.proj_g = P.attention.proj_g;
+    t.proj_z_norm_scale = P.attention.proj_z_norm_scale;
+    t.proj_z_norm_bias = P.attention.proj_z_norm_bias;
+    t.proj_z = P.attention.proj_z;
+    t.proj_o = P.attention.proj_o;
+    return t;
+  };
+  __nv_bfloat16* sn = reinterpret_cast<__nv_bfloat16*>(ws + pl.sn);
+  float* partial = reinterpret_cast<float*>(ws + pl.partial);
+  __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(ws + pl.h);
+  uint8_t* att = ws + pl.att;
+  RowArgs row = {};
+  row.rows = n;
+  row.c = c_s;
+  row.eps = a->eps;
+  std::optional<SideStream> lease;
+  if (single) {
+    // (one block alone has only the projection to overlap: less than the fork and the join cost)
+    lease.emplace(stream, a->n_blocks > 1);
+    const b200tri_pairformer_block_params P = params_of(0);
+    row.base = a->s_in;
+    row.scale = P.pre_norm_s_scale;
+    row.bias = P.pre_norm_s_bias;
+    row.pieces = sn;
+    cudaStream_t st = lease->stream ? lease->stream : stream;
+    const b200tri_attention_pair_bias_args t = attention_args(P);
+    if ((rc = lease->fork()) || (rc = launch_row_norm(row, st, false)) || (rc = single_project(&t, sn, sn, att, st)) ||
+        (rc = lease->mark()))
+      return rc;
+  }
+
   PdlChain chain(false);
   for (int layer = 0; layer < a->n_blocks; ++layer) {
-    const b200tri_pairformer_block_params P =
-        a->stacked ? unstack(first, layer, c_s, a->heads_s) : a->params[layer];
-    int rc;
+    const b200tri_pairformer_block_params P = params_of(layer);
     // ---- pair track: the four triangle updates ping-pong between z_out and w (the first one
     // reads the caller's z_in), residual adds fused; with the pair gate, dropped pairs are
     // zeroed before the first update and after every update
@@ -274,45 +327,16 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     }
     z_cur = a->z_out;
     if (!single) continue;
+    SideStream& side = *lease;
 
-    // ---- single track, float32: s += attention(LN(s), z), s += transition(s), each sum taken
-    // by the row kernel that also normalises the rows for the product behind it
-    __nv_bfloat16* sn = reinterpret_cast<__nv_bfloat16*>(ws + pl.sn);
-    float* partial = reinterpret_cast<float*>(ws + pl.partial);
-    __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(ws + pl.h);
-    RowArgs row = {};
-    row.rows = n;
-    row.c = c_s;
-    row.eps = a->eps;
-    if (layer == 0) {
-      row.base = a->s_in;
-      row.scale = P.pre_norm_s_scale;
-      row.bias = P.pre_norm_s_bias;
-      row.pieces = sn;
-      if ((rc = launch_row_norm(row, stream, true))) return rc;
-    }
-    b200tri_attention_pair_bias_args t = {};
-    t.n = n;
-    t.c_s = c_s;
-    t.c_z = 128;
-    t.heads = a->heads_s;
-    t.eps = a->eps;
-    t.inf = a->att_inf;
-    t.z = a->z_out;
-    t.mask = token_mask;
-    t.proj_q = P.attention.proj_q;
-    t.proj_q_bias = P.attention.proj_q_bias;
-    t.proj_k = P.attention.proj_k;
-    t.proj_v = P.attention.proj_v;
-    t.proj_g = P.attention.proj_g;
-    t.proj_z_norm_scale = P.attention.proj_z_norm_scale;
-    t.proj_z_norm_bias = P.attention.proj_z_norm_bias;
-    t.proj_z = P.attention.proj_z;
-    t.proj_o = P.attention.proj_o;
+    // ---- single track; the last block's is on the caller's stream
+    const bool last = layer + 1 == a->n_blocks, forked = side.stream != nullptr;
+    const b200tri_attention_pair_bias_args t = attention_args(P);
+    if ((rc = side.join()) || (rc = single_pair_bias(&t, att, stream, !forked))) return rc;
+    if (!last && (rc = side.fork())) return rc;
+    cudaStream_t st = last || !forked ? stream : side.stream;
     int splits = 1;
-    if ((rc = single_project(&t, sn, sn, ws + pl.att, stream)) || (rc = single_pair_bias(&t, ws + pl.att, stream)) ||
-        (rc = single_attend(&t, ws + pl.att, partial, &splits, stream)))
-      return rc;
+    if ((rc = single_attend(&t, att, partial, &splits, st, last || !forked))) return rc;
     row.base = layer == 0 ? a->s_in : a->s_out;
     row.partial = partial;
     row.splits = splits;
@@ -321,27 +345,28 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     row.bias = P.transition_s.norm_bias;
     row.sum_out = a->s_out;
     row.pieces = sn;
-    if ((rc = launch_row_norm(row, stream, true))) return rc;
+    if ((rc = launch_row_norm(row, st, true))) return rc;
     // transition_s: LN -> fc1 | fc2 -> silu(fc1) * fc2 -> fc3, added to s (transition.py:99-112)
     const int hid = P.transition_s.hidden;
     const long long hp = round_up(hid, 8);
-    if ((rc = launch_swiglu(sn, n, c_s, P.transition_s.fc1, P.transition_s.fc2, hid, ws + pl.fc[0], ws + pl.fc[1], h, hp,
-                            stream, true)))
+    if ((rc = launch_swiglu(sn, n, c_s, P.transition_s.fc1, P.transition_s.fc2, hid, ws + pl.fc[0], ws + pl.fc[1], h, hp, st,
+                            true)))
       return rc;
-    if ((rc = launch_linear_partial(h, hp, n, hid, P.transition_s.fc3, c_s, ws + pl.fc[2], partial, &splits, stream, true)))
+    if ((rc = launch_linear_partial(h, hp, n, hid, P.transition_s.fc3, c_s, ws + pl.fc[2], partial, &splits, st, true)))
       return rc;
     row.base = a->s_out;
     row.splits = splits;
-    const bool last = layer + 1 == a->n_blocks;
-    if (!last) {
-      const b200tri_pairformer_block_params next =
-          a->stacked ? unstack(first, layer + 1, c_s, a->heads_s) : a->params[layer + 1];
-      row.scale = next.pre_norm_s_scale;
-      row.bias = next.pre_norm_s_bias;
-    } else {
+    if (last) {
       row.pieces = nullptr;
+      if ((rc = launch_row_norm(row, st, true))) return rc;
+      break;
     }
-    if ((rc = launch_row_norm(row, stream, true))) return rc;
+    const b200tri_pairformer_block_params next = params_of(layer + 1);
+    row.scale = next.pre_norm_s_scale;
+    row.bias = next.pre_norm_s_bias;
+    if ((rc = launch_row_norm(row, st, true))) return rc;
+    const b200tri_attention_pair_bias_args t_next = attention_args(next);
+    if ((rc = single_project(&t_next, sn, sn, att, st)) || (rc = side.mark())) return rc;
   }
   return B200TRI_OK;
 }

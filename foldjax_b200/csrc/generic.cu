@@ -950,6 +950,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       s.mask_bias = mb;
       s.scale = 1.0f;
       s.o = ws + pl.o;
+      s.pdl = true;
       if ((rc = launch_att_split(s, stream))) return rc;
     }
     {

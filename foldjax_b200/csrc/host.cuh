@@ -114,6 +114,25 @@ struct PdlChain {
 };
 bool pdl_chained();
 
+// A second stream for work of one call that does not depend on what the caller's stream does
+// meanwhile. Taken from a per-device pool for the duration of the call (several host threads
+// each get their own) and given back with the call's work enqueued: everything put on it is
+// ordered by events, so the next user may follow at once. `stream` is null when there is none to
+// be had or the caller's stream is being captured (a stream of the pool must not stay part of
+// somebody's capture), and the call stays on one stream.
+struct SideStream {
+  cudaStream_t main, stream = nullptr;
+  cudaEvent_t to_side = nullptr, to_main = nullptr;
+  bool joined = true;
+  SideStream(cudaStream_t main, bool want);
+  ~SideStream();  // joins if need be
+  SideStream(const SideStream&) = delete;
+  SideStream& operator=(const SideStream&) = delete;
+  int fork();  // what follows on the side stream comes after what is on the main stream now
+  int mark();  // `join` waits for what is on the side stream now
+  int join();  // what follows on the main stream comes after the last mark
+};
+
 // A weight as TMA needs it: `w` itself when it is 16-byte aligned, else a copy in `scratch`.
 int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stream, const void** out);
 

@@ -75,6 +75,80 @@ void PdlChain::set() { t_pdl_chain = true; }
 PdlChain::~PdlChain() { t_pdl_chain = before; }
 bool pdl_chained() { return t_pdl_chain; }
 
+namespace {
+struct SideEntry {
+  cudaStream_t stream;
+  cudaEvent_t to_side, to_main;
+};
+constexpr size_t SIDE_POOL = 8;  // idle entries kept per device; what exceeds them is destroyed
+std::mutex g_side_mu;
+std::vector<SideEntry> g_side[kMaxDevices];
+
+void destroy_side(const SideEntry& e) {
+  if (e.to_side) cudaEventDestroy(e.to_side);
+  if (e.to_main) cudaEventDestroy(e.to_main);
+  if (e.stream) cudaStreamDestroy(e.stream);  // (returns at once; the stream's work still completes)
+}
+}  // namespace
+
+SideStream::SideStream(cudaStream_t main_, bool want) : main(main_) {
+  if (!want) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(main, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+  std::vector<SideEntry>& pool = g_side[current_device_slot()];
+  SideEntry e = {};
+  {
+    std::lock_guard<std::mutex> lock(g_side_mu);
+    if (!pool.empty()) {
+      e = pool.back();
+      pool.pop_back();
+    }
+  }
+  if (!e.stream) {
+    if (cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e.to_side, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e.to_main, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      destroy_side(e);
+      return;
+    }
+  }
+  stream = e.stream;
+  to_side = e.to_side;
+  to_main = e.to_main;
+}
+SideStream::~SideStream() {
+  if (!stream) return;
+  if (!joined && mark() == B200TRI_OK) join();
+  const SideEntry e = {stream, to_side, to_main};
+  std::vector<SideEntry>& pool = g_side[current_device_slot()];
+  {
+    std::lock_guard<std::mutex> lock(g_side_mu);
+    if (pool.size() < SIDE_POOL) {
+      pool.push_back(e);
+      return;
+    }
+  }
+  destroy_side(e);
+}
+int SideStream::fork() {
+  if (!stream) return B200TRI_OK;
+  B200_CUDA_OK(cudaEventRecord(to_side, main));
+  B200_CUDA_OK(cudaStreamWaitEvent(stream, to_side, 0));
+  joined = false;
+  return B200TRI_OK;
+}
+int SideStream::mark() {
+  if (stream) B200_CUDA_OK(cudaEventRecord(to_main, stream));
+  return B200TRI_OK;
+}
+int SideStream::join() {
+  if (!stream || joined) return B200TRI_OK;
+  B200_CUDA_OK(cudaStreamWaitEvent(main, to_main, 0));
+  joined = true;
+  return B200TRI_OK;
+}
+
 int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stream, const void** out) {
   *out = w;
   if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) return B200TRI_OK;

@@ -49,8 +49,9 @@ SingleAttentionWork single_attention_work(int n, int c_s, int heads);
 int single_project(const b200tri_attention_pair_bias_args* a, const __nv_bfloat16* xq, const __nv_bfloat16* xk, uint8_t* work,
                    cudaStream_t stream);
 // the projected pair bias and the mask row (reads z and the token mask only);
-int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream);
+int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream, bool pdl);
 // partial[splits][n][c_s] = (g * softmax(q k^T / sqrt(d) + bias + mask) v) @ Wo.
-int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream);
+int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream,
+                  bool pdl);
 
 }  // namespace b200

@@ -578,7 +578,7 @@ int single_project(const b200tri_attention_pair_bias_args* a, const __nv_bfloat1
   return B200TRI_OK;
 }
 
-int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream) {
+int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, cudaStream_t stream, bool pdl) {
   const int n = a->n;
   const SingleAttentionWork off = single_attention_work(n, a->c_s, a->heads);
   const long long n_pairs = static_cast<long long>(n) * n;
@@ -609,10 +609,11 @@ int single_pair_bias(const b200tri_attention_pair_bias_args* a, uint8_t* work, c
   const long long tiles = (n_pairs + 127) / 128, slots = 2ll * sm_count();
   TimedLaunch timed(K_PAIR_BIAS, stream);
   return launch(pair_bias_kernel, dim3(static_cast<unsigned>(tiles < slots ? tiles : slots)), dim3(PB_THREADS), PB_SMEM, stream,
-                true, tm_z, p);
+                pdl, tm_z, p);
 }
 
-int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream) {
+int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, float* partial, int* splits, cudaStream_t stream,
+                  bool pdl) {
   const int n = a->n, c_s = a->c_s;
   const SingleAttentionWork off = single_attention_work(n, c_s, a->heads);
   AttSplitArgs s = {};
@@ -630,6 +631,7 @@ int single_attend(const b200tri_attention_pair_bias_args* a, uint8_t* work, floa
   s.scale = 1.0f / sqrtf(static_cast<float>(HD));
   s.gate = reinterpret_cast<float*>(work + off.g);
   s.pieces = reinterpret_cast<__nv_bfloat16*>(work + off.ao);
+  s.pdl = pdl;
   const int rc = launch_att_split(s, stream);
   if (rc) return rc;
   return launch_linear_partial(s.pieces, c_s, n, c_s, a->proj_o, c_s, work + off.w[4], partial, splits, stream, true);
@@ -700,8 +702,8 @@ extern "C" int b200tri_attention_pair_bias(const b200tri_attention_pair_bias_arg
     if ((rc = launch_row_norm(row, stream, false))) return rc;
   }
   int splits = 1;
-  if ((rc = single_project(a, xq, xk, ws + pl.work, stream)) || (rc = single_pair_bias(a, ws + pl.work, stream)) ||
-      (rc = single_attend(a, ws + pl.work, partial, &splits, stream)))
+  if ((rc = single_project(a, xq, xk, ws + pl.work, stream)) || (rc = single_pair_bias(a, ws + pl.work, stream, true)) ||
+      (rc = single_attend(a, ws + pl.work, partial, &splits, stream, true)))
     return rc;
   row.base = nullptr;
   row.partial = partial;
