@@ -1,11 +1,9 @@
-// Layer norm of one 128-channel pair held in a K-major, 128-byte-swizzled
-// operand tile (two 16 KiB slabs of 64 channels; row = pair). One thread owns
-// one row: it reads its 256 bytes, computes the statistics in fp32 exactly as
-// the reference does (mean, then mean of squared deviations, rsqrt(var + eps);
-// src/foldjax/models/boltz2/models/primitives/_common.py:15-26), rounds the
-// normalised value to bf16 before the affine step like the reference, and
-// writes the result back in place, so the tile TMA delivered becomes the
-// tensor-core operand without a second buffer.
+// Layer norm of 128-channel pairs held in a K-major, 128-byte-swizzled operand tile (two 16 KiB
+// slabs of 64 channels; row = pair). Statistics in fp32 as the reference takes them (mean, then mean
+// of squared deviations, rsqrt(var + eps); src/foldjax/models/boltz2/models/primitives/
+// _common.py:15-26), the normalised value rounded to bf16 before the affine step like the
+// reference, the result written back in place: the tile TMA delivered becomes the tensor-core
+// operand without a second buffer. The fp32 arithmetic runs two channels an instruction.
 #pragma once
 #include "tc.cuh"
 
@@ -19,87 +17,85 @@ __device__ __forceinline__ uint32_t ln_param_pair(const void* p, int i) {
   return static_cast<uint32_t>(h[0]) | (static_cast<uint32_t>(h[1]) << 16);
 }
 
+// The operations below and their order are part of the result: a statistic that differs in its last
+// bit flips some roundings to bf16 later on, and a stack of blocks amplifies those. Where two
+// operations of the same kind are independent they share an instruction.
+
+// bf16 pair -> float pair
+__device__ __forceinline__ float2 ln_unpack(uint32_t w) { return make_float2(bf16_lo(w), bf16_hi(w)); }
+// normed.astype(bf16) * scale + bias, each step rounded to bf16
+__device__ __forceinline__ uint32_t ln_affine(uint32_t w, float2 minus_mean, float2 rstd, uint32_t gamma, uint32_t beta) {
+  const float2 n = __fmul2_rn(__fadd2_rn(ln_unpack(w), minus_mean), rstd);
+  return bf16x2_add(bf16x2_mul(pack_bf16x2(n.x, n.y), gamma), beta);
+}
+// One step of each statistic in one accumulator: a word's two channels are added to each other
+// first; their squared deviations one after the other.
+__device__ __forceinline__ float ln_add4(float sum, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+  const float2 a = __fadd2_rn(make_float2(bf16_lo(w0), bf16_lo(w1)), make_float2(bf16_hi(w0), bf16_hi(w1)));
+  const float2 b = __fadd2_rn(make_float2(bf16_lo(w2), bf16_lo(w3)), make_float2(bf16_hi(w2), bf16_hi(w3)));
+  return (((sum + a.x) + a.y) + b.x) + b.y;
+}
+__device__ __forceinline__ float ln_square(float sq, uint32_t w, float2 minus_mean) {
+  const float2 d = __fadd2_rn(ln_unpack(w), minus_mean);
+  return fmaf(d.y, d.y, fmaf(d.x, d.x, sq));
+}
+
+// One thread per row, the row's 64 packed words in registers. gamma2 / beta2: scale and bias as
+// 64 packed bf16 pairs in shared memory, 16-byte aligned (every thread reads the same address, a
+// broadcast).
+__device__ __forceinline__ void ln_row_words(uint4 (&v)[16], const uint32_t* gamma2, const uint32_t* beta2, float eps) {
+  float sum = 0.f, sq = 0.f;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) sum = ln_add4(sum, v[c].x, v[c].y, v[c].z, v[c].w);
+  const float mean = sum * (1.0f / 128.0f);
+  const float2 mm = make_float2(-mean, -mean);
+#pragma unroll
+  for (int c = 0; c < 16; ++c) sq = ln_square(ln_square(ln_square(ln_square(sq, v[c].x, mm), v[c].y, mm), v[c].z, mm), v[c].w, mm);
+  const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
+  const float2 rr = make_float2(rstd, rstd);
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    const uint4 g = reinterpret_cast<const uint4*>(gamma2)[c], b = reinterpret_cast<const uint4*>(beta2)[c];
+    v[c] = make_uint4(ln_affine(v[c].x, mm, rr, g.x, b.x), ln_affine(v[c].y, mm, rr, g.y, b.y),
+                      ln_affine(v[c].z, mm, rr, g.z, b.z), ln_affine(v[c].w, mm, rr, g.w, b.w));
+  }
+}
 // v[0..7] = slab 0 chunks, v[8..15] = slab 1 chunks (16 bytes = 8 channels each).
 __device__ __forceinline__ void ln_load_row(const uint8_t* tile, int row, uint4 (&v)[16]) {
 #pragma unroll
-  for (int s = 0; s < 2; ++s)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) v[s * 8 + c] = *reinterpret_cast<const uint4*>(tile + s * SLAB_BYTES + sw128_offset(row, c));
+  for (int c = 0; c < 16; ++c) v[c] = *reinterpret_cast<const uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
 }
-
 __device__ __forceinline__ void ln_store_row(uint8_t* tile, int row, const uint4 (&v)[16]) {
 #pragma unroll
-  for (int s = 0; s < 2; ++s)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tile + s * SLAB_BYTES + sw128_offset(row, c)) = v[s * 8 + c];
+  for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7)) = v[c];
 }
 
-// In-register layer norm of the 128 bf16 values packed in v. gamma2/beta2 are
-// the scale and bias as 64 packed bf16 pairs in shared memory (every thread
-// reads the same address, a broadcast).
-__device__ __forceinline__ void ln_rows_inplace(uint4 (&v)[16], const uint32_t* gamma2, const uint32_t* beta2,
-                                                float eps) {
-  uint32_t* w = reinterpret_cast<uint32_t*>(v);  // 64 words, 2 channels each
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < 64; ++i) sum += bf16_lo(w[i]) + bf16_hi(w[i]);
-  const float mean = sum * (1.0f / 128.0f);
-  float sq = 0.f;
-#pragma unroll
-  for (int i = 0; i < 64; ++i) {
-    const float a = bf16_lo(w[i]) - mean, b = bf16_hi(w[i]) - mean;
-    sq = fmaf(a, a, sq);
-    sq = fmaf(b, b, sq);
-  }
-  const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
-#pragma unroll
-  for (int i = 0; i < 64; ++i) {
-    const float a = (bf16_lo(w[i]) - mean) * rstd;
-    const float b = (bf16_hi(w[i]) - mean) * rstd;
-    // normed.astype(bf16) * scale + bias, each step rounded to bf16
-    w[i] = bf16x2_add(bf16x2_mul(pack_bf16x2(a, b), gamma2[i]), beta2[i]);
-  }
-}
-
-// The same layer norm (same operations in the same order, so the same bits) as three
-// sweeps over the row in shared memory - mean, variance, normalise - holding four words
-// at a time instead of the whole row: for kernels whose other roles leave the
-// layer-norm warps few registers.
+// The same layer norm (the same bits) as three sweeps over the row in shared memory - mean,
+// variance, normalise - holding four words at a time instead of the whole row: for kernels whose
+// other roles leave the layer-norm warps few registers.
 __device__ __forceinline__ void ln_row_sweeps(uint8_t* tile, int row, const uint32_t* gamma2, const uint32_t* beta2,
                                               float eps) {
-  float sum = 0.f;
+  float sum = 0.f, sq = 0.f;
 #pragma unroll 4
   for (int c = 0; c < 16; ++c) {
     const uint4 v = *reinterpret_cast<const uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) sum += bf16_lo(w[e]) + bf16_hi(w[e]);
+    sum = ln_add4(sum, v.x, v.y, v.z, v.w);
   }
   const float mean = sum * (1.0f / 128.0f);
-  float sq = 0.f;
+  const float2 mm = make_float2(-mean, -mean);
 #pragma unroll 4
   for (int c = 0; c < 16; ++c) {
     const uint4 v = *reinterpret_cast<const uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float a = bf16_lo(w[e]) - mean, b = bf16_hi(w[e]) - mean;
-      sq = fmaf(a, a, sq);
-      sq = fmaf(b, b, sq);
-    }
+    sq = ln_square(ln_square(ln_square(ln_square(sq, v.x, mm), v.y, mm), v.z, mm), v.w, mm);
   }
   const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
+  const float2 rr = make_float2(rstd, rstd);
 #pragma unroll 4
   for (int c = 0; c < 16; ++c) {
     uint4* ptr = reinterpret_cast<uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
-    const uint4 v = *ptr;
-    uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float a = (bf16_lo(w[e]) - mean) * rstd, b = (bf16_hi(w[e]) - mean) * rstd;
-      w[e] = bf16x2_add(bf16x2_mul(pack_bf16x2(a, b), gamma2[4 * c + e]), beta2[4 * c + e]);
-    }
-    *ptr = make_uint4(w[0], w[1], w[2], w[3]);
+    const uint4 v = *ptr, g = reinterpret_cast<const uint4*>(gamma2)[c], b = reinterpret_cast<const uint4*>(beta2)[c];
+    *ptr = make_uint4(ln_affine(v.x, mm, rr, g.x, b.x), ln_affine(v.y, mm, rr, g.y, b.y), ln_affine(v.z, mm, rr, g.z, b.z),
+                      ln_affine(v.w, mm, rr, g.w, b.w));
   }
 }
 
@@ -107,37 +103,44 @@ __device__ __forceinline__ void ln_row_sweeps(uint8_t* tile, int row, const uint
 // rows; `half` = l >> 4 takes the 64 channels of slab `half`, and the two partial sums
 // meet through one shuffle each. Half the instructions and half the dependency chain
 // per thread, and twice the warps: the layer norm is what a projection tile waits for.
-// Must be called by all 32 lanes of the warp. Same rounding points as ln_rows_inplace;
+// Must be called by all 32 lanes of the warp. Same rounding points as ln_row_words;
 // the fp32 statistics are summed in a different order (four partial sums per thread).
 __device__ __forceinline__ void ln_row_two_threads(uint8_t* tile, int row, int half, const uint32_t* gamma2,
                                                    const uint32_t* beta2, float eps) {
   uint4 v[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const uint4*>(tile + half * SLAB_BYTES + sw128_offset(row, c));
-  uint32_t* w = reinterpret_cast<uint32_t*>(v);  // 32 words, 2 channels each
-  float s4[4] = {0.f, 0.f, 0.f, 0.f};
+  float2 s[2] = {}, q[2] = {};  // the four partial sums: words 0, 1 | 2, 3 of each chunk
 #pragma unroll
-  for (int i = 0; i < 32; ++i) s4[i & 3] += bf16_lo(w[i]) + bf16_hi(w[i]);
-  float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+  for (int c = 0; c < 8; ++c) {
+    s[0] = __fadd2_rn(s[0], __fadd2_rn(make_float2(bf16_lo(v[c].x), bf16_lo(v[c].y)), make_float2(bf16_hi(v[c].x), bf16_hi(v[c].y))));
+    s[1] = __fadd2_rn(s[1], __fadd2_rn(make_float2(bf16_lo(v[c].z), bf16_lo(v[c].w)), make_float2(bf16_hi(v[c].z), bf16_hi(v[c].w))));
+  }
+  float sum = (s[0].x + s[0].y) + (s[1].x + s[1].y);
   sum += __shfl_xor_sync(0xffffffffu, sum, 16);
   const float mean = sum * (1.0f / 128.0f);
-  float q4[4] = {0.f, 0.f, 0.f, 0.f};
+  const float2 mm = make_float2(-mean, -mean);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const float a = bf16_lo(w[i]) - mean, b = bf16_hi(w[i]) - mean;
-    q4[i & 3] = fmaf(a, a, q4[i & 3]);
-    q4[i & 3] = fmaf(b, b, q4[i & 3]);
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float2 a = __fadd2_rn(make_float2(bf16_lo(w[2 * u]), bf16_lo(w[2 * u + 1])), mm);
+      const float2 b = __fadd2_rn(make_float2(bf16_hi(w[2 * u]), bf16_hi(w[2 * u + 1])), mm);
+      q[u] = __ffma2_rn(b, b, __ffma2_rn(a, a, q[u]));
+    }
   }
-  float sq = (q4[0] + q4[1]) + (q4[2] + q4[3]);
+  float sq = (q[0].x + q[0].y) + (q[1].x + q[1].y);
   sq += __shfl_xor_sync(0xffffffffu, sq, 16);
   const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
+  const float2 rr = make_float2(rstd, rstd);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const float a = (bf16_lo(w[i]) - mean) * rstd, b = (bf16_hi(w[i]) - mean) * rstd;
-    w[i] = bf16x2_add(bf16x2_mul(pack_bf16x2(a, b), gamma2[half * 32 + i]), beta2[half * 32 + i]);
+  for (int c = 0; c < 8; ++c) {
+    const uint4 g = reinterpret_cast<const uint4*>(gamma2)[half * 8 + c], b = reinterpret_cast<const uint4*>(beta2)[half * 8 + c];
+    *reinterpret_cast<uint4*>(tile + half * SLAB_BYTES + sw128_offset(row, c)) =
+        make_uint4(ln_affine(v[c].x, mm, rr, g.x, b.x), ln_affine(v[c].y, mm, rr, g.y, b.y),
+                   ln_affine(v[c].z, mm, rr, g.z, b.z), ln_affine(v[c].w, mm, rr, g.w, b.w));
   }
-#pragma unroll
-  for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tile + half * SLAB_BYTES + sw128_offset(row, c)) = v[c];
 }
 
 }  // namespace b200

@@ -51,7 +51,7 @@ struct Smem {
   uint8_t w3[WSTAGES][SLAB_BYTES];       // fc3 of the chunk: two boxes [64 hidden][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
   uint8_t h[SLAB_BYTES];                 // [128 pairs][64 hidden]
-  uint32_t gamma2[64], beta2[64];
+  alignas(16) uint32_t gamma2[64], beta2[64];
   uint64_t w_full[WSTAGES], w_empty[WSTAGES], x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES];
   uint64_t d1_full[2], d1_empty[2], h_full, h_empty, out_full[2], out_empty[2];
   uint32_t tmem_base;

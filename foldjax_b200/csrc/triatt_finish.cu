@@ -10,14 +10,15 @@
 // frame; x and out are addressed as base + o*stride_outer + t*stride_inner.
 //
 // One tile = 128 consecutive pairs. Persistent, one CTA per SM:
-//   warp 0      TMA producer (Wg, Wo once; x and o tiles, 2-stage ring)
-//   warp 1      MMA issuer: G = LN(x).Wg^T, then OUT = (o*g).Wo^T
-//   warps 2-5   layer norm of x in place, then the gating of o in place
-//               (the o tile becomes the A operand of the second product)
-//   warps 6-9   epilogue of OUT
-// The gating of tile t is done after the layer norm of tile t+1, so the first
-// product of the next tile runs while this tile is gated.
-// Bound: HBM (read x and o, write out: 3 * n*n*128*2 bytes; + residual).
+//   warp 0       TMA producer (Wg, Wo once; x tiles in a 2-stage ring, o tiles in a 3-stage ring)
+//   warp 1       MMA issuer: G = LN(x).Wg^T, then OUT = (o*g).Wo^T
+//   warps 2-5    layer norm of x in place, one thread per pair
+//   warps 6-9    gating of o in place, one thread per pair (the o tile becomes the A operand of the
+//                second product)
+//   warps 10-17  epilogue of OUT, 64 channels per warpgroup: residual fetched before the product
+//                is waited for, sum staged in the o tile (dead by then), one TMA store per warpgroup
+// Bound: HBM (read x and o, write out: 3 * n*n*128*2 bytes; + residual) - once enough warps
+// hide the latencies of TMEM and of the row-wise accesses.
 #include "host.cuh"
 #include "ln.cuh"
 #include "tc.cuh"
@@ -26,26 +27,17 @@ namespace b200 {
 
 namespace {
 
-constexpr int STAGES = 2;
+constexpr int XSTAGES = 2, OSTAGES = 3;  // an x tile is free after the first product, an o tile once it is stored
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
-constexpr int THREADS = 320;
-constexpr int EPI_THREAD0 = 192;  // first thread of the epilogue warps
-// 1: the epilogue stages the output tile in shared memory ([128 pairs][128 channels] as two
-// swizzled slabs) and writes it with two TMA stores through the caller's strides; 0: every
-// thread stores its pair's row itself, 64 bytes at a time (32 cache lines per warp store).
-#ifndef B200_AFIN_TMASTORE
-#define B200_AFIN_TMASTORE 1
-#endif
+constexpr int LN_WARPS = 4, GATE_WARPS = 4, EPI_WARPS = 8;
+constexpr int THREADS = 64 + (LN_WARPS + GATE_WARPS + EPI_WARPS) * 32;
 
 struct Smem {
   uint8_t w[4 * SLAB_BYTES];  // Wg, Wo: two boxes [128 in][64 out] each, MN-major
-  uint8_t x[STAGES][TILE_BYTES];
-  uint8_t o[STAGES][TILE_BYTES];
-#if B200_AFIN_TMASTORE
-  uint8_t out[TILE_BYTES];
-#endif
-  uint32_t gamma2[64], beta2[64];
-  uint64_t w_full, in_full[STAGES], xn_full[STAGES], y_full[STAGES], in_empty[STAGES];
+  uint8_t x[XSTAGES][TILE_BYTES];
+  uint8_t o[OSTAGES][TILE_BYTES];
+  alignas(16) uint32_t gamma2[64], beta2[64];
+  uint64_t w_full, x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES], o_full[OSTAGES], y_full[OSTAGES], o_empty[OSTAGES];
   uint64_t g_full[2], g_empty[2], out_full[2], out_empty[2];
   uint32_t tmem_base;
 };
@@ -53,12 +45,11 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 
 struct Params {
   int n_outer, n_inner, tiles_inner;
-  long long total_tiles;
+  uint32_t total_tiles;
   const void* gamma;
   const void* beta;
   bool early_weights;  // the weights may be read before pdl_wait()
   const __nv_bfloat16* residual;
-  __nv_bfloat16* out;
   long long os_outer, os_inner;
   float eps;
   int* status;
@@ -82,17 +73,21 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     tma_prefetch_desc(&tm_wg);
     tma_prefetch_desc(&tm_wo);
     mbar_init(&sm.w_full, 1);
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&sm.in_full[s], 1);
-      mbar_init(&sm.xn_full[s], 128);
-      mbar_init(&sm.y_full[s], 128);
-      mbar_init(&sm.in_empty[s], 1);
+    for (int s = 0; s < XSTAGES; ++s) {
+      mbar_init(&sm.x_full[s], 1);
+      mbar_init(&sm.xn_full[s], LN_WARPS);
+      mbar_init(&sm.x_empty[s], 1);
+    }
+    for (int s = 0; s < OSTAGES; ++s) {
+      mbar_init(&sm.o_full[s], 1);
+      mbar_init(&sm.y_full[s], GATE_WARPS);
+      mbar_init(&sm.o_empty[s], 2);  // the two warpgroups' stores
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sm.g_full[a], 1);
-      mbar_init(&sm.g_empty[a], 4);
+      mbar_init(&sm.g_empty[a], GATE_WARPS);
       mbar_init(&sm.out_full[a], 1);
-      mbar_init(&sm.out_empty[a], 4);
+      mbar_init(&sm.out_empty[a], EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -119,23 +114,29 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   if (p.early_weights) pdl_wait();
   pdl_trigger();
 
+  // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
+  auto locate = [&](uint32_t tile, int& o, int& t0) {
+    const uint32_t q = tile / static_cast<uint32_t>(p.tiles_inner);
+    o = q;
+    t0 = (tile - q * p.tiles_inner) * 128;
+  };
+  const uint32_t n_my = blockIdx.x < p.total_tiles ? (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-        const int o = static_cast<int>(tile / p.tiles_inner);
-        const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
-        if (!mbar_wait(&sm.in_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.in_full[stage], 2 * TILE_BYTES);
-        tma_load_3d(sm.x[stage], &tm_x, &sm.in_full[stage], 0, t0, o);
-        tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.in_full[stage], 64, t0, o);
-        tma_load_3d(sm.o[stage], &tm_o, &sm.in_full[stage], 0, t0, o);
-        tma_load_3d(sm.o[stage] + SLAB_BYTES, &tm_o, &sm.in_full[stage], 64, t0, o);
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
+      uint32_t it = 0;
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+        int o, t0;
+        locate(tile, o, t0);
+        const uint32_t xs = it % XSTAGES, os = it % OSTAGES;
+        if (!mbar_wait(&sm.x_empty[xs], ((it / XSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
+        tma_load_3d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, t0, o);
+        tma_load_3d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, t0, o);
+        if (!mbar_wait(&sm.o_empty[os], ((it / OSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        mbar_expect_tx(&sm.o_full[os], TILE_BYTES);
+        tma_load_3d(sm.o[os], &tm_o, &sm.o_full[os], 0, t0, o);
+        tma_load_3d(sm.o[os] + SLAB_BYTES, &tm_o, &sm.o_full[os], 64, t0, o);
       }
     }
   } else if (warp == 1) {
@@ -152,158 +153,141 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           umma_bf16_ss(d_tmem, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc, k != 0);
         }
       };
-      long long n_my = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) ++n_my;
-      for (long long it = 0; it <= n_my && alive; ++it) {
+      for (uint32_t it = 0; it <= n_my && alive; ++it) {
         if (it < n_my) {  // first product of tile `it`
-          const int stage = static_cast<int>(it % STAGES);
-          const uint32_t phase = static_cast<uint32_t>((it / STAGES) & 1);
+          const uint32_t stage = it % XSTAGES, phase = (it / XSTAGES) & 1;
           const uint32_t a = static_cast<uint32_t>(it & 1), aph = static_cast<uint32_t>((it >> 1) & 1);
           if (!mbar_wait(&sm.g_empty[a], aph ^ 1, p.status, ST_TIMEOUT_MMA)) break;
           if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
           product(tmem_base + a * 256, smem_u32(sm.x[stage]), 0);
+          umma_commit(&sm.x_empty[stage]);
           umma_commit(&sm.g_full[a]);
         }
         if (it > 0) {  // second product of tile `it - 1`
-          const long long jt = it - 1;
-          const int stage = static_cast<int>(jt % STAGES);
-          const uint32_t phase = static_cast<uint32_t>((jt / STAGES) & 1);
+          const uint32_t jt = it - 1;
+          const uint32_t stage = jt % OSTAGES, phase = (jt / OSTAGES) & 1;
           const uint32_t a = static_cast<uint32_t>(jt & 1), aph = static_cast<uint32_t>((jt >> 1) & 1);
           if (!mbar_wait(&sm.out_empty[a], aph ^ 1, p.status, ST_TIMEOUT_MMA)) break;
           if (!mbar_wait(&sm.y_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
           product(tmem_base + a * 256 + 128, smem_u32(sm.o[stage]), 1);
-          umma_commit(&sm.in_empty[stage]);
           umma_commit(&sm.out_full[a]);
         }
       }
     }
-  } else if (warp < 6) {
-    const int r = threadIdx.x - 64;
-    const int quarter = warp & 3;
-    // This thread's TMEM lane must be its warp's quarter; rows are assigned so
-    // that thread r handles tile row `row`.
-    const int row = quarter * 32 + lane;
+  } else if (warp < 2 + LN_WARPS) {
+    const int row = (warp - 2) * 32 + lane;
+    for (uint32_t it = 0; it < n_my; ++it) {
+      const uint32_t stage = it % XSTAGES, phase = (it / XSTAGES) & 1;
+      if (!mbar_wait(&sm.x_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
+      ln_row_sweeps(sm.x[stage], row, sm.gamma2, sm.beta2, p.eps);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
+    }
+  } else if (warp < 2 + LN_WARPS + GATE_WARPS) {  // o <- bf16(o * bf16(sigmoid(bf16(G))))
+    const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    (void)r;
-    long long n_my = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) ++n_my;
-    bool alive = true;
-    for (long long it = 0; it <= n_my && alive; ++it) {
-      if (it < n_my) {  // layer norm of tile `it`
-        const int stage = static_cast<int>(it % STAGES);
-        const uint32_t phase = static_cast<uint32_t>((it / STAGES) & 1);
-        if (!mbar_wait(&sm.in_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-        uint4 v[16];
-        ln_load_row(sm.x[stage], row, v);
-        ln_rows_inplace(v, sm.gamma2, sm.beta2, p.eps);
-        ln_store_row(sm.x[stage], row, v);
-        fence_proxy_async();
-        mbar_arrive(&sm.xn_full[stage]);
-      }
-      if (it > 0) {  // gating of tile `it - 1`: o <- bf16(o * bf16(sigmoid(bf16(G))))
-        const long long jt = it - 1;
-        const int stage = static_cast<int>(jt % STAGES);
-        const uint32_t a = static_cast<uint32_t>(jt & 1), aph = static_cast<uint32_t>((jt >> 1) & 1);
-        if (!mbar_wait(&sm.g_full[a], aph, p.status, ST_TIMEOUT_PROLOGUE)) break;
-        tc_fence_after();
-        uint8_t* otile = sm.o[stage];
+    for (uint32_t it = 0; it < n_my; ++it) {
+      const uint32_t stage = it % OSTAGES, phase = (it / OSTAGES) & 1;
+      const uint32_t a = it & 1, aph = (it >> 1) & 1;
+      if (!mbar_wait(&sm.o_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE) ||
+          !mbar_wait(&sm.g_full[a], aph, p.status, ST_TIMEOUT_PROLOGUE))
+        break;
+      __syncwarp();
+      tc_fence_after();
 #pragma unroll 1
-        for (int chunk = 0; chunk < 4; ++chunk) {  // 32 channels = 4 sixteen-byte chunks of one slab
-          uint32_t g[32];
-          tmem_ld32(lane_addr + a * 256 + chunk * 32, g);
-          tmem_ld_wait();
-          const int slab = chunk >> 1;
+      for (int chunk = 0; chunk < 4; ++chunk) {  // 32 channels = 4 sixteen-byte chunks of one slab
+        uint32_t g[32];
+        tmem_ld32(lane_addr + a * 256 + chunk * 32, g);
+        tmem_ld_wait();
 #pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            const int c = (chunk & 1) * 4 + c4;  // chunk index inside the slab
-            uint4* ptr = reinterpret_cast<uint4*>(otile + slab * SLAB_BYTES + sw128_offset(row, c));
-            uint4 ov = *ptr;
-            ov.x = bf16x2_mul(ov.x, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 0]), __uint_as_float(g[8 * c4 + 1])));
-            ov.y = bf16x2_mul(ov.y, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 2]), __uint_as_float(g[8 * c4 + 3])));
-            ov.z = bf16x2_mul(ov.z, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 4]), __uint_as_float(g[8 * c4 + 5])));
-            ov.w = bf16x2_mul(ov.w, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 6]), __uint_as_float(g[8 * c4 + 7])));
-            *ptr = ov;
-          }
+        for (int c4 = 0; c4 < 4; ++c4) {
+          uint4* ptr = reinterpret_cast<uint4*>(sm.o[stage] + (chunk >> 1) * SLAB_BYTES + sw128_offset(row, (chunk & 1) * 4 + c4));
+          uint4 ov = *ptr;
+          ov.x = bf16x2_mul(ov.x, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 0]), __uint_as_float(g[8 * c4 + 1])));
+          ov.y = bf16x2_mul(ov.y, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 2]), __uint_as_float(g[8 * c4 + 3])));
+          ov.z = bf16x2_mul(ov.z, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 4]), __uint_as_float(g[8 * c4 + 5])));
+          ov.w = bf16x2_mul(ov.w, sigmoid_bf16x2(__uint_as_float(g[8 * c4 + 6]), __uint_as_float(g[8 * c4 + 7])));
+          *ptr = ov;
         }
-        tc_fence_before();
-        fence_proxy_async();
+      }
+      tc_fence_before();
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
         mbar_arrive(&sm.y_full[stage]);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.g_empty[a]);
+        mbar_arrive(&sm.g_empty[a]);
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, half = (warp - 2 - LN_WARPS - GATE_WARPS) >> 2;  // 64 channels per warpgroup
     const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 128 + half * 64;
     uint32_t it = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
-      const int o = static_cast<int>(tile / p.tiles_inner);
-      const int t = static_cast<int>(tile % p.tiles_inner) * 128 + row;
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      int o, t0;
+      locate(tile, o, t0);
       const uint32_t a = it & 1, aph = (it >> 1) & 1;
-#if B200_AFIN_TMASTORE
-      // the previous tile must have left the staging buffer; the vote makes the outcome of the
-      // bounded wait the same for all 128 threads, which meet at a barrier below
-      if (threadIdx.x == EPI_THREAD0) tma_store_wait_read();
-      if (!named_barrier_and(1, 128, mbar_wait(&sm.out_full[a], aph, p.status, ST_TIMEOUT_EPILOGUE))) break;
-#else
-      if (!mbar_wait(&sm.out_full[a], aph, p.status, ST_TIMEOUT_EPILOGUE)) break;
-#endif
+      uint8_t* stage_out = sm.o[it % OSTAGES] + half * SLAB_BYTES;
+      uint4 res[8];  // residual of the warp's 32 pairs, 8 lanes to a pair's 64 channels (whole lines)
+      if (p.residual) {
+        const int t = t0 + quarter * 32 + (lane >> 3);
+        const __nv_bfloat16* src = p.residual + static_cast<long long>(o) * p.os_outer + half * 64 + (lane & 7) * 8;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          res[q] = t + 4 * q < p.n_inner ? *reinterpret_cast<const uint4*>(src + static_cast<long long>(t + 4 * q) * p.os_inner)
+                                      : make_uint4(0u, 0u, 0u, 0u);
+      }
+      // (the vote makes the outcome of the bounded wait the same for all 128 threads, which meet at
+      // a barrier below)
+      if (!named_barrier_and(1 + half, 128, mbar_wait(&sm.out_full[a], aph, p.status, ST_TIMEOUT_EPILOGUE))) break;
       tc_fence_after();
-      const long long off = static_cast<long long>(o) * p.os_outer + static_cast<long long>(t) * p.os_inner;
-#pragma unroll 1
+#pragma unroll
       for (int chunk = 0; chunk < 4; ++chunk) {
-        uint32_t v[32];
-        tmem_ld32(lane_addr + a * 256 + 128 + chunk * 32, v);
+        uint32_t v[16];
+        tmem_ld16(lane_addr + a * 256 + chunk * 16, v);
         tmem_ld_wait();
-        if (t < p.n_inner) {
-#if !B200_AFIN_TMASTORE
-          uint4* dst = reinterpret_cast<uint4*>(p.out + off + chunk * 32);
-#endif
-          const uint4* res = p.residual ? reinterpret_cast<const uint4*>(p.residual + off + chunk * 32) : nullptr;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t u[4];
+        for (int q = 0; q < 2; ++q) {
+          uint32_t u[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
-            if (res) {
-              const uint4 rv = res[q];
-              u[0] = bf16x2_add(rv.x, u[0]);
-              u[1] = bf16x2_add(rv.y, u[1]);
-              u[2] = bf16x2_add(rv.z, u[2]);
-              u[3] = bf16x2_add(rv.w, u[3]);
-            }
-#if B200_AFIN_TMASTORE
-            *reinterpret_cast<uint4*>(sm.out + (chunk >> 1) * SLAB_BYTES + sw128_offset(row, (chunk & 1) * 4 + q)) =
-                make_uint4(u[0], u[1], u[2], u[3]);
-#else
-            dst[q] = make_uint4(u[0], u[1], u[2], u[3]);
-#endif
-          }
+          for (int e = 0; e < 4; ++e)
+            u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
+          *reinterpret_cast<uint4*>(stage_out + sw128_offset(row, chunk * 2 + q)) = make_uint4(u[0], u[1], u[2], u[3]);
         }
       }
-#if B200_AFIN_TMASTORE
+      if (p.residual) {  // the caller's z + update, one more bf16 rounding, in the residual's arrangement
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          uint4* ptr = reinterpret_cast<uint4*>(stage_out + sw128_offset(quarter * 32 + 4 * q + (lane >> 3), lane & 7));
+          uint4 u = *ptr;
+          u.x = bf16x2_add(res[q].x, u.x);
+          u.y = bf16x2_add(res[q].y, u.y);
+          u.z = bf16x2_add(res[q].z, u.z);
+          u.w = bf16x2_add(res[q].w, u.w);
+          *ptr = u;
+        }
+      }
+      tc_fence_before();
       fence_proxy_async();
-      named_barrier(1, 128);
-      if (threadIdx.x == EPI_THREAD0) {  // rows past n_inner are outside the tensor and are not written
-        const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
-        tma_store_3d(&tm_out, sm.out, 0, t0, o);
-        tma_store_3d(&tm_out, sm.out + SLAB_BYTES, 64, t0, o);
+      named_barrier(1 + half, 128);
+      if (leader) {  // rows past n_inner are outside the tensor and are not written
+        tma_store_3d(&tm_out, stage_out, half * 64, t0, o);
         tma_store_commit();
       }
-#endif
-      tc_fence_before();
-      __syncwarp();
       if (lane == 0) mbar_arrive(&sm.out_empty[a]);
+      if (leader) {
+        tma_store_wait_read();
+        mbar_arrive(&sm.o_empty[it % OSTAGES]);
+      }
     }
+    if (leader) tma_store_wait_all();
   }
 
-#if B200_AFIN_TMASTORE
-  if (threadIdx.x == EPI_THREAD0) tma_store_wait_all();
-#endif
   if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
     for (int i = 0; i < 100; ++i) __nanosleep(1000);
   tc_fence_before();
@@ -371,12 +355,13 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
   p.n_outer = a->n_outer;
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
-  p.total_tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  const long long tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "att finish: too many tiles (%lld)", tiles);
+  p.total_tiles = static_cast<uint32_t>(tiles);
   p.gamma = a->norm_scale;
   p.beta = a->norm_bias;
   p.early_weights = pdl_chained() && w_g == a->w_g && w_o == a->w_o;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
-  p.out = static_cast<__nv_bfloat16*>(a->out);
   p.os_outer = a->os_outer;
   p.os_inner = a->os_inner;
   p.eps = a->eps;
@@ -386,7 +371,7 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_finish_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const long long grid = tiles < sm_count() ? tiles : sm_count();
   {
     TimedLaunch timed(K_TRIATT_FINISH, stream);
     return launch(att_finish_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_o,

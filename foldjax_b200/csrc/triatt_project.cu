@@ -22,11 +22,12 @@
 // projection of order one, so only the exact range matters in practice.
 //
 // One tile = 128 consecutive pairs (o, t0..t0+127). Persistent, one CTA per SM:
-//   warp 0      TMA producer (weights once, x tiles in a 3-stage ring)
+//   warp 0      TMA producer (weights once, x tiles in a 2-stage ring)
 //   warp 1      MMA issuer: [q|k] = xn.[Wq|Wk]^T (N=256), bias = xn.Wb^T (N=16),
 //               vT = Wv.xn^T ("transposed": a TMEM lane is a channel)
 //   warps 2-9   layer norm in place (two threads per pair)
-//   warps 10-13 epilogue
+//   warps 10-17 epilogue: one warpgroup per 64 channels of q and k and per 64 pairs of vT, each
+//               with a staging slab and TMA stores of its own
 // TMEM: [q|k] 256 columns, vT 128, bias 16; each group is released on its own
 // so the next tile's MMAs overlap this tile's epilogue.
 // Bound: HBM (read x, write q, k, vT: 4 * n*n*128*2 bytes).
@@ -40,23 +41,12 @@ namespace b200 {
 
 namespace {
 
-// 1: q, k and vT tiles are staged in shared memory and written with TMA stores (one elected
-// thread, two 16 KiB boxes each); 0: every thread stores its row's 64-byte pieces itself, so a
-// warp's store instruction touches 32 cache lines and the L1 pipe bounds the kernel.
-#ifndef B200_APROJ_TMASTORE
-#define B200_APROJ_TMASTORE 1
-#endif
-#if B200_APROJ_TMASTORE
 constexpr int XSTAGES = 2;
-#else
-constexpr int XSTAGES = 3;
-#endif
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
 constexpr int W_BYTES = 6 * SLAB_BYTES;  // Wq, Wk, Wv: two boxes [128 in][64 out] each, MN-major
 constexpr int WB_SLAB = 16 * 128;        // Wb, K-major: [16 heads (4 used)][64 in], two slabs
-constexpr int LN_WARPS = 8;  // two threads per pair
-constexpr int THREADS = 64 + LN_WARPS * 32 + 128;
-constexpr int EPI_THREAD0 = 64 + LN_WARPS * 32;  // first thread of the epilogue warps
+constexpr int LN_WARPS = 8, EPI_WARPS = 8;
+constexpr int THREADS = 64 + (LN_WARPS + EPI_WARPS) * 32;
 constexpr uint32_t TM_QK = 0, TM_V = 256, TM_B = 384;
 enum { G_QK = 0, G_B = 1, G_V = 2 };
 
@@ -64,11 +54,8 @@ struct Smem {
   uint8_t w[W_BYTES];
   uint8_t wb[2 * WB_SLAB];
   uint8_t x[XSTAGES][TILE_BYTES];
-#if B200_APROJ_TMASTORE
-  uint8_t out[TILE_BYTES];  // staging of one 32 KiB output tile (q, then k, then vT)
-#endif
-  uint32_t gamma2[64];
-  uint32_t beta2[64];
+  uint8_t out[TILE_BYTES];  // staging, one 16 KiB slab per epilogue warpgroup (q, then k, then vT)
+  alignas(16) uint32_t gamma2[64], beta2[64];
   uint64_t w_full, x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES], acc_full[3], acc_empty[3];
   uint32_t tmem_base;
 };
@@ -76,17 +63,14 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 
 struct Params {
   int n_outer, n_inner, tiles_inner;
-  long long total_tiles;
+  uint32_t total_tiles;
   const void* gamma;
   const void* beta;
   const __nv_bfloat16* w_bias;  // [128][4]
   bool early_weights;           // the weights may be read before pdl_wait()
   MaskBiasOut mb;               // mb.out null: no mask-bias rows wanted
-  __nv_bfloat16* q;
-  __nv_bfloat16* k;
-  __half* vt;
   __nv_bfloat16* bias;
-  long long ld;           // pitch of vT rows and of bias rows (elements)
+  long long ld;           // pitch of bias rows (elements)
   long long bias_head_stride;
   float q_scale;          // bf16(sqrt(head_dim))
   float eps;
@@ -115,12 +99,12 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < XSTAGES; ++s) {
       mbar_init(&sm.x_full[s], 1);
-      mbar_init(&sm.xn_full[s], LN_WARPS * 32);
+      mbar_init(&sm.xn_full[s], LN_WARPS);
       mbar_init(&sm.x_empty[s], 1);
     }
     for (int g = 0; g < 3; ++g) {
       mbar_init(&sm.acc_full[g], 1);
-      mbar_init(&sm.acc_empty[g], 4);
+      mbar_init(&sm.acc_empty[g], g == G_B ? 4 : EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -152,13 +136,20 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   if (p.early_weights) pdl_wait();
   pdl_trigger();
 
+  // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
+  auto locate = [&](uint32_t tile, int& o, int& t0) {
+    const uint32_t q = tile / static_cast<uint32_t>(p.tiles_inner);
+    o = q;
+    t0 = (tile - q * p.tiles_inner) * 128;
+  };
+
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-        const int o = static_cast<int>(tile / p.tiles_inner);
-        const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+        int o, t0;
+        locate(tile, o, t0);
         if (!mbar_wait(&sm.x_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.x_full[stage], TILE_BYTES);
         tma_load_3d(sm.x[stage], &tm_x, &sm.x_full[stage], 0, t0, o);
@@ -177,7 +168,7 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
         if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
         const uint32_t xs = smem_u32(sm.x[stage]);
@@ -228,9 +219,11 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     const int r = (warp - 2) * 16 + (lane & 15);  // pair of the tile; lanes l and l ^ 16 share it
     int stage = 0;
     uint32_t phase = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
       if (p.mb.out && lane < 16) {  // the core's mask-bias row of these pairs, pitch padding included
-        const int o = static_cast<int>(tile / p.tiles_inner), t = static_cast<int>(tile % p.tiles_inner) * 128 + r;
+        int o, t;
+        locate(tile, o, t);
+        t += r;
         if (t < p.mb.ld)
           p.mb.out[static_cast<long long>(o) * p.mb.ld + t] =
               t >= p.n_inner ? -INFINITY
@@ -238,46 +231,44 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                              : 0.0f;
       }
       if (!mbar_wait(&sm.x_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
+      __syncwarp();
       ln_row_two_threads(sm.x[stage], r, lane >> 4, sm.gamma2, sm.beta2, p.eps);
       fence_proxy_async();
-      mbar_arrive(&sm.xn_full[stage]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
       if (++stage == XSTAGES) {
         stage = 0;
         phase ^= 1;
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, group = (warp - 2 - LN_WARPS) >> 2;
     const int row = quarter * 32 + lane;  // TMEM lane: a pair for q/k/bias, a channel for vT
+    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    uint8_t* out = sm.out + group * SLAB_BYTES;
     const uint32_t qs = pack_bf16x2(p.q_scale, p.q_scale);
     const float q_inv = 1.0f / bf16_lo(qs);
     uint32_t it = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
-      const int o = static_cast<int>(tile / p.tiles_inner);
-      const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
-      const int t = t0 + row;
-#if !B200_APROJ_TMASTORE
-      const long long pair_off = (static_cast<long long>(o) * p.n_inner + t) * 128;
-#endif
-      // ---- q and k: thread = pair, 128 + 128 channels
-#if B200_APROJ_TMASTORE
-      // (votes: the outcome of each bounded wait is made the same for all 128 threads, which
-      // meet at named barriers around the staging buffer)
-      if (!named_barrier_and(1, 128, mbar_wait(&sm.acc_full[G_QK], it & 1, p.status, ST_TIMEOUT_EPILOGUE))) break;
-#else
-      if (!mbar_wait(&sm.acc_full[G_QK], it & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
-#endif
+    // (votes: the outcome of each bounded wait is made the same for the warpgroup's 128 threads,
+    // which meet at named barriers around its staging slab)
+    auto acc_wait = [&](int g) {
+      return named_barrier_and(1 + group, 128, mbar_wait(&sm.acc_full[g], it & 1, p.status, ST_TIMEOUT_EPILOGUE));
+    };
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      int o, t0;
+      locate(tile, o, t0);
+      // ---- q and k: thread = pair, 64 channels of each
+      if (!acc_wait(G_QK)) break;
       tc_fence_after();
-#if B200_APROJ_TMASTORE
 #pragma unroll 1
-      for (int part = 0; part < 2; ++part) {  // q, then k: one staged 32 KiB tile each
-        if (threadIdx.x == EPI_THREAD0) tma_store_wait_read();
-        named_barrier(1, 128);
-#pragma unroll 1
-        for (int c4 = 0; c4 < 4; ++c4) {
+      for (int part = 0; part < 2; ++part) {  // q, then k
+        if (leader) tma_store_wait_read();
+        named_barrier(1 + group, 128);
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
           uint32_t r[32];
-          tmem_ld32(lane_addr + TM_QK + (part * 4 + c4) * 32, r);
+          tmem_ld32(lane_addr + TM_QK + part * 128 + group * 64 + c2 * 32, r);
           tmem_ld_wait();
 #pragma unroll
           for (int g4 = 0; g4 < 4; ++g4) {
@@ -290,87 +281,45 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
               if (part == 0) v2 = pack_bf16x2(bf16_lo(v2) * q_inv, bf16_hi(v2) * q_inv);
               u[e] = v2;
             }
-            // row = pair, 16-byte chunk = 8 channels: channels 32*c4 + 8*g4 .. +7
-            *reinterpret_cast<uint4*>(sm.out + (c4 >> 1) * SLAB_BYTES + sw128_offset(row, (c4 & 1) * 4 + g4)) =
-                make_uint4(u[0], u[1], u[2], u[3]);
+            // row = pair, 16-byte chunk = 8 channels
+            *reinterpret_cast<uint4*>(out + sw128_offset(row, c2 * 4 + g4)) = make_uint4(u[0], u[1], u[2], u[3]);
           }
         }
         fence_proxy_async();
-        named_barrier(1, 128);
-        if (threadIdx.x == EPI_THREAD0) {  // pairs past n_inner are outside the tensor and are not written
-          const CUtensorMap* tm = part ? &tm_k : &tm_q;
-          tma_store_3d(tm, sm.out, 0, t0, o);
-          tma_store_3d(tm, sm.out + SLAB_BYTES, 64, t0, o);
+        named_barrier(1 + group, 128);
+        if (leader) {  // pairs past n_inner are outside the tensor and are not written
+          tma_store_3d(part ? &tm_k : &tm_q, out, group * 64, t0, o);
           tma_store_commit();
         }
       }
-#else
-#pragma unroll 1
-      for (int chunk = 0; chunk < 8; ++chunk) {
-        uint32_t r[32];
-        tmem_ld32(lane_addr + TM_QK + chunk * 32, r);
-        tmem_ld_wait();
-        if (t < p.n_inner) {
-          __nv_bfloat16* base = (chunk < 4 ? p.q : p.k) + pair_off + (chunk & 3) * 32;
-          uint4* dst = reinterpret_cast<uint4*>(base);
-#pragma unroll
-          for (int g4 = 0; g4 < 4; ++g4) {
-            uint32_t u[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              uint32_t v2 = pack_bf16x2(__uint_as_float(r[8 * g4 + 2 * e]), __uint_as_float(r[8 * g4 + 2 * e + 1]));
-              // q / sqrt(d): the quotient of two bf16 numbers, rounded to bf16. The divisor
-              // is bf16(sqrt(32)) = 181/32 and q has an 8-bit significand, so the exact
-              // quotient is a multiple of 1/181 of its ulp scale and never closer than
-              // ~1e-5 (relative) to a bf16 rounding boundary: any fp32 value within 1e-6 of
-              // it, such as the product with the rounded reciprocal, rounds to the same bf16
-              // as the true division.
-              if (chunk < 4) v2 = pack_bf16x2(bf16_lo(v2) * q_inv, bf16_hi(v2) * q_inv);
-              u[e] = v2;
-            }
-            dst[g4] = make_uint4(u[0], u[1], u[2], u[3]);
-          }
-        }
-      }
-#endif
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.acc_empty[G_QK]);
-      // ---- bias: thread = pair, 4 heads
-#if B200_APROJ_TMASTORE
-      if (!named_barrier_and(1, 128, mbar_wait(&sm.acc_full[G_B], it & 1, p.status, ST_TIMEOUT_EPILOGUE))) break;
-#else
-      if (!mbar_wait(&sm.acc_full[G_B], it & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
-#endif
-      tc_fence_after();
-      {
+      if (group == 0) {  // ---- bias: thread = pair, 4 heads
+        if (!acc_wait(G_B)) break;
+        tc_fence_after();
         uint32_t r[16];
         tmem_ld16(lane_addr + TM_B, r);
         tmem_ld_wait();
+        const int t = t0 + row;
         if (t < p.n_inner) {
 #pragma unroll
           for (int h = 0; h < 4; ++h)
             p.bias[h * p.bias_head_stride + static_cast<long long>(o) * p.ld + t] =
                 __float2bfloat16_rn(__uint_as_float(r[h]));
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.acc_empty[G_B]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.acc_empty[G_B]);
-      // ---- vT: thread = channel, 128 pairs -> one contiguous run of the row
-#if B200_APROJ_TMASTORE
-      if (!named_barrier_and(1, 128, mbar_wait(&sm.acc_full[G_V], it & 1, p.status, ST_TIMEOUT_EPILOGUE))) break;
-#else
-      if (!mbar_wait(&sm.acc_full[G_V], it & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
-#endif
+      // ---- vT: thread = channel, 64 pairs -> one contiguous run of the row
+      if (leader) tma_store_wait_read();
+      if (!acc_wait(G_V)) break;
       tc_fence_after();
-#if B200_APROJ_TMASTORE
-      if (threadIdx.x == EPI_THREAD0) tma_store_wait_read();
-      named_barrier(1, 128);
-#pragma unroll 1
-      for (int chunk = 0; chunk < 4; ++chunk) {
+#pragma unroll
+      for (int c2 = 0; c2 < 2; ++c2) {
         uint32_t r[32];
-        tmem_ld32(lane_addr + TM_V + chunk * 32, r);
+        tmem_ld32(lane_addr + TM_V + group * 64 + c2 * 32, r);
         tmem_ld_wait();
 #pragma unroll
         for (int g4 = 0; g4 < 4; ++g4) {
@@ -382,57 +331,22 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
             const __half2 h2 = __floats2half2_rn(bf16_lo(b2), bf16_hi(b2));
             u[e] = *reinterpret_cast<const uint32_t*>(&h2);
           }
-          // row = channel, 16-byte chunk = 8 pairs: pairs 32*chunk + 8*g4 .. +7 of the tile
-          *reinterpret_cast<uint4*>(sm.out + (chunk >> 1) * SLAB_BYTES + sw128_offset(row, (chunk & 1) * 4 + g4)) =
-              make_uint4(u[0], u[1], u[2], u[3]);
+          // row = channel, 16-byte chunk = 8 pairs
+          *reinterpret_cast<uint4*>(out + sw128_offset(row, c2 * 4 + g4)) = make_uint4(u[0], u[1], u[2], u[3]);
         }
       }
+      tc_fence_before();
       fence_proxy_async();
-      named_barrier(1, 128);
-      if (threadIdx.x == EPI_THREAD0) {
-        tma_store_3d(&tm_vt, sm.out, t0, 0, o);
-        if (t0 + 64 < p.n_inner) tma_store_3d(&tm_vt, sm.out + SLAB_BYTES, t0 + 64, 0, o);
+      named_barrier(1 + group, 128);
+      if (leader && t0 + group * 64 < p.n_inner) {
+        tma_store_3d(&tm_vt, out, t0 + group * 64, 0, o);
         tma_store_commit();
       }
-#else
-      __half* vrow = p.vt + (static_cast<long long>(o) * 128 + row) * p.ld + t0;
-#pragma unroll 1
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        uint32_t r[32];
-        tmem_ld32(lane_addr + TM_V + chunk * 32, r);
-        tmem_ld_wait();
-        uint32_t packed[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const uint32_t b2 = pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));  // bf16(xn @ Wv)
-          const __half2 h2 = __floats2half2_rn(bf16_lo(b2), bf16_hi(b2));
-          packed[e] = *reinterpret_cast<const uint32_t*>(&h2);
-        }
-        const int tc = t0 + chunk * 32;
-        if (tc + 32 <= p.n_inner) {
-          uint4* d4 = reinterpret_cast<uint4*>(vrow + chunk * 32);
-#pragma unroll
-          for (int g4 = 0; g4 < 4; ++g4)
-            d4[g4] = make_uint4(packed[4 * g4], packed[4 * g4 + 1], packed[4 * g4 + 2], packed[4 * g4 + 3]);
-        } else if (tc < p.n_inner) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (tc + e < p.n_inner) {
-              const uint32_t w = packed[e >> 1];
-              vrow[chunk * 32 + e] = __ushort_as_half(static_cast<unsigned short>((e & 1) ? (w >> 16) : (w & 0xffffu)));
-            }
-        }
-      }
-#endif
-      tc_fence_before();
-      __syncwarp();
       if (lane == 0) mbar_arrive(&sm.acc_empty[G_V]);
     }
+    if (leader) tma_store_wait_all();
   }
 
-#if B200_APROJ_TMASTORE
-  if (threadIdx.x == EPI_THREAD0) tma_store_wait_all();
-#endif
   if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
     for (int i = 0; i < 100; ++i) __nanosleep(1000);
   tc_fence_before();
@@ -509,15 +423,14 @@ int b200::att_project_launch(const b200tri_triatt_project_args* a, const MaskBia
   p.n_outer = a->n_outer;
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
-  p.total_tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  const long long tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "att project: too many tiles (%lld)", tiles);
+  p.total_tiles = static_cast<uint32_t>(tiles);
   p.gamma = a->norm_scale;
   p.beta = a->norm_bias;
   p.w_bias = static_cast<const __nv_bfloat16*>(a->w_bias);
   p.early_weights = pdl_chained() && in_place;
   p.mb = mb ? *mb : MaskBiasOut{};
-  p.q = static_cast<__nv_bfloat16*>(a->q);
-  p.k = static_cast<__nv_bfloat16*>(a->k);
-  p.vt = static_cast<__half*>(a->vt);
   p.bias = static_cast<__nv_bfloat16*>(a->bias);
   p.ld = a->ld;
   p.bias_head_stride = a->bias_head_stride;
@@ -529,7 +442,7 @@ int b200::att_project_launch(const b200tri_triatt_project_args* a, const MaskBia
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_project_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const long long grid = tiles < sm_count() ? tiles : sm_count();
   {
     TimedLaunch timed(K_TRIATT_PROJECT, stream);
     return launch(att_project_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x,

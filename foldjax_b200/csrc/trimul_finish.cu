@@ -9,12 +9,16 @@
 // the same bytes as reading a stored gate would, and saves writing it.
 //
 // One tile = 128 consecutive pairs (i, j0..j0+127). Persistent, one CTA per SM:
-//   warp 0      TMA producer: two 128x128 weights once; per tile the x tile
-//               (K-major, swizzled) and the t tile ([channel][pair], plain)
-//   warp 1      MMA issuer: D1 = LN_in(x) . g_out^T, D2 = LN_out(t) . p_out^T
-//   warps 2-5   layer norms, one thread per pair; the t tile is transposed into
-//               operand layout in place (read column, mbarrier, write row)
-//   warps 6-9   epilogue: D2 * sigmoid(D1) (+ residual) -> bf16 -> shared-memory tile -> TMA store
+//   warp 0       TMA producer: two 128x128 weights once; per tile the x tile
+//                (K-major, swizzled) and the t tile ([channel][pair], two swizzled slabs of 64 pairs)
+//   warp 1       MMA issuer: D1 = LN_in(x) . g_out^T, D2 = LN_out(t) . p_out^T
+//                (warps 2 and 3 idle: registers move between whole warpgroups)
+//   warps 4-7    layer norm of x in place, one thread per pair
+//   warps 8-11   layer norm of t, one thread per pair: the tile is turned into operand layout in
+//                place (read column, mbarrier, write row), which holds a row in registers
+//   warps 12-19  epilogue: D2 * sigmoid(D1) (+ residual) -> bf16 -> shared-memory tile -> TMA
+//                store, 64 channels per warpgroup, the residual fetched before the products are
+//                waited for
 // TMEM: 2 x (D1, D2) so the epilogue overlaps the next tile's MMAs.
 //
 // Bound: HBM (read t and x, write out: 3 * n_i*n_j*128*2 bytes; + residual).
@@ -28,23 +32,15 @@ namespace {
 
 constexpr int STAGES = 2;
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
-constexpr int THREADS = 320;
-constexpr int EPI_THREAD0 = 192;  // first thread of the epilogue warps
-// 1: the epilogue stages the output tile in shared memory ([128 pairs][128 channels] as two
-// swizzled slabs) and writes it with two TMA stores; 0: every thread stores its pair's row
-// itself, 64 bytes at a time, so that a warp's store instruction touches 32 cache lines.
-#ifndef B200_FIN_TMASTORE
-#define B200_FIN_TMASTORE 1
-#endif
+constexpr int WORK_WARPS = 8, EPI_WARPS = 8;  // half of the working warps per layer norm
+constexpr int THREADS = 128 + (WORK_WARPS + EPI_WARPS) * 32;
 
 struct Smem {
   uint8_t w[4 * SLAB_BYTES];  // g_out, p_out: two boxes [128 in][64 out] each, MN-major
   uint8_t x[STAGES][TILE_BYTES];
   uint8_t t[STAGES][TILE_BYTES];
-#if B200_FIN_TMASTORE
-  uint8_t out[TILE_BYTES];
-#endif
-  uint32_t gamma_in[64], beta_in[64], gamma_out[64], beta_out[64];
+  uint8_t out[TILE_BYTES];  // two slabs of 64 channels, one per epilogue warpgroup
+  alignas(16) uint32_t gamma_in[64], beta_in[64], gamma_out[64], beta_out[64];
   uint64_t w_full, in_full[STAGES], xn_full[STAGES], in_empty[STAGES], col_read[STAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
 };
@@ -52,11 +48,10 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 
 struct FinishParams {
   int n_i, n_j, tiles_j;
-  long long total_tiles;
+  uint32_t total_tiles;
   const void* ln[4];    // gamma_in, beta_in, gamma_out, beta_out
   bool early_weights;   // the weights may be read before pdl_wait()
   const __nv_bfloat16* residual;
-  __nv_bfloat16* out;
   long long os_i, os_j;
   float eps;
   int t_rpb;  // rows per block of t
@@ -84,13 +79,13 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.in_full[s], 1);
-      mbar_init(&sm.xn_full[s], 128);
+      mbar_init(&sm.xn_full[s], WORK_WARPS);
       mbar_init(&sm.in_empty[s], 1);
-      mbar_init(&sm.col_read[s], 128);
+      mbar_init(&sm.col_read[s], WORK_WARPS / 2);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sm.acc_full[a], 1);
-      mbar_init(&sm.acc_empty[a], 4);
+      mbar_init(&sm.acc_empty[a], EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -119,18 +114,29 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   if (p.early_weights) pdl_wait();
   pdl_trigger();
 
+  // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
+  auto locate = [&](uint32_t tile, int& i, int& j0) {
+    const uint32_t q = tile / static_cast<uint32_t>(p.tiles_j);
+    i = q;
+    j0 = (tile - q * p.tiles_j) * 128;
+  };
+
+  // 640 threads x 96 registers = 128 x (48 + 80 + 144 + 2 x 104)
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-        const int i = static_cast<int>(tile / p.tiles_j);
-        const int j0 = static_cast<int>(tile % p.tiles_j) * 128;
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+        int i, j0;
+        locate(tile, i, j0);
         if (!mbar_wait(&sm.in_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.in_full[stage], 2 * TILE_BYTES);
         tma_load_3d(sm.x[stage], &tm_x, &sm.in_full[stage], 0, j0, i);
         tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.in_full[stage], 64, j0, i);
-        tma_load_4d(sm.t[stage], &tm_t, &sm.in_full[stage], j0, i % p.t_rpb, 0, i / p.t_rpb);
+        const int block = i / p.t_rpb, in_block = i - block * p.t_rpb;
+        for (int half = 0; half < 2; ++half)
+          tma_load_4d(sm.t[stage] + half * SLAB_BYTES, &tm_t, &sm.in_full[stage], j0 + half * 64, in_block, 0, block);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;
@@ -143,7 +149,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
         if (!mbar_wait(&sm.acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
@@ -167,112 +173,124 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         }
       }
     }
-  } else if (warp < 6) {
-    const int r = threadIdx.x - 64;
+  } else if (warp >= 4 && warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    const int r = threadIdx.x - 128;  // pair of the tile
     int stage = 0;
     uint32_t phase = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
       if (!mbar_wait(&sm.in_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      uint4 v[16];
-      // x tile: in-place layer norm of this thread's row.
-      ln_load_row(sm.x[stage], r, v);
-      ln_rows_inplace(v, sm.gamma_in, sm.beta_in, p.eps);
-      ln_store_row(sm.x[stage], r, v);
-      // t tile: gather this pair's column of the [channel][pair] tile.
-      {
-        const unsigned short* tcol = reinterpret_cast<const unsigned short*>(sm.t[stage]) + r;
-        uint32_t* w = reinterpret_cast<uint32_t*>(v);
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          w[i] = static_cast<uint32_t>(tcol[(2 * i) * 128]) | (static_cast<uint32_t>(tcol[(2 * i + 1) * 128]) << 16);
-      }
-      ln_rows_inplace(v, sm.gamma_out, sm.beta_out, p.eps);
-      // Rows may overwrite the tile only once every column has been read.
-      mbar_arrive(&sm.col_read[stage]);
-      if (!mbar_wait(&sm.col_read[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      ln_store_row(sm.t[stage], r, v);
+      ln_row_sweeps(sm.x[stage], r, sm.gamma_in, sm.beta_in, p.eps);
       fence_proxy_async();
-      mbar_arrive(&sm.xn_full[stage]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
       if (++stage == STAGES) {
         stage = 0;
         phase ^= 1;
       }
     }
-  } else {
-    const int quarter = warp & 3;
+  } else if (warp >= 8 && warp < 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    const int r = threadIdx.x - 256;  // pair of the tile
+    int stage = 0;
+    uint32_t phase = 0;
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+      if (!mbar_wait(&sm.in_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
+      uint4 v[16];
+      {
+        const uint8_t* slab = sm.t[stage] + (r >> 6) * SLAB_BYTES;
+        uint32_t* w = reinterpret_cast<uint32_t*>(v);
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {  // channels 2 * i and 2 * i + 1 of this pair
+          const uint32_t lo = *reinterpret_cast<const unsigned short*>(slab + sw128_offset(2 * i, (r & 63) >> 3) + (r & 7) * 2);
+          const uint32_t hi = *reinterpret_cast<const unsigned short*>(slab + sw128_offset(2 * i + 1, (r & 63) >> 3) + (r & 7) * 2);
+          w[i] = lo | (hi << 16);
+        }
+        // Rows may overwrite the tile only once every column has been read.
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.col_read[stage]);
+        ln_row_words(v, sm.gamma_out, sm.beta_out, p.eps);
+        if (!mbar_wait(&sm.col_read[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
+        ln_store_row(sm.t[stage], r, v);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
+      if (++stage == STAGES) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+  } else if (warp >= 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int quarter = warp & 3, half = (warp - 12) >> 2;  // 64 channels per warpgroup
     const int pr = quarter * 32 + lane;  // pair inside the tile = TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * 64;
+    uint8_t* stage_out = sm.out + half * SLAB_BYTES;
     uint32_t it = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
-      const int i = static_cast<int>(tile / p.tiles_j);
-      const int j = static_cast<int>(tile % p.tiles_j) * 128 + pr;
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      int i, j0;
+      locate(tile, i, j0);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-#if B200_FIN_TMASTORE
+      uint4 res[8];  // residual of the warp's 32 pairs, 8 lanes to a pair's 64 channels (whole lines)
+      if (p.residual) {
+        const int t = j0 + quarter * 32 + (lane >> 3);
+        const __nv_bfloat16* src = p.residual + static_cast<long long>(i) * p.os_i + half * 64 + (lane & 7) * 8;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          res[q] = t + 4 * q < p.n_j ? *reinterpret_cast<const uint4*>(src + static_cast<long long>(t + 4 * q) * p.os_j)
+                                      : make_uint4(0u, 0u, 0u, 0u);
+      }
       // the previous tile must have left the staging buffer; the vote makes the outcome of the
       // bounded wait the same for all 128 threads, which meet at a barrier below
-      if (threadIdx.x == EPI_THREAD0) tma_store_wait_read();
-      if (!named_barrier_and(1, 128, mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE))) break;
-#else
-      if (!mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE)) break;
-#endif
+      if (leader) tma_store_wait_read();
+      if (!named_barrier_and(1 + half, 128, mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE))) break;
       tc_fence_after();
-      const long long off = static_cast<long long>(i) * p.os_i + static_cast<long long>(j) * p.os_j;
-#pragma unroll 1
+#pragma unroll
       for (int chunk = 0; chunk < 4; ++chunk) {
-        uint32_t g[32], o[32];
-        tmem_ld32(lane_addr + acc * 256 + chunk * 32, g);
-        tmem_ld32(lane_addr + acc * 256 + 128 + chunk * 32, o);
+        uint32_t g[16], o[16];
+        tmem_ld16(lane_addr + acc * 256 + chunk * 16, g);
+        tmem_ld16(lane_addr + acc * 256 + 128 + chunk * 16, o);
         tmem_ld_wait();
-        if (j < p.n_j) {
-#if !B200_FIN_TMASTORE
-          uint4* dst = reinterpret_cast<uint4*>(p.out + off + chunk * 32);
-#endif
-          const uint4* res = p.residual ? reinterpret_cast<const uint4*>(p.residual + off + chunk * 32) : nullptr;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t u[4];
+        for (int q = 0; q < 2; ++q) {
+          uint32_t u[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int c = 8 * q + 2 * e;
-              const uint32_t ov = pack_bf16x2(__uint_as_float(o[c]), __uint_as_float(o[c + 1]));
-              const uint32_t sg = sigmoid_bf16x2(__uint_as_float(g[c]), __uint_as_float(g[c + 1]));
-              u[e] = bf16x2_mul(ov, sg);
-            }
-            if (res) {  // the caller's z + update, one more bf16 rounding
-              const uint4 rv = res[q];
-              u[0] = bf16x2_add(rv.x, u[0]);
-              u[1] = bf16x2_add(rv.y, u[1]);
-              u[2] = bf16x2_add(rv.z, u[2]);
-              u[3] = bf16x2_add(rv.w, u[3]);
-            }
-#if B200_FIN_TMASTORE
-            *reinterpret_cast<uint4*>(sm.out + (chunk >> 1) * SLAB_BYTES + sw128_offset(pr, (chunk & 1) * 4 + q)) =
-                make_uint4(u[0], u[1], u[2], u[3]);
-#else
-            dst[q] = make_uint4(u[0], u[1], u[2], u[3]);
-#endif
+          for (int e = 0; e < 4; ++e) {
+            const int c = 8 * q + 2 * e;
+            const uint32_t ov = pack_bf16x2(__uint_as_float(o[c]), __uint_as_float(o[c + 1]));
+            const uint32_t sg = sigmoid_bf16x2(__uint_as_float(g[c]), __uint_as_float(g[c + 1]));
+            u[e] = bf16x2_mul(ov, sg);
           }
+          *reinterpret_cast<uint4*>(stage_out + sw128_offset(pr, chunk * 2 + q)) = make_uint4(u[0], u[1], u[2], u[3]);
         }
       }
-#if B200_FIN_TMASTORE
+      if (p.residual) {  // the caller's z + update, one more bf16 rounding, in the residual's arrangement
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          uint4* ptr = reinterpret_cast<uint4*>(stage_out + sw128_offset(quarter * 32 + 4 * q + (lane >> 3), lane & 7));
+          uint4 u = *ptr;
+          u.x = bf16x2_add(res[q].x, u.x);
+          u.y = bf16x2_add(res[q].y, u.y);
+          u.z = bf16x2_add(res[q].z, u.z);
+          u.w = bf16x2_add(res[q].w, u.w);
+          *ptr = u;
+        }
+      }
+      tc_fence_before();
       fence_proxy_async();
-      named_barrier(1, 128);
-      if (threadIdx.x == EPI_THREAD0) {  // rows past n_j are outside the tensor and are not written
-        const int j0 = static_cast<int>(tile % p.tiles_j) * 128;
-        tma_store_3d(&tm_out, sm.out, 0, j0, i);
-        tma_store_3d(&tm_out, sm.out + SLAB_BYTES, 64, j0, i);
+      named_barrier(1 + half, 128);
+      if (leader) {  // rows past n_j are outside the tensor and are not written
+        tma_store_3d(&tm_out, stage_out, half * 64, j0, i);
         tma_store_commit();
       }
-#endif
-      tc_fence_before();
-      __syncwarp();
       if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
     }
+    if (leader) tma_store_wait_all();
   }
 
-#if B200_FIN_TMASTORE
-  if (threadIdx.x == EPI_THREAD0) tma_store_wait_all();
-#endif
   if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
     for (int i = 0; i < 100; ++i) __nanosleep(1000);
   tc_fence_before();
@@ -337,8 +355,8 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
     const uint64_t dims[4] = {(uint64_t)a->n_j, rpb, 128, blocks};
     const uint64_t str[3] = {(uint64_t)a->t_ld * 2, (uint64_t)a->t_chan_stride * 2,
                              (uint64_t)(blocked ? a->t_block_stride : a->t_chan_stride * 128) * 2};
-    const uint32_t box[4] = {128, 1, 128, 1};
-    int rc = make_tmap(&tm_t, a->t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::None);
+    const uint32_t box[4] = {64, 1, 128, 1};
+    int rc = make_tmap(&tm_t, a->t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B128);
     if (rc) return rc;
   }
   {
@@ -349,14 +367,15 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
   p.n_i = a->n_i;
   p.n_j = a->n_j;
   p.tiles_j = (a->n_j + 127) / 128;
-  p.total_tiles = static_cast<long long>(p.tiles_j) * a->n_i;
+  const long long tiles = static_cast<long long>(p.tiles_j) * a->n_i;
+  B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "finish: too many tiles (%lld)", tiles);
+  p.total_tiles = static_cast<uint32_t>(tiles);
   p.ln[0] = a->norm_in_scale;
   p.ln[1] = a->norm_in_bias;
   p.ln[2] = a->norm_out_scale;
   p.ln[3] = a->norm_out_bias;
   p.early_weights = pdl_chained() && w_g == a->g_out && w_p == a->p_out;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
-  p.out = static_cast<__nv_bfloat16*>(a->out);
   p.os_i = a->os_i;
   p.os_j = a->os_j;
   p.eps = a->eps;
@@ -367,7 +386,7 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(finish_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const long long grid = tiles < sm_count() ? tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_FINISH, stream);
     return launch(finish_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_t,

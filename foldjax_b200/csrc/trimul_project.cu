@@ -12,11 +12,13 @@
 // lane is an output channel and a thread of the epilogue owns 128 consecutive
 // pairs of one channel, i.e. one contiguous 256-byte run of the output.
 //
-// Persistent kernel, one CTA per SM, 10 warps:
-//   warp 0      TMA producer: weights once (128 KiB, resident), x tiles in a 3-stage ring
-//   warp 1      MMA issuer: 4 groups (p_a, g_a, p_b, g_b) of 128x128x128 per tile
-//   warps 2-9   layer norm, in place in the tile TMA delivered (two threads per pair)
-//   warps 10-13 epilogue: TMEM -> sigmoid gate -> mask -> bf16 -> global
+// Persistent kernel, one CTA per SM:
+//   warp 0       TMA producer: weights once (128 KiB, resident), x tiles in a 2-stage ring
+//   warp 1       MMA issuer: 4 groups (p_a, g_a, p_b, g_b) of 128x128x128 per tile
+//   warps 2-9    layer norm, in place in the tile TMA delivered (two threads per pair)
+//   warps 10-17  epilogue: TMEM -> sigmoid gate -> mask -> bf16 -> shared memory -> TMA store,
+//                64 pairs per warpgroup (stored by the threads themselves, each 64-byte run went to
+//                another channel plane: 32 lines per instruction, and the L1 pipe was the bound)
 // TMEM: four 128-column accumulators; the a-half and the b-half are released
 // separately so the MMAs of the next tile overlap the epilogue of this one.
 //
@@ -29,19 +31,19 @@ namespace b200 {
 
 namespace {
 
-constexpr int XSTAGES = 3;
+constexpr int XSTAGES = 2;
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;  // 32 KiB: 128 pairs x 128 channels bf16
 constexpr int W_BYTES = 8 * SLAB_BYTES;     // 128 KiB: 4 groups x 2 K-slabs
 constexpr int MASK_SLOTS = 4;
-constexpr int LN_WARPS = 8;  // two threads per pair
-constexpr int THREADS = 64 + LN_WARPS * 32 + 128;
+constexpr int LN_WARPS = 8, EPI_WARPS = 8;
+constexpr int THREADS = 64 + (LN_WARPS + EPI_WARPS) * 32;
 
 struct Smem {
   uint8_t w[W_BYTES];  // group g (p_a, g_a, p_b, g_b): two boxes [128 in][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
+  uint8_t out[2][SLAB_BYTES];           // per epilogue warpgroup: [128 channels][64 pairs]
   __nv_bfloat16 mask[MASK_SLOTS][128];  // mask.astype(bf16), as the reference casts it
-  uint32_t gamma2[64];
-  uint32_t beta2[64];
+  alignas(16) uint32_t gamma2[64], beta2[64];
   uint64_t w_full, x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
 };
@@ -49,15 +51,12 @@ static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 
 struct ProjParams {
   int n_outer, n_inner, tiles_inner;
-  long long total_tiles;
+  uint32_t total_tiles;
   const float* mask;
   long long ms_outer, ms_inner;
   const void* gamma;
   const void* beta;
   bool early_weights;  // the weights may be read before pdl_wait()
-  __nv_bfloat16* a;
-  __nv_bfloat16* b;
-  long long ld, chan_stride, block_stride;
   int rows_per_block;
   float eps;
   int* status;
@@ -65,7 +64,8 @@ struct ProjParams {
 
 __global__ void __launch_bounds__(THREADS, 1)
 project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_p,
-               const __grid_constant__ CUtensorMap tm_g, const ProjParams p) {
+               const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_a,
+               const __grid_constant__ CUtensorMap tm_b, const ProjParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -82,12 +82,12 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     mbar_init(&sm.w_full, 1);
     for (int s = 0; s < XSTAGES; ++s) {
       mbar_init(&sm.x_full[s], 1);
-      mbar_init(&sm.xn_full[s], LN_WARPS * 32);
+      mbar_init(&sm.xn_full[s], LN_WARPS);
       mbar_init(&sm.x_empty[s], 1);
     }
     for (int h = 0; h < 2; ++h) {
       mbar_init(&sm.acc_full[h], 1);
-      mbar_init(&sm.acc_empty[h], 4);
+      mbar_init(&sm.acc_empty[h], EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -113,13 +113,20 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   if (p.early_weights) pdl_wait();
   pdl_trigger();
 
+  // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
+  auto locate = [&](uint32_t tile, int& o, int& t0) {
+    const uint32_t q = tile / static_cast<uint32_t>(p.tiles_inner);
+    o = q;
+    t0 = (tile - q * p.tiles_inner) * 128;
+  };
+
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-        const int o = static_cast<int>(tile / p.tiles_inner);
-        const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+        int o, t0;
+        locate(tile, o, t0);
         if (!mbar_wait(&sm.x_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&sm.x_full[stage], TILE_BYTES);
         tma_load_3d(sm.x[stage], &tm_x, &sm.x_full[stage], 0, t0, o);
@@ -136,7 +143,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
       int stage = 0;
       uint32_t phase = 0, it = 0;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
         if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
         const uint32_t xs = smem_u32(sm.x[stage]);
@@ -170,83 +177,83 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     const int r = (warp - 2) * 16 + (lane & 15);
     int stage = 0;
     uint32_t phase = 0, it = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
-      const int o = static_cast<int>(tile / p.tiles_inner);
-      const int t = static_cast<int>(tile % p.tiles_inner) * 128 + r;
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      int o, t;
+      locate(tile, o, t);
+      t += r;
       float mval = 0.f;
       if (t < p.n_inner) mval = p.mask ? p.mask[o * p.ms_outer + t * p.ms_inner] : 1.0f;
       if (!mbar_wait(&sm.x_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
+      __syncwarp();
       ln_row_two_threads(sm.x[stage], r, lane >> 4, sm.gamma2, sm.beta2, p.eps);
       if (lane < 16) sm.mask[it & (MASK_SLOTS - 1)][r] = __float2bfloat16_rn(mval);
       fence_proxy_async();
-      mbar_arrive(&sm.xn_full[stage]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
       if (++stage == XSTAGES) {
         stage = 0;
         phase ^= 1;
       }
     }
   } else {
-    // ---- epilogue: thread = output channel (TMEM lane), columns = pairs
-    const int quarter = warp & 3;
+    // ---- epilogue: thread = output channel (TMEM lane), columns = pairs, 64 per warpgroup
+    const int quarter = warp & 3, part = (warp - 2 - LN_WARPS) >> 2;
     const int chan = quarter * 32 + lane;
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
+    uint8_t* out = sm.out[part];
     uint32_t it = 0;
     bool alive = true;
-    for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
-      const int o = static_cast<int>(tile / p.tiles_inner);
-      const int t0 = static_cast<int>(tile % p.tiles_inner) * 128;
-      const long long row_off = static_cast<long long>(o / p.rows_per_block) * p.block_stride +
-                                static_cast<long long>(chan) * p.chan_stride +
-                                static_cast<long long>(o % p.rows_per_block) * p.ld + t0;
-      const uint32_t* mrow = reinterpret_cast<const uint32_t*>(sm.mask[it & (MASK_SLOTS - 1)]);
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+      int o, t0;
+      locate(tile, o, t0);
+      t0 += part * 64;
+      const uint32_t* mrow = reinterpret_cast<const uint32_t*>(sm.mask[it & (MASK_SLOTS - 1)]) + part * 32;
       for (int half = 0; half < 2; ++half) {
-        if (!mbar_wait(&sm.acc_full[half], it & 1, p.status, ST_TIMEOUT_EPILOGUE)) {
+        // the previous tile must have left the staging buffer; the vote makes the outcome of the
+        // bounded wait the same for all 128 threads, which meet at a barrier below
+        if (leader) tma_store_wait_read();
+        if (!named_barrier_and(1 + part, 128, mbar_wait(&sm.acc_full[half], it & 1, p.status, ST_TIMEOUT_EPILOGUE))) {
           alive = false;
           break;
         }
         tc_fence_after();
-        __nv_bfloat16* dst = (half ? p.b : p.a) + row_off;
-#pragma unroll 1
+#pragma unroll
         for (int chunk = 0; chunk < 4; ++chunk) {
-          uint32_t pr[32], gr[32];
-          tmem_ld32(lane_addr + half * 256 + chunk * 32, pr);
-          tmem_ld32(lane_addr + half * 256 + 128 + chunk * 32, gr);
+          uint32_t pr[16], gr[16];
+          tmem_ld16(lane_addr + half * 256 + chunk * 16, pr);
+          tmem_ld16(lane_addr + half * 256 + 128 + chunk * 16, gr);
           tmem_ld_wait();
           // bf16 rounding after the two products, the sigmoid, the gating and the
           // mask, as on the reference's bf16 trunk.
-          uint32_t packed[16];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint4 m = *reinterpret_cast<const uint4*>(mrow + chunk * 16 + 4 * q);
+          for (int q = 0; q < 2; ++q) {
+            const uint4 m = *reinterpret_cast<const uint4*>(mrow + chunk * 8 + 4 * q);
             const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
+            uint32_t packed[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int c = 8 * q + 2 * e;
               const uint32_t pv = pack_bf16x2(__uint_as_float(pr[c]), __uint_as_float(pr[c + 1]));
               const uint32_t sg = sigmoid_bf16x2(__uint_as_float(gr[c]), __uint_as_float(gr[c + 1]));
-              packed[4 * q + e] = bf16x2_mul(bf16x2_mul(sg, pv), mm[e]);
+              packed[e] = bf16x2_mul(bf16x2_mul(sg, pv), mm[e]);
             }
-          }
-          const int tc = t0 + chunk * 32;
-          if (tc + 32 <= p.n_inner) {
-            uint4* d4 = reinterpret_cast<uint4*>(dst + chunk * 32);
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              d4[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-          } else if (tc < p.n_inner) {
-#pragma unroll
-            for (int q = 0; q < 32; ++q)
-              if (tc + q < p.n_inner) {
-                const uint32_t w = packed[q >> 1];
-                dst[chunk * 32 + q] = __ushort_as_bfloat16(static_cast<unsigned short>((q & 1) ? (w >> 16) : (w & 0xffffu)));
-              }
+            *reinterpret_cast<uint4*>(out + sw128_offset(chan, chunk * 2 + q)) =
+                make_uint4(packed[0], packed[1], packed[2], packed[3]);
           }
         }
         tc_fence_before();
-        __syncwarp();
+        fence_proxy_async();
+        named_barrier(1 + part, 128);
+        if (leader && t0 < p.n_inner) {  // pairs past n_inner are outside the tensor and are not written
+          const int block = o / p.rows_per_block;
+          tma_store_4d(half ? &tm_b : &tm_a, out, t0, o - block * p.rows_per_block, 0, block);
+          tma_store_commit();
+        }
         if (lane == 0) mbar_arrive(&sm.acc_empty[half]);
       }
     }
+    if (leader) tma_store_wait_all();
   }
 
   if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
@@ -304,23 +311,31 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
     int rc = make_weight_map(&tm_p, w_p, 128, 256, 128);
     if (rc || (rc = make_weight_map(&tm_g, w_g, 128, 256, 128))) return rc;
   }
+  CUtensorMap tm_out[2];  // (pair, row in block, channel, block), written as tiles of [128 channels][64 pairs]
+  const int rpb = a->rows_per_block < a->n_outer ? a->rows_per_block : a->n_outer;
+  for (int i = 0; i < 2; ++i) {
+    const int blocks = (a->n_outer + rpb - 1) / rpb;
+    const uint64_t dims[4] = {(uint64_t)a->n_inner, (uint64_t)rpb, 128, (uint64_t)blocks};
+    const uint64_t str[3] = {(uint64_t)a->ld * 2, (uint64_t)a->chan_stride * 2,
+                             (uint64_t)(blocks > 1 ? a->block_stride : a->chan_stride * 128) * 2};
+    const uint32_t box[4] = {64, 1, 128, 1};
+    int rc = make_tmap(&tm_out[i], i ? a->b : a->a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B128);
+    if (rc) return rc;
+  }
   ProjParams p;
   p.n_outer = a->n_outer;
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
-  p.total_tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  const long long tiles = static_cast<long long>(p.tiles_inner) * a->n_outer;
+  B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "project: too many tiles (%lld)", tiles);
+  p.total_tiles = static_cast<uint32_t>(tiles);
   p.mask = a->mask;
   p.ms_outer = a->ms_outer;
   p.ms_inner = a->ms_inner;
   p.gamma = a->norm_in_scale;
   p.beta = a->norm_in_bias;
   p.early_weights = chained && w_p == a->p_in && w_g == a->g_in;
-  p.a = static_cast<__nv_bfloat16*>(a->a);
-  p.b = static_cast<__nv_bfloat16*>(a->b);
-  p.ld = a->ld;
-  p.chan_stride = a->chan_stride;
-  p.block_stride = a->block_stride;
-  p.rows_per_block = a->rows_per_block;
+  p.rows_per_block = rpb;
   p.eps = a->eps;
   p.status = status;
 
@@ -328,10 +343,10 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(project_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const long long grid = tiles < sm_count() ? tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_PROJECT, stream);
     return launch(project_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_p,
-                  tm_g, p);
+                  tm_g, tm_out[0], tm_out[1], p);
   }
 }
