@@ -16,21 +16,25 @@
 // into 64 hidden values per pair by the activation warps, goes back to shared
 // memory as the A operand of the second product and is consumed there.
 // The weights (384 KiB as bf16) do not fit in shared memory; they stream from
-// L2 through a 3-stage ring, one chunk (W1 rows, W2 rows, W3 columns: 48 KiB)
-// per stage.
+// L2 through two rings: fc1 and fc2 of a chunk (32 KiB) until its first product is through, fc3
+// (16 KiB) until its second.
 //
 // Persistent, one CTA per SM:
-//   warp 0        TMA producer (x tiles, weight chunks)
-//   warp 1        MMA issuer: D1[chunk] = xn . [W1c ; W2c]^T, then OUT += h . W3c^T
-//   warps 2-5     layer norm of the x tile in place (three register-light sweeps over
-//                 shared memory); epilogue of OUT (+ residual)
-//   warps 6-21    activation: four warpgroups, each turns 16 of the 64 [a | b] column
-//                 pairs of every row into hidden values per chunk (four threads per
-//                 pair). All of them must have stored their part before the second
-//                 product of the chunk can start, so these warps carry no other duty.
+//   warp 0        TMA producer of the weight chunks
+//   warp 1        MMA issuer: D1[chunk] = xn . [W1c ; W2c]^T, then OUT += h . W3c^T two chunks later
+//   warp 2        TMA producer of the x tiles        (warp 3 idle)
+//   warps 4-7     layer norm of the x tile in place (three register-light sweeps)
+//   warps 8-11    epilogue of OUT: residual fetched in whole lines before the products are waited
+//                 for, sum staged in shared memory, TMA stores per warp
+//   warps 12-27   activation: two groups of two warpgroups that take alternate chunks, each with a
+//                 D1 and an h buffer of its own; a warpgroup turns 32 of the 64 [a | b] column pairs
+//                 of every row into hidden values
 // Bound: the activation (two MUFU operations per hidden unit: 1024 per pair) and
 // the tensor pipe (393 kflop per pair) are within 25 % of each other; HBM moves
-// 2 x 256 B per pair (x doubles as the residual when the caller adds in place).
+// 2 x 256 B per pair (x doubles as the residual when the caller adds in place). What bounded it
+// before was neither: one warpgroup had layer norm and epilogue in turn, with every pair's row
+// stored and its residual loaded by one thread, and everything else waited for it.
+// 1024 x 1024 pairs, hidden 512: 575 us then, 434 so (251 at the tensor cores' rate).
 #include "host.cuh"
 #include "ln.cuh"
 #include "tc.cuh"
@@ -40,32 +44,34 @@ namespace b200 {
 namespace {
 
 constexpr int HC = 64;  // hidden units per chunk
-constexpr int WSTAGES = 3;
+constexpr int WSTAGES = 2;   // fc1 and fc2 of a chunk
+constexpr int W3STAGES = 3;  // fc3 of a chunk: used two chunks after those
 constexpr int XSTAGES = 2;
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
-constexpr int NWORK = 4;  // activation warpgroups
-constexpr int THREADS = 64 + 128 + NWORK * 128;
+constexpr int NWORK = 4;  // activation warpgroups, two per chunk parity
+constexpr int THREADS = 3 * 128 + NWORK * 128;
 
 struct Smem {
   uint8_t w12[WSTAGES][2 * SLAB_BYTES];  // fc1 and fc2 of the chunk: [128 in][64 hidden] each, MN-major
-  uint8_t w3[WSTAGES][SLAB_BYTES];       // fc3 of the chunk: two boxes [64 hidden][64 out], MN-major
+  uint8_t w3[W3STAGES][SLAB_BYTES];      // fc3 of the chunk: two boxes [64 hidden][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
-  uint8_t h[SLAB_BYTES];                 // [128 pairs][64 hidden]
+  uint8_t h[2][SLAB_BYTES];              // [128 pairs][64 hidden], by chunk parity
+  uint8_t out[SLAB_BYTES];               // [128 pairs][64 channels], a quarter per epilogue warp
   alignas(16) uint32_t gamma2[64], beta2[64];
-  uint64_t w_full[WSTAGES], w_empty[WSTAGES], x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES];
-  uint64_t d1_full[2], d1_empty[2], h_full, h_empty, out_full[2], out_empty[2];
+  uint64_t w_full[WSTAGES], w_empty[WSTAGES], w3_full[W3STAGES], w3_empty[W3STAGES], x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES];
+  uint64_t d1_full[2], d1_empty[2], h_full[2], h_empty[2], out_full[2], out_empty[2];
   uint32_t tmem_base;
 };
 static_assert(sizeof(Smem) <= 232448, "shared memory budget");
 
 struct Params {
-  long long rows, total_tiles;
-  int nchunks;         // hidden / 64
+  long long rows;
+  uint32_t total_tiles, nchunks;  // nchunks = hidden / 64
+  bool early_weights;             // the weights may be read before pdl_wait()
   const void* gamma;
   const void* beta;
   const __nv_bfloat16* residual;
   const float* row_mask;
-  __nv_bfloat16* out;
   float eps;
   int* status;
 };
@@ -81,7 +87,7 @@ __device__ __forceinline__ uint32_t swiglu_bf16x2(float a0, float a1, float b0, 
 __global__ void __launch_bounds__(THREADS, 1)
 pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1,
                        const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_w3,
-                       const Params p) {
+                       const __grid_constant__ CUtensorMap tm_out, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -99,86 +105,100 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       mbar_init(&sm.w_full[s], 1);
       mbar_init(&sm.w_empty[s], 1);
     }
+    for (int s = 0; s < W3STAGES; ++s) {
+      mbar_init(&sm.w3_full[s], 1);
+      mbar_init(&sm.w3_empty[s], 1);
+    }
     for (int s = 0; s < XSTAGES; ++s) {
       mbar_init(&sm.x_full[s], 1);
-      mbar_init(&sm.xn_full[s], 128);
+      mbar_init(&sm.xn_full[s], 4);
       mbar_init(&sm.x_empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sm.d1_full[a], 1);
-      mbar_init(&sm.d1_empty[a], NWORK * 4);
+      mbar_init(&sm.d1_empty[a], NWORK / 2 * 4);
+      mbar_init(&sm.h_full[a], NWORK / 2 * 4);
+      mbar_init(&sm.h_empty[a], 1);
       mbar_init(&sm.out_full[a], 1);
-      mbar_init(&sm.out_empty[a], 4);  // the four warps of the warpgroup on epilogue duty
+      mbar_init(&sm.out_empty[a], 4);
     }
-    mbar_init(&sm.h_full, NWORK * 128);
-    mbar_init(&sm.h_empty, 1);
     fence_barrier_init();
   }
   if (warp == 1) {
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
-  pdl_wait();
-  pdl_trigger();
+  if (!p.early_weights) pdl_wait();
   if (threadIdx.x >= 64 && threadIdx.x < 128) {
     sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
     sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
+  }
+  const uint32_t nchunks = p.nchunks;
+  const uint32_t n_my = (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;  // (the grid is at most total_tiles)
+  const uint32_t total_n = n_my * nchunks;                                         // chunk steps of this CTA
+  auto load_w12 = [&](uint32_t n, uint32_t c) {
+    const uint32_t s = n % WSTAGES;
+    mbar_expect_tx(&sm.w_full[s], 2 * SLAB_BYTES);
+    tma_load_2d(sm.w12[s], &tm_w1, &sm.w_full[s], c * HC, 0);
+    tma_load_2d(sm.w12[s] + SLAB_BYTES, &tm_w2, &sm.w_full[s], c * HC, 0);
+  };
+  auto load_w3 = [&](uint32_t n, uint32_t c) {
+    const uint32_t s = n % W3STAGES;
+    mbar_expect_tx(&sm.w3_full[s], SLAB_BYTES);
+    tma_load_2d(sm.w3[s], &tm_w3, &sm.w3_full[s], 0, c * HC);
+    tma_load_2d(sm.w3[s] + SLAB_BYTES / 2, &tm_w3, &sm.w3_full[s], 64, c * HC);
+  };
+  if (warp == 0 && lane == 0) {  // the first chunk's weights (the thread that initialised the barriers)
+    load_w12(0, 0);
+    load_w3(0, 0);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  if (p.early_weights) pdl_wait();
+  pdl_trigger();
   // TMEM: D1 (the chunk's [a | b], 128 columns) double-buffered at 0 and 128;
   // OUT (128 columns) double-buffered over tiles at 256 and 384.
-  long long n_my = 0;
-  for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) ++n_my;
-  const int nchunks = p.nchunks;
-  const long long total_n = n_my * nchunks;  // chunk steps of this CTA
 
   if (warp == 0) {
     if (elect_one()) {
-      auto load_x = [&](long long it) -> bool {
-        const int xs = static_cast<int>(it % XSTAGES);
-        const uint32_t ph = static_cast<uint32_t>((it / XSTAGES) & 1);
-        if (!mbar_wait(&sm.x_empty[xs], ph ^ 1, p.status, ST_TIMEOUT_PRODUCER)) return false;
-        const long long tile = blockIdx.x + it * static_cast<long long>(gridDim.x);
-        const int r0 = static_cast<int>(tile * 128);
+      uint32_t c = 0;  // chunk of step n
+      for (uint32_t n = 0; n < total_n; ++n) {
+        if (n > 0) {
+          if (!mbar_wait(&sm.w_empty[n % WSTAGES], ((n / WSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+          load_w12(n, c);
+          if (!mbar_wait(&sm.w3_empty[n % W3STAGES], ((n / W3STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+          load_w3(n, c);
+        }
+        if (++c == nchunks) c = 0;
+      }
+    }
+  } else if (warp == 2) {
+    if (elect_one()) {
+      for (uint32_t it = 0; it < n_my; ++it) {
+        const uint32_t xs = it % XSTAGES;
+        if (!mbar_wait(&sm.x_empty[xs], ((it / XSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+        const int r0 = static_cast<int>((blockIdx.x + it * gridDim.x) * 128u);
         mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
         tma_load_2d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, r0);
         tma_load_2d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, r0);
-        return true;
-      };
-      bool alive = n_my > 0 && load_x(0);
-      // The next tile's x is requested a few chunks into the current tile, when its
-      // buffer (the previous tile's) has certainly been released.
-      const int x_at = nchunks > WSTAGES ? WSTAGES : nchunks - 1;
-      for (long long n = 0; n < total_n && alive; ++n) {
-        const long long it = n / nchunks;
-        const int c = static_cast<int>(n % nchunks);
-        if (c == x_at && it + 1 < n_my && !load_x(it + 1)) break;
-        const int ws = static_cast<int>(n % WSTAGES);
-        const uint32_t ph = static_cast<uint32_t>((n / WSTAGES) & 1);
-        if (!mbar_wait(&sm.w_empty[ws], ph ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.w_full[ws], 3 * SLAB_BYTES);
-        tma_load_2d(sm.w12[ws], &tm_w1, &sm.w_full[ws], c * HC, 0);
-        tma_load_2d(sm.w12[ws] + SLAB_BYTES, &tm_w2, &sm.w_full[ws], c * HC, 0);
-        tma_load_2d(sm.w3[ws], &tm_w3, &sm.w_full[ws], 0, c * HC);
-        tma_load_2d(sm.w3[ws] + SLAB_BYTES / 2, &tm_w3, &sm.w_full[ws], 64, c * HC);
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
-      for (long long n = 0; n <= total_n; ++n) {
+      uint32_t it = 0, c = 0, jt = 0, e = 0;  // tile and chunk of the first product, of the second
+      // Second products follow two chunks behind, so that each activation group finds its next D1
+      // ready; one behind where a tile has one chunk (two ahead would need a tile whose layer norm
+      // comes after the epilogue of this one).
+      const uint32_t lag = nchunks > 1 ? 2 : 1;
+      for (uint32_t n = 0; n < total_n + lag; ++n) {
         if (n < total_n) {  // first product of chunk step n
-          const long long it = n / nchunks;
-          const int c = static_cast<int>(n % nchunks);
-          const int xs = static_cast<int>(it % XSTAGES);
-          const int ws = static_cast<int>(n % WSTAGES);
-          const uint32_t d = static_cast<uint32_t>(n & 1);
-          if (c == 0 && !mbar_wait(&sm.xn_full[xs], static_cast<uint32_t>((it / XSTAGES) & 1), p.status, ST_TIMEOUT_MMA)) break;
-          if (!mbar_wait(&sm.w_full[ws], static_cast<uint32_t>((n / WSTAGES) & 1), p.status, ST_TIMEOUT_MMA)) break;
-          if (!mbar_wait(&sm.d1_empty[d], static_cast<uint32_t>(((n >> 1) & 1) ^ 1), p.status, ST_TIMEOUT_MMA)) break;
+          const uint32_t xs = it % XSTAGES, ws = n % WSTAGES, d = n & 1;
+          if (c == 0 && !mbar_wait(&sm.xn_full[xs], (it / XSTAGES) & 1, p.status, ST_TIMEOUT_MMA)) break;
+          if (!mbar_wait(&sm.w_full[ws], (n / WSTAGES) & 1, p.status, ST_TIMEOUT_MMA)) break;
+          if (!mbar_wait(&sm.d1_empty[d], ((n >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
           const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w12[ws]), SLAB_BYTES);
 #pragma unroll
@@ -187,127 +207,147 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
             umma_bf16_ss(tmem_base + d * 128, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc,
                          k != 0);
           }
+          umma_commit(&sm.w_empty[ws]);
           umma_commit(&sm.d1_full[d]);
-          if (c == nchunks - 1) umma_commit(&sm.x_empty[xs]);  // every first product of the tile has been issued
+          if (++c == nchunks) {
+            umma_commit(&sm.x_empty[xs]);  // every first product of the tile has been issued
+            c = 0;
+            ++it;
+          }
         }
-        if (n > 0) {  // second product of chunk step n - 1
-          const long long m = n - 1;
-          const long long it = m / nchunks;
-          const int c = static_cast<int>(m % nchunks);
-          const int ws = static_cast<int>(m % WSTAGES);
-          const uint32_t tb = static_cast<uint32_t>(it & 1);
-          if (c == 0 && !mbar_wait(&sm.out_empty[tb], static_cast<uint32_t>(((it >> 1) & 1) ^ 1), p.status, ST_TIMEOUT_MMA)) break;
-          if (!mbar_wait(&sm.h_full, static_cast<uint32_t>(m & 1), p.status, ST_TIMEOUT_MMA)) break;
+        if (n >= lag) {  // second product of chunk step n - lag
+          const uint32_t m = n - lag, ws = m % W3STAGES, hb = m & 1, tb = jt & 1;
+          if (e == 0 && !mbar_wait(&sm.out_empty[tb], ((jt >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) break;
+          if (!mbar_wait(&sm.w3_full[ws], (m / W3STAGES) & 1, p.status, ST_TIMEOUT_MMA)) break;
+          if (!mbar_wait(&sm.h_full[hb], (m >> 1) & 1, p.status, ST_TIMEOUT_MMA)) break;
           tc_fence_after();
-          const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.h), 128);
+          const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.h[hb]), 128);
           const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w3[ws]), SLAB_BYTES / 2);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             umma_bf16_ss(tmem_base + 256 + tb * 128, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 2048),
-                         idesc, (c | k) != 0);
-          umma_commit(&sm.w_empty[ws]);  // covers both products that read this stage
-          umma_commit(&sm.h_empty);
-          if (c == nchunks - 1) umma_commit(&sm.out_full[tb]);
-        }
-      }
-    }
-  } else {
-    const bool act = warp >= 6;
-    const int wg = act ? (warp - 6) >> 2 : 0;
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;  // pair inside the tile = TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    bool alive = true;
-
-    // Layer norm of one row in place (the register-light form).
-    auto layer_norm_tile = [&](long long it) {
-      const int xs = static_cast<int>(it % XSTAGES);
-      if (!mbar_wait(&sm.x_full[xs], static_cast<uint32_t>((it / XSTAGES) & 1), p.status, ST_TIMEOUT_PROLOGUE)) {
-        alive = false;
-        return;
-      }
-      ln_row_sweeps(sm.x[xs], row, sm.gamma2, sm.beta2, p.eps);
-      fence_proxy_async();
-      mbar_arrive(&sm.xn_full[xs]);
-    };
-
-    auto epilogue_tile = [&](long long jt) {
-      const uint32_t tb = static_cast<uint32_t>(jt & 1);
-      if (!mbar_wait(&sm.out_full[tb], static_cast<uint32_t>((jt >> 1) & 1), p.status, ST_TIMEOUT_EPILOGUE)) {
-        alive = false;
-        return;
-      }
-      tc_fence_after();
-      const long long r = (blockIdx.x + jt * static_cast<long long>(gridDim.x)) * 128 + row;
-      const long long off = r * 128;
-      // optional per-row mask on the update (before the residual add), rounded to the trunk dtype
-      const float mkf = (p.row_mask && r < p.rows) ? p.row_mask[r] : 1.0f;
-      const uint32_t mk2 = pack_bf16x2(mkf, mkf);
-#pragma unroll 1
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        uint32_t v[32];
-        tmem_ld32(lane_addr + 256 + tb * 128 + chunk * 32, v);
-        tmem_ld_wait();
-        if (r < p.rows) {
-          uint4* dst = reinterpret_cast<uint4*>(p.out + off + chunk * 32);
-          const uint4* res = p.residual ? reinterpret_cast<const uint4*>(p.residual + off + chunk * 32) : nullptr;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t u[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
-            if (p.row_mask) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) u[e] = bf16x2_mul(u[e], mk2);
-            }
-            if (res) {
-              const uint4 rv = res[q];
-              u[0] = bf16x2_add(rv.x, u[0]);
-              u[1] = bf16x2_add(rv.y, u[1]);
-              u[2] = bf16x2_add(rv.z, u[2]);
-              u[3] = bf16x2_add(rv.w, u[3]);
-            }
-            dst[q] = make_uint4(u[0], u[1], u[2], u[3]);
+                         idesc, (e | k) != 0);
+          umma_commit(&sm.w3_empty[ws]);
+          umma_commit(&sm.h_empty[hb]);
+          if (++e == nchunks) {
+            umma_commit(&sm.out_full[tb]);
+            e = 0;
+            ++jt;
           }
         }
       }
+    }
+  } else if (warp >= 4 && warp < 8) {
+    const int row = threadIdx.x - 128;
+    for (uint32_t it = 0; it < n_my; ++it) {
+      const uint32_t xs = it % XSTAGES;
+      if (!mbar_wait(&sm.x_full[xs], (it / XSTAGES) & 1, p.status, ST_TIMEOUT_PROLOGUE)) break;
+      ln_row_sweeps(sm.x[xs], row, sm.gamma2, sm.beta2, p.eps);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xn_full[xs]);
+    }
+  } else if (warp >= 8 && warp < 12) {
+    const int quarter = warp & 3, row = quarter * 32 + lane;  // pair inside the tile = TMEM lane
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 256;
+    bool alive = true;
+    for (uint32_t it = 0; it < n_my && alive; ++it) {
+      const uint32_t tb = it & 1;
+      const long long r0 = static_cast<long long>(blockIdx.x + it * gridDim.x) * 128 + quarter * 32;  // the warp's first pair
+      // optional per-row mask on the update (before the residual add), rounded to the trunk dtype
+      const float mkf = p.row_mask && r0 + lane < p.rows ? p.row_mask[r0 + lane] : 1.0f;
+      const uint32_t mk2 = pack_bf16x2(mkf, mkf);
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {  // 64 channels at a time
+        uint4 res[8];  // residual of the warp's 32 pairs, 8 lanes to a pair's 64 channels (whole lines)
+        if (p.residual) {
+          const long long r = r0 + (lane >> 3);
+          const __nv_bfloat16* src = p.residual + r * 128 + half * 64 + (lane & 7) * 8;
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            res[q] = r + 4 * q < p.rows ? *reinterpret_cast<const uint4*>(src + 512 * q) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (half == 0 && !mbar_wait(&sm.out_full[tb], (it >> 1) & 1, p.status, ST_TIMEOUT_EPILOGUE)) {
+          alive = false;
+          break;
+        }
+        if (lane == 0) tma_store_wait_read();  // the previous half has left the staging rows
+        __syncwarp();
+        tc_fence_after();
+#pragma unroll
+        for (int chunk = 0; chunk < 4; ++chunk) {
+          uint32_t v[16];
+          tmem_ld16(lane_addr + tb * 128 + half * 64 + chunk * 16, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            uint32_t u[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
+              if (p.row_mask) u[e] = bf16x2_mul(u[e], mk2);
+            }
+            *reinterpret_cast<uint4*>(sm.out + sw128_offset(row, chunk * 2 + q)) = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+        }
+        if (p.residual) {  // the caller's z + update, one more bf16 rounding, in the residual's arrangement
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            uint4* ptr = reinterpret_cast<uint4*>(sm.out + sw128_offset(quarter * 32 + 4 * q + (lane >> 3), lane & 7));
+            uint4 u = *ptr;
+            u.x = bf16x2_add(res[q].x, u.x);
+            u.y = bf16x2_add(res[q].y, u.y);
+            u.z = bf16x2_add(res[q].z, u.z);
+            u.w = bf16x2_add(res[q].w, u.w);
+            *ptr = u;
+          }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0 && r0 < p.rows) {  // rows past the end are outside the tensor and are not written
+          tma_store_2d(&tm_out, sm.out + quarter * 4096, half * 64, static_cast<int>(r0));
+          tma_store_commit();
+        }
+      }
+      if (!alive) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.out_empty[tb]);
-    };
-
-    if (!act) {
-      // ---- layer norm of tile `it`, then the output epilogue of tile `it - 1`
-      for (long long it = 0; it <= n_my && alive; ++it) {
-        if (it < n_my) layer_norm_tile(it);
-        if (it > 0 && alive) epilogue_tile(it - 1);
-      }
     }
-    for (long long n = 0; act && n < total_n; ++n) {
-      // ---- activation: this thread's 16 columns of a and of b -> 16 hidden values
-      const uint32_t d = static_cast<uint32_t>(n & 1);
-      if (!mbar_wait(&sm.d1_full[d], static_cast<uint32_t>((n >> 1) & 1), p.status, ST_TIMEOUT_EPILOGUE)) break;
+    if (lane == 0) tma_store_wait_all();
+  } else if (warp >= 12) {
+    // ---- activation: 32 columns of a and of b -> 32 hidden values, 16 at a time
+    const int quarter = warp & 3, row = quarter * 32 + lane;  // pair inside the tile = TMEM lane
+    const uint32_t group = (warp - 12) >> 3, half = ((warp - 12) >> 2) & 1;
+    const uint32_t d1 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * 128 + half * 32;
+    for (uint32_t n = group; n < total_n; n += 2) {
+      if (!mbar_wait(&sm.d1_full[group], (n >> 1) & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
-      uint32_t a[16], b[16], hv[8];
-      tmem_ld16(lane_addr + d * 128 + wg * 16, a);
-      tmem_ld16(lane_addr + d * 128 + HC + wg * 16, b);
-      tmem_ld_wait();
+      uint32_t hv[16];
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint32_t a[16], b[16];
+        tmem_ld16(d1 + part * 16, a);
+        tmem_ld16(d1 + HC + part * 16, b);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          hv[part * 8 + e] = swiglu_bf16x2(__uint_as_float(a[2 * e]), __uint_as_float(a[2 * e + 1]), __uint_as_float(b[2 * e]),
+                                           __uint_as_float(b[2 * e + 1]));
+      }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.d1_empty[d]);
+      if (lane == 0) mbar_arrive(&sm.d1_empty[group]);
+      // this group's previous second product must have read h before it is overwritten
+      if (!mbar_wait(&sm.h_empty[group], ((n >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        hv[e] = swiglu_bf16x2(__uint_as_float(a[2 * e]), __uint_as_float(a[2 * e + 1]), __uint_as_float(b[2 * e]),
-                              __uint_as_float(b[2 * e + 1]));
-      // the previous chunk's second product must have read h before it is overwritten
-      if (!mbar_wait(&sm.h_empty, static_cast<uint32_t>((n & 1) ^ 1), p.status, ST_TIMEOUT_EPILOGUE)) break;
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-        *reinterpret_cast<uint4*>(sm.h + sw128_offset(row, wg * 2 + q)) =
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(sm.h[group] + sw128_offset(row, half * 4 + q)) =
             make_uint4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
       fence_proxy_async();
-      mbar_arrive(&sm.h_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.h_full[group]);
     }
   }
 
@@ -356,7 +396,14 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
     if (rc) return rc;
   }
 
-  CUtensorMap tm_x, tm_w1, tm_w2, tm_w3;
+  CUtensorMap tm_x, tm_w1, tm_w2, tm_w3, tm_out;
+  {  // the result, one box per warp: [32 pairs][64 channels]
+    const uint64_t dims[2] = {128, (uint64_t)a->rows};
+    const uint64_t str[1] = {256};
+    const uint32_t box[2] = {64, 32};
+    int rc = make_tmap(&tm_out, a->out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, str, box, Swz::B128);
+    if (rc) return rc;
+  }
   {
     const uint64_t dims[2] = {128, (uint64_t)a->rows};
     const uint64_t str[1] = {256};
@@ -371,13 +418,13 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
   }
   Params p;
   p.rows = a->rows;
-  p.total_tiles = (a->rows + 127) / 128;
+  p.total_tiles = static_cast<uint32_t>((a->rows + 127) / 128);
+  p.early_weights = pdl_chained() && w[0] == w_in[0] && w[1] == w_in[1] && w[2] == w_in[2];
   p.nchunks = a->hidden / HC;
   p.gamma = a->norm_scale;
   p.beta = a->norm_bias;
   p.residual = static_cast<const __nv_bfloat16*>(a->residual);
   p.row_mask = a->row_mask;
-  p.out = static_cast<__nv_bfloat16*>(a->out);
   p.eps = a->eps;
   p.status = status;
 
@@ -385,10 +432,10 @@ extern "C" int b200tri_pair_transition(const b200tri_pair_transition_args* a, b2
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(pair_transition_kernel), (int)sizeof(Smem));
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const uint32_t sms = sm_count(), grid = p.total_tiles < sms ? p.total_tiles : sms;
   {
     TimedLaunch timed(K_PAIR_TRANSITION, stream);
-    return launch(pair_transition_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x,
-                  tm_w1, tm_w2, tm_w3, p);
+    return launch(pair_transition_kernel, dim3(grid), dim3(THREADS), sizeof(Smem), stream, true, tm_x,
+                  tm_w1, tm_w2, tm_w3, tm_out, p);
   }
 }
