@@ -71,26 +71,27 @@ __device__ __forceinline__ void ln_store_row(uint8_t* tile, int row, const uint4
 }
 
 // The same layer norm (the same bits) as three sweeps over the row in shared memory - mean,
-// variance, normalise - holding four words at a time instead of the whole row: for kernels whose
-// other roles leave the layer-norm warps few registers.
+// variance, normalise - holding UNROLL words of 16 bytes at a time instead of the whole row: for
+// kernels whose other roles leave the layer-norm warps few registers.
+template <int UNROLL>
 __device__ __forceinline__ void ln_row_sweeps(uint8_t* tile, int row, const uint32_t* gamma2, const uint32_t* beta2,
                                               float eps) {
   float sum = 0.f, sq = 0.f;
-#pragma unroll 4
+#pragma unroll UNROLL
   for (int c = 0; c < 16; ++c) {
     const uint4 v = *reinterpret_cast<const uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
     sum = ln_add4(sum, v.x, v.y, v.z, v.w);
   }
   const float mean = sum * (1.0f / 128.0f);
   const float2 mm = make_float2(-mean, -mean);
-#pragma unroll 4
+#pragma unroll UNROLL
   for (int c = 0; c < 16; ++c) {
     const uint4 v = *reinterpret_cast<const uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
     sq = ln_square(ln_square(ln_square(ln_square(sq, v.x, mm), v.y, mm), v.z, mm), v.w, mm);
   }
   const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
   const float2 rr = make_float2(rstd, rstd);
-#pragma unroll 4
+#pragma unroll UNROLL
   for (int c = 0; c < 16; ++c) {
     uint4* ptr = reinterpret_cast<uint4*>(tile + (c >> 3) * SLAB_BYTES + sw128_offset(row, c & 7));
     const uint4 v = *ptr, g = reinterpret_cast<const uint4*>(gamma2)[c], b = reinterpret_cast<const uint4*>(beta2)[c];

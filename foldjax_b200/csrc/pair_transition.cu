@@ -242,7 +242,7 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     for (uint32_t it = 0; it < n_my; ++it) {
       const uint32_t xs = it % XSTAGES;
       if (!mbar_wait(&sm.x_full[xs], (it / XSTAGES) & 1, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      ln_row_sweeps(sm.x[xs], row, sm.gamma2, sm.beta2, p.eps);
+      ln_row_sweeps<8>(sm.x[xs], row, sm.gamma2, sm.beta2, p.eps);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.xn_full[xs]);

@@ -12,11 +12,12 @@
 // One tile = 128 consecutive pairs. Persistent, one CTA per SM:
 //   warp 0       TMA producer (Wg, Wo once; x tiles in a 2-stage ring, o tiles in a 3-stage ring)
 //   warp 1       MMA issuer: G = LN(x).Wg^T, then OUT = (o*g).Wo^T
-//   warps 2-5    layer norm of x in place, one thread per pair
-//   warps 6-9    gating of o in place, one thread per pair (the o tile becomes the A operand of the
+//                (warps 2 and 3 idle: registers move between whole warpgroups)
+//   warps 4-7    layer norm of x in place, one thread per pair, the row in its registers
+//   warps 8-11   gating of o in place, one thread per pair (the o tile becomes the A operand of the
 //                second product)
-//   warps 10-17  epilogue of OUT, 64 channels per warpgroup: residual fetched before the product
-//                is waited for, sum staged in the o tile (dead by then), one TMA store per warpgroup
+//   warps 12-15  epilogue of OUT: residual fetched before the product is waited for, sum staged in
+//                the o tile (dead by then), TMA stores per warp
 // Bound: HBM (read x and o, write out: 3 * n*n*128*2 bytes; + residual) - once enough warps
 // hide the latencies of TMEM and of the row-wise accesses.
 #include "host.cuh"
@@ -29,8 +30,8 @@ namespace {
 
 constexpr int XSTAGES = 2, OSTAGES = 3;  // an x tile is free after the first product, an o tile once it is stored
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;
-constexpr int LN_WARPS = 4, GATE_WARPS = 4, EPI_WARPS = 8;
-constexpr int THREADS = 64 + (LN_WARPS + GATE_WARPS + EPI_WARPS) * 32;
+constexpr int LN_WARPS = 4, GATE_WARPS = 4, EPI_WARPS = 4;
+constexpr int THREADS = 128 + (LN_WARPS + GATE_WARPS + EPI_WARPS) * 32;
 
 struct Smem {
   uint8_t w[4 * SLAB_BYTES];  // Wg, Wo: two boxes [128 in][64 out] each, MN-major
@@ -81,7 +82,7 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     for (int s = 0; s < OSTAGES; ++s) {
       mbar_init(&sm.o_full[s], 1);
       mbar_init(&sm.y_full[s], GATE_WARPS);
-      mbar_init(&sm.o_empty[s], 2);  // the two warpgroups' stores
+      mbar_init(&sm.o_empty[s], EPI_WARPS);  // their stores
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sm.g_full[a], 1);
@@ -122,6 +123,8 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   };
   const uint32_t n_my = blockIdx.x < p.total_tiles ? (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
 
+  // 512 threads x 128 registers = 128 x (72 + 144 + 128 + 168)
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     if (elect_one()) {
       uint32_t it = 0;
@@ -176,17 +179,21 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         }
       }
     }
-  } else if (warp < 2 + LN_WARPS) {
-    const int row = (warp - 2) * 32 + lane;
+  } else if (warp >= 4 && warp < 8) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    const int row = (warp - 4) * 32 + lane;
     for (uint32_t it = 0; it < n_my; ++it) {
       const uint32_t stage = it % XSTAGES, phase = (it / XSTAGES) & 1;
       if (!mbar_wait(&sm.x_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      ln_row_sweeps(sm.x[stage], row, sm.gamma2, sm.beta2, p.eps);
+      uint4 v[16];
+      ln_load_row(sm.x[stage], row, v);
+      ln_row_words(v, sm.gamma2, sm.beta2, p.eps);
+      ln_store_row(sm.x[stage], row, v);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
     }
-  } else if (warp < 2 + LN_WARPS + GATE_WARPS) {  // o <- bf16(o * bf16(sigmoid(bf16(G))))
+  } else if (warp >= 8 && warp < 12) {  // o <- bf16(o * bf16(sigmoid(bf16(G))))
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     for (uint32_t it = 0; it < n_my; ++it) {
@@ -221,71 +228,76 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         mbar_arrive(&sm.g_empty[a]);
       }
     }
-  } else {
-    const int quarter = warp & 3, half = (warp - 2 - LN_WARPS - GATE_WARPS) >> 2;  // 64 channels per warpgroup
-    const int row = quarter * 32 + lane;
-    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 128 + half * 64;
+  } else if (warp >= 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 128;
     uint32_t it = 0;
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
       int o, t0;
       locate(tile, o, t0);
+      t0 += quarter * 32;  // the warp's first pair
       const uint32_t a = it & 1, aph = (it >> 1) & 1;
-      uint8_t* stage_out = sm.o[it % OSTAGES] + half * SLAB_BYTES;
-      uint4 res[8];  // residual of the warp's 32 pairs, 8 lanes to a pair's 64 channels (whole lines)
+      uint4 res[2][8];  // residual of the warp's 32 pairs, 8 lanes to a pair's 64 channels (whole lines)
       if (p.residual) {
-        const int t = t0 + quarter * 32 + (lane >> 3);
-        const __nv_bfloat16* src = p.residual + static_cast<long long>(o) * p.os_outer + half * 64 + (lane & 7) * 8;
+        const int t = t0 + (lane >> 3);
+        const __nv_bfloat16* src = p.residual + static_cast<long long>(o) * p.os_outer + (lane & 7) * 8;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          res[q] = t + 4 * q < p.n_inner ? *reinterpret_cast<const uint4*>(src + static_cast<long long>(t + 4 * q) * p.os_inner)
-                                      : make_uint4(0u, 0u, 0u, 0u);
+        for (int q = 0; q < 16; ++q)
+          res[q >> 3][q & 7] = t + 4 * (q & 7) < p.n_inner
+                                   ? *reinterpret_cast<const uint4*>(src + static_cast<long long>(t + 4 * (q & 7)) * p.os_inner +
+                                                                     (q >> 3) * 64)
+                                   : make_uint4(0u, 0u, 0u, 0u);
       }
-      // (the vote makes the outcome of the bounded wait the same for all 128 threads, which meet at
-      // a barrier below)
-      if (!named_barrier_and(1 + half, 128, mbar_wait(&sm.out_full[a], aph, p.status, ST_TIMEOUT_EPILOGUE))) break;
+      if (!mbar_wait(&sm.out_full[a], aph, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      __syncwarp();
       tc_fence_after();
 #pragma unroll
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        uint32_t v[16];
-        tmem_ld16(lane_addr + a * 256 + chunk * 16, v);
-        tmem_ld_wait();
+      for (int half = 0; half < 2; ++half) {  // 64 channels at a time
+        uint8_t* stage_out = sm.o[it % OSTAGES] + half * SLAB_BYTES;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint32_t u[4];
+        for (int chunk = 0; chunk < 4; ++chunk) {
+          uint32_t v[16];
+          tmem_ld16(lane_addr + a * 256 + half * 64 + chunk * 16, v);
+          tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
-          *reinterpret_cast<uint4*>(stage_out + sw128_offset(row, chunk * 2 + q)) = make_uint4(u[0], u[1], u[2], u[3]);
+          for (int q = 0; q < 2; ++q) {
+            uint32_t u[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              u[e] = pack_bf16x2(__uint_as_float(v[8 * q + 2 * e]), __uint_as_float(v[8 * q + 2 * e + 1]));
+            *reinterpret_cast<uint4*>(stage_out + sw128_offset(row, chunk * 2 + q)) = make_uint4(u[0], u[1], u[2], u[3]);
+          }
         }
-      }
-      if (p.residual) {  // the caller's z + update, one more bf16 rounding, in the residual's arrangement
-        __syncwarp();
+        if (p.residual) {  // the caller's z + update, one more bf16 rounding, in the residual's arrangement
+          __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          uint4* ptr = reinterpret_cast<uint4*>(stage_out + sw128_offset(quarter * 32 + 4 * q + (lane >> 3), lane & 7));
-          uint4 u = *ptr;
-          u.x = bf16x2_add(res[q].x, u.x);
-          u.y = bf16x2_add(res[q].y, u.y);
-          u.z = bf16x2_add(res[q].z, u.z);
-          u.w = bf16x2_add(res[q].w, u.w);
-          *ptr = u;
+          for (int q = 0; q < 8; ++q) {
+            uint4* ptr = reinterpret_cast<uint4*>(stage_out + sw128_offset(quarter * 32 + 4 * q + (lane >> 3), lane & 7));
+            uint4 u = *ptr;
+            u.x = bf16x2_add(res[half][q].x, u.x);
+            u.y = bf16x2_add(res[half][q].y, u.y);
+            u.z = bf16x2_add(res[half][q].z, u.z);
+            u.w = bf16x2_add(res[half][q].w, u.w);
+            *ptr = u;
+          }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0 && t0 < p.n_inner) {  // rows past n_inner are outside the tensor and are not written
+          tma_store_3d(&tm_out, stage_out + quarter * 4096, half * 64, t0, o);
+          tma_store_commit();
         }
       }
       tc_fence_before();
-      fence_proxy_async();
-      named_barrier(1 + half, 128);
-      if (leader) {  // rows past n_inner are outside the tensor and are not written
-        tma_store_3d(&tm_out, stage_out, half * 64, t0, o);
-        tma_store_commit();
-      }
-      if (lane == 0) mbar_arrive(&sm.out_empty[a]);
-      if (leader) {
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&sm.out_empty[a]);
         tma_store_wait_read();
         mbar_arrive(&sm.o_empty[it % OSTAGES]);
       }
     }
-    if (leader) tma_store_wait_all();
+    if (lane == 0) tma_store_wait_all();
   }
 
   if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
@@ -329,7 +341,7 @@ extern "C" int b200tri_triatt_finish(const b200tri_triatt_finish_args* a, b200tr
   {  // the result through the caller's strides (the ending node lands transposed back in place)
     const uint64_t dims[3] = {128, (uint64_t)a->n_inner, (uint64_t)a->n_outer};
     const uint64_t str[2] = {(uint64_t)a->os_inner * 2, (uint64_t)a->os_outer * 2};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, 32, 1};
     int rc = make_tmap(&tm_out, a->out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
   }

@@ -180,7 +180,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     uint32_t phase = 0;
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
       if (!mbar_wait(&sm.in_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      ln_row_sweeps(sm.x[stage], r, sm.gamma_in, sm.beta_in, p.eps);
+      ln_row_sweeps<4>(sm.x[stage], r, sm.gamma_in, sm.beta_in, p.eps);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.xn_full[stage]);

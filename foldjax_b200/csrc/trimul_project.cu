@@ -16,8 +16,8 @@
 //   warp 0       TMA producer: weights once (128 KiB, resident), x tiles in a 2-stage ring
 //   warp 1       MMA issuer: 4 groups (p_a, g_a, p_b, g_b) of 128x128x128 per tile
 //   warps 2-9    layer norm, in place in the tile TMA delivered (two threads per pair)
-//   warps 10-17  epilogue: TMEM -> sigmoid gate -> mask -> bf16 -> shared memory -> TMA store,
-//                64 pairs per warpgroup (stored by the threads themselves, each 64-byte run went to
+//   warps 10-25  epilogue: TMEM -> sigmoid gate -> mask -> bf16 -> shared memory -> TMA store,
+//                32 pairs per warpgroup (stored by the threads themselves, each 64-byte run went to
 //                another channel plane: 32 lines per instruction, and the L1 pipe was the bound)
 // TMEM: four 128-column accumulators; the a-half and the b-half are released
 // separately so the MMAs of the next tile overlap the epilogue of this one.
@@ -35,13 +35,13 @@ constexpr int XSTAGES = 2;
 constexpr int TILE_BYTES = 2 * SLAB_BYTES;  // 32 KiB: 128 pairs x 128 channels bf16
 constexpr int W_BYTES = 8 * SLAB_BYTES;     // 128 KiB: 4 groups x 2 K-slabs
 constexpr int MASK_SLOTS = 4;
-constexpr int LN_WARPS = 8, EPI_WARPS = 8;
+constexpr int LN_WARPS = 8, EPI_WARPS = 16;  // the sigmoids of a tile want many warps: see below
 constexpr int THREADS = 64 + (LN_WARPS + EPI_WARPS) * 32;
 
 struct Smem {
   uint8_t w[W_BYTES];  // group g (p_a, g_a, p_b, g_b): two boxes [128 in][64 out], MN-major
   uint8_t x[XSTAGES][TILE_BYTES];
-  uint8_t out[2][SLAB_BYTES];           // per epilogue warpgroup: [128 channels][64 pairs]
+  uint8_t out[4][SLAB_BYTES / 2];       // per epilogue warpgroup: [128 channels][32 pairs], 64-byte swizzle
   __nv_bfloat16 mask[MASK_SLOTS][128];  // mask.astype(bf16), as the reference casts it
   alignas(16) uint32_t gamma2[64], beta2[64];
   uint64_t w_full, x_full[XSTAGES], xn_full[XSTAGES], x_empty[XSTAGES], acc_full[2], acc_empty[2];
@@ -196,19 +196,19 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       }
     }
   } else {
-    // ---- epilogue: thread = output channel (TMEM lane), columns = pairs, 64 per warpgroup
+    // ---- epilogue: thread = output channel (TMEM lane), columns = pairs, 32 per warpgroup
     const int quarter = warp & 3, part = (warp - 2 - LN_WARPS) >> 2;
     const int chan = quarter * 32 + lane;
     const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 32;
     uint8_t* out = sm.out[part];
     uint32_t it = 0;
     bool alive = true;
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
       int o, t0;
       locate(tile, o, t0);
-      t0 += part * 64;
-      const uint32_t* mrow = reinterpret_cast<const uint32_t*>(sm.mask[it & (MASK_SLOTS - 1)]) + part * 32;
+      t0 += part * 32;
+      const uint32_t* mrow = reinterpret_cast<const uint32_t*>(sm.mask[it & (MASK_SLOTS - 1)]) + part * 16;
       for (int half = 0; half < 2; ++half) {
         // the previous tile must have left the staging buffer; the vote makes the outcome of the
         // bounded wait the same for all 128 threads, which meet at a barrier below
@@ -219,7 +219,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         }
         tc_fence_after();
 #pragma unroll
-        for (int chunk = 0; chunk < 4; ++chunk) {
+        for (int chunk = 0; chunk < 2; ++chunk) {
           uint32_t pr[16], gr[16];
           tmem_ld16(lane_addr + half * 256 + chunk * 16, pr);
           tmem_ld16(lane_addr + half * 256 + 128 + chunk * 16, gr);
@@ -238,7 +238,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
               const uint32_t sg = sigmoid_bf16x2(__uint_as_float(gr[c]), __uint_as_float(gr[c + 1]));
               packed[e] = bf16x2_mul(bf16x2_mul(sg, pv), mm[e]);
             }
-            *reinterpret_cast<uint4*>(out + sw128_offset(chan, chunk * 2 + q)) =
+            *reinterpret_cast<uint4*>(out + chan * 64 + (((chunk * 2 + q) ^ ((chan >> 1) & 3)) << 4)) =
                 make_uint4(packed[0], packed[1], packed[2], packed[3]);
           }
         }
@@ -311,15 +311,15 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
     int rc = make_weight_map(&tm_p, w_p, 128, 256, 128);
     if (rc || (rc = make_weight_map(&tm_g, w_g, 128, 256, 128))) return rc;
   }
-  CUtensorMap tm_out[2];  // (pair, row in block, channel, block), written as tiles of [128 channels][64 pairs]
+  CUtensorMap tm_out[2];  // (pair, row in block, channel, block), written as tiles of [128 channels][32 pairs]
   const int rpb = a->rows_per_block < a->n_outer ? a->rows_per_block : a->n_outer;
   for (int i = 0; i < 2; ++i) {
     const int blocks = (a->n_outer + rpb - 1) / rpb;
     const uint64_t dims[4] = {(uint64_t)a->n_inner, (uint64_t)rpb, 128, (uint64_t)blocks};
     const uint64_t str[3] = {(uint64_t)a->ld * 2, (uint64_t)a->chan_stride * 2,
                              (uint64_t)(blocks > 1 ? a->block_stride : a->chan_stride * 128) * 2};
-    const uint32_t box[4] = {64, 1, 128, 1};
-    int rc = make_tmap(&tm_out[i], i ? a->b : a->a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B128);
+    const uint32_t box[4] = {32, 1, 128, 1};
+    int rc = make_tmap(&tm_out[i], i ? a->b : a->a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B64);
     if (rc) return rc;
   }
   ProjParams p;
