@@ -8,11 +8,17 @@
 //   warp 1      MMA issuer     (128x256x16 tcgen05.mma, fp32 accumulators in
 //                               TMEM, two accumulators so the epilogue of one
 //                               tile overlaps the main loop of the next)
-//   warps 2..5  epilogue       (TMEM -> registers -> bf16/fp32 -> global)
+//   warps 4-11  epilogue       two warpgroups, 128 columns each: TMEM -> bf16 -> shared memory ->
+//                              TMA store per warp, 32 rows x 64 columns at a time; float32 results
+//                              and running sums go to global memory directly
 // Tiles are walked channel by channel so the A_d/B_d panels of the channel in
 // flight (2 * N*N*2 bytes) stay in L2 while all SMs work on them.
 //
-// Bound: tensor pipe. Algorithmic work 2*128*n_i*n_j*n_k*n_src flop.
+// Bound: large n_k, the operand traffic into the SM (48 KiB per k step, 768 clocks at 64 B/clk,
+// against 512 of products); small n_k, the epilogue. Algorithmic work 2*128*n_i*n_j*n_k*n_src flop.
+// With one warpgroup whose threads stored 64 bytes of a row each (32 lines per instruction) a tile
+// of n = 200 took 11 400 clocks, four times its products and loads. Now 20 -> 15 us at n = 203, 71 -> 49
+// at 500 and 262 -> 228 at 1024.
 #include "host.cuh"
 #include "tc.cuh"
 
@@ -25,15 +31,18 @@ constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_BYTES = BN * BK * 2;  // 32 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + slack for 1 KiB alignment
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 8, STAGED = 32 * 128;  // bytes a warp stages: 32 rows x 64 bf16
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STAGED + 1024;  // + slack for 1 KiB alignment
+constexpr int THREADS = 128 + EPI_WARPS * 32;
 
 struct ContractParams {
   int n_i, n_j, n_src;
   ContractTerms terms;
   int kb_per_src;  // ceil(n_k / BK)
   int tiles_m, tiles_n;
-  long long total_tiles;
+  uint32_t total_tiles;
+  bool staged;  // the bf16 result is all that is wanted and a warp's 32 rows share a block
+  bool out_blocked;
   const float* acc_in;
   float* out_f32;
   __nv_bfloat16* out_bf16;
@@ -45,7 +54,7 @@ struct ContractParams {
 
 __global__ void __launch_bounds__(THREADS, 1)
 contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                const ContractParams p) {
+                const __grid_constant__ CUtensorMap tm_out, const ContractParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -63,7 +72,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);
+      mbar_init(&acc_empty[a], EPI_WARPS);
     }
     fence_barrier_init();
   }
@@ -79,17 +88,25 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   const uint32_t tmem_base = tmem_base_s;
 
   const int k_iters = p.n_src * p.kb_per_src;
-  const long long tiles_per_chan = static_cast<long long>(p.tiles_m) * p.tiles_n;
+  // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
+  const uint32_t tiles_per_chan = static_cast<uint32_t>(p.tiles_m) * p.tiles_n;
+  auto locate = [&](uint32_t tile, int& d, int& mi, int& nj) {
+    d = tile / tiles_per_chan;
+    const uint32_t rem = tile - d * tiles_per_chan;
+    mi = rem / p.tiles_n;
+    nj = rem - mi * p.tiles_n;
+  };
 
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x) {
-        const int d = static_cast<int>(tile / tiles_per_chan);
-        const int rem = static_cast<int>(tile % tiles_per_chan);
-        const int mi = rem / p.tiles_n, nj = rem % p.tiles_n;
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x) {
+        int d, mi, nj;
+        locate(tile, d, mi, nj);
+        const int a_block = mi * BM / p.a_rpb, a_row = mi * BM - a_block * p.a_rpb;
+        const int b_block = nj * BN / p.b_rpb, b_row = nj * BN - b_block * p.b_rpb;
         for (int s = 0; s < p.n_src && alive; ++s) {
           for (int kb = 0; kb < p.kb_per_src; ++kb) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
@@ -99,9 +116,9 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             uint8_t* sa = smem + stage * STAGE_BYTES;
             mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
             // rows are (block, row in block): a tile starts at block row0 / rpb
-            tma_load_5d(sa, &tm_a, &full_bar[stage], kb * BK, (mi * BM) % p.a_rpb, (mi * BM) / p.a_rpb, d,
+            tma_load_5d(sa, &tm_a, &full_bar[stage], kb * BK, a_row, a_block, d,
                         p.terms.n ? p.terms.a[s] : s);
-            tma_load_5d(sa + A_BYTES, &tm_b, &full_bar[stage], kb * BK, (nj * BN) % p.b_rpb, (nj * BN) / p.b_rpb, d,
+            tma_load_5d(sa + A_BYTES, &tm_b, &full_bar[stage], kb * BK, b_row, b_block, d,
                         p.terms.n ? p.terms.b[s] : s);
             if (++stage == STAGES) {
               stage = 0;
@@ -118,7 +135,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       uint32_t phase = 0;
       uint32_t it = 0;
       bool alive = true;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
@@ -145,23 +162,78 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         if (alive) umma_commit(&acc_full[acc]);
       }
     }
-  } else {
+  } else if (warp >= 4) {
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
+    const int cols = (warp - 4) >> 2;  // which 128 columns of the tile
+    uint8_t* staging = smem + STAGES * STAGE_BYTES + (warp - 4) * STAGED;
     uint32_t it = 0;
-    for (long long tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
-      const int d = static_cast<int>(tile / tiles_per_chan);
-      const int rem = static_cast<int>(tile % tiles_per_chan);
-      const int mi = rem / p.tiles_n, nj = rem % p.tiles_n;
+    for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      int d, mi, nj;
+      locate(tile, d, mi, nj);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       if (!mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      __syncwarp();
       tc_fence_after();
-      const int row = mi * BM + quarter * 32 + lane;
+      const int row0 = mi * BM + quarter * 32, row = row0 + lane;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      if (p.staged) {
+        const int block = row0 / p.out_rpb, in_block = row0 - block * p.out_rpb;
+#pragma unroll 1
+        for (int half = cols * 2; half < cols * 2 + 2; ++half) {
+          const int col0 = nj * BN + half * 64;
+          if (row0 >= p.n_i || col0 >= p.n_j) break;
+          uint32_t r[2][32];
+          tmem_ld32(taddr + half * 64, r[0]);
+          tmem_ld32(taddr + half * 64 + 32, r[1]);
+          if (lane == 0) tma_store_wait_read();  // the staging rows are free again
+          tmem_ld_wait();
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            uint32_t u[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              u[e] = pack_bf16x2(__uint_as_float(r[q >> 2][8 * (q & 3) + 2 * e]), __uint_as_float(r[q >> 2][8 * (q & 3) + 2 * e + 1]));
+            *reinterpret_cast<uint4*>(staging + sw128_offset(lane, q)) = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (row0 + 32 <= p.n_i || !p.out_blocked) {
+            if (lane == 0) {  // what lies past n_i and n_j is outside the tensor and is not written
+              tma_store_4d(&tm_out, staging, col0, in_block, d, block);
+              tma_store_commit();
+            }
+          } else {  // the last block may end in rows that do not exist but lie inside the tensor
+            __nv_bfloat16* dst = p.out_bf16 + static_cast<long long>(block) * p.out_block_stride +
+                                 static_cast<long long>(d) * p.out_chan_stride +
+                                 static_cast<long long>(in_block) * p.out_ld + col0 + (lane & 7) * 8;
+            const int left = p.n_j - col0 - (lane & 7) * 8;  // columns from this lane's chunk on
+            for (int rr = lane >> 3; rr < p.n_i - row0; rr += 4) {
+              const uint4 u = *reinterpret_cast<const uint4*>(staging + sw128_offset(rr, lane & 7));
+              if (left >= 8) {
+                *reinterpret_cast<uint4*>(dst + static_cast<long long>(rr) * p.out_ld) = u;
+              } else {
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  if (e < left)
+                    dst[static_cast<long long>(rr) * p.out_ld + e] =
+                        __ushort_as_bfloat16(static_cast<unsigned short>((e & 1) ? (w[e >> 1] >> 16) : (w[e >> 1] & 0xffffu)));
+              }
+            }
+            __syncwarp();
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        continue;
+      }
       const long long row_off = static_cast<long long>(row / p.out_rpb) * p.out_block_stride +
                                 static_cast<long long>(d) * p.out_chan_stride +
                                 static_cast<long long>(row % p.out_rpb) * p.out_ld;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
 #pragma unroll 1
-      for (int chunk = 0; chunk < BN / 32; ++chunk) {
+      for (int chunk = cols * 4; chunk < cols * 4 + 4; ++chunk) {
         uint32_t r[32];
         tmem_ld32(taddr + chunk * 32, r);
         tmem_ld_wait();
@@ -223,6 +295,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
     }
+    if (lane == 0) tma_store_wait_all();
   }
 
   // Tear-down. After a timeout give in-flight bulk copies time to land first.
@@ -310,7 +383,21 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
     int rc = make_tmap(&tm_b, a->b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, box, Swz::B128);
     if (rc) return rc;
   }
+  const int out_rows = a->out_rows_per_block > 0 && a->out_rows_per_block < a->n_i ? a->out_rows_per_block : a->n_i;
+  const int out_blocks = (a->n_i + out_rows - 1) / out_rows;
+  const bool staged = a->out_bf16 && !a->out_f32 && !a->acc_in && (out_blocks == 1 || out_rows % 32 == 0);
+  CUtensorMap tm_out = tm_a;  // (unused without staging)
+  if (staged) {
+    const uint64_t dims[4] = {(uint64_t)a->n_j, (uint64_t)out_rows, (uint64_t)channels, (uint64_t)out_blocks};
+    const uint64_t str[3] = {(uint64_t)a->out_ld * 2, (uint64_t)a->out_chan_stride * 2,
+                             (uint64_t)(out_blocks > 1 ? a->out_block_stride : a->out_chan_stride * channels) * 2};
+    const uint32_t box[4] = {64, 32, 1, 1};
+    int rc = make_tmap(&tm_out, a->out_bf16, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B128);
+    if (rc) return rc;
+  }
   ContractParams p;
+  p.staged = staged;
+  p.out_blocked = out_blocks > 1;
   p.n_i = a->n_i;
   p.n_j = a->n_j;
   p.n_src = terms.n ? terms.n : a->n_src;
@@ -318,7 +405,9 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   p.kb_per_src = (a->n_k + BK - 1) / BK;
   p.tiles_m = (a->n_i + BM - 1) / BM;
   p.tiles_n = (a->n_j + BN - 1) / BN;
-  p.total_tiles = static_cast<long long>(channels) * p.tiles_m * p.tiles_n;
+  const long long tiles = static_cast<long long>(channels) * p.tiles_m * p.tiles_n;
+  B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "contract: too many tiles (%lld)", tiles);
+  p.total_tiles = static_cast<uint32_t>(tiles);
   p.acc_in = a->acc_in;
   p.out_f32 = a->out_f32;
   p.out_bf16 = static_cast<__nv_bfloat16*>(a->out_bf16);
@@ -326,7 +415,7 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   p.out_chan_stride = a->out_chan_stride;
   p.a_rpb = a_rows;
   p.b_rpb = b_rows;
-  p.out_rpb = (a->out_rows_per_block > 0 && a->out_rows_per_block < a->n_i) ? a->out_rows_per_block : (a->n_i > 0 ? a->n_i : 1);
+  p.out_rpb = out_rows;
   p.out_block_stride = a->out_block_stride;
   p.status = status;
 
@@ -334,10 +423,10 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(contract_kernel), SMEM_BYTES);
     if (rc) return rc;
   }
-  const long long grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+  const long long grid = tiles < sm_count() ? tiles : sm_count();
   {
     TimedLaunch timed(K_TRIMUL_CONTRACT, stream);
     return launch(contract_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, stream, true,
-                  tm_a, tm_b, p);
+                  tm_a, tm_b, tm_out, p);
   }
 }
