@@ -82,7 +82,14 @@ struct GemmShape {
 //   EPI, CTAS                                     epilogue warps, CTAs per SM
 //   struct Params                                 arguments
 //   load_a / load_b(maps, params, seg, k, tile, piece, dst, bar)  one piece of one k step
-//   epilogue(params, m_tile, n_tile, split, accumulators, quarter, col0, col1, lane)   columns [col0, col1)
+//   Pre, prefetch(params, m_tile, n_tile, quarter, col0, col1, lane, pre)   what the epilogue reads from
+//                     global memory, requested before the accumulators are waited for (or NoPrefetch)
+//   epilogue(params, m_tile, n_tile, split, accumulators, quarter, col0, col1, lane, pre)   columns [col0, col1)
+struct NoPrefetch {
+  struct Pre {};
+  template <class... A>
+  static __device__ __forceinline__ void prefetch(const A&...) {}
+};
 template <class P>
 constexpr int gemm_acc_count() {  // accumulators of one segment
   return P::NMAIN + (P::PA * P::PB > 1 ? 1 : 0);
@@ -276,6 +283,8 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
       int split, m_tile, n_tile;
       locate(tile, split, m_tile, n_tile);
       const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
+      typename P::Pre pre;
+      P::prefetch(ep, m_tile, n_tile, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
       if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) break;
       tc_fence_after();
       Accum<P> acc;
@@ -285,7 +294,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
         const int per = (g.kb[seg] + g.splits - 1) / g.splits;
         acc.used[seg] = min(g.kb[seg], (split + 1) * per) - split * per;
       }
-      P::epilogue(ep, m_tile, n_tile, split, acc, quarter, part * SHARE, (part + 1) * SHARE, lane);
+      P::epilogue(ep, m_tile, n_tile, split, acc, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);

@@ -369,6 +369,25 @@ int map_rows(CUtensorMap* out, const void* base, int k, int n, long long s_inner
   return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, dims, str, bx, Swz::B128);
 }
 
+// A bf16 row's share of an epilogue warp, one row per thread: requested before the accumulators are
+// waited for. Loaded after them it cost a gate tile two memory latencies, most of its time.
+template <int COLS>
+struct RowPrefetch {
+  uint4 row[COLS > 0 ? COLS / 8 : 1];
+  __device__ __forceinline__ void load(const __nv_bfloat16* src, int left) {  // `left` columns exist
+#pragma unroll
+    for (int q = 0; q < COLS / 8; ++q)
+      row[q] = 8 * q < left ? reinterpret_cast<const uint4*>(src)[q] : make_uint4(0u, 0u, 0u, 0u);
+  }
+  // Eight neighbouring values rounded to bf16, with the prefetched residual added (one more rounding).
+  __device__ __forceinline__ void store(__nv_bfloat16* dst, int q, bool residual, const float* v) const {
+    uint4 u = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+    if (residual)
+      u = make_uint4(bf16x2_add(row[q].x, u.x), bf16x2_add(row[q].y, u.y), bf16x2_add(row[q].z, u.z), bf16x2_add(row[q].w, u.w));
+    *reinterpret_cast<uint4*>(dst) = u;
+  }
+};
+
 // Tile `tile` of rows walked `box` inner positions at a time.
 struct RowTile {
   int b, o, t0;
@@ -404,20 +423,30 @@ struct GluPolicy {
     const RowTile r(n_tile, p.n, p.tiles_t, BN);
     tma_load_5d(dst, &maps.b[0], bar, k, r.t0, r.o, r.b, piece);
   }
+  static constexpr bool BF = PIECES == 1;
+  struct Pre {
+    float mask[BN / (EPI / 4) / 16];  // of pair lane & 15 of each run of 16
+  };
+  static __device__ void prefetch(const Params& p, int, int n_tile, int, int col0, int, int lane, Pre& pre) {
+    const RowTile rt(n_tile, p.n, p.tiles_t, BN);
+#pragma unroll
+    for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
+      const int t = rt.t0 + col0 + 16 * i + (lane & 15);
+      pre.mask[i] = p.mask && t < p.n ? p.mask[rt.b * p.ms_b + rt.o * p.ms_o + t * p.ms_i] : 1.0f;
+    }
+  }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<GluPolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
-    constexpr bool BF = PIECES == 1;
+                                  int col0, int, int lane, const Pre& pre) {
     const RowTile rt(n_tile, p.n, p.tiles_t, BN);
     const int c = m_tile * GEMM_BM + quarter * 32 + lane;
     const int chan = c < p.c_h ? c : c - p.c_h;
     __nv_bfloat16* dst = (c < p.c_h ? p.a : p.b) +
                          ((static_cast<long long>(rt.b) * p.c_h + chan) * p.n + rt.o) * p.ld + rt.t0;
-#pragma unroll 1
-    for (int col = col0; col < col1; col += 16) {
+#pragma unroll
+    for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
+      const int col = col0 + 16 * i;
       if (rt.t0 + col >= p.n) break;
-      const int t = rt.t0 + col + (lane & 15);
-      float mk = 1.0f;
-      if (p.mask && t < p.n) mk = Rb<BF>::r(p.mask[rt.b * p.ms_b + rt.o * p.ms_o + t * p.ms_i]);
+      const float mk = Rb<BF>::r(pre.mask[i]);
       float v[16], g[16];
       acc.load(0, col, v);
       acc.load(1, col, g);
@@ -455,6 +484,15 @@ struct OutGatePolicy {
     O* out;
     bool aligned;
   };
+  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
+    if constexpr (BF) {
+      if (!p.res || !p.aligned) return;
+      const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
+      const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
+      pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0);
+    }
+  }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int seg, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
     const RowTile r(m_tile, p.n, p.tiles_j, GEMM_BM);
@@ -465,13 +503,13 @@ struct OutGatePolicy {
     gemm_load_mn(&maps.b[seg], dst, bar, BN / 64, n_tile * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<OutGatePolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
+                                  int col0, int, int lane, const Pre& pre) {
     const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
     const int j = rt.t0 + quarter * 32 + lane;
     const long long off = ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z;
-#pragma unroll 1
-    for (int col = col0; col < col1; col += 16) {
-      const int c0 = n_tile * BN + col;
+#pragma unroll(BF ? 4 : 1)
+    for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
+      const int col = col0 + 16 * i, c0 = n_tile * BN + col;
       if (c0 >= p.c_z) break;
       float v[16], g[16];
       acc.load(0, col, v);
@@ -490,8 +528,15 @@ struct OutGatePolicy {
       }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        if (c0 + 8 * q < p.c_z)
+        if (c0 + 8 * q < p.c_z) {
+          if constexpr (BF) {
+            if (p.aligned) {
+              pre.store(p.out + off + c0 + 8 * q, 2 * i + q, p.res != nullptr, v + 8 * q);
+              continue;
+            }
+          }
           store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+        }
     }
   }
 };
@@ -499,7 +544,7 @@ struct OutGatePolicy {
 // q / sqrt(d), k: rows [piece][pair][hd]. v: transposed, [piece][(b, o)][hd][ld]. bias: [b][head][o][ld] in the trunk dtype. Column tiles walk
 // the four weights in turn.
 template <int PIECES, int NM, int BN_>
-struct QkvbPolicy {
+struct QkvbPolicy : NoPrefetch {
   static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
@@ -507,7 +552,7 @@ struct QkvbPolicy {
   struct Params {
     int n, hd, heads, tiles_w, ld;
     uint32_t pairs;
-    float q_scale;
+    float q_scale, q_scale_inv;
     long long row_piece, v_piece;  // elements between pieces of q / k and of v
     __nv_bfloat16 *q, *k, *vt;
     void* bias;
@@ -523,7 +568,7 @@ struct QkvbPolicy {
     gemm_load_mn(&maps.b[w], dst, bar, BN / 64, (n_tile - w * p.tiles_w) * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvbPolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
+                                  int col0, int col1, int lane, const Pre&) {
     const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
     const uint32_t bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
     const int w = which(p, n_tile);
@@ -538,7 +583,10 @@ struct QkvbPolicy {
         __nv_bfloat16* dst = (w ? p.k : p.q) + static_cast<long long>(pair) * p.hd + c0;
         if (w == 0)
 #pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = Rb<BF>::r(v[e]) / p.q_scale;
+          // bf16: the product with the rounded reciprocal rounds like the quotient. The divisor is an odd
+          // integer below 256 times a power of two and the dividend has 8 bits, so that the quotient is
+          // representable or at least 1e-5 away from a rounding boundary.
+          for (int e = 0; e < 16; ++e) v[e] = BF ? round_bf16(v[e]) * p.q_scale_inv : v[e] / p.q_scale;
 #pragma unroll
         for (int q = 0; q < 2; ++q)
           if (c0 + 8 * q < p.hd) store_eight<PIECES>(dst + 8 * q, p.row_piece, v + 8 * q);
@@ -583,6 +631,14 @@ struct GatePolicy {
     const float* o;
     __nv_bfloat16* y;
   };
+  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
+    if constexpr (BF) {
+      const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
+      const int c0 = n_tile * BN + col0;
+      pre.load(p.y + pair * p.hd + c0, pair < p.pairs ? p.hd - c0 : 0);
+    }
+  }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
     tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
@@ -592,11 +648,11 @@ struct GatePolicy {
     gemm_load_mn(&maps.b[0], dst, bar, BN / 64, n_tile * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<GatePolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
+                                  int col0, int, int lane, const Pre& pre) {
     const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
-#pragma unroll 1
-    for (int col = col0; col < col1; col += 16) {
-      const int c0 = n_tile * BN + col;
+#pragma unroll(BF ? 4 : 1)
+    for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
+      const int col = col0 + 16 * i, c0 = n_tile * BN + col;
       if (c0 >= p.hd) break;
       float g[16];
       acc.load(0, col, g);
@@ -605,14 +661,13 @@ struct GatePolicy {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         if (c0 + 8 * q >= p.hd) break;
-        if (BF) {
-          uint4* ptr = reinterpret_cast<uint4*>(p.y + off + 8 * q);
-          uint4 w = *ptr;
+        if constexpr (BF) {
+          uint4 w = pre.row[2 * i + q];
           w.x = bf16x2_mul(w.x, sigmoid_bf16x2(g[8 * q + 0], g[8 * q + 1]));
           w.y = bf16x2_mul(w.y, sigmoid_bf16x2(g[8 * q + 2], g[8 * q + 3]));
           w.z = bf16x2_mul(w.z, sigmoid_bf16x2(g[8 * q + 4], g[8 * q + 5]));
           w.w = bf16x2_mul(w.w, sigmoid_bf16x2(g[8 * q + 6], g[8 * q + 7]));
-          *ptr = w;
+          *reinterpret_cast<uint4*>(p.y + off + 8 * q) = w;
         } else {
           float v[8];
 #pragma unroll
@@ -648,6 +703,19 @@ struct ProjOutPolicy {
     O* out;
     bool aligned;
   };
+  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  static __device__ long long offset(const Params& p, uint32_t pair) {
+    const uint32_t n = p.n, bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
+    return b * p.s_b + o * p.s_o + t * p.s_i;
+  }
+  static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
+    if constexpr (BF) {
+      if (!p.res || !p.aligned) return;
+      const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane;
+      const int c0 = n_tile * BN + col0;
+      pre.load(p.res + offset(p, pair) + c0, pair < p.pairs ? p.c_z - c0 : 0);
+    }
+  }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
     tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
@@ -657,21 +725,27 @@ struct ProjOutPolicy {
     gemm_load_mn(&maps.b[0], dst, bar, BN / 64, n_tile * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<ProjOutPolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
-    const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
-    const uint32_t bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
-    const long long off = b * p.s_b + o * p.s_o + t * p.s_i;
-#pragma unroll 1
-    for (int col = col0; col < col1; col += 16) {
-      const int c0 = n_tile * BN + col;
+                                  int col0, int, int lane, const Pre& pre) {
+    const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane;
+    const long long off = offset(p, pair);
+#pragma unroll(BF ? 4 : 1)
+    for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
+      const int col = col0 + 16 * i, c0 = n_tile * BN + col;
       if (c0 >= p.c_z) break;
       float v[16];
       acc.load(0, col, v);
       if (pair >= p.pairs) continue;
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        if (c0 + 8 * q < p.c_z)
+        if (c0 + 8 * q < p.c_z) {
+          if constexpr (BF) {
+            if (p.aligned) {
+              pre.store(p.out + off + c0 + 8 * q, 2 * i + q, p.res != nullptr, v + 8 * q);
+              continue;
+            }
+          }
           store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+        }
     }
   }
 };
@@ -924,7 +998,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         const int tiles_w = (hd + Pol::BN - 1) / Pol::BN;
         const GemmShape g = {m_tiles, 3 * tiles_w + (heads + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
         const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
-        return launch_piece_gemm<Pol>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, pairs * hd,
+        return launch_piece_gemm<Pol>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
                                                 ws + pl.bias},
                                       stream, true);

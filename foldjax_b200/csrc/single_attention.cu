@@ -301,7 +301,7 @@ __global__ void pad_weight_kernel(const __nv_bfloat16* __restrict__ src, int k, 
 //
 // [q | k | v | g] in one launch: column tiles of 64 walk the four weights in turn. q and k leave as
 // pieces, v as transposed pieces (both as the token attention reads them), the gate in float32.
-struct QkvgPolicy {
+struct QkvgPolicy : NoPrefetch {
   static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = 8, CTAS = 1;
@@ -321,7 +321,7 @@ struct QkvgPolicy {
     gemm_load_mn(&maps.b[p.first_w + n_tile / p.tiles_per_w], dst, bar, 1, n_tile % p.tiles_per_w * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvgPolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
+                                  int col0, int col1, int lane, const Pre&) {
     const int row = m_tile * GEMM_BM + quarter * 32 + lane;
     const int which = p.first_w + n_tile / p.tiles_per_w;
     const long long plane = static_cast<long long>(p.rows) * p.c, off = static_cast<long long>(row) * p.c;
@@ -372,7 +372,7 @@ struct QkvgPolicy {
 };
 
 // float32 partial sums, one plane per K split.
-struct PartialPolicy {
+struct PartialPolicy : NoPrefetch {
   static constexpr int BN = 64, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = 8, CTAS = 1;
@@ -389,7 +389,7 @@ struct PartialPolicy {
     gemm_load_mn(&maps.b[0], dst, bar, 1, n_tile * BN, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int split, const Accum<PartialPolicy>& acc,
-                                  int quarter, int col0, int col1, int lane) {
+                                  int quarter, int col0, int col1, int lane, const Pre&) {
     const int row = m_tile * GEMM_BM + quarter * 32 + lane;
 #pragma unroll 1
     for (int col = col0; col < col1; col += 16) {
@@ -408,7 +408,7 @@ struct PartialPolicy {
 
 // 64 columns of x @ fc1 beside the same 64 of x @ fc2; silu(a) * b leaves as pieces
 // (transition.py:108).
-struct SwigluPolicy {
+struct SwigluPolicy : NoPrefetch {
   static constexpr int BN = 128, PA = 3, PB = 1, NSEG = 1, NMAIN = 3;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = 8, CTAS = 1;
@@ -426,7 +426,7 @@ struct SwigluPolicy {
     for (int w = 0; w < 2; ++w) gemm_load_mn(&maps.b[w], dst + w * 8192, bar, 1, n_tile * 64, k, piece);
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<SwigluPolicy>& acc, int quarter,
-                                  int col0, int col1, int lane) {
+                                  int col0, int col1, int lane, const Pre&) {
     const int row = m_tile * GEMM_BM + quarter * 32 + lane;
     const long long plane = static_cast<long long>(p.rows) * p.pitch;
 #pragma unroll 1
