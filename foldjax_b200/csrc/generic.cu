@@ -129,8 +129,8 @@ __global__ void weight_kernel(const WeightJobs jobs) {
 }
 
 // ------------------------------------------------------------------ layer norm + gather
-// xn[piece][(b, o, t)][:] = LN(x[b][o * xs_o + t * xs_i + :]). A warp takes W successive t of one
-// row, each in registers (V channel pairs per lane), so that the loads of all of them are in
+// xn[piece][(b, o, t)][:] = LN(x[b][o * xs_o + t * xs_i + :]). A warp takes a few successive t of
+// one row, each in the registers of a group of lanes, so that the loads of all of them are in
 // flight together. Optionally the pair's mask bias of the attention core, mb[(b, o)][t] (the
 // pitch padding with the last pair of a row).
 // Bound: HBM / L2 traffic. The grid is (t, o, b): no divisions.
@@ -142,7 +142,7 @@ struct LnArgs {
   const void* bias;
   float eps;
   __nv_bfloat16* xn;
-  bool aligned;  // x is read two channels at a time
+  bool aligned, aligned_params;  // x, and scale and bias, start on a 16-byte boundary
   float* mb;     // or null
   const float* mask;
   long long ms_b, ms_o, ms_i;
@@ -150,106 +150,126 @@ struct LnArgs {
   int mb_ld;
 };
 constexpr int LN_WARPS = 8;
-template <bool BF, int V, int W>
+// Eight neighbouring values of a row as floats (p 16-byte aligned, or anywhere).
+template <bool BF, typename X>
+__device__ __forceinline__ void load_eight(const X* p, bool aligned, float (&v)[8]) {
+  if (aligned) {
+    uint4 raw[BF ? 1 : 2];
+#pragma unroll
+    for (int w = 0; w < (BF ? 1 : 2); ++w) raw[w] = reinterpret_cast<const uint4*>(p)[w];
+    const X* x = reinterpret_cast<const X*>(raw);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = static_cast<float>(x[e]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = static_cast<float>(p[e]);
+  }
+}
+// L neighbouring lanes per row, K chunks of eight channels per lane, R rows of a lane group in
+// flight. (With a row per warp and two channels per lane the 64-channel case took 24 us for
+// 160 000 rows, half of it the five exchanges of every sum; three are left.)
+template <bool BF, int L, int K, int R>
 __global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a) {
   using X = typename std::conditional<BF, __nv_bfloat16, float>::type;
-  using X2 = typename std::conditional<BF, __nv_bfloat162, float2>::type;
+  constexpr int GROUPS = 32 / L, ROWS = GROUPS * R;  // rows of a warp
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31;
-  const int t0 = (blockIdx.x * LN_WARPS + (threadIdx.x >> 5)) * W, o = blockIdx.y, b = blockIdx.z;
+  const int t0 = (blockIdx.x * LN_WARPS + (threadIdx.x >> 5)) * ROWS, o = blockIdx.y, b = blockIdx.z;
   if (t0 >= a.n) return;
   const int bo = b * a.n + o;
   if (a.mb) {
     float* row = a.mb + static_cast<long long>(bo) * a.mb_ld;
-    if (lane < W && t0 + lane < a.n)
+    if (lane < ROWS && t0 + lane < a.n)
       row[t0 + lane] = a.mask ? fmaxf(a.inf * (a.mask[b * a.ms_b + o * a.ms_o + (t0 + lane) * a.ms_i] - 1.0f), SPLIT_MASK_MIN) : 0.f;
-    if (t0 + W >= a.n)
+    if (t0 + ROWS >= a.n)
       for (int e = a.n + lane; e < a.mb_ld; e += 32) row[e] = SPLIT_MASK_PAD;
   }
-  const X* src = static_cast<const X*>(a.x) + b * a.xs_b + o * a.xs_o + t0 * a.xs_i;
-  float2 v[W][V];
+  const int c0 = (lane % L) * 8, t_lane = t0 + lane / L;  // the lane's rows are t_lane + GROUPS * r
+  const X* src = static_cast<const X*>(a.x) + b * a.xs_b + o * a.xs_o;
+  float v[R][K][8];
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    const X* row = src + (t0 + w < a.n ? w : 0) * a.xs_i;
+  for (int r = 0; r < R; ++r) {
+    const X* row = src + min(t_lane + GROUPS * r, a.n - 1) * a.xs_i;
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      const int i = 2 * (lane + 32 * e);
-      v[w][e] = make_float2(0.f, 0.f);
-      if (i < a.c) {
-        if (a.aligned) {
-          const X2 q = *reinterpret_cast<const X2*>(row + i);
-          v[w][e] = make_float2(static_cast<float>(q.x), static_cast<float>(q.y));
-        } else {
-          v[w][e] = make_float2(static_cast<float>(row[i]), static_cast<float>(row[i + 1]));
-        }
+    for (int k = 0; k < K; ++k) {
+      const int c = c0 + k * L * 8;
+      if (c < a.c) {
+        load_eight<BF>(row + c, a.aligned, v[r][k]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[r][k][e] = 0.f;
       }
     }
   }
   const float inv_c = 1.0f / a.c;
-  float s[W], q[W];
+  float s[R], q[R];
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    s[w] = 0.f;
+  for (int r = 0; r < R; ++r) {
+    s[r] = 0.f;
 #pragma unroll
-    for (int e = 0; e < V; ++e) s[w] += v[w][e].x + v[w][e].y;
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) s[r] += v[r][k][e] + v[r][k][e + 1];
   }
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1)
+  for (int d = L / 2; d > 0; d >>= 1)
 #pragma unroll
-    for (int w = 0; w < W; ++w) s[w] += __shfl_xor_sync(0xffffffffu, s[w], d);
+    for (int r = 0; r < R; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], d);
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    s[w] *= inv_c;
-    q[w] = 0.f;
+  for (int r = 0; r < R; ++r) {
+    s[r] *= inv_c;
+    q[r] = 0.f;
 #pragma unroll
-    for (int e = 0; e < V; ++e)
-      if (2 * (lane + 32 * e) < a.c) {
-        const float dx = v[w][e].x - s[w], dy = v[w][e].y - s[w];
-        q[w] = fmaf(dx, dx, fmaf(dy, dy, q[w]));
-      }
+    for (int k = 0; k < K; ++k)
+      if (c0 + k * L * 8 < a.c)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float d = v[r][k][e] - s[r];
+          q[r] = fmaf(d, d, q[r]);
+        }
   }
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1)
+  for (int d = L / 2; d > 0; d >>= 1)
 #pragma unroll
-    for (int w = 0; w < W; ++w) q[w] += __shfl_xor_sync(0xffffffffu, q[w], d);
+    for (int r = 0; r < R; ++r) q[r] += __shfl_xor_sync(0xffffffffu, q[r], d);
 #pragma unroll
-  for (int w = 0; w < W; ++w) q[w] = 1.0f / sqrtf(q[w] * inv_c + a.eps);
-  const X* scale = static_cast<const X*>(a.scale);
-  const X* bias = static_cast<const X*>(a.bias);
+  for (int r = 0; r < R; ++r) q[r] = 1.0f / sqrtf(q[r] * inv_c + a.eps);
   const long long plane = static_cast<long long>(a.batch) * a.n * a.n * a.c;
-  __nv_bfloat16* dst = a.xn + (static_cast<long long>(bo) * a.n + t0) * a.c;
+  __nv_bfloat16* dst = a.xn + (static_cast<long long>(bo) * a.n + t_lane) * a.c;
 #pragma unroll
-  for (int e = 0; e < V; ++e) {
-    const int i = 2 * (lane + 32 * e);
-    if (i >= a.c) continue;
-    const float g[2] = {static_cast<float>(scale[i]), static_cast<float>(scale[i + 1])};
-    const float h[2] = {static_cast<float>(bias[i]), static_cast<float>(bias[i + 1])};
+  for (int k = 0; k < K; ++k) {
+    const int c = c0 + k * L * 8;
+    if (c >= a.c) continue;
+    float g[8], h[8];
+    load_eight<BF>(static_cast<const X*>(a.scale) + c, a.aligned_params, g);
+    load_eight<BF>(static_cast<const X*>(a.bias) + c, a.aligned_params, h);
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      if (t0 + w >= a.n) break;
-      float r[2] = {v[w][e].x, v[w][e].y};
+    for (int r = 0; r < R; ++r) {
+      if (t_lane + GROUPS * r >= a.n) break;
+      float u[8];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {  // cast before the affine step
-        const float normed = Rb<BF>::r((r[u] - s[w]) * q[w]);
-        r[u] = Rb<BF>::r(Rb<BF>::r(normed * g[u]) + h[u]);
-      }
-      store_pair<BF ? 1 : 3>(dst + w * a.c + i, plane, r[0], r[1]);
+      for (int e = 0; e < 8; ++e)  // cast before the affine step
+        u[e] = Rb<BF>::r(Rb<BF>::r(Rb<BF>::r((v[r][k][e] - s[r]) * q[r]) * g[e]) + h[e]);
+      store_eight<BF ? 1 : 3>(dst + GROUPS * r * a.c + c, plane, u);
     }
   }
 }
 
 template <bool BF>
 int launch_ln_gather(LnArgs a, cudaStream_t stream, bool pdl) {
-  a.aligned = (reinterpret_cast<uintptr_t>(a.x) & (BF ? 3 : 7)) == 0;
-  auto go = [&](auto kernel, int w) {
-    const dim3 grid((a.n + LN_WARPS * w - 1) / (LN_WARPS * w), static_cast<unsigned>(a.n), static_cast<unsigned>(a.batch));
+  a.aligned = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0;  // (rows are multiples of eight values apart)
+  a.aligned_params = ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.bias)) & 15) == 0;
+  auto go = [&](auto kernel, int rows) {
+    const int per_block = LN_WARPS * rows;
+    const dim3 grid((a.n + per_block - 1) / per_block, static_cast<unsigned>(a.n), static_cast<unsigned>(a.batch));
     return launch(kernel, grid, dim3(LN_WARPS * 32), 0, stream, pdl, a);
   };
-  if (a.c <= 64) return go(ln_gather_kernel<BF, 1, 4>, 4);
-  if (a.c <= 128) return go(ln_gather_kernel<BF, 2, 4>, 4);
-  if (a.c <= 384) return go(ln_gather_kernel<BF, 6, 2>, 2);
-  return go(ln_gather_kernel<BF, 16, 1>, 1);
+  if (a.c <= 64) return go(ln_gather_kernel<BF, 8, 1, 2>, 8);
+  if (a.c <= 128) return go(ln_gather_kernel<BF, 16, 1, 2>, 4);
+  if (a.c <= 256) return go(ln_gather_kernel<BF, 32, 1, 2>, 2);
+  if (a.c <= 384) return go(ln_gather_kernel<BF, 16, 3, 1>, 2);
+  return go(ln_gather_kernel<BF, 32, 4, 1>, 1);
 }
 
 // ------------------------------------------------------------ tri-mult: LN of the contraction
@@ -259,21 +279,23 @@ int launch_ln_gather(LnArgs a, cudaStream_t stream, bool pdl) {
 // memory. A lane owns one word of that row - two j in bf16, one in float32 - and a warp an
 // eighth of the channels, so that the statistics are plain sums per lane (one exchange of eight
 // partial sums each) and nothing is shuffled: 40 instructions per pair where one warp per pair
-// took 209. Eight neighbouring channels leave per lane as one 16-byte store.
+// took 209. Eight neighbouring channels per lane are 16 bytes; in bf16, up to 64 * G channels, they
+// are put together in shared memory (over the values, when all have been read) and leave as one
+// contiguous run: stored by the lanes themselves they went to 64 rows, half a sector each.
 constexpr int LNT_WARPS = 8;
 template <bool BF>
 constexpr int lnt_j() {
   return BF ? 64 : 32;
 }
 inline int lnt_smem(int c_h) { return c_h * 128 + 2 * LNT_WARPS * 64 * 4; }
-template <bool BF>
+template <bool BF, int G>
 __global__ void __launch_bounds__(LNT_WARPS * 32)
 ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, const void* __restrict__ scale_,
                         const void* __restrict__ bias_, float eps, long long pairs, __nv_bfloat16* __restrict__ tn) {
   using X = typename std::conditional<BF, __nv_bfloat16, float>::type;
   constexpr int JT = lnt_j<BF>(), JL = JT / 32;  // j of a block, of a lane
   extern __shared__ uint32_t tile[];             // [c_h][32 words], then the partial sums
-  float* part = reinterpret_cast<float*>(tile + c_h * 32);
+  float* part = reinterpret_cast<float*>(tile + (c_h + 63) / 64 * 64 * 32);
   pdl_wait();
   pdl_trigger();
   const int i = blockIdx.y, b = blockIdx.z, j0 = blockIdx.x * JT;
@@ -329,6 +351,46 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
   }
   const X* scale = static_cast<const X*>(scale_);
   const X* bias = static_cast<const X*>(bias_);
+  if constexpr (G > 0) {
+    uint4 out[G][JL];
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int g = warp + k * LNT_WARPS;
+      if (g >= groups) continue;
+      float v[JL][8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int c = g * 8 + e;
+        const uint32_t w = tile[c * 32 + lane];
+        const float sc = static_cast<float>(scale[c]), bi = static_cast<float>(bias[c]);
+#pragma unroll
+        for (int u = 0; u < JL; ++u) v[u][e] = Rb<BF>::r(Rb<BF>::r((value(w, u) - s[u]) * q[u]) * sc) + bi;
+      }
+#pragma unroll
+      for (int u = 0; u < JL; ++u)
+        out[k][u] = make_uint4(pack_bf16x2(v[u][0], v[u][1]), pack_bf16x2(v[u][2], v[u][3]), pack_bf16x2(v[u][4], v[u][5]),
+                               pack_bf16x2(v[u][6], v[u][7]));
+    }
+    __syncthreads();
+    // rows of `pitch` 16-byte chunks, chunks swapped by the lane that writes them: no bank conflicts
+    const int pitch = (groups + 7) & ~7;
+    uint4* rows = reinterpret_cast<uint4*>(tile);
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int g = warp + k * LNT_WARPS;
+      if (g >= groups) continue;
+#pragma unroll
+      for (int u = 0; u < JL; ++u) rows[(lane * JL + u) * pitch + (g ^ (lane & 7))] = out[k][u];
+    }
+    __syncthreads();
+    uint4* dst = reinterpret_cast<uint4*>(tn + ((static_cast<long long>(b) * n + i) * n + j0) * c_h);
+    const int count = min(JT, n - j0) * groups;
+    for (int idx = threadIdx.x; idx < count; idx += LNT_WARPS * 32) {
+      const int j = idx / groups, g = idx - j * groups;
+      dst[idx] = rows[j * pitch + (g ^ ((j / JL) & 7))];
+    }
+    return;
+  }
   __nv_bfloat16* dst = tn + ((static_cast<long long>(b) * n + i) * n + j0 + lane * JL) * c_h;
   for (int g = warp; g < groups; g += LNT_WARPS) {
     float v[JL][8];
@@ -350,11 +412,18 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
 template <bool BF>
 int launch_ln_channel_major(const void* t, int n, int batch, int ld, int c_h, const void* scale, const void* bias, float eps,
                             __nv_bfloat16* tn, cudaStream_t stream) {
-  const int rc = ensure_smem_limit(reinterpret_cast<const void*>(ln_channel_major_kernel<BF>), lnt_smem(1024));
-  if (rc) return rc;
   const dim3 grid((n + lnt_j<BF>() - 1) / lnt_j<BF>(), static_cast<unsigned>(n), static_cast<unsigned>(batch));
-  return launch(ln_channel_major_kernel<BF>, grid, dim3(LNT_WARPS * 32), lnt_smem(c_h), stream, true, t, n, ld, c_h, scale, bias,
-                eps, static_cast<long long>(batch) * n * n, tn);
+  auto go = [&](auto kernel) {
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), lnt_smem(1024));
+    if (rc) return rc;
+    return launch(kernel, grid, dim3(LNT_WARPS * 32), lnt_smem(round_up(c_h, 64)), stream, true, t, n, ld, c_h, scale, bias, eps,
+                  static_cast<long long>(batch) * n * n, tn);
+  };
+  if constexpr (BF) {
+    if (c_h <= 128) return go(ln_channel_major_kernel<BF, 2>);
+    if (c_h <= 384) return go(ln_channel_major_kernel<BF, 6>);
+  }
+  return go(ln_channel_major_kernel<BF, 0>);
 }
 
 // ------------------------------------------------------------------- product policies
