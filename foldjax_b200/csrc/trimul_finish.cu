@@ -21,7 +21,11 @@
 //                waited for
 // TMEM: 2 x (D1, D2) so the epilogue overlaps the next tile's MMAs.
 //
-// Bound: HBM (read t and x, write out: 3 * n_i*n_j*128*2 bytes; + residual).
+// Bound: HBM (read t and x, write out: 3 * n_i*n_j*128*2 bytes; + residual) by the bytes; in fact
+// the layer norms, chains of 192 dependent additions per row beside 900 other instructions: 6700
+// clocks a tile for x, at five warps per scheduler. n = 1024: 247 us with one warpgroup for both
+// layer norms and one thread per row of the residual, 226 so (123 by the bytes). Measured and not
+// better: x in registers (spills), alternate warpgroups per tile, t transposed by ldmatrix.
 #include "host.cuh"
 #include "ln.cuh"
 #include "tc.cuh"
@@ -247,7 +251,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
       if (leader) tma_store_wait_read();
       if (!named_barrier_and(1 + half, 128, mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE))) break;
       tc_fence_after();
-#pragma unroll
+#pragma unroll 1  // (the roles' unrolled code competes for the instruction cache)
       for (int chunk = 0; chunk < 4; ++chunk) {
         uint32_t g[16], o[16];
         tmem_ld16(lane_addr + acc * 256 + chunk * 16, g);
