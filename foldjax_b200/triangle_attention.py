@@ -44,8 +44,8 @@ def triangle_attention_forward(
     """Boltz TriangleAttention, starting or ending node.
 
     ``x`` is ``[B, N, N, 128]`` (or ``[N, N, 128]``), ``mask`` ``[B, N, N]`` or None (= ones).
-    ``dtype`` selects the trunk: "bfloat16" (default) or "float32" (every step in float32 on
-    the CUDA cores, the reference's float32 trunk, 1e-4); a float32 CUDA tensor selects
+    ``dtype`` selects the trunk: "bfloat16" (default) or "float32" (float32 accuracy
+    throughout, the reference's float32 trunk, 1e-4); a float32 CUDA tensor selects
     float32 by itself. ``params`` is the reference's mapping ``{"layer_norm": {scale,
     bias}, "linear": {kernel [128, 4]}, "mha": {"linear_q" | "linear_k" |
     "linear_v" | "linear_g" | "linear_o": {kernel [128, 128]}}}``. Device tensors in

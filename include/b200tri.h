@@ -260,8 +260,8 @@ typedef struct {
   int32_t dtype; /* B200TRI_DTYPE_*, as in b200tri_trimul_args */
   /* 0 = 128. x is [n, n, c_z]; linear (w_bias) [c_z, heads]; linear_q/k/v/g [c_z, heads *
    * head_dim]; linear_o [heads * head_dim, c_z]. bf16 with c_z = 128 and 4 heads x 32 runs the
-   * tensor-core kernels; other shapes (head widths 8, 16, 24, 32, 48, 64) or float32 run the
-   * general CUDA-core path. */
+   * fused kernels; other shapes (head widths 8, 16, 24, 32, 48, 64) or float32 run the general
+   * path (unfused tensor-core products). */
   int32_t c_z;
   int32_t batch; /* as in b200tri_trimul_args */
 } b200tri_triatt_args;
