@@ -321,6 +321,236 @@ int launch_piece_gemm(const GemmMaps& maps, GemmShape g, const typename P::Param
   return launch(piece_gemm_kernel<P>, dim3(grid), dim3(gemm_threads<P>()), gemm_smem_bytes<P>(), stream, pdl, maps, g, ep);
 }
 
+// The same product with one operand resident: a CTA keeps the rows of a slow-direction tile (A, or
+// with M_FAST the B tile that both segments share) for all its k steps and streams the other
+// operand for a run of fast-direction tiles. A 128 x 128 tile reads 32 KiB per k step into the SM
+// otherwise, 512 clocks for 256 of products; so it reads half. The resident k steps have barriers
+// of their own and are refilled one by one behind the last tile's products.
+// Gated projection, 65 536 pairs x 384 -> 768 channels: 104 -> 94 us; 160 000 x 64 -> 256: 72 -> 67;
+// q, k, v and bias, 160 000 x 64: 56 -> 45 (384 channels: 96 -> 107, left streaming).
+constexpr int RES_KB = 8, RES_STAGES = 8;  // most k steps kept, most streamed stages
+template <class P>
+constexpr int gemm_res_bytes() {
+  return P::M_FAST ? P::PB * P::BN * 128 : P::PA * GEMM_A_BYTES;
+}
+template <class P>
+constexpr int gemm_stream_bytes() {
+  return gemm_stage_bytes<P>() - gemm_res_bytes<P>();
+}
+template <class P>
+int gemm_res_stages(int kb) {  // 0: does not fit
+  const int left = 222 * 1024 - kb * gemm_res_bytes<P>();
+  const int stages = kb > RES_KB || left < 0 ? 0 : left / gemm_stream_bytes<P>();
+  return stages < 3 ? 0 : stages > RES_STAGES ? RES_STAGES : stages;
+}
+struct GemmRuns {
+  int fast, parts, stages;  // fast-direction tiles, runs they are cut into, streamed stages
+  uint32_t units;           // slow-direction tiles x parts
+};
+
+template <class P>
+__global__ void __launch_bounds__(gemm_threads<P>(), 1)
+piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, const GemmRuns runs,
+                           const typename P::Params ep) {
+  static_assert(P::CTAS == 1 && (P::M_FAST || P::NSEG == 1), "one operand for all segments");
+  constexpr int RES = gemm_res_bytes<P>(), STREAM = gemm_stream_bytes<P>();
+  constexpr int SEG = gemm_acc_count<P>() * P::BN, ACC = P::NSEG * SEG;
+  constexpr uint32_t NBUF = 2 * ACC <= 512 ? 2 : 1;
+  constexpr int USED = NBUF * ACC, TMEM_COLS = USED <= 64 ? 64 : USED <= 128 ? 128 : USED <= 256 ? 256 : 512;
+  static_assert(NBUF * ACC <= 512, "tile does not fit");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int kbs = g.kb[0], stages = runs.stages;
+  uint8_t* ring = smem + kbs * RES;
+  __shared__ uint64_t res_full[RES_KB], res_empty[RES_KB], full_bar[RES_STAGES], empty_bar[RES_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_s;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0 && lane == 0) {
+    for (int s = 0; s < P::NSEG; ++s) tma_prefetch_desc(&maps.a[s]);
+    tma_prefetch_desc(&maps.b[0]);
+    for (int s = 0; s < RES_KB; ++s) {
+      mbar_init(&res_full[s], 1);
+      mbar_init(&res_empty[s], 1);
+    }
+    for (int s = 0; s < RES_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], P::EPI);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_base_s, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t tmem_base = tmem_base_s;
+  auto locate = [&](uint32_t unit, int& slow, int& f0, int& f1) {
+    const uint32_t s = unit / static_cast<uint32_t>(runs.parts), part = unit - s * runs.parts;
+    slow = s;
+    f0 = part * runs.fast / runs.parts;
+    f1 = (part + 1) * runs.fast / runs.parts;
+  };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0, u = 0;
+      bool alive = true;
+      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, ++u) {
+        int slow, f0, f1;
+        locate(unit, slow, f0, f1);
+        for (int f = f0; f < f1 && alive; ++f) {
+          const int m_tile = P::M_FAST ? f : slow, n_tile = P::M_FAST ? slow : f;
+          for (int seg = 0; seg < P::NSEG && alive; ++seg)
+            for (int kb = 0; kb < kbs; ++kb) {
+              if (f == f0 && seg == 0) {
+                if (!mbar_wait(&res_empty[kb], (u & 1) ^ 1, g.status, ST_TIMEOUT_PRODUCER)) {
+                  alive = false;
+                  break;
+                }
+                mbar_expect_tx(&res_full[kb], RES);
+                for (int pc = 0; pc < (P::M_FAST ? P::PB : P::PA); ++pc) {
+                  if (P::M_FAST)
+                    P::load_b(maps, ep, 0, kb * GEMM_BK, n_tile, pc, smem + kb * RES + pc * P::BN * 128, &res_full[kb]);
+                  else
+                    P::load_a(maps, ep, 0, kb * GEMM_BK, m_tile, pc, smem + kb * RES + pc * GEMM_A_BYTES, &res_full[kb]);
+                }
+              }
+              if (!mbar_wait(&empty_bar[stage], phase ^ 1, g.status, ST_TIMEOUT_PRODUCER)) {
+                alive = false;
+                break;
+              }
+              mbar_expect_tx(&full_bar[stage], STREAM);
+              for (int pc = 0; pc < (P::M_FAST ? P::PA : P::PB); ++pc) {
+                if (P::M_FAST)
+                  P::load_a(maps, ep, seg, kb * GEMM_BK, m_tile, pc, ring + stage * STREAM + pc * GEMM_A_BYTES, &full_bar[stage]);
+                else
+                  P::load_b(maps, ep, seg, kb * GEMM_BK, n_tile, pc, ring + stage * STREAM + pc * P::BN * 128, &full_bar[stage]);
+              }
+              if (++stage == stages) {
+                stage = 0;
+                phase ^= 1;
+              }
+            }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, P::BN) | (P::A_MN ? UMMA_A_MN : 0u) | (P::B_MN ? UMMA_B_MN : 0u);
+      using T = Terms<P::PA, P::PB>;
+      int stage = 0;
+      uint32_t phase = 0, it = 0, u = 0;
+      bool alive = true;
+      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, ++u) {
+        int slow, f0, f1;
+        locate(unit, slow, f0, f1);
+        for (int f = f0; f < f1 && alive; ++f, ++it) {
+          const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
+          if (!mbar_wait(&acc_empty[buf], buf_phase ^ 1, g.status, ST_TIMEOUT_MMA)) {
+            alive = false;
+            break;
+          }
+          tc_fence_after();
+          for (int seg = 0; seg < P::NSEG && alive; ++seg)
+            for (int kb = 0; kb < kbs; ++kb) {
+              if ((f == f0 && seg == 0 && !mbar_wait(&res_full[kb], u & 1, g.status, ST_TIMEOUT_MMA)) ||
+                  !mbar_wait(&full_bar[stage], phase, g.status, ST_TIMEOUT_MMA)) {
+                alive = false;
+                break;
+              }
+              tc_fence_after();
+              const uint32_t kept = smem_u32(smem + kb * RES), streamed = smem_u32(ring + stage * STREAM);
+              const uint32_t sa = P::M_FAST ? streamed : kept, sb = P::M_FAST ? kept : streamed;
+#pragma unroll
+              for (int t = 0; t < T::N; ++t) {
+                const uint64_t adesc = P::A_MN ? umma_desc_mnmajor(sa + T::a(t) * GEMM_A_BYTES, 8192)
+                                               : umma_desc_kmajor(sa + T::a(t) * GEMM_A_BYTES, 128);
+                const uint64_t bdesc = P::B_MN ? umma_desc_mnmajor(sb + T::b(t) * P::BN * 128, 8192)
+                                               : umma_desc_kmajor(sb + T::b(t) * P::BN * 128, 128);
+                const bool lead = t == T::N - 1;
+                const uint32_t d_tmem = tmem_base + buf * ACC + seg * SEG + (lead ? kb % P::NMAIN : P::NMAIN) * P::BN;
+                const int fresh = lead ? kb < P::NMAIN : (kb == 0 && t == 0);  // first product into it
+#pragma unroll
+                for (int k = 0; k < GEMM_BK / 16; ++k)
+                  umma_bf16_ss(d_tmem, umma_desc_advance(adesc, P::A_MN ? k * 2048 : k * 32),
+                               umma_desc_advance(bdesc, P::B_MN ? k * 2048 : k * 32), idesc, !(fresh && k == 0));
+              }
+              umma_commit(&empty_bar[stage]);
+              if (f == f1 - 1 && seg == P::NSEG - 1) umma_commit(&res_empty[kb]);
+              if (++stage == stages) {
+                stage = 0;
+                phase ^= 1;
+              }
+            }
+          if (alive) umma_commit(&acc_full[buf]);
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    const int quarter = warp & 3, part = (warp - 4) >> 2;
+    constexpr int SHARE = P::BN / (P::EPI / 4);
+    uint32_t it = 0;
+    bool alive = true;
+    for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x) {
+      int slow, f0, f1;
+      locate(unit, slow, f0, f1);
+      for (int f = f0; f < f1; ++f, ++it) {
+        const int m_tile = P::M_FAST ? f : slow, n_tile = P::M_FAST ? slow : f;
+        const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
+        typename P::Pre pre;
+        P::prefetch(ep, m_tile, n_tile, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
+        if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) {
+          alive = false;
+          break;
+        }
+        tc_fence_after();
+        Accum<P> acc;
+        acc.base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
+#pragma unroll
+        for (int seg = 0; seg < P::NSEG; ++seg) acc.used[seg] = kbs;
+        P::epilogue(ep, m_tile, n_tile, 0, acc, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      }
+    }
+  }
+
+  if (*reinterpret_cast<volatile int*>(g.status) != ST_OK)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// The caller has checked gemm_res_stages<P>(kb) and that all segments have g.kb[0] k steps.
+template <class P>
+int launch_piece_gemm_resident(const GemmMaps& maps, GemmShape g, const typename P::Params& ep, cudaStream_t stream, bool pdl) {
+  g.status = device_status_word();
+  B200_REQUIRE(g.status != nullptr, B200TRI_ERR_CUDA, "gemm: no current CUDA device");
+  int rc = ensure_smem_limit(reinterpret_cast<const void*>(piece_gemm_resident_kernel<P>), 223 * 1024);
+  if (rc) return rc;
+  const int slow = P::M_FAST ? g.n_tiles : g.m_tiles;
+  GemmRuns r = {P::M_FAST ? g.m_tiles : g.n_tiles, 1, gemm_res_stages<P>(g.kb[0]), 0};
+  // enough runs that the last wave matters little, of at least two tiles
+  while (static_cast<long long>(slow) * r.parts < 6ll * sm_count() && r.fast / r.parts >= 4) r.parts *= 2;
+  const long long units = static_cast<long long>(slow) * r.parts;
+  B200_REQUIRE(units < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "gemm: too many tiles (%lld)", units);
+  r.units = static_cast<uint32_t>(units);
+  const unsigned grid = static_cast<unsigned>(units < sm_count() ? units : sm_count());
+  const size_t smem = static_cast<size_t>(g.kb[0]) * gemm_res_bytes<P>() + r.stages * gemm_stream_bytes<P>() + 1024;
+  return launch(piece_gemm_resident_kernel<P>, dim3(grid), dim3(gemm_threads<P>()), smem, stream, pdl, maps, g, r, ep);
+}
+
 // Activations: bf16 pieces [pieces][rows][k], row pitch `pitch` elements (a multiple of 8);
 // `box_rows` rows per load.
 inline int gemm_map_kmajor(CUtensorMap* out, const void* base, int pieces, long long rows, int k, long long pitch,

@@ -29,6 +29,8 @@
 
 #include <type_traits>
 
+#include <string.h>
+
 #include "att_split.cuh"
 #include "gemm.cuh"
 #include "host.cuh"
@@ -471,11 +473,11 @@ struct RowTile {
 // [a|b] = R(R(sigmoid(xn g)) * (xn p)) * mask, channel-major planes [piece][b * c_h + channel][o][ld].
 // Transposed product (a TMEM lane is a channel of the 2 * c_h, segment 0 the values, 1 the
 // gates), so that a thread stores runs of neighbouring pairs.
-template <int PIECES, int NM>
+template <int PIECES, int NM, bool RES = false>
 struct GluPolicy {
   static constexpr int BN = PIECES == 1 ? 128 : 64, PA = PIECES, PB = PIECES, NSEG = 2, NMAIN = NM;
   static constexpr bool A_MN = true, B_MN = false, M_FAST = true;
-  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   struct Params {
     int n, tiles_t, c_h, ld;
     long long piece;  // elements between pieces of a plane set
@@ -612,11 +614,11 @@ struct OutGatePolicy {
 
 // q / sqrt(d), k: rows [piece][pair][hd]. v: transposed, [piece][(b, o)][hd][ld]. bias: [b][head][o][ld] in the trunk dtype. Column tiles walk
 // the four weights in turn.
-template <int PIECES, int NM, int BN_>
+template <int PIECES, int NM, int BN_, bool RES = false>
 struct QkvbPolicy : NoPrefetch {
   static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
-  static constexpr int EPI = PIECES == 1 ? 8 : 16, CTAS = PIECES == 1 ? 2 : 1;
+  static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   static constexpr bool BF = PIECES == 1;
   struct Params {
     int n, hd, heads, tiles_w, ld;
@@ -821,6 +823,21 @@ struct ProjOutPolicy {
 
 int ksteps(int k) { return (k + GEMM_BK - 1) / GEMM_BK; }
 
+// The product with both operands streamed, or with one kept (`keep`, where its k steps fit beside
+// three stages of the other and there are several tiles to use it for).
+template <class Streamed, class Resident>
+int launch_either(const GemmMaps& maps, const GemmShape& g, const typename Streamed::Params& ep, bool keep,
+                  cudaStream_t stream) {
+  const int fast = Streamed::M_FAST ? g.m_tiles : g.n_tiles;
+  if (keep && fast >= 2 && gemm_res_stages<Resident>(g.kb[0]) > 0) {
+    typename Resident::Params r;
+    static_assert(sizeof(r) == sizeof(ep), "the same arguments");
+    memcpy(&r, &ep, sizeof(r));
+    return launch_piece_gemm_resident<Resident>(maps, g, r, stream, true);
+  }
+  return launch_piece_gemm<Streamed>(maps, g, ep, stream, true);
+}
+
 // ------------------------------------------------------------------------- workspaces
 struct Offsets {
   size_t off = 0;
@@ -954,16 +971,15 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       if ((rc = map_rows(&glu.b[0], at(pl.xn), c_z, n, c_z, static_cast<long long>(n) * c_z, nb, P, pairs * c_z, BN))) return rc;
       const int tiles_t = (n + BN - 1) / BN;
       const GemmShape g = {(2 * c_h + GEMM_BM - 1) / GEMM_BM, nb * n * tiles_t, 1, {ksteps(c_z), ksteps(c_z)}, nullptr};
-      auto go = [&](auto policy) {
+      auto go = [&](auto policy, auto kept) {
         using Pol = decltype(policy);
-        return launch_piece_gemm<Pol>(glu, g, {n, tiles_t, c_h, ld, piece, mask, nn, a->incoming ? 1ll : n,
-                                               a->incoming ? n : 1ll, at(pl.ap), at(pl.bp)},
-                                      stream, true);
+        return launch_either<Pol, decltype(kept)>(glu, g, {n, tiles_t, c_h, ld, piece, mask, nn, a->incoming ? 1ll : n,
+                                               a->incoming ? n : 1ll, at(pl.ap), at(pl.bp)}, true, stream);
       };
       if constexpr (BF)
-        rc = go(GluPolicy<1, 1>{});
+        rc = go(GluPolicy<1, 1>{}, GluPolicy<1, 1, true>{});
       else  // (a longer K wants its leading term in more accumulators than double buffering leaves room for)
-        rc = c_z <= 128 ? go(GluPolicy<3, 1>{}) : go(GluPolicy<3, 3>{});
+        rc = c_z <= 128 ? go(GluPolicy<3, 1>{}, GluPolicy<3, 1, true>{}) : go(GluPolicy<3, 3>{}, GluPolicy<3, 3, true>{});
       if (rc) return rc;
     }
     {
@@ -1062,20 +1078,21 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
     const int m_tiles = static_cast<int>((pairs + GEMM_BM - 1) / GEMM_BM);
     {
       if ((rc = gemm_map_kmajor(&proj.a[0], at(pl.xn), P, pairs, c_z, c_z, GEMM_BM))) return rc;
-      auto go = [&](auto policy) {
+      auto go = [&](auto policy, auto kept) {
         using Pol = decltype(policy);
         const int tiles_w = (hd + Pol::BN - 1) / Pol::BN;
         const GemmShape g = {m_tiles, 3 * tiles_w + (heads + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
         const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
-        return launch_piece_gemm<Pol>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
+        // (with more k steps two streaming CTAs per SM hide each other's epilogues better)
+        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
-                                                ws + pl.bias},
-                                      stream, true);
+                                                ws + pl.bias}, ksteps(c_z) <= 2, stream);
       };
       if constexpr (BF)
-        rc = hd <= 64 ? go(QkvbPolicy<1, 1, 64>{}) : go(QkvbPolicy<1, 1, 128>{});
+        rc = hd <= 64 ? go(QkvbPolicy<1, 1, 64>{}, QkvbPolicy<1, 1, 64, true>{})
+                     : go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
       else
-        rc = go(QkvbPolicy<3, 3, 64>{});
+        rc = go(QkvbPolicy<3, 3, 64>{}, QkvbPolicy<3, 3, 64, true>{});
       if (rc) return rc;
     }
     {
@@ -1104,7 +1121,8 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         return launch_piece_gemm<Pol>(gate, g, {pairs, hd, reinterpret_cast<const float*>(ws + pl.o), at(pl.y)}, stream, true);
       };
       if constexpr (BF)
-        rc = hd <= 64 ? go(GatePolicy<1, 1, 64>{}) : go(GatePolicy<1, 1, 128>{});
+        rc = hd <= 64 ? go(GatePolicy<1, 1, 64>{})
+                     : go(GatePolicy<1, 1, 128>{});
       else
         rc = go(GatePolicy<3, 3, 64>{});
       if (rc) return rc;
@@ -1117,7 +1135,8 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res)}, stream, true);
       };
       if constexpr (BF)
-        rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{}) : go(ProjOutPolicy<1, 1, 128>{});
+        rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{})
+                      : go(ProjOutPolicy<1, 1, 128>{});
       else
         rc = go(ProjOutPolicy<3, 3, 64>{});
       if (rc) return rc;
