@@ -4,10 +4,9 @@
 //
 // 128 independent N x N x N matrix products with both operands K-major, the
 // shape tcgen05.mma consumes directly. Persistent kernel, one CTA per SM:
-//   warp 0      TMA producer   (A 128x64 and B 256x64 bf16 tiles, 4-stage ring)
+//   warp 0      TMA producer   (A 128x64 or 256x64 and B 256x64 bf16 tiles, ring of 4 or 3 stages)
 //   warp 1      MMA issuer     (128x256x16 tcgen05.mma, fp32 accumulators in
-//                               TMEM, two accumulators so the epilogue of one
-//                               tile overlaps the main loop of the next)
+//                               TMEM, two accumulators: see Cfg)
 //   warps 4-11  epilogue       two warpgroups, 128 columns each: TMEM -> bf16 -> shared memory ->
 //                              TMA store per warp, 32 rows x 64 columns at a time; float32 results
 //                              and running sums go to global memory directly
@@ -18,7 +17,7 @@
 // against 512 of products); small n_k, the epilogue. Algorithmic work 2*128*n_i*n_j*n_k*n_src flop.
 // With one warpgroup whose threads stored 64 bytes of a row each (32 lines per instruction) a tile
 // of n = 200 took 11 400 clocks, four times its products and loads. Now 20 -> 15 us at n = 203, 71 -> 49
-// at 500 and 262 -> 228 at 1024.
+// at 500 and 262 -> 214 at 1024.
 #include "host.cuh"
 #include "tc.cuh"
 
@@ -26,13 +25,20 @@ namespace b200 {
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int STAGES = 4;
+constexpr int BM = 128, BN = 256, BK = 64;  // BM: rows of one accumulator
 constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_BYTES = BN * BK * 2;  // 32 KiB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_WARPS = 8, STAGED = 32 * 128;  // bytes a warp stages: 32 rows x 64 bf16
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STAGED + 1024;  // + slack for 1 KiB alignment
+// H = 1: tiles of 128 rows, two accumulators in turn, so that the epilogue of one tile overlaps the
+// products of the next. H = 2: tiles of 256 rows that share each k step's B, one accumulator per
+// half: 64 KiB into the SM per 1024 clocks of products instead of 48 per 512, and an epilogue that
+// only overlaps the loads of the next tile.
+// n = 768 / 1024 / 3072: 111 / 226 / 5300 us with H = 1, 108 / 214 / 5000 with H = 2.
+template <int H>
+struct Cfg {
+  static constexpr int STAGE_BYTES = H * A_BYTES + B_BYTES, STAGES = H == 1 ? 4 : 3;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STAGED + 1024;  // + slack for 1 KiB alignment
+};
 constexpr int THREADS = 128 + EPI_WARPS * 32;
 
 struct ContractParams {
@@ -52,9 +58,11 @@ struct ContractParams {
   int* status;
 };
 
+template <int H>
 __global__ void __launch_bounds__(THREADS, 1)
 contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                 const __grid_constant__ CUtensorMap tm_out, const ContractParams p) {
+  constexpr int STAGES = Cfg<H>::STAGES, STAGE_BYTES = Cfg<H>::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
@@ -72,7 +80,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], EPI_WARPS);
+      mbar_init(&acc_empty[a], EPI_WARPS / H);
     }
     fence_barrier_init();
   }
@@ -105,7 +113,13 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x) {
         int d, mi, nj;
         locate(tile, d, mi, nj);
-        const int a_block = mi * BM / p.a_rpb, a_row = mi * BM - a_block * p.a_rpb;
+        int a_block[H], a_row[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          const int row = (mi * H + h) * BM;
+          a_block[h] = row / p.a_rpb;
+          a_row[h] = row - a_block[h] * p.a_rpb;
+        }
         const int b_block = nj * BN / p.b_rpb, b_row = nj * BN - b_block * p.b_rpb;
         for (int s = 0; s < p.n_src && alive; ++s) {
           for (int kb = 0; kb < p.kb_per_src; ++kb) {
@@ -116,9 +130,11 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             uint8_t* sa = smem + stage * STAGE_BYTES;
             mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
             // rows are (block, row in block): a tile starts at block row0 / rpb
-            tma_load_5d(sa, &tm_a, &full_bar[stage], kb * BK, a_row, a_block, d,
-                        p.terms.n ? p.terms.a[s] : s);
-            tma_load_5d(sa + A_BYTES, &tm_b, &full_bar[stage], kb * BK, b_row, b_block, d,
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+              tma_load_5d(sa + h * A_BYTES, &tm_a, &full_bar[stage], kb * BK, a_row[h], a_block[h], d,
+                          p.terms.n ? p.terms.a[s] : s);
+            tma_load_5d(sa + H * A_BYTES, &tm_b, &full_bar[stage], kb * BK, b_row, b_block, d,
                         p.terms.n ? p.terms.b[s] : s);
             if (++stage == STAGES) {
               stage = 0;
@@ -136,10 +152,12 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       uint32_t it = 0;
       bool alive = true;
       for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
-        const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
+        // (one tile's accumulator out of two in turn, or one accumulator per half)
+        const uint32_t acc = it & 1, acc_phase = (H == 1 ? it >> 1 : it) & 1;
+        if (!mbar_wait(&acc_empty[H == 1 ? acc : 0], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
+        if (H == 2 && !mbar_wait(&acc_empty[1], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + (H == 1 ? acc * BN : 0);
         for (int ki = 0; ki < k_iters; ++ki) {
           if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_MMA)) {
             alive = false;
@@ -147,44 +165,49 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
-          const uint64_t adesc = umma_desc_kmajor(sa, 128);
-          const uint64_t bdesc = umma_desc_kmajor(sa + A_BYTES, 128);
+          const uint64_t bdesc = umma_desc_kmajor(sa + H * A_BYTES, 128);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_bf16_ss(d_tmem, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
-                         (ki | k) != 0);
+          for (int h = 0; h < H; ++h) {
+            const uint64_t adesc = umma_desc_kmajor(sa + h * A_BYTES, 128);
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              umma_bf16_ss(d_tmem + h * BN, umma_desc_advance(adesc, k * 32), umma_desc_advance(bdesc, k * 32), idesc,
+                           (ki | k) != 0);
+          }
           umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (alive) umma_commit(&acc_full[acc]);
+        if (alive) umma_commit(&acc_full[H == 1 ? acc : 0]);
       }
     }
   } else if (warp >= 4) {
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    const int cols = (warp - 4) >> 2;  // which 128 columns of the tile
+    const int group = (warp - 4) >> 2;  // which 128 columns of the tile, or which half of its rows
+    constexpr int COLS = BN / (3 - H);   // columns of a warp
+    const int first = H == 1 ? group * COLS : 0;
     uint8_t* staging = smem + STAGES * STAGE_BYTES + (warp - 4) * STAGED;
     uint32_t it = 0;
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
       int d, mi, nj;
       locate(tile, d, mi, nj);
-      const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      const uint32_t acc = H == 1 ? it & 1 : group, acc_phase = (H == 1 ? it >> 1 : it) & 1;
+      if (!mbar_wait(&acc_full[H == 1 ? acc : 0], acc_phase, p.status, ST_TIMEOUT_EPILOGUE)) break;
       __syncwarp();
       tc_fence_after();
-      const int row0 = mi * BM + quarter * 32, row = row0 + lane;
+      const int row0 = (mi * H + (H == 1 ? 0 : group)) * BM + quarter * 32, row = row0 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
       if (p.staged) {
         const int block = row0 / p.out_rpb, in_block = row0 - block * p.out_rpb;
 #pragma unroll 1
-        for (int half = cols * 2; half < cols * 2 + 2; ++half) {
-          const int col0 = nj * BN + half * 64;
+        for (int c = first; c < first + COLS; c += 64) {
+          const int col0 = nj * BN + c;
           if (row0 >= p.n_i || col0 >= p.n_j) break;
           uint32_t r[2][32];
-          tmem_ld32(taddr + half * 64, r[0]);
-          tmem_ld32(taddr + half * 64 + 32, r[1]);
+          tmem_ld32(taddr + c, r[0]);
+          tmem_ld32(taddr + c + 32, r[1]);
           if (lane == 0) tma_store_wait_read();  // the staging rows are free again
           tmem_ld_wait();
           __syncwarp();
@@ -233,7 +256,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                                 static_cast<long long>(d) * p.out_chan_stride +
                                 static_cast<long long>(row % p.out_rpb) * p.out_ld;
 #pragma unroll 1
-      for (int chunk = cols * 4; chunk < cols * 4 + 4; ++chunk) {
+      for (int chunk = first / 32; chunk < (first + COLS) / 32; ++chunk) {
         uint32_t r[32];
         tmem_ld32(taddr + chunk * 32, r);
         tmem_ld_wait();
@@ -403,9 +426,16 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   p.n_src = terms.n ? terms.n : a->n_src;
   p.terms = terms;
   p.kb_per_src = (a->n_k + BK - 1) / BK;
-  p.tiles_m = (a->n_i + BM - 1) / BM;
   p.tiles_n = (a->n_j + BN - 1) / BN;
-  const long long tiles = static_cast<long long>(channels) * p.tiles_m * p.tiles_n;
+  // Tiles of 128 or 256 rows, whichever is through first: rounds over the SMs times the clocks of a
+  // tile (loads, with the epilogue behind them where it is longer; products and epilogue).
+  const long long sms = sm_count(), kb = static_cast<long long>(p.n_src) * p.kb_per_src;
+  auto tiles_of = [&](int rows) { return static_cast<long long>(channels) * ((a->n_i + rows - 1) / rows) * p.tiles_n; };
+  const long long narrow = (tiles_of(BM) + sms - 1) / sms * (kb * 768 > 3000 ? kb * 768 : 3000);
+  const long long wide = (tiles_of(2 * BM) + sms - 1) / sms * (kb * 1024 + 3500);
+  const int halves = wide < narrow ? 2 : 1;
+  p.tiles_m = (a->n_i + halves * BM - 1) / (halves * BM);
+  const long long tiles = tiles_of(halves * BM);
   B200_REQUIRE(tiles < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "contract: too many tiles (%lld)", tiles);
   p.total_tiles = static_cast<uint32_t>(tiles);
   p.acc_in = a->acc_in;
@@ -419,14 +449,12 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   p.out_block_stride = a->out_block_stride;
   p.status = status;
 
-  {
-    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(contract_kernel), SMEM_BYTES);
+  const long long grid = tiles < sms ? tiles : sms;
+  auto go = [&](auto kernel, int smem) {
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), smem);
     if (rc) return rc;
-  }
-  const long long grid = tiles < sm_count() ? tiles : sm_count();
-  {
     TimedLaunch timed(K_TRIMUL_CONTRACT, stream);
-    return launch(contract_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, stream, true,
-                  tm_a, tm_b, tm_out, p);
-  }
+    return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), smem, stream, true, tm_a, tm_b, tm_out, p);
+  };
+  return halves == 2 ? go(contract_kernel<2>, Cfg<2>::SMEM_BYTES) : go(contract_kernel<1>, Cfg<1>::SMEM_BYTES);
 }

@@ -1,0 +1,47 @@
+"""The contraction in tiles of 256 rows (large n_k): a last tile whose second half has one row, a
+ragged one, or none, columns that end in partial blocks, one and two sources, bf16 results and
+float32 running sums; the last shape takes tiles of 128 rows.
+
+The float32 sum of m products is within m * 2^-23 of sum |a||b| of the exact one, however it is
+rounded; bf16 results are rounded once more (2^-8 relative)."""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("n_i,n_j,n_k,n_src", [(385, 513, 640, 2), (400, 40, 1000, 1), (521, 72, 1536, 1), (264, 300, 200, 1)])
+@pytest.mark.parametrize("running", [False, True])
+def test_contract(cuda_device, n_i, n_j, n_k, n_src, running):
+    from foldjax_b200 import _lib, _device as dev
+
+    torch.manual_seed(n_i + n_k)
+    ld, ld_j = (n_k + 7) // 8 * 8, (n_j + 7) // 8 * 8
+    a = torch.randn(n_src, 128, n_i, ld, device=cuda_device).bfloat16()
+    b = torch.randn(n_src, 128, n_j, ld, device=cuda_device).bfloat16()
+    a[..., n_k:] = b[..., n_k:] = 0
+    ref = sum(s.double() @ t.double().mT for s, t in zip(a, b))
+    bound = n_src * n_k * 2.0 ** -23 * sum(s.float().abs() @ t.float().abs().mT for s, t in zip(a, b))
+    out = torch.full((128, n_i, ld_j), float("nan"), dtype=torch.float32 if running else torch.bfloat16, device=cuda_device)
+    acc = torch.randn_like(out) if running else None
+    args = _lib.TrimulContractArgs(
+        n_i=n_i, n_j=n_j, n_k=n_k, n_src=n_src,
+        a=a.data_ptr(), a_ld=ld, a_chan_stride=n_i * ld, a_src_stride=128 * n_i * ld,
+        b=b.data_ptr(), b_ld=ld, b_chan_stride=n_j * ld, b_src_stride=128 * n_j * ld,
+        acc_in=acc.data_ptr() if running else None, out_f32=out.data_ptr() if running else None,
+        out_bf16=None if running else out.data_ptr(), out_ld=ld_j, out_chan_stride=n_i * ld_j,
+    )
+    _lib.check(_lib.load().b200tri_trimul_contract(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    _lib.device_status()
+    if running:
+        ref = ref + acc[..., :n_j].double()
+        bound = bound + 2.0 ** -23 * ref.abs()
+    else:
+        bound = bound * 1.01 + 2.0 ** -8 * ref.abs()
+    got = out[..., :n_j].double()
+    assert bool(((got - ref).abs() <= bound).all())  # (false where a value was not written)
