@@ -154,11 +154,16 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   B200_REQUIRE(!single || (a->s_out && a->c_s > 0 && a->heads_s > 0), B200TRI_ERR_INVALID,
                "pairformer: the single track needs s_out, c_s and heads_s");
   const b200tri_pairformer_block_params& first = a->params[0];
-  const int hidden_z = first.transition_z.hidden, hidden_s = single ? first.transition_s.hidden : 0;
+  int hidden_z = 0, hidden_s = 0;  // of the widest block: the scratch is shared by all of them
+  for (int layer = 0; layer < (a->stacked ? 1 : a->n_blocks); ++layer) {
+    const int hz = a->params[layer].transition_z.hidden, hs = a->params[layer].transition_s.hidden;
+    B200_REQUIRE(hz > 0 && (!single || hs > 0), B200TRI_ERR_INVALID, "pairformer: transition widths missing");
+    hidden_z = hz > hidden_z ? hz : hidden_z;
+    hidden_s = single && hs > hidden_s ? hs : hidden_s;
+  }
   B200_REQUIRE(!single || (a->heads_s <= 16 && a->c_s == a->heads_s * 24), B200TRI_ERR_UNSUPPORTED,
                "pairformer: the single track is built for up to 16 heads of width 24 (got c_s %d, %d heads)", a->c_s,
                a->heads_s);
-  B200_REQUIRE(hidden_z > 0 && (!single || hidden_s > 0), B200TRI_ERR_INVALID, "pairformer: transition widths missing");
   const Plan pl = plan(a->n, a->c_s, a->heads_s, hidden_z, hidden_s, single);
   B200_REQUIRE(a->workspace && a->workspace_bytes >= pl.total, B200TRI_ERR_WORKSPACE,
                "pairformer: workspace of %zu bytes needed, got %zu", pl.total, a->workspace_bytes);

@@ -161,7 +161,8 @@ def pairformer_forward(
     heads_s = packed[0].heads_s
     if single and c_s != heads_s * 24:
         raise ValueError(f"libb200tri is built for single-track heads of width 24; got c_s {c_s}, {heads_s} heads")
-    nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s, packed[0].hidden_z, packed[0].hidden_s)
+    nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s,
+                                  max(p.hidden_z for p in packed), max(p.hidden_s for p in packed))
     ws = dev.workspace(nbytes, "pairformer")
     z_out = torch.empty_like(zd)
     s_out = torch.empty_like(sd) if single else None

@@ -713,6 +713,7 @@ typedef struct {
   int32_t attention_first;
 } b200tri_pairformer_args;
 
+/* hidden_z, hidden_s: of the widest block (the blocks of a list share the scratch) */
 size_t b200tri_pairformer_workspace_bytes(int32_t n, int32_t c_s, int32_t heads_s, int32_t hidden_z, int32_t hidden_s);
 int b200tri_pairformer_forward(const b200tri_pairformer_args* args, b200tri_stream_t stream);
 

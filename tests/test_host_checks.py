@@ -81,3 +81,22 @@ def test_block_variant_names_are_checked_before_any_device_work():
     z = torch.zeros(1, 8, 8, 128, dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="Unsupported pairformer variant"):
         pairformer_forward([{}], None, z, None, None, variant="alphafold2")
+
+
+def test_pairformer_workspace_is_that_of_the_widest_block():
+    """The blocks of a list may have transitions of different widths, and all use the same scratch: a
+    workspace that only holds the first block's is refused before anything is launched."""
+    import ctypes as C
+
+    from foldjax_b200 import _lib
+
+    lib = _lib.load()
+    blocks = (_lib.PairformerBlockParams * 2)()
+    for block, (hidden_z, hidden_s) in zip(blocks, [(512, 384), (256, 1536)]):
+        block.transition_z.hidden, block.transition_s.hidden = hidden_z, hidden_s
+    first, widest = (lib.b200tri_pairformer_workspace_bytes(64, 384, 16, 512, h) for h in (384, 1536))
+    assert first < widest
+    address = 1 << 20  # (never dereferenced: the call is refused)
+    args = _lib.PairformerArgs(n=64, c_s=384, heads_s=16, n_blocks=2, params=blocks, z_in=address, z_out=address, s_in=address,
+                               s_out=address, workspace=address, workspace_bytes=widest - 1025)
+    assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_WORKSPACE

@@ -81,6 +81,29 @@ def test_trunk_call_equals_block_by_block_and_stacked_leaves(cuda_device):
     assert torch.equal(zd, dev.to_device(z, torch.bfloat16))  # inputs untouched
 
 
+def test_blocks_of_different_transition_widths(cuda_device):
+    """A list whose later block is wider than its first, in one call == block by block."""
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.pairformer import pairformer_forward
+
+    _, s, z, mask, pair_mask = _case(8, 72, 5)
+    rng = np.random.default_rng(8)
+    layers = []
+    for hidden_z, hidden_s in ((256, 384), (512, 1536), (128, 200)):
+        layer = orc.random_pairformer_params(rng, std=0.03, ln_noise=0.1)
+        for name, c, hidden in (("transition_z", 128, hidden_z), ("transition_s", 384, hidden_s)):
+            for fc, shape in (("fc1", (c, hidden)), ("fc2", (c, hidden)), ("fc3", (hidden, c))):
+                layer[name][fc] = {"kernel": (0.05 * rng.standard_normal(shape)).astype(np.float32)}
+        layers.append(orc.round_params(layer, "bfloat16"))
+    sd, zd = dev.to_device(s, torch.float32), dev.to_device(z, torch.bfloat16)
+    md, pmd = dev.to_device(mask, torch.float32), dev.to_device(pair_mask, torch.float32)
+    s_all, z_all = pairformer_forward(layers, sd, zd, md, pmd)
+    for layer in layers:
+        sd, zd = pairformer_forward([layer], sd, zd, md, pmd)
+    _lib.device_status()
+    assert torch.equal(z_all, zd) and torch.equal(s_all, sd)
+
+
 def test_pair_track_only_equals_the_per_op_block(cuda_device):
     from foldjax_b200 import _device as dev
     from foldjax_b200.block import triangle_block_forward
