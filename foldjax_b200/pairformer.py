@@ -14,7 +14,9 @@ the whole stack in one call.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import struct
+from functools import lru_cache
 from typing import Any, Mapping, Sequence
 
 import numpy as np
@@ -52,6 +54,23 @@ _FC1_Z, _PROJ_Z, _FC1_S = (leaves.index(path) for leaves, path in (
 _BLOCK_LAYOUT = struct.Struct(f"@{len(_PAIR_LEAVES)}Pi{len(_SINGLE_LEAVES)}Pi4x")
 
 
+def _transition_shapes(c: int, hidden: int) -> list[tuple[int, ...]]:
+    return [(c,), (c,), (c, hidden), (c, hidden), (hidden, c)]
+
+
+@lru_cache(maxsize=64)
+def _block_shapes(hidden_z: int, c_s: int, heads_s: int, hidden_s: int) -> list[tuple[int, ...]]:
+    """The shape of every parameter of a block, in the order of the leaves (c_s 0: pair track only)."""
+    c = C_Z
+    mul = [(c,), (c,), (c, 2 * c), (c, 2 * c), (c,), (c,), (c, c), (c, c)]
+    att = [(c,), (c,), (c, 4)] + 5 * [(c, c)]
+    shapes = 2 * mul + 2 * att + _transition_shapes(c, hidden_z)
+    if c_s:
+        sq = (c_s, c_s)
+        shapes += [(c_s,), (c_s,), sq, (c_s,), sq, sq, sq, (c,), (c,), (c, heads_s), sq] + _transition_shapes(c_s, hidden_s)
+    return shapes
+
+
 class _Packed:
     """Device copies of one block's (or one stack's) parameters and the C struct pointing at them."""
 
@@ -70,6 +89,17 @@ class _Packed:
         found = [_leaf(params, *path) for path in paths]
         self.keep += found
         return found
+
+    def check(self, c_s: int, heads_s: int, stacked: bool, blocks: int) -> None:
+        """The kernels get bare pointers: a leaf of another shape would be read past its end. Stacked
+        leaves carry a leading axis of at least ``blocks`` layers."""
+        want = _block_shapes(self.hidden_z, c_s, heads_s, self.hidden_s)
+        if not stacked and [t.shape for t in self.keep] == want:
+            return
+        for path, leaf, shape in zip(_PAIR_LEAVES + _SINGLE_LEAVES, self.keep, want):
+            if leaf.shape[-len(shape):] != shape or leaf.numel() < blocks * math.prod(shape):
+                raise ValueError(f"pairformer parameter {'.'.join(path)} has shape {tuple(leaf.shape)}, expected "
+                                 f"{shape}" + (f" behind an axis of {blocks} layers" if blocks > 1 else ""))
 
 
 #: what distinguishes the block of each model family at the level of this driver
@@ -161,6 +191,8 @@ def pairformer_forward(
     heads_s = packed[0].heads_s
     if single and c_s != heads_s * 24:
         raise ValueError(f"libb200tri is built for single-track heads of width 24; got c_s {c_s}, {heads_s} heads")
+    for p in packed:
+        p.check(c_s, heads_s, bool(stacked), blocks if stacked else 1)
     nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s,
                                   max(p.hidden_z for p in packed), max(p.hidden_s for p in packed))
     ws = dev.workspace(nbytes, "pairformer")

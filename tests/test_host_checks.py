@@ -100,3 +100,51 @@ def test_pairformer_workspace_is_that_of_the_widest_block():
     args = _lib.PairformerArgs(n=64, c_s=384, heads_s=16, n_blocks=2, params=blocks, z_in=address, z_out=address, s_in=address,
                                s_out=address, workspace=address, workspace_bytes=widest - 1025)
     assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_WORKSPACE
+
+
+@pytest.mark.parametrize("stacked", [False, True])
+@pytest.mark.parametrize("path,shape", [
+    (("tri_mul_out", "p_in", "kernel"), (128, 128)), (("tri_att_end", "linear", "kernel"), (128, 3)),
+    (("transition_z", "fc3", "kernel"), (256, 128)), (("transition_s", "fc2", "kernel"), (48, 96)),
+    (("attention", "proj_q", "bias"), (24,)), (("transition_s", "norm", "scale"), (47,))])
+def test_pairformer_parameters_of_another_shape_are_refused(monkeypatch, stacked, path, shape):
+    """A block's parameters go to the kernels as bare pointers, so their shapes are compared first."""
+    import numpy as np
+
+    from foldjax_b200 import _lib
+    from foldjax_b200.pairformer import pairformer_forward
+    from oracle import triangle_oracle as orc
+
+    class Reached(Exception):
+        pass
+
+    def reached(*_):
+        raise Reached
+
+    monkeypatch.setattr(dev, "require_cuda", lambda: None)
+    monkeypatch.setattr(dev, "to_device", lambda x, dtype=None, device=None: torch.as_tensor(x).to(dtype).contiguous())
+    monkeypatch.setattr(_lib, "workspace_bytes", reached)
+    blocks = 3
+    params = orc.random_pairformer_params(np.random.default_rng(0), c_s=48, heads_s=2)
+
+    def lead(node):
+        return {k: lead(v) for k, v in node.items()} if isinstance(node, dict) else np.stack([node] * blocks)
+
+    def call(p, n=blocks):
+        args = (torch.zeros(1, 8, 48), torch.zeros(1, 8, 8, 128), torch.ones(1, 8), torch.ones(1, 8, 8))
+        return pairformer_forward(p, *args, num_blocks=n) if stacked else pairformer_forward([p], *args)
+
+    good = lead(params) if stacked else params
+    with pytest.raises(Reached):
+        call(good)
+    if stacked:
+        with pytest.raises(Reached):
+            call(good, blocks - 1)  # the first layers of a longer stack
+        with pytest.raises(ValueError, match="behind an axis of 4 layers"):
+            call(good, blocks + 1)
+    node = good
+    for key in path[:-1]:
+        node = node[key]
+    node[path[-1]] = np.zeros((blocks,) * stacked + shape, np.float32)
+    with pytest.raises(ValueError, match=".".join(path)):
+        call(good)
