@@ -233,7 +233,9 @@ __device__ __forceinline__ float row_sum(float v, float* scratch) {
   __syncthreads();
   return (scratch[0] + scratch[1]) + scratch[2];
 }
-__global__ void __launch_bounds__(ROW_THREADS) row_norm_kernel(const RowArgs a) {
+// `aligned`: base and sum_out, the caller's tensors, start on a 16-byte boundary (rows are 32 bytes
+// apart or a multiple of that; the partials lie in the workspace).
+__global__ void __launch_bounds__(ROW_THREADS) row_norm_kernel(const RowArgs a, const bool aligned) {
   static_assert(ROW_THREADS == 96, "three warps");
   __shared__ float scratch[2][3];
   pdl_wait();
@@ -249,7 +251,10 @@ __global__ void __launch_bounds__(ROW_THREADS) row_norm_kernel(const RowArgs a) 
     for (int p = 0; p < SINGLE_MAX_SPLITS; ++p)
       part[p] = a.partial && p < a.splits ? *reinterpret_cast<const float4*>(a.partial + p * plane + off)
                                           : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.base) base = *reinterpret_cast<const float4*>(a.base + off);
+    if (a.base) {
+      const float* src = a.base + off;
+      base = aligned ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+    }
 #pragma unroll
     for (int p = 0; p < SINGLE_MAX_SPLITS; ++p) {
       v[0] += part[p].x;
@@ -262,7 +267,14 @@ __global__ void __launch_bounds__(ROW_THREADS) row_norm_kernel(const RowArgs a) 
     v[2] = base.z + v[2];
     v[3] = base.w + v[3];
   }
-  if (a.sum_out && live) *reinterpret_cast<float4*>(a.sum_out + off) = make_float4(v[0], v[1], v[2], v[3]);
+  if (a.sum_out && live) {
+    if (aligned) {
+      *reinterpret_cast<float4*>(a.sum_out + off) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a.sum_out[off + e] = v[e];
+    }
+  }
   if (!a.pieces) return;
   if (a.scale) {
     const float mean = row_sum((v[0] + v[1]) + (v[2] + v[3]), scratch[0]) / a.c;
@@ -462,7 +474,8 @@ struct SwigluPolicy : NoPrefetch {
 }  // namespace
 
 int launch_row_norm(const RowArgs& a, cudaStream_t stream, bool pdl) {
-  return launch(row_norm_kernel, dim3(a.rows), dim3(ROW_THREADS), 0, stream, pdl, a);
+  const bool aligned = ((reinterpret_cast<uintptr_t>(a.base) | reinterpret_cast<uintptr_t>(a.sum_out)) & 15) == 0;
+  return launch(row_norm_kernel, dim3(a.rows), dim3(ROW_THREADS), 0, stream, pdl, a, aligned);
 }
 
 // Enough splits that the tiles cover the SMs, at least two k steps each, none of them empty.

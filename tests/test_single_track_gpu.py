@@ -60,3 +60,31 @@ def test_single_track_against_float64(cuda_device, n, heads, hidden, shift):
     ref = s + orc.attention_pair_bias(params["attention"], sn, z_got, mask, k_in=sn, dtype="float64")
     ref = ref + orc.transition(params["transition_s"], ref, dtype="float64")
     np.testing.assert_allclose(s_got, ref, rtol=2e-4, atol=2e-4)
+
+
+@pytest.mark.parametrize("n,heads", [(1, 1), (40, 3), (129, 16)])
+def test_single_representation_off_the_16_byte_grid(cuda_device, monkeypatch, n, heads):
+    """Views that start one float past a 16-byte boundary, as input and as result: the same bits."""
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.attention import attention_pair_bias_forward
+    from foldjax_b200.pairformer import pairformer_forward
+
+    rng = np.random.default_rng(n)
+    pd = dev.params_to_device(_params(rng, heads, 64))
+    z = dev.to_device(rng.standard_normal((1, n, n, 128)).astype(np.float32), torch.bfloat16)
+    s, k_in = (torch.from_numpy(rng.standard_normal((1, n, 24 * heads)).astype(np.float32)).cuda() for _ in range(2))
+    mask = torch.ones(1, n, device="cuda")
+
+    def run(move):
+        return [attention_pair_bias_forward(pd["attention"], move(s), z, mask, k_in=move(k_in)),
+                *pairformer_forward([pd, pd], move(s), z, mask, None)]
+
+    want = run(lambda t: t)
+    _lib.device_status()
+    new = torch.empty_like
+    monkeypatch.setattr(torch, "empty_like", lambda t: _misaligned(new(t)) if t.dtype == torch.float32 else new(t))
+    got = run(_misaligned)
+    _lib.device_status()
+    assert got[0].data_ptr() % 16 and got[1].data_ptr() % 16
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
