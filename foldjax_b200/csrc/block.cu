@@ -150,6 +150,8 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   B200_REQUIRE(a != nullptr && a->params != nullptr, B200TRI_ERR_INVALID, "pairformer: null args or params");
   B200_REQUIRE(a->n > 0 && a->n_blocks >= 1, B200TRI_ERR_INVALID, "pairformer: n and n_blocks must be positive");
   B200_REQUIRE(a->z_in && a->z_out, B200TRI_ERR_INVALID, "pairformer: z_in/z_out must not be null");
+  B200_REQUIRE(((reinterpret_cast<uintptr_t>(a->z_in) | reinterpret_cast<uintptr_t>(a->z_out)) & 15) == 0, B200TRI_ERR_INVALID,
+               "pairformer: z_in/z_out must be 16-byte aligned");
   const bool single = a->s_in != nullptr;
   B200_REQUIRE(!single || (a->s_out && a->c_s > 0 && a->heads_s > 0), B200TRI_ERR_INVALID,
                "pairformer: the single track needs s_out, c_s and heads_s");

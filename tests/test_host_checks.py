@@ -148,3 +148,22 @@ def test_pairformer_parameters_of_another_shape_are_refused(monkeypatch, stacked
     node[path[-1]] = np.zeros((blocks,) * stacked + shape, np.float32)
     with pytest.raises(ValueError, match=".".join(path)):
         call(good)
+
+
+@pytest.mark.parametrize("gate", [0, 1])
+def test_pairformer_refuses_a_pair_tensor_off_the_16_byte_grid(gate):
+    """Before its first launch: the pair gate reads 16 bytes at a time."""
+    import ctypes as C
+
+    from foldjax_b200 import _lib
+
+    lib = _lib.load()
+    blocks = (_lib.PairformerBlockParams * 1)()
+    blocks[0].transition_z.hidden = 512
+    address = 1 << 20  # (never dereferenced)
+    size = lib.b200tri_pairformer_workspace_bytes(64, 0, 0, 512, 0)
+    for z_in, z_out in ((address + 2, address), (address, address + 8)):
+        args = _lib.PairformerArgs(n=64, n_blocks=1, params=blocks, z_in=z_in, z_out=z_out, pair_mask=address, pair_gate=gate,
+                                   workspace=address, workspace_bytes=size)
+        assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_INVALID
+        assert b"16-byte aligned" in lib.b200tri_last_error()
