@@ -249,9 +249,19 @@ int make_tmap(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, int
   CUtensorMapSwizzle s = CU_TENSOR_MAP_SWIZZLE_NONE;
   if (swz == Swz::B64) s = CU_TENSOR_MAP_SWIZZLE_64B;
   if (swz == Swz::B128) s = CU_TENSOR_MAP_SWIZZLE_128B;
-  CUresult r = fn(out, dtype, static_cast<cuuint32_t>(rank), const_cast<void*>(base), dims, strides_bytes, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, s, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(out, dtype, static_cast<cuuint32_t>(rank), const_cast<void*>(base), dims, strides_bytes, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, s, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    // A host thread that has made no runtime call yet has no context for the driver's entry point;
+    // setting its device gives it the device's primary one.
+    int dev = 0;
+    B200_CUDA_OK(cudaGetDevice(&dev));
+    B200_CUDA_OK(cudaSetDevice(dev));
+    r = encode();
+  }
   B200_REQUIRE(r == CUDA_SUCCESS, B200TRI_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return B200TRI_OK;
 }
