@@ -7,13 +7,26 @@ runs on the data path; all arithmetic happens inside libb200tri.
 
 from __future__ import annotations
 
+import threading
+import weakref
 from typing import Any, Mapping
 
 import numpy as np
 import torch
 
-_workspaces: dict[tuple[int, str], torch.Tensor] = {}
+# Scratch buffers one thread keeps per device: those of the streams it used last.
+STREAMS_KEPT = 4
 
+
+class _Scratch:
+    """One thread's scratch buffers, (device, stream) -> {tag: buffer}, the stream used last at the end."""
+
+    def __init__(self) -> None:
+        self.streams: dict[tuple[int, int], dict[str, torch.Tensor]] = {}
+
+
+_local = threading.local()
+_scratches: "weakref.WeakSet[_Scratch]" = weakref.WeakSet()
 
 _cuda_seen = False
 
@@ -33,15 +46,36 @@ def stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def workspace(nbytes: int, tag: str = "default") -> torch.Tensor:
-    """A cached, grow-only scratch buffer per (device, tag); 1 KiB aligned."""
+def workspace(nbytes: int, tag: str = "default", stream: int | None = None) -> torch.Tensor:
+    """A grow-only scratch buffer, 1 KiB aligned, of the calling thread, the current device, its
+    current stream and ``tag`` (``stream``: what ``stream_ptr()`` gave a caller that has asked).
+
+    Whatever uses a buffer next comes after its previous use in the order of one stream: two streams
+    have buffers of their own, and so have two threads, whose launches on one stream may alternate.
+    That also makes dropping a buffer safe (it grew, its stream has not been used for a while, its
+    thread ended), because the allocator gives its memory to nobody but that stream until then."""
     dev = torch.cuda.current_device()
-    key = (dev, tag)
-    buf = _workspaces.get(key)
+    scratch = getattr(_local, "scratch", None)
+    if scratch is None:
+        scratch = _local.scratch = _Scratch()
+        _scratches.add(scratch)
+    streams = scratch.streams
+    if stream is None:
+        stream = stream_ptr() if torch.cuda.is_initialized() else 0
+    key = (dev, stream)
+    bufs = streams.get(key)
+    if bufs is None:
+        kept = [k for k in streams if k[0] == dev]
+        for old in kept[:max(0, len(kept) - STREAMS_KEPT + 1)]:
+            streams.pop(old, None)
+        bufs = streams[key] = {}
+    elif len(streams) > 1:
+        streams[key] = streams.pop(key, bufs)  # to the end
+    buf = bufs.get(tag)
     if buf is None or buf.numel() < nbytes + 1024:  # callers round the pointer up by up to 1023 B
-        _workspaces.pop(key, None)
+        bufs.pop(tag, None)
         buf = torch.empty(int(nbytes) + 1024, dtype=torch.uint8, device=f"cuda:{dev}")
-        _workspaces[key] = buf
+        bufs[tag] = buf
     return buf
 
 
@@ -91,7 +125,9 @@ def check_device_status() -> None:
 
 
 def release_workspaces() -> None:
-    _workspaces.clear()
+    """Drop the scratch buffers of all threads (a call under way keeps its own until it is enqueued)."""
+    for scratch in list(_scratches):
+        scratch.streams.clear()
 
 
 def ready(x: Any, dtype: torch.dtype | None) -> bool:

@@ -55,6 +55,58 @@ def test_workspace_reuse_accounts_for_the_alignment_slack(monkeypatch):
     dev.release_workspaces()
 
 
+def _host_scratch(monkeypatch):
+    """dev.workspace on host memory; returns the stream handle it sees, to be changed by the test."""
+    real_empty, stream = torch.empty, [1]
+    monkeypatch.setattr(dev.torch, "empty", lambda n, dtype=None, device=None: real_empty(int(n), dtype=torch.uint8))
+    monkeypatch.setattr(dev.torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(dev.torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(dev, "stream_ptr", lambda: stream[0])
+    dev.release_workspaces()
+    return stream
+
+
+def test_streams_do_not_share_scratch(monkeypatch):
+    stream = _host_scratch(monkeypatch)
+    a = dev.workspace(4096, "t")
+    stream[0] = 2
+    b = dev.workspace(4096, "t")
+    assert a is not b and dev.workspace(4096, "t") is b
+    stream[0] = 1
+    assert dev.workspace(4096, "t") is a
+    # a program that goes through many streams keeps the buffers of the last few
+    for stream[0] in range(3, 2 + dev.STREAMS_KEPT):
+        dev.workspace(4096, "t")
+    stream[0] = 1
+    assert dev.workspace(4096, "t") is a
+    stream[0] = 2
+    assert dev.workspace(4096, "t") is not b
+    dev.release_workspaces()
+
+
+def test_threads_do_not_share_scratch(monkeypatch):
+    import gc
+    import threading
+    import weakref
+
+    _host_scratch(monkeypatch)
+    mine = dev.workspace(4096, "t")
+    seen = []
+
+    def other():
+        buf = dev.workspace(4096, "t")
+        assert buf is not mine and dev.workspace(4096, "t") is buf
+        seen.append(weakref.ref(buf))
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    thread.join()
+    gc.collect()
+    assert seen and seen[0]() is None  # given back with the thread
+    assert dev.workspace(4096, "t") is mine
+    dev.release_workspaces()
+
+
 def test_streamed_blocks_refuse_mismatched_host_buffers():
     """stream_host_blocks checks its host buffers before it touches a device."""
     from foldjax_b200.block import stream_host_blocks
