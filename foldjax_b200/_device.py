@@ -46,35 +46,46 @@ def stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def workspace(nbytes: int, tag: str = "default", stream: int | None = None) -> torch.Tensor:
+def place() -> tuple[int, int]:
+    """The current device and its current stream as a raw handle."""
+    device = torch._C._cuda_getDevice()
+    return device, torch._C._cuda_getCurrentRawStream(device)
+
+
+def workspace(nbytes: int, tag: str = "default", at: tuple[int, int] | None = None) -> torch.Tensor:
     """A grow-only scratch buffer, 1 KiB aligned, of the calling thread, the current device, its
-    current stream and ``tag`` (``stream``: what ``stream_ptr()`` gave a caller that has asked).
+    current stream and ``tag`` (``at``: what ``place()`` gave a caller that has asked).
 
     Whatever uses a buffer next comes after its previous use in the order of one stream: two streams
     have buffers of their own, and so have two threads, whose launches on one stream may alternate.
     That also makes dropping a buffer safe (it grew, its stream has not been used for a while, its
-    thread ended), because the allocator gives its memory to nobody but that stream until then."""
-    dev = torch.cuda.current_device()
+    thread ended), because the allocator gives its memory to nobody but that stream until then.
+
+    A call that is being captured gets a buffer of the graph's memory pool and none is kept: the graph
+    holds the address for as long as it lives, whatever becomes of the buffers kept here, and may be
+    replayed beside other calls on its stream."""
+    initialized = at is not None or torch.cuda.is_initialized()
+    if at is None:
+        at = (torch.cuda.current_device(), stream_ptr() if initialized else 0)
+    if initialized and torch.cuda.is_current_stream_capturing():
+        return torch.empty(int(nbytes) + 1024, dtype=torch.uint8, device=f"cuda:{at[0]}")
     scratch = getattr(_local, "scratch", None)
     if scratch is None:
         scratch = _local.scratch = _Scratch()
         _scratches.add(scratch)
     streams = scratch.streams
-    if stream is None:
-        stream = stream_ptr() if torch.cuda.is_initialized() else 0
-    key = (dev, stream)
-    bufs = streams.get(key)
+    bufs = streams.get(at)
     if bufs is None:
-        kept = [k for k in streams if k[0] == dev]
+        kept = [k for k in streams if k[0] == at[0]]
         for old in kept[:max(0, len(kept) - STREAMS_KEPT + 1)]:
             streams.pop(old, None)
-        bufs = streams[key] = {}
+        bufs = streams[at] = {}
     elif len(streams) > 1:
-        streams[key] = streams.pop(key, bufs)  # to the end
+        streams[at] = streams.pop(at, bufs)  # to the end
     buf = bufs.get(tag)
     if buf is None or buf.numel() < nbytes + 1024:  # callers round the pointer up by up to 1023 B
         bufs.pop(tag, None)
-        buf = torch.empty(int(nbytes) + 1024, dtype=torch.uint8, device=f"cuda:{dev}")
+        buf = torch.empty(int(nbytes) + 1024, dtype=torch.uint8, device=f"cuda:{at[0]}")
         bufs[tag] = buf
     return buf
 

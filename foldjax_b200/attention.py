@@ -70,8 +70,8 @@ def attention_pair_bias_forward(
         raise ValueError(f"libb200tri is built for heads of width {HEAD_DIM} and c_z = {C_Z}; got c_s {c_s}, {heads} heads")
     out = torch.empty_like(sd)
     nbytes = _lib.workspace_bytes("b200tri_attention_pair_bias_workspace_bytes", n, c_s, heads)
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "attention_pair_bias", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "attention_pair_bias", at)
     for bi in range(b):
         args = _lib.AttentionPairBiasArgs(
             n=n, c_s=c_s, c_z=C_Z, heads=heads, eps=float(eps), inf=float(inf),
@@ -79,7 +79,7 @@ def attention_pair_bias_forward(
             out=out[bi].data_ptr(), workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes,
             **{k: v.data_ptr() for k, v in lv.items()},
         )
-        _lib.check(lib.b200tri_attention_pair_bias(C.byref(args), stream))
+        _lib.check(lib.b200tri_attention_pair_bias(C.byref(args), at[1]))
     if host_in:
         host = out.cpu()
         return host.numpy() if numpy_in else host

@@ -195,8 +195,8 @@ def pairformer_forward(
         p.check(c_s, heads_s, bool(stacked), blocks if stacked else 1)
     nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s,
                                   max(p.hidden_z for p in packed), max(p.hidden_s for p in packed))
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "pairformer", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "pairformer", at)
     z_out = torch.empty_like(zd)
     s_out = torch.empty_like(sd) if single else None
     for bi in range(b):
@@ -207,7 +207,7 @@ def pairformer_forward(
             pair_mask=pmd[bi].data_ptr() if pmd is not None else None, mask=md[bi].data_ptr() if md is not None else None,
             workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes,
             pair_gate=int(gate), mask_transition=int(mask_trans), attention_first=int(bool(attention_first)))
-        _lib.check(lib.b200tri_pairformer_forward(C.byref(args), stream))
+        _lib.check(lib.b200tri_pairformer_forward(C.byref(args), at[1]))
     if squeeze:
         z_out = z_out[0]
         s_out = s_out[0] if single and np.ndim(s) == 2 else s_out

@@ -90,13 +90,13 @@ def transition_forward(
         if md.numel() != rows:
             raise ValueError(f"mask shape {tuple(md.shape)} does not give one value per row of x {tuple(xd.shape)}")
     nbytes = _lib.workspace_bytes("b200tri_pair_transition_workspace_bytes", hidden)
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "pair_transition", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "pair_transition", at)
     # (the leaves are in the order of the struct's fields)
     args = _lib.pack_pair_transition(rows, C_Z, hidden, float(eps), xd.data_ptr(),
                                      *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(),
                                      dev.aligned_ptr(ws), nbytes, _ptr(md))
-    _lib.check(lib.b200tri_pair_transition(C.byref(args), stream))
+    _lib.check(lib.b200tri_pair_transition(C.byref(args), at[1]))
     if host_in:
         host = out.float().cpu() if numpy_in else out.cpu()
         dev.check_device_status()

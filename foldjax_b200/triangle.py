@@ -152,13 +152,13 @@ def triangle_multiplication_forward(
     nbytes = _lib.workspace_bytes("b200tri_trimul_workspace_bytes_shape", n, code, c_z, c_hidden)
     if b > 1 and (code, c_z, c_hidden) != (_lib.DTYPE_BF16, C_Z, C_Z):
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "trimul", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "trimul", at)
     # (the leaves are in the order of the struct's fields)
     args = _lib.pack_trimul(n, int(direction == "incoming"), float(eps), xd.data_ptr(), _ptr(md),
                             *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, c_hidden, b)
-    _lib.check(lib.b200tri_trimul_forward(C.byref(args), stream))
+    _lib.check(lib.b200tri_trimul_forward(C.byref(args), at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

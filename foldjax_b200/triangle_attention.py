@@ -94,13 +94,13 @@ def triangle_attention_forward(
     nbytes = _lib.workspace_bytes("b200tri_triatt_workspace_bytes_shape", n, code, c_z, heads, head_dim)
     if b > 1 and (code, c_z, heads, head_dim) != (_lib.DTYPE_BF16, C_Z, HEADS, HEAD_DIM):
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "triatt", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "triatt", at)
     # (the leaves are in the order of the struct's fields)
     args = _lib.pack_triatt(n, int(bool(starting)), heads, head_dim, C.c_float(inf).value, float(eps), xd.data_ptr(), _ptr(md),
                             *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, b)
-    _lib.check(lib.b200tri_triatt_forward(C.byref(args), stream))
+    _lib.check(lib.b200tri_triatt_forward(C.byref(args), at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()
@@ -152,12 +152,12 @@ def attention_core(q, k, v, tri_bias, mask_bias, scale: float | None = None):
     md = _operand(mask_bias, torch.float32)
     out = torch.empty(q.shape, dtype=torch.bfloat16, device=q.device)
     nbytes = _lib.workspace_bytes("b200tri_attention_core_workspace_bytes", n_i, n_j, n_k)
-    stream = dev.stream_ptr()
-    ws = dev.workspace(nbytes, "attention_core", stream)
+    at = dev.place()
+    ws = dev.workspace(nbytes, "attention_core", at)
     args = _lib.pack_attention_core(bsz, n_i, n_j, n_k, h, d, int(vd.dtype is torch.float32), int(bd.dtype is torch.float32),
                                     qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), bd.data_ptr(), md.data_ptr(),
                                     out.data_ptr(), dev.aligned_ptr(ws), nbytes)
-    _lib.check(lib.b200tri_attention_core(C.byref(args), stream))
+    _lib.check(lib.b200tri_attention_core(C.byref(args), at[1]))
     return out if v.dtype is torch.bfloat16 else out.to(v.dtype)
 
 

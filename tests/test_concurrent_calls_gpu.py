@@ -1,5 +1,6 @@
-"""The same operator on two streams, and from two threads, at once: every call gets the bits it gets
-alone. Sizes differ, so that shared scratch would show in either direction."""
+"""The same operator on two streams, and from two threads, at once, and captured
+in graphs: every call gets the bits it gets alone. Sizes differ, so that shared scratch would show in
+either direction."""
 
 from __future__ import annotations
 
@@ -92,3 +93,38 @@ def test_concurrent_calls_equal_calls_one_by_one(cuda_device, name, threads):
         assert len(results) == repeats
         for r in results:
             assert torch.equal(r, w)
+
+
+@pytest.mark.parametrize("name", ["mul", "attn", "attn f32", "transition", "core", "trunk"])
+def test_captured_calls(cuda_device, name):
+    """Two graphs captured on one stream, replayed on two, while eager calls of a larger size run and
+    the kept scratch is dropped."""
+    from foldjax_b200 import _device as dev, _lib
+
+    call = _calls(cuda_device)[name]
+    inputs = _inputs(cuda_device, (200, 136, 264))
+    want = [call(z, m) for z, m in inputs]
+    torch.cuda.synchronize()
+    capture, graphs = torch.cuda.Stream(), []
+    with torch.cuda.stream(capture):
+        call(*inputs[1])
+    torch.cuda.synchronize()
+    for z, m in inputs[:2]:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=capture):
+            out = call(z, m)
+        graphs.append((graph, out))
+    dev.release_workspaces()
+    streams = [torch.cuda.Stream() for _ in graphs]
+    eager = []
+    for _ in range(4):
+        for (graph, _), stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        eager.append(call(*inputs[2]))
+    torch.cuda.synchronize()
+    _lib.device_status()
+    for (_, out), w in zip(graphs, want):
+        assert torch.equal(out, w)
+    for e in eager:
+        assert torch.equal(e, want[2])

@@ -61,6 +61,7 @@ def _host_scratch(monkeypatch):
     monkeypatch.setattr(dev.torch, "empty", lambda n, dtype=None, device=None: real_empty(int(n), dtype=torch.uint8))
     monkeypatch.setattr(dev.torch.cuda, "current_device", lambda: 0)
     monkeypatch.setattr(dev.torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(dev.torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(dev, "stream_ptr", lambda: stream[0])
     dev.release_workspaces()
     return stream
@@ -81,6 +82,19 @@ def test_streams_do_not_share_scratch(monkeypatch):
     assert dev.workspace(4096, "t") is a
     stream[0] = 2
     assert dev.workspace(4096, "t") is not b
+    dev.release_workspaces()
+
+
+def test_captured_calls_keep_no_scratch(monkeypatch):
+    """A graph holds its buffers' addresses: nothing a later call can drop or write beside a replay."""
+    _host_scratch(monkeypatch)
+    kept = dev.workspace(4096, "t")
+    monkeypatch.setattr(dev.torch.cuda, "is_current_stream_capturing", lambda: True)
+    a = dev.workspace(4096, "t", (0, 1))
+    b = dev.workspace(4096, "t", (0, 1))
+    assert a is not kept and b is not kept and a is not b
+    monkeypatch.setattr(dev.torch.cuda, "is_current_stream_capturing", lambda: False)
+    assert dev.workspace(4096, "t") is kept
     dev.release_workspaces()
 
 
