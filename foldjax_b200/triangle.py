@@ -158,7 +158,8 @@ def triangle_multiplication_forward(
     args = _lib.pack_trimul(n, int(direction == "incoming"), float(eps), xd.data_ptr(), _ptr(md),
                             *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, c_hidden, b)
-    _lib.check(lib.b200tri_trimul_forward(C.byref(args), at[1]))
+    if b:  # (an empty batch has an empty result)
+        _lib.check(lib.b200tri_trimul_forward(C.byref(args), at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

@@ -100,7 +100,8 @@ def triangle_attention_forward(
     args = _lib.pack_triatt(n, int(bool(starting)), heads, head_dim, C.c_float(inf).value, float(eps), xd.data_ptr(), _ptr(md),
                             *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, b)
-    _lib.check(lib.b200tri_triatt_forward(C.byref(args), at[1]))
+    if b:  # (an empty batch has an empty result)
+        _lib.check(lib.b200tri_triatt_forward(C.byref(args), at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()
@@ -157,7 +158,8 @@ def attention_core(q, k, v, tri_bias, mask_bias, scale: float | None = None):
     args = _lib.pack_attention_core(bsz, n_i, n_j, n_k, h, d, int(vd.dtype is torch.float32), int(bd.dtype is torch.float32),
                                     qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), bd.data_ptr(), md.data_ptr(),
                                     out.data_ptr(), dev.aligned_ptr(ws), nbytes)
-    _lib.check(lib.b200tri_attention_core(C.byref(args), at[1]))
+    if bsz:  # (an empty batch has an empty result)
+        _lib.check(lib.b200tri_attention_core(C.byref(args), at[1]))
     return out if v.dtype is torch.bfloat16 else out.to(v.dtype)
 
 

@@ -105,3 +105,21 @@ def test_leading_batch_axes_are_folded(cuda_device):
     att = triangle_attention_forward(pa, x, mask, starting=False)
     assert att.shape == x.shape
     assert torch.equal(att[0, 1], triangle_attention_forward(pa, x[0, 1], mask[0, 1], starting=False))
+
+
+@pytest.mark.parametrize("c_z,dtype", [(128, "bfloat16"), (64, "bfloat16"), (128, "float32")])
+def test_empty_batch(cuda_device, c_z, dtype):
+    """No items in, no items out, as for every other operator of a model that slices its batch."""
+    from foldjax_b200.triangle import triangle_multiplication_forward
+    from foldjax_b200.triangle_attention import attention_core, triangle_attention_forward
+
+    rng = np.random.default_rng(0)
+    mul = orc.random_trimul_params(rng, c_z=c_z)
+    att = orc.random_triatt_params(rng, c_z=c_z)
+    z = torch.empty(0, 12, 12, c_z, device=cuda_device, dtype=getattr(torch, dtype))
+    mask = torch.empty(0, 12, 12, device=cuda_device)
+    assert triangle_multiplication_forward(mul, z, mask, "outgoing", residual=z).shape == z.shape
+    assert triangle_attention_forward(att, z, mask, residual=z).shape == z.shape
+    q = torch.empty(0, 5, 4, 7, 32, device=cuda_device, dtype=z.dtype)
+    got = attention_core(q, q, q, q.new_empty(0, 1, 4, 7, 7), torch.empty(0, 5, 1, 1, 7, device=cuda_device))
+    assert got.shape == q.shape and got.dtype == q.dtype
