@@ -894,13 +894,21 @@ TriattPlan triatt_plan(int n, int batch, int c_z, int heads, int head_dim, bool 
   return pl;
 }
 
-// Batch items one pass can take with the workspace the caller gave.
+// Batch items one pass can take with the workspace the caller gave: pair indices are 32-bit inside
+// the kernels, and a grid's third dimension, which the layer norms count the items in, ends at 65535.
 template <class F>
 int items_per_pass(int batch, int n, size_t bytes, F total_of) {
-  int g = batch;
-  // (pair indices are 32-bit inside the kernels)
-  while (g > 1 && (total_of(g) > bytes || static_cast<long long>(g) * n * n > 4000000000ll)) --g;
-  return g;
+  const long long by_pairs = 4000000000ll / (static_cast<long long>(n) * n);
+  int low = 1, high = batch < 65535 ? batch : 65535;
+  high = by_pairs < high ? static_cast<int>(by_pairs) : high;
+  while (low < high) {  // the scratch grows with the items
+    const int mid = high - (high - low) / 2;
+    if (total_of(mid) <= bytes)
+      low = mid;
+    else
+      high = mid - 1;
+  }
+  return low;
 }
 
 // Weights of one op: read in place where TMA can, else listed for one weight_kernel launch.

@@ -123,3 +123,20 @@ def test_empty_batch(cuda_device, c_z, dtype):
     q = torch.empty(0, 5, 4, 7, 32, device=cuda_device, dtype=z.dtype)
     got = attention_core(q, q, q, q.new_empty(0, 1, 4, 7, 7), torch.empty(0, 5, 1, 1, 7, device=cuda_device))
     assert got.shape == q.shape and got.dtype == q.dtype
+
+
+def test_more_items_than_a_grid_dimension(cuda_device):
+    """65 600 pair tensors of one token: more than one launch can count in its grid's third dimension."""
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.triangle import triangle_multiplication_forward
+    from foldjax_b200.triangle_attention import triangle_attention_forward
+
+    rng = np.random.default_rng(0)
+    mul = dev.params_to_device(orc.random_trimul_params(rng, c_z=8, c_hidden=8, std=0.3))
+    att = dev.params_to_device(orc.random_triatt_params(rng, c_z=8, heads=1, c_hidden=8, std=0.3))
+    z = torch.randn(65600, 1, 1, 8, generator=torch.Generator(cuda_device).manual_seed(1), device=cuda_device).bfloat16()
+    for call in (lambda x: triangle_multiplication_forward(mul, x, None, "outgoing"),
+                 lambda x: triangle_attention_forward(att, x)):
+        got = call(z)
+        _lib.device_status()
+        assert torch.equal(got, torch.cat([call(part) for part in z.split(20000)]))
