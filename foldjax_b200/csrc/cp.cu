@@ -984,7 +984,7 @@ extern "C" int b200tri_trimul_cp(b200tri_comm* cm, const b200tri_trimul_cp_args*
     b200::SmReserve room(last ? 0 : cm->sm_reserve);
     log_launch(cm, B200TRI_CP_EVENT_CONTRACT, g, ca.n_i, ca.n_j, static_cast<const uint8_t*>(ca.a) - ws,
                static_cast<const uint8_t*>(ca.b) - ws, static_cast<uint8_t*>(ca.out_bf16) - ws, ca.a_src_stride * 2);
-    if (!cm->dry && (rc = b200tri_trimul_contract(&ca, stream_))) return rc;
+    if (!cm->dry && (rc = contract_launch(&ca, 128, ContractTerms{}, true, stream))) return rc;
 
     // output stage of the same rows (or columns): it is local to a pair
     const int64_t row0 = by_cols ? 0 : static_cast<int64_t>(s) * n_c + static_cast<int64_t>(q) * h;

@@ -1004,7 +1004,7 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       else
         ca.out_f32 = reinterpret_cast<float*>(ws + pl.t);
       const ContractTerms terms = BF ? ContractTerms{} : ContractTerms{6, {2, 0, 1, 1, 0, 0}, {0, 2, 1, 0, 1, 0}};
-      if ((rc = contract_launch(&ca, nb * c_h, terms, stream))) return rc;
+      if ((rc = contract_launch(&ca, nb * c_h, terms, true, stream))) return rc;
     }
     if ((rc = launch_ln_channel_major<BF>(ws + pl.t, n, nb, ld, c_h, a->norm_out_scale, a->norm_out_bias, a->eps, at(pl.tn),
                                           stream)))

@@ -144,11 +144,14 @@ int make_weight_map(CUtensorMap* out, const void* w, int k, int n, int box_k);
 // of operand-plane pairs accumulated one after the other in the same float32 accumulator: the
 // piece products of split operands, smallest first, so that only the leading one is summed at
 // full magnitude.
+// TMA clips the rows of a bf16 result at a multiple of 16 bytes. `pad_is_scratch`: the columns from
+// n_j up to a multiple of 8 may be written, so the result may leave by TMA whatever n_j is.
 struct ContractTerms {
   int n;
   uint8_t a[8], b[8];
 };
-int contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms, cudaStream_t stream);
+int contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms, bool pad_is_scratch,
+                    cudaStream_t stream);
 
 // The mask-bias rows of the attention core, written by the projection stage of the same call.
 struct MaskBiasOut {

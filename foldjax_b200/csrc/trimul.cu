@@ -157,7 +157,7 @@ extern "C" int b200tri_trimul_forward(const b200tri_trimul_args* a, b200tri_stre
   ca.out_chan_stride = pl.chan_stride;
   ca.a_rows_per_block = ca.b_rows_per_block = ca.out_rows_per_block = RPB;
   ca.a_block_stride = ca.b_block_stride = ca.out_block_stride = pl.block_stride;
-  rc = b200tri_trimul_contract(&ca, stream);
+  rc = contract_launch(&ca, 128, ContractTerms{}, true, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
 
   b200tri_trimul_finish_args fa = {};

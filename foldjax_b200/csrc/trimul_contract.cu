@@ -47,7 +47,7 @@ struct ContractParams {
   int kb_per_src;  // ceil(n_k / BK)
   int tiles_m, tiles_n;
   uint32_t total_tiles;
-  bool staged;  // the bf16 result is all that is wanted and a warp's 32 rows share a block
+  bool staged;  // the result leaves by TMA: it is bf16 only and a warp's 32 rows share a block
   bool out_blocked;
   const float* acc_in;
   float* out_f32;
@@ -222,7 +222,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           fence_proxy_async();
           __syncwarp();
           if (row0 + 32 <= p.n_i || !p.out_blocked) {
-            if (lane == 0) {  // what lies past n_i and n_j is outside the tensor and is not written
+            if (lane == 0) {  // rows past n_i, and columns past n_j up to a multiple of 8, are not written
               tma_store_4d(&tm_out, staging, col0, in_block, d, block);
               tma_store_commit();
             }
@@ -334,10 +334,10 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 }  // namespace b200
 
 extern "C" int b200tri_trimul_contract(const b200tri_trimul_contract_args* a, b200tri_stream_t stream) {
-  return b200::contract_launch(a, 128, b200::ContractTerms{}, reinterpret_cast<cudaStream_t>(stream));
+  return b200::contract_launch(a, 128, b200::ContractTerms{}, false, reinterpret_cast<cudaStream_t>(stream));
 }
 
-int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms,
+int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, const ContractTerms& terms, bool pad_is_scratch,
                           cudaStream_t stream) {
   B200_REQUIRE(a != nullptr, B200TRI_ERR_INVALID, "contract: null args");
   B200_REQUIRE(a->a && a->b, B200TRI_ERR_INVALID, "contract: null operand");
@@ -408,7 +408,8 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   }
   const int out_rows = a->out_rows_per_block > 0 && a->out_rows_per_block < a->n_i ? a->out_rows_per_block : a->n_i;
   const int out_blocks = (a->n_i + out_rows - 1) / out_rows;
-  const bool staged = a->out_bf16 && !a->out_f32 && !a->acc_in && (out_blocks == 1 || out_rows % 32 == 0);
+  const bool staged = a->out_bf16 && !a->out_f32 && !a->acc_in && (out_blocks == 1 || out_rows % 32 == 0) &&
+                      (pad_is_scratch || a->n_j % 8 == 0);
   CUtensorMap tm_out = tm_a;  // (unused without staging)
   if (staged) {
     const uint64_t dims[4] = {(uint64_t)a->n_j, (uint64_t)out_rows, (uint64_t)channels, (uint64_t)out_blocks};
