@@ -876,7 +876,7 @@ extern "C" int b200tri_trimul_cp(b200tri_comm* cm, const b200tri_trimul_cp_args*
   pa.workspace_bytes = b200tri_trimul_project_workspace_bytes();
   log_launch(cm, B200TRI_CP_EVENT_PROJECT, -1, pa.n_outer, pa.n_inner, static_cast<uint8_t*>(pa.a) - ws,
              static_cast<uint8_t*>(pa.b) - ws, 0, 0);
-  if (!cm->dry && (rc = b200tri_trimul_project(&pa, stream_))) return rc;
+  if (!cm->dry && (rc = mul_project_launch(&pa, true, stream))) return rc;
 
   // Exchange and contraction, in row chunks: the output rows of the tile are cut into G chunks
   // (k_split per n_c-row block); group g of the exchange carries chunk g of every `a` message

@@ -140,12 +140,17 @@ int aligned_weight(const void* w, size_t bytes, void* scratch, cudaStream_t stre
 // columns x `box_k` rows: MN-major operand tiles under the 128-byte swizzle.
 int make_weight_map(CUtensorMap* out, const void* w, int k, int n, int box_k);
 
+// TMA clips the rows of a bf16 output at a multiple of 16 bytes. `pad_is_scratch`: what lies between a
+// row's end and the next multiple of 8 elements may be written, so an output may leave by TMA whatever
+// its width.
+
+// The projection stage of the multiplicative update.
+int mul_project_launch(const b200tri_trimul_project_args* a, bool pad_is_scratch, cudaStream_t stream);
+
 // A contraction over `channels` channel planes. `terms` (if any) replaces the sources by a list
 // of operand-plane pairs accumulated one after the other in the same float32 accumulator: the
 // piece products of split operands, smallest first, so that only the leading one is summed at
 // full magnitude.
-// TMA clips the rows of a bf16 result at a multiple of 16 bytes. `pad_is_scratch`: the columns from
-// n_j up to a multiple of 8 may be written, so the result may leave by TMA whatever n_j is.
 struct ContractTerms {
   int n;
   uint8_t a[8], b[8];

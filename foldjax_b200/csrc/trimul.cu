@@ -139,7 +139,7 @@ extern "C" int b200tri_trimul_forward(const b200tri_trimul_args* a, b200tri_stre
   pa.rows_per_block = RPB;
   pa.workspace = ws + pl.off_proj;
   pa.workspace_bytes = b200tri_trimul_project_workspace_bytes();
-  int rc = b200tri_trimul_project(&pa, stream);
+  int rc = mul_project_launch(&pa, true, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
   PdlChain chain;
 

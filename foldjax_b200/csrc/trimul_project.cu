@@ -58,10 +58,15 @@ struct ProjParams {
   const void* beta;
   bool early_weights;  // the weights may be read before pdl_wait()
   int rows_per_block;
+  __nv_bfloat16 *a, *b;  // the outputs and their strides, where rows do not end on 16 bytes
+  long long ld, chan_stride, block_stride;
   float eps;
   int* status;
 };
 
+// RAGGED: rows end inside 16 bytes and what lies behind them is not ours. TMA would write it, so the
+// maps end at the last whole 16 bytes and the threads store the rest.
+template <bool RAGGED>
 __global__ void __launch_bounds__(THREADS, 1)
 project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_p,
                const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_a,
@@ -245,10 +250,19 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         tc_fence_before();
         fence_proxy_async();
         named_barrier(1 + part, 128);
-        if (leader && t0 < p.n_inner) {  // pairs past n_inner are outside the tensor and are not written
+        const int whole = RAGGED ? p.n_inner & ~7 : p.n_inner;
+        if (leader && t0 < whole) {  // pairs past the tensor's end are not written
           const int block = o / p.rows_per_block;
           tma_store_4d(half ? &tm_b : &tm_a, out, t0, o - block * p.rows_per_block, 0, block);
           tma_store_commit();
+        }
+        if (RAGGED && t0 <= whole && whole < t0 + 32) {  // (this thread's own row of the staged tile)
+          const int block = o / p.rows_per_block;
+          __nv_bfloat16* dst = (half ? p.b : p.a) + block * p.block_stride + chan * p.chan_stride +
+                               (o - block * p.rows_per_block) * p.ld + whole;
+          const __nv_bfloat16* src =
+              reinterpret_cast<const __nv_bfloat16*>(out + chan * 64 + ((((whole - t0) >> 3) ^ ((chan >> 1) & 3)) << 4));
+          for (int e = 0; e < p.n_inner - whole; ++e) dst[e] = src[e];
         }
         if (lane == 0) mbar_arrive(&sm.acc_empty[half]);
       }
@@ -271,9 +285,11 @@ extern "C" size_t b200tri_trimul_project_workspace_bytes(void) {
   return 512 * 128 * 2 + 1024;  // copies of weights that are not 16-byte aligned
 }
 
-extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200tri_stream_t stream_) {
-  using namespace b200;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200tri_stream_t stream) {
+  return b200::mul_project_launch(a, false, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int b200::mul_project_launch(const b200tri_trimul_project_args* a, bool pad_is_scratch, cudaStream_t stream) {
   B200_REQUIRE(a != nullptr, B200TRI_ERR_INVALID, "project: null args");
   B200_REQUIRE(a->x && a->a && a->b && a->p_in && a->g_in && a->norm_in_scale && a->norm_in_bias, B200TRI_ERR_INVALID,
                "project: null pointer argument");
@@ -312,10 +328,12 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
     if (rc || (rc = make_weight_map(&tm_g, w_g, 128, 256, 128))) return rc;
   }
   CUtensorMap tm_out[2];  // (pair, row in block, channel, block), written as tiles of [128 channels][32 pairs]
+  const bool ragged = !pad_is_scratch && a->n_inner % 8 != 0;
+  const int whole = a->n_inner < 8 ? 8 : a->n_inner & ~7;
   const int rpb = a->rows_per_block < a->n_outer ? a->rows_per_block : a->n_outer;
   for (int i = 0; i < 2; ++i) {
     const int blocks = (a->n_outer + rpb - 1) / rpb;
-    const uint64_t dims[4] = {(uint64_t)a->n_inner, (uint64_t)rpb, 128, (uint64_t)blocks};
+    const uint64_t dims[4] = {(uint64_t)(ragged ? whole : a->n_inner), (uint64_t)rpb, 128, (uint64_t)blocks};
     const uint64_t str[3] = {(uint64_t)a->ld * 2, (uint64_t)a->chan_stride * 2,
                              (uint64_t)(blocks > 1 ? a->block_stride : a->chan_stride * 128) * 2};
     const uint32_t box[4] = {32, 1, 128, 1};
@@ -336,17 +354,21 @@ extern "C" int b200tri_trimul_project(const b200tri_trimul_project_args* a, b200
   p.beta = a->norm_in_bias;
   p.early_weights = chained && w_p == a->p_in && w_g == a->g_in;
   p.rows_per_block = rpb;
+  p.a = static_cast<__nv_bfloat16*>(a->a);
+  p.b = static_cast<__nv_bfloat16*>(a->b);
+  p.ld = a->ld;
+  p.chan_stride = a->chan_stride;
+  p.block_stride = a->block_stride;
   p.eps = a->eps;
   p.status = status;
 
-  {
-    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(project_kernel), (int)sizeof(Smem));
-    if (rc) return rc;
-  }
   const long long grid = tiles < sm_count() ? tiles : sm_count();
-  {
+  auto go = [&](auto kernel) {
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem));
+    if (rc) return rc;
     TimedLaunch timed(K_TRIMUL_PROJECT, stream);
-    return launch(project_kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_p,
-                  tm_g, tm_out[0], tm_out[1], p);
-  }
+    return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_p, tm_g,
+                  tm_out[0], tm_out[1], p);
+  };
+  return ragged ? go(project_kernel<true>) : go(project_kernel<false>);
 }

@@ -212,3 +212,35 @@ def test_large_case_properties(cuda_device):
     ref = pr.r(o * g)
     got = out[0, rows].float().cpu().numpy()
     print(assert_parity(ref, got, label="trimul n=1024 sampled rows"))
+
+
+@pytest.mark.parametrize("n", [5, 77, 161, 203])
+def test_project_leaves_the_pitch_padding(cuda_device, n):
+    """Rows that end inside 16 bytes: the bits of the same pairs in longer rows, and nothing behind them."""
+    from foldjax_b200 import _lib, _device as dev
+
+    lib = _lib.load()
+    n_outer, n8, ld, untouched = 70, (n + 7) // 8 * 8, (n + 63) // 64 * 64, 12352.0
+    params = dev.params_to_device(orc.random_trimul_params(np.random.default_rng(n), std=0.1, ln_noise=0.1))
+    x = torch.randn(n_outer, n8, 128, device=cuda_device).bfloat16()
+    mask = (torch.rand(n_outer, n8, device=cuda_device) > 0.2).float()
+    nbytes = lib.b200tri_trimul_project_workspace_bytes()
+    ws = torch.empty(nbytes + 1024, dtype=torch.uint8, device=cuda_device)
+    chan, block = 64 * ld, 128 * 64 * ld
+    outs = {}
+    for n_inner in (n, n8):
+        a, b = outs[n_inner] = [torch.full((2, 128, 64, ld), untouched, dtype=torch.bfloat16, device=cuda_device) for _ in range(2)]
+        args = _lib.TrimulProjectArgs(
+            n_outer=n_outer, n_inner=n_inner, eps=1e-5, x=x.data_ptr(), xs_outer=n8 * 128, xs_inner=128,
+            mask=mask.data_ptr(), ms_outer=n8, ms_inner=1,
+            norm_in_scale=params["norm_in"]["scale"].data_ptr(), norm_in_bias=params["norm_in"]["bias"].data_ptr(),
+            p_in=params["p_in"]["kernel"].data_ptr(), g_in=params["g_in"]["kernel"].data_ptr(),
+            a=a.data_ptr(), b=b.data_ptr(), ld=ld, chan_stride=chan, block_stride=block, rows_per_block=64,
+            workspace=dev.aligned_ptr(ws), workspace_bytes=nbytes)
+        _lib.check(lib.b200tri_trimul_project(C.byref(args), C.c_void_p(dev.stream_ptr())))
+        _lib.device_status()
+    for got, want in zip(outs[n], outs[n8]):
+        got, want = (t.transpose(0, 1).reshape(128, 128, ld) for t in (got, want))
+        assert torch.equal(got[:, :n_outer, :n], want[:, :n_outer, :n])
+        assert bool((want[:, :n_outer, :n8] != untouched).all())
+        assert bool((got[:, :n_outer, n:] == untouched).all()) and bool((got[:, n_outer:] == untouched).all())
