@@ -1,6 +1,6 @@
 """Parity at the benchmark's own sizes: N = 3072 with the last 60 tokens padded (the
 per-block work of the 48-block trunk) and N = 1024 with the last 21 padded (the
-one-block config), through the public operators.
+one-block config), and a ragged N = 1003, through the public operators.
 
 The CPU restatement cannot produce a whole N = 3072 output in reasonable time, but an
 output element (i, j) of either op depends on two rows of the input only (rows i and
@@ -54,7 +54,7 @@ def _gather(x, mask, rows, cols, transposed):
     return f(xi), f(mi), f(xj), f(mj), f(xij)
 
 
-@pytest.mark.parametrize("n,n_pad", [(3072, 60), (1024, 21)])
+@pytest.mark.parametrize("n,n_pad", [(3072, 60), (1024, 21), (1003, 0)])  # (1003: ragged tiles of 256 rows in 64-row blocks)
 @pytest.mark.parametrize("direction", ["outgoing", "incoming"])
 def test_triangle_multiplication_sampled_elements(cuda_device, n, n_pad, direction):
     from foldjax_b200 import _device as dev, _lib

@@ -1,5 +1,5 @@
 """The triangle ops at the shapes of their other call sites, through the C ABI's general
-path (CUDA-core stages around the tensor-core contraction):
+path (unfused tensor-core products between layer-norm passes):
 
 * the template stacks' c_z = 64 with c_hidden = 128, which the reference's fused
   cuEquivariance kernel rejects (src/foldjax/models/protenix/models/triangle/triangle.py:131-137);
