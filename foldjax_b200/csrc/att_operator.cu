@@ -146,7 +146,8 @@ extern "C" int b200tri_attention_core(const b200tri_attention_core_args* a, b200
       __nv_bfloat16* copy = reinterpret_cast<__nv_bfloat16*>(ws + pl.bias);
       const long long rows = static_cast<long long>(HEADS) * a->n_j;
       const long long want = (rows * ld + 255) / 256;
-      const dim3 bias_grid(static_cast<unsigned>(want < 148 * 16 ? want : 148 * 16));
+      const long long most = 16ll * sm_count();
+      const dim3 bias_grid(static_cast<unsigned>(want < most ? want : most));
       if (a->bias_f32)
         rc = launch(bias_kernel<float>, bias_grid, block, 0, stream, false, reinterpret_cast<const float*>(bias), copy, rows,
                     a->n_k, ld);

@@ -478,9 +478,12 @@ int launch_row_norm(const RowArgs& a, cudaStream_t stream, bool pdl) {
   return launch(row_norm_kernel, dim3(a.rows), dim3(ROW_THREADS), 0, stream, pdl, a, aligned);
 }
 
-// Enough splits that the tiles cover the SMs, at least two k steps each, none of them empty.
+// Enough splits that the tiles cover the SMs, at least two k steps each, none of them empty. A B200's
+// SM count and not the limit that may be set on it: the splits are float32 sums of their own, and the
+// bits of a result are not to depend on how many SMs it was computed on.
 int single_splits(int tiles, int kb) {
-  int s = 148 / (tiles > 0 ? tiles : 1);
+  constexpr int SMS = 148;
+  int s = SMS / (tiles > 0 ? tiles : 1);
   s = s > kb / 2 ? kb / 2 : s;
   s = s > SINGLE_MAX_SPLITS ? SINGLE_MAX_SPLITS : s;
   if (s <= 1) return 1;

@@ -353,7 +353,6 @@ __device__ __forceinline__ float fast_rcp(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float sigmoid_f32(float x) { return fast_rcp(1.0f + fast_exp2(-1.4426950408889634f * x)); }
 __device__ __forceinline__ float2 sigmoid_f32x2(float2 x) {
   const float2 t = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
   const float2 d = __fadd2_rn(make_float2(fast_exp2(t.x), fast_exp2(t.y)), make_float2(1.0f, 1.0f));

@@ -88,3 +88,24 @@ def test_single_representation_off_the_16_byte_grid(cuda_device, monkeypatch, n,
     assert got[0].data_ptr() % 16 and got[1].data_ptr() % 16
     for w, g in zip(want, got):
         assert torch.equal(w, g)
+
+
+def test_results_do_not_depend_on_the_sm_limit(cuda_device):
+    """Fewer SMs, the same K splits and therefore the same bits."""
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.pairformer import pairformer_forward
+
+    rng = np.random.default_rng(9)
+    n, lib = 136, _lib.load()
+    pd = dev.params_to_device(_params(rng, 16, 1536))
+    z = dev.to_device(rng.standard_normal((1, n, n, 128)).astype(np.float32), torch.bfloat16)
+    s = torch.from_numpy(rng.standard_normal((1, n, 384)).astype(np.float32)).cuda()
+    want = pairformer_forward([pd, pd], s, z, torch.ones(1, n, device="cuda"), None)
+    _lib.check(lib.b200tri_set_sm_limit(40))
+    try:
+        got = pairformer_forward([pd, pd], s, z, torch.ones(1, n, device="cuda"), None)
+        _lib.device_status()
+    finally:
+        _lib.check(lib.b200tri_set_sm_limit(0))
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
