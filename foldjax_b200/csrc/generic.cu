@@ -888,7 +888,7 @@ TriattPlan triatt_plan(int n, int batch, int c_z, int heads, int head_dim, bool 
   pl.bias = w.take(rows * heads * ld * (f32 ? 4 : 2));
   pl.mb = w.take(rows * ld * 4);
   pl.o = w.take(pairs * hd * (f32 ? 4 : 2));
-  pl.y = f32 ? w.take(pieces * pairs * hd * 2) : pl.o;
+  pl.y = f32 ? pl.q : pl.o;  // the gated output: over the queries, which the core has read, or in place
   for (int i = 0; i < 6; ++i) pl.w[i] = w.take(pieces * c_z * (i == 3 ? static_cast<size_t>(round_up(heads, 8)) : hd) * 2);
   pl.total = w.total();
   return pl;

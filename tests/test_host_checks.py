@@ -233,3 +233,14 @@ def test_pairformer_refuses_a_pair_tensor_off_the_16_byte_grid(gate):
                                    workspace=address, workspace_bytes=size)
         assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_INVALID
         assert b"16-byte aligned" in lib.b200tri_last_error()
+
+
+def test_float32_attention_scratch_holds_nothing_twice():
+    """Per pair and channel: the normalised row, q, k and v as three bf16 pieces each and the float32
+    output; the gated output's pieces take the place of q's."""
+    from foldjax_b200 import _lib
+
+    n, c = 1024, 128
+    size = _lib.load().b200tri_triatt_workspace_bytes_shape(n, _lib.DTYPE_F32, c, 4, 32)
+    rows = n * n * c * (4 * 3 * 2 + 4)
+    assert rows < size < 1.01 * rows
