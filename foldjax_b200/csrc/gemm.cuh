@@ -12,6 +12,14 @@
 // have an accumulator of their own, where that half ulp is 2^-8 smaller, and the leading term
 // alternates between NMAIN accumulators; the epilogue adds them in float32.
 //
+// Single bf16 pieces have one accumulator for all of K. Against float64 without any rounding the
+// triangle ops are as far off as with float32 fma chains on the CUDA cores: 7.46e-3 (multiplication)
+// and 7.1e-3 (attention) of the result at 384 channels, equal to 3e-5 of that on average and to 2e-4
+// in every case of 48 to 311 tokens; it is the bf16 roundings that count. Against the same bf16
+// roundings with exact sums between them more results round the other way: of the 384-channel
+// multiplication 7.9 % instead of 6.1, of the attention 6.0 instead of 4.4; at 64 channels 1.65
+// instead of 1.6 and 0.69 instead of 0.63.
+//
 // piece_gemm_kernel: persistent, tiles of 128 x BN.
 //   warp 0       TMA producer: per k step of 64 every piece of A [128][64] and of B [BN][64],
 //                each K-major (activations) or MN-major (weights as stored, [in][out])

@@ -17,8 +17,8 @@
 // and an attention five
 //   layer norm -> q, k, v, bias product -> core -> gate product -> output product
 // (plus one that splits or pads weights where they cannot be read as stored). The layer norms
-// are CUDA-core kernels. Before, everything but the contraction ran on CUDA cores: 26.2 ms for the four
-// updates of a 256-token 384-channel refiner block, 6.9 ms for four 200-token templates.
+// are CUDA-core kernels. The four updates of a 256-token 384-channel refiner block take 1.32 ms and
+// those of four 200-token templates 0.81 (26.2 and 6.9 with the products on the CUDA cores).
 //
 // With a bf16 trunk every point where the reference's bf16 arrays round (after each matmul,
 // the sigmoid, each elementwise product or sum, the two steps of the layer-norm affine,
@@ -1091,7 +1091,11 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         const int tiles_w = (hd + Pol::BN - 1) / Pol::BN;
         const GemmShape g = {m_tiles, 3 * tiles_w + (heads + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
         const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
-        // (with more k steps two streaming CTAs per SM hide each other's epilogues better)
+        // (Kept / streamed, us of the whole bf16 attention of 256 tokens: 128 channels of 8 x 16 heads
+        // 172 / 184, of 12 x 32 304 / 294; 192 of 6 x 32 213 / 220; 256 of 8 x 32 246 / 252; 320 of 10 x 32
+        // 314 / 311; 384 of 12 x 32 367 / 363. Keeping pays where a weight is few column tiles wide, in
+        // float32 up to 128 channels: 455 / 491 for four 200-token templates, 333 / 313 at 192. The rule
+        // goes by k steps, which is within 4 % of the better side.)
         return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
                                                 ws + pl.bias}, ksteps(c_z) <= 2, stream);

@@ -34,14 +34,18 @@
 //
 // Bound: not the tensor pipe and not HBM. Per score the SM issues about 7 instructions (3-input
 // max, packed fma, ex2 or the cubic with its exponent insertion, clamp, half a cvt) against 128
-// tensor flops, and the MUFU unit delivers 16 exponentials per clock and SM: the kernel runs
-// at about 60 % of its issue slots with the tensor pipe under 40 % busy at head dim 32. What a
+// tensor flops, and the MUFU unit delivers 16 exponentials per clock and SM: the kernel issues in
+// 62 % of its slots with the tensor pipe 40 % and the MUFU unit 39 % busy (n = 1024, counters). The
+// other slots are waits: TMEM loads, fixed latencies and the barriers between the roles. What a
 // step costs beyond that is registers: 64 scores per thread under the 128-register limit of 512
 // threads. So nothing that an item's end needs is kept across its steps (the position is worked
 // out again there, with 32-bit divisions) and its result is read back in halves; a warp, not a
 // thread, arrives on the barriers; the next item's queries are loaded while this one still runs.
-// Clocks per step of three rows at n = 256 / 512 / 1024 / 2048: 2970 / 2450 / 2130 / 2020 with
-// the position kept in registers, 2645 / 2315 / 2055 / 1960 so. Measured and not better: score
+// With the position kept in registers a step took 3 to 12 % more.
+// SM clocks of a launch per step of three rows and SM (counter, set-up and last wave included) at
+// n = 256 / 512 / 1024 / 2048: 4010 / 2510 / 2170 / 2070. By time x sampled clock, under the power
+// limit, 2280 / 2195 / 2175 at 1024 / 2048 / 3072: a longer key loop does not cost more clocks, it
+// runs at fewer MHz (1965 while the launches are short, 1690 at n = 3072). Measured and not better: score
 // buffers in pairs, a ring of their own for K and the bias, four stages, 7 or 9 of 16 pairs on
 // the FMA pipe, results staged for a TMA store.
 #include <cuda_fp16.h>
@@ -60,7 +64,7 @@ constexpr int KT = 64;
 constexpr int STAGES = 3;
 constexpr int POLY = 8;    // of every 16 pairs of exponentials, this many are evaluated on the FMA pipe
 constexpr int QBUF = 2;    // the next item's queries arrive while the last steps of this one run
-constexpr int THREADS = 128 + NWG * 128;  // warpgroup 0: producer, MMA issuer, 2 idle warps; then the softmax warpgroups
+constexpr int THREADS = 128 + NWG * 128;  // warpgroup 0: producer, two MMA issuers, an idle warp; then the softmax warpgroups
 constexpr int Q_BYTES = 128 * 64;    // [128 j][32 d] bf16
 constexpr int BIAS_BYTES = 128 * 128;  // [128 j][64 k] bf16
 constexpr int K_BYTES = KT * 64;     // [64 k][32 d] bf16

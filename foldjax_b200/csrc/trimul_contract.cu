@@ -13,11 +13,12 @@
 // Tiles are walked channel by channel so the A_d/B_d panels of the channel in
 // flight (2 * N*N*2 bytes) stay in L2 while all SMs work on them.
 //
-// Bound: large n_k, the operand traffic into the SM (48 KiB per k step, 768 clocks at 64 B/clk,
-// against 512 of products); small n_k, the epilogue. Algorithmic work 2*128*n_i*n_j*n_k*n_src flop.
-// With one warpgroup whose threads stored 64 bytes of a row each (32 lines per instruction) a tile
-// of n = 200 took 11 400 clocks, four times its products and loads. Now 20 -> 15 us at n = 203, 71 -> 49
-// at 500 and 262 -> 214 at 1024.
+// Bound: large n_k, in the narrow form the operand traffic into the SM (48 KiB per k step, 768 clocks
+// at 64 B/clk, against 512 of products), in the wide one an epilogue that no product overlaps (64 KiB
+// for 1024 clocks of products: tensor pipe 68 % busy at n = 1024); small n_k, the epilogue.
+// Algorithmic work 2*128*n_i*n_j*n_k*n_src flop. One epilogue warpgroup whose threads store 64 bytes
+// of a row each (32 lines per instruction) spends 11 400 clocks on a tile of n = 200, four times its
+// products and loads: 20 / 71 / 262 us at n = 203 / 500 / 1024, staged 15 / 49 / 214.
 #include "host.cuh"
 #include "tc.cuh"
 
