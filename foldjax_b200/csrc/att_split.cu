@@ -21,10 +21,10 @@
 //   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
 //   warpgroups  softmax, one thread per query
 // Bound: issue slots. A score costs about 2 instructions of exponential, 4.5 of split and 2-4
-// others, most of them packed two to an instruction; with bf16 operands 52 % of the slots were busy
-// with two softmax warpgroups, 62 % are with three (float32: two, 41 %). With bf16 operands a third one fits, because there the probabilities overwrite
-// the scores in TMEM (OVERLAY): the scores of the next step then wait for this step's P.V, which
-// the other two warpgroups hide.
+// others, most of them packed two to an instruction. Two softmax warpgroups fill 41 % of the slots with
+// float32 operands and 52 % with bf16 ones; there a third one fits (62 %), because the probabilities
+// overwrite the scores in TMEM (OVERLAY): the scores of the next step then wait for this step's P.V,
+// which the other two warpgroups hide.
 #include "att_split.cuh"
 #include "gemm.cuh"
 #include "tc.cuh"

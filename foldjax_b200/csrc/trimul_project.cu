@@ -25,6 +25,8 @@
 // Bound: HBM by the bytes (read x once, write a and b once: 3 * n*n*128*2 bytes, 123 us at n = 1024);
 // in fact the MUFU unit, two operations for each of a pair's 256 sigmoids: 70 % busy over the 213 us
 // of a launch at n = 1024 (285 with one epilogue warpgroup that stored each thread's run directly).
+#include <type_traits>
+
 #include "host.cuh"
 #include "ln.cuh"
 #include "tc.cuh"
@@ -60,10 +62,12 @@ struct ProjParams {
   const void* beta;
   bool early_weights;  // the weights may be read before pdl_wait()
   int rows_per_block;
-  __nv_bfloat16 *a, *b;  // the outputs and their strides, where rows do not end on 16 bytes
-  long long ld, chan_stride, block_stride;
   float eps;
   int* status;
+};
+struct RaggedParams : ProjParams {  // the outputs as the threads address them
+  __nv_bfloat16 *a, *b;
+  long long ld, chan_stride, block_stride;
 };
 
 // RAGGED: rows end inside 16 bytes and what lies behind them is not ours. TMA would write it, so the
@@ -72,7 +76,8 @@ template <bool RAGGED>
 __global__ void __launch_bounds__(THREADS, 1)
 project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_p,
                const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_a,
-               const __grid_constant__ CUtensorMap tm_b, const ProjParams p) {
+               const __grid_constant__ CUtensorMap tm_b,
+               const typename std::conditional<RAGGED, RaggedParams, ProjParams>::type p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -258,13 +263,15 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           tma_store_4d(half ? &tm_b : &tm_a, out, t0, o - block * p.rows_per_block, 0, block);
           tma_store_commit();
         }
-        if (RAGGED && t0 <= whole && whole < t0 + 32) {  // (this thread's own row of the staged tile)
-          const int block = o / p.rows_per_block;
-          __nv_bfloat16* dst = (half ? p.b : p.a) + block * p.block_stride + chan * p.chan_stride +
-                               (o - block * p.rows_per_block) * p.ld + whole;
-          const __nv_bfloat16* src =
-              reinterpret_cast<const __nv_bfloat16*>(out + chan * 64 + ((((whole - t0) >> 3) ^ ((chan >> 1) & 3)) << 4));
-          for (int e = 0; e < p.n_inner - whole; ++e) dst[e] = src[e];
+        if constexpr (RAGGED) {
+          if (t0 <= whole && whole < t0 + 32) {  // (this thread's own row of the staged tile)
+            const int block = o / p.rows_per_block;
+            __nv_bfloat16* dst = (half ? p.b : p.a) + block * p.block_stride + chan * p.chan_stride +
+                                 (o - block * p.rows_per_block) * p.ld + whole;
+            const __nv_bfloat16* src =
+                reinterpret_cast<const __nv_bfloat16*>(out + chan * 64 + ((((whole - t0) >> 3) ^ ((chan >> 1) & 3)) << 4));
+            for (int e = 0; e < p.n_inner - whole; ++e) dst[e] = src[e];
+          }
         }
         if (lane == 0) mbar_arrive(&sm.acc_empty[half]);
       }
@@ -342,7 +349,7 @@ int b200::mul_project_launch(const b200tri_trimul_project_args* a, bool pad_is_s
     int rc = make_tmap(&tm_out[i], i ? a->b : a->a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, str, box, Swz::B64);
     if (rc) return rc;
   }
-  ProjParams p;
+  RaggedParams p;
   p.n_outer = a->n_outer;
   p.n_inner = a->n_inner;
   p.tiles_inner = (a->n_inner + 127) / 128;
@@ -365,12 +372,12 @@ int b200::mul_project_launch(const b200tri_trimul_project_args* a, bool pad_is_s
   p.status = status;
 
   const long long grid = tiles < sm_count() ? tiles : sm_count();
-  auto go = [&](auto kernel) {
+  auto go = [&](auto kernel, const auto& params) {
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem));
     if (rc) return rc;
     TimedLaunch timed(K_TRIMUL_PROJECT, stream);
     return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_x, tm_p, tm_g,
-                  tm_out[0], tm_out[1], p);
+                  tm_out[0], tm_out[1], params);
   };
-  return ragged ? go(project_kernel<true>) : go(project_kernel<false>);
+  return ragged ? go(project_kernel<true>, p) : go(project_kernel<false>, static_cast<const ProjParams&>(p));
 }
