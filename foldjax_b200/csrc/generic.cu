@@ -131,6 +131,19 @@ __global__ void weight_kernel(const WeightJobs jobs) {
 }
 
 // ------------------------------------------------------------------ layer norm + gather
+// Means over c channels. The product with the rounded reciprocal alone is off to the same side in
+// every row unless c is a power of two: where the mean is 5000 deviations the float32 attention of 384
+// channels was 5.1e-4 from float64, 7 times what it is with quotients. One correction by the residual
+// (Markstein, 1990) gives the rounded quotient; a division costs 1 % of a template stack.
+struct Channels {
+  float c, inv;
+  __device__ explicit Channels(int n) : c(static_cast<float>(n)), inv(1.0f / c) {}
+  __device__ __forceinline__ float mean(float sum) const {
+    const float q = sum * inv;
+    return fmaf(fmaf(-q, c, sum), inv, q);
+  }
+};
+
 // xn[piece][(b, o, t)][:] = LN(x[b][o * xs_o + t * xs_i + :]). A warp takes a few successive t of
 // one row, each in the registers of a group of lanes, so that the loads of all of them are in
 // flight together. Optionally the pair's mask bias of the attention core, mb[(b, o)][t] (the
@@ -204,7 +217,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a
       }
     }
   }
-  const float inv_c = 1.0f / a.c;
+  const Channels chans(a.c);
   float s[R], q[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -220,7 +233,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a
     for (int r = 0; r < R; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], d);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    s[r] *= inv_c;
+    s[r] = chans.mean(s[r]);
     q[r] = 0.f;
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -236,7 +249,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a
 #pragma unroll
     for (int r = 0; r < R; ++r) q[r] += __shfl_xor_sync(0xffffffffu, q[r], d);
 #pragma unroll
-  for (int r = 0; r < R; ++r) q[r] = 1.0f / sqrtf(q[r] * inv_c + a.eps);
+  for (int r = 0; r < R; ++r) q[r] = 1.0f / sqrtf(chans.mean(q[r]) + a.eps);
   const long long plane = static_cast<long long>(a.batch) * a.n * a.n * a.c;
   __nv_bfloat16* dst = a.xn + (static_cast<long long>(bo) * a.n + t_lane) * a.c;
 #pragma unroll
@@ -322,13 +335,13 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
 #pragma unroll
   for (int u = 0; u < JL; ++u) part[(warp * JL + u) * 32 + lane] = s[u];
   __syncthreads();
-  const float inv_c = 1.0f / c_h;
+  const Channels chans(c_h);
 #pragma unroll
   for (int u = 0; u < JL; ++u) {
     s[u] = 0.f;
 #pragma unroll
     for (int w = 0; w < LNT_WARPS; ++w) s[u] += part[(w * JL + u) * 32 + lane];
-    s[u] *= inv_c;  // the mean
+    s[u] = chans.mean(s[u]);
   }
   for (int g = warp; g < groups; g += LNT_WARPS)
 #pragma unroll
@@ -349,7 +362,7 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
     q[u] = 0.f;
 #pragma unroll
     for (int w = 0; w < LNT_WARPS; ++w) q[u] += part_q[(w * JL + u) * 32 + lane];
-    q[u] = 1.0f / sqrtf(q[u] * inv_c + eps);
+    q[u] = 1.0f / sqrtf(chans.mean(q[u]) + eps);
   }
   const X* scale = static_cast<const X*>(scale_);
   const X* bias = static_cast<const X*>(bias_);

@@ -121,3 +121,30 @@ def test_float32_cuda_tensor_selects_the_mode_and_stays_on_device(cuda_device):
     assert _max_abs(ref, out.cpu().numpy()) <= F32_TOL
     with pytest.raises(ValueError, match="Unsupported dtype"):
         triangle_multiplication_forward(params, x, None, "outgoing", dtype="float16")
+
+
+@pytest.mark.parametrize("c_z,heads", [(72, 2), (200, 6), (384, 12)])
+def test_layer_norm_of_rows_far_from_zero(cuda_device, c_z, heads):
+    """Means of 5000 deviations over channel counts that are no power of two.
+
+    A mean rounded once is off by 1.4e-7 rms (half an ulp of 5 at most), its sum about as much again;
+    1 / sqrt(1e-6 + 1e-5) makes 4 to 6e-5 of that in normalised rows of rms 0.3, with a sign of its own in
+    every row: 2e-4 of the values, and of their average over the keys, which shrinks both alike; 4e-4
+    with a factor of two to spare. An error on the same side in every row (a rounded 1 / c in place of
+    the division, 5e-8 to 1.6e-7 here) is not averaged away: sqrt(96) times its share, 5e-4 to 1.6e-3."""
+    from foldjax_b200 import _lib
+    from foldjax_b200.triangle_attention import triangle_attention_forward
+
+    n, rng = 96, np.random.default_rng(c_z)
+    w = lambda a, b: {"kernel": (rng.standard_normal((a, b)) * a ** -0.5).astype(np.float32)}
+    width = heads * 32
+    params = {"layer_norm": {"scale": np.ones(c_z, np.float32), "bias": np.zeros(c_z, np.float32)}, "linear": w(c_z, heads),
+              "mha": {k: w(c_z, width) for k in ("linear_q", "linear_k", "linear_v", "linear_g")} | {"linear_o": w(width, c_z)}}
+    x = (5.0 + 1e-3 * rng.standard_normal((1, n, n, c_z))).astype(np.float32)
+    mask = np.ones((1, n, n), np.float32)
+    got = triangle_attention_forward(params, x, mask, dtype="float32")
+    _lib.device_status()
+    ref = orc.triangle_attention(params, x, mask, True, dtype="float64")
+    err = np.linalg.norm(got - ref) / np.linalg.norm(ref)
+    print(f"c_z {c_z}: {err:.2e}")
+    assert err < 4e-4
