@@ -177,27 +177,22 @@ def pad_pair(grid: Grid, z: torch.Tensor, mask: torch.Tensor | None):
     return zp, mp
 
 
-def _ws(tag: str, nbytes: int) -> tuple[int, int]:
-    raw = dev.workspace(nbytes + 1024, tag)
-    return dev.aligned_ptr(raw), nbytes
-
-
-
-
-def _exchange_workspace(ctx: CPContext, n: int) -> tuple[int | None, int]:
-    """(workspace pointer or None, bytes) for the two context-parallel ops at ``n`` tokens. None
-    selects the communicator's own workspace, sized here for both ops (collective: every rank
-    reaches this call with the same ``n`` at the same point of its op sequence)."""
+def _exchange_workspace(ctx: CPContext, n: int) -> tuple[torch.Tensor | None, int | None, int]:
+    """(buffer, pointer into it, bytes) for the two context-parallel ops at ``n`` tokens; the caller
+    holds the buffer until its op is enqueued (under capture nobody else does). None selects the
+    communicator's own workspace, sized here for both ops (collective: every rank reaches this call
+    with the same ``n`` at the same point of its op sequence)."""
     lib = _lib.load()
     need = max(lib.b200tri_trimul_cp_workspace_bytes(C.c_void_p(ctx.comm), n),
                lib.b200tri_triatt_cp_workspace_bytes(C.c_void_p(ctx.comm), n))
     if TRANSPORT == "nccl":
-        return _ws("cp_exchange", need)
+        buf = dev.workspace(need, "cp_exchange")
+        return buf, dev.aligned_ptr(buf), need
     if TRANSPORT not in ("push", "pull"):
         raise ValueError(f"B200TRI_CP_TRANSPORT must be 'push', 'pull' or 'nccl', got {TRANSPORT!r}")
     out = C.c_void_p()
     _lib.check(lib.b200tri_comm_workspace(C.c_void_p(ctx.comm), need, C.byref(out)))
-    return None, 0
+    return None, None, 0
 
 
 def _tile_checks(ctx: CPContext, x: torch.Tensor, mask, residual, out) -> tuple[int, torch.Tensor]:
@@ -244,7 +239,7 @@ def triangle_multiplication_cp(
     lv = {k: _leaf(params, *k.split(".")) for k in (
         "norm_in.scale", "norm_in.bias", "p_in.kernel", "g_in.kernel", "norm_out.scale", "norm_out.bias",
         "p_out.kernel", "g_out.kernel")}
-    wp, wb = _exchange_workspace(ctx, n)
+    buf, wp, wb = _exchange_workspace(ctx, n)  # (buf: held until the call below returns)
     args = _lib.TrimulCpArgs(
         n=n, incoming=int(direction == "incoming"), eps=float(eps), x=x.data_ptr(),
         mask=None if mask is None else mask.data_ptr(),
@@ -283,7 +278,7 @@ def triangle_attention_cp(
     lv = {k: _leaf(params, *k.split(".")) for k in (
         "layer_norm.scale", "layer_norm.bias", "linear.kernel", "mha.linear_q.kernel", "mha.linear_k.kernel",
         "mha.linear_v.kernel", "mha.linear_g.kernel", "mha.linear_o.kernel")}
-    wp, wb = _exchange_workspace(ctx, n)
+    buf, wp, wb = _exchange_workspace(ctx, n)  # (buf: held until the call below returns)
     args = _lib.TriattCpArgs(
         n=n, starting=int(bool(starting)), heads=4, head_dim=32, inf=float(inf), eps=float(eps), x=x.data_ptr(),
         mask=None if mask is None else mask.data_ptr(),

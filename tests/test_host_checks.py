@@ -98,6 +98,22 @@ def test_captured_calls_keep_no_scratch(monkeypatch):
     dev.release_workspaces()
 
 
+def test_exchange_scratch_is_held_by_the_op(monkeypatch):
+    """A captured call's buffer is kept by nobody else: its pointer alone would outlive it."""
+    from types import SimpleNamespace
+
+    from foldjax_b200 import _lib, cp
+
+    _host_scratch(monkeypatch)
+    monkeypatch.setattr(dev.torch.cuda, "is_current_stream_capturing", lambda: True)
+    size = SimpleNamespace(b200tri_trimul_cp_workspace_bytes=lambda *_: 4096, b200tri_triatt_cp_workspace_bytes=lambda *_: 8192)
+    monkeypatch.setattr(_lib, "load", lambda: size)
+    monkeypatch.setattr(cp, "TRANSPORT", "nccl")
+    buf, pointer, nbytes = cp._exchange_workspace(SimpleNamespace(comm=0), 64)
+    assert nbytes == 8192 and pointer % 1024 == 0
+    assert buf.data_ptr() <= pointer and pointer + nbytes <= buf.data_ptr() + buf.numel()
+
+
 def test_threads_do_not_share_scratch(monkeypatch):
     import gc
     import threading
