@@ -48,6 +48,15 @@
 // runs at fewer MHz (1965 while the launches are short, 1690 at n = 3072). Measured and not better: score
 // buffers in pairs, a ring of their own for K and the bias, four stages, 7 or 9 of 16 pairs on
 // the FMA pipe, results staged for a TMA store.
+// Attention operator, us, n = 256 / 384 / 1024 / 3072: with every role's index and loops divergent (a
+// thread of its own, operands through vector registers) and P.V of the step before waited for ahead
+// of the maximum, 43.5 / 113.3 / 1505 / 39600; the warp index through a shuffle 43.2 / 110.6 / 1458; the
+// wait moved behind the exponentials 42.1 / 109.5 / 1432; uniform issuer loops 41.2 / 106.6 / 1402 /
+// 37500; the two waits at a step's start as one and the producer's loop uniform 41.1 / 105.3 / 1364 /
+// 36800. A product takes its issuer 60 to 90 clocks and the tensor pipe 48 (A from shared memory) or
+// 24 (P, 128x48), 386 for a row's step measured alone. Measured and not better: a second Q.K^T issuer
+// (1498), four rows with 32 scores at a time and an issuer per row and product (1459 with the same
+// offsets; the rows fall into phase and queue for the same unit).
 #include <cuda_fp16.h>
 
 #include <mutex>
@@ -149,7 +158,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ TileMaps tm, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5;
+  // (through a shuffle, so that the compiler knows it to be the same in all lanes)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   if ((smem_u32(smem_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
@@ -223,24 +233,28 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0, item_it = 0;
-      bool alive = true;
-      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
-        int h, i0, j0;
-        locate(item, h, i0, j0);
-        const uint32_t qb = item_it % QBUF;
-        if (!mbar_wait(&sm.q_empty[qb], ((item_it / QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+    // ---- TMA producer (like the issuers: all lanes walk the loops, one issues)
+    const bool leader = elect_one();
+    int stage = 0;
+    uint32_t phase = 0, item_it = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+      int h, i0, j0;
+      locate(item, h, i0, j0);
+      const uint32_t qb = item_it % QBUF;
+      if (!mbar_wait(&sm.q_empty[qb], ((item_it / QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+      if (leader) {
         mbar_expect_tx(&sm.q_full[qb], NWG * Q_BYTES);
         for (int g = 0; g < NWG; ++g) tma_load_4d(sm.q[qb][g], &tm_q, &sm.q_full[qb], 0, h, j0, i0 + g);
-        for (int t = 0; t < p.steps; ++t) {
-          if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
-            alive = false;
-            break;
-          }
-          const int tile = t / p.steps_per_tile;
-          const int k0 = (t - tile * p.steps_per_tile) * KT;
+      }
+      for (int t = 0; t < p.steps; ++t) {
+        if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
+          alive = false;
+          break;
+        }
+        const int tile = t / p.steps_per_tile;
+        const int k0 = (t - tile * p.steps_per_tile) * KT;
+        if (leader) {
           mbar_expect_tx(&sm.st_full[stage], STAGE_TX);
           tma_load_3d(sm.bias[stage], &tm.b[tile], &sm.st_full[stage], k0, j0, h);
           for (int g = 0; g < NWG; ++g) {
@@ -248,92 +262,94 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             tma_load_2d(sm.mb[stage][g], &tm.m[tile], &sm.st_full[stage], k0, i0 + g);
             tma_load_3d(sm.v[stage][g], &tm.v[tile], &sm.st_full[stage], k0, h * 32, i0 + g);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ---- Q.K^T issuer: S[wg] = Q[wg] . K[stage][wg]^T as soon as the warpgroup has
     // taken the previous scores out of TMEM. Kept apart from the P.V issuer so that
-    // neither product waits behind the other's barrier; both are single threads
-    // competing with four softmax warps for issue slots on their sub-partition.
-    if (elect_one()) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, KT);
-      int stage = 0;
-      uint32_t phase = 0, item_it = 0, g = 0;  // g: global step counter
-      bool alive = true;
-      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
-        const uint32_t qb = item_it % QBUF;
-        if (!mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA)) break;
-        for (int t = 0; t < p.steps && alive; ++t, ++g) {
-          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
+    // neither product waits behind the other's barrier. All lanes walk the loops and one of
+    // them issues, so that control flow and descriptors stay in uniform registers.
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(128, KT);
+    const uint64_t identdesc = desc_sw128(smem_u32(sm.ident));
+    int stage = 0;
+    uint32_t phase = 0, item_it = 0, g = 0;  // g: global step counter
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+      const uint32_t qb = item_it % QBUF;
+      if (!mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA)) break;
+      for (int t = 0; t < p.steps && alive; ++t, ++g) {
+        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
+          alive = false;
+          break;
+        }
+        const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
+#pragma unroll
+        for (int wg = 0; wg < NWG; ++wg) {
+          if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
             alive = false;
             break;
           }
-          for (int wg = 0; wg < NWG; ++wg) {
-            if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
-            const uint64_t adesc = desc_sw64(smem_u32(sm.q[qb][wg]));
-            const uint64_t bdesc = desc_sw64(smem_u32(sm.k[stage][wg]));
-            const uint32_t d = tmem_base + wg * TM_WG + TM_S;
-            const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
-            const uint64_t identdesc = desc_sw128(smem_u32(sm.ident));
+          tc_fence_after();
+          const uint64_t adesc = desc_sw64(smem_u32(sm.q[qb][wg]));
+          const uint64_t bdesc = desc_sw64(smem_u32(sm.k[stage][wg]));
+          const uint32_t d = tmem_base + wg * TM_WG + TM_S;
+          if (leader) {
 #pragma unroll
             for (int kk = 0; kk < KT / 16; ++kk)
-              umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_qk,
-                           kk != 0);
+              umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_qk, kk != 0);
             umma_bf16_ss(d, adesc, bdesc, idesc_qk, 1);
             umma_bf16_ss(d, umma_desc_advance(adesc, 32), umma_desc_advance(bdesc, 32), idesc_qk, 1);
             umma_commit(&sm.s_full[wg]);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
         }
-        if (alive) umma_commit(&sm.q_empty[qb]);  // every Q.K^T of the item has been issued
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
+      if (alive && leader) umma_commit(&sm.q_empty[qb]);  // every Q.K^T of the item has been issued
     }
   } else if (warp == 2) {
     // ---- P.V issuer: O[wg] (+)= P[wg] . V[stage][wg], P read from TMEM.
-    if (elect_one()) {
-      constexpr uint32_t idesc_pv = idesc_f16(128, V_ROWS);
-      int stage = 0;
-      uint32_t phase = 0, g = 0;
-      bool alive = true;
-      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
-        for (int t = 0; t < p.steps && alive; ++t, ++g) {
-          // (already complete when P arrives; observed here so this thread's products
-          // are ordered after the TMA writes of V)
-          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
-          for (int wg = 0; wg < NWG; ++wg) {
-            if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
-            const uint64_t vdesc = desc_sw128(smem_u32(sm.v[stage][wg]));
-            const uint32_t d = tmem_base + wg * TM_WG + TM_O;
-            const uint32_t a = tmem_base + wg * TM_WG + TM_P;
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_pv = idesc_f16(128, V_ROWS);
+    int stage = 0;
+    uint32_t phase = 0, g = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
+      for (int t = 0; t < p.steps && alive; ++t, ++g) {
+        // (already complete when P arrives; observed here so this thread's products
+        // are ordered after the TMA writes of V)
+        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
+        for (int wg = 0; wg < NWG; ++wg) {
+          if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
+            alive = false;
+            break;
+          }
+          tc_fence_after();
+          const uint64_t vdesc = desc_sw128(smem_u32(sm.v[stage][wg]));
+          const uint32_t d = tmem_base + wg * TM_WG + TM_O;
+          const uint32_t a = tmem_base + wg * TM_WG + TM_P;
+          if (leader) {
 #pragma unroll
             for (int k = 0; k < KT / 16; ++k)
               umma_bf16_ts(d, a + k * 8, umma_desc_advance(vdesc, k * 32), idesc_pv, (t | k | p.resume) != 0);
             umma_commit(&sm.pv_done[wg]);
           }
-          if (!alive) break;
-          // K of this stage was consumed before the softmax saw its scores, V by the
-          // products just issued: the stage is free once they complete.
-          umma_commit(&sm.st_empty[stage]);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        if (!alive) break;
+        // K of this stage was consumed before the softmax saw its scores, V by the
+        // products just issued: the stage is free once they complete.
+        if (leader) umma_commit(&sm.st_empty[stage]);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
@@ -389,8 +405,10 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_fence_before();
       }
       for (int t = 0; t < p.steps; ++t, ++g) {
-        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) ||
-            !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+        // (both asked at once: nearly always there already, and one latency instead of two)
+        const bool st_there = mbar_test(&sm.st_full[stage], phase), s_there = mbar_test(&sm.s_full[wg], g & 1);
+        if ((!st_there && !mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX)) ||
+            (!s_there && !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX))) {
           alive = false;
           break;
         }
@@ -432,13 +450,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
-        // P buffer free and O stable once the previous step's P.V has completed (it
-        // was issued before this step's Q.K^T, so this wait does not stall).
-        if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
-          alive = false;
-          break;
-        }
-        tc_fence_after();
         // four independent chains, so the reduction is not one 32-deep dependency
         float mxa = fmaxf(u[0].x, u[0].y), mxb = fmaxf(u[1].x, u[1].y);
         float mxc = fmaxf(u[2].x, u[2].y), mxd = fmaxf(u[3].x, u[3].y);
@@ -470,6 +481,9 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const float2 log2e2 = make_float2(LOG2E, LOG2E);
           const float2 nm2 = make_float2(-m2_used, -m2_used);
           const float2 mm2 = make_float2(EXP_MAGIC - m2_used, EXP_MAGIC - m2_used);
+          // P buffer free and O stable once the previous step's P.V has completed: asked here, needed
+          // (and by then nearly always so) when the first half of P is there.
+          const bool p_free = mbar_test(&sm.pv_done[wg], (g & 1) ^ 1);
           const float u_min = (m2_used - 120.0f) * LN2;  // keeps the polynomial path's t above about -120
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
@@ -489,9 +503,14 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const __half2 h2 = __floats2half2_rn(ex.x, ex.y);
               packed[e] = *reinterpret_cast<const uint32_t*>(&h2);
             }
+            if (half == 0) {
+              if (!p_free && !mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) alive = false;
+              tc_fence_after();
+            }
             tmem_st16(t_wg + TM_P + 16 * half, packed);
           }
         }
+        if (!alive) break;
         if ((t > 0 || p.resume) && any_need) {
           uint32_t o[32];
           tmem_ld32(t_wg + TM_O, o);
