@@ -62,7 +62,8 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_out, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5;
+  // (through a shuffle, so that the compiler knows it to be the same in all lanes)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   if ((smem_u32(smem_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);

@@ -69,7 +69,8 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
 
-  const int warp = threadIdx.x >> 5;
+  // (through a shuffle, so that the compiler knows it to be the same in all lanes)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
   if (warp == 0 && lane == 0) {
