@@ -296,7 +296,8 @@ int launch_ln_gather(LnArgs a, cudaStream_t stream, bool pdl) {
 // partial sums each) and nothing is shuffled: 40 instructions per pair where one warp per pair
 // took 209. Eight neighbouring channels per lane are 16 bytes; in bf16, up to 64 * G channels, they
 // are put together in shared memory (over the values, when all have been read) and leave as one
-// contiguous run: stored by the lanes themselves they went to 64 rows, half a sector each.
+// contiguous run: stored by the lanes themselves they went to 64 rows, half a sector each. In
+// float32, up to 384 channels, the three pieces have a place of their own behind the values (G = 1).
 constexpr int LNT_WARPS = 8;
 template <bool BF>
 constexpr int lnt_j() {
@@ -366,7 +367,37 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
   }
   const X* scale = static_cast<const X*>(scale_);
   const X* bias = static_cast<const X*>(bias_);
-  if constexpr (G > 0) {
+  if constexpr (!BF && G > 0) {
+    const int pitch = (groups + 7) & ~7;  // (as below)
+    uint4* rows = reinterpret_cast<uint4*>(part + 2 * LNT_WARPS * 64);
+    for (int g = warp; g < groups; g += LNT_WARPS) {
+      uint32_t w[3][4];
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const int c = g * 8 + e;
+        float v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          v[u] = (__uint_as_float(tile[(c + u) * 32 + lane]) - s[0]) * q[0] * static_cast<float>(scale[c + u]) +
+                 static_cast<float>(bias[c + u]);
+        split3x2(v[0], v[1], w[0][e / 2], w[1][e / 2], w[2][e / 2]);
+      }
+#pragma unroll
+      for (int x = 0; x < 3; ++x)
+        rows[(x * 32 + lane) * pitch + (g ^ (lane & 7))] = make_uint4(w[x][0], w[x][1], w[x][2], w[x][3]);
+    }
+    __syncthreads();
+    const int count = min(JT, n - j0) * groups;
+    for (int x = 0; x < 3; ++x) {
+      uint4* dst = reinterpret_cast<uint4*>(tn + x * pairs * c_h + ((static_cast<long long>(b) * n + i) * n + j0) * c_h);
+      for (int idx = threadIdx.x; idx < count; idx += LNT_WARPS * 32) {
+        const int j = idx / groups, g = idx - j * groups;
+        dst[idx] = rows[(x * 32 + j) * pitch + (g ^ (j & 7))];
+      }
+    }
+    return;
+  }
+  if constexpr (BF && G > 0) {
     uint4 out[G][JL];
 #pragma unroll
     for (int k = 0; k < G; ++k) {
@@ -428,15 +459,17 @@ template <bool BF>
 int launch_ln_channel_major(const void* t, int n, int batch, int ld, int c_h, const void* scale, const void* bias, float eps,
                             __nv_bfloat16* tn, cudaStream_t stream) {
   const dim3 grid((n + lnt_j<BF>() - 1) / lnt_j<BF>(), static_cast<unsigned>(n), static_cast<unsigned>(batch));
-  auto go = [&](auto kernel) {
-    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), lnt_smem(1024));
+  auto go = [&](auto kernel, int staged = 0) {
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), staged ? lnt_smem(384) + 384 * 192 : lnt_smem(1024));
     if (rc) return rc;
-    return launch(kernel, grid, dim3(LNT_WARPS * 32), lnt_smem(round_up(c_h, 64)), stream, true, t, n, ld, c_h, scale, bias, eps,
+    return launch(kernel, grid, dim3(LNT_WARPS * 32), lnt_smem(round_up(c_h, 64)) + staged, stream, true, t, n, ld, c_h, scale, bias, eps,
                   static_cast<long long>(batch) * n * n, tn);
   };
   if constexpr (BF) {
     if (c_h <= 128) return go(ln_channel_major_kernel<BF, 2>);
     if (c_h <= 384) return go(ln_channel_major_kernel<BF, 6>);
+  } else if (c_h <= 384) {
+    return go(ln_channel_major_kernel<BF, 1>, round_up(c_h, 64) * 192);
   }
   return go(ln_channel_major_kernel<BF, 0>);
 }
