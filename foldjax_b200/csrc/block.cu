@@ -53,13 +53,19 @@ struct Offsets {
 };
 
 struct Plan {
-  size_t w, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
+  size_t w, w2, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
 };
+
+// One tile of the pair track's stage kernels per SM and some SMs over (a contraction has 128 tiles
+// there): what runs on the side stream has SMs of its own.
+constexpr int LEFT_OVER_BELOW = 128;
+bool leaves_sms(int n) { return n <= LEFT_OVER_BELOW; }
 
 Plan plan(int n, int c_s, int heads_s, int hidden_z, int hidden_s, bool single) {
   Plan p = {};
   Offsets o;
   p.w = o.take(static_cast<size_t>(n) * n * 128 * 2);
+  if (single && leaves_sms(n)) p.w2 = o.take(static_cast<size_t>(n) * n * 128 * 2);
   size_t sub = b200tri_trimul_workspace_bytes(n);
   const size_t cand[2] = {b200tri_triatt_workspace_bytes(n), b200tri_pair_transition_workspace_bytes(hidden_z)};
   for (size_t c : cand) sub = c > sub ? c : sub;
@@ -247,9 +253,16 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
       return rc;
   }
 
+  // Where the pair track leaves SMs over, the pair bias is on the side stream as well, on those SMs,
+  // while the next block's pair track runs on z in a buffer of its own (blocks end in z_out and w2 in
+  // turn, the last one in z_out).
+  const bool bias_aside = single && lease->stream && leaves_sms(n) && sm_count() >= LEFT_OVER_BELOW + 16;
+  const int over = bias_aside ? sm_count() - LEFT_OVER_BELOW : 0;
+
   PdlChain chain(false);
   for (int layer = 0; layer < a->n_blocks; ++layer) {
     const b200tri_pairformer_block_params P = params_of(layer);
+    void* z_end = bias_aside && (a->n_blocks - 1 - layer) % 2 ? static_cast<void*>(ws + pl.w2) : a->z_out;
     // ---- pair track: the four triangle updates ping-pong between z_out and w (the first one
     // reads the caller's z_in), residual adds fused; with the pair gate, dropped pairs are
     // zeroed before the first update and after every update
@@ -260,7 +273,7 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
     for (int k = 0; k < 4; ++k) {
       // Boltz-2 / Protenix / OpenFold3 default: multiplications first; attention_first swaps the halves
       const int op = a->attention_first ? (k + 2) % 4 : k;  // 0 out, 1 in, 2 start, 3 end
-      void* dst = z_cur == w ? a->z_out : w;
+      void* dst = z_cur == w ? z_end : w;
       if (op < 2) {
         const b200tri_trimul_params& m = op == 0 ? P.tri_mul_out : P.tri_mul_in;
         b200tri_trimul_args t = {};
@@ -311,37 +324,46 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
       if (gate && (rc = gate_pairs(dst, dst))) return rc;
       z_cur = dst;
     }
-    // four updates from z_in (or z_out) end in z_out
+    // four updates from wherever the block before ended end in z_end
     {
       b200tri_pair_transition_args t = {};
       t.rows = static_cast<int64_t>(n) * n;
       t.channels = 128;
       t.hidden = P.transition_z.hidden;
       t.eps = a->eps;
-      t.x = a->z_out;
+      t.x = z_end;
       t.norm_scale = P.transition_z.norm_scale;
       t.norm_bias = P.transition_z.norm_bias;
       t.fc1 = P.transition_z.fc1;
       t.fc2 = P.transition_z.fc2;
       t.fc3 = P.transition_z.fc3;
-      t.residual = a->z_out;
-      t.out = a->z_out;  // row-local: in place
+      t.residual = z_end;
+      t.out = z_end;  // row-local: in place
       t.workspace = ws + pl.sub;
       t.workspace_bytes = pl.sub_bytes;
       t.row_mask = a->mask_transition ? a->pair_mask : nullptr;
       if ((rc = b200tri_pair_transition(&t, stream_))) return rc;
-      if (gate && (rc = gate_pairs(a->z_out, a->z_out))) return rc;
+      if (gate && (rc = gate_pairs(z_end, z_end))) return rc;
     }
-    z_cur = a->z_out;
+    z_cur = z_end;
     if (!single) continue;
     SideStream& side = *lease;
 
     // ---- single track; the last block's is on the caller's stream
     const bool last = layer + 1 == a->n_blocks, forked = side.stream != nullptr;
-    const b200tri_attention_pair_bias_args t = attention_args(P);
-    if ((rc = side.join()) || (rc = single_pair_bias(&t, att, stream, !forked))) return rc;
-    if (!last && (rc = side.fork())) return rc;
+    b200tri_attention_pair_bias_args t = attention_args(P);
+    t.z = z_end;
     cudaStream_t st = last || !forked ? stream : side.stream;
+    if (bias_aside && !last) {
+      // (z of the block before, which the next block overwrites, has been read)
+      if (layer > 0 && (rc = side.join_early())) return rc;
+      if ((rc = side.fork())) return rc;
+      SmReserve others(sm_count() - over);
+      if ((rc = single_pair_bias(&t, att, st, false)) || (rc = side.mark_early())) return rc;
+    } else {
+      if ((rc = side.join()) || (rc = single_pair_bias(&t, att, stream, !forked))) return rc;
+      if (!last && (rc = side.fork())) return rc;
+    }
     int splits = 1;
     if ((rc = single_attend(&t, att, partial, &splits, st, last || !forked))) return rc;
     row.base = layer == 0 ? a->s_in : a->s_out;

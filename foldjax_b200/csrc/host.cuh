@@ -122,7 +122,7 @@ bool pdl_chained();
 // somebody's capture), and the call stays on one stream.
 struct SideStream {
   cudaStream_t main, stream = nullptr;
-  cudaEvent_t to_side = nullptr, to_main = nullptr;
+  cudaEvent_t to_side = nullptr, to_main = nullptr, early = nullptr;
   bool joined = true;
   SideStream(cudaStream_t main, bool want);
   ~SideStream();  // joins if need be
@@ -131,6 +131,9 @@ struct SideStream {
   int fork();  // what follows on the side stream comes after what is on the main stream now
   int mark();  // `join` waits for what is on the side stream now
   int join();  // what follows on the main stream comes after the last mark
+  // A mark and a join of their own for something the main stream needs sooner than the rest.
+  int mark_early();
+  int join_early();
 };
 
 // A weight as TMA needs it: `w` itself when it is 16-byte aligned, else a copy in `scratch`.

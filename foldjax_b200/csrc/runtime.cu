@@ -78,7 +78,7 @@ bool pdl_chained() { return t_pdl_chain; }
 namespace {
 struct SideEntry {
   cudaStream_t stream;
-  cudaEvent_t to_side, to_main;
+  cudaEvent_t to_side, to_main, early;
 };
 constexpr size_t SIDE_POOL = 8;  // idle entries kept per device; what exceeds them is destroyed
 std::mutex g_side_mu;
@@ -87,6 +87,7 @@ std::vector<SideEntry> g_side[kMaxDevices];
 void destroy_side(const SideEntry& e) {
   if (e.to_side) cudaEventDestroy(e.to_side);
   if (e.to_main) cudaEventDestroy(e.to_main);
+  if (e.early) cudaEventDestroy(e.early);
   if (e.stream) cudaStreamDestroy(e.stream);  // (returns at once; the stream's work still completes)
 }
 }  // namespace
@@ -107,7 +108,8 @@ SideStream::SideStream(cudaStream_t main_, bool want) : main(main_) {
   if (!e.stream) {
     if (cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&e.to_side, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&e.to_main, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&e.to_main, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&e.early, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       destroy_side(e);
       return;
@@ -116,11 +118,12 @@ SideStream::SideStream(cudaStream_t main_, bool want) : main(main_) {
   stream = e.stream;
   to_side = e.to_side;
   to_main = e.to_main;
+  early = e.early;
 }
 SideStream::~SideStream() {
   if (!stream) return;
   if (!joined && mark() == B200TRI_OK) join();
-  const SideEntry e = {stream, to_side, to_main};
+  const SideEntry e = {stream, to_side, to_main, early};
   std::vector<SideEntry>& pool = g_side[current_device_slot()];
   {
     std::lock_guard<std::mutex> lock(g_side_mu);
@@ -140,6 +143,14 @@ int SideStream::fork() {
 }
 int SideStream::mark() {
   if (stream) B200_CUDA_OK(cudaEventRecord(to_main, stream));
+  return B200TRI_OK;
+}
+int SideStream::mark_early() {
+  if (stream) B200_CUDA_OK(cudaEventRecord(early, stream));
+  return B200TRI_OK;
+}
+int SideStream::join_early() {
+  if (stream) B200_CUDA_OK(cudaStreamWaitEvent(main, early, 0));
   return B200TRI_OK;
 }
 int SideStream::join() {
