@@ -180,6 +180,20 @@ __device__ __forceinline__ void load_eight(const X* p, bool aligned, float (&v)[
     for (int e = 0; e < 8; ++e) v[e] = static_cast<float>(p[e]);
   }
 }
+// The same as they are, of a bf16 row.
+__device__ __forceinline__ uint4 eight_raw(const __nv_bfloat16* p, bool aligned) {
+  if (aligned) return *reinterpret_cast<const uint4*>(p);
+  const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+  return make_uint4(u[0] | (static_cast<uint32_t>(u[1]) << 16), u[2] | (static_cast<uint32_t>(u[3]) << 16),
+                    u[4] | (static_cast<uint32_t>(u[5]) << 16), u[6] | (static_cast<uint32_t>(u[7]) << 16));
+}
+// bf16(bf16(bf16((v - mean) * rstd) * scale) + bias) of two values. Value by value, with conversions to
+// and from float32 at every rounding, the layer norms issued 35 to 46 instructions per value and nothing
+// else bounded them: 160 000 rows of 64 channels took 17 us, their channel-major form of 128 channels 40.
+__device__ __forceinline__ uint32_t affine_bf16x2(float2 v, float2 minus_mean, float2 rstd, uint32_t scale, uint32_t bias) {
+  const float2 t = __fmul2_rn(__fadd2_rn(v, minus_mean), rstd);
+  return bf16x2_add(bf16x2_mul(pack_bf16x2(t.x, t.y), scale), bias);
+}
 // L neighbouring lanes per row, K chunks of eight channels per lane, R rows of a lane group in
 // flight. (With a row per warp and two channels per lane the 64-channel case took 24 us for
 // 160 000 rows, half of it the five exchanges of every sum; three are left.)
@@ -256,6 +270,22 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_gather_kernel(const LnArgs a
   for (int k = 0; k < K; ++k) {
     const int c = c0 + k * L * 8;
     if (c >= a.c) continue;
+    if constexpr (BF) {  // cast before the affine step, whose two roundings are those of packed bf16 operations
+      const uint4 g4 = eight_raw(static_cast<const __nv_bfloat16*>(a.scale) + c, a.aligned_params);
+      const uint4 h4 = eight_raw(static_cast<const __nv_bfloat16*>(a.bias) + c, a.aligned_params);
+      const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, h[4] = {h4.x, h4.y, h4.z, h4.w};
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (t_lane + GROUPS * r >= a.n) break;
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          w[e] = affine_bf16x2(make_float2(v[r][k][2 * e], v[r][k][2 * e + 1]), make_float2(-s[r], -s[r]),
+                               make_float2(q[r], q[r]), g[e], h[e]);
+        *reinterpret_cast<uint4*>(dst + GROUPS * r * a.c + c) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      continue;
+    }
     float g[8], h[8];
     load_eight<BF>(static_cast<const X*>(a.scale) + c, a.aligned_params, g);
     load_eight<BF>(static_cast<const X*>(a.bias) + c, a.aligned_params, h);
@@ -303,17 +333,23 @@ template <bool BF>
 constexpr int lnt_j() {
   return BF ? 64 : 32;
 }
-inline int lnt_smem(int c_h) { return c_h * 128 + 2 * LNT_WARPS * 64 * 4; }
+inline int lnt_smem(int c_h) { return c_h * 128 + 2 * LNT_WARPS * 64 * 4 + c_h * 8; }
 template <bool BF, int G>
 __global__ void __launch_bounds__(LNT_WARPS * 32)
 ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, const void* __restrict__ scale_,
                         const void* __restrict__ bias_, float eps, long long pairs, __nv_bfloat16* __restrict__ tn) {
   using X = typename std::conditional<BF, __nv_bfloat16, float>::type;
   constexpr int JT = lnt_j<BF>(), JL = JT / 32;  // j of a block, of a lane
-  extern __shared__ uint32_t tile[];             // [c_h][32 words], then the partial sums
+  extern __shared__ uint32_t tile[];             // [c_h][32 words], then the partial sums, then scale and bias
   float* part = reinterpret_cast<float*>(tile + (c_h + 63) / 64 * 64 * 32);
+  uint2* affine = reinterpret_cast<uint2*>(part + 2 * LNT_WARPS * 64);  // bf16: each twice in a word
   pdl_wait();
   pdl_trigger();
+  if constexpr (BF)
+    for (int c = threadIdx.x; c < c_h; c += LNT_WARPS * 32) {
+      const uint32_t sc = static_cast<const unsigned short*>(scale_)[c], bi = static_cast<const unsigned short*>(bias_)[c];
+      affine[c] = make_uint2(sc | sc << 16, bi | bi << 16);
+    }
   const int i = blockIdx.y, b = blockIdx.z, j0 = blockIdx.x * JT;
   const X* src = static_cast<const X*>(t_) + (static_cast<long long>(b) * c_h * n + i) * ld + j0;
   const long long chan = static_cast<long long>(n) * ld;
@@ -322,16 +358,26 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
   const int groups = c_h / 8;
   auto value = [&](uint32_t w, int u) { return BF ? (u ? bf16_hi(w) : bf16_lo(w)) : __uint_as_float(w); };
   float s[JL] = {}, q[JL] = {};
-  for (int g = warp; g < groups; g += LNT_WARPS) {
+  // (two j of a lane as one packed value; per j the order of the sums is that of the channels)
+  float2 s2 = make_float2(0.f, 0.f), q2 = s2;
+  const X* col = src + warp * 8 * chan;
+  for (int g = warp; g < groups; g += LNT_WARPS, col += LNT_WARPS * 8 * chan) {
     uint32_t w[8];
+    const X* p = col;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) w[e] = reinterpret_cast<const uint32_t*>(src + (g * 8 + e) * chan)[lane];
+    for (int e = 0; e < 8; ++e, p += chan) w[e] = reinterpret_cast<const uint32_t*>(p)[lane];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       tile[(g * 8 + e) * 32 + lane] = w[e];
-#pragma unroll
-      for (int u = 0; u < JL; ++u) s[u] += value(w[e], u);
+      if constexpr (BF)
+        s2 = __fadd2_rn(s2, make_float2(bf16_lo(w[e]), bf16_hi(w[e])));
+      else
+        s[0] += __uint_as_float(w[e]);
     }
+  }
+  if constexpr (BF) {
+    s[0] = s2.x;
+    s[JL - 1] = s2.y;
   }
 #pragma unroll
   for (int u = 0; u < JL; ++u) part[(warp * JL + u) * 32 + lane] = s[u];
@@ -344,16 +390,23 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
     for (int w = 0; w < LNT_WARPS; ++w) s[u] += part[(w * JL + u) * 32 + lane];
     s[u] = chans.mean(s[u]);
   }
+  const float2 minus_mean = make_float2(-s[0], -s[JL - 1]);
   for (int g = warp; g < groups; g += LNT_WARPS)
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const uint32_t w = tile[(g * 8 + e) * 32 + lane];  // (this thread's own words)
-#pragma unroll
-      for (int u = 0; u < JL; ++u) {
-        const float d = value(w, u) - s[u];
-        q[u] = fmaf(d, d, q[u]);
+      if constexpr (BF) {
+        const float2 d = __fadd2_rn(make_float2(bf16_lo(w), bf16_hi(w)), minus_mean);
+        q2 = __ffma2_rn(d, d, q2);
+      } else {
+        const float d = __uint_as_float(w) - s[0];
+        q[0] = fmaf(d, d, q[0]);
       }
     }
+  if constexpr (BF) {
+    q[0] = q2.x;
+    q[JL - 1] = q2.y;
+  }
   float* part_q = part + LNT_WARPS * JL * 32;
 #pragma unroll
   for (int u = 0; u < JL; ++u) part_q[(warp * JL + u) * 32 + lane] = q[u];
@@ -365,11 +418,12 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
     for (int w = 0; w < LNT_WARPS; ++w) q[u] += part_q[(w * JL + u) * 32 + lane];
     q[u] = 1.0f / sqrtf(chans.mean(q[u]) + eps);
   }
+  const float2 rstd = make_float2(q[0], q[JL - 1]);
   const X* scale = static_cast<const X*>(scale_);
   const X* bias = static_cast<const X*>(bias_);
   if constexpr (!BF && G > 0) {
     const int pitch = (groups + 7) & ~7;  // (as below)
-    uint4* rows = reinterpret_cast<uint4*>(part + 2 * LNT_WARPS * 64);
+    uint4* rows = reinterpret_cast<uint4*>(affine + (c_h + 63) / 64 * 64);
     for (int g = warp; g < groups; g += LNT_WARPS) {
       uint32_t w[3][4];
 #pragma unroll
@@ -403,19 +457,21 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
     for (int k = 0; k < G; ++k) {
       const int g = warp + k * LNT_WARPS;
       if (g >= groups) continue;
-      float v[JL][8];
+      uint32_t o[JL][4];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int c = g * 8 + e;
-        const uint32_t w = tile[c * 32 + lane];
-        const float sc = static_cast<float>(scale[c]), bi = static_cast<float>(bias[c]);
+      for (int e = 0; e < 8; e += 2) {  // two channels of two j, turned round
+        uint32_t y[2];
 #pragma unroll
-        for (int u = 0; u < JL; ++u) v[u][e] = Rb<BF>::r(Rb<BF>::r((value(w, u) - s[u]) * q[u]) * sc) + bi;
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t w = tile[(g * 8 + e + u) * 32 + lane];
+          const uint2 sb = affine[g * 8 + e + u];
+          y[u] = affine_bf16x2(make_float2(bf16_lo(w), bf16_hi(w)), minus_mean, rstd, sb.x, sb.y);
+        }
+        o[0][e / 2] = __byte_perm(y[0], y[1], 0x5410);
+        o[JL - 1][e / 2] = __byte_perm(y[0], y[1], 0x7632);
       }
 #pragma unroll
-      for (int u = 0; u < JL; ++u)
-        out[k][u] = make_uint4(pack_bf16x2(v[u][0], v[u][1]), pack_bf16x2(v[u][2], v[u][3]), pack_bf16x2(v[u][4], v[u][5]),
-                               pack_bf16x2(v[u][6], v[u][7]));
+      for (int u = 0; u < JL; ++u) out[k][u] = make_uint4(o[u][0], o[u][1], o[u][2], o[u][3]);
     }
     __syncthreads();
     // rows of `pitch` 16-byte chunks, chunks swapped by the lane that writes them: no bank conflicts
