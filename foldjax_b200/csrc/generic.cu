@@ -60,6 +60,18 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16* dst, long long plane, 
     *reinterpret_cast<uint32_t*>(dst + 2 * plane) = lo;
   }
 }
+// 32 bytes in one store (dst 32-byte aligned): a whole sector of L2 instead of two halves.
+__device__ __forceinline__ void store_sector(void* dst, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ void load_sector(const void* src, uint4& a, uint4& b) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+               : "l"(src)
+               : "memory");
+}
 // Eight neighbouring values the same way (dst 16-byte aligned).
 template <int PIECES>
 __device__ __forceinline__ void store_eight(__nv_bfloat16* dst, long long plane, const float* v) {
@@ -511,6 +523,95 @@ ln_channel_major_kernel(const void* __restrict__ t_, int n, int ld, int c_h, con
   }
 }
 
+// The same in bf16, up to 64 * G channels: a lane's words stay in its registers from the load, all of
+// them requested at once, to the result. (Through shared memory and in two batches of loads the 128
+// channels of four 200-token templates took 36 us at 2.7 TB/s, and 25 so. With 384 channels it is the other
+// way round, 27 us for 256 tokens and 29 in the registers of 16 warps.)
+template <int G>
+__global__ void __launch_bounds__(LNT_WARPS * 32, 4)
+ln_channel_major_bf16_kernel(const __nv_bfloat16* __restrict__ t, int n, int ld, int c_h, const unsigned short* __restrict__ scale,
+                             const unsigned short* __restrict__ bias, float eps, __nv_bfloat16* __restrict__ tn) {
+  constexpr int JT = 64;
+  extern __shared__ uint32_t tile[];  // the results, then partial sums, scale and bias (each twice in a word)
+  float2* part = reinterpret_cast<float2*>(tile + (c_h + 63) / 64 * 64 * 32);
+  uint2* affine = reinterpret_cast<uint2*>(part + 2 * LNT_WARPS * 32);
+  pdl_wait();
+  pdl_trigger();
+  const int i = blockIdx.y, b = blockIdx.z, j0 = blockIdx.x * JT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, groups = c_h / 8;
+  const long long chan = static_cast<long long>(n) * ld;
+  const __nv_bfloat16* col = t + (static_cast<long long>(b) * c_h * n + i) * ld + j0 + warp * 8 * chan;
+  uint32_t w[G][8];
+#pragma unroll
+  for (int k = 0; k < G; ++k, col += LNT_WARPS * 8 * chan) {
+    const __nv_bfloat16* p = col;
+#pragma unroll
+    for (int e = 0; e < 8; ++e, p += chan)
+      w[k][e] = warp + k * LNT_WARPS < groups ? reinterpret_cast<const uint32_t*>(p)[lane] : 0u;
+  }
+  for (int c = threadIdx.x; c < c_h; c += LNT_WARPS * 32) {
+    const uint32_t sc = scale[c], bi = bias[c];
+    affine[c] = make_uint2(sc | sc << 16, bi | bi << 16);
+  }
+  const Channels chans(c_h);
+  float2 sum = make_float2(0.f, 0.f), var = sum;
+#pragma unroll
+  for (int k = 0; k < G; ++k)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sum = __fadd2_rn(sum, make_float2(bf16_lo(w[k][e]), bf16_hi(w[k][e])));
+  part[warp * 32 + lane] = sum;
+  __syncthreads();
+  sum = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int x = 0; x < LNT_WARPS; ++x) sum = __fadd2_rn(sum, part[x * 32 + lane]);
+  const float2 minus_mean = make_float2(-chans.mean(sum.x), -chans.mean(sum.y));
+#pragma unroll
+  for (int k = 0; k < G; ++k)
+    if (warp + k * LNT_WARPS < groups)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 d = __fadd2_rn(make_float2(bf16_lo(w[k][e]), bf16_hi(w[k][e])), minus_mean);
+        var = __ffma2_rn(d, d, var);
+      }
+  float2* part_var = part + LNT_WARPS * 32;
+  part_var[warp * 32 + lane] = var;
+  __syncthreads();
+  var = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int x = 0; x < LNT_WARPS; ++x) var = __fadd2_rn(var, part_var[x * 32 + lane]);
+  const float2 rstd = make_float2(1.0f / sqrtf(chans.mean(var.x) + eps), 1.0f / sqrtf(chans.mean(var.y) + eps));
+  // rows of `pitch` 16-byte chunks, chunks swapped by the lane that writes them: no bank conflicts
+  const int pitch = (groups + 7) & ~7;
+  uint4* rows = reinterpret_cast<uint4*>(tile);
+#pragma unroll
+  for (int k = 0; k < G; ++k) {
+    const int g = warp + k * LNT_WARPS;
+    if (g >= groups) continue;
+    uint32_t o[2][4];
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {  // two channels of two j, turned round
+      uint32_t y[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint2 sb = affine[g * 8 + e + u];
+        y[u] = affine_bf16x2(make_float2(bf16_lo(w[k][e + u]), bf16_hi(w[k][e + u])), minus_mean, rstd, sb.x, sb.y);
+      }
+      o[0][e / 2] = __byte_perm(y[0], y[1], 0x5410);
+      o[1][e / 2] = __byte_perm(y[0], y[1], 0x7632);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      rows[(lane * 2 + u) * pitch + (g ^ (lane & 7))] = make_uint4(o[u][0], o[u][1], o[u][2], o[u][3]);
+  }
+  __syncthreads();
+  uint4* dst = reinterpret_cast<uint4*>(tn + ((static_cast<long long>(b) * n + i) * n + j0) * c_h);
+  const int count = min(JT, n - j0) * groups;
+  for (int idx = threadIdx.x; idx < count; idx += LNT_WARPS * 32) {
+    const int j = idx / groups, g = idx - j * groups;
+    dst[idx] = rows[j * pitch + (g ^ ((j / 2) & 7))];
+  }
+}
+
 template <bool BF>
 int launch_ln_channel_major(const void* t, int n, int batch, int ld, int c_h, const void* scale, const void* bias, float eps,
                             __nv_bfloat16* tn, cudaStream_t stream) {
@@ -522,7 +623,14 @@ int launch_ln_channel_major(const void* t, int n, int batch, int ld, int c_h, co
                   static_cast<long long>(batch) * n * n, tn);
   };
   if constexpr (BF) {
-    if (c_h <= 128) return go(ln_channel_major_kernel<BF, 2>);
+    auto go_bf16 = [&](auto kernel) {
+      const int smem = lnt_smem(round_up(c_h, 64)), rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), lnt_smem(128));
+      if (rc) return rc;
+      return launch(kernel, grid, dim3(LNT_WARPS * 32), smem, stream, true, static_cast<const __nv_bfloat16*>(t), n, ld, c_h,
+                    static_cast<const unsigned short*>(scale), static_cast<const unsigned short*>(bias), eps, tn);
+    };
+    if (c_h <= 64) return go_bf16(ln_channel_major_bf16_kernel<1>);
+    if (c_h <= 128) return go_bf16(ln_channel_major_bf16_kernel<2>);
     if (c_h <= 384) return go(ln_channel_major_kernel<BF, 6>);
   } else if (c_h <= 384) {
     return go(ln_channel_major_kernel<BF, 1>, round_up(c_h, 64) * 192);
@@ -547,17 +655,40 @@ int map_rows(CUtensorMap* out, const void* base, int k, int n, long long s_inner
 template <int COLS>
 struct RowPrefetch {
   uint4 row[COLS > 0 ? COLS / 8 : 1];
-  __device__ __forceinline__ void load(const __nv_bfloat16* src, int left) {  // `left` columns exist
+  // `left` columns exist. `sectors`: rows start on 32-byte boundaries and have whole runs of 16 columns,
+  // which then are one access: half an L2 sector at a time, what 128 rows of a tile cost the load/store
+  // unit and L2 was most of a product's epilogue.
+  __device__ __forceinline__ void load(const __nv_bfloat16* src, int left, bool sectors) {
+    if constexpr (COLS % 16 == 0) {
+      if (sectors) {
+#pragma unroll
+        for (int q = 0; q < COLS / 8; q += 2) {
+          row[q] = row[q + 1] = make_uint4(0u, 0u, 0u, 0u);
+          if (8 * q < left) load_sector(src + 8 * q, row[q], row[q + 1]);
+        }
+        return;
+      }
+    }
 #pragma unroll
     for (int q = 0; q < COLS / 8; ++q)
       row[q] = 8 * q < left ? reinterpret_cast<const uint4*>(src)[q] : make_uint4(0u, 0u, 0u, 0u);
   }
   // Eight neighbouring values rounded to bf16, with the prefetched residual added (one more rounding).
-  __device__ __forceinline__ void store(__nv_bfloat16* dst, int q, bool residual, const float* v) const {
+  __device__ __forceinline__ uint4 rounded(int q, bool residual, const float* v) const {
     uint4 u = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
     if (residual)
       u = make_uint4(bf16x2_add(row[q].x, u.x), bf16x2_add(row[q].y, u.y), bf16x2_add(row[q].z, u.z), bf16x2_add(row[q].w, u.w));
-    *reinterpret_cast<uint4*>(dst) = u;
+    return u;
+  }
+  // Sixteen of them, `left` of which exist.
+  __device__ __forceinline__ void store(__nv_bfloat16* dst, int q, bool residual, const float* v, int left, bool sectors) const {
+    const uint4 a = rounded(q, residual, v), b = rounded(q + 1, residual, v + 8);
+    if (sectors) {
+      store_sector(dst, a, b);
+      return;
+    }
+    *reinterpret_cast<uint4*>(dst) = a;
+    if (left > 8) reinterpret_cast<uint4*>(dst)[1] = b;
   }
 };
 
@@ -619,26 +750,31 @@ struct GluPolicy {
     for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
       const int col = col0 + 16 * i;
       if (rt.t0 + col >= p.n) break;
-      const float mk = Rb<BF>::r(pre.mask[i]);
+      const float mk = pre.mask[i];
       float v[16], g[16];
       acc.load(0, col, v);
       acc.load(1, col, g);
+      // (the pitch is a multiple of 64: the padding takes what lies past n)
+      if constexpr (BF) {
+        const uint32_t mk2 = pack_bf16x2(mk, __shfl_down_sync(0xffffffffu, mk, 1));  // of two pairs, in the lane of the first
+        uint32_t u[8];
 #pragma unroll
-      for (int e = 0; e < 16; e += 2) {
-        const float m0 = __shfl_sync(0xffffffffu, mk, e), m1 = __shfl_sync(0xffffffffu, mk, e + 1);
-        if (BF) {
-          const uint32_t u = bf16x2_mul(bf16x2_mul(sigmoid_bf16x2(g[e], g[e + 1]), pack_bf16x2(v[e], v[e + 1])),
-                                        pack_bf16x2(m0, m1));
-          v[e] = bf16_lo(u);
-          v[e + 1] = bf16_hi(u);
-        } else {
+        for (int e = 0; e < 16; e += 2)
+          u[e / 2] = bf16x2_mul(bf16x2_mul(sigmoid_bf16x2(g[e], g[e + 1]), pack_bf16x2(v[e], v[e + 1])),
+                                __shfl_sync(0xffffffffu, mk2, e));
+        // a lane's 16 pairs are a whole sector of its channel
+        if (c < 2 * p.c_h) store_sector(dst + col, make_uint4(u[0], u[1], u[2], u[3]), make_uint4(u[4], u[5], u[6], u[7]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+          const float m0 = __shfl_sync(0xffffffffu, mk, e), m1 = __shfl_sync(0xffffffffu, mk, e + 1);
           v[e] = sigmoid_exact(g[e]) * v[e] * m0;
           v[e + 1] = sigmoid_exact(g[e + 1]) * v[e + 1] * m1;
         }
-      }
-      if (c < 2 * p.c_h)  // (the pitch is a multiple of 64: the padding takes what lies past n)
+        if (c < 2 * p.c_h)
 #pragma unroll
-        for (int q = 0; q < 2; ++q) store_eight<PIECES>(dst + col + 8 * q, p.piece, v + 8 * q);
+          for (int q = 0; q < 2; ++q) store_eight<PIECES>(dst + col + 8 * q, p.piece, v + 8 * q);
+      }
     }
   }
 };
@@ -655,7 +791,7 @@ struct OutGatePolicy {
     int n, tiles_j, c_z;
     const O* res;
     O* out;
-    bool aligned;
+    bool aligned, sectors;  // 16-byte and 32-byte accesses
   };
   using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
@@ -663,7 +799,7 @@ struct OutGatePolicy {
       if (!p.res || !p.aligned) return;
       const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
       const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
-      pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0);
+      pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0, p.sectors);
     }
   }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int seg, int k, int m_tile, int piece, uint8_t* dst,
@@ -699,15 +835,15 @@ struct OutGatePolicy {
           v[e + 1] *= sigmoid_exact(g[e + 1]);
         }
       }
+      if constexpr (BF) {
+        if (p.aligned) {
+          pre.store(p.out + off + c0, 2 * i, p.res != nullptr, v, p.c_z - c0, p.sectors);
+          continue;
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
         if (c0 + 8 * q < p.c_z) {
-          if constexpr (BF) {
-            if (p.aligned) {
-              pre.store(p.out + off + c0 + 8 * q, 2 * i + q, p.res != nullptr, v + 8 * q);
-              continue;
-            }
-          }
           store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
         }
     }
@@ -760,6 +896,14 @@ struct QkvbPolicy : NoPrefetch {
           // integer below 256 times a power of two and the dividend has 8 bits, so that the quotient is
           // representable or at least 1e-5 away from a rounding boundary.
           for (int e = 0; e < 16; ++e) v[e] = BF ? round_bf16(v[e]) * p.q_scale_inv : v[e] / p.q_scale;
+        if constexpr (BF) {
+          if (p.hd % 16 == 0) {
+            store_sector(dst, make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7])),
+                         make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
+                                    pack_bf16x2(v[14], v[15])));
+            continue;
+          }
+        }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
           if (c0 + 8 * q < p.hd) store_eight<PIECES>(dst + 8 * q, p.row_piece, v + 8 * q);
@@ -809,7 +953,7 @@ struct GatePolicy {
     if constexpr (BF) {
       const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
       const int c0 = n_tile * BN + col0;
-      pre.load(p.y + pair * p.hd + c0, pair < p.pairs ? p.hd - c0 : 0);
+      pre.load(p.y + pair * p.hd + c0, pair < p.pairs ? p.hd - c0 : 0, p.hd % 16 == 0);
     }
   }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
@@ -831,17 +975,26 @@ struct GatePolicy {
       acc.load(0, col, g);
       if (pair >= p.pairs) continue;
       const long long off = pair * p.hd + c0;
+      if constexpr (BF) {
+        uint4 w[2];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (c0 + 8 * q >= p.hd) break;
-        if constexpr (BF) {
-          uint4 w = pre.row[2 * i + q];
-          w.x = bf16x2_mul(w.x, sigmoid_bf16x2(g[8 * q + 0], g[8 * q + 1]));
-          w.y = bf16x2_mul(w.y, sigmoid_bf16x2(g[8 * q + 2], g[8 * q + 3]));
-          w.z = bf16x2_mul(w.z, sigmoid_bf16x2(g[8 * q + 4], g[8 * q + 5]));
-          w.w = bf16x2_mul(w.w, sigmoid_bf16x2(g[8 * q + 6], g[8 * q + 7]));
-          *reinterpret_cast<uint4*>(p.y + off + 8 * q) = w;
+        for (int q = 0; q < 2; ++q) {
+          const uint4 o = pre.row[2 * i + q];
+          w[q].x = bf16x2_mul(o.x, sigmoid_bf16x2(g[8 * q + 0], g[8 * q + 1]));
+          w[q].y = bf16x2_mul(o.y, sigmoid_bf16x2(g[8 * q + 2], g[8 * q + 3]));
+          w[q].z = bf16x2_mul(o.z, sigmoid_bf16x2(g[8 * q + 4], g[8 * q + 5]));
+          w[q].w = bf16x2_mul(o.w, sigmoid_bf16x2(g[8 * q + 6], g[8 * q + 7]));
+        }
+        if (p.hd % 16 == 0) {
+          store_sector(p.y + off, w[0], w[1]);
         } else {
+          *reinterpret_cast<uint4*>(p.y + off) = w[0];
+          if (c0 + 8 < p.hd) reinterpret_cast<uint4*>(p.y + off)[1] = w[1];
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (c0 + 8 * q >= p.hd) break;
           float v[8];
 #pragma unroll
           for (int h4 = 0; h4 < 2; ++h4) {
@@ -874,7 +1027,7 @@ struct ProjOutPolicy {
     long long s_b, s_o, s_i;
     const O* res;
     O* out;
-    bool aligned;
+    bool aligned, sectors;  // 16-byte and 32-byte accesses
   };
   using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
   static __device__ long long offset(const Params& p, uint32_t pair) {
@@ -886,7 +1039,7 @@ struct ProjOutPolicy {
       if (!p.res || !p.aligned) return;
       const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane;
       const int c0 = n_tile * BN + col0;
-      pre.load(p.res + offset(p, pair) + c0, pair < p.pairs ? p.c_z - c0 : 0);
+      pre.load(p.res + offset(p, pair) + c0, pair < p.pairs ? p.c_z - c0 : 0, p.sectors);
     }
   }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
@@ -908,15 +1061,15 @@ struct ProjOutPolicy {
       float v[16];
       acc.load(0, col, v);
       if (pair >= p.pairs) continue;
+      if constexpr (BF) {
+        if (p.aligned) {
+          pre.store(p.out + off + c0, 2 * i, p.res != nullptr, v, p.c_z - c0, p.sectors);
+          continue;
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
         if (c0 + 8 * q < p.c_z) {
-          if constexpr (BF) {
-            if (p.aligned) {
-              pre.store(p.out + off + c0 + 8 * q, 2 * i + q, p.res != nullptr, v + 8 * q);
-              continue;
-            }
-          }
           store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
         }
     }
@@ -1032,6 +1185,9 @@ struct WeightStage {
   }
 };
 
+bool aligned32(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 31) == 0;
+}
 bool aligned16(const void* a, const void* b) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
 }
@@ -1120,7 +1276,7 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {nb * n * tiles_j, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_h), ksteps(c_z)}, nullptr};
-        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res), c_z % 16 == 0 && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(OutGatePolicy<1, 1, 64>{}) : go(OutGatePolicy<1, 1, 128>{});
@@ -1246,7 +1402,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {m_tiles, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(hd), 0}, nullptr};
-        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res), c_z % 16 == 0 && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{})
