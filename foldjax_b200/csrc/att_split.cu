@@ -456,14 +456,22 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           tmem_ld16(t_wg + C::TM_O + part * 16, r);
           tmem_ld_wait();
           if (!live) continue;
+          uint4 w[2];
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            uint32_t w[4];
+            uint32_t u[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              w[e] = pack_bf16x2(__uint_as_float(r[8 * q + 2 * e]) * inv, __uint_as_float(r[8 * q + 2 * e + 1]) * inv);
-            if (part * 16 + q * 8 < p.head_dim)
-              *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.o) + off + part * 16 + q * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+              u[e] = pack_bf16x2(__uint_as_float(r[8 * q + 2 * e]) * inv, __uint_as_float(r[8 * q + 2 * e + 1]) * inv);
+            w[q] = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.o) + off + part * 16);
+          if (p.head_dim % 16 == 0 && part * 16 < p.head_dim) {
+            store_sector(dst, w[0], w[1]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+              if (part * 16 + q * 8 < p.head_dim) dst[q] = w[q];
           }
         }
       }
@@ -484,10 +492,13 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         }
       } else if constexpr (!C::OVERLAY) {
 #pragma unroll
-        for (int d = 0; d < HDP; d += 4)
-          if (live && d < p.head_dim)
-            *reinterpret_cast<float4*>(static_cast<float*>(p.o) + off + d) =
-                make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
+        for (int d = 0; d < HDP; d += 8)
+          if (live && d < p.head_dim) {  // (a multiple of 8)
+            uint32_t w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(o[d + e] * inv);
+            store_sector(static_cast<float*>(p.o) + off + d, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));
+          }
       }
     }
   }

@@ -60,18 +60,6 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16* dst, long long plane, 
     *reinterpret_cast<uint32_t*>(dst + 2 * plane) = lo;
   }
 }
-// 32 bytes in one store (dst 32-byte aligned): a whole sector of L2 instead of two halves.
-__device__ __forceinline__ void store_sector(void* dst, const uint4& a, const uint4& b) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
-               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
-               : "memory");
-}
-__device__ __forceinline__ void load_sector(const void* src, uint4& a, uint4& b) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-               : "l"(src)
-               : "memory");
-}
 // Eight neighbouring values the same way (dst 16-byte aligned).
 template <int PIECES>
 __device__ __forceinline__ void store_eight(__nv_bfloat16* dst, long long plane, const float* v) {
@@ -87,12 +75,43 @@ __device__ __forceinline__ void store_eight(__nv_bfloat16* dst, long long plane,
 #pragma unroll
   for (int q = 0; q < PIECES; ++q) *reinterpret_cast<uint4*>(dst + q * plane) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
 }
+// Sixteen of them (dst and plane on 32-byte boundaries), a sector per piece.
+template <int PIECES>
+__device__ __forceinline__ void store_sixteen(__nv_bfloat16* dst, long long plane, const float* v) {
+  uint32_t w[3][8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    if (PIECES == 1) {
+      w[0][e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+    } else {
+      split3x2(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < PIECES; ++q)
+    store_sector(dst + q * plane, make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]), make_uint4(w[q][4], w[q][5], w[q][6], w[q][7]));
+}
 // Eight neighbouring values to the caller's tensor, with the caller's residual added (one more
 // rounding of the trunk dtype).
 template <bool BF, typename O>
-__device__ __forceinline__ void store_out(O* dst, const O* res, float* v, bool aligned) {
+__device__ __forceinline__ void store_out(O* dst, const O* res, float* v, bool aligned, bool sectors) {
 #pragma unroll
   for (int e = 0; e < 8; ++e) v[e] = Rb<BF>::r(v[e]);
+  if constexpr (!BF) {
+    if (sectors) {
+      uint4 a, b;
+      if (res) {
+        load_sector(res, a, b);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(w[e]) + v[e];
+      }
+      a = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+      b = make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
+      store_sector(dst, a, b);
+      return;
+    }
+  }
   if (aligned) {
     constexpr int W = 8 * sizeof(O) / 16;
     uint4 raw[W];
@@ -771,9 +790,7 @@ struct GluPolicy {
           v[e] = sigmoid_exact(g[e]) * v[e] * m0;
           v[e + 1] = sigmoid_exact(g[e + 1]) * v[e + 1] * m1;
         }
-        if (c < 2 * p.c_h)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) store_eight<PIECES>(dst + col + 8 * q, p.piece, v + 8 * q);
+        if (c < 2 * p.c_h) store_sixteen<PIECES>(dst + col, p.piece, v);
       }
     }
   }
@@ -844,7 +861,7 @@ struct OutGatePolicy {
 #pragma unroll
       for (int q = 0; q < 2; ++q)
         if (c0 + 8 * q < p.c_z) {
-          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
         }
     }
   }
@@ -896,13 +913,9 @@ struct QkvbPolicy : NoPrefetch {
           // integer below 256 times a power of two and the dividend has 8 bits, so that the quotient is
           // representable or at least 1e-5 away from a rounding boundary.
           for (int e = 0; e < 16; ++e) v[e] = BF ? round_bf16(v[e]) * p.q_scale_inv : v[e] / p.q_scale;
-        if constexpr (BF) {
-          if (p.hd % 16 == 0) {
-            store_sector(dst, make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7])),
-                         make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                                    pack_bf16x2(v[14], v[15])));
-            continue;
-          }
+        if (p.hd % 16 == 0) {
+          store_sixteen<PIECES>(dst, p.row_piece, v);
+          continue;
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
@@ -991,6 +1004,17 @@ struct GatePolicy {
           *reinterpret_cast<uint4*>(p.y + off) = w[0];
           if (c0 + 8 < p.hd) reinterpret_cast<uint4*>(p.y + off)[1] = w[1];
         }
+      } else if (p.hd % 16 == 0) {
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          uint4 a, b;
+          load_sector(p.o + off + 8 * q, a, b);
+          const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[8 * q + e] = __uint_as_float(w[e]) * sigmoid_exact(g[8 * q + e]);
+        }
+        store_sixteen<PIECES>(p.y + off, p.pairs * p.hd, v);
       } else {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -1070,7 +1094,7 @@ struct ProjOutPolicy {
 #pragma unroll
       for (int q = 0; q < 2; ++q)
         if (c0 + 8 * q < p.c_z) {
-          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned);
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
         }
     }
   }
@@ -1276,7 +1300,7 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {nb * n * tiles_j, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_h), ksteps(c_z)}, nullptr};
-        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res), c_z % 16 == 0 && aligned32(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(OutGatePolicy<1, 1, 64>{}) : go(OutGatePolicy<1, 1, 128>{});
@@ -1402,7 +1426,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {m_tiles, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(hd), 0}, nullptr};
-        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res), c_z % 16 == 0 && aligned32(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{})

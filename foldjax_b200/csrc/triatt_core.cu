@@ -122,6 +122,7 @@ struct Params {
   uint32_t total_items;
   __nv_bfloat16* o;
   long long o_token, o_head, o_row;  // strides of o in elements
+  bool o_sectors;                    // a head of o is two 32-byte sectors
   float* row_max;    // optional [n_i][heads][n_j]: offset m used (natural log units)
   float* row_sum;    // optional: sum of exp(S - m)
   float* acc_o;      // fp32 running numerator [n_i][n_j][128] (ring attention)
@@ -555,13 +556,20 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tmem_ld_wait();
         if (p.normalize) {
           uint4* dst = reinterpret_cast<uint4*>(p.o + i * p.o_row + h * p.o_head + j * p.o_token + part * 16);
+          uint4 w[2];
 #pragma unroll
           for (int q4 = 0; q4 < 2; ++q4) {
-            uint32_t w[4];
+            uint32_t u[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              w[e] = pack_bf16x2(__uint_as_float(o[8 * q4 + 2 * e]) * inv, __uint_as_float(o[8 * q4 + 2 * e + 1]) * inv);
-            if (in_range) dst[q4] = make_uint4(w[0], w[1], w[2], w[3]);
+              u[e] = pack_bf16x2(__uint_as_float(o[8 * q4 + 2 * e]) * inv, __uint_as_float(o[8 * q4 + 2 * e + 1]) * inv);
+            w[q4] = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+          if (in_range && p.o_sectors) {
+            store_sector(dst, w[0], w[1]);
+          } else if (in_range) {
+            dst[0] = w[0];
+            dst[1] = w[1];
           }
         } else if (in_range) {
           float4* dst = reinterpret_cast<float4*>(p.acc_o + (static_cast<long long>(i) * p.n_j + j) * 128 + h * 32 + part * 16);
@@ -742,6 +750,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   p.o_token = st.token;
   p.o_head = st.head_j;
   p.o_row = st.row_j;
+  p.o_sectors = (reinterpret_cast<uintptr_t>(a->o) & 31) == 0 && (st.token | st.head_j | st.row_j) % 16 == 0;
   p.o = static_cast<__nv_bfloat16*>(a->o);
   p.row_max = a->row_max;
   p.row_sum = a->row_sum;

@@ -50,6 +50,7 @@ struct ContractParams {
   uint32_t total_tiles;
   bool staged;  // the result leaves by TMA: it is bf16 only and a warp's 32 rows share a block
   bool out_blocked;
+  bool f32_sectors;  // rows of the float32 result start on 32-byte boundaries
   const float* acc_in;
   float* out_f32;
   __nv_bfloat16* out_bf16;
@@ -286,10 +287,17 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           if (p.out_f32) {
             if (full) {
               float4* dst = reinterpret_cast<float4*>(p.out_f32 + off);
+              if (p.f32_sectors) {
 #pragma unroll
-              for (int q = 0; q < 8; ++q)
-                dst[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
-                                     __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+                for (int q = 0; q < 4; ++q)
+                  store_sector(dst + 2 * q, make_uint4(r[8 * q], r[8 * q + 1], r[8 * q + 2], r[8 * q + 3]),
+                               make_uint4(r[8 * q + 4], r[8 * q + 5], r[8 * q + 6], r[8 * q + 7]));
+              } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                  dst[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                       __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+              }
             } else {
 #pragma unroll
               for (int q = 0; q < 32; ++q)
@@ -443,6 +451,8 @@ int b200::contract_launch(const b200tri_trimul_contract_args* a, int channels, c
   p.total_tiles = static_cast<uint32_t>(tiles);
   p.acc_in = a->acc_in;
   p.out_f32 = a->out_f32;
+  p.f32_sectors = (reinterpret_cast<uintptr_t>(a->out_f32) & 31) == 0 &&
+                  (a->out_ld | a->out_chan_stride | a->out_block_stride) % 8 == 0;
   p.out_bf16 = static_cast<__nv_bfloat16*>(a->out_bf16);
   p.out_ld = a->out_ld;
   p.out_chan_stride = a->out_chan_stride;
