@@ -1,6 +1,8 @@
 """The general path's epilogues move 32 bytes at a time where rows lie on that grid: tensors that are
 16 bytes off it, and channel and head counts whose rows cannot, give the bits of the aligned ones."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -55,6 +57,30 @@ def test_attention_operator_off_the_sector_grid(cuda_device, n_k):
     got = attention_core(*(_off_by_16_bytes(t) for t in (q, k, v, bias)), mask)
     _lib.device_status()
     assert torch.equal(ref, got)
+
+
+def test_core_result_off_the_sector_grid(cuda_device):
+    """The attention core's C entry with its result on and 16 bytes off the 32-byte grid: same bits."""
+    from foldjax_b200 import _device as dev, _lib
+
+    lib = _lib.load()
+    n_i, n_j, n_k, h, d, ld = 5, 130, 70, 4, 32, 128
+    g = torch.Generator("cuda").manual_seed(3)
+    draw = lambda *shape, dtype=torch.bfloat16: (torch.randn(shape, generator=g, device="cuda") * 0.4).to(dtype)
+    q, k, vt, bias = draw(n_i, n_j, h * d), draw(n_i, n_k, h * d), draw(n_i, h * d, ld, dtype=torch.float16), draw(h, n_j, ld)
+    mask = torch.ones(n_i, n_k, device="cuda")
+    nb = lib.b200tri_triatt_core_workspace_bytes(n_i, n_k)
+    ws = torch.empty(nb + 1024, dtype=torch.uint8, device="cuda")
+    on = torch.full((n_i, n_j, h * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    off = _off_by_16_bytes(on)
+    for o in (on, off):
+        args = _lib.TriattCoreArgs(
+            n_i=n_i, n_j=n_j, n_k=n_k, heads=h, head_dim=d, q=q.data_ptr(), k=k.data_ptr(), vt=vt.data_ptr(), v_ld=ld,
+            bias=bias.data_ptr(), bias_ld=ld, bias_head_stride=n_j * ld, mask=mask.data_ptr(), ms_i=n_k, ms_k=1, inf=1e9,
+            o=o.data_ptr(), unnormalized=0, workspace=dev.aligned_ptr(ws), workspace_bytes=nb)
+        _lib.check(lib.b200tri_triatt_core(C.byref(args), C.c_void_p(dev.stream_ptr())))
+    _lib.device_status()
+    assert bool(torch.isfinite(on.float()).all()) and torch.equal(on, off)
 
 
 @pytest.mark.parametrize("n,blocks", [(16, 4), (128, 3), (128, 4), (129, 3)])
