@@ -400,16 +400,20 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             o[4 * q4 + 3] = __float_as_uint(f.w);
           }
         }
+        __syncwarp();
         tmem_st32(t_wg + TM_O, o);
         tmem_st16(t_wg + TM_L, lcol);
         tmem_st_wait();
         tc_fence_before();
       }
       for (int t = 0; t < p.steps; ++t, ++g) {
-        // (both asked at once: nearly always there already, and one latency instead of two)
+        // (both asked at once: nearly always there already, and one latency instead of two. Each lane polls
+        // for itself; the vote brings them together again, as the TMEM accesses need, and has all or
+        // none of them leave)
         const bool st_there = mbar_test(&sm.st_full[stage], phase), s_there = mbar_test(&sm.s_full[wg], g & 1);
-        if ((!st_there && !mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX)) ||
-            (!s_there && !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX))) {
+        alive = alive && (st_there || mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX)) &&
+                (s_there || mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX));
+        if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
           break;
         }
@@ -505,13 +509,13 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               packed[e] = *reinterpret_cast<const uint32_t*>(&h2);
             }
             if (half == 0) {
-              if (!p_free && !mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) alive = false;
+              if (!p_free) alive = mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
+              __syncwarp();
               tc_fence_after();
             }
             tmem_st16(t_wg + TM_P + 16 * half, packed);
           }
         }
-        if (!alive) break;
         if ((t > 0 || p.resume) && any_need) {
           uint32_t o[32];
           tmem_ld32(t_wg + TM_O, o);
@@ -537,7 +541,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (!alive) break;
       // ---- item epilogue: O / l -> bf16 -> o[i][j][h*32 ..]
-      if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) break;
+      alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
+      if (!__all_sync(0xffffffffu, alive)) break;
       tc_fence_after();
       int h, i, j;
       locate(item, h, i, j);
@@ -552,6 +557,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         uint32_t o[16];
+        __syncwarp();  // (rows past the end part from the others at the stores)
         tmem_ld16(t_wg + TM_O + part * 16, o);
         tmem_ld_wait();
         if (p.normalize) {
