@@ -234,28 +234,31 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    // ---- TMA producer (like the issuers: all lanes walk the loops, one issues)
+    // ---- TMA producer. Here and in the issuers all lanes walk the loops and wait, and one of them
+    // issues. A join follows every wait whose barrier can complete its next phase by what the leader
+    // does behind it (the others cannot come round before the next such join): a lane left behind
+    // would miss the phase it waits for. So no lane may leave early either: one whose wait has
+    // run out stops waiting and issuing and walks on.
     const bool leader = elect_one();
     int stage = 0;
     uint32_t phase = 0, item_it = 0;
     bool alive = true;
-    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
       int h, i0, j0;
       locate(item, h, i0, j0);
       const uint32_t qb = item_it % QBUF;
-      if (!mbar_wait(&sm.q_empty[qb], ((item_it / QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-      if (leader) {
+      alive = alive && mbar_wait(&sm.q_empty[qb], ((item_it / QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER);
+      __syncwarp();
+      if (leader && alive) {
         mbar_expect_tx(&sm.q_full[qb], NWG * Q_BYTES);
         for (int g = 0; g < NWG; ++g) tma_load_4d(sm.q[qb][g], &tm_q, &sm.q_full[qb], 0, h, j0, i0 + g);
       }
       for (int t = 0; t < p.steps; ++t) {
-        if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
-          alive = false;
-          break;
-        }
+        alive = alive && mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER);
+        __syncwarp();
         const int tile = t / p.steps_per_tile;
         const int k0 = (t - tile * p.steps_per_tile) * KT;
-        if (leader) {
+        if (leader && alive) {
           mbar_expect_tx(&sm.st_full[stage], STAGE_TX);
           tma_load_3d(sm.bias[stage], &tm.b[tile], &sm.st_full[stage], k0, j0, h);
           for (int g = 0; g < NWG; ++g) {
@@ -281,26 +284,21 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int stage = 0;
     uint32_t phase = 0, item_it = 0, g = 0;  // g: global step counter
     bool alive = true;
-    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
       const uint32_t qb = item_it % QBUF;
-      if (!mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA)) break;
-      for (int t = 0; t < p.steps && alive; ++t, ++g) {
-        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
-          alive = false;
-          break;
-        }
+      alive = alive && mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA);
+      for (int t = 0; t < p.steps; ++t, ++g) {
+        alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
         const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
 #pragma unroll
         for (int wg = 0; wg < NWG; ++wg) {
-          if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
-            alive = false;
-            break;
-          }
+          alive = alive && mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA);
+          __syncwarp();
           tc_fence_after();
           const uint64_t adesc = desc_sw64(smem_u32(sm.q[qb][wg]));
           const uint64_t bdesc = desc_sw64(smem_u32(sm.k[stage][wg]));
           const uint32_t d = tmem_base + wg * TM_WG + TM_S;
-          if (leader) {
+          if (leader && alive) {
 #pragma unroll
             for (int kk = 0; kk < KT / 16; ++kk)
               umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_qk, kk != 0);
@@ -314,7 +312,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           phase ^= 1;
         }
       }
-      if (alive && leader) umma_commit(&sm.q_empty[qb]);  // every Q.K^T of the item has been issued
+      if (leader && alive) umma_commit(&sm.q_empty[qb]);  // every Q.K^T of the item has been issued
     }
   } else if (warp == 2) {
     // ---- P.V issuer: O[wg] (+)= P[wg] . V[stage][wg], P read from TMEM.
@@ -323,31 +321,28 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int stage = 0;
     uint32_t phase = 0, g = 0;
     bool alive = true;
-    for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
-      for (int t = 0; t < p.steps && alive; ++t, ++g) {
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
+      for (int t = 0; t < p.steps; ++t, ++g) {
         // (already complete when P arrives; observed here so this thread's products
         // are ordered after the TMA writes of V)
-        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
+        alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
         for (int wg = 0; wg < NWG; ++wg) {
-          if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
-            alive = false;
-            break;
-          }
+          alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
+          __syncwarp();
           tc_fence_after();
           const uint64_t vdesc = desc_sw128(smem_u32(sm.v[stage][wg]));
           const uint32_t d = tmem_base + wg * TM_WG + TM_O;
           const uint32_t a = tmem_base + wg * TM_WG + TM_P;
-          if (leader) {
+          if (leader && alive) {
 #pragma unroll
             for (int k = 0; k < KT / 16; ++k)
               umma_bf16_ts(d, a + k * 8, umma_desc_advance(vdesc, k * 32), idesc_pv, (t | k | p.resume) != 0);
             umma_commit(&sm.pv_done[wg]);
           }
         }
-        if (!alive) break;
         // K of this stage was consumed before the softmax saw its scores, V by the
         // products just issued: the stage is free once they complete.
-        if (leader) umma_commit(&sm.st_empty[stage]);
+        if (leader && alive) umma_commit(&sm.st_empty[stage]);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;

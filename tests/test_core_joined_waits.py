@@ -38,3 +38,15 @@ def test_tensor_memory_is_accessed_by_joined_warps():
     softmax = _roles()[1]
     assert len(re.findall(WAIT, softmax)) >= 6 and len(re.findall(TMEM, softmax)) >= 10
     assert not _not_joined(softmax, TMEM)
+
+
+def test_issuing_lane_does_not_run_ahead_of_its_warp():
+    """All lanes of the loading and issuing warps wait on barriers that tell two phases apart, and one lane
+    makes the next phase come: it may pass a wait only together with the others. No lane leaves the loops
+    before the others, which would wait for it at a join."""
+    control = _roles()[0]
+    issued = r"\bif \([^)]*\bleader\b"
+    assert len(re.findall(issued, control)) == 6
+    assert not _not_joined(control, issued)
+    assert "break" not in control and "return" not in control
+    assert not re.search(r"for \([^;]*;[^;]*alive", control)
