@@ -340,6 +340,7 @@ SIGNATURES = {
     "b200tri_triatt_cp_workspace_bytes": (C.c_size_t, [C.c_void_p, C.c_int32]),
     "b200tri_triatt_cp": (C.c_int, [C.c_void_p, C.POINTER(TriattCpArgs), C.c_void_p]),
     "b200tri_pairformer_workspace_bytes": (C.c_size_t, [C.c_int32] * 5),
+    "b200tri_pairformer_stack_workspace_bytes": (C.c_size_t, [C.c_int32] * 6),
     "b200tri_pairformer_forward": (C.c_int, [C.POINTER(PairformerArgs), C.c_void_p]),
     "b200tri_pair_transition_workspace_bytes": (C.c_size_t, [C.c_int32]),
     "b200tri_pair_transition": (C.c_int, [C.POINTER(PairTransitionArgs), C.c_void_p]),

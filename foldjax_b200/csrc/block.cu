@@ -53,19 +53,20 @@ struct Offsets {
 };
 
 struct Plan {
-  size_t w, w2, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
+  size_t w, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
 };
 
 // One tile of the pair track's stage kernels per SM and some SMs over (a contraction has 128 tiles
 // there): what runs on the side stream has SMs of its own.
 constexpr int LEFT_OVER_BELOW = 128;
 bool leaves_sms(int n) { return n <= LEFT_OVER_BELOW; }
+// The second buffer that blocks of a stack end in where the workspace has room for it, behind the plan's total.
+size_t second_end_bytes(int n) { return (static_cast<size_t>(n) * n * 128 * 2 + 1023) / 1024 * 1024; }
 
 Plan plan(int n, int c_s, int heads_s, int hidden_z, int hidden_s, bool single) {
   Plan p = {};
   Offsets o;
   p.w = o.take(static_cast<size_t>(n) * n * 128 * 2);
-  if (single && leaves_sms(n)) p.w2 = o.take(static_cast<size_t>(n) * n * 128 * 2);
   size_t sub = b200tri_trimul_workspace_bytes(n);
   const size_t cand[2] = {b200tri_triatt_workspace_bytes(n), b200tri_pair_transition_workspace_bytes(hidden_z)};
   for (size_t c : cand) sub = c > sub ? c : sub;
@@ -150,6 +151,12 @@ extern "C" size_t b200tri_pairformer_workspace_bytes(int32_t n, int32_t c_s, int
                                                      int32_t hidden_s) {
   if (n <= 0 || hidden_z <= 0) return 0;
   return plan(n, c_s, heads_s, hidden_z, hidden_s, c_s > 0).total + 1024;
+}
+
+extern "C" size_t b200tri_pairformer_stack_workspace_bytes(int32_t n, int32_t c_s, int32_t heads_s, int32_t hidden_z,
+                                                           int32_t hidden_s, int32_t n_blocks) {
+  const size_t least = b200tri_pairformer_workspace_bytes(n, c_s, heads_s, hidden_z, hidden_s);
+  return least && n_blocks > 1 && c_s > 0 && leaves_sms(n) ? least + second_end_bytes(n) : least;
 }
 
 extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200tri_stream_t stream_) {
@@ -255,15 +262,18 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   }
 
   // Where the pair track leaves SMs over, the pair bias is on the side stream as well, on those SMs,
-  // while the next block's pair track runs on z in a buffer of its own (blocks end in z_out and w2 in
-  // turn, the last one in z_out).
-  const bool bias_aside = single && lease->stream && leaves_sms(n) && sm_count() >= LEFT_OVER_BELOW + 16;
+  // while the next block's pair track runs on z in a buffer of its own: blocks end in z_out and w2 in
+  // turn, the last one in z_out. (In one buffer, with the wait for the pair bias ahead of the next
+  // block's second update, 24 blocks took 3430 instead of 3340 us at n = 128 and 3040 instead of 3075 at 100.)
+  const bool bias_aside = single && lease->stream && leaves_sms(n) && sm_count() >= LEFT_OVER_BELOW + 16 &&
+                          a->workspace_bytes >= pl.total + second_end_bytes(n);
+  void* w2 = bias_aside ? ws + pl.total : nullptr;
   const int over = bias_aside ? sm_count() - LEFT_OVER_BELOW : 0;
 
   PdlChain chain(false);
   for (int layer = 0; layer < a->n_blocks; ++layer) {
     const b200tri_pairformer_block_params P = params_of(layer);
-    void* z_end = bias_aside && (a->n_blocks - 1 - layer) % 2 ? static_cast<void*>(ws + pl.w2) : a->z_out;
+    void* z_end = bias_aside && (a->n_blocks - 1 - layer) % 2 ? w2 : a->z_out;
     // ---- pair track: the four triangle updates ping-pong between z_out and w (the first one
     // reads the caller's z_in), residual adds fused; with the pair gate, dropped pairs are
     // zeroed before the first update and after every update

@@ -193,8 +193,8 @@ def pairformer_forward(
         raise ValueError(f"libb200tri is built for single-track heads of width 24; got c_s {c_s}, {heads_s} heads")
     for p in packed:
         p.check(c_s, heads_s, bool(stacked), blocks if stacked else 1)
-    nbytes = _lib.workspace_bytes("b200tri_pairformer_workspace_bytes", n, c_s, heads_s,
-                                  max(p.hidden_z for p in packed), max(p.hidden_s for p in packed))
+    nbytes = _lib.workspace_bytes("b200tri_pairformer_stack_workspace_bytes", n, c_s, heads_s,
+                                  max(p.hidden_z for p in packed), max(p.hidden_s for p in packed), blocks)
     at = dev.place()
     ws = dev.workspace(nbytes, "pairformer", at)
     z_out = torch.empty_like(zd)

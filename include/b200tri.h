@@ -697,7 +697,7 @@ typedef struct {
   float* s_out;
   const float* pair_mask; /* [n][n] or NULL (= ones) */
   const float* mask;      /* [n] or NULL (= ones) */
-  void* workspace;        /* b200tri_pairformer_workspace_bytes, 1 KiB aligned */
+  void* workspace;        /* b200tri_pairformer_workspace_bytes or .._stack_workspace_bytes, 1 KiB aligned */
   size_t workspace_bytes;
   /* Variants of the block in the other model families (all 0 = the Boltz-2 block):
    * pair_gate: z is multiplied by (pair_mask != 0) before the first update and after every
@@ -715,6 +715,10 @@ typedef struct {
 
 /* hidden_z, hidden_s: of the widest block (the blocks of a list share the scratch) */
 size_t b200tri_pairformer_workspace_bytes(int32_t n, int32_t c_s, int32_t heads_s, int32_t hidden_z, int32_t hidden_s);
+/* What a stack of n_blocks can make use of, at least the above: with up to 128 tokens a second buffer for
+ * z, so that a block's pair bias runs beside the next block's pair track. Same results either way. */
+size_t b200tri_pairformer_stack_workspace_bytes(int32_t n, int32_t c_s, int32_t heads_s, int32_t hidden_z, int32_t hidden_s,
+                                                int32_t n_blocks);
 int b200tri_pairformer_forward(const b200tri_pairformer_args* args, b200tri_stream_t stream);
 
 #ifdef __cplusplus

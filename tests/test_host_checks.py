@@ -184,6 +184,23 @@ def test_pairformer_workspace_is_that_of_the_widest_block():
     assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_WORKSPACE
 
 
+def test_pairformer_needs_no_second_buffer_for_z():
+    """What a stack of few tokens can make use of beyond the scratch of a block is not asked of a caller:
+    scratch that was sized for a block is enough, and the single track's share grows with the tokens."""
+    from foldjax_b200 import _lib
+
+    lib = _lib.load()
+    block = {n: lib.b200tri_pairformer_workspace_bytes(n, 384, 16, 512, 1536) for n in range(100, 140)}
+    single = [block[n] - lib.b200tri_pairformer_workspace_bytes(n, 0, 0, 512, 0) for n in block]
+    assert single == sorted(single)
+    for n, least in block.items():
+        more = lib.b200tri_pairformer_stack_workspace_bytes(n, 384, 16, 512, 1536, 48) - least
+        assert more == (-(-n * n * 256 // 1024) * 1024 if n <= 128 else 0)
+        assert lib.b200tri_pairformer_stack_workspace_bytes(n, 384, 16, 512, 1536, 1) == least
+    assert lib.b200tri_pairformer_stack_workspace_bytes(64, 0, 0, 512, 0, 48) == lib.b200tri_pairformer_workspace_bytes(64, 0, 0, 512, 0)
+    assert lib.b200tri_pairformer_stack_workspace_bytes(0, 384, 16, 512, 1536, 48) == 0
+
+
 @pytest.mark.parametrize("stacked", [False, True])
 @pytest.mark.parametrize("path,shape", [
     (("tri_mul_out", "p_in", "kernel"), (128, 128)), (("tri_att_end", "linear", "kernel"), (128, 3)),
