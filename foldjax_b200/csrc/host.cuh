@@ -66,9 +66,10 @@ inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 // SMs the persistent kernels of the current device may use (its SM count, or the limit
 // set for that device with b200tri_set_sm_limit).
 int sm_count();
-// While one of these lives, sm_count() on this host thread returns `keep` SMs fewer: the
-// context-parallel ops leave room beside a persistent kernel for the small NCCL kernels that
-// carry their tokens (a kernel that fills every SM would hold them back until it ends).
+// While one of these lives, sm_count() on this host thread returns `keep` SMs fewer than before
+// (one inside another adds to it): the context-parallel ops leave room beside a persistent kernel
+// for the small NCCL kernels that carry their tokens (a kernel that fills every SM would hold them
+// back until it ends), and a stack of blocks keeps its pair bias to the SMs that are left over.
 struct SmReserve {
   int before;
   explicit SmReserve(int keep);

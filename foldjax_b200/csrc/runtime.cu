@@ -58,7 +58,7 @@ static int sm_count_device();
 
 static thread_local int t_sm_reserve = 0;
 
-SmReserve::SmReserve(int keep) : before(t_sm_reserve) { t_sm_reserve = keep > 0 ? keep : 0; }
+SmReserve::SmReserve(int keep) : before(t_sm_reserve) { t_sm_reserve = before + (keep > 0 ? keep : 0); }
 SmReserve::~SmReserve() { t_sm_reserve = before; }
 
 int sm_count() {

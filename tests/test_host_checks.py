@@ -184,6 +184,29 @@ def test_pairformer_workspace_is_that_of_the_widest_block():
     assert lib.b200tri_pairformer_forward(C.byref(args), None) == _lib.ERR_WORKSPACE
 
 
+def test_sm_reserves_add_up():
+    """An inner reserve must not hand out the SMs that the one around it keeps free."""
+    import ctypes as C
+
+    from foldjax_b200 import _lib
+
+    lib = _lib.load()
+    # (C++ of the library's own: b200::sm_count, and b200::SmReserve's constructor and destructor)
+    count, reserve, release = (getattr(lib, name) for name in ("_ZN4b2008sm_countEv", "_ZN4b2009SmReserveC1Ei", "_ZN4b2009SmReserveD1Ev"))
+    reserve.argtypes, reserve.restype, release.argtypes, release.restype = [C.c_void_p, C.c_int], None, [C.c_void_p], None
+    outer, inner = C.create_string_buffer(64), C.create_string_buffer(64)
+    sms = count()
+    for keep_outer, keep_inner in ((8, 5), (4, 100), (6, 0)):
+        reserve(outer, keep_outer)
+        assert count() == sms - keep_outer
+        reserve(inner, keep_inner)
+        assert count() == sms - keep_outer - keep_inner
+        release(inner)
+        assert count() == sms - keep_outer
+        release(outer)
+        assert count() == sms
+
+
 def test_pairformer_needs_no_second_buffer_for_z():
     """What a stack of few tokens can make use of beyond the scratch of a block is not asked of a caller:
     scratch that was sized for a block is enough, and the single track's share grows with the tokens."""
