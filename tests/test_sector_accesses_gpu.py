@@ -86,7 +86,7 @@ def test_core_result_off_the_sector_grid(cuda_device):
 @pytest.mark.parametrize("n,blocks", [(16, 4), (128, 3), (128, 4), (129, 3)])
 def test_stack_with_and_without_left_over_sms(cuda_device, n, blocks):
     """Up to 128 tokens the pair bias of a stack runs aside and blocks end in two buffers in turn:
-    the bits of one call per block, in place as well."""
+    the bits of one call per block."""
     from foldjax_b200 import _device as dev, _lib
     from foldjax_b200.pairformer import pairformer_forward, pairformer_layer_forward
 

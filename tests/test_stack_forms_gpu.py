@@ -68,3 +68,76 @@ def test_scratch_for_a_block_is_enough_for_a_stack(cuda_device, n, blocks):
     for stack_scratch in (False, True):
         got = _in_one_call(*inputs, stack_scratch=stack_scratch)
         assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("n,blocks", [(40, 2), (100, 3), (128, 4)])
+@pytest.mark.parametrize("flags", [{}, {"pair_gate": True}, {"mask_transition": True}, {"attention_first": True},
+                                   {"pair_gate": True, "mask_transition": True, "attention_first": True}], ids=lambda f: "+".join(f) or "plain")
+def test_stack_variants_and_in_place(cuda_device, n, blocks, flags):
+    params, s, z, mask, pair = _inputs(n, blocks)
+    # (dropped pairs that no token mask explains, so that the gate before the first update counts)
+    pair = pair * (torch.rand(pair.shape, generator=torch.Generator("cuda").manual_seed(n), device="cuda") > 0.05)
+    pair[0].fill_diagonal_(1.0)
+    pair *= mask[:, :, None] * mask[:, None, :]
+    want = _one_by_one(params, s, z, mask, pair, **flags)
+    for in_place in (False, True):
+        got = _in_one_call(params, s, z, mask, pair, in_place=in_place, **flags)
+        assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_stacks_at_once(cuda_device, threads):
+    """Two streams fed by one thread, or two threads that feed one stream each: the side streams of the
+    calls run beside one another."""
+    import threading
+
+    from foldjax_b200 import _lib
+    from foldjax_b200.pairformer import pairformer_forward
+
+    inputs = [_inputs(n, 4) for n in (100, 128)]
+    want = [_one_by_one(*i) for i in inputs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in inputs], [[] for _ in inputs]
+
+    def feed(k, count):
+        with torch.cuda.stream(streams[k]):
+            got[k] += [pairformer_forward(*inputs[k]) for _ in range(count)]
+
+    if threads:
+        workers = [threading.Thread(target=feed, args=(k, 10)) for k in range(2)]
+        for w in workers:
+            w.start()
+        for w in workers:
+            w.join()
+    else:
+        for _ in range(10):
+            for k in range(2):
+                feed(k, 1)
+    torch.cuda.synchronize()
+    _lib.device_status()
+    for w, results in zip(want, got):
+        assert len(results) == 10 and all(torch.equal(w[0], s) and torch.equal(w[1], z) for s, z in results)
+
+
+def test_captured_stack(cuda_device):
+    """While a stream is captured the stack stays on it: replays beside an eager call, same bits."""
+    from foldjax_b200 import _lib
+    from foldjax_b200.pairformer import pairformer_forward
+
+    captured, eager = _inputs(100, 3), _inputs(128, 3)
+    want, beside = _one_by_one(*captured), _one_by_one(*eager)
+    torch.cuda.synchronize()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        pairformer_forward(*captured)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        s, z = pairformer_forward(*captured)
+    for _ in range(3):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        s2, z2 = pairformer_forward(*eager)
+        torch.cuda.synchronize()
+        assert torch.equal(want[0], s) and torch.equal(want[1], z)
+        assert torch.equal(beside[0], s2) and torch.equal(beside[1], z2)
+    _lib.device_status()
