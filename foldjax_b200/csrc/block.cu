@@ -56,10 +56,15 @@ struct Plan {
   size_t w, sub, sub_bytes, sn, partial, h, att, fc[3], ones, total;
 };
 
-// One tile of the pair track's stage kernels per SM and some SMs over (a contraction has 128 tiles
-// there): what runs on the side stream has SMs of its own.
-constexpr int LEFT_OVER_BELOW = 128;
-bool leaves_sms(int n) { return n <= LEFT_OVER_BELOW; }
+// Up to this many tokens the pair track's stage kernels have one tile per SM (as many as tokens, a
+// contraction 128) and leave SMs over for what runs on the side stream. The attention core does not:
+// 4 * ceil(n / 3) items are more than the SMs from n = 109 on, and what meets it there delays it (17
+// instead of 12 us at n = 128). All in all the pair bias aside gains at every such size, 24 blocks,
+// us, n = 48 / 97 / 112 / 128: 2850 / 3195 / 3439 / 3669 without, 2730 / 3063 / 3287 / 3337 with, attention
+// first 2884 / 3213 / 3418 / 3471 and 2754 / 3066 / 3264 / 3395. With more tokens a row of pairs takes two
+// tiles, and the stage kernels fill every SM.
+constexpr int LEFT_OVER_UP_TO = 128;
+bool leaves_sms(int n) { return n <= LEFT_OVER_UP_TO; }
 // The second buffer that blocks of a stack end in where the workspace has room for it, behind the plan's total.
 size_t second_end_bytes(int n) { return (static_cast<size_t>(n) * n * 128 * 2 + 1023) / 1024 * 1024; }
 
@@ -265,10 +270,10 @@ extern "C" int b200tri_pairformer_forward(const b200tri_pairformer_args* a, b200
   // while the next block's pair track runs on z in a buffer of its own: blocks end in z_out and w2 in
   // turn, the last one in z_out. (In one buffer, with the wait for the pair bias ahead of the next
   // block's second update, 24 blocks took 3430 instead of 3340 us at n = 128 and 3040 instead of 3075 at 100.)
-  const bool bias_aside = single && lease->stream && leaves_sms(n) && sm_count() >= LEFT_OVER_BELOW + 16 &&
+  const bool bias_aside = single && lease->stream && leaves_sms(n) && sm_count() >= LEFT_OVER_UP_TO + 16 &&
                           a->workspace_bytes >= pl.total + second_end_bytes(n);
   void* w2 = bias_aside ? ws + pl.total : nullptr;
-  const int over = bias_aside ? sm_count() - LEFT_OVER_BELOW : 0;
+  const int over = bias_aside ? sm_count() - LEFT_OVER_UP_TO : 0;
 
   PdlChain chain(false);
   for (int layer = 0; layer < a->n_blocks; ++layer) {

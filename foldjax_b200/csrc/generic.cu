@@ -360,7 +360,11 @@ int launch_ln_gather(LnArgs a, cudaStream_t stream, bool pdl) {
 // took 209. Eight neighbouring channels per lane are 16 bytes; in bf16, up to 64 * G channels, they
 // are put together in shared memory (over the values, when all have been read) and leave as one
 // contiguous run: stored by the lanes themselves they went to 64 rows, half a sector each. In
-// float32, up to 384 channels, the three pieces have a place of their own behind the values (G = 1).
+// float32, up to 384 channels, the three pieces have a place of their own behind the values (G = 1). That
+// leaves 3 / 2 / 1 blocks to an SM at 192 / 256 / 384 channels. The whole multiplication staged and not,
+// us: 128 channels, 256 tokens 181 / 192; 192, 96 and 256 tokens 110 / 128 and 415 / 429; 256, 96 and 256 tokens
+// 140 / 154 and 619 / 614; 320, 96 and 256 tokens 198 / 225 and 890 / 906; 384, 96 and 256 tokens 252 / 269 and
+// 1202 / 1175 (of the latter 270 and 1250 with 16-byte accesses).
 constexpr int LNT_WARPS = 8;
 template <bool BF>
 constexpr int lnt_j() {

@@ -31,8 +31,8 @@
 //                 of every row into hidden values
 // Bound: the activation (two MUFU operations per hidden unit: 1024 per pair) and
 // the tensor pipe (393 kflop per pair) are within 25 % of each other; HBM moves
-// 2 x 256 B per pair (x doubles as the residual when the caller adds in place). MUFU unit 65 % busy,
-// tensor pipe 49 %. 1024 x 1024 pairs, hidden 512: 415 us (251 at the tensor cores' rate); 575 with
+// 2 x 256 B per pair (x doubles as the residual when the caller adds in place). MUFU unit 68 % busy,
+// tensor pipe 51 %. 1024 x 1024 pairs, hidden 512: 415 us (251 at the tensor cores' rate); 575 with
 // one warpgroup for layer norm and epilogue in turn and a thread per pair's row and residual, for
 // which everything else waits.
 #include "host.cuh"

@@ -32,31 +32,32 @@
 // tensor core accumulates sum_k P next to P.V). Registers are moved from the control warpgroup
 // to the softmax warpgroups at start-up (setmaxnreg).
 //
-// Bound: not the tensor pipe and not HBM. Per score the SM issues 6.5 instructions (3-input
+// Bound: not the tensor pipe and not HBM. Per score the SM issues 6.7 instructions (3-input
 // max, packed fma, ex2 or the cubic with its exponent insertion, clamp, half a cvt) against 128
 // tensor flops, and the MUFU unit delivers 16 exponentials per clock and SM: the kernel issues in
-// 65 % of its slots with the tensor pipe 45 % and the MUFU unit 43 % busy (n = 1024, counters). The
+// 65 % of its slots with the tensor pipe 44 % and the MUFU unit 42 % busy (n = 1024, counters). The
 // other slots are waits: TMEM loads, fixed latencies and the barriers between the roles. What a
 // step costs beyond that is registers: 64 scores per thread under the 128-register limit of 512
 // threads. So nothing that an item's end needs is kept across its steps (the position is worked
 // out again there, with 32-bit divisions) and its result is read back in halves; a warp, not a
 // thread, arrives on the barriers; the next item's queries are loaded while this one still runs.
-// With the position kept in registers a step took 3 to 12 % more.
-// SM clocks of a launch per step of three rows and SM (counter, set-up and last wave included): 1990 at
-// n = 1024 (2170 before the steps below). A longer key loop does not cost more clocks, it runs at fewer
-// MHz under the power limit (1965 while the launches are short, 1700 at n = 3072). Measured and not
-// better: score buffers in pairs, a ring of their own for K and the bias, four stages, 7 or 9 of 16 pairs
-// on the FMA pipe, results staged for a TMA store.
-// Attention operator, us, n = 256 / 384 / 1024 / 3072: with every role's index and loops divergent (a
-// thread of its own, operands through vector registers) and P.V of the step before waited for ahead
-// of the maximum, 43.5 / 113.3 / 1505 / 39600; the warp index through a shuffle 43.2 / 110.6 / 1458; the
-// wait moved behind the exponentials 42.1 / 109.5 / 1432; uniform issuer loops 41.2 / 106.6 / 1402 /
-// 37500; the two waits at a step's start as one and the producer's loop uniform 41.1 / 105.3 / 1364 /
-// 36800; the result in 32-byte stores 39.3 / 102.8 / 1348. A product takes its issuer 60 to 90 clocks and the tensor pipe 48 (A from shared memory) or
-// 24 (P, 128x48), 386 for a row's step measured alone. Measured and not better: a second Q.K^T issuer
-// (1498), four rows with 32 scores at a time and an issuer per row and product (1459 with the same
-// offsets; the rows fall into phase and queue for the same unit), two rows to an item where that saves
-// none a round, no more CTAs than whole rounds need (the successor sets up on the SMs that end early).
+// With the position kept in registers a step took 3 to 12 % more. A longer key loop does not cost
+// more clocks, it runs at fewer MHz under the power limit (1965 while the launches are short, 1700
+// at n = 3072).
+// A product takes its issuer 60 to 90 clocks and the tensor pipe 48 (A from shared memory) or 24 (P,
+// 128x48), 386 for a row's step measured alone: so warp indices go through a shuffle and the issuers'
+// loops are the whole warp's, which keeps control flow and operands in uniform registers, P.V of the
+// step before is waited for behind the exponentials, and the two waits at a step's start are asked as
+// one; results leave in 32-byte stores. Attention operator, us, n = 256 / 384 / 512 / 3072: 45.0 / 113.7 /
+// 229.6 / 40 800 before those, 40.6 / 103.2 / 211.6 / 37 300 now. Of that the joins that hold the lanes of a warp together cost the
+// issuers 0.5 / 1.6 / 4.1 / 100 and gave the softmax 0.9 / 1.6 / 1.4 / 400. Measured instead of
+// __syncwarp behind the issuers' waits: a vote on each wait (213 at n = 512), elect.sync (212), the
+// waits in the leader's branch, which needs no join (261).
+// Measured and not better: score buffers in pairs, a ring of their own for K and the bias, four stages,
+// 7 or 9 of 16 pairs on the FMA pipe, results staged for a TMA store, a second Q.K^T issuer, four rows
+// with 32 scores at a time and an issuer per row and product (the rows fall into phase and queue for the
+// same unit), two rows to an item where that saves none a round, no more CTAs than whole rounds need (the
+// successor sets up on the SMs that end early).
 #include <cuda_fp16.h>
 
 #include <mutex>

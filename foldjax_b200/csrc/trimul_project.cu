@@ -23,7 +23,7 @@
 // separately so the MMAs of the next tile overlap the epilogue of this one.
 //
 // Bound: HBM by the bytes (read x once, write a and b once: 3 * n*n*128*2 bytes, 123 us at n = 1024);
-// in fact the MUFU unit, two operations for each of a pair's 256 sigmoids: 75 % busy over the 200 us
+// in fact the MUFU unit, two operations for each of a pair's 256 sigmoids: 74 % busy over the 204 us
 // of a launch at n = 1024 (213 with a warp index the compiler did not know to be uniform, 285 with one
 // epilogue warpgroup that stored each thread's run directly).
 #include <type_traits>
