@@ -4,29 +4,23 @@
 //
 //   S = (q . k) * scale + mask_bias + bias        o = softmax(S) . v
 //
-// q, k, v arrive as IN bf16 pieces each (gemm.cuh): three when they are float32, one when the
-// trunk is bf16. The probabilities are split into three pieces by the thread that computes
-// them, so P.V is as exact as a float32 product. The piece products of one result are issued
+// q, k, v arrive as bf16 pieces (gemm.cuh): three when they are float32, one when the trunk is bf16,
+// which has a kernel of its own below. The probabilities are split into three pieces by the thread that
+// computes them, so P.V is as exact as a float32 product. The piece products of one result are issued
 // smallest first into one float32 accumulator, so that only the leading one is summed at full
 // magnitude. Everything in between is float32 as in the reference (_attention_block,
 // src/foldjax/models/boltz2/models/triangle/triangle_attention.py:428-455;
 // _attention_qblock, primitives/attention.py:124-140): softmax in float32. With float32 operands
 // the running numerator stays in registers (P.V of a step starts from zero and is added by the
-// thread, which also makes the rescale a register fma). With bf16 operands it accumulates in TMEM
-// and is rescaled only when the maximum grew by more than RESCALE; the bias is bf16 too then and is
-// added by the tensor core, as in triatt_core.cu (S = bias . I + q . k).
+// thread, which also makes the rescale a register fma).
 //
 // One CTA per SM, persistent; an item is (head, NWG rows, 128 queries), or with one row (head,
 // NWG tiles of 128 queries), walked in steps of 64 keys:
 //   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
 //   warpgroups  softmax, one thread per query
-// Bound: issue slots. A score costs about 2 instructions of exponential, 4.5 of split and 2-4
-// others, most of them packed two to an instruction. Two softmax warpgroups fill 41 % of the slots with
-// float32 operands and 52 % with bf16 ones; there a third one fits (62 %), because the probabilities
-// overwrite the scores in TMEM (OVERLAY): the scores of the next step then wait for this step's P.V,
-// which the other two warpgroups hide. Measured and not better: P as two tf32 pieces against V as
-// float32 (705 us against 697 for a template stack), leaving out the groups of 16 keys past the last one
-// (721 against 691: the conditions in the loop cost more), one arrival per warp on the barriers.
+// Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (a score costs about 2
+// instructions of exponential, 4.5 of split and 4 others, most of them packed two to an instruction); the
+// rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
 #include "att_split.cuh"
 #include "gemm.cuh"
 #include "tc.cuh"
@@ -38,32 +32,27 @@ namespace {
 constexpr int KT = 64;
 constexpr float RESCALE = 5.5f;  // probabilities stay below e^5.5
 
-template <int HDP, int IN, bool TOKEN>
+template <int HDP, bool TOKEN>
 struct Cfg {
-  static constexpr bool OVERLAY = IN == 1;
-  static constexpr int NWG = HDP == 32 ? (IN == 1 ? 3 : 2) : (IN == 1 ? 2 : 1);
+  static constexpr int NWG = HDP == 32 ? 2 : 1;
   static constexpr int KV = TOKEN ? 1 : NWG;  // rows whose keys a step loads
   static constexpr int NB = TOKEN ? NWG : 1;  // bias tiles of a step
-  static constexpr int STAGES = IN == 1 ? 3 : 2;
+  static constexpr int STAGES = 2;
   static constexpr int THREADS = 128 + NWG * 128;
   static constexpr int Q_BYTES = 128 * HDP * 2, K_BYTES = KT * HDP * 2, V_BYTES = HDP * 128;
-  static constexpr int BIAS_BYTES = 128 * KT * (IN == 1 ? 2 : 4);
-  static constexpr uint32_t TM_S = 0, TM_P = OVERLAY ? 0 : 64, TM_O = TM_P + 96, TM_WG = TM_O + HDP;
+  static constexpr int BIAS_BYTES = 128 * KT * 4;
+  static constexpr uint32_t TM_S = 0, TM_P = 64, TM_O = TM_P + 96, TM_WG = TM_O + HDP;
   static_assert(NWG * TM_WG <= 512, "tensor memory budget");
-  // three warpgroups: registers move from the control warpgroup (512 x 128 = 128 x 80 + 384 x 144)
-  static constexpr bool SHIFT_REGS = NWG == 3;
-  static constexpr uint32_t STAGE_TX = KV * IN * (K_BYTES + V_BYTES) + NB * BIAS_BYTES + KV * KT * 4;
+  static constexpr uint32_t STAGE_TX = KV * 3 * (K_BYTES + V_BYTES) + NB * BIAS_BYTES + KV * KT * 4;
 };
 
-template <int HDP, int IN, bool TOKEN>
+template <int HDP, bool TOKEN>
 struct Smem {
-  using C = Cfg<HDP, IN, TOKEN>;
-  uint8_t q[C::NWG][IN][C::Q_BYTES];
-  uint8_t k[C::STAGES][C::KV][IN][C::K_BYTES];
-  uint8_t v[C::STAGES][C::KV][IN][C::V_BYTES];
-  // float32: two boxes of 32 keys, [128 queries][32 floats]; bf16: [128 queries][64]
-  uint8_t bias[C::STAGES][C::NB][C::BIAS_BYTES];
-  uint8_t ident[IN == 1 ? KT * 128 : 128];  // 64 x 64 bf16 identity
+  using C = Cfg<HDP, TOKEN>;
+  uint8_t q[C::NWG][3][C::Q_BYTES];
+  uint8_t k[C::STAGES][C::KV][3][C::K_BYTES];
+  uint8_t v[C::STAGES][C::KV][3][C::V_BYTES];
+  uint8_t bias[C::STAGES][C::NB][C::BIAS_BYTES];  // two boxes of 32 keys, [128 queries][32 floats]
   alignas(128) float mb[C::STAGES][C::KV][KT];
   uint64_t q_full, q_empty, st_full[C::STAGES], st_empty[C::STAGES], s_full[C::NWG], s_free[C::NWG], p_full[C::NWG],
       pv_done[C::NWG];
@@ -101,16 +90,16 @@ __device__ __forceinline__ void split3f2(float2 v, uint32_t& hi, uint32_t& mid, 
   lo = pack_bf16x2(q.x, q.y);
 }
 
-template <int HDP, int IN, bool TOKEN>
-__global__ void __launch_bounds__(Cfg<HDP, IN, TOKEN>::THREADS, 1)
+template <int HDP, bool TOKEN>
+__global__ void __launch_bounds__(Cfg<HDP, TOKEN>::THREADS, 1)
 att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
-  using C = Cfg<HDP, IN, TOKEN>;
-  using TQ = Terms<IN, IN>;  // q . k
-  using TP = Terms<3, IN>;   // P . v
+  using C = Cfg<HDP, TOKEN>;
+  using TQ = Terms<3, 3>;  // q . k
+  using TP = Terms<3, 3>;  // P . v
   constexpr int NWG = C::NWG, STAGES = C::STAGES;
-  static_assert(sizeof(Smem<HDP, IN, TOKEN>) <= 232448, "shared memory budget");
+  static_assert(sizeof(Smem<HDP, TOKEN>) <= 232448, "shared memory budget");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  Smem<HDP, IN, TOKEN>& sm = *reinterpret_cast<Smem<HDP, IN, TOKEN>*>(smem_raw);
+  Smem<HDP, TOKEN>& sm = *reinterpret_cast<Smem<HDP, TOKEN>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((smem_u32(smem_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
@@ -139,14 +128,6 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
-  if (IN == 1) {  // the identity, K-major under the 128-byte swizzle
-    for (int idx = threadIdx.x; idx < KT * 32; idx += C::THREADS) {
-      const int r = idx / 32, w = idx % 32;
-      const int e0 = ((w >> 2) ^ (r & 7)) * 8 + (w & 3) * 2;  // logical element of the word's low half
-      reinterpret_cast<uint32_t*>(sm.ident)[idx] = e0 == r ? 0x00003F80u : e0 + 1 == r ? 0x3F800000u : 0u;
-    }
-    fence_proxy_async();
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -165,7 +146,6 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
     j0 = tile * (TOKEN ? NWG * 128 : 128);
   };
 
-  if (C::SHIFT_REGS && warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
@@ -173,12 +153,12 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       bool alive = true;
       for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
         if (!mbar_wait(&sm.q_empty, (item_it & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.q_full, NWG * IN * C::Q_BYTES);
+        mbar_expect_tx(&sm.q_full, NWG * 3 * C::Q_BYTES);
         int b, h, i, j0;
         locate(item, b, h, i, j0);
         const int row = b * p.n_i + i;
         for (int g = 0; g < NWG; ++g)
-          for (int pc = 0; pc < IN; ++pc)
+          for (int pc = 0; pc < 3; ++pc)
             tma_load_5d(sm.q[g][pc], &tm.q, &sm.q_full, 0, h, TOKEN ? j0 + g * 128 : j0, TOKEN ? row : row + g, pc);
         for (int t = 0; t < p.steps; ++t) {
           if (!mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
@@ -190,14 +170,14 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
 #pragma unroll 1
           for (int g = 0; g < C::KV; ++g) {
 #pragma unroll 1
-            for (int pc = 0; pc < IN; ++pc) {
+            for (int pc = 0; pc < 3; ++pc) {
               tma_load_5d(sm.k[stage][g][pc], &tm.k, &sm.st_full[stage], 0, h, k0, row + g, pc);
               tma_load_5d(sm.v[stage][g][pc], &tm.v, &sm.st_full[stage], k0, 0, h, row + g, pc);
             }
             tma_load_2d(sm.mb[stage][g], &tm.m, &sm.st_full[stage], k0, row + g);
           }
           for (int g = 0; g < C::NB; ++g) {
-            for (int half = 0; half < (IN == 1 ? 1 : 2); ++half)
+            for (int half = 0; half < 2; ++half)
               tma_load_4d(sm.bias[stage][g] + half * 16384, &tm.b, &sm.st_full[stage], k0 + half * 32, j0 + g * 128, h, b);
           }
           if (++stage == STAGES) {
@@ -221,20 +201,12 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
             break;
           }
           for (int wg = 0; wg < NWG; ++wg) {
-            // the scores' columns are free once they have been read, or (overlaid) once P.V is through
-            if (!mbar_wait(C::OVERLAY ? &sm.pv_done[wg] : &sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
+            if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
               alive = false;
               break;
             }
             tc_fence_after();
             const uint32_t d = tmem_base + wg * C::TM_WG + C::TM_S;
-            if (IN == 1) {
-              const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[stage][0]), 128);
-              const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
-#pragma unroll
-              for (int kk = 0; kk < KT / 16; ++kk)
-                umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
-            }
 #pragma unroll
             for (int term = 0; term < TQ::N; ++term) {
               const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[wg][TQ::a(term)]), HDP * 2);
@@ -242,7 +214,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
 #pragma unroll
               for (int kk = 0; kk < HDP / 16; ++kk)
                 umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc,
-                             IN == 1 || (term | kk) != 0);
+                             (term | kk) != 0);
             }
             umma_commit(&sm.s_full[wg]);
           }
@@ -279,7 +251,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
 #pragma unroll
               for (int kk = 0; kk < KT / 16; ++kk)
                 umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
-                             idesc, (C::OVERLAY && t > 0) || (term | kk) != 0);
+                             idesc, (term | kk) != 0);
             }
             umma_commit(&sm.pv_done[wg]);
           }
@@ -293,7 +265,6 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       }
     }
   } else if (warp >= 4) {
-    if (C::SHIFT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
     const int wg = (warp - 4) >> 2, quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t t_wg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + wg * C::TM_WG;
@@ -302,9 +273,9 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
     bool alive = true;
     for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
       float m_run = -INFINITY, l_run = 0.f, alpha = 0.f;
-      float o[C::OVERLAY ? 1 : HDP];
+      float o[HDP];
 #pragma unroll
-      for (int d = 0; d < (C::OVERLAY ? 1 : HDP); ++d) o[d] = 0.f;
+      for (int d = 0; d < HDP; ++d) o[d] = 0.f;
       auto take_pv = [&] {  // o = o * (rescale of the step P.V belongs to) + P.V
 #pragma unroll
         for (int part = 0; part < HDP / 16; ++part) {
@@ -313,7 +284,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           tmem_ld_wait();
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            float& acc = o[C::OVERLAY ? 0 : part * 16 + e];
+            float& acc = o[part * 16 + e];
             acc = fmaf(acc, alpha, __uint_as_float(r[e]));
           }
         }
@@ -321,11 +292,6 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       for (int t = 0; t < p.steps; ++t, ++g) {
         if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) ||
             !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX)) {
-          alive = false;
-          break;
-        }
-        // (overlaid scores can only have been formed after the previous P.V: no wait, but its order)
-        if (C::OVERLAY && !mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
           alive = false;
           break;
         }
@@ -344,37 +310,27 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           }
         }
         tc_fence_before();
-        if (!C::OVERLAY) mbar_arrive(&sm.s_free[wg]);
+        mbar_arrive(&sm.s_free[wg]);
         const float* mrow = sm.mb[stage][TOKEN ? 0 : wg];
         const bool masked = __any_sync(0xffffffffu, mrow[lane] != 0.f || mrow[lane + 32] != 0.f);
-        if (IN == 1) {  // the bias is in already
-          if (masked)
+        // the reference's order of the two sums
+        const uint8_t* brow = sm.bias[stage][TOKEN ? wg : 0];
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
-              s[2 * c] = __fadd2_rn(s[2 * c], make_float2(m4.x, m4.y));
-              s[2 * c + 1] = __fadd2_rn(s[2 * c + 1], make_float2(m4.z, m4.w));
-              if ((c & 1) == 1) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
-            }
-        } else {  // the reference's order of the two sums
-          const uint8_t* brow = sm.bias[stage][TOKEN ? wg : 0];
+        for (int c = 0; c < 16; ++c) {
+          const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * 16384 + sw128_offset(row, c & 7));
+          const float2 b2[2] = {make_float2(b4.x, b4.y), make_float2(b4.z, b4.w)};
+          float2 m2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          if ((c & 1) == 1) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
+          if (masked) {
+            const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
+            m2[0] = make_float2(m4.x, m4.y);
+            m2[1] = make_float2(m4.z, m4.w);
+          }
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * 16384 + sw128_offset(row, c & 7));
-            const float2 b2[2] = {make_float2(b4.x, b4.y), make_float2(b4.z, b4.w)};
-            float2 m2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            if ((c & 1) == 1) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
-            if (masked) {
-              const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
-              m2[0] = make_float2(m4.x, m4.y);
-              m2[1] = make_float2(m4.z, m4.w);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              float2& x = s[2 * c + u];
-              x = TOKEN ? __fadd2_rn(__ffma2_rn(x, make_float2(p.scale, p.scale), b2[u]), m2[u])
-                        : __fadd2_rn(__fadd2_rn(x, m2[u]), b2[u]);
-            }
+          for (int u = 0; u < 2; ++u) {
+            float2& x = s[2 * c + u];
+            x = TOKEN ? __fadd2_rn(__ffma2_rn(x, make_float2(p.scale, p.scale), b2[u]), m2[u])
+                      : __fadd2_rn(__fadd2_rn(x, m2[u]), b2[u]);
           }
         }
         __syncwarp();
@@ -385,23 +341,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           mxa = fmax3(mxa, s[e].x, s[e].y);
           mxb = fmax3(mxb, s[e + 1].x, s[e + 1].y);
         }
-        float mx = fmaxf(mxa, mxb);  // (with the running maximum in it)
-        if (C::OVERLAY) {  // keep the offset unless the maximum grew a lot
-          const bool need = mx - m_run > RESCALE;  // true on the first step
-          if (!need) mx = m_run;
-          if (__any_sync(0xffffffffu, need) && t > 0) {
-            const float scale = fast_exp2((m_run - mx) * 1.44269504f);
-#pragma unroll
-            for (int part = 0; part < HDP / 16; ++part) {
-              uint32_t r[16];
-              tmem_ld16(t_wg + C::TM_O + part * 16, r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * scale);
-              tmem_st16(t_wg + C::TM_O + part * 16, r);
-            }
-          }
-        }
+        const float mx = fmaxf(mxa, mxb);  // (with the running maximum in it)
         const float alpha_new = fast_exp2((m_run - mx) * 1.44269504f);  // 0 on the first step
         m_run = mx;
         float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -411,14 +351,13 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           l2[e & 1] = __fadd2_rn(l2[e & 1], s[e]);
         }
         l_run = fmaf(l_run, alpha_new, (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));
-        if (!C::OVERLAY) {  // the previous step's P.V: its result is taken, then P may be overwritten
-          if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
-            alive = false;
-            break;
-          }
-          tc_fence_after();
-          if (t > 0) take_pv();
+        // the previous step's P.V: its result is taken, then P may be overwritten
+        if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+          alive = false;
+          break;
         }
+        tc_fence_after();
+        if (t > 0) take_pv();
         alpha = alpha_new;
 #pragma unroll
         for (int oct = 0; oct < 4; ++oct) {  // 16 keys at a time: few live registers
@@ -440,7 +379,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) break;
       tc_fence_after();
       __syncwarp();
-      if (!C::OVERLAY) take_pv();
+      take_pv();
       int b, h, i, j0;
       locate(item, b, h, i, j0);
       if (TOKEN)
@@ -451,34 +390,8 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       const bool live = i < p.n_i && j < p.n;
       const long long off = ((static_cast<long long>(b * p.n_i + i) * p.n + j) * p.heads + h) * p.head_dim;
       const float inv = 1.0f / l_run;
-      if (C::OVERLAY) {
-#pragma unroll
-        for (int part = 0; part < HDP / 16; ++part) {
-          uint32_t r[16];
-          tmem_ld16(t_wg + C::TM_O + part * 16, r);
-          tmem_ld_wait();
-          if (!live) continue;
-          uint4 w[2];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            uint32_t u[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              u[e] = pack_bf16x2(__uint_as_float(r[8 * q + 2 * e]) * inv, __uint_as_float(r[8 * q + 2 * e + 1]) * inv);
-            w[q] = make_uint4(u[0], u[1], u[2], u[3]);
-          }
-          uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.o) + off + part * 16);
-          if (p.head_dim % 16 == 0 && part * 16 < p.head_dim) {
-            store_sector(dst, w[0], w[1]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < 2; ++q)
-              if (part * 16 + q * 8 < p.head_dim) dst[q] = w[q];
-          }
-        }
-      }
       tc_fence_before();
-      if constexpr (!C::OVERLAY && TOKEN) {
+      if constexpr (TOKEN) {
         const long long plane = static_cast<long long>(p.n) * p.heads * p.head_dim;
 #pragma unroll
         for (int d = 0; d < HDP; d += 8) {
@@ -492,7 +405,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           for (int q = 0; q < 3; ++q)
             *reinterpret_cast<uint4*>(p.pieces + q * plane + off + d) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
         }
-      } else if constexpr (!C::OVERLAY) {
+      } else {
 #pragma unroll
         for (int d = 0; d < HDP; d += 8)
           if (live && d < p.head_dim) {  // (a multiple of 8)
@@ -512,9 +425,9 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-template <int HDP, int IN, bool TOKEN>
+template <int HDP, bool TOKEN>
 int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
-  using C = Cfg<HDP, IN, TOKEN>;
+  using C = Cfg<HDP, TOKEN>;
   const int tiles = (p.n + 127) / 128;
   p.groups = TOKEN ? 1 : (p.n_i + C::NWG - 1) / C::NWG;
   p.tiles_j = TOKEN ? (tiles + C::NWG - 1) / C::NWG : tiles;
@@ -522,11 +435,446 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "float32 attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
   const int rc =
-      ensure_smem_limit(reinterpret_cast<const void*>(att_split_kernel<HDP, IN, TOKEN>), (int)sizeof(Smem<HDP, IN, TOKEN>));
+      ensure_smem_limit(reinterpret_cast<const void*>(att_split_kernel<HDP, TOKEN>), (int)sizeof(Smem<HDP, TOKEN>));
   if (rc) return rc;
   const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
-  return launch(att_split_kernel<HDP, IN, TOKEN>, dim3(grid), dim3(C::THREADS),
-                sizeof(Smem<HDP, IN, TOKEN>), stream, pdl, tm, p);
+  return launch(att_split_kernel<HDP, TOKEN>, dim3(grid), dim3(C::THREADS),
+                sizeof(Smem<HDP, TOKEN>), stream, pdl, tm, p);
+}
+
+
+// ------------------------------------------------------------------------- bf16 operands
+// The same core where q, k, v and the bias are bf16. The bias is added by the tensor core, as in
+// triatt_core.cu (S = bias . I + q . k), the numerator accumulates in TMEM and is rescaled only when
+// the maximum grew by more than RESCALE, and the probabilities overwrite the scores they came from, so
+// that four softmax warpgroups fit (128 columns each).
+//   warp 0       TMA producer       warps 1, 2   issuers, each of all products of its rows
+//   warpgroups   softmax, one thread per query
+// The scores of a row's next step are issued right behind P.V of this one, by the same thread: the
+// tensor pipe works a thread's products off in the order they were issued in, so the scores cannot overtake
+// the P.V that still reads the columns they go to, and one barrier tells the softmax that both are
+// through. The softmax offset is an integer in log2 units (one fma per pair of exponentials, exact
+// powers of two to rescale by) except where scores are so large that integers are no finer than they are.
+//
+// Bound: a row's step is a chain of softmax (1.2 us with the other rows' warps beside it, 8 instructions a
+// score) and products (18 of them, 0.35 us, and the trips between the warps), and the rows in flight hide
+// each other's: with three rows, scores and P.V issued by two warps that waited for each other's products, and
+// products and sums of float32 pairs unpacked from the pieces instead of mixed-precision fmas, a step of
+// three rows took 2.35 us where one of four takes 2.66. Four updates of four 200-token templates 700 -> 649 us, of a
+// 256-token refiner 1161 -> 1119, attention of 4 x 320 tokens 541 -> 444.
+// Measured and not better: an issuer per row, rows started a fraction of a step apart, P as two tf32 pieces
+// against V as float32, ending an item with its rows' last kept key (the flags cost the issuers 4 %, which
+// only paddings of a whole step pay back), the difference of two bf16 by a subtraction.
+template <int HDP, int NWG>
+struct BfCfg {
+  static constexpr int STAGES = 3, QBUF = 2, THREADS = 128 + NWG * 128;
+  static constexpr int ISSUERS = NWG == 3 ? 1 : 2, ROWS = NWG / ISSUERS;  // rows of an issuer
+  // Registers of the control and of the softmax warpgroups, out of those the block is launched with:
+  // 512 x 128 = 128 x 56 + 384 x 152, 640 x 96 = 128 x 32 + 512 x 112 (two rows have enough as they are)
+  static constexpr int CONTROL_REGS = NWG == 4 ? 32 : 56, SOFTMAX_REGS = NWG == 4 ? 112 : 152;
+  static constexpr int Q_BYTES = 128 * HDP * 2, K_BYTES = KT * HDP * 2, V_BYTES = HDP * 128, BIAS_BYTES = 128 * KT * 2;
+  static constexpr uint32_t TM_P = 0, TM_O = 96, TM_WG = TM_O + HDP;  // P (three pieces) over S (64 columns)
+  static_assert(NWG * TM_WG <= 512, "tensor memory budget");
+  static constexpr uint32_t STAGE_TX = NWG * (K_BYTES + V_BYTES + KT * 4) + BIAS_BYTES;
+};
+
+template <int HDP, int NWG>
+struct BfSmem {
+  using C = BfCfg<HDP, NWG>;
+  uint8_t q[C::QBUF][NWG][C::Q_BYTES];
+  uint8_t k[C::STAGES][NWG][C::K_BYTES];
+  uint8_t v[C::STAGES][NWG][C::V_BYTES];
+  uint8_t bias[C::STAGES][C::BIAS_BYTES];  // [128 queries][64 keys]
+  uint8_t ident[KT * 128];                 // 64 x 64 bf16 identity
+  alignas(128) float mb[C::STAGES][NWG][KT];
+  uint64_t q_full[C::QBUF], q_empty[C::QBUF], st_full[C::STAGES], st_empty[C::STAGES], s_full[NWG], p_full[NWG], o_full[NWG];
+  uint32_t tmem_base;
+};
+
+constexpr float LOG2E = 1.44269504f;
+constexpr float INTEGER_OFFSETS = 8388608.0f;  // 2^23: floats beyond are integers themselves
+
+
+// v - (the pair's two values), one instruction each (8 % of the kernel, against two to unpack and half a packed one).
+__device__ __forceinline__ float2 less_bf16x2(float2 v, uint32_t w) {
+  float2 r;
+  asm("{\n"
+      " .reg .b16 lo, hi, m;\n"
+      " mov.b32 {lo, hi}, %2;\n"
+      " mov.b16 m, 0xBF80;\n"
+      " fma.rn.f32.bf16 %0, lo, m, %3;\n"
+      " fma.rn.f32.bf16 %1, hi, m, %4;\n"
+      "}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "r"(w), "f"(v.x), "f"(v.y));
+  return r;
+}
+__device__ __forceinline__ void split3n2(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16x2(v.x, v.y);
+  const float2 r = less_bf16x2(v, hi);
+  mid = pack_bf16x2(r.x, r.y);
+  const float2 q = less_bf16x2(r, mid);
+  lo = pack_bf16x2(q.x, q.y);
+}
+
+template <int HDP, int NWG>
+__global__ void __launch_bounds__(BfCfg<HDP, NWG>::THREADS, 1)
+att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
+  using C = BfCfg<HDP, NWG>;
+  using TP = Terms<3, 1>;  // P . v
+  constexpr int STAGES = C::STAGES;
+  static_assert(sizeof(BfSmem<HDP, NWG>) <= 232448, "shared memory budget");
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  BfSmem<HDP, NWG>& sm = *reinterpret_cast<BfSmem<HDP, NWG>*>(smem_raw);
+  // (through a shuffle, so that the compiler knows it to be the same in all lanes)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  if ((smem_u32(smem_raw) & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
+    return;
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm.q);
+    tma_prefetch_desc(&tm.k);
+    tma_prefetch_desc(&tm.v);
+    tma_prefetch_desc(&tm.b);
+    for (int b = 0; b < C::QBUF; ++b) {
+      mbar_init(&sm.q_full[b], 1);
+      mbar_init(&sm.q_empty[b], C::ISSUERS);
+    }
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&sm.st_full[s], 1);
+      mbar_init(&sm.st_empty[s], C::ISSUERS + NWG * 4);
+    }
+    for (int g = 0; g < NWG; ++g) {
+      mbar_init(&sm.s_full[g], 1);
+      mbar_init(&sm.p_full[g], 4);
+      mbar_init(&sm.o_full[g], 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&sm.tmem_base, 512);
+    tmem_relinquish();
+  }
+  for (int idx = threadIdx.x; idx < KT * 32; idx += C::THREADS) {  // the identity, K-major under the 128-byte swizzle
+    const int r = idx / 32, w = idx % 32;
+    const int e0 = ((w >> 2) ^ (r & 7)) * 8 + (w & 3) * 2;  // logical element of the word's low half
+    reinterpret_cast<uint32_t*>(sm.ident)[idx] = e0 == r ? 0x00003F80u : e0 + 1 == r ? 0x3F800000u : 0u;
+  }
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t tmem_base = sm.tmem_base;
+  const uint32_t items_per_head = p.groups * p.tiles_j;
+  // item -> head, batch item, first row inside it and first query
+  auto locate = [&](uint32_t item, int& b, int& h, int& i, int& j0) {
+    const uint32_t bh = item / items_per_head, rem = item - bh * items_per_head;
+    b = bh / p.heads;
+    h = bh - b * p.heads;
+    const uint32_t grp = rem / p.tiles_j;
+    i = grp * NWG;
+    j0 = (rem - grp * p.tiles_j) * 128;
+  };
+
+  // In warps 0 to 2 all lanes walk the loops and wait, and one of them issues; none leaves early: one whose
+  // wait has run out stops waiting and issuing and walks on. Joins as in triatt_core.cu.
+  if (warp < 4) {
+    if (NWG > 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::CONTROL_REGS));
+    if (warp == 0) {
+      const bool leader = elect_one();
+      int stage = 0;
+      uint32_t phase = 0, item_it = 0;
+      bool alive = true;
+      for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+        int b, h, i, j0;
+        locate(item, b, h, i, j0);
+        const int row = b * p.n_i + i;
+        const uint32_t qb = item_it % C::QBUF;
+        alive = alive && mbar_wait(&sm.q_empty[qb], ((item_it / C::QBUF) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER);
+        __syncwarp();
+        if (leader && alive) {
+          mbar_expect_tx(&sm.q_full[qb], NWG * C::Q_BYTES);
+          for (int g = 0; g < NWG; ++g) tma_load_5d(sm.q[qb][g], &tm.q, &sm.q_full[qb], 0, h, j0, row + g, 0);
+        }
+        for (int t = 0; t < p.steps; ++t) {
+          alive = alive && mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER);
+          __syncwarp();
+          const int k0 = t * KT;
+          if (leader && alive) {
+            mbar_expect_tx(&sm.st_full[stage], C::STAGE_TX);
+            tma_load_4d(sm.bias[stage], &tm.b, &sm.st_full[stage], k0, j0, h, b);
+            for (int g = 0; g < NWG; ++g) {
+              tma_load_5d(sm.k[stage][g], &tm.k, &sm.st_full[stage], 0, h, k0, row + g, 0);
+              tma_load_2d(sm.mb[stage][g], &tm.m, &sm.st_full[stage], k0, row + g);
+              tma_load_5d(sm.v[stage][g], &tm.v, &sm.st_full[stage], k0, 0, h, row + g, 0);
+            }
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    } else if (warp <= C::ISSUERS) {
+      const bool leader = elect_one();
+      const int r0 = (warp - 1) * C::ROWS;
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, KT), idesc_o = umma_idesc_bf16(128, HDP);
+      const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
+      bool alive = true;
+      // scores of a row's step in stage `st`, queries in buffer `qb`
+      auto scores = [&](int wg, int st, int qb) {
+        const uint32_t d = tmem_base + wg * C::TM_WG;
+        const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[st]), 128);
+        const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[qb][wg]), HDP * 2);
+        const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.k[st][wg]), HDP * 2);
+        if (leader && alive) {
+#pragma unroll
+          for (int kk = 0; kk < KT / 16; ++kk)
+            umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_s, kk != 0);
+#pragma unroll
+          for (int kk = 0; kk < HDP / 16; ++kk)
+            umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc_s, 1);
+          umma_commit(&sm.s_full[wg]);
+        }
+      };
+      int stage = 0, next_qb = 0;          // stage of the step whose P.V comes next, queries of the one after
+      uint32_t phase = 0, item_it = 0, g = 0;  // g: steps so far
+      if (blockIdx.x < p.total_items) {    // the first step's scores
+        alive = mbar_wait(&sm.q_full[0], 0, p.status, ST_TIMEOUT_MMA) && mbar_wait(&sm.st_full[0], 0, p.status, ST_TIMEOUT_MMA);
+        __syncwarp();
+        tc_fence_after();
+        for (int u = 0; u < C::ROWS; ++u) scores(r0 + u, 0, 0);
+        if (p.steps == 1 && leader && alive) umma_commit(&sm.q_empty[0]);
+      }
+      for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+        for (int t = 0; t < p.steps; ++t, ++g) {
+          const bool last = t + 1 == p.steps, more = !last || item + gridDim.x < p.total_items;
+          const int next = stage + 1 == STAGES ? 0 : stage + 1;
+          const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
+          if (last) next_qb ^= 1;
+#pragma unroll 1
+          for (int u = 0; u < C::ROWS; ++u) {
+            const int wg = r0 + u;
+            alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
+            if (u == 0 && more) {
+              alive = alive && mbar_wait(&sm.st_full[next], next_phase, p.status, ST_TIMEOUT_MMA);
+              if (last)
+                alive = alive && mbar_wait(&sm.q_full[next_qb], ((item_it + 1) / C::QBUF) & 1, p.status, ST_TIMEOUT_MMA);
+            }
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t base = tmem_base + wg * C::TM_WG;
+            const uint64_t vdesc = umma_desc_kmajor(smem_u32(sm.v[stage][wg]), 128);
+            if (leader && alive) {
+#pragma unroll
+              for (int term = 0; term < TP::N; ++term)
+#pragma unroll
+                for (int kk = 0; kk < KT / 16; ++kk)
+                  umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
+                               idesc_o, t > 0 || (term | kk) != 0);
+              if (last) umma_commit(&sm.o_full[wg]);
+            }
+            if (more) scores(wg, next, next_qb);
+          }
+          if (leader && alive) {
+            umma_commit(&sm.st_empty[stage]);
+            // the last product with a buffer of queries has been issued: that of its item's last step
+            if (t + 2 == p.steps || (p.steps == 1 && more)) umma_commit(&sm.q_empty[next_qb]);
+          }
+          stage = next;
+          phase = next_phase;
+        }
+      }
+    }
+  } else {
+    if (NWG > 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::SOFTMAX_REGS));
+    const int wg = (warp - 4) >> 2, quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    const uint32_t t_wg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + wg * C::TM_WG;
+    int stage = 0;
+    uint32_t phase = 0, g = 0, item_it = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+      float m_run = -INFINITY, l_run = 0.f;
+      for (int t = 0; t < p.steps; ++t, ++g) {
+        const bool st_there = mbar_test(&sm.st_full[stage], phase), s_there = mbar_test(&sm.s_full[wg], g & 1);
+        alive = (st_there || mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX)) &&
+                (s_there || mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX));
+        if (!__all_sync(0xffffffffu, alive)) {
+          alive = false;
+          break;
+        }
+        tc_fence_after();
+        const float mk0 = sm.mb[stage][wg][lane], mk1 = sm.mb[stage][wg][lane + 32];
+        float2 s[KT / 2];
+        {
+          uint32_t r0[32], r1[32];
+          tmem_ld32(t_wg, r0);
+          tmem_ld32(t_wg + 32, r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            s[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
+            s[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
+          }
+        }
+        if (__any_sync(0xffffffffu, mk0 != 0.f || mk1 != 0.f)) {
+          const float* mrow = sm.mb[stage][wg];
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
+            s[2 * c] = __fadd2_rn(s[2 * c], make_float2(m4.x, m4.y));
+            s[2 * c + 1] = __fadd2_rn(s[2 * c + 1], make_float2(m4.z, m4.w));
+            if ((c & 3) == 3) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
+        float mxa = fmaxf(s[0].x, s[0].y), mxb = fmaxf(s[1].x, s[1].y);
+        float mxc = fmaxf(s[2].x, s[2].y), mxd = fmaxf(s[3].x, s[3].y);
+#pragma unroll
+        for (int e = 4; e < KT / 2; e += 4) {
+          mxa = fmax3(mxa, s[e].x, s[e].y);
+          mxb = fmax3(mxb, s[e + 1].x, s[e + 1].y);
+          mxc = fmax3(mxc, s[e + 2].x, s[e + 2].y);
+          mxd = fmax3(mxd, s[e + 3].x, s[e + 3].y);
+        }
+        const float mx = fmaxf(fmaxf(mxa, mxb), fmaxf(mxc, mxd));
+        const bool need = mx - m_run > RESCALE;  // true on the first step
+        if (__any_sync(0xffffffffu, need)) {     // the offset moves only where the maximum grew a lot
+          float scale = 1.0f;
+          if (need) {
+            const float off = rintf(m_run * LOG2E), off_new = rintf(mx * LOG2E);
+            // (0 on the first step; beyond integers, offsets are the maxima themselves)
+            scale = fast_exp2(fminf(fabsf(off), fabsf(off_new)) < INTEGER_OFFSETS ? off - off_new : (m_run - mx) * LOG2E);
+            m_run = mx;
+            l_run *= scale;
+          }
+          __syncwarp();
+          if (t > 0) {
+#pragma unroll
+            for (int part = 0; part < HDP / 16; ++part) {
+              uint32_t r[16];
+              tmem_ld16(t_wg + C::TM_O + part * 16, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * scale);
+              tmem_st16(t_wg + C::TM_O + part * 16, r);
+            }
+          }
+        }
+        // e^(s - m) = 2^(s log2e - offset): the product is exact in the fma and the offset an integer
+        float minus_off = -rintf(m_run * LOG2E);
+        if (__any_sync(0xffffffffu, fabsf(minus_off) >= INTEGER_OFFSETS)) {
+          float2 minus_m = make_float2(0.f, 0.f);
+          if (fabsf(minus_off) >= INTEGER_OFFSETS) {
+            minus_m = make_float2(-m_run, -m_run);
+            minus_off = 0.f;
+          }
+#pragma unroll
+          for (int e = 0; e < KT / 2; ++e) s[e] = __fadd2_rn(s[e], minus_m);
+          __syncwarp();
+        }
+        const float2 log2e2 = make_float2(LOG2E, LOG2E), off2 = make_float2(minus_off, minus_off);
+        float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int half = 0; half < 4; ++half) {
+          uint32_t pc[3][8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float2 x = __ffma2_rn(s[half * 8 + e], log2e2, off2);
+            const float2 w = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+            l2[e & 1] = __fadd2_rn(l2[e & 1], w);
+            split3n2(w, pc[0][e], pc[1][e], pc[2][e]);
+          }
+#pragma unroll
+          for (int q = 0; q < 3; ++q) tmem_st8(t_wg + C::TM_P + q * 32 + half * 8, pc[q]);
+        }
+        l_run += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.p_full[wg]);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      alive = alive && mbar_wait(&sm.o_full[wg], item_it & 1, p.status, ST_TIMEOUT_SOFTMAX);
+      if (!__all_sync(0xffffffffu, alive)) break;
+      tc_fence_after();
+      int b, h, i, j0;
+      locate(item, b, h, i, j0);
+      i += wg;
+      const int j = j0 + row;
+      const bool live = i < p.n_i && j < p.n;
+      __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.o) +
+                           ((static_cast<long long>(b * p.n_i + i) * p.n + j) * p.heads + h) * p.head_dim;
+      const float inv = 1.0f / l_run;
+#pragma unroll
+      for (int part = 0; part < HDP / 16; ++part) {
+        __syncwarp();
+        uint32_t r[16];
+        tmem_ld16(t_wg + C::TM_O + part * 16, r);
+        tmem_ld_wait();
+        if (!live) continue;
+        uint4 w[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          uint32_t u[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            u[e] = pack_bf16x2(__uint_as_float(r[8 * q + 2 * e]) * inv, __uint_as_float(r[8 * q + 2 * e + 1]) * inv);
+          w[q] = make_uint4(u[0], u[1], u[2], u[3]);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(out + part * 16);
+        if (p.head_dim % 16 == 0 && part * 16 < p.head_dim) {
+          store_sector(dst, w[0], w[1]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (part * 16 + q * 8 < p.head_dim) dst[q] = w[q];
+        }
+      }
+      __syncwarp();
+      tc_fence_before();
+    }
+  }
+
+  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
+template <int HDP, int NWG>
+int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
+  using C = BfCfg<HDP, NWG>;
+  p.groups = (p.n_i + NWG - 1) / NWG;
+  p.tiles_j = (p.n + 127) / 128;
+  const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
+  B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "attention: too many tiles");
+  p.total_items = static_cast<uint32_t>(items);
+  const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_bf16_kernel<HDP, NWG>), (int)sizeof(BfSmem<HDP, NWG>));
+  if (rc) return rc;
+  const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
+  return launch(att_bf16_kernel<HDP, NWG>, dim3(grid), dim3(C::THREADS), sizeof(BfSmem<HDP, NWG>), stream, pdl, tm, p);
+}
+
+// Rows of an item. A step of four takes 1.2 times as long as one of three (2.66 and 2.2 us), which pays
+// unless as many rounds of items are needed: 12 heads x 100 tokens, attention 63.4 us with four and 59.8 with three
+// (three rounds either way), 4 x 4 heads x 200 tokens 193 and 207 (11 and 15 rounds).
+int launch_bf16_narrow(const Maps& tm, const Params& p, bool pdl, cudaStream_t stream) {
+  auto rounds = [&](int rows) {
+    const long long items = static_cast<long long>(p.total_items) * ((p.n_i + rows - 1) / rows) * ((p.n + 127) / 128);
+    return (items + sm_count() - 1) / sm_count();
+  };
+  return 5 * rounds(3) < 6 * rounds(4) ? launch_bf16<32, 3>(tm, p, pdl, stream) : launch_bf16<32, 4>(tm, p, pdl, stream);
 }
 
 }  // namespace
@@ -586,9 +934,9 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   p.pieces = a.pieces;
   p.status = device_status_word();
   B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "float32 attention: no current CUDA device");
-  if (token) return launch_cfg<32, 3, true>(tm, p, a.pdl, stream);
-  if (a.bf16) return hdp == 32 ? launch_cfg<32, 1, false>(tm, p, a.pdl, stream) : launch_cfg<64, 1, false>(tm, p, a.pdl, stream);
-  return hdp == 32 ? launch_cfg<32, 3, false>(tm, p, a.pdl, stream) : launch_cfg<64, 3, false>(tm, p, a.pdl, stream);
+  if (token) return launch_cfg<32, true>(tm, p, a.pdl, stream);
+  if (a.bf16) return hdp == 32 ? launch_bf16_narrow(tm, p, a.pdl, stream) : launch_bf16<64, 2>(tm, p, a.pdl, stream);
+  return hdp == 32 ? launch_cfg<32, false>(tm, p, a.pdl, stream) : launch_cfg<64, false>(tm, p, a.pdl, stream);
 }
 
 }  // namespace b200
