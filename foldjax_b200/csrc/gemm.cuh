@@ -189,6 +189,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
   tc_fence_after();
   pdl_wait();
   pdl_trigger();
+  int status = -1;
   const uint32_t tmem_base = tmem_base_s;
   // (32-bit tile arithmetic: a 64-bit division costs a role several hundred cycles per tile)
   const uint32_t total = static_cast<uint32_t>(g.m_tiles) * g.n_tiles * g.splits;
@@ -293,7 +294,10 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
       const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
       typename P::Pre pre;
       P::prefetch(ep, m_tile, n_tile, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
-      if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) break;
+      if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) {
+        status = -1;
+        break;
+      }
       tc_fence_after();
       Accum<P> acc;
       acc.base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
@@ -302,6 +306,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
         const int per = (g.kb[seg] + g.splits - 1) / g.splits;
         acc.used[seg] = min(g.kb[seg], (split + 1) * per) - split * per;
       }
+      status = ask_status(g.status);  // (arrives during the epilogue)
       P::epilogue(ep, m_tile, n_tile, split, acc, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
       tc_fence_before();
       __syncwarp();
@@ -309,8 +314,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
     }
   }
 
-  if (*reinterpret_cast<volatile int*>(g.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, g.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
@@ -399,6 +403,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
   tc_fence_after();
   pdl_wait();
   pdl_trigger();
+  int status = -1;
   const uint32_t tmem_base = tmem_base_s;
   auto locate = [&](uint32_t unit, int& slow, int& f0, int& f1) {
     const uint32_t s = unit / static_cast<uint32_t>(runs.parts), part = unit - s * runs.parts;
@@ -518,6 +523,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
         P::prefetch(ep, m_tile, n_tile, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
         if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) {
           alive = false;
+          status = -1;
           break;
         }
         tc_fence_after();
@@ -525,6 +531,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
         acc.base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
 #pragma unroll
         for (int seg = 0; seg < P::NSEG; ++seg) acc.used[seg] = kbs;
+        status = ask_status(g.status);  // (arrives during the epilogue)
         P::epilogue(ep, m_tile, n_tile, 0, acc, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
         tc_fence_before();
         __syncwarp();
@@ -533,8 +540,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
     }
   }
 
-  if (*reinterpret_cast<volatile int*>(g.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, g.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);

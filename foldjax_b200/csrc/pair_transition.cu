@@ -157,7 +157,15 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
+  int status = -1;
+  auto load_x = [&](uint32_t xs, uint32_t tile) {
+    const int r0 = static_cast<int>(tile * 128u);
+    mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
+    tma_load_2d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, r0);
+    tma_load_2d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, r0);
+  };
   if (p.early_weights) pdl_wait();
+  if (threadIdx.x == 0) load_x(0, blockIdx.x);  // right behind the wait
   pdl_trigger();
   // TMEM: D1 (the chunk's [a | b], 128 columns) double-buffered at 0 and 128;
   // OUT (128 columns) double-buffered over tiles at 256 and 384.
@@ -177,13 +185,10 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     }
   } else if (warp == 2) {
     if (elect_one()) {
-      for (uint32_t it = 0; it < n_my; ++it) {
+      for (uint32_t it = 1; it < n_my; ++it) {
         const uint32_t xs = it % XSTAGES;
         if (!mbar_wait(&sm.x_empty[xs], ((it / XSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        const int r0 = static_cast<int>((blockIdx.x + it * gridDim.x) * 128u);
-        mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
-        tma_load_2d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, r0);
-        tma_load_2d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, r0);
+        load_x(xs, blockIdx.x + it * gridDim.x);
       }
     }
   } else if (warp == 1) {
@@ -316,7 +321,7 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.out_empty[tb]);
     }
-    if (lane == 0) tma_store_wait_all();
+    status = stores_read_and_status(lane == 0, p.status);
   } else if (warp >= 12) {
     // ---- activation: 32 columns of a and of b -> 32 hidden values, 16 at a time
     const int quarter = warp & 3, row = quarter * 32 + lane;  // pair inside the tile = TMEM lane
@@ -352,8 +357,7 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     }
   }
 
-  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);

@@ -186,8 +186,26 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Until the stores committed so far have READ their shared-memory source (it may be reused).
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// Until the stores committed so far are complete (written and visible).
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// The end of a kernel that stores by TMA. The device status word is asked for while the last stores read their
+// tiles (a trip to L2 on its own otherwise, 0.3 us of a launch of one tile per SM); the grid is complete when they
+// are written, so nothing waits for that here. Nothing that can give up on a wait follows in the warp.
+__device__ __forceinline__ int ask_status(const int* status) {
+  int st;
+  asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(st) : "l"(status) : "memory");
+  return st;
+}
+__device__ __forceinline__ int stores_read_and_status(bool stored, const int* status) {
+  const int st = ask_status(status);
+  if (stored) tma_store_wait_read();
+  return st;
+}
+// Tear-down of a warp: `status` as it was asked for, or -1. After a timeout (of this warp, or of another: that
+// one comes here too, and they meet at a barrier next) give in-flight bulk copies time to land first.
+__device__ __forceinline__ void settle(int status, const int* word) {
+  if ((status >= 0 ? status : *reinterpret_cast<const volatile int*>(word)) != ST_OK)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+}
 
 // ---------------------------------------------------------------- TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_in_smem, uint32_t ncols) {

@@ -113,8 +113,7 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
   // TMEM: buffer a (= tile parity): G at a*256, OUT at a*256 + 128.
-  if (p.early_weights) pdl_wait();
-  pdl_trigger();
+  int status = -1;
 
   // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
   auto locate = [&](uint32_t tile, int& o, int& t0) {
@@ -122,25 +121,39 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     o = q;
     t0 = (tile - q * p.tiles_inner) * 128;
   };
+  auto load_x = [&](int xs, int o, int t0) {
+    mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
+    tma_load_3d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, t0, o);
+    tma_load_3d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, t0, o);
+  };
+  auto load_o = [&](int os, int o, int t0) {
+    mbar_expect_tx(&sm.o_full[os], TILE_BYTES);
+    tma_load_3d(sm.o[os], &tm_o, &sm.o_full[os], 0, t0, o);
+    tma_load_3d(sm.o[os] + SLAB_BYTES, &tm_o, &sm.o_full[os], 64, t0, o);
+  };
+  int first_o, first_t0;  // the first tile, located ahead of the wait and requested right behind it
+  locate(blockIdx.x, first_o, first_t0);
+  if (p.early_weights) pdl_wait();
+  if (threadIdx.x == 0) {
+    load_x(0, first_o, first_t0);
+    load_o(0, first_o, first_t0);
+  }
+  pdl_trigger();
   const uint32_t n_my = blockIdx.x < p.total_tiles ? (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
 
   // 512 threads x 128 registers = 128 x (72 + 144 + 128 + 168)
   if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     if (elect_one()) {
-      uint32_t it = 0;
-      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+      uint32_t it = 1;  // (the first tile is on its way)
+      for (uint32_t tile = blockIdx.x + gridDim.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
         int o, t0;
         locate(tile, o, t0);
         const uint32_t xs = it % XSTAGES, os = it % OSTAGES;
         if (!mbar_wait(&sm.x_empty[xs], ((it / XSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.x_full[xs], TILE_BYTES);
-        tma_load_3d(sm.x[xs], &tm_x, &sm.x_full[xs], 0, t0, o);
-        tma_load_3d(sm.x[xs] + SLAB_BYTES, &tm_x, &sm.x_full[xs], 64, t0, o);
+        load_x(xs, o, t0);
         if (!mbar_wait(&sm.o_empty[os], ((it / OSTAGES) & 1) ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.o_full[os], TILE_BYTES);
-        tma_load_3d(sm.o[os], &tm_o, &sm.o_full[os], 0, t0, o);
-        tma_load_3d(sm.o[os] + SLAB_BYTES, &tm_o, &sm.o_full[os], 64, t0, o);
+        load_o(os, o, t0);
       }
     }
   } else if (warp == 1) {
@@ -298,11 +311,10 @@ att_finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         mbar_arrive(&sm.o_empty[it % OSTAGES]);
       }
     }
-    if (lane == 0) tma_store_wait_all();
+    status = stores_read_and_status(lane == 0, p.status);
   }
 
-  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);

@@ -94,8 +94,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();
-  pdl_trigger();
+  int status = -1;
   const uint32_t tmem_base = tmem_base_s;
 
   const int k_iters = p.n_src * p.kb_per_src;
@@ -108,22 +107,31 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     nj = rem - mi * p.tiles_n;
   };
 
+  // where the producer finds a tile's operands: the first one's worked out ahead of the wait
+  int src_d, a_block[H], a_row[H], b_block, b_row;
+  auto origin = [&](uint32_t tile) {
+    int mi, nj;
+    locate(tile, src_d, mi, nj);
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int row = (mi * H + h) * BM;
+      a_block[h] = row / p.a_rpb;
+      a_row[h] = row - a_block[h] * p.a_rpb;
+    }
+    b_block = nj * BN / p.b_rpb;
+    b_row = nj * BN - b_block * p.b_rpb;
+  };
+  if (warp == 0) origin(blockIdx.x);
+  pdl_wait();
+  pdl_trigger();
+
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
       for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x) {
-        int d, mi, nj;
-        locate(tile, d, mi, nj);
-        int a_block[H], a_row[H];
-#pragma unroll
-        for (int h = 0; h < H; ++h) {
-          const int row = (mi * H + h) * BM;
-          a_block[h] = row / p.a_rpb;
-          a_row[h] = row - a_block[h] * p.a_rpb;
-        }
-        const int b_block = nj * BN / p.b_rpb, b_row = nj * BN - b_block * p.b_rpb;
+        if (tile != blockIdx.x) origin(tile);
         for (int s = 0; s < p.n_src && alive; ++s) {
           for (int kb = 0; kb < p.kb_per_src; ++kb) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) {
@@ -135,9 +143,9 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             // rows are (block, row in block): a tile starts at block row0 / rpb
 #pragma unroll
             for (int h = 0; h < H; ++h)
-              tma_load_5d(sa + h * A_BYTES, &tm_a, &full_bar[stage], kb * BK, a_row[h], a_block[h], d,
+              tma_load_5d(sa + h * A_BYTES, &tm_a, &full_bar[stage], kb * BK, a_row[h], a_block[h], src_d,
                           p.terms.n ? p.terms.a[s] : s);
-            tma_load_5d(sa + H * A_BYTES, &tm_b, &full_bar[stage], kb * BK, b_row, b_block, d,
+            tma_load_5d(sa + H * A_BYTES, &tm_b, &full_bar[stage], kb * BK, b_row, b_block, src_d,
                         p.terms.n ? p.terms.b[s] : s);
             if (++stage == STAGES) {
               stage = 0;
@@ -328,12 +336,10 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
     }
-    if (lane == 0) tma_store_wait_all();
+    status = stores_read_and_status(lane == 0, p.status);
   }
 
-  // Tear-down. After a timeout give in-flight bulk copies time to land first.
-  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);

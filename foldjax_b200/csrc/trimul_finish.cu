@@ -116,8 +116,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
-  if (p.early_weights) pdl_wait();
-  pdl_trigger();
+  int status = -1;
 
   // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
   auto locate = [&](uint32_t tile, int& i, int& j0) {
@@ -125,23 +124,32 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     i = q;
     j0 = (tile - q * p.tiles_j) * 128;
   };
+  auto load_in = [&](int stage, int i, int j0, int block, int in_block) {
+    mbar_expect_tx(&sm.in_full[stage], 2 * TILE_BYTES);
+    tma_load_3d(sm.x[stage], &tm_x, &sm.in_full[stage], 0, j0, i);
+    tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.in_full[stage], 64, j0, i);
+    for (int half = 0; half < 2; ++half)
+      tma_load_4d(sm.t[stage] + half * SLAB_BYTES, &tm_t, &sm.in_full[stage], j0 + half * 64, in_block, 0, block);
+  };
+  int first_i, first_j0;  // the first tile, located ahead of the wait and requested right behind it
+  locate(blockIdx.x, first_i, first_j0);
+  const int first_block = first_i / p.t_rpb;
+  if (p.early_weights) pdl_wait();
+  if (threadIdx.x == 0) load_in(0, first_i, first_j0, first_block, first_i - first_block * p.t_rpb);
+  pdl_trigger();
 
   // 640 threads x 96 registers = 128 x (48 + 80 + 144 + 2 x 104)
   if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
+      int stage = 1;  // (stage 0 has the first tile)
       uint32_t phase = 0;
-      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+      for (uint32_t tile = blockIdx.x + gridDim.x; tile < p.total_tiles; tile += gridDim.x) {
         int i, j0;
         locate(tile, i, j0);
+        const int block = i / p.t_rpb;
         if (!mbar_wait(&sm.in_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.in_full[stage], 2 * TILE_BYTES);
-        tma_load_3d(sm.x[stage], &tm_x, &sm.in_full[stage], 0, j0, i);
-        tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.in_full[stage], 64, j0, i);
-        const int block = i / p.t_rpb, in_block = i - block * p.t_rpb;
-        for (int half = 0; half < 2; ++half)
-          tma_load_4d(sm.t[stage] + half * SLAB_BYTES, &tm_t, &sm.in_full[stage], j0 + half * 64, in_block, 0, block);
+        load_in(stage, i, j0, block, i - block * p.t_rpb);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;
@@ -293,11 +301,10 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
       }
       if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
     }
-    if (leader) tma_store_wait_all();
+    status = stores_read_and_status(leader, p.status);
   }
 
-  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);

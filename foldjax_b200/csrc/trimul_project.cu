@@ -124,8 +124,7 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
-  if (p.early_weights) pdl_wait();
-  pdl_trigger();
+  int status = -1;
 
   // (32-bit: a 64-bit division costs a role hundreds of cycles per tile)
   auto locate = [&](uint32_t tile, int& o, int& t0) {
@@ -133,18 +132,26 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     o = q;
     t0 = (tile - q * p.tiles_inner) * 128;
   };
+  auto load_x = [&](int stage, int o, int t0) {
+    mbar_expect_tx(&sm.x_full[stage], TILE_BYTES);
+    tma_load_3d(sm.x[stage], &tm_x, &sm.x_full[stage], 0, t0, o);
+    tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.x_full[stage], 64, t0, o);
+  };
+  int first_o, first_t0;  // the first tile, located ahead of the wait and requested right behind it
+  locate(blockIdx.x, first_o, first_t0);
+  if (p.early_weights) pdl_wait();
+  if (threadIdx.x == 0) load_x(0, first_o, first_t0);
+  pdl_trigger();
 
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
+      int stage = 1;  // (stage 0 has the first tile)
       uint32_t phase = 0;
-      for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+      for (uint32_t tile = blockIdx.x + gridDim.x; tile < p.total_tiles; tile += gridDim.x) {
         int o, t0;
         locate(tile, o, t0);
         if (!mbar_wait(&sm.x_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&sm.x_full[stage], TILE_BYTES);
-        tma_load_3d(sm.x[stage], &tm_x, &sm.x_full[stage], 0, t0, o);
-        tma_load_3d(sm.x[stage] + SLAB_BYTES, &tm_x, &sm.x_full[stage], 64, t0, o);
+        load_x(stage, o, t0);
         if (++stage == XSTAGES) {
           stage = 0;
           phase ^= 1;
@@ -278,11 +285,10 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         if (lane == 0) mbar_arrive(&sm.acc_empty[half]);
       }
     }
-    if (leader) tma_store_wait_all();
+    status = stores_read_and_status(leader, p.status);
   }
 
-  if (*reinterpret_cast<volatile int*>(p.status) != ST_OK)
-    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  settle(status, p.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);
