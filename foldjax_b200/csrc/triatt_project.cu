@@ -27,10 +27,12 @@
 //               vT = Wv.xn^T ("transposed": a TMEM lane is a channel)
 //   warps 2-9   layer norm in place (two threads per pair)
 //   warps 10-17 epilogue: one warpgroup per 64 channels of q and k and per 64 pairs of vT, each
-//               with a staging slab and TMA stores of its own
+//               with a staging slab, of which a warp fills and stores 32 rows
 // TMEM: [q|k] 256 columns, vT 128, bias 16; each group is released on its own
 // so the next tile's MMAs overlap this tile's epilogue.
-// Bound: HBM (read x, write q, k, vT: 4 * n*n*128*2 bytes).
+// Bound: HBM (read x, write q, k, vT: 4 * n*n*128*2 bytes). By events around the launch, n = 200 / 512 / 1003:
+// 19.0 / 54.5 / 187 us with a store per warpgroup, behind two barriers and the read of the store before;
+// 16.9 / 52.0 / 183 with one per warp, whose read is waited for while the accumulators are fetched.
 #include <cuda_fp16.h>
 
 #include "host.cuh"
@@ -252,16 +254,18 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   } else {
     const int quarter = warp & 3, group = (warp - 2 - LN_WARPS) >> 2;
     const int row = quarter * 32 + lane;  // TMEM lane: a pair for q/k/bias, a channel for vT
-    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     uint8_t* out = sm.out + group * SLAB_BYTES;
     const uint32_t qs = pack_bf16x2(p.q_scale, p.q_scale);
     const float q_inv = 1.0f / bf16_lo(qs);
     uint32_t it = 0;
-    // (votes: the outcome of each bounded wait is made the same for the warpgroup's 128 threads,
-    // which meet at named barriers around its staging slab)
+    // (a vote: TMEM accesses take the whole warp. Each warp stages and stores its own 32 rows)
     auto acc_wait = [&](int g) {
-      return named_barrier_and(1 + group, 128, mbar_wait(&sm.acc_full[g], it & 1, p.status, ST_TIMEOUT_EPILOGUE));
+      return __all_sync(0xffffffffu, mbar_wait(&sm.acc_full[g], it & 1, p.status, ST_TIMEOUT_EPILOGUE));
+    };
+    auto rows_free = [&] {  // the warp's previous store has read them: asked when there is something to go there
+      if (lane == 0) tma_store_wait_read();
+      __syncwarp();
     };
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
       int o, t0;
@@ -271,12 +275,11 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       tc_fence_after();
 #pragma unroll 1
       for (int part = 0; part < 2; ++part) {  // q, then k
-        if (leader) tma_store_wait_read();
-        named_barrier(1 + group, 128);
 #pragma unroll
         for (int c2 = 0; c2 < 2; ++c2) {
           uint32_t r[32];
           tmem_ld32(lane_addr + TM_QK + part * 128 + group * 64 + c2 * 32, r);
+          if (c2 == 0) rows_free();
           tmem_ld_wait();
 #pragma unroll
           for (int g4 = 0; g4 < 4; ++g4) {
@@ -294,9 +297,9 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
           }
         }
         fence_proxy_async();
-        named_barrier(1 + group, 128);
-        if (leader) {  // pairs past n_inner are outside the tensor and are not written
-          tma_store_3d(part ? &tm_k : &tm_q, out, group * 64, t0, o);
+        __syncwarp();
+        if (lane == 0 && t0 + quarter * 32 < p.n_inner) {  // pairs past n_inner are outside the tensor and are not written
+          tma_store_3d(part ? &tm_k : &tm_q, out + quarter * 4096, group * 64, t0 + quarter * 32, o);
           tma_store_commit();
         }
       }
@@ -321,13 +324,13 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         if (lane == 0) mbar_arrive(&sm.acc_empty[G_B]);
       }
       // ---- vT: thread = channel, 64 pairs -> one contiguous run of the row
-      if (leader) tma_store_wait_read();
       if (!acc_wait(G_V)) break;
       tc_fence_after();
 #pragma unroll
       for (int c2 = 0; c2 < 2; ++c2) {
         uint32_t r[32];
         tmem_ld32(lane_addr + TM_V + group * 64 + c2 * 32, r);
+        if (c2 == 0) rows_free();
         tmem_ld_wait();
 #pragma unroll
         for (int g4 = 0; g4 < 4; ++g4) {
@@ -345,14 +348,14 @@ att_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
       tc_fence_before();
       fence_proxy_async();
-      named_barrier(1 + group, 128);
-      if (leader && t0 + group * 64 < p.n_inner) {
-        tma_store_3d(&tm_vt, out, t0 + group * 64, 0, o);
+      __syncwarp();
+      if (lane == 0 && t0 + group * 64 < p.n_inner) {
+        tma_store_3d(&tm_vt, out + quarter * 4096, t0 + group * 64, quarter * 32, o);
         tma_store_commit();
       }
       if (lane == 0) mbar_arrive(&sm.acc_empty[G_V]);
     }
-    status = stores_read_and_status(leader, p.status);
+    status = stores_read_and_status(lane == 0, p.status);
   }
 
   settle(status, p.status);
@@ -399,19 +402,19 @@ int b200::att_project_launch(const b200tri_triatt_project_args* a, const MaskBia
     in_place = in_place && w[i] == w_in[i];
   }
   CUtensorMap tm_x, tm_w[3], tm_q, tm_k, tm_vt;
-  {  // q and k [n_outer][n_inner][128], written as tiles of [128 pairs][64 channels]
+  {  // q and k [n_outer][n_inner][128], written as tiles of [32 pairs][64 channels]
     const uint64_t dims[3] = {128, (uint64_t)a->n_inner, (uint64_t)a->n_outer};
     const uint64_t str[2] = {256, (uint64_t)a->n_inner * 256};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, 32, 1};
     int rc = make_tmap(&tm_q, a->q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
     rc = make_tmap(&tm_k, a->k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
   }
-  {  // vT [n_outer][128][ld] fp16, written as tiles of [128 channels][64 pairs]
+  {  // vT [n_outer][128][ld] fp16, written as tiles of [32 channels][64 pairs]
     const uint64_t dims[3] = {(uint64_t)a->n_inner, 128, (uint64_t)a->n_outer};
     const uint64_t str[2] = {(uint64_t)a->ld * 2, (uint64_t)a->ld * 2 * 128};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, 32, 1};
     int rc = make_tmap(&tm_vt, a->vt, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
   }

@@ -22,10 +22,12 @@
 // TMEM: 2 x (D1, D2) so the epilogue overlaps the next tile's MMAs.
 //
 // Bound: HBM (read t and x, write out: 3 * n_i*n_j*128*2 bytes; + residual) by the bytes; in fact
-// the layer norms, chains of 192 dependent additions per row beside 900 other instructions: 6700
-// clocks a tile for x, at five warps per scheduler. n = 1024: 247 us with one warpgroup for both
-// layer norms and one thread per row of the residual, 226 so (123 by the bytes). Measured and not
-// better: x in registers (spills), alternate warpgroups per tile, t transposed by ldmatrix.
+// the layer norms, chains of 192 dependent additions per row beside 900 other instructions: the warps of x are
+// at it 97 % of the time (t 68 %, epilogue 77 %), at five warps per scheduler. n = 1024: 247 us with one
+// warpgroup for both layer norms and one thread per row of the residual, 226 with two (123 by the bytes); by events
+// around the launch at n = 1003 258 with four words of x at a time and a store per warpgroup, 248 with eight
+// and a store per warp. Measured and not better: x in registers (spills), two threads per row whose
+// chains follow each other (263), alternate warpgroups per tile, t transposed by ldmatrix.
 #include "host.cuh"
 #include "ln.cuh"
 #include "tc.cuh"
@@ -138,8 +140,9 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   if (threadIdx.x == 0) load_in(0, first_i, first_j0, first_block, first_i - first_block * p.t_rpb);
   pdl_trigger();
 
-  // 640 threads x 96 registers = 128 x (48 + 80 + 144 + 2 x 104)
-  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+  // 640 threads x 96 registers = 128 x (40 + 88 + 144 + 2 x 104)
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
   if (warp == 0) {
     if (elect_one()) {
       int stage = 1;  // (stage 0 has the first tile)
@@ -186,14 +189,15 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         }
       }
     }
-  } else if (warp >= 4 && warp < 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+  }
+  } else if (warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     const int r = threadIdx.x - 128;  // pair of the tile
     int stage = 0;
     uint32_t phase = 0;
     for (uint32_t tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
       if (!mbar_wait(&sm.in_full[stage], phase, p.status, ST_TIMEOUT_PROLOGUE)) break;
-      ln_row_sweeps<4>(sm.x[stage], r, sm.gamma_in, sm.beta_in, p.eps);
+      ln_row_sweeps<8>(sm.x[stage], r, sm.gamma_in, sm.beta_in, p.eps);
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.xn_full[stage]);
@@ -202,7 +206,7 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         phase ^= 1;
       }
     }
-  } else if (warp >= 8 && warp < 12) {
+  } else if (warp < 12) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
     const int r = threadIdx.x - 256;  // pair of the tile
     int stage = 0;
@@ -234,11 +238,10 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
         phase ^= 1;
       }
     }
-  } else if (warp >= 12) {
+  } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const int quarter = warp & 3, half = (warp - 12) >> 2;  // 64 channels per warpgroup
     const int pr = quarter * 32 + lane;  // pair inside the tile = TMEM lane
-    const bool leader = quarter == 0 && lane == 0;  // issues the warpgroup's stores
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * 64;
     uint8_t* stage_out = sm.out + half * SLAB_BYTES;
     uint32_t it = 0;
@@ -255,11 +258,11 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
           res[q] = t + 4 * q < p.n_j ? *reinterpret_cast<const uint4*>(src + static_cast<long long>(t + 4 * q) * p.os_j)
                                       : make_uint4(0u, 0u, 0u, 0u);
       }
-      // the previous tile must have left the staging buffer; the vote makes the outcome of the
-      // bounded wait the same for all 128 threads, which meet at a barrier below
-      if (leader) tma_store_wait_read();
-      if (!named_barrier_and(1 + half, 128, mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE))) break;
+      // (a vote: TMEM accesses take the whole warp. Each warp stages and stores its own 32 pairs)
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.acc_full[acc], acc_phase, p.status, ST_TIMEOUT_EPILOGUE))) break;
       tc_fence_after();
+      if (lane == 0) tma_store_wait_read();  // the previous tile has left them
+      __syncwarp();
 #pragma unroll 1  // (the roles' unrolled code competes for the instruction cache)
       for (int chunk = 0; chunk < 4; ++chunk) {
         uint32_t g[16], o[16];
@@ -294,14 +297,14 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
       }
       tc_fence_before();
       fence_proxy_async();
-      named_barrier(1 + half, 128);
-      if (leader) {  // rows past n_j are outside the tensor and are not written
-        tma_store_3d(&tm_out, stage_out, half * 64, j0, i);
+      __syncwarp();
+      if (lane == 0 && j0 + quarter * 32 < p.n_j) {  // rows past n_j are outside the tensor and are not written
+        tma_store_3d(&tm_out, stage_out + quarter * 4096, half * 64, j0 + quarter * 32, i);
         tma_store_commit();
       }
       if (lane == 0) mbar_arrive(&sm.acc_empty[acc]);
     }
-    status = stores_read_and_status(leader, p.status);
+    status = stores_read_and_status(lane == 0, p.status);
   }
 
   settle(status, p.status);
@@ -347,7 +350,7 @@ extern "C" int b200tri_trimul_finish(const b200tri_trimul_finish_args* a, b200tr
   {
     const uint64_t dims[3] = {128, (uint64_t)a->n_j, (uint64_t)a->n_i};
     const uint64_t str[2] = {(uint64_t)a->os_j * 2, (uint64_t)a->os_i * 2};
-    const uint32_t box[3] = {64, 128, 1};
+    const uint32_t box[3] = {64, 32, 1};
     int rc = make_tmap(&tm_out, a->out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dims, str, box, Swz::B128);
     if (rc) return rc;
   }

@@ -25,7 +25,11 @@
 // Bound: HBM by the bytes (read x once, write a and b once: 3 * n*n*128*2 bytes, 123 us at n = 1024);
 // in fact the MUFU unit, two operations for each of a pair's 256 sigmoids: 74 % busy over the 204 us
 // of a launch at n = 1024 (213 with a warp index the compiler did not know to be uniform, 285 with one
-// epilogue warpgroup that stored each thread's run directly).
+// epilogue warpgroup that stored each thread's run directly). It is not the only bound: the epilogue warps are at it
+// 94 % of the time and the layer norm's 83 %, and what takes work off the MUFU unit or brings the epilogue forward
+// costs the others as much. Measured and not better, by events around the launch at n = 1003 (226 us): the
+// sigmoids' reciprocals on the FMA pipe (two Newton steps, the same bf16 results; 237-245 for half of them, three
+// quarters and all), a store per warp (241), the previous store's read waited for behind the first loads (241).
 #include <type_traits>
 
 #include "host.cuh"
