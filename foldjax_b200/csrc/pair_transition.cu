@@ -130,10 +130,8 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     tmem_relinquish();
   }
   if (!p.early_weights) pdl_wait();
-  if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
-    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
-  }
+  LnParam ln_param;
+  if (threadIdx.x >= 128 && threadIdx.x < 256) ln_param.request(threadIdx.x < 192 ? p.gamma : p.beta, threadIdx.x & 63);
   const uint32_t nchunks = p.nchunks;
   const uint32_t n_my = (p.total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;  // (the grid is at most total_tiles)
   const uint32_t total_n = n_my * nchunks;                                         // chunk steps of this CTA
@@ -244,6 +242,8 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       }
     }
   } else if (warp >= 4 && warp < 8) {
+    (threadIdx.x < 192 ? sm.gamma2 : sm.beta2)[threadIdx.x & 63] = ln_param.word();
+    named_barrier(1, 128);
     const int row = threadIdx.x - 128;
     for (uint32_t it = 0; it < n_my; ++it) {
       const uint32_t xs = it % XSTAGES;

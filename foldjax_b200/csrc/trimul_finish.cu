@@ -101,13 +101,9 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     tmem_relinquish();
   }
   if (!p.early_weights) pdl_wait();
-  if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    const int q = threadIdx.x - 64;
-    sm.gamma_in[q] = ln_param_pair(p.ln[0], q);
-    sm.beta_in[q] = ln_param_pair(p.ln[1], q);
-    sm.gamma_out[q] = ln_param_pair(p.ln[2], q);
-    sm.beta_out[q] = ln_param_pair(p.ln[3], q);
-  }
+  LnParam ln_param;
+  if (threadIdx.x >= 128 && threadIdx.x < 384) 
+    ln_param.request(threadIdx.x < 192 ? p.ln[0] : threadIdx.x < 256 ? p.ln[1] : threadIdx.x < 320 ? p.ln[2] : p.ln[3], threadIdx.x & 63);
   if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
     mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
     for (int g = 0; g < 2; ++g)
@@ -192,6 +188,8 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    (threadIdx.x < 192 ? sm.gamma_in : sm.beta_in)[threadIdx.x & 63] = ln_param.word();
+    named_barrier(1, 128);
     const int r = threadIdx.x - 128;  // pair of the tile
     int stage = 0;
     uint32_t phase = 0;
@@ -208,6 +206,8 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     }
   } else if (warp < 12) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    (threadIdx.x < 320 ? sm.gamma_out : sm.beta_out)[threadIdx.x & 63] = ln_param.word();
+    named_barrier(2, 128);
     const int r = threadIdx.x - 256;  // pair of the tile
     int stage = 0;
     uint32_t phase = 0;

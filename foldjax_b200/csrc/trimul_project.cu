@@ -114,10 +114,8 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     tmem_relinquish();
   }
   if (!p.early_weights) pdl_wait();
-  if (threadIdx.x >= 64 && threadIdx.x < 128) {
-    sm.gamma2[threadIdx.x - 64] = ln_param_pair(p.gamma, threadIdx.x - 64);
-    sm.beta2[threadIdx.x - 64] = ln_param_pair(p.beta, threadIdx.x - 64);
-  }
+  LnParam ln_param;
+  if (threadIdx.x >= 64 && threadIdx.x < 192) ln_param.request(threadIdx.x < 128 ? p.gamma : p.beta, threadIdx.x & 63);
   if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
     mbar_expect_tx(&sm.w_full, W_BYTES);
     for (int g = 0; g < 4; ++g)
@@ -199,6 +197,8 @@ project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     }
   } else if (warp < 2 + LN_WARPS) {
     // ---- layer norm, two threads per pair of the tile (lanes l and l ^ 16)
+    if (threadIdx.x < 192) (threadIdx.x < 128 ? sm.gamma2 : sm.beta2)[threadIdx.x & 63] = ln_param.word();
+    named_barrier(1 + EPI_WARPS / 4, LN_WARPS * 32);
     const int r = (warp - 2) * 16 + (lane & 15);
     int stage = 0;
     uint32_t phase = 0, it = 0;
