@@ -10,7 +10,6 @@ another implementation.
 
 from __future__ import annotations
 
-import ctypes as C
 from typing import Any, Mapping
 
 import numpy as np
@@ -96,7 +95,7 @@ def transition_forward(
     args = _lib.pack_pair_transition(rows, C_Z, hidden, float(eps), xd.data_ptr(),
                                      *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(),
                                      dev.aligned_ptr(ws), nbytes, _ptr(md))
-    _lib.check(lib.b200tri_pair_transition(C.byref(args), at[1]))
+    _lib.check(lib.b200tri_pair_transition_packed(args, at[1]))
     if host_in:
         host = out.float().cpu() if numpy_in else out.cpu()
         dev.check_device_status()

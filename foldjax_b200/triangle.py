@@ -9,7 +9,7 @@ falls back to another implementation.
 
 from __future__ import annotations
 
-import ctypes as C
+from functools import lru_cache
 from typing import Any, Mapping
 
 import numpy as np
@@ -41,13 +41,26 @@ def _unfold(t: torch.Tensor, lead: tuple) -> torch.Tensor:
     return t if len(lead) == 1 else t.reshape(tuple(lead) + tuple(t.shape[1:]))
 
 
+def _as_leaf(node: Any, dtype: torch.dtype) -> torch.Tensor:
+    if not isinstance(node, torch.Tensor) or node.dtype is not dtype or not node.is_cuda:
+        node = dev.to_device(node, dtype)
+    return node if node.is_contiguous() else node.contiguous()
+
+
 def _leaf(params: Mapping, *path: str, dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     node: Any = params
     for key in path:
         node = node[key]
-    if not isinstance(node, torch.Tensor) or node.dtype is not dtype or not node.is_cuda:
-        node = dev.to_device(node, dtype)
-    return node if node.is_contiguous() else node.contiguous()
+    return _as_leaf(node, dtype)
+
+
+def _as_leaves(nodes: list, dtype: torch.dtype) -> list[torch.Tensor]:
+    """``_as_leaf`` of each; nearly always they are leaves already, and a call for each takes three times as long as
+    the checks in line."""
+    for node in nodes:
+        if not (isinstance(node, torch.Tensor) and node.dtype is dtype and node.is_cuda and node.is_contiguous()):
+            return [_as_leaf(node, dtype) for node in nodes]
+    return nodes
 
 
 def _check_leaves(leaves: Mapping[str, torch.Tensor], want: Mapping[str, tuple], what: str, where: str) -> None:
@@ -72,13 +85,23 @@ def resolve_dtype(x: Any, dtype: str | None) -> tuple[torch.dtype, int]:
     float32 CUDA tensor and bfloat16 for everything else (host arrays are float32 containers
     of either trunk, so they say nothing). Returns (torch dtype, the C ABI's dtype code)."""
     if dtype is None:
-        dtype = "float32" if isinstance(x, torch.Tensor) and x.is_cuda and x.dtype == torch.float32 else "bfloat16"
+        if isinstance(x, torch.Tensor) and x.is_cuda and x.dtype is torch.float32:
+            return torch.float32, _lib.DTYPE_F32
+        return torch.bfloat16, _lib.DTYPE_BF16
     name = {"bf16": "bfloat16", "fp32": "float32"}.get(str(dtype), str(dtype))
     if name == "bfloat16":
         return torch.bfloat16, _lib.DTYPE_BF16
     if name == "float32":
         return torch.float32, _lib.DTYPE_F32
     raise ValueError(f"Unsupported dtype: {dtype!r} (expected 'bfloat16' or 'float32')")
+
+
+_FIELDS = ("norm_in_scale", "norm_in_bias", "p_in", "g_in", "norm_out_scale", "norm_out_bias", "p_out", "g_out")
+
+
+@lru_cache(maxsize=64)
+def _shapes(c_z: int, c_hidden: int) -> list[tuple]:
+    return [(c_z,), (c_z,), (c_z, 2 * c_hidden), (c_z, 2 * c_hidden), (c_hidden,), (c_hidden,), (c_hidden, c_z), (c_z, c_z)]
 
 
 def triangle_multiplication_forward(
@@ -133,20 +156,14 @@ def triangle_multiplication_forward(
         if isinstance(out, torch.Tensor) and out.numel() == xd.numel() and out.is_contiguous():
             out = out.view(xd.shape) if tuple(out.shape[-3:]) == tuple(xd.shape[-3:]) else out
         dev.check_out(out, xd)
-    leaves = {
-        "norm_in_scale": _leaf(params, "norm_in", "scale", dtype=tdt),
-        "norm_in_bias": _leaf(params, "norm_in", "bias", dtype=tdt),
-        "p_in": _leaf(params, "p_in", "kernel", dtype=tdt),
-        "g_in": _leaf(params, "g_in", "kernel", dtype=tdt),
-        "norm_out_scale": _leaf(params, "norm_out", "scale", dtype=tdt),
-        "norm_out_bias": _leaf(params, "norm_out", "bias", dtype=tdt),
-        "p_out": _leaf(params, "p_out", "kernel", dtype=tdt),
-        "g_out": _leaf(params, "g_out", "kernel", dtype=tdt),
-    }
-    c_hidden = leaves["p_out"].shape[0]
-    want = {"norm_in_scale": (c_z,), "norm_in_bias": (c_z,), "p_in": (c_z, 2 * c_hidden), "g_in": (c_z, 2 * c_hidden),
-            "norm_out_scale": (c_hidden,), "norm_out_bias": (c_hidden,), "p_out": (c_hidden, c_z), "g_out": (c_z, c_z)}
-    _check_leaves(leaves, want, "triangle multiplication", f"c_z = {c_z}, c_hidden = {c_hidden}")
+    norm_in, norm_out = params["norm_in"], params["norm_out"]
+    leaves = _as_leaves([norm_in["scale"], norm_in["bias"], params["p_in"]["kernel"], params["g_in"]["kernel"],
+                         norm_out["scale"], norm_out["bias"], params["p_out"]["kernel"], params["g_out"]["kernel"]], tdt)
+    c_hidden = leaves[6].shape[0]
+    want = _shapes(c_z, c_hidden)
+    if [t.shape for t in leaves] != want:
+        _check_leaves(dict(zip(_FIELDS, leaves)), dict(zip(_FIELDS, want)), "triangle multiplication",
+                      f"c_z = {c_z}, c_hidden = {c_hidden}")
     if c_hidden % 8 or c_hidden > 1024:
         raise ValueError(f"libb200tri takes hidden widths that are multiples of 8 up to 1024; got {c_hidden}")
     nbytes = _lib.workspace_bytes("b200tri_trimul_workspace_bytes_shape", n, code, c_z, c_hidden)
@@ -154,12 +171,11 @@ def triangle_multiplication_forward(
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     at = dev.place()
     ws = dev.workspace(nbytes, "trimul", at)
-    # (the leaves are in the order of the struct's fields)
     args = _lib.pack_trimul(n, int(direction == "incoming"), float(eps), xd.data_ptr(), _ptr(md),
-                            *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
+                            *[v.data_ptr() for v in leaves], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, c_hidden, b)
     if b:  # (an empty batch has an empty result)
-        _lib.check(lib.b200tri_trimul_forward(C.byref(args), at[1]))
+        _lib.check(lib.b200tri_trimul_forward_packed(args, at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()

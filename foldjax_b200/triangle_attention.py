@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+from functools import lru_cache
 from typing import Any, Mapping
 
 import numpy as np
@@ -19,10 +20,18 @@ import torch
 
 from . import _device as dev
 from . import _lib
-from .triangle import C_Z, _check_leaves, _check_pair, _leaf, _pair_mask, _ptr, _unfold, resolve_dtype
+from .triangle import C_Z, _as_leaves, _check_leaves, _check_pair, _pair_mask, _ptr, _unfold, resolve_dtype
 
 HEADS = 4
 HEAD_DIM = 32
+FLOAT_MAX = 3.4028234e38
+
+_FIELDS = ("norm_scale", "norm_bias", "w_bias", "w_q", "w_k", "w_v", "w_g", "w_o")
+
+
+@lru_cache(maxsize=64)
+def _shapes(c_z: int, heads: int, width: int) -> list[tuple]:
+    return [(c_z,), (c_z,), (c_z, heads), (c_z, width), (c_z, width), (c_z, width), (c_z, width), (width, c_z)]
 
 
 def triangle_attention_forward(
@@ -73,22 +82,16 @@ def triangle_attention_forward(
         if isinstance(out, torch.Tensor) and out.numel() == xd.numel() and out.is_contiguous():
             out = out.view(xd.shape) if tuple(out.shape[-3:]) == tuple(xd.shape[-3:]) else out
         dev.check_out(out, xd)
-    leaves = {
-        "norm_scale": _leaf(params, "layer_norm", "scale", dtype=tdt),
-        "norm_bias": _leaf(params, "layer_norm", "bias", dtype=tdt),
-        "w_bias": _leaf(params, "linear", "kernel", dtype=tdt),
-        "w_q": _leaf(params, "mha", "linear_q", "kernel", dtype=tdt),
-        "w_k": _leaf(params, "mha", "linear_k", "kernel", dtype=tdt),
-        "w_v": _leaf(params, "mha", "linear_v", "kernel", dtype=tdt),
-        "w_g": _leaf(params, "mha", "linear_g", "kernel", dtype=tdt),
-        "w_o": _leaf(params, "mha", "linear_o", "kernel", dtype=tdt),
-    }
-    heads = leaves["w_bias"].shape[-1]
-    width = leaves["w_g"].shape[-1]
+    norm, mha = params["layer_norm"], params["mha"]
+    leaves = _as_leaves([norm["scale"], norm["bias"], params["linear"]["kernel"], mha["linear_q"]["kernel"], mha["linear_k"]["kernel"],
+                         mha["linear_v"]["kernel"], mha["linear_g"]["kernel"], mha["linear_o"]["kernel"]], tdt)
+    heads = leaves[2].shape[-1]
+    width = leaves[6].shape[-1]
     head_dim = width // max(heads, 1)
-    want = {"norm_scale": (c_z,), "norm_bias": (c_z,), "w_bias": (c_z, heads), "w_q": (c_z, width), "w_k": (c_z, width),
-            "w_v": (c_z, width), "w_g": (c_z, width), "w_o": (width, c_z)}
-    _check_leaves(leaves, want, "triangle attention", f"c_z = {c_z}, {heads} heads x {head_dim}")
+    want = _shapes(c_z, heads, width)
+    if [t.shape for t in leaves] != want:
+        _check_leaves(dict(zip(_FIELDS, leaves)), dict(zip(_FIELDS, want)), "triangle attention",
+                      f"c_z = {c_z}, {heads} heads x {head_dim}")
     if heads * head_dim != width or head_dim not in (8, 16, 24, 32, 48, 64):
         raise ValueError(f"libb200tri takes head widths 8, 16, 24, 32, 48 and 64; got {heads} heads over {width} channels")
     nbytes = _lib.workspace_bytes("b200tri_triatt_workspace_bytes_shape", n, code, c_z, heads, head_dim)
@@ -96,12 +99,13 @@ def triangle_attention_forward(
         nbytes = dev.batch_bytes(nbytes, b)  # the general path takes several items per launch
     at = dev.place()
     ws = dev.workspace(nbytes, "triatt", at)
-    # (the leaves are in the order of the struct's fields)
-    args = _lib.pack_triatt(n, int(bool(starting)), heads, head_dim, C.c_float(inf).value, float(eps), xd.data_ptr(), _ptr(md),
-                            *[v.data_ptr() for v in leaves.values()], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
+    if not -FLOAT_MAX < inf < FLOAT_MAX:
+        inf = C.c_float(inf).value
+    args = _lib.pack_triatt(n, int(bool(starting)), heads, head_dim, inf, float(eps), xd.data_ptr(), _ptr(md),
+                            *[v.data_ptr() for v in leaves], _ptr(rd), out.data_ptr(), dev.aligned_ptr(ws),
                             nbytes, code, c_z, b)
     if b:  # (an empty batch has an empty result)
-        _lib.check(lib.b200tri_triatt_forward(C.byref(args), at[1]))
+        _lib.check(lib.b200tri_triatt_forward_packed(args, at[1]))
     result = _unfold(out, lead)
     if host_in:
         host = result.float().cpu() if numpy_in else result.cpu()
@@ -159,11 +163,12 @@ def attention_core(q, k, v, tri_bias, mask_bias, scale: float | None = None):
                                     qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), bd.data_ptr(), md.data_ptr(),
                                     out.data_ptr(), dev.aligned_ptr(ws), nbytes)
     if bsz:  # (an empty batch has an empty result)
-        _lib.check(lib.b200tri_attention_core(C.byref(args), at[1]))
+        _lib.check(lib.b200tri_attention_core_packed(args, at[1]))
     return out if v.dtype is torch.bfloat16 else out.to(v.dtype)
 
 
 def _operand(t: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     """``t`` as the library reads it: dense, of ``dtype`` and 16-byte aligned (a slice need not be)."""
-    t = t.to(dtype).contiguous()
+    if t.dtype is not dtype or not t.is_contiguous():
+        t = t.to(dtype).contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
