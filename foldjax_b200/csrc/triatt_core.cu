@@ -111,9 +111,11 @@ constexpr uint32_t STAGE_TX = BIAS_BYTES + NWG * (K_BYTES + V_TMA_BYTES + KT * 4
 
 // One launch can walk several key tiles (ring attention: the tiles of the peers, each in
 // its own buffers): per tile one tensor map for K, V^T, the pair bias and the mask-bias rows.
+// (One tile, as everywhere but there, has a kernel whose arguments are its maps alone.)
 constexpr int MAX_KEY_TILES = 7;
+template <int TILES>
 struct TileMaps {
-  CUtensorMap k[MAX_KEY_TILES], v[MAX_KEY_TILES], b[MAX_KEY_TILES], m[MAX_KEY_TILES];
+  CUtensorMap k[TILES], v[TILES], b[TILES], m[TILES];
 };
 
 struct Params {
@@ -196,9 +198,9 @@ inline bool may_end_early(int n_k, int steps) {
   return steps >= LIVE_STEPS_FROM && steps <= LIVE_STEPS_TO && n_k - (steps - 1) * KT <= n_k / 8;
 }
 
-template <bool ENDS>
+template <bool ENDS, int TILES>
 __global__ void __launch_bounds__(THREADS, 1)
-att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ TileMaps tm, const Params p) {
+att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ TileMaps<TILES> tm, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   // (through a shuffle, so that the compiler knows it to be the same in all lanes)
@@ -301,7 +303,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           steps = live_steps(p.mb + static_cast<long long>(i0) * p.mb_ld, p.mb_ld, p.n_i - i0, steps, LIVE_STEPS_LEAST);
         alive = alive && mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER);
         __syncwarp();
-        const int tile = t / p.steps_per_tile;
+        const int tile = TILES == 1 ? 0 : t / p.steps_per_tile;
         const int k0 = (t - tile * p.steps_per_tile) * KT;
         if (leader && alive) {
           if (ENDS) sm.last[stage] = t + 1 == steps;
@@ -736,7 +738,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   const int ldm = round_up(a->n_k, 64);
   // q, k and o: [row][token][head][32] unless the caller says otherwise
   const CoreStrides st = strides ? *strides : CoreStrides{128, 32, 32, 128ll * a->n_j, 128ll * a->n_k};
-  TileMaps tm;
+  TileMaps<MAX_KEY_TILES> tm;
   for (int t = 0; t < n_tiles; ++t) {
     const b200tri_triatt_core_args* ti = tiles + t;
     B200_REQUIRE(ti->k && ti->vt && ti->bias, B200TRI_ERR_INVALID, "att core: null k/vt/bias in key tile %d", t);
@@ -781,7 +783,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
       if (rc) return rc;
     }
   }
-  for (int t = n_tiles; t < MAX_KEY_TILES; ++t) {  // unused slots: valid descriptors, never read
+  for (int t = n_tiles; n_tiles > 1 && t < MAX_KEY_TILES; ++t) {  // unused slots: valid descriptors, never read
     tm.k[t] = tm.k[0];
     tm.v[t] = tm.v[0];
     tm.b[t] = tm.b[0];
@@ -822,13 +824,15 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   p.status = status;
 
   const long long grid = items < sm_count() ? items : sm_count();
-  auto go = [&](auto kernel) {
+  auto go = [&](auto kernel, const auto& tiles_maps) {
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem));
     if (rc) return rc;
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
-    return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tm, p);
+    return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tiles_maps, p);
   };
-  return n_tiles == 1 && may_end_early(a->n_k, p.steps) ? go(att_core_kernel<true>) : go(att_core_kernel<false>);
+  if (n_tiles > 1) return go(att_core_kernel<false, MAX_KEY_TILES>, tm);
+  const TileMaps<1> one = {{tm.k[0]}, {tm.v[0]}, {tm.b[0]}, {tm.m[0]}};
+  return may_end_early(a->n_k, p.steps) ? go(att_core_kernel<true, 1>, one) : go(att_core_kernel<false, 1>, one);
 }
 }  // namespace
 
