@@ -462,6 +462,9 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
 // products and sums of float32 pairs unpacked from the pieces instead of mixed-precision fmas, a step of
 // three rows took 2.35 us where one of four takes 2.66. Four updates of four 200-token templates 700 -> 649 us, of a
 // 256-token refiner 1161 -> 1119, attention of 4 x 320 tokens 541 -> 444.
+// HDP: a head's width in the products, rounded up to 16, 32 or 64. Heads of 16 as 32 pay for a product of
+// zeros a step and twice the columns in P.V, and read back twice the result: the templates 650 us, 635 as 16 (the
+// same bits).
 // Measured and not better: an issuer per row, rows started a fraction of a step apart, P as two tf32 pieces
 // against V as float32, ending an item with its rows' last kept key (the flags cost the issuers 4 %, which
 // only paddings of a whole step pay back), the difference of two bf16 by a subtraction.
@@ -473,7 +476,7 @@ struct BfCfg {
   // 512 x 128 = 128 x 56 + 384 x 152, 640 x 96 = 128 x 32 + 512 x 112 (two rows have enough as they are)
   static constexpr int CONTROL_REGS = NWG == 4 ? 32 : 56, SOFTMAX_REGS = NWG == 4 ? 112 : 152;
   static constexpr int Q_BYTES = 128 * HDP * 2, K_BYTES = KT * HDP * 2, V_BYTES = HDP * 128, BIAS_BYTES = 128 * KT * 2;
-  static constexpr uint32_t TM_P = 0, TM_O = 96, TM_WG = TM_O + HDP;  // P (three pieces) over S (64 columns)
+  static constexpr uint32_t TM_P = 0, TM_O = 96, TM_WG = HDP <= 32 ? 128 : TM_O + HDP;  // P (three pieces) over S (64 columns)
   static_assert(NWG * TM_WG <= 512, "tensor memory budget");
   static constexpr uint32_t STAGE_TX = NWG * (K_BYTES + V_BYTES + KT * 4) + BIAS_BYTES;
 };
@@ -869,12 +872,13 @@ int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
 // Rows of an item. A step of four takes 1.2 times as long as one of three (2.66 and 2.2 us), which pays
 // unless as many rounds of items are needed: 12 heads x 100 tokens, attention 63.4 us with four and 59.8 with three
 // (three rounds either way), 4 x 4 heads x 200 tokens 193 and 207 (11 and 15 rounds).
+template <int HDP>
 int launch_bf16_narrow(const Maps& tm, const Params& p, bool pdl, cudaStream_t stream) {
   auto rounds = [&](int rows) {
     const long long items = static_cast<long long>(p.total_items) * ((p.n_i + rows - 1) / rows) * ((p.n + 127) / 128);
     return (items + sm_count() - 1) / sm_count();
   };
-  return 5 * rounds(3) < 6 * rounds(4) ? launch_bf16<32, 3>(tm, p, pdl, stream) : launch_bf16<32, 4>(tm, p, pdl, stream);
+  return 5 * rounds(3) < 6 * rounds(4) ? launch_bf16<HDP, 3>(tm, p, pdl, stream) : launch_bf16<HDP, 4>(tm, p, pdl, stream);
 }
 
 }  // namespace
@@ -885,8 +889,8 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   const bool token = a.pieces != nullptr;
   B200_REQUIRE(!token || (!a.bf16 && a.batch == 1 && a.n_i == 1 && a.head_dim <= 32), B200TRI_ERR_INVALID,
                "float32 attention: the gated form takes one row of heads up to 32 wide");
-  const uint32_t hdp = a.head_dim <= 32 ? 32 : 64;
-  const Swz qk_swz = hdp == 32 ? Swz::B64 : Swz::B128;
+  const uint32_t hdp = a.bf16 && a.head_dim <= 16 ? 16 : a.head_dim <= 32 ? 32 : 64;
+  const Swz qk_swz = hdp == 16 ? Swz::B32 : hdp == 32 ? Swz::B64 : Swz::B128;
   const uint64_t hd = a.head_dim, heads = a.heads, width = hd * heads, n = a.n;
   const uint64_t rows = static_cast<uint64_t>(a.n_i) * a.batch, in = a.bf16 ? 1 : 3;
   Maps tm;
@@ -935,7 +939,8 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   p.status = device_status_word();
   B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "float32 attention: no current CUDA device");
   if (token) return launch_cfg<32, true>(tm, p, a.pdl, stream);
-  if (a.bf16) return hdp == 32 ? launch_bf16_narrow(tm, p, a.pdl, stream) : launch_bf16<64, 2>(tm, p, a.pdl, stream);
+  if (a.bf16 && hdp == 16) return launch_bf16_narrow<16>(tm, p, a.pdl, stream);
+  if (a.bf16) return hdp == 32 ? launch_bf16_narrow<32>(tm, p, a.pdl, stream) : launch_bf16<64, 2>(tm, p, a.pdl, stream);
   return hdp == 32 ? launch_cfg<32, false>(tm, p, a.pdl, stream) : launch_cfg<64, false>(tm, p, a.pdl, stream);
 }
 

@@ -39,7 +39,7 @@ int* device_status_word();
     }                                 \
   } while (0)
 
-enum class Swz { None, B64, B128 };
+enum class Swz { None, B32, B64, B128 };
 
 // Encode a tiled tensor map over `rank` dimensions (innermost first).
 // strides_bytes[i] is the byte stride of dimension i+1 (dimension 0 is dense).

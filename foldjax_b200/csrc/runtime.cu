@@ -258,6 +258,7 @@ int make_tmap(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, int
                  static_cast<unsigned long long>(strides_bytes[i]));
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUtensorMapSwizzle s = CU_TENSOR_MAP_SWIZZLE_NONE;
+  if (swz == Swz::B32) s = CU_TENSOR_MAP_SWIZZLE_32B;
   if (swz == Swz::B64) s = CU_TENSOR_MAP_SWIZZLE_64B;
   if (swz == Swz::B128) s = CU_TENSOR_MAP_SWIZZLE_128B;
   auto encode = [&] {

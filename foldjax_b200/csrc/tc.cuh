@@ -268,7 +268,7 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
 }
 
 // Shared-memory matrix descriptor, K-major tile. `row_bytes` is 128 (swizzle
-// 128B) or 64 (swizzle 64B); eight rows form one swizzle atom and atoms follow
+// 128B), 64 (swizzle 64B) or 32 (swizzle 32B); eight rows form one swizzle atom and atoms follow
 // one another every 8*row_bytes bytes.
 __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t saddr, uint32_t row_bytes) {
   const uint64_t swz = (row_bytes == 128) ? 2ull : (row_bytes == 64 ? 4ull : 6ull);

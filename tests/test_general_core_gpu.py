@@ -23,6 +23,7 @@ pytestmark = pytest.mark.gpu
     (65, 4, 16, 0.1), (100, 12, 32, 0.1),  # two steps; three rows to an item
     (130, 4, 16, 0.2), (193, 8, 24, 0.1),  # three, with larger scores; four steps
     (129, 2, 64, 0.2), (257, 4, 16, 0.1),  # wide heads, two rows; five steps
+    (70, 4, 8, 0.1), (131, 6, 8, 0.2),     # heads that fill half a tile of 16
 ])
 def test_general_core(cuda_device, n, heads, head_dim, std):
     from foldjax_b200 import _lib
