@@ -49,7 +49,7 @@
 // loops are the whole warp's, which keeps control flow and operands in uniform registers, P.V of the
 // step before is waited for behind the exponentials, and the two waits at a step's start are asked as
 // one; results leave in 32-byte stores. Attention operator, us, n = 256 / 384 / 512 / 3072: 45.0 / 113.7 /
-// 229.6 / 40 800 before those, 40.6 / 103.2 / 211.6 / 37 300 now. Of that the joins that hold the lanes of a warp together cost the
+// 229.6 / 40 800 before those, 40.6 / 103.2 / 211.6 / 37 300 with them. Of that the joins that hold the lanes of a warp together cost the
 // issuers 0.5 / 1.6 / 4.1 / 100 and gave the softmax 0.9 / 1.6 / 1.4 / 400. Measured instead of
 // __syncwarp behind the issuers' waits: a vote on each wait (213 at n = 512), elect.sync (212), the
 // waits in the leader's branch, which needs no join (261).
@@ -111,8 +111,11 @@ constexpr uint32_t STAGE_TX = BIAS_BYTES + NWG * (K_BYTES + V_TMA_BYTES + KT * 4
 
 // One launch can walk several key tiles (ring attention: the tiles of the peers, each in
 // its own buffers): per tile one tensor map for K, V^T, the pair bias and the mask-bias rows.
-// (One tile, as everywhere but there, has a kernel whose arguments are its maps alone.)
-constexpr int MAX_KEY_TILES = 7;
+// One tile, as everywhere but there, has a kernel whose arguments are its maps alone, which starts sooner: attention
+// operator, 384 tokens, 97.3 -> 96.3 us. It gains up to some 32 steps: whole block, ms, with all maps and with one,
+// 1344 tokens 12.08 and 12.01, 2048 34.60 and 34.58, 3072 106.7 and 107.6. (Both give the same bits; with more steps the
+// power limit decides, and the start counts for nothing.)
+constexpr int MAX_KEY_TILES = 7, ONE_MAP_STEPS = 32;
 template <int TILES>
 struct TileMaps {
   CUtensorMap k[TILES], v[TILES], b[TILES], m[TILES];
@@ -191,8 +194,8 @@ __device__ __forceinline__ int live_steps(const float* mb, int ld, int rows, int
 // first LIVE_STEPS_LEAST - 1 steps on their way (so many there are in any case), and marks the stage that holds
 // the last step. Only where a padding of an eighth of the keys would empty the last step, and in items of
 // LIVE_STEPS_FROM to LIVE_STEPS_TO steps: attention operator, us, without and with: 512 tokens of which 64 are padding
-// 214 and 199, nothing to leave out at 203, 256, 384 tokens 38.2 and 38.2, 37.9 and 37.9, 103.3 and 104.0, at
-// 3072 37 250 and 38 130.
+// 214 and 199 (191.5 with the maps of one tile), nothing to leave out at 203, 256, 384 tokens 38.2 and 38.2, 37.9 and
+// 37.9, 103.3 and 104.0, at 3072 37 250 and 38 130.
 constexpr int LIVE_STEPS_FROM = 4, LIVE_STEPS_TO = 20, LIVE_STEPS_LEAST = 3;
 inline bool may_end_early(int n_k, int steps) {
   return steps >= LIVE_STEPS_FROM && steps <= LIVE_STEPS_TO && n_k - (steps - 1) * KT <= n_k / 8;
@@ -738,6 +741,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   const int ldm = round_up(a->n_k, 64);
   // q, k and o: [row][token][head][32] unless the caller says otherwise
   const CoreStrides st = strides ? *strides : CoreStrides{128, 32, 32, 128ll * a->n_j, 128ll * a->n_k};
+  const bool many_maps = n_tiles > 1 || a->n_k > ONE_MAP_STEPS * KT;
   TileMaps<MAX_KEY_TILES> tm;
   for (int t = 0; t < n_tiles; ++t) {
     const b200tri_triatt_core_args* ti = tiles + t;
@@ -783,7 +787,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
       if (rc) return rc;
     }
   }
-  for (int t = n_tiles; n_tiles > 1 && t < MAX_KEY_TILES; ++t) {  // unused slots: valid descriptors, never read
+  for (int t = n_tiles; many_maps && t < MAX_KEY_TILES; ++t) {  // unused slots: valid descriptors, never read
     tm.k[t] = tm.k[0];
     tm.v[t] = tm.v[0];
     tm.b[t] = tm.b[0];
@@ -830,7 +834,7 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
     return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tiles_maps, p);
   };
-  if (n_tiles > 1) return go(att_core_kernel<false, MAX_KEY_TILES>, tm);
+  if (many_maps) return go(att_core_kernel<false, MAX_KEY_TILES>, tm);
   const TileMaps<1> one = {{tm.k[0]}, {tm.v[0]}, {tm.b[0]}, {tm.m[0]}};
   return may_end_early(a->n_k, p.steps) ? go(att_core_kernel<true, 1>, one) : go(att_core_kernel<false, 1>, one);
 }
