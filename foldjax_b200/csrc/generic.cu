@@ -18,7 +18,7 @@
 //   layer norm -> q, k, v, bias product -> core -> gate product -> output product
 // (plus one that splits or pads weights where they cannot be read as stored). The layer norms
 // are CUDA-core kernels. The four updates of a 256-token 384-channel refiner block take 1.12 ms and
-// those of four 200-token templates 0.65 (26.2 and 6.9 with the products on the CUDA cores). What the
+// those of four 200-token templates 0.62 (26.2 and 6.9 with the products on the CUDA cores). What the
 // threads of an epilogue move, each along a row of its own, goes 32 bytes at a time: with 16 those
 // stacks took 1.29 and 0.80 ms and a 256-token float32 stack 1.01 instead of 0.91.
 //
