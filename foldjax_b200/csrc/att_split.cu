@@ -80,15 +80,6 @@ __device__ __forceinline__ float2 exp_below(float2 s, float2 minus_m) {
   const float2 t = __fmul2_rn(__fadd2_rn(s, minus_m), make_float2(1.44269504f, 1.44269504f));
   return make_float2(fast_exp2(t.x), fast_exp2(t.y));
 }
-// split3x2 with packed subtractions
-__device__ __forceinline__ void split3f2(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const float2 minus = make_float2(-1.0f, -1.0f);
-  hi = pack_bf16x2(v.x, v.y);
-  const float2 r = __ffma2_rn(make_float2(bf16_lo(hi), bf16_hi(hi)), minus, v);
-  mid = pack_bf16x2(r.x, r.y);
-  const float2 q = __ffma2_rn(make_float2(bf16_lo(mid), bf16_hi(mid)), minus, r);
-  lo = pack_bf16x2(q.x, q.y);
-}
 
 template <int HDP, bool TOKEN>
 __global__ void __launch_bounds__(Cfg<HDP, TOKEN>::THREADS, 1)
@@ -363,7 +354,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         for (int oct = 0; oct < 4; ++oct) {  // 16 keys at a time: few live registers
           uint32_t pc[3][8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) split3f2(s[oct * 8 + e], pc[0][e], pc[1][e], pc[2][e]);
+          for (int e = 0; e < 8; ++e) split3x2(s[oct * 8 + e].x, s[oct * 8 + e].y, pc[0][e], pc[1][e], pc[2][e]);
 #pragma unroll
           for (int q = 0; q < 3; ++q) tmem_st8(t_wg + C::TM_P + q * 32 + oct * 8, pc[q]);
         }
@@ -498,21 +489,6 @@ struct BfSmem {
 constexpr float LOG2E = 1.44269504f;
 constexpr float INTEGER_OFFSETS = 8388608.0f;  // 2^23: floats beyond are integers themselves
 
-
-// v - (the pair's two values), one instruction each (8 % of the kernel, against two to unpack and half a packed one).
-__device__ __forceinline__ float2 less_bf16x2(float2 v, uint32_t w) {
-  float2 r;
-  asm("{\n"
-      " .reg .b16 lo, hi, m;\n"
-      " mov.b32 {lo, hi}, %2;\n"
-      " mov.b16 m, 0xBF80;\n"
-      " fma.rn.f32.bf16 %0, lo, m, %3;\n"
-      " fma.rn.f32.bf16 %1, hi, m, %4;\n"
-      "}\n"
-      : "=f"(r.x), "=f"(r.y)
-      : "r"(w), "f"(v.x), "f"(v.y));
-  return r;
-}
 // hi + mid + lo = v exactly, and all three go into P.V: bf16 is the upper half of a float, and its 8 bits leave 16 and
 // then 8 of the 24. Cut off instead of rounded, as exact and a byte permutation for two instead of a conversion:
 // templates 634 -> 623 us, 4 x 320 tokens 445 -> 434; error against float64 over 40 inputs within 1e-5 of itself either way,
