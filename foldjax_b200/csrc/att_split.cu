@@ -19,7 +19,7 @@
 //   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
 //   warpgroups  softmax, one thread per query
 // Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (a score costs about 2
-// instructions of exponential, 4.5 of split and 4 others, most of them packed two to an instruction); the
+// instructions of exponential, 3.5 of split and 4 others, most of them packed two to an instruction); the
 // rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
 #include "att_split.cuh"
 #include "gemm.cuh"
