@@ -57,7 +57,10 @@
 // 7 or 9 of 16 pairs on the FMA pipe, results staged for a TMA store, a second Q.K^T issuer, four rows
 // with 32 scores at a time and an issuer per row and product (the rows fall into phase and queue for the
 // same unit), two rows to an item where that saves none a round, no more CTAs than whole rounds need (the
-// successor sets up on the SMs that end early).
+// successor sets up on the SMs that end early), an item's steps up to its rows' last kept key. (That last is right only
+// where the offsets lie well above MASKED_SCORE and the values left out are finite, which a weight of zero does not
+// hide. With the softmax saying so after the first step and V of the steps left out multiplied by zeros, the same bits, 512
+// keys of which 64 are dropped took 223 us, walking them all 217.)
 #include <cuda_fp16.h>
 
 #include <mutex>
@@ -90,8 +93,9 @@ constexpr float EXP_MAGIC = 12582912.0f;  // 1.5 * 2^23: adding it leaves round(
 // (|q.k + bias| < 32 is below half an ulp of 1e9): every dropped key ends up with
 // the same score, so a row with no valid key becomes a uniform average. Here a
 // mask bias at or below MASKED_SCORE REPLACES the score with that constant, which
-// has the same two effects (zero weight beside any valid key, uniform without one)
-// while keeping the softmax offset small enough for a single fp32 fma per
+// has the same two effects (zero weight beside any valid key that scores above some -29 980, uniform
+// without one; a query whose valid keys all score lower, by a pair bias or soft mask values used as
+// masks, spreads weight over its dropped keys) while keeping the softmax offset small enough for a single fp32 fma per
 // exponent. Smaller mask biases (soft masks) are added as they are.
 // (MASKED_SCORE and the rule itself: mask_bias() in tc.cuh)
 
@@ -102,7 +106,6 @@ struct Smem {
   uint8_t k[STAGES][NWG][K_BYTES];
   uint8_t v[STAGES][NWG][V_BYTES];
   float mb[STAGES][NWG][KT];
-  int last[STAGES];  // the stage holds its item's last step (only with ENDS)
   uint64_t q_full[QBUF], q_empty[QBUF], st_full[STAGES], st_empty[STAGES], s_full[NWG], s_free[NWG], p_full[NWG], pv_done[NWG];
   uint32_t tmem_base;
 };
@@ -127,8 +130,6 @@ struct Params {
   int heads;
   int groups, tiles_j, steps;
   uint32_t total_items;
-  const float* mb;  // the mask-bias rows
-  int mb_ld;
   __nv_bfloat16* o;
   long long o_token, o_head, o_row;  // strides of o in elements
   bool o_sectors;                    // a head of o is two 32-byte sectors
@@ -164,44 +165,7 @@ __device__ __forceinline__ float2 poly_exp2x2(float2 u, float2 log2e2, float2 ma
                      __int_as_float(__float_as_int(q.y) + (__float_as_int(y.y) << 23)));
 }
 
-// Steps of 64 keys that an item has to walk: keys behind a row's last kept one have weights of exactly zero,
-// and steps of nothing else add nothing. `mb`: the mask-bias values of the item's `rows` rows, pitch `ld`. A row
-// without a kept key in the last LOOK steps makes it all of them: it may have none at all, and then every key
-// counts. By a whole warp; the same in all lanes.
-__device__ __forceinline__ int live_steps(const float* mb, int ld, int rows, int steps, int least) {
-  constexpr int LOOK = 4;
-  const int lane = threadIdx.x & 31;
-  int need = least;
-  uint32_t open = (1u << (rows < NWG ? rows : NWG)) - 1;  // rows without a kept key so far
-  for (int s = steps; s > 0 && s > steps - LOOK && open != 0; --s) {
-    float v[NWG][2];
-#pragma unroll
-    for (int r = 0; r < NWG; ++r)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        v[r][u] = open >> r & 1 ? mb[static_cast<long long>(r) * ld + (s - 1) * KT + u * 32 + lane] : MASKED_SCORE;
-#pragma unroll
-    for (int r = 0; r < NWG; ++r)
-      if (__any_sync(0xffffffffu, !(v[r][0] <= MASKED_SCORE && v[r][1] <= MASKED_SCORE))) {
-        open &= ~(1u << r);
-        need = s > need ? s : need;
-      }
-    if (need == steps) break;
-  }
-  return open != 0 ? steps : need;
-}
-// ENDS: an item's steps end with its rows' last kept key. The producer looks at the mask, with the loads of the
-// first LIVE_STEPS_LEAST - 1 steps on their way (so many there are in any case), and marks the stage that holds
-// the last step. Only where a padding of an eighth of the keys would empty the last step, and in items of
-// LIVE_STEPS_FROM to LIVE_STEPS_TO steps: attention operator, us, without and with: 512 tokens of which 64 are padding
-// 214 and 199 (191.5 with the maps of one tile), nothing to leave out at 203, 256, 384 tokens 38.2 and 38.2, 37.9 and
-// 37.9, 103.3 and 104.0, at 3072 37 250 and 38 130.
-constexpr int LIVE_STEPS_FROM = 4, LIVE_STEPS_TO = 20, LIVE_STEPS_LEAST = 3;
-inline bool may_end_early(int n_k, int steps) {
-  return steps >= LIVE_STEPS_FROM && steps <= LIVE_STEPS_TO && n_k - (steps - 1) * KT <= n_k / 8;
-}
-
-template <bool ENDS, int TILES>
+template <int TILES>
 __global__ void __launch_bounds__(THREADS, 1)
 att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ TileMaps<TILES> tm, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -225,7 +189,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.st_full[s], 1);
-      mbar_init(&sm.st_empty[s], ENDS ? 1 : 1 + NWG * 4);
+      mbar_init(&sm.st_empty[s], 1 + NWG * 4);
     }
     for (int g = 0; g < NWG; ++g) {
       mbar_init(&sm.s_full[g], 1);
@@ -300,16 +264,12 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         mbar_expect_tx(&sm.q_full[qb], NWG * Q_BYTES);
         for (int g = 0; g < NWG; ++g) tma_load_4d(sm.q[qb][g], &tm_q, &sm.q_full[qb], 0, h, j0, i0 + g);
       }
-      int steps = p.steps;
-      for (int t = 0; t < steps; ++t) {
-        if (ENDS && t == LIVE_STEPS_LEAST - 1)
-          steps = live_steps(p.mb + static_cast<long long>(i0) * p.mb_ld, p.mb_ld, p.n_i - i0, steps, LIVE_STEPS_LEAST);
+      for (int t = 0; t < p.steps; ++t) {
         alive = alive && mbar_wait(&sm.st_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER);
         __syncwarp();
         const int tile = TILES == 1 ? 0 : t / p.steps_per_tile;
         const int k0 = (t - tile * p.steps_per_tile) * KT;
         if (leader && alive) {
-          if (ENDS) sm.last[stage] = t + 1 == steps;
           mbar_expect_tx(&sm.st_full[stage], STAGE_TX);
           tma_load_3d(sm.bias[stage], &tm.b[tile], &sm.st_full[stage], k0, j0, h);
           for (int g = 0; g < NWG; ++g) {
@@ -338,10 +298,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
       const uint32_t qb = item_it % QBUF;
       alive = alive && mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA);
-      bool more = true;
-      for (int t = 0; ENDS ? more : t < p.steps; ++t, ++g) {
+      for (int t = 0; t < p.steps; ++t, ++g) {
         alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
-        const int last = ENDS ? sm.last[stage] : 0;
         const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
 #pragma unroll
         for (int wg = 0; wg < NWG; ++wg) {
@@ -360,7 +318,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             umma_commit(&sm.s_full[wg]);
           }
         }
-        if (ENDS) more = __shfl_sync(0xffffffffu, alive && last == 0, 0);  // (one lane's word, so that none goes its own way)
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;
@@ -376,12 +333,10 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint32_t phase = 0, g = 0;
     bool alive = true;
     for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
-      bool more = true;
-      for (int t = 0; ENDS ? more : t < p.steps; ++t, ++g) {
+      for (int t = 0; t < p.steps; ++t, ++g) {
         // (already complete when P arrives; observed here so this thread's products
         // are ordered after the TMA writes of V)
         alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
-        const int last = ENDS ? sm.last[stage] : 0;
         for (int wg = 0; wg < NWG; ++wg) {
           alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
           __syncwarp();
@@ -397,10 +352,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         // K of this stage was consumed before the softmax saw its scores, V by the
-        // products just issued: the stage is free once they complete. (With ENDS the softmax warps read the
-        // stage until they have P, which these products waited for, and arrive on its barrier only through them.)
+        // products just issued: the stage is free once they complete.
         if (leader && alive) umma_commit(&sm.st_empty[stage]);
-        if (ENDS) more = __shfl_sync(0xffffffffu, alive && last == 0, 0);
         if (++stage == STAGES) {
           stage = 0;
           phase ^= 1;
@@ -459,8 +412,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tmem_st_wait();
         tc_fence_before();
       }
-      bool more = true;
-      for (int t = 0; ENDS ? more : t < p.steps; ++t, ++g) {
+      for (int t = 0; t < p.steps; ++t, ++g) {
         // (both asked at once: nearly always there already, and one latency instead of two. Each lane polls
         // for itself; the vote brings them together again, as the TMEM accesses need, and has all or
         // none of them leave)
@@ -507,10 +459,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if ((c & 3) == 3) asm volatile("" ::: "memory");  // keep the loads from piling up in registers
           }
         }
-        if (!ENDS) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
         // four independent chains, so the reduction is not one 32-deep dependency
         float mxa = fmaxf(u[0].x, u[0].y), mxb = fmaxf(u[1].x, u[1].y);
         float mxc = fmaxf(u[2].x, u[2].y), mxd = fmaxf(u[3].x, u[3].y);
@@ -526,14 +476,12 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // 2^8 (then it exceeds every earlier maximum too, which stayed within the threshold).
         const bool need = (mx2 - m2_used) > RESCALE_THRESHOLD;  // true on the first step (m2_used = -inf)
         float alpha = 1.f;
-        const bool old_offset = m2_used != -INFINITY;
         if (need) {
           const float m2_new = rintf(mx2);
           alpha = fast_exp2(m2_used - m2_new);  // an exact power of two; 0 on the first step
           m2_used = m2_new;
         }
-        // (nothing to rescale on the first step, whose products overwrite O)
-        const bool any_need = __any_sync(0xffffffffu, ENDS ? need && old_offset : need);
+        const bool any_need = __any_sync(0xffffffffu, need);
         // exp(u - m) = 2^(u * log2e - m2): one fma per pair feeds the MUFU unit (|m2| < 2^17, so
         // the sum is exact to the last bit of the product and cancels exactly for the keys that
         // equal the offset). POLY of every 16 pairs take the polynomial path instead: the
@@ -574,7 +522,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             tmem_st16(t_wg + TM_P + 16 * half, packed);
           }
         }
-        if ((ENDS || t > 0 || p.resume) && any_need) {
+        if ((t > 0 || p.resume) && any_need) {
           uint32_t o[32];
           tmem_ld32(t_wg + TM_O, o);
           tmem_ld_wait();
@@ -588,7 +536,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int e = 0; e < 16; ++e) lcol[e] = __float_as_uint(__uint_as_float(lcol[e]) * alpha);
           tmem_st16(t_wg + TM_L, lcol);
         }
-        if (ENDS) more = sm.last[stage] == 0;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -810,8 +757,6 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   p.tiles_j = (a->n_j + 127) / 128;
   p.steps_per_tile = (a->n_k + KT - 1) / KT;
   p.steps = p.steps_per_tile * n_tiles;
-  p.mb = static_cast<const float*>(a->workspace);
-  p.mb_ld = ldm;
   const long long items = static_cast<long long>(a->heads) * p.groups * p.tiles_j;
   B200_REQUIRE(items < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "att core: too many rows times queries for one launch");
   p.total_items = static_cast<uint32_t>(items);
@@ -834,9 +779,9 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
     return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tiles_maps, p);
   };
-  if (many_maps) return go(att_core_kernel<false, MAX_KEY_TILES>, tm);
+  if (many_maps) return go(att_core_kernel<MAX_KEY_TILES>, tm);
   const TileMaps<1> one = {{tm.k[0]}, {tm.v[0]}, {tm.b[0]}, {tm.m[0]}};
-  return may_end_early(a->n_k, p.steps) ? go(att_core_kernel<true, 1>, one) : go(att_core_kernel<false, 1>, one);
+  return go(att_core_kernel<1>, one);
 }
 }  // namespace
 

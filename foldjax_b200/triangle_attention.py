@@ -127,7 +127,9 @@ def attention_core(q, k, v, tri_bias, mask_bias, scale: float | None = None):
     The additive mask bias goes to the kernel as it is (no round trip through a 0/1 mask), so
     soft and hard entries can be mixed; a row with no kept key comes out as the uniform average
     over its keys, the convention of the finite -1e9 mask (triangle_attention.py:138-142), not as
-    the zeros of the reference's 2-D ring (src/foldjax/models/_cp_attention.py:380-385).
+    the zeros of the reference's 2-D ring (src/foldjax/models/_cp_attention.py:380-385). A dropped key
+    (mask bias of -30000 or less) scores -30000 and so has no weight beside kept keys that score above
+    some -29980; a query whose kept keys all score less (a pair bias used as a mask) gives its dropped keys weight.
     Enqueue-only: nothing here waits for the device. bf16 operands are read where they are (the
     library transposes v, builds the mask rows and, only where its rows are off TMA's 16-byte
     grid or float32, copies the bias); other element types are converted first.
