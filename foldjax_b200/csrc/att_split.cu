@@ -439,24 +439,23 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
 // triatt_core.cu (S = bias . I + q . k), the numerator accumulates in TMEM and is rescaled only when
 // the maximum grew by more than RESCALE, and the probabilities overwrite the scores they came from, so
 // that four softmax warpgroups fit (128 columns each).
-//   warp 0       TMA producer       warps 1, 2   issuers, each of all products of its rows
-//   warpgroups   softmax, one thread per query
-// The scores of a row's next step are issued right behind P.V of this one, by the same thread: the
-// tensor pipe works a thread's products off in the order they were issued in, so the scores cannot overtake
-// the P.V that still reads the columns they go to, and one barrier tells the softmax that both are
-// through. The softmax offset is an integer in log2 units (one fma per pair of exponentials, exact
+//   warp 0       TMA producer            warps 1, 2   P.V issuers, each of half of the rows (three rows: one)
+//   warp 3       issuer of all scores    warpgroups   softmax, one thread per query
+// A row's next scores go to columns that P.V of this step reads. Products of other shapes into other accumulators
+// have no order that is promised, whoever issued them, so warp 3 waits until P.V is through; s_full then tells the
+// softmax that both are. A warp of its own, because one that issued P.V too kept its other rows' P.V waiting
+// (attention of 320 tokens, 4 heads x 32, 155 us; 150 with both issued back to back and no wait; 148 so).
+// The softmax offset is an integer in log2 units (one fma per pair of exponentials, exact
 // powers of two to rescale by) except where scores are so large that integers are no finer than they are.
 //
 // Bound: a row's step is a chain of softmax (1.2 us with the other rows' warps beside it, 8 instructions a
 // score) and products (18 of them, 0.35 us, and the trips between the warps), and the rows in flight hide
-// each other's: with three rows, scores and P.V issued by two warps that waited for each other's products, and
-// products and sums of float32 pairs unpacked from the pieces instead of mixed-precision fmas, a step of
-// three rows took 2.35 us where one of four takes 2.66. Four updates of four 200-token templates 700 -> 649 us, of a
-// 256-token refiner 1161 -> 1119, attention of 4 x 320 tokens 541 -> 444. It issues in 71 % of its slots with 61 % of the
-// MUFU unit busy (counters, 4 x 400 tokens, 4 heads x 16).
+// each other's. Three rows, P.V issued by one warp, padded heads of 16, rounded pieces and pairs unpacked from them
+// took 695 us for the four updates of four 200-token templates, 1 178 for those of a 256-token refiner, 112 and 247 for
+// attention of 200 and 320 tokens with 4 heads x 64; now 615, 1 126, 105 and 219. It issued in 71 % of its slots with 61 % of
+// the MUFU unit busy when the P.V issuers still issued the scores (counters, 4 x 400 tokens, 4 heads x 16).
 // HDP: a head's width in the products, rounded up to 16, 32 or 64. Heads of 16 as 32 pay for a product of
-// zeros a step and twice the columns in P.V, and read back twice the result: the templates 650 us, 635 as 16 (the
-// same bits).
+// zeros a step and twice the columns in P.V, and read back twice the result: 2.3 % of the templates' time (the same bits).
 // Measured and not better: an issuer per row, rows started a fraction of a step apart, P as two tf32 pieces
 // against V as float32, ending an item with its rows' last kept key (the flags cost the issuers 4 %, which
 // only paddings of a whole step pay back), the difference of two bf16 by a subtraction.
@@ -482,7 +481,7 @@ struct BfSmem {
   uint8_t bias[C::STAGES][C::BIAS_BYTES];  // [128 queries][64 keys]
   uint8_t ident[KT * 128];                 // 64 x 64 bf16 identity
   alignas(128) float mb[C::STAGES][NWG][KT];
-  uint64_t q_full[C::QBUF], q_empty[C::QBUF], st_full[C::STAGES], st_empty[C::STAGES], s_full[NWG], p_full[NWG], o_full[NWG];
+  uint64_t q_full[C::QBUF], q_empty[C::QBUF], st_full[C::STAGES], st_empty[C::STAGES], s_full[NWG], p_full[NWG], pv_done[NWG];
   uint32_t tmem_base;
 };
 
@@ -526,7 +525,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     tma_prefetch_desc(&tm.b);
     for (int b = 0; b < C::QBUF; ++b) {
       mbar_init(&sm.q_full[b], 1);
-      mbar_init(&sm.q_empty[b], C::ISSUERS);
+      mbar_init(&sm.q_empty[b], 1);
     }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.st_full[s], 1);
@@ -535,7 +534,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     for (int g = 0; g < NWG; ++g) {
       mbar_init(&sm.s_full[g], 1);
       mbar_init(&sm.p_full[g], 4);
-      mbar_init(&sm.o_full[g], 1);
+      mbar_init(&sm.pv_done[g], 1);
     }
     fence_barrier_init();
   }
@@ -566,7 +565,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     j0 = (rem - grp * p.tiles_j) * 128;
   };
 
-  // In warps 0 to 2 all lanes walk the loops and wait, and one of them issues; none leaves early: one whose
+  // In warps 0 to 3 all lanes walk the loops and wait, and one of them issues; none leaves early: one whose
   // wait has run out stops waiting and issuing and walks on. Joins as in triatt_core.cu.
   if (warp < 4) {
     if (NWG > 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::CONTROL_REGS));
@@ -608,49 +607,19 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     } else if (warp <= C::ISSUERS) {
       const bool leader = elect_one();
       const int r0 = (warp - 1) * C::ROWS;
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, KT), idesc_o = umma_idesc_bf16(128, HDP);
-      const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
+      constexpr uint32_t idesc = umma_idesc_bf16(128, HDP);
+      int stage = 0;
+      uint32_t phase = 0, g = 0;  // g: steps so far
       bool alive = true;
-      // scores of a row's step in stage `st`, queries in buffer `qb`
-      auto scores = [&](int wg, int st, int qb) {
-        const uint32_t d = tmem_base + wg * C::TM_WG;
-        const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[st]), 128);
-        const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[qb][wg]), HDP * 2);
-        const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.k[st][wg]), HDP * 2);
-        if (leader && alive) {
-#pragma unroll
-          for (int kk = 0; kk < KT / 16; ++kk)
-            umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_s, kk != 0);
-#pragma unroll
-          for (int kk = 0; kk < HDP / 16; ++kk)
-            umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc_s, 1);
-          umma_commit(&sm.s_full[wg]);
-        }
-      };
-      int stage = 0, next_qb = 0;          // stage of the step whose P.V comes next, queries of the one after
-      uint32_t phase = 0, item_it = 0, g = 0;  // g: steps so far
-      if (blockIdx.x < p.total_items) {    // the first step's scores
-        alive = mbar_wait(&sm.q_full[0], 0, p.status, ST_TIMEOUT_MMA) && mbar_wait(&sm.st_full[0], 0, p.status, ST_TIMEOUT_MMA);
-        __syncwarp();
-        tc_fence_after();
-        for (int u = 0; u < C::ROWS; ++u) scores(r0 + u, 0, 0);
-        if (p.steps == 1 && leader && alive) umma_commit(&sm.q_empty[0]);
-      }
-      for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+      for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
         for (int t = 0; t < p.steps; ++t, ++g) {
-          const bool last = t + 1 == p.steps, more = !last || item + gridDim.x < p.total_items;
-          const int next = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t next_phase = next == 0 ? phase ^ 1 : phase;
-          if (last) next_qb ^= 1;
+          // (already complete when P arrives; observed here so that this thread's products are ordered after the
+          // TMA writes of V)
+          alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
 #pragma unroll 1
           for (int u = 0; u < C::ROWS; ++u) {
             const int wg = r0 + u;
             alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
-            if (u == 0 && more) {
-              alive = alive && mbar_wait(&sm.st_full[next], next_phase, p.status, ST_TIMEOUT_MMA);
-              if (last)
-                alive = alive && mbar_wait(&sm.q_full[next_qb], ((item_it + 1) / C::QBUF) & 1, p.status, ST_TIMEOUT_MMA);
-            }
             __syncwarp();
             tc_fence_after();
             const uint32_t base = tmem_base + wg * C::TM_WG;
@@ -661,19 +630,55 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
 #pragma unroll
                 for (int kk = 0; kk < KT / 16; ++kk)
                   umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
-                               idesc_o, t > 0 || (term | kk) != 0);
-              if (last) umma_commit(&sm.o_full[wg]);
+                               idesc, t > 0 || (term | kk) != 0);
+              umma_commit(&sm.pv_done[wg]);
             }
-            if (more) scores(wg, next, next_qb);
           }
-          if (leader && alive) {
-            umma_commit(&sm.st_empty[stage]);
-            // the last product with a buffer of queries has been issued: that of its item's last step
-            if (t + 2 == p.steps || (p.steps == 1 && more)) umma_commit(&sm.q_empty[next_qb]);
+          if (leader && alive) umma_commit(&sm.st_empty[stage]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
           }
-          stage = next;
-          phase = next_phase;
         }
+      }
+    } else if (warp == 3) {
+      const bool leader = elect_one();
+      constexpr uint32_t idesc = umma_idesc_bf16(128, KT);
+      const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
+      int stage = 0;
+      uint32_t phase = 0, item_it = 0, g = 0;
+      bool alive = true;
+      for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+        const uint32_t qb = item_it % C::QBUF;
+        alive = alive && mbar_wait(&sm.q_full[qb], (item_it / C::QBUF) & 1, p.status, ST_TIMEOUT_MMA);
+        for (int t = 0; t < p.steps; ++t, ++g) {
+          alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+          const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[stage]), 128);
+#pragma unroll 1
+          for (int wg = 0; wg < NWG; ++wg) {
+            // the scores' columns are free once the products that read P in them are through
+            alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA);
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t d = tmem_base + wg * C::TM_WG;
+            const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[qb][wg]), HDP * 2);
+            const uint64_t bdesc = umma_desc_kmajor(smem_u32(sm.k[stage][wg]), HDP * 2);
+            if (leader && alive) {
+#pragma unroll
+              for (int kk = 0; kk < KT / 16; ++kk)
+                umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
+#pragma unroll
+              for (int kk = 0; kk < HDP / 16; ++kk)
+                umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc, 1);
+              umma_commit(&sm.s_full[wg]);
+            }
+          }
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (leader && alive) umma_commit(&sm.q_empty[qb]);  // every product with these queries has been issued
       }
     }
   } else {
@@ -682,9 +687,9 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     const int row = quarter * 32 + lane;
     const uint32_t t_wg = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + wg * C::TM_WG;
     int stage = 0;
-    uint32_t phase = 0, g = 0, item_it = 0;
+    uint32_t phase = 0, g = 0;
     bool alive = true;
-    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
       float m_run = -INFINITY, l_run = 0.f;
       for (int t = 0; t < p.steps; ++t, ++g) {
         const bool st_there = mbar_test(&sm.st_full[stage], phase), s_there = mbar_test(&sm.s_full[wg], g & 1);
@@ -790,7 +795,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
           phase ^= 1;
         }
       }
-      alive = alive && mbar_wait(&sm.o_full[wg], item_it & 1, p.status, ST_TIMEOUT_SOFTMAX);
+      alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
       if (!__all_sync(0xffffffffu, alive)) break;
       tc_fence_after();
       int b, h, i, j0;
@@ -852,9 +857,10 @@ int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   return launch(att_bf16_kernel<HDP, NWG>, dim3(grid), dim3(C::THREADS), sizeof(BfSmem<HDP, NWG>), stream, pdl, tm, p);
 }
 
-// Rows of an item. A step of four takes 1.2 times as long as one of three (2.66 and 2.2 us), which pays
-// unless as many rounds of items are needed: 12 heads x 100 tokens, attention 63.4 us with four and 59.8 with three
-// (three rounds either way), 4 x 4 heads x 200 tokens 193 and 207 (11 and 15 rounds).
+// Rows of an item. A step of four takes some 1.2 times as long as one of three, which pays
+// unless as many rounds of items are needed: 12 heads x 100 tokens, attention 58.8 us with four and 55.7 with three
+// (three rounds either way), 4 x 4 heads x 200 tokens 173 and 183 (11 and 15 rounds). (Over 91 shapes of 20 to 320
+// tokens the rule takes the faster or loses up to 5 %, most with one or two rounds of one step.)
 template <int HDP>
 int launch_bf16_narrow(const Maps& tm, const Params& p, bool pdl, cudaStream_t stream) {
   auto rounds = [&](int rows) {

@@ -1,0 +1,36 @@
+"""The general bf16 attention core's products and what they read and overwrite. A row's scores go to tensor memory that the
+probabilities of the step before still occupy. Products of different shapes into different accumulators have no
+order among each other that the instruction set promises, so the warp that issues scores first waits for the products
+that read those probabilities. No run tells an order that was waited for from one that the
+hardware happens to keep, so this reads the kernel's source."""
+
+import re
+from pathlib import Path
+
+from test_core_joined_waits import _not_joined
+
+SOURCE = Path(__file__).resolve().parents[1] / "foldjax_b200" / "csrc" / "att_split.cu"
+
+
+def _control():
+    """The kernel's text of the warps that load and issue, one piece for each role."""
+    text = re.sub(r"//[^\n]*", "", SOURCE.read_text())
+    text = text[text.index("att_bf16_kernel("):]
+    text = text[text.index("setmaxnreg.dec"):text.index("setmaxnreg.inc")]
+    return re.split(r"\belse if \(warp\b", text)
+
+
+def test_scores_wait_for_the_products_that_read_the_probabilities():
+    scores = [role for role in _control() if "umma_bf16_ss(" in role]
+    values = [role for role in _control() if "umma_bf16_ts(" in role]
+    assert len(scores) == 1 and len(values) == 1 and scores != values
+    rows = scores[0][scores[0].rindex("for (int wg"):]
+    wait = r"mbar_wait\(&sm\.pv_done\[wg\], \(g & 1\) \^ 1,"
+    assert re.search(wait, rows[:rows.index("umma_bf16_ss(")])
+    assert re.search(r"umma_bf16_ts\([^;]*;\s*umma_commit\(&sm\.pv_done\[wg\]\);", values[0])
+
+
+def test_issuing_lane_does_not_run_ahead_of_its_warp():
+    for role in _control():
+        assert not _not_joined(role, r"\bif \([^)]*\bleader\b")
+        assert "break" not in role and "return" not in role
