@@ -328,7 +328,8 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     const uint32_t group = (warp - 12) >> 3, half = ((warp - 12) >> 2) & 1;
     const uint32_t d1 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * 128 + half * 32;
     for (uint32_t n = group; n < total_n; n += 2) {
-      if (!mbar_wait(&sm.d1_full[group], (n >> 1) & 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      // (a vote: each lane polls for itself, TMEM accesses take the whole warp, and all or none of it leave)
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.d1_full[group], (n >> 1) & 1, p.status, ST_TIMEOUT_EPILOGUE))) break;
       tc_fence_after();
       uint32_t hv[16];
 #pragma unroll
@@ -346,7 +347,7 @@ pair_transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.d1_empty[group]);
       // this group's previous second product must have read h before it is overwritten
-      if (!mbar_wait(&sm.h_empty[group], ((n >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_EPILOGUE)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.h_empty[group], ((n >> 1) & 1) ^ 1, p.status, ST_TIMEOUT_EPILOGUE))) break;
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         *reinterpret_cast<uint4*>(sm.h[group] + sw128_offset(row, half * 4 + q)) =
