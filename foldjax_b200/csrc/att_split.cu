@@ -281,13 +281,14 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         }
       };
       for (int t = 0; t < p.steps; ++t, ++g) {
-        if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) ||
-            !mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+        // (votes: each lane polls for itself, TMEM accesses take the whole warp, and all or none of it leave)
+        alive = mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) &&
+                mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX);
+        if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
           break;
         }
         tc_fence_after();
-        __syncwarp();
         float2 s[KT / 2];
         {
           uint32_t r0[32], r1[32];
@@ -343,7 +344,8 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         }
         l_run = fmaf(l_run, alpha_new, (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));
         // the previous step's P.V: its result is taken, then P may be overwritten
-        if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) {
+        alive = mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
+        if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
           break;
         }
@@ -367,9 +369,8 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         }
       }
       if (!alive) break;
-      if (!mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX))) break;
       tc_fence_after();
-      __syncwarp();
       take_pv();
       int b, h, i, j0;
       locate(item, b, h, i, j0);
