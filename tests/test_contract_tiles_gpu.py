@@ -1,7 +1,8 @@
 """The contraction in tiles of 256 rows (large n_k): a last tile whose second half has one row, a
 ragged one, or none, columns that end in partial blocks, one and two sources, bf16 results and
-float32 running sums; the last shape takes tiles of 128 rows. Then the same tiles over operands and a
-result in blocks of 64 rows, as the fused multiplication lays them out.
+float32 running sums; a shape with small n_k takes tiles of 128 rows, and so do, with 128 columns, the two of no
+more than 128 columns. Then the same tiles over operands and a result in blocks of 64 rows, as the fused
+multiplication lays them out.
 
 The float32 sum of m products is within m * 2^-23 of sum |a||b| of the exact one, however it is
 rounded; bf16 results are rounded once more (2^-8 relative)."""
@@ -16,7 +17,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("n_i,n_j,n_k,n_src", [(385, 513, 640, 2), (400, 40, 1000, 1), (521, 72, 1536, 1), (264, 300, 200, 1)])
+@pytest.mark.parametrize("n_i,n_j,n_k,n_src", [(385, 513, 640, 2), (400, 40, 1000, 1), (521, 72, 1536, 1), (264, 300, 200, 1),
+                                               (400, 140, 1000, 1), (400, 264, 1000, 1), (521, 140, 1536, 1), (521, 520, 1536, 1)])
 @pytest.mark.parametrize("running", [False, True])
 def test_contract(cuda_device, n_i, n_j, n_k, n_src, running):
     from foldjax_b200 import _lib, _device as dev
