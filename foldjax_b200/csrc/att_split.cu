@@ -18,9 +18,9 @@
 // NWG tiles of 128 queries), walked in steps of 64 keys:
 //   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
 //   warpgroups  softmax, one thread per query
-// Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (a score costs about 2
-// instructions of exponential, 3.5 of split and 4 others, most of them packed two to an instruction); the
-// rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
+// Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (counters, 512 tokens, 4 heads x
+// 32, 565 us; a score costs about 2 instructions of exponential, 3.5 of split and 4 others, most of them packed two to an
+// instruction; with 4.5 of split it was 41 % and 575); the rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
 #include "att_split.cuh"
 #include "gemm.cuh"
 #include "tc.cuh"
@@ -30,7 +30,6 @@ namespace b200 {
 namespace {
 
 constexpr int KT = 64;
-constexpr float RESCALE = 5.5f;  // probabilities stay below e^5.5
 
 template <int HDP, bool TOKEN>
 struct Cfg {
@@ -486,6 +485,9 @@ struct BfSmem {
   uint32_t tmem_base;
 };
 
+// The numerator is rescaled when a maximum exceeds the one that gave the offset by so much. An offset in whole log2
+// units lies up to half a unit below its maximum, so weights stay below e^5.5 * 2^0.5 = 346.
+constexpr float RESCALE = 5.5f;
 constexpr float LOG2E = 1.44269504f;
 constexpr float INTEGER_OFFSETS = 8388608.0f;  // 2^23: floats beyond are integers themselves
 
@@ -850,7 +852,7 @@ int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   p.groups = (p.n_i + NWG - 1) / NWG;
   p.tiles_j = (p.n + 127) / 128;
   const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
-  B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "attention: too many tiles");
+  B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "general attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
   const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_bf16_kernel<HDP, NWG>), (int)sizeof(BfSmem<HDP, NWG>));
   if (rc) return rc;
@@ -875,10 +877,10 @@ int launch_bf16_narrow(const Maps& tm, const Params& p, bool pdl, cudaStream_t s
 
 int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   B200_REQUIRE(a.head_dim % 8 == 0 && a.head_dim >= 8 && a.head_dim <= 64, B200TRI_ERR_UNSUPPORTED,
-               "float32 attention: head widths are multiples of 8 up to 64 (got %d)", a.head_dim);
+               "general attention: head widths are multiples of 8 up to 64 (got %d)", a.head_dim);
   const bool token = a.pieces != nullptr;
   B200_REQUIRE(!token || (!a.bf16 && a.batch == 1 && a.n_i == 1 && a.head_dim <= 32), B200TRI_ERR_INVALID,
-               "float32 attention: the gated form takes one row of heads up to 32 wide");
+               "general attention: the gated form takes one row of heads up to 32 wide");
   const uint32_t hdp = a.bf16 && a.head_dim <= 16 ? 16 : a.head_dim <= 32 ? 32 : 64;
   const Swz qk_swz = hdp == 16 ? Swz::B32 : hdp == 32 ? Swz::B64 : Swz::B128;
   const uint64_t hd = a.head_dim, heads = a.heads, width = hd * heads, n = a.n;
@@ -927,7 +929,7 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   p.gate = a.gate;
   p.pieces = a.pieces;
   p.status = device_status_word();
-  B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "float32 attention: no current CUDA device");
+  B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "general attention: no current CUDA device");
   if (token) return launch_cfg<32, true>(tm, p, a.pdl, stream);
   if (a.bf16 && hdp == 16) return launch_bf16_narrow<16>(tm, p, a.pdl, stream);
   if (a.bf16) return hdp == 32 ? launch_bf16_narrow<32>(tm, p, a.pdl, stream) : launch_bf16<64, 2>(tm, p, a.pdl, stream);

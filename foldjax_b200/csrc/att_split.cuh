@@ -1,4 +1,4 @@
-// Attention core with float32 operands carried as bf16 pieces (att_split.cu).
+// Attention core of any head shape, with bf16 operands or float32 ones carried as bf16 pieces (att_split.cu).
 #pragma once
 #include <cuda_bf16.h>
 

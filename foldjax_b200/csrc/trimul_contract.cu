@@ -197,7 +197,7 @@ contract_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     }
   } else if (warp >= 4) {
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    const int group = (warp - 4) >> 2;  // which 128 columns of the tile, or which half of its rows
+    const int group = (warp - 4) >> 2;  // which half of the tile's columns, or which of its rows
     constexpr int COLS = BN / (3 - H);   // columns of a warp
     const int first = H == 1 ? group * COLS : 0;
     uint8_t* staging = smem + STAGES * STAGE_BYTES + (warp - 4) * STAGED;

@@ -102,8 +102,12 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   }
   if (!p.early_weights) pdl_wait();
   LnParam ln_param;
-  if (threadIdx.x >= 128 && threadIdx.x < 384) 
-    ln_param.request(threadIdx.x < 192 ? p.ln[0] : threadIdx.x < 256 ? p.ln[1] : threadIdx.x < 320 ? p.ln[2] : p.ln[3], threadIdx.x & 63);
+  if (threadIdx.x >= 128 && threadIdx.x < 384)
+    ln_param.request(threadIdx.x < 192   ? p.ln[0]
+                     : threadIdx.x < 256 ? p.ln[1]
+                     : threadIdx.x < 320 ? p.ln[2]
+                                         : p.ln[3],
+                     threadIdx.x & 63);
   if (warp == 0 && lane == 0) {  // (the thread that initialised the barrier)
     mbar_expect_tx(&sm.w_full, 4 * SLAB_BYTES);
     for (int g = 0; g < 2; ++g)
@@ -139,53 +143,53 @@ finish_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
   // 640 threads x 96 registers = 128 x (40 + 88 + 144 + 2 x 104)
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-  if (warp == 0) {
-    if (elect_one()) {
-      int stage = 1;  // (stage 0 has the first tile)
-      uint32_t phase = 0;
-      for (uint32_t tile = blockIdx.x + gridDim.x; tile < p.total_tiles; tile += gridDim.x) {
-        int i, j0;
-        locate(tile, i, j0);
-        const int block = i / p.t_rpb;
-        if (!mbar_wait(&sm.in_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
-        load_in(stage, i, j0, block, i - block * p.t_rpb);
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
-      bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
-      int stage = 0;
-      uint32_t phase = 0, it = 0;
-      for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
-        const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&sm.acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
-        if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const uint32_t d_tmem = tmem_base + acc * 256 + g * 128;
-          const uint32_t in = smem_u32(g == 0 ? sm.x[stage] : sm.t[stage]);
-          const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w + g * 2 * SLAB_BYTES), SLAB_BYTES);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const uint64_t adesc = umma_desc_kmajor(in + (k >> 2) * SLAB_BYTES, 128);
-            umma_bf16_ss(d_tmem, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc, k != 0);
+    if (warp == 0) {
+      if (elect_one()) {
+        int stage = 1;  // (stage 0 has the first tile)
+        uint32_t phase = 0;
+        for (uint32_t tile = blockIdx.x + gridDim.x; tile < p.total_tiles; tile += gridDim.x) {
+          int i, j0;
+          locate(tile, i, j0);
+          const int block = i / p.t_rpb;
+          if (!mbar_wait(&sm.in_empty[stage], phase ^ 1, p.status, ST_TIMEOUT_PRODUCER)) break;
+          load_in(stage, i, j0, block, i - block * p.t_rpb);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
           }
         }
-        umma_commit(&sm.in_empty[stage]);
-        umma_commit(&sm.acc_full[acc]);
-        if (++stage == STAGES) {
-          stage = 0;
-          phase ^= 1;
+      }
+    } else if (warp == 1) {
+      if (elect_one()) {
+        constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | UMMA_B_MN;
+        bool alive = mbar_wait(&sm.w_full, 0, p.status, ST_TIMEOUT_MMA);
+        int stage = 0;
+        uint32_t phase = 0, it = 0;
+        for (uint32_t tile = blockIdx.x; tile < p.total_tiles && alive; tile += gridDim.x, ++it) {
+          const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
+          if (!mbar_wait(&sm.acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_MMA)) break;
+          if (!mbar_wait(&sm.xn_full[stage], phase, p.status, ST_TIMEOUT_MMA)) break;
+          tc_fence_after();
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const uint32_t d_tmem = tmem_base + acc * 256 + g * 128;
+            const uint32_t in = smem_u32(g == 0 ? sm.x[stage] : sm.t[stage]);
+            const uint64_t bdesc = umma_desc_mnmajor(smem_u32(sm.w + g * 2 * SLAB_BYTES), SLAB_BYTES);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const uint64_t adesc = umma_desc_kmajor(in + (k >> 2) * SLAB_BYTES, 128);
+              umma_bf16_ss(d_tmem, umma_desc_advance(adesc, (k & 3) * 32), umma_desc_advance(bdesc, k * 2048), idesc, k != 0);
+            }
+          }
+          umma_commit(&sm.in_empty[stage]);
+          umma_commit(&sm.acc_full[acc]);
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
       }
     }
-  }
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     (threadIdx.x < 192 ? sm.gamma_in : sm.beta_in)[threadIdx.x & 63] = ln_param.word();
