@@ -337,7 +337,8 @@ typedef struct {
    * triangle_attention_forward builds its mask bias (triangle_attention.py:138-142).
    * 1: `mask` already is the additive mask bias [n_i][n_k] the reference's attention-core
    * operators receive (0, a soft negative bias, -1e9 or -infinity); `inf` is ignored.
-   * Either way a bias at or below -30000 drops the key. */
+   * Either way a bias at or below -30000 drops the key: its score is -30000, which has no weight beside
+   * kept keys that score above some -29980. */
   int32_t mask_additive;
 } b200tri_triatt_core_args;
 
