@@ -35,24 +35,21 @@ struct LnParam {
 
 // The operations below and their order are part of the result: a statistic that differs in its last
 // bit flips some roundings to bf16 later on, and a stack of blocks amplifies those. Where two
-// operations of the same kind are independent they share an instruction.
+// operations of the same kind are independent they share an instruction, and a bf16 value is added by a mixed-precision
+// fma instead of being unpacked for it (multiplication of 1003 tokens 737 -> 725 us, block of 203 278 -> 276, the same bits).
 
-// bf16 pair -> float pair
-__device__ __forceinline__ float2 ln_unpack(uint32_t w) { return make_float2(bf16_lo(w), bf16_hi(w)); }
 // normed.astype(bf16) * scale + bias, each step rounded to bf16
 __device__ __forceinline__ uint32_t ln_affine(uint32_t w, float2 minus_mean, float2 rstd, uint32_t gamma, uint32_t beta) {
-  const float2 n = __fmul2_rn(__fadd2_rn(ln_unpack(w), minus_mean), rstd);
+  const float2 n = __fmul2_rn(add_bf16x2(minus_mean, w), rstd);
   return bf16x2_add(bf16x2_mul(pack_bf16x2(n.x, n.y), gamma), beta);
 }
 // One step of each statistic in one accumulator: a word's two channels are added to each other
 // first; their squared deviations one after the other.
 __device__ __forceinline__ float ln_add4(float sum, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
-  const float2 a = __fadd2_rn(make_float2(bf16_lo(w0), bf16_lo(w1)), make_float2(bf16_hi(w0), bf16_hi(w1)));
-  const float2 b = __fadd2_rn(make_float2(bf16_lo(w2), bf16_lo(w3)), make_float2(bf16_hi(w2), bf16_hi(w3)));
-  return (((sum + a.x) + a.y) + b.x) + b.y;
+  return (((sum + sum_bf16x2(w0)) + sum_bf16x2(w1)) + sum_bf16x2(w2)) + sum_bf16x2(w3);
 }
 __device__ __forceinline__ float ln_square(float sq, uint32_t w, float2 minus_mean) {
-  const float2 d = __fadd2_rn(ln_unpack(w), minus_mean);
+  const float2 d = add_bf16x2(minus_mean, w);
   return fmaf(d.y, d.y, fmaf(d.x, d.x, sq));
 }
 
@@ -130,8 +127,8 @@ __device__ __forceinline__ void ln_row_two_threads(uint8_t* tile, int row, int h
   float2 s[2] = {}, q[2] = {};  // the four partial sums: words 0, 1 | 2, 3 of each chunk
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    s[0] = __fadd2_rn(s[0], __fadd2_rn(make_float2(bf16_lo(v[c].x), bf16_lo(v[c].y)), make_float2(bf16_hi(v[c].x), bf16_hi(v[c].y))));
-    s[1] = __fadd2_rn(s[1], __fadd2_rn(make_float2(bf16_lo(v[c].z), bf16_lo(v[c].w)), make_float2(bf16_hi(v[c].z), bf16_hi(v[c].w))));
+    s[0] = __fadd2_rn(s[0], make_float2(sum_bf16x2(v[c].x), sum_bf16x2(v[c].y)));
+    s[1] = __fadd2_rn(s[1], make_float2(sum_bf16x2(v[c].z), sum_bf16x2(v[c].w)));
   }
   float sum = (s[0].x + s[0].y) + (s[1].x + s[1].y);
   sum += __shfl_xor_sync(0xffffffffu, sum, 16);
@@ -142,8 +139,8 @@ __device__ __forceinline__ void ln_row_two_threads(uint8_t* tile, int row, int h
     const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const float2 a = __fadd2_rn(make_float2(bf16_lo(w[2 * u]), bf16_lo(w[2 * u + 1])), mm);
-      const float2 b = __fadd2_rn(make_float2(bf16_hi(w[2 * u]), bf16_hi(w[2 * u + 1])), mm);
+      const float2 d0 = add_bf16x2(mm, w[2 * u]), d1 = add_bf16x2(mm, w[2 * u + 1]);
+      const float2 a = make_float2(d0.x, d1.x), b = make_float2(d0.y, d1.y);
       q[u] = __ffma2_rn(b, b, __ffma2_rn(a, a, q[u]));
     }
   }

@@ -369,6 +369,33 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// v + a packed pair's two values, rounded once: an instruction each, against two to unpack and half a packed addition.
+__device__ __forceinline__ float2 add_bf16x2(float2 v, uint32_t w) {
+  float2 r;
+  asm("{\n"
+      " .reg .b16 lo, hi, one;\n"
+      " mov.b32 {lo, hi}, %2;\n"
+      " mov.b16 one, 0x3F80;\n"
+      " fma.rn.f32.bf16 %0, lo, one, %3;\n"
+      " fma.rn.f32.bf16 %1, hi, one, %4;\n"
+      "}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "r"(w), "f"(v.x), "f"(v.y));
+  return r;
+}
+// The sum of a packed pair's two values.
+__device__ __forceinline__ float sum_bf16x2(uint32_t w) {
+  float r;
+  asm("{\n"
+      " .reg .b16 lo, hi, one;\n"
+      " mov.b32 {lo, hi}, %1;\n"
+      " mov.b16 one, 0x3F80;\n"
+      " fma.rn.f32.bf16 %0, lo, one, %2;\n"
+      "}\n"
+      : "=f"(r)
+      : "r"(w), "f"(bf16_hi(w)));
+  return r;
+}
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Packed bf16 arithmetic (the _rn forms, which the compiler may not contract into
