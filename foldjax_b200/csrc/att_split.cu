@@ -21,6 +21,8 @@
 // Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (counters, 512 tokens, 4 heads x
 // 32, 565 us; a score costs about 2 instructions of exponential, 3.5 of split and 4 others, most of them packed two to an
 // instruction; with 4.5 of split it was 41 % and 575); the rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
+#include <type_traits>
+
 #include "att_split.cuh"
 #include "gemm.cuh"
 #include "tc.cuh"
@@ -80,7 +82,7 @@ __device__ __forceinline__ float2 exp_below(float2 s, float2 minus_m) {
   return make_float2(fast_exp2(t.x), fast_exp2(t.y));
 }
 
-template <int HDP, bool TOKEN>
+template <int HDP, bool TOKEN, int LAST>
 __global__ void __launch_bounds__(Cfg<HDP, TOKEN>::THREADS, 1)
 att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
   using C = Cfg<HDP, TOKEN>;
@@ -179,7 +181,6 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, KT);
       int stage = 0;
       uint32_t phase = 0, item_it = 0, g = 0;
       bool alive = true;
@@ -190,6 +191,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
             alive = false;
             break;
           }
+          const uint32_t idesc = umma_idesc_bf16(128, LAST < KT && t + 1 == p.steps ? LAST : KT);
           for (int wg = 0; wg < NWG; ++wg) {
             if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
               alive = false;
@@ -228,6 +230,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
             alive = false;
             break;
           }
+          const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
           for (int wg = 0; wg < NWG; ++wg) {
             if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
               alive = false;
@@ -240,7 +243,8 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
               const uint64_t vdesc = umma_desc_kmajor(smem_u32(sm.v[stage][TOKEN ? 0 : wg][TP::b(term)]), 128);
 #pragma unroll
               for (int kk = 0; kk < KT / 16; ++kk)
-                umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
+                if (kk * 16 < LAST || kk * 16 < cols)
+                  umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
                              idesc, (term | kk) != 0);
             }
             umma_commit(&sm.pv_done[wg]);
@@ -279,35 +283,36 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           }
         }
       };
-      for (int t = 0; t < p.steps; ++t, ++g) {
+      // A step of COLS keys; what the last one leaves out of 64 are keys that do not exist.
+      auto step = [&](auto width, int t) -> bool {
+        constexpr int COLS = decltype(width)::value;
         // (votes: each lane polls for itself, TMEM accesses take the whole warp, and all or none of it leave)
         alive = mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX) &&
                 mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX);
         if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
-          break;
+          return false;
         }
         tc_fence_after();
-        float2 s[KT / 2];
+        float2 s[COLS / 2];
         {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(t_wg + C::TM_S, r0);
-          tmem_ld32(t_wg + C::TM_S + 32, r1);
+          uint32_t r[COLS];
+          if constexpr (COLS >= 32) tmem_ld32(t_wg + C::TM_S, reinterpret_cast<uint32_t(&)[32]>(r));
+          if constexpr (COLS == 64) tmem_ld32(t_wg + C::TM_S + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+          if constexpr (COLS % 32 == 16) tmem_ld16(t_wg + C::TM_S + COLS - 16, reinterpret_cast<uint32_t(&)[16]>(r[COLS - 16]));
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            s[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
-            s[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
-          }
+          for (int e = 0; e < COLS / 2; ++e) s[e] = make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
         }
         tc_fence_before();
         mbar_arrive(&sm.s_free[wg]);
         const float* mrow = sm.mb[stage][TOKEN ? 0 : wg];
-        const bool masked = __any_sync(0xffffffffu, mrow[lane] != 0.f || mrow[lane + 32] != 0.f);
+        const bool masked = __any_sync(0xffffffffu, ((COLS >= 32 || lane < COLS) && mrow[lane] != 0.f) ||
+                                                         ((COLS == 64 || lane + 32 < COLS) && mrow[lane + 32] != 0.f));
         // the reference's order of the two sums
         const uint8_t* brow = sm.bias[stage][TOKEN ? wg : 0];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < COLS / 4; ++c) {
           const float4 b4 = *reinterpret_cast<const float4*>(brow + (c >> 3) * 16384 + sw128_offset(row, c & 7));
           const float2 b2[2] = {make_float2(b4.x, b4.y), make_float2(b4.z, b4.w)};
           float2 m2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
@@ -328,7 +333,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         if (lane == 0) mbar_arrive(&sm.st_empty[stage]);
         float mxa = m_run, mxb = s[0].x;
 #pragma unroll
-        for (int e = 0; e < KT / 2; e += 2) {
+        for (int e = 0; e < COLS / 2; e += 2) {
           mxa = fmax3(mxa, s[e].x, s[e].y);
           mxb = fmax3(mxb, s[e + 1].x, s[e + 1].y);
         }
@@ -337,7 +342,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         m_run = mx;
         float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-        for (int e = 0; e < KT / 2; ++e) {
+        for (int e = 0; e < COLS / 2; ++e) {
           s[e] = exp_below(s[e], make_float2(-mx, -mx));
           l2[e & 1] = __fadd2_rn(l2[e & 1], s[e]);
         }
@@ -346,13 +351,13 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
         alive = mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
         if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
-          break;
+          return false;
         }
         tc_fence_after();
         if (t > 0) take_pv();
         alpha = alpha_new;
 #pragma unroll
-        for (int oct = 0; oct < 4; ++oct) {  // 16 keys at a time: few live registers
+        for (int oct = 0; oct < COLS / 16; ++oct) {  // 16 keys at a time: few live registers
           uint32_t pc[3][8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) split3x2(s[oct * 8 + e].x, s[oct * 8 + e].y, pc[0][e], pc[1][e], pc[2][e]);
@@ -366,6 +371,14 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
           stage = 0;
           phase ^= 1;
         }
+        return true;
+      };
+      const int whole = LAST < KT ? p.steps - 1 : p.steps;
+      for (int t = 0; t < whole; ++t, ++g)
+        if (!step(std::integral_constant<int, KT>{}, t)) break;
+      if constexpr (LAST < KT) {
+        if (alive) step(std::integral_constant<int, LAST>{}, whole);
+        ++g;
       }
       if (!alive) break;
       if (!__all_sync(0xffffffffu, mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX))) break;
@@ -416,6 +429,19 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
+// Calls go with the columns of an item's last step as a constant: 16, 32, 48 or 64, whichever hold the keys that are left.
+// (Templates of 200 tokens 610 -> 590 us, 150-token refiner 499 -> 487, 200-token float32 stack 644 -> 642, blocks of 136 and
+// 203 tokens, single track only, 198.7 -> 197.2 and 262.7 -> 261.6; the same bits.)
+template <class F>
+int with_last_columns(const Params& p, const F& go) {
+  switch (round_up(p.n - KT * (p.steps - 1), 16)) {
+    case 16: return go(std::integral_constant<int, 16>{});
+    case 32: return go(std::integral_constant<int, 32>{});
+    case 48: return go(std::integral_constant<int, 48>{});
+  }
+  return go(std::integral_constant<int, KT>{});
+}
+
 template <int HDP, bool TOKEN>
 int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   using C = Cfg<HDP, TOKEN>;
@@ -425,12 +451,13 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "float32 attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
-  const int rc =
-      ensure_smem_limit(reinterpret_cast<const void*>(att_split_kernel<HDP, TOKEN>), (int)sizeof(Smem<HDP, TOKEN>));
-  if (rc) return rc;
-  const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
-  return launch(att_split_kernel<HDP, TOKEN>, dim3(grid), dim3(C::THREADS),
-                sizeof(Smem<HDP, TOKEN>), stream, pdl, tm, p);
+  return with_last_columns(p, [&](auto last) {
+    const auto kernel = att_split_kernel<HDP, TOKEN, decltype(last)::value>;
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem<HDP, TOKEN>));
+    if (rc) return rc;
+    const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
+    return launch(kernel, dim3(grid), dim3(C::THREADS), sizeof(Smem<HDP, TOKEN>), stream, pdl, tm, p);
+  });
 }
 
 
@@ -505,7 +532,7 @@ __device__ __forceinline__ void split3n2(float2 v, uint32_t& hi, uint32_t& mid, 
   lo = upper_halves(less_bf16x2(r, mid));
 }
 
-template <int HDP, int NWG>
+template <int HDP, int NWG, int LAST>
 __global__ void __launch_bounds__(BfCfg<HDP, NWG>::THREADS, 1)
 att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
   using C = BfCfg<HDP, NWG>;
@@ -619,6 +646,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
           // (already complete when P arrives; observed here so that this thread's products are ordered after the
           // TMA writes of V)
           alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+          const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
 #pragma unroll 1
           for (int u = 0; u < C::ROWS; ++u) {
             const int wg = r0 + u;
@@ -632,8 +660,9 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
               for (int term = 0; term < TP::N; ++term)
 #pragma unroll
                 for (int kk = 0; kk < KT / 16; ++kk)
-                  umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
-                               idesc, t > 0 || (term | kk) != 0);
+                  if (kk * 16 < LAST || kk * 16 < cols)
+                    umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
+                                 idesc, t > 0 || (term | kk) != 0);
               umma_commit(&sm.pv_done[wg]);
             }
           }
@@ -646,7 +675,6 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
       }
     } else if (warp == 3) {
       const bool leader = elect_one();
-      constexpr uint32_t idesc = umma_idesc_bf16(128, KT);
       const uint64_t identdesc = umma_desc_kmajor(smem_u32(sm.ident), 128);
       int stage = 0;
       uint32_t phase = 0, item_it = 0, g = 0;
@@ -656,6 +684,8 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
         alive = alive && mbar_wait(&sm.q_full[qb], (item_it / C::QBUF) & 1, p.status, ST_TIMEOUT_MMA);
         for (int t = 0; t < p.steps; ++t, ++g) {
           alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+          const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
+          const uint32_t idesc = umma_idesc_bf16(128, cols);
           const uint64_t biasdesc = umma_desc_kmajor(smem_u32(sm.bias[stage]), 128);
 #pragma unroll 1
           for (int wg = 0; wg < NWG; ++wg) {
@@ -669,7 +699,8 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
             if (leader && alive) {
 #pragma unroll
               for (int kk = 0; kk < KT / 16; ++kk)
-                umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
+                if (kk * 16 < LAST || kk * 16 < cols)
+                  umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
 #pragma unroll
               for (int kk = 0; kk < HDP / 16; ++kk)
                 umma_bf16_ss(d, umma_desc_advance(adesc, kk * 32), umma_desc_advance(bdesc, kk * 32), idesc, 1);
@@ -694,32 +725,33 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
     bool alive = true;
     for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
       float m_run = -INFINITY, l_run = 0.f;
-      for (int t = 0; t < p.steps; ++t, ++g) {
+      // (a step of COLS keys, as above)
+      auto step = [&](auto width, int t) -> bool {
+        constexpr int COLS = decltype(width)::value;
         const bool st_there = mbar_test(&sm.st_full[stage], phase), s_there = mbar_test(&sm.s_full[wg], g & 1);
         alive = (st_there || mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_SOFTMAX)) &&
                 (s_there || mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX));
         if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
-          break;
+          return false;
         }
         tc_fence_after();
-        const float mk0 = sm.mb[stage][wg][lane], mk1 = sm.mb[stage][wg][lane + 32];
-        float2 s[KT / 2];
+        const float mk0 = COLS >= 32 || lane < COLS ? sm.mb[stage][wg][lane] : 0.f;
+        const float mk1 = COLS == 64 || lane + 32 < COLS ? sm.mb[stage][wg][lane + 32] : 0.f;
+        float2 s[COLS / 2];
         {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(t_wg, r0);
-          tmem_ld32(t_wg + 32, r1);
+          uint32_t r[COLS];
+          if constexpr (COLS >= 32) tmem_ld32(t_wg, reinterpret_cast<uint32_t(&)[32]>(r));
+          if constexpr (COLS == 64) tmem_ld32(t_wg + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+          if constexpr (COLS % 32 == 16) tmem_ld16(t_wg + COLS - 16, reinterpret_cast<uint32_t(&)[16]>(r[COLS - 16]));
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            s[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
-            s[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
-          }
+          for (int e = 0; e < COLS / 2; ++e) s[e] = make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
         }
         if (__any_sync(0xffffffffu, mk0 != 0.f || mk1 != 0.f)) {
           const float* mrow = sm.mb[stage][wg];
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
+          for (int c = 0; c < COLS / 4; ++c) {
             const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
             s[2 * c] = __fadd2_rn(s[2 * c], make_float2(m4.x, m4.y));
             s[2 * c + 1] = __fadd2_rn(s[2 * c + 1], make_float2(m4.z, m4.w));
@@ -731,7 +763,7 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
         float mxa = fmaxf(s[0].x, s[0].y), mxb = fmaxf(s[1].x, s[1].y);
         float mxc = fmaxf(s[2].x, s[2].y), mxd = fmaxf(s[3].x, s[3].y);
 #pragma unroll
-        for (int e = 4; e < KT / 2; e += 4) {
+        for (int e = 4; e < COLS / 2; e += 4) {
           mxa = fmax3(mxa, s[e].x, s[e].y);
           mxb = fmax3(mxb, s[e + 1].x, s[e + 1].y);
           mxc = fmax3(mxc, s[e + 2].x, s[e + 2].y);
@@ -770,13 +802,13 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
             minus_off = 0.f;
           }
 #pragma unroll
-          for (int e = 0; e < KT / 2; ++e) s[e] = __fadd2_rn(s[e], minus_m);
+          for (int e = 0; e < COLS / 2; ++e) s[e] = __fadd2_rn(s[e], minus_m);
           __syncwarp();
         }
         const float2 log2e2 = make_float2(LOG2E, LOG2E), off2 = make_float2(minus_off, minus_off);
         float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-        for (int half = 0; half < 4; ++half) {
+        for (int half = 0; half < COLS / 16; ++half) {
           uint32_t pc[3][8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
@@ -797,6 +829,14 @@ att_bf16_kernel(const __grid_constant__ Maps tm, const Params p) {
           stage = 0;
           phase ^= 1;
         }
+        return true;
+      };
+      const int whole = LAST < KT ? p.steps - 1 : p.steps;
+      for (int t = 0; t < whole; ++t, ++g)
+        if (!step(std::integral_constant<int, KT>{}, t)) break;
+      if constexpr (LAST < KT) {
+        if (alive) step(std::integral_constant<int, LAST>{}, whole);
+        ++g;
       }
       alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
       if (!__all_sync(0xffffffffu, alive)) break;
@@ -854,10 +894,13 @@ int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "general attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
-  const int rc = ensure_smem_limit(reinterpret_cast<const void*>(att_bf16_kernel<HDP, NWG>), (int)sizeof(BfSmem<HDP, NWG>));
-  if (rc) return rc;
-  const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
-  return launch(att_bf16_kernel<HDP, NWG>, dim3(grid), dim3(C::THREADS), sizeof(BfSmem<HDP, NWG>), stream, pdl, tm, p);
+  return with_last_columns(p, [&](auto last) {
+    const auto kernel = att_bf16_kernel<HDP, NWG, decltype(last)::value>;
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(BfSmem<HDP, NWG>));
+    if (rc) return rc;
+    const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
+    return launch(kernel, dim3(grid), dim3(C::THREADS), sizeof(BfSmem<HDP, NWG>), stream, pdl, tm, p);
+  });
 }
 
 // Rows of an item. A step of four takes some 1.2 times as long as one of three, which pays

@@ -64,6 +64,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "host.cuh"
 #include "tc.cuh"
@@ -165,7 +166,11 @@ __device__ __forceinline__ float2 poly_exp2x2(float2 u, float2 log2e2, float2 ma
                      __int_as_float(__float_as_int(q.y) + (__float_as_int(y.y) << 23)));
 }
 
-template <int TILES>
+// LAST: columns of an item's last step that are computed, 16, 32, 48 or 64, whichever hold the keys that are left.
+// A constant, because a choice by size inside one kernel cost the whole steps 3 to 4 % (n = 384: 99.6 us, 102.8
+// so). Attention operator of 136 / 203 / 300 tokens 20.1 -> 18.7, 32.8 -> 30.6, 73.6 -> 71.8 us, block of 203 tokens 266.7 ->
+// 261.6. More than ONE_MAP_STEPS steps have little to gain and key tiles are whole steps: those walk 64.
+template <int TILES, int LAST>
 __global__ void __launch_bounds__(THREADS, 1)
 att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ TileMaps<TILES> tm, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -290,7 +295,6 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // neither product waits behind the other's barrier. All lanes walk the loops and one of
     // them issues, so that control flow and descriptors stay in uniform registers.
     const bool leader = elect_one();
-    constexpr uint32_t idesc_qk = umma_idesc_bf16(128, KT);
     const uint64_t identdesc = desc_sw128(smem_u32(sm.ident));
     int stage = 0;
     uint32_t phase = 0, item_it = 0, g = 0;  // g: global step counter
@@ -300,6 +304,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       alive = alive && mbar_wait(&sm.q_full[qb], (item_it / QBUF) & 1, p.status, ST_TIMEOUT_MMA);
       for (int t = 0; t < p.steps; ++t, ++g) {
         alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+        const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
+        const uint32_t idesc = umma_idesc_bf16(128, cols);
         const uint64_t biasdesc = desc_sw128(smem_u32(sm.bias[stage]));
 #pragma unroll
         for (int wg = 0; wg < NWG; ++wg) {
@@ -312,9 +318,10 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (leader && alive) {
 #pragma unroll
             for (int kk = 0; kk < KT / 16; ++kk)
-              umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc_qk, kk != 0);
-            umma_bf16_ss(d, adesc, bdesc, idesc_qk, 1);
-            umma_bf16_ss(d, umma_desc_advance(adesc, 32), umma_desc_advance(bdesc, 32), idesc_qk, 1);
+              if (kk * 16 < LAST || kk * 16 < cols)
+                umma_bf16_ss(d, umma_desc_advance(biasdesc, kk * 32), umma_desc_advance(identdesc, kk * 32), idesc, kk != 0);
+            umma_bf16_ss(d, adesc, bdesc, idesc, 1);
+            umma_bf16_ss(d, umma_desc_advance(adesc, 32), umma_desc_advance(bdesc, 32), idesc, 1);
             umma_commit(&sm.s_full[wg]);
           }
         }
@@ -337,6 +344,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // (already complete when P arrives; observed here so this thread's products
         // are ordered after the TMA writes of V)
         alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+        const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
         for (int wg = 0; wg < NWG; ++wg) {
           alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
           __syncwarp();
@@ -347,7 +355,8 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (leader && alive) {
 #pragma unroll
             for (int k = 0; k < KT / 16; ++k)
-              umma_bf16_ts(d, a + k * 8, umma_desc_advance(vdesc, k * 32), idesc_pv, (t | k | p.resume) != 0);
+              if (k * 16 < LAST || k * 16 < cols)
+                umma_bf16_ts(d, a + k * 8, umma_desc_advance(vdesc, k * 32), idesc_pv, (t | k | p.resume) != 0);
             umma_commit(&sm.pv_done[wg]);
           }
         }
@@ -412,7 +421,10 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tmem_st_wait();
         tc_fence_before();
       }
-      for (int t = 0; t < p.steps; ++t, ++g) {
+      // A step of COLS keys. What the last one (LAST) leaves out of 64 are keys that do not exist, whose weights are zero:
+      // the same bits.
+      auto step = [&](auto width, int t) -> bool {
+        constexpr int COLS = decltype(width)::value;
         // (both asked at once: nearly always there already, and one latency instead of two. Each lane polls
         // for itself; the vote brings them together again, as the TMEM accesses need, and has all or
         // none of them leave)
@@ -421,25 +433,24 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 (s_there || mbar_wait(&sm.s_full[wg], g & 1, p.status, ST_TIMEOUT_SOFTMAX));
         if (!__all_sync(0xffffffffu, alive)) {
           alive = false;
-          break;
+          return false;
         }
         tc_fence_after();
         // (fetched here, long before the vote that needs them)
-        const float mk0 = sm.mb[stage][wg][lane], mk1 = sm.mb[stage][wg][lane + 32];
+        const float mk0 = COLS >= 32 || lane < COLS ? sm.mb[stage][wg][lane] : 0.f;
+        const float mk1 = COLS == 64 || lane + 32 < COLS ? sm.mb[stage][wg][lane + 32] : 0.f;
         // Scores, bias and mask travel as fp32 pairs: sm_100 adds/multiplies two
         // fp32 values per instruction (add/fma .f32x2), halving the softmax's ALU work.
-        float2 u[KT / 2];
+        float2 u[COLS / 2];
         {
-          // q.k + bias arrives from the tensor core; both halves are requested at once.
-          uint32_t r0[32], r1[32];
-          tmem_ld32(t_wg + TM_S, r0);
-          tmem_ld32(t_wg + TM_S + 32, r1);
+          // q.k + bias arrives from the tensor core; all columns are requested at once.
+          uint32_t r[COLS];
+          if constexpr (COLS >= 32) tmem_ld32(t_wg + TM_S, reinterpret_cast<uint32_t(&)[32]>(r));
+          if constexpr (COLS == 64) tmem_ld32(t_wg + TM_S + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+          if constexpr (COLS % 32 == 16) tmem_ld16(t_wg + TM_S + COLS - 16, reinterpret_cast<uint32_t(&)[16]>(r[COLS - 16]));
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            u[e] = make_float2(__uint_as_float(r0[2 * e]), __uint_as_float(r0[2 * e + 1]));
-            u[16 + e] = make_float2(__uint_as_float(r1[2 * e]), __uint_as_float(r1[2 * e + 1]));
-          }
+          for (int e = 0; e < COLS / 2; ++e) u[e] = make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.s_free[wg]);  // (an arrival per thread keeps the LSU busier)
@@ -448,7 +459,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const bool masked = __any_sync(0xffffffffu, (mk0 != 0.f) || (mk1 != 0.f));
         if (masked) {
 #pragma unroll
-          for (int c = 0; c < KT / 4; ++c) {
+          for (int c = 0; c < COLS / 4; ++c) {
             const float4 m4 = *reinterpret_cast<const float4*>(mrow + 4 * c);
             const float mv[4] = {m4.x, m4.y, m4.z, m4.w};
             float uu[4] = {u[2 * c].x, u[2 * c].y, u[2 * c + 1].x, u[2 * c + 1].y};
@@ -465,7 +476,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         float mxa = fmaxf(u[0].x, u[0].y), mxb = fmaxf(u[1].x, u[1].y);
         float mxc = fmaxf(u[2].x, u[2].y), mxd = fmaxf(u[3].x, u[3].y);
 #pragma unroll
-        for (int e = 4; e < KT / 2; e += 4) {
+        for (int e = 4; e < COLS / 2; e += 4) {
           mxa = fmax3(mxa, u[e].x, u[e].y);
           mxb = fmax3(mxb, u[e + 1].x, u[e + 1].y);
           mxc = fmax3(mxc, u[e + 2].x, u[e + 2].y);
@@ -497,10 +508,13 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const bool p_free = mbar_test(&sm.pv_done[wg], (g & 1) ^ 1);
           const float u_min = (m2_used - 120.0f) * LN2;  // keeps the polynomial path's t above about -120
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            uint32_t packed[16];
+          for (int half = 0; half < (COLS + 31) / 32; ++half) {
+            constexpr int MOST = COLS < 32 ? 8 : 16;
+            const int pairs = COLS == 48 && half == 1 ? 8 : MOST;
+            uint32_t packed[MOST];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
+            for (int e = 0; e < MOST; ++e) {
+              if (e >= pairs) continue;
               const float2 ue = u[16 * half + e];
               float2 ex;
               if (((e + 1) * POLY) / 16 != (e * POLY) / 16) {  // spread evenly over the half
@@ -519,7 +533,10 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               __syncwarp();
               tc_fence_after();
             }
-            tmem_st16(t_wg + TM_P + 16 * half, packed);
+            if constexpr (MOST == 16) {
+              if (pairs == 16) tmem_st16(t_wg + TM_P + 16 * half, packed);
+            }
+            if (pairs == 8) tmem_st8(t_wg + TM_P + 16 * half, reinterpret_cast<const uint32_t(&)[8]>(packed));
           }
         }
         if ((t > 0 || p.resume) && any_need) {
@@ -544,8 +561,15 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           stage = 0;
           phase ^= 1;
         }
+        return true;
+      };
+      const int whole = LAST < KT ? p.steps - 1 : p.steps;
+      for (int t = 0; t < whole; ++t, ++g)
+        if (!step(std::integral_constant<int, KT>{}, t)) break;
+      if constexpr (LAST < KT) {  // (all lanes, also where a wait has run out: its vote has them leave together)
+        step(std::integral_constant<int, LAST>{}, whole);
+        ++g;
       }
-      if (!alive) break;
       // ---- item epilogue: O / l -> bf16 -> o[i][j][h*32 ..]
       alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
       if (!__all_sync(0xffffffffu, alive)) break;
@@ -779,9 +803,14 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
     TimedLaunch timed(K_TRIATT_CORE, stream, may_time);
     return launch(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), sizeof(Smem), stream, true, tm_q, tiles_maps, p);
   };
-  if (many_maps) return go(att_core_kernel<MAX_KEY_TILES>, tm);
+  if (many_maps) return go(att_core_kernel<MAX_KEY_TILES, KT>, tm);
   const TileMaps<1> one = {{tm.k[0]}, {tm.v[0]}, {tm.b[0]}, {tm.m[0]}};
-  return go(att_core_kernel<1>, one);
+  switch (round_up(a->n_k - KT * (p.steps - 1), 16)) {
+    case 16: return go(att_core_kernel<1, 16>, one);
+    case 32: return go(att_core_kernel<1, 32>, one);
+    case 48: return go(att_core_kernel<1, 48>, one);
+  }
+  return go(att_core_kernel<1, KT>, one);
 }
 }  // namespace
 
