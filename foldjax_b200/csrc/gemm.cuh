@@ -101,6 +101,9 @@ struct GemmShape {
   int m_tiles, n_tiles, splits;
   int kb[2];  // k steps of 64 per segment
   int* status;
+  // set by the launch: k steps of a split, and what tile numbers are divided by
+  int per[2];
+  Divisor by_splits, fast;  // (fast: tiles of the direction that successive tiles walk)
 };
 
 // What a policy P provides:
@@ -212,13 +215,10 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
   // (32-bit tile arithmetic: a 64-bit division costs a role several hundred cycles per tile)
   const uint32_t total = static_cast<uint32_t>(g.m_tiles) * g.n_tiles * g.splits;
   auto locate = [&](uint32_t tile, int& split, int& m_tile, int& n_tile) {
-    split = 0;
-    if (g.splits > 1) {
-      split = static_cast<int>(tile % g.splits);
-      tile /= g.splits;
-    }
-    const uint32_t fast = P::M_FAST ? g.m_tiles : g.n_tiles;
-    const int hi = static_cast<int>(tile / fast), lo = static_cast<int>(tile - hi * fast);
+    const uint32_t whole = g.by_splits.quotient(tile);
+    split = static_cast<int>(tile - whole * g.by_splits.d);
+    tile = whole;
+    const int hi = static_cast<int>(g.fast.quotient(tile)), lo = static_cast<int>(tile - hi * g.fast.d);
     m_tile = P::M_FAST ? lo : hi;
     n_tile = P::M_FAST ? hi : lo;
   };
@@ -232,7 +232,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
         int split, m_tile, n_tile;
         locate(tile, split, m_tile, n_tile);
         for (int seg = 0; seg < P::NSEG && alive; ++seg) {
-          const int per = (g.kb[seg] + g.splits - 1) / g.splits;
+          const int per = g.per[seg];
           const int k1 = min(g.kb[seg], (split + 1) * per);
           for (int kb = split * per; kb < k1; ++kb) {
             if (!mbar_wait(&empty_bar[stage], phase ^ 1, g.status, ST_TIMEOUT_PRODUCER)) {
@@ -262,13 +262,13 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
       uint32_t phase = 0, it = 0;
       bool alive = true;
       for (uint32_t tile = blockIdx.x; tile < total && alive; tile += gridDim.x, ++it) {
-        const int split = g.splits > 1 ? static_cast<int>(tile % g.splits) : 0;
+        const int split = static_cast<int>(tile - g.by_splits.quotient(tile) * g.by_splits.d);
         const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
         if (!mbar_wait(&acc_empty[buf], buf_phase ^ 1, g.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
         for (int seg = 0; seg < P::NSEG && alive; ++seg) {
           const uint32_t d_seg = tmem_base + buf * ACC + seg * SEG;
-          const int per = (g.kb[seg] + g.splits - 1) / g.splits;
+          const int per = g.per[seg];
           const int k0 = split * per, k1 = min(g.kb[seg], (split + 1) * per);
           for (int kb = k0; kb < k1; ++kb) {
             if (!mbar_wait(&full_bar[stage], phase, g.status, ST_TIMEOUT_MMA)) {
@@ -321,7 +321,7 @@ piece_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, cons
       acc.base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * ACC;
 #pragma unroll
       for (int seg = 0; seg < P::NSEG; ++seg) {
-        const int per = (g.kb[seg] + g.splits - 1) / g.splits;
+        const int per = g.per[seg];
         acc.used[seg] = min(g.kb[seg], (split + 1) * per) - split * per;
       }
       if (tile + gridDim.x >= total) status = ask_status(g.status);  // (arrives during the last epilogue)
@@ -346,6 +346,9 @@ int launch_piece_gemm(const GemmMaps& maps, GemmShape g, const typename P::Param
   if (rc) return rc;
   const long long total = static_cast<long long>(g.m_tiles) * g.n_tiles * g.splits;
   B200_REQUIRE(total < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "gemm: too many tiles (%lld)", total);
+  for (int seg = 0; seg < 2; ++seg) g.per[seg] = (g.kb[seg] + g.splits - 1) / g.splits;
+  g.by_splits = Divisor(g.splits);
+  g.fast = Divisor(P::M_FAST ? g.m_tiles : g.n_tiles);
   const long long slots = static_cast<long long>(P::CTAS) * sm_count();
   const unsigned grid = static_cast<unsigned>(total < slots ? total : slots);
   return launch(piece_gemm_kernel<P>, dim3(grid), dim3(gemm_threads<P>()), gemm_smem_bytes<P>(), stream, pdl, maps, g, ep);
@@ -374,7 +377,7 @@ int gemm_res_stages(int kb) {  // 0: does not fit
   return stages < 3 ? 0 : stages > RES_STAGES ? RES_STAGES : stages;
 }
 struct GemmRuns {
-  int fast, parts, stages;  // fast-direction tiles, runs they are cut into, streamed stages
+  int fast, log_parts, stages;  // fast-direction tiles, runs they are cut into (log2), streamed stages
   uint32_t units;           // slow-direction tiles x parts
 };
 
@@ -424,10 +427,10 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
   int status = -1;
   const uint32_t tmem_base = tmem_base_s;
   auto locate = [&](uint32_t unit, int& slow, int& f0, int& f1) {
-    const uint32_t s = unit / static_cast<uint32_t>(runs.parts), part = unit - s * runs.parts;
+    const uint32_t s = unit >> runs.log_parts, part = unit - (s << runs.log_parts);
     slow = s;
-    f0 = part * runs.fast / runs.parts;
-    f1 = (part + 1) * runs.fast / runs.parts;
+    f0 = part * runs.fast >> runs.log_parts;
+    f1 = (part + 1) * runs.fast >> runs.log_parts;
   };
 
   if (warp == 0) {
@@ -572,10 +575,10 @@ int launch_piece_gemm_resident(const GemmMaps& maps, GemmShape g, const typename
   int rc = ensure_smem_limit(reinterpret_cast<const void*>(piece_gemm_resident_kernel<P>), 223 * 1024);
   if (rc) return rc;
   const int slow = P::M_FAST ? g.n_tiles : g.m_tiles;
-  GemmRuns r = {P::M_FAST ? g.m_tiles : g.n_tiles, 1, gemm_res_stages<P>(g.kb[0]), 0};
+  GemmRuns r = {P::M_FAST ? g.m_tiles : g.n_tiles, 0, gemm_res_stages<P>(g.kb[0]), 0};
   // enough runs that the last wave matters little, of at least two tiles
-  while (static_cast<long long>(slow) * r.parts < 6ll * sm_count() && r.fast / r.parts >= 4) r.parts *= 2;
-  const long long units = static_cast<long long>(slow) * r.parts;
+  while ((static_cast<long long>(slow) << r.log_parts) < 6ll * sm_count() && r.fast >> r.log_parts >= 4) ++r.log_parts;
+  const long long units = static_cast<long long>(slow) << r.log_parts;
   B200_REQUIRE(units < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "gemm: too many tiles (%lld)", units);
   r.units = static_cast<uint32_t>(units);
   const unsigned grid = static_cast<unsigned>(units < sm_count() ? units : sm_count());

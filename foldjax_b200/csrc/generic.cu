@@ -720,10 +720,10 @@ struct RowPrefetch {
 // Tile `tile` of rows walked `box` inner positions at a time.
 struct RowTile {
   int b, o, t0;
-  __device__ RowTile(uint32_t tile, uint32_t n, uint32_t tiles_t, int box) {
-    const uint32_t bo = tile / tiles_t, bb = bo / n;
-    t0 = static_cast<int>(tile - bo * tiles_t) * box;
-    o = static_cast<int>(bo - bb * n);
+  __device__ RowTile(uint32_t tile, const Divisor& n, const Divisor& tiles_t, int box) {
+    const uint32_t bo = tiles_t.quotient(tile), bb = n.quotient(bo);
+    t0 = static_cast<int>(tile - bo * tiles_t.d) * box;
+    o = static_cast<int>(bo - bb * n.d);
     b = static_cast<int>(bb);
   }
 };
@@ -737,7 +737,8 @@ struct GluPolicy {
   static constexpr bool A_MN = true, B_MN = false, M_FAST = true;
   static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   struct Params {
-    int n, tiles_t, c_h, ld;
+    int n, c_h, ld;
+    Divisor by_n, tiles_t;
     long long piece;  // elements between pieces of a plane set
     const float* mask;
     long long ms_b, ms_o, ms_i;
@@ -749,7 +750,7 @@ struct GluPolicy {
   }
   static __device__ void load_b(const GemmMaps& maps, const Params& p, int, int k, int n_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
-    const RowTile r(n_tile, p.n, p.tiles_t, BN);
+    const RowTile r(n_tile, p.by_n, p.tiles_t, BN);
     tma_load_5d(dst, &maps.b[0], bar, k, r.t0, r.o, r.b, piece);
   }
   static constexpr bool BF = PIECES == 1;
@@ -757,7 +758,7 @@ struct GluPolicy {
     float mask[BN / (EPI / 4) / 16];  // of pair lane & 15 of each run of 16
   };
   static __device__ void prefetch(const Params& p, int, int n_tile, int, int col0, int, int lane, Pre& pre) {
-    const RowTile rt(n_tile, p.n, p.tiles_t, BN);
+    const RowTile rt(n_tile, p.by_n, p.tiles_t, BN);
 #pragma unroll
     for (int i = 0; i < BN / (EPI / 4) / 16; ++i) {
       const int t = rt.t0 + col0 + 16 * i + (lane & 15);
@@ -766,7 +767,7 @@ struct GluPolicy {
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<GluPolicy>& acc, int quarter,
                                   int col0, int, int lane, const Pre& pre) {
-    const RowTile rt(n_tile, p.n, p.tiles_t, BN);
+    const RowTile rt(n_tile, p.by_n, p.tiles_t, BN);
     const int c = m_tile * GEMM_BM + quarter * 32 + lane;
     const int chan = c < p.c_h ? c : c - p.c_h;
     __nv_bfloat16* dst = (c < p.c_h ? p.a : p.b) +
@@ -781,20 +782,22 @@ struct GluPolicy {
       acc.load(1, col, g);
       // (the pitch is a multiple of 64: the padding takes what lies past n)
       if constexpr (BF) {
-        const uint32_t mk2 = pack_bf16x2(mk, __shfl_down_sync(0xffffffffu, mk, 1));  // of two pairs, in the lane of the first
         uint32_t u[8];
 #pragma unroll
-        for (int e = 0; e < 16; e += 2)
-          u[e / 2] = bf16x2_mul(bf16x2_mul(sigmoid_bf16x2(g[e], g[e + 1]), pack_bf16x2(v[e], v[e + 1])),
-                                __shfl_sync(0xffffffffu, mk2, e));
+        for (int e = 0; e < 16; e += 2) u[e / 2] = bf16x2_mul(sigmoid_bf16x2(g[e], g[e + 1]), pack_bf16x2(v[e], v[e + 1]));
+        if (!__all_sync(0xffffffffu, mk == 1.0f)) {  // (a factor of one changes nothing)
+          const uint32_t mk2 = pack_bf16x2(mk, __shfl_down_sync(0xffffffffu, mk, 1));  // of two pairs, in the lane of the first
+#pragma unroll
+          for (int e = 0; e < 16; e += 2) u[e / 2] = bf16x2_mul(u[e / 2], __shfl_sync(0xffffffffu, mk2, e));
+        }
         // a lane's 16 pairs are a whole sector of its channel
         if (c < 2 * p.c_h) store_sector(dst + col, make_uint4(u[0], u[1], u[2], u[3]), make_uint4(u[4], u[5], u[6], u[7]));
       } else {
 #pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-          const float m0 = __shfl_sync(0xffffffffu, mk, e), m1 = __shfl_sync(0xffffffffu, mk, e + 1);
-          v[e] = sigmoid_exact(g[e]) * v[e] * m0;
-          v[e + 1] = sigmoid_exact(g[e + 1]) * v[e + 1] * m1;
+        for (int e = 0; e < 16; ++e) v[e] = sigmoid_exact(g[e]) * v[e];
+        if (!__all_sync(0xffffffffu, mk == 1.0f)) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] *= __shfl_sync(0xffffffffu, mk, e);
         }
         if (c < 2 * p.c_h) store_sixteen<PIECES>(dst + col, p.piece, v);
       }
@@ -811,7 +814,8 @@ struct OutGatePolicy {
   static constexpr bool BF = PIECES == 1;
   using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
   struct Params {
-    int n, tiles_j, c_z;
+    int n, c_z;
+    Divisor by_n, tiles_j;
     const O* res;
     O* out;
     bool aligned, sectors;  // 16-byte and 32-byte accesses
@@ -820,14 +824,14 @@ struct OutGatePolicy {
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
     if constexpr (BF) {
       if (!p.res || !p.aligned) return;
-      const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
+      const RowTile rt(m_tile, p.by_n, p.tiles_j, GEMM_BM);
       const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
       pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0, p.sectors);
     }
   }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int seg, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
-    const RowTile r(m_tile, p.n, p.tiles_j, GEMM_BM);
+    const RowTile r(m_tile, p.by_n, p.tiles_j, GEMM_BM);
     tma_load_5d(dst, &maps.a[seg], bar, k, r.t0, r.o, r.b, piece);
   }
   static __device__ void load_b(const GemmMaps& maps, const Params&, int seg, int k, int n_tile, int piece, uint8_t* dst,
@@ -836,7 +840,7 @@ struct OutGatePolicy {
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<OutGatePolicy>& acc, int quarter,
                                   int col0, int, int lane, const Pre& pre) {
-    const RowTile rt(m_tile, p.n, p.tiles_j, GEMM_BM);
+    const RowTile rt(m_tile, p.by_n, p.tiles_j, GEMM_BM);
     const int j = rt.t0 + quarter * 32 + lane;
     const long long off = ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z;
 #pragma unroll(BF ? 4 : 1)
@@ -883,13 +887,16 @@ struct QkvbPolicy : NoPrefetch {
   static constexpr bool BF = PIECES == 1;
   struct Params {
     int n, hd, heads, tiles_w, ld;
+    Divisor by_n;
     uint32_t pairs;
     float q_scale, q_scale_inv;
     long long row_piece, v_piece;  // elements between pieces of q / k and of v
     __nv_bfloat16 *q, *k, *vt;
     void* bias;
   };
-  static __device__ int which(const Params& p, int n_tile) { return n_tile / p.tiles_w < 3 ? n_tile / p.tiles_w : 3; }
+  static __device__ int which(const Params& p, int n_tile) {
+    return (n_tile >= p.tiles_w) + (n_tile >= 2 * p.tiles_w) + (n_tile >= 3 * p.tiles_w);
+  }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
     tma_load_3d(dst, &maps.a[0], bar, k, m_tile * GEMM_BM, piece);
@@ -902,7 +909,7 @@ struct QkvbPolicy : NoPrefetch {
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvbPolicy>& acc, int quarter,
                                   int col0, int col1, int lane, const Pre&) {
     const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
-    const uint32_t bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
+    const uint32_t bo = p.by_n.quotient(pair), t = pair - bo * n, b = p.by_n.quotient(bo), o = bo - b * n;
     const int w = which(p, n_tile);
 #pragma unroll 1
     for (int col = col0; col < col1; col += 16) {
@@ -1053,7 +1060,8 @@ struct ProjOutPolicy {
   using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
   struct Params {
     long long pairs;
-    int n, c_z;
+    int c_z;
+    Divisor by_n;
     long long s_b, s_o, s_i;
     const O* res;
     O* out;
@@ -1061,7 +1069,7 @@ struct ProjOutPolicy {
   };
   using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
   static __device__ long long offset(const Params& p, uint32_t pair) {
-    const uint32_t n = p.n, bo = pair / n, t = pair - bo * n, b = bo / n, o = bo - b * n;
+    const uint32_t n = p.by_n.d, bo = p.by_n.quotient(pair), t = pair - bo * n, b = p.by_n.quotient(bo), o = bo - b * n;
     return b * p.s_b + o * p.s_o + t * p.s_i;
   }
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
@@ -1269,7 +1277,7 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       const GemmShape g = {(2 * c_h + GEMM_BM - 1) / GEMM_BM, nb * n * tiles_t, 1, {ksteps(c_z), ksteps(c_z)}, nullptr};
       auto go = [&](auto policy, auto kept) {
         using Pol = decltype(policy);
-        return launch_either<Pol, decltype(kept)>(glu, g, {n, tiles_t, c_h, ld, piece, mask, nn, a->incoming ? 1ll : n,
+        return launch_either<Pol, decltype(kept)>(glu, g, {n, c_h, ld, Divisor(n), Divisor(tiles_t), piece, mask, nn, a->incoming ? 1ll : n,
                                                a->incoming ? n : 1ll, at(pl.ap), at(pl.bp)}, true, stream);
       };
       if constexpr (BF)
@@ -1306,7 +1314,7 @@ int trimul_generic(const b200tri_trimul_args* a, int c_z, int c_h, cudaStream_t 
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {nb * n * tiles_j, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_h), ksteps(c_z)}, nullptr};
-        return launch_piece_gemm<Pol>(fin, g, {n, tiles_j, c_z, res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(fin, g, {n, c_z, Divisor(n), Divisor(tiles_j), res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(OutGatePolicy<1, 1, 64>{}) : go(OutGatePolicy<1, 1, 128>{});
@@ -1384,7 +1392,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         // 314 / 311; 384 of 12 x 32 367 / 363. Keeping pays where a weight is few column tiles wide, in
         // float32 up to 128 channels: 455 / 491 for four 200-token templates, 333 / 313 at 192. The rule
         // goes by k steps, which is within 4 % of the better side.)
-        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, tiles_w, ld, static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
+        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, tiles_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
                                                 ws + pl.bias}, ksteps(c_z) <= 2, stream);
       };
@@ -1432,7 +1440,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       auto go = [&](auto policy) {
         using Pol = decltype(policy);
         const GemmShape g = {m_tiles, (c_z + Pol::BN - 1) / Pol::BN, 1, {ksteps(hd), 0}, nullptr};
-        return launch_piece_gemm<Pol>(outp, g, {pairs, n, c_z, nn * c_z, s_o, s_i, res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
+        return launch_piece_gemm<Pol>(outp, g, {pairs, c_z, Divisor(n), nn * c_z, s_o, s_i, res, out, aligned16(out, res), (!BF || c_z % 16 == 0) && aligned32(out, res)}, stream, true);
       };
       if constexpr (BF)
         rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{})
