@@ -361,7 +361,7 @@ int launch_piece_gemm(const GemmMaps& maps, GemmShape g, const typename P::Param
 // of their own and are refilled one by one behind the last tile's products.
 // Gated projection, 65 536 pairs x 384 -> 768 channels: 104 -> 94 us; 160 000 x 64 -> 256: 72 -> 67;
 // q, k, v and bias, 160 000 x 64: 56 -> 45 (384 channels: 96 -> 107, left streaming).
-constexpr int RES_KB = 8, RES_STAGES = 8;  // most k steps kept, most streamed stages
+constexpr int RES_KB = 8, RES_STAGES = 8, RES_SLOTS = 16;  // most k steps kept, streamed stages, places of either
 template <class P>
 constexpr int gemm_res_bytes() {
   return P::M_FAST ? P::PB * P::BN * 128 : P::PA * GEMM_A_BYTES;
@@ -377,11 +377,13 @@ int gemm_res_stages(int kb) {  // 0: does not fit
   return stages < 3 ? 0 : stages > RES_STAGES ? RES_STAGES : stages;
 }
 struct GemmRuns {
-  int fast, log_parts, stages;  // fast-direction tiles, runs they are cut into (log2), streamed stages
+  int fast, log_parts, slots, stages;  // fast-direction tiles, runs they are cut into (log2), kept places, streamed stages
   uint32_t units;           // slow-direction tiles x parts
 };
 
-template <class P>
+// ONCE: the stages hold the whole streamed operand (the weights), which is loaded for a CTA's first unit and stays, and
+// there are places for several units' k steps.
+template <class P, bool ONCE>
 __global__ void __launch_bounds__(gemm_threads<P>(), 1)
 piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, const GemmRuns runs,
                            const typename P::Params ep) {
@@ -393,19 +395,17 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
   static_assert(NBUF * ACC <= 512, "tile does not fit");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int kbs = g.kb[0], stages = runs.stages;
-  uint8_t* ring = smem + kbs * RES;
-  __shared__ uint64_t res_full[RES_KB], res_empty[RES_KB], full_bar[RES_STAGES], empty_bar[RES_STAGES], acc_full[2], acc_empty[2];
+  const int kbs = g.kb[0], slots = ONCE ? runs.slots : kbs, stages = runs.stages;
+  uint8_t* ring = smem + slots * RES;
+  __shared__ uint64_t res_full[RES_SLOTS], res_empty[RES_SLOTS], full_bar[RES_SLOTS], empty_bar[RES_SLOTS], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && lane == 0) {
     for (int s = 0; s < P::NSEG; ++s) tma_prefetch_desc(&maps.a[s]);
     tma_prefetch_desc(&maps.b[0]);
-    for (int s = 0; s < RES_KB; ++s) {
+    for (int s = 0; s < RES_SLOTS; ++s) {
       mbar_init(&res_full[s], 1);
       mbar_init(&res_empty[s], 1);
-    }
-    for (int s = 0; s < RES_STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -426,6 +426,19 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
   pdl_trigger();
   int status = -1;
   const uint32_t tmem_base = tmem_base_s;
+  // the place of a unit's k step, counted from that of its first one, and the first place of the next unit
+  auto place = [&](int kept, int kb) { return !ONCE ? kb : kept + kb < slots ? kept + kb : kept + kb - slots; };
+  auto next_kept = [&](int& kept, uint32_t& round) {
+    if (!ONCE) {
+      round ^= 1;
+      return;
+    }
+    kept += kbs;
+    if (kept >= slots) {
+      kept -= slots;
+      round ^= 1;
+    }
+  };
   auto locate = [&](uint32_t unit, int& slow, int& f0, int& f1) {
     const uint32_t s = unit >> runs.log_parts, part = unit - (s << runs.log_parts);
     slow = s;
@@ -435,10 +448,10 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
 
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0, u = 0;
+      int stage = 0, kept = 0;  // kept: slot of the unit's first k step
+      uint32_t phase = 0, round = 0;
       bool alive = true;
-      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, ++u) {
+      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, next_kept(kept, round)) {
         int slow, f0, f1;
         locate(unit, slow, f0, f1);
         for (int f = f0; f < f1 && alive; ++f) {
@@ -446,18 +459,20 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
           for (int seg = 0; seg < P::NSEG && alive; ++seg)
             for (int kb = 0; kb < kbs; ++kb) {
               if (f == f0 && seg == 0) {
-                if (!mbar_wait(&res_empty[kb], (u & 1) ^ 1, g.status, ST_TIMEOUT_PRODUCER)) {
+                const int slot = place(kept, kb);
+                if (!mbar_wait(&res_empty[slot], round ^ (slot >= kept), g.status, ST_TIMEOUT_PRODUCER)) {
                   alive = false;
                   break;
                 }
-                mbar_expect_tx(&res_full[kb], RES);
+                mbar_expect_tx(&res_full[slot], RES);
                 for (int pc = 0; pc < (P::M_FAST ? P::PB : P::PA); ++pc) {
                   if (P::M_FAST)
-                    P::load_b(maps, ep, 0, kb * GEMM_BK, n_tile, pc, smem + kb * RES + pc * P::BN * 128, &res_full[kb]);
+                    P::load_b(maps, ep, 0, kb * GEMM_BK, n_tile, pc, smem + slot * RES + pc * P::BN * 128, &res_full[slot]);
                   else
-                    P::load_a(maps, ep, 0, kb * GEMM_BK, m_tile, pc, smem + kb * RES + pc * GEMM_A_BYTES, &res_full[kb]);
+                    P::load_a(maps, ep, 0, kb * GEMM_BK, m_tile, pc, smem + slot * RES + pc * GEMM_A_BYTES, &res_full[slot]);
                 }
               }
+              if (ONCE && unit != blockIdx.x) continue;
               if (!mbar_wait(&empty_bar[stage], phase ^ 1, g.status, ST_TIMEOUT_PRODUCER)) {
                 alive = false;
                 break;
@@ -481,10 +496,10 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, P::BN) | (P::A_MN ? UMMA_A_MN : 0u) | (P::B_MN ? UMMA_B_MN : 0u);
       using T = Terms<P::PA, P::PB>;
-      int stage = 0;
-      uint32_t phase = 0, it = 0, u = 0;
+      int stage = 0, kept = 0;
+      uint32_t phase = 0, it = 0, round = 0;
       bool alive = true;
-      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, ++u) {
+      for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x, next_kept(kept, round)) {
         int slow, f0, f1;
         locate(unit, slow, f0, f1);
         for (int f = f0; f < f1 && alive; ++f, ++it) {
@@ -496,14 +511,15 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
           tc_fence_after();
           for (int seg = 0; seg < P::NSEG && alive; ++seg)
             for (int kb = 0; kb < kbs; ++kb) {
-              if ((f == f0 && seg == 0 && !mbar_wait(&res_full[kb], u & 1, g.status, ST_TIMEOUT_MMA)) ||
-                  !mbar_wait(&full_bar[stage], phase, g.status, ST_TIMEOUT_MMA)) {
+              const int slot = place(kept, kb);
+              if ((f == f0 && seg == 0 && !mbar_wait(&res_full[slot], round ^ (slot < kept), g.status, ST_TIMEOUT_MMA)) ||
+                  ((!ONCE || unit == blockIdx.x) && !mbar_wait(&full_bar[stage], phase, g.status, ST_TIMEOUT_MMA))) {
                 alive = false;
                 break;
               }
               tc_fence_after();
-              const uint32_t kept = smem_u32(smem + kb * RES), streamed = smem_u32(ring + stage * STREAM);
-              const uint32_t sa = P::M_FAST ? streamed : kept, sb = P::M_FAST ? kept : streamed;
+              const uint32_t resident = smem_u32(smem + slot * RES), streamed = smem_u32(ring + stage * STREAM);
+              const uint32_t sa = P::M_FAST ? streamed : resident, sb = P::M_FAST ? resident : streamed;
 #pragma unroll
               for (int t = 0; t < T::N; ++t) {
                 const uint64_t adesc = P::A_MN ? umma_desc_mnmajor(sa + T::a(t) * GEMM_A_BYTES, 8192)
@@ -518,8 +534,8 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
                   umma_bf16_ss(d_tmem, umma_desc_advance(adesc, P::A_MN ? k * 2048 : k * 32),
                                umma_desc_advance(bdesc, P::B_MN ? k * 2048 : k * 32), idesc, !(fresh && k == 0));
               }
-              umma_commit(&empty_bar[stage]);
-              if (f == f1 - 1 && seg == P::NSEG - 1) umma_commit(&res_empty[kb]);
+              if (!ONCE) umma_commit(&empty_bar[stage]);
+              if (f == f1 - 1 && seg == P::NSEG - 1) umma_commit(&res_empty[slot]);
               if (++stage == stages) {
                 stage = 0;
                 phase ^= 1;
@@ -572,18 +588,38 @@ template <class P>
 int launch_piece_gemm_resident(const GemmMaps& maps, GemmShape g, const typename P::Params& ep, cudaStream_t stream, bool pdl) {
   g.status = device_status_word();
   B200_REQUIRE(g.status != nullptr, B200TRI_ERR_CUDA, "gemm: no current CUDA device");
-  int rc = ensure_smem_limit(reinterpret_cast<const void*>(piece_gemm_resident_kernel<P>), 223 * 1024);
-  if (rc) return rc;
   const int slow = P::M_FAST ? g.n_tiles : g.m_tiles;
-  GemmRuns r = {P::M_FAST ? g.m_tiles : g.n_tiles, 0, gemm_res_stages<P>(g.kb[0]), 0};
-  // enough runs that the last wave matters little, of at least two tiles
-  while ((static_cast<long long>(slow) << r.log_parts) < 6ll * sm_count() && r.fast >> r.log_parts >= 4) ++r.log_parts;
-  const long long units = static_cast<long long>(slow) << r.log_parts;
+  GemmRuns r = {P::M_FAST ? g.m_tiles : g.n_tiles, 0, g.kb[0], gemm_res_stages<P>(g.kb[0]), 0};
+  // enough runs that the last wave matters little, of at least two tiles, or of one where they all run at once
+  // (64 tokens: template 81.0 -> 77.3 us, float32 stack 153.5 -> 142.1)
+  auto runs_of = [&](int log) { return static_cast<long long>(slow) << log; };
+  while ((runs_of(r.log_parts) < 6ll * sm_count() && r.fast >> r.log_parts >= 4) ||
+         (runs_of(r.log_parts + 1) <= sm_count() && r.fast >> r.log_parts >= 2))
+    ++r.log_parts;
+  const long long units = runs_of(r.log_parts);
   B200_REQUIRE(units < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "gemm: too many tiles (%lld)", units);
   r.units = static_cast<uint32_t>(units);
   const unsigned grid = static_cast<unsigned>(units < sm_count() ? units : sm_count());
-  const size_t smem = static_cast<size_t>(g.kb[0]) * gemm_res_bytes<P>() + r.stages * gemm_stream_bytes<P>() + 1024;
-  return launch(piece_gemm_resident_kernel<P>, dim3(grid), dim3(gemm_threads<P>()), smem, stream, pdl, maps, g, r, ep);
+  auto go = [&](auto kernel) {
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), 223 * 1024);
+    if (rc) return rc;
+    const size_t smem = static_cast<size_t>(r.slots) * gemm_res_bytes<P>() + r.stages * gemm_stream_bytes<P>() + 1024;
+    return launch(kernel, dim3(grid), dim3(gemm_threads<P>()), smem, stream, pdl, maps, g, r, ep);
+  };
+  // Weights of up to 16 k steps stay where two units' rows fit beside them. Streamed, all SMs fetched the same few lines
+  // from L2 at a time (64 rows of 16 bytes for a bias of 4 heads), and loads and products alone took 28 of the 41 us of the
+  // projection of four 200-token templates; now it takes 29 (four updates 568 -> 551 us, 320 tokens 407 -> 392).
+  if constexpr (P::PA * P::PB == 1) {
+    const int all = r.fast * P::NSEG * g.kb[0];
+    const int left = (222 * 1024 - all * gemm_stream_bytes<P>()) / gemm_res_bytes<P>();
+    if (r.log_parts == 0 && all <= RES_SLOTS && left >= 2 * g.kb[0]) {
+      const int most = 4 * g.kb[0] < RES_SLOTS ? 4 * g.kb[0] : RES_SLOTS;
+      r.slots = left < most ? left : most;
+      r.stages = all;
+      return go(piece_gemm_resident_kernel<P, true>);
+    }
+  }
+  return go(piece_gemm_resident_kernel<P, false>);
 }
 
 // Activations: bf16 pieces [pieces][rows][k], row pitch `pitch` elements (a multiple of 8);

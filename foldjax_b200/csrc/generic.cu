@@ -878,7 +878,7 @@ struct OutGatePolicy {
 };
 
 // q / sqrt(d), k: rows [piece][pair][hd]. v: transposed, [piece][(b, o)][hd][ld]. bias: [b][head][o][ld] in the trunk dtype. Column tiles walk
-// the four weights in turn.
+// the four weights in turn, in groups of 64 (so that narrow heads have tiles of 128 columns too).
 template <int PIECES, int NM, int BN_, bool RES = false>
 struct QkvbPolicy : NoPrefetch {
   static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
@@ -886,7 +886,7 @@ struct QkvbPolicy : NoPrefetch {
   static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   static constexpr bool BF = PIECES == 1;
   struct Params {
-    int n, hd, heads, tiles_w, ld;
+    int n, hd, heads, groups_w, ld;  // groups_w: groups of 64 columns of a weight
     Divisor by_n;
     uint32_t pairs;
     float q_scale, q_scale_inv;
@@ -894,8 +894,8 @@ struct QkvbPolicy : NoPrefetch {
     __nv_bfloat16 *q, *k, *vt;
     void* bias;
   };
-  static __device__ int which(const Params& p, int n_tile) {
-    return (n_tile >= p.tiles_w) + (n_tile >= 2 * p.tiles_w) + (n_tile >= 3 * p.tiles_w);
+  static __device__ int which(const Params& p, int group) {
+    return (group >= p.groups_w) + (group >= 2 * p.groups_w) + (group >= 3 * p.groups_w);
   }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
@@ -903,17 +903,22 @@ struct QkvbPolicy : NoPrefetch {
   }
   static __device__ void load_b(const GemmMaps& maps, const Params& p, int, int k, int n_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
-    const int w = which(p, n_tile);
-    gemm_load_mn(&maps.b[w], dst, bar, BN / 64, (n_tile - w * p.tiles_w) * BN, k, piece);
+#pragma unroll
+    for (int g = 0; g < BN / 64; ++g) {  // (a group behind the last one is columns that its map does not have: zeros)
+      const int group = n_tile * (BN / 64) + g, w = which(p, group);
+      gemm_load_mn(&maps.b[w], dst + g * 8192, bar, 1, (group - w * p.groups_w) * 64, k, piece);
+    }
   }
   static __device__ void epilogue(const Params& p, int m_tile, int n_tile, int, const Accum<QkvbPolicy>& acc, int quarter,
                                   int col0, int col1, int lane, const Pre&) {
     const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane, n = p.n;
     const uint32_t bo = p.by_n.quotient(pair), t = pair - bo * n, b = p.by_n.quotient(bo), o = bo - b * n;
-    const int w = which(p, n_tile);
+    // a warp's columns are those of one weight
+    static_assert(64 % (BN / (EPI / 4)) == 0, "");
+    const int group = n_tile * (BN / 64) + col0 / 64, w = which(p, group);
 #pragma unroll 1
     for (int col = col0; col < col1; col += 16) {
-      const int c0 = (n_tile - w * p.tiles_w) * BN + col;
+      const int c0 = (group - w * p.groups_w) * 64 + col % 64;
       if (c0 >= (w == 3 ? p.heads : p.hd)) break;
       float v[16];
       acc.load(0, col, v);
@@ -1384,21 +1389,20 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       if ((rc = gemm_map_kmajor(&proj.a[0], at(pl.xn), P, pairs, c_z, c_z, GEMM_BM))) return rc;
       auto go = [&](auto policy, auto kept) {
         using Pol = decltype(policy);
-        const int tiles_w = (hd + Pol::BN - 1) / Pol::BN;
-        const GemmShape g = {m_tiles, 3 * tiles_w + (heads + Pol::BN - 1) / Pol::BN, 1, {ksteps(c_z), 0}, nullptr};
+        const int groups_w = (hd + 63) / 64, groups = 3 * groups_w + (heads + 63) / 64;
+        const GemmShape g = {m_tiles, (groups + Pol::BN / 64 - 1) / (Pol::BN / 64), 1, {ksteps(c_z), 0}, nullptr};
         const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
         // (Kept / streamed, us of the whole bf16 attention of 256 tokens: 128 channels of 8 x 16 heads
         // 172 / 184, of 12 x 32 304 / 294; 192 of 6 x 32 213 / 220; 256 of 8 x 32 246 / 252; 320 of 10 x 32
         // 314 / 311; 384 of 12 x 32 367 / 363. Keeping pays where a weight is few column tiles wide, in
         // float32 up to 128 channels: 455 / 491 for four 200-token templates, 333 / 313 at 192. The rule
         // goes by k steps, which is within 4 % of the better side.)
-        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, tiles_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
+        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, groups_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
                                                 ws + pl.bias}, ksteps(c_z) <= 2, stream);
       };
       if constexpr (BF)
-        rc = hd <= 64 ? go(QkvbPolicy<1, 1, 64>{}, QkvbPolicy<1, 1, 64, true>{})
-                     : go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
+        rc = go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
       else
         rc = go(QkvbPolicy<3, 3, 64>{}, QkvbPolicy<3, 3, 64, true>{});
       if (rc) return rc;
