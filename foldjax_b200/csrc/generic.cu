@@ -717,6 +717,30 @@ struct RowPrefetch {
   }
 };
 
+// The same of a float32 row (256- and 150-token float32 stacks 860 -> 855 and 432 -> 426 us against loads behind the accumulators;
+// 849 and 424 with no accumulator that K of 128 leaves unused).
+template <int COLS>
+struct RowPrefetchF {
+  uint4 row[COLS / 4];
+  __device__ __forceinline__ void load(const float* src, int left, bool sectors) {
+#pragma unroll
+    for (int q = 0; q < COLS / 4; q += 2) {
+      row[q] = row[q + 1] = make_uint4(0u, 0u, 0u, 0u);
+      if (4 * q >= left) continue;  // (a multiple of eight)
+      if (sectors) {
+        load_sector(src + 4 * q, row[q], row[q + 1]);
+      } else {
+        row[q] = reinterpret_cast<const uint4*>(src)[q];
+        row[q + 1] = reinterpret_cast<const uint4*>(src)[q + 1];
+      }
+    }
+  }
+  __device__ __forceinline__ float at(int e) const {
+    const uint4& w = row[e / 4];
+    return __uint_as_float(e % 4 == 0 ? w.x : e % 4 == 1 ? w.y : e % 4 == 2 ? w.z : w.w);
+  }
+};
+
 // Tile `tile` of rows walked `box` inner positions at a time.
 struct RowTile {
   int b, o, t0;
@@ -820,14 +844,12 @@ struct OutGatePolicy {
     O* out;
     bool aligned, sectors;  // 16-byte and 32-byte accesses
   };
-  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  using Pre = typename std::conditional<BF, RowPrefetch<BN / (EPI / 4)>, RowPrefetchF<BN / (EPI / 4)>>::type;
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
-    if constexpr (BF) {
-      if (!p.res || !p.aligned) return;
-      const RowTile rt(m_tile, p.by_n, p.tiles_j, GEMM_BM);
-      const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
-      pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0, p.sectors);
-    }
+    if (!p.res || !p.aligned) return;
+    const RowTile rt(m_tile, p.by_n, p.tiles_j, GEMM_BM);
+    const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
+    pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0, p.sectors);
   }
   static __device__ void load_a(const GemmMaps& maps, const Params& p, int seg, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
@@ -868,11 +890,16 @@ struct OutGatePolicy {
           continue;
         }
       }
+      const bool there = !BF && p.res && p.aligned;  // the residual has been asked for
+      if constexpr (!BF) {
+        if (there)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] = pre.at(16 * i + e) + v[e];
+      }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        if (c0 + 8 * q < p.c_z) {
-          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
-        }
+        if (c0 + 8 * q < p.c_z)
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res && !there ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
     }
   }
 };
@@ -979,13 +1006,14 @@ struct GatePolicy {
     const float* o;
     __nv_bfloat16* y;
   };
-  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  using Pre = typename std::conditional<BF, RowPrefetch<BN / (EPI / 4)>, RowPrefetchF<BN / (EPI / 4)>>::type;
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
-    if constexpr (BF) {
-      const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
-      const int c0 = n_tile * BN + col0;
+    const long long pair = static_cast<long long>(m_tile) * GEMM_BM + quarter * 32 + lane;
+    const int c0 = n_tile * BN + col0;
+    if constexpr (BF)
       pre.load(p.y + pair * p.hd + c0, pair < p.pairs ? p.hd - c0 : 0, p.hd % 16 == 0);
-    }
+    else
+      pre.load(p.o + pair * p.hd + c0, pair < p.pairs ? p.hd - c0 : 0, true);
   }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
@@ -1022,33 +1050,16 @@ struct GatePolicy {
           *reinterpret_cast<uint4*>(p.y + off) = w[0];
           if (c0 + 8 < p.hd) reinterpret_cast<uint4*>(p.y + off)[1] = w[1];
         }
-      } else if (p.hd % 16 == 0) {
+      } else {
         float v[16];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint4 a, b;
-          load_sector(p.o + off + 8 * q, a, b);
-          const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        for (int e = 0; e < 16; ++e) v[e] = pre.at(16 * i + e) * sigmoid_exact(g[e]);
+        if (p.hd % 16 == 0) {
+          store_sixteen<PIECES>(p.y + off, p.pairs * p.hd, v);
+        } else {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[8 * q + e] = __uint_as_float(w[e]) * sigmoid_exact(g[8 * q + e]);
-        }
-        store_sixteen<PIECES>(p.y + off, p.pairs * p.hd, v);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (c0 + 8 * q >= p.hd) break;
-          float v[8];
-#pragma unroll
-          for (int h4 = 0; h4 < 2; ++h4) {
-            const float4 f = *reinterpret_cast<const float4*>(p.o + off + 8 * q + 4 * h4);
-            v[4 * h4 + 0] = f.x;
-            v[4 * h4 + 1] = f.y;
-            v[4 * h4 + 2] = f.z;
-            v[4 * h4 + 3] = f.w;
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] *= sigmoid_exact(g[8 * q + e]);
-          store_eight<PIECES>(p.y + off + 8 * q, p.pairs * p.hd, v);
+          for (int q = 0; q < 2; ++q)
+            if (c0 + 8 * q < p.hd) store_eight<PIECES>(p.y + off + 8 * q, p.pairs * p.hd, v + 8 * q);
         }
       }
     }
@@ -1072,18 +1083,16 @@ struct ProjOutPolicy {
     O* out;
     bool aligned, sectors;  // 16-byte and 32-byte accesses
   };
-  using Pre = RowPrefetch<BF ? BN / (EPI / 4) : 0>;
+  using Pre = typename std::conditional<BF, RowPrefetch<BN / (EPI / 4)>, RowPrefetchF<BN / (EPI / 4)>>::type;
   static __device__ long long offset(const Params& p, uint32_t pair) {
     const uint32_t n = p.by_n.d, bo = p.by_n.quotient(pair), t = pair - bo * n, b = p.by_n.quotient(bo), o = bo - b * n;
     return b * p.s_b + o * p.s_o + t * p.s_i;
   }
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
-    if constexpr (BF) {
-      if (!p.res || !p.aligned) return;
-      const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane;
-      const int c0 = n_tile * BN + col0;
-      pre.load(p.res + offset(p, pair) + c0, pair < p.pairs ? p.c_z - c0 : 0, p.sectors);
-    }
+    if (!p.res || !p.aligned) return;
+    const uint32_t pair = static_cast<uint32_t>(m_tile) * GEMM_BM + quarter * 32 + lane;
+    const int c0 = n_tile * BN + col0;
+    pre.load(p.res + offset(p, pair) + c0, pair < p.pairs ? p.c_z - c0 : 0, p.sectors);
   }
   static __device__ void load_a(const GemmMaps& maps, const Params&, int, int k, int m_tile, int piece, uint8_t* dst,
                                 uint64_t* bar) {
@@ -1110,11 +1119,16 @@ struct ProjOutPolicy {
           continue;
         }
       }
+      const bool there = !BF && p.res && p.aligned;  // the residual has been asked for
+      if constexpr (!BF) {
+        if (there)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] = pre.at(16 * i + e) + v[e];
+      }
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        if (c0 + 8 * q < p.c_z) {
-          store_out<BF>(p.out + off + c0 + 8 * q, p.res ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
-        }
+        if (c0 + 8 * q < p.c_z)
+          store_out<BF>(p.out + off + c0 + 8 * q, p.res && !there ? p.res + off + c0 + 8 * q : nullptr, v + 8 * q, p.aligned, p.sectors);
     }
   }
 };
@@ -1404,7 +1418,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
       if constexpr (BF)
         rc = go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
       else
-        rc = go(QkvbPolicy<3, 3, 64>{}, QkvbPolicy<3, 3, 64, true>{});
+        rc = ksteps(c_z) <= 2 ? go(QkvbPolicy<3, 2, 64>{}, QkvbPolicy<3, 2, 64, true>{}) : go(QkvbPolicy<3, 3, 64>{}, QkvbPolicy<3, 3, 64, true>{});
       if (rc) return rc;
     }
     {
@@ -1436,7 +1450,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         rc = hd <= 64 ? go(GatePolicy<1, 1, 64>{})
                      : go(GatePolicy<1, 1, 128>{});
       else
-        rc = go(GatePolicy<3, 3, 64>{});
+        rc = ksteps(c_z) <= 2 ? go(GatePolicy<3, 2, 64>{}) : go(GatePolicy<3, 3, 64>{});
       if (rc) return rc;
     }
     {
@@ -1450,7 +1464,7 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         rc = c_z <= 64 ? go(ProjOutPolicy<1, 1, 64>{})
                       : go(ProjOutPolicy<1, 1, 128>{});
       else
-        rc = go(ProjOutPolicy<3, 3, 64>{});
+        rc = ksteps(hd) <= 2 ? go(ProjOutPolicy<3, 2, 64>{}) : go(ProjOutPolicy<3, 3, 64>{});
       if (rc) return rc;
     }
   }
