@@ -8,8 +8,9 @@
 // to fp16 [row][head * 32 + d][key], and the mask-bias rows. The pair bias is read where it is
 // unless its rows are off the 16-byte grid TMA needs, or float32.
 //
-// Bound of the preparation: memory, 2 + 2 bytes per element of V. 4 heads x 384 x 384 x 32: 115 us
-// with the core; relayout copies of all five operands alone are 250.
+// Bound of the preparation: memory, 2 + 2 bytes per element of V. 4 heads x 384 x 384 x 32: 99 us
+// with the core; relayout copies of all five operands alone are 250. Small operators are launches: with the bias
+// rows in one of their own 60 / 100 / 203 tokens took 10.1 / 12.2 / 30.6 us, 7.8 / 10.7 / 29.0 so.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -34,12 +35,32 @@ __device__ __forceinline__ Chunk load_chunk(const float* p) {
   return {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 
-// One block per (row, 64 keys): all four heads, so that every thread has four loads in flight.
-template <typename T>
+// One block per (row, 64 keys): all four heads, so that every thread has four loads in flight. Behind those blocks, where the pair
+// bias [4 * n_j][n_k] is to be copied to bf16 rows of pitch ld, one per eight of its rows.
+struct BiasCopy {
+  const void* src;  // or null
+  __nv_bfloat16* dst;
+  long long rows;
+};
+template <typename T, typename B>
 __global__ void __launch_bounds__(256)
 prepare_kernel(const T* __restrict__ v, const float* __restrict__ mask, __half* __restrict__ vt, float* __restrict__ mb,
-               int n_k, int ld) {
+               int n_k, int ld, unsigned blocks, const BiasCopy bias, bool chained) {
   __shared__ __half tile[HEADS][D][PITCH];
+  if (chained) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.x >= blocks) {
+    const long long r = static_cast<long long>(blockIdx.x - blocks) * 8 + warp;
+    if (r >= bias.rows) return;
+    const B* src = static_cast<const B*>(bias.src) + r * n_k;
+    __nv_bfloat16* dst = bias.dst + r * ld;
+#pragma unroll 4
+    for (int k = lane; k < ld; k += 32) dst[k] = __float2bfloat16_rn(k < n_k ? static_cast<float>(src[k]) : 0.f);
+    return;
+  }
   const int tiles = ld / KT;
   const int i = blockIdx.x / tiles, k0 = (blockIdx.x - i * tiles) * KT;
   const int key = threadIdx.x >> 2, c = (threadIdx.x & 3) * 8;
@@ -58,22 +79,10 @@ prepare_kernel(const T* __restrict__ v, const float* __restrict__ mask, __half* 
         k < n_k ? mask_bias(mask[static_cast<long long>(i) * n_k + k], 0.f, true) : -INFINITY;
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __half* dst = vt + static_cast<long long>(i) * HEADS * D * ld + k0;
   for (int r = warp; r < HEADS * D; r += 8)
     reinterpret_cast<uint32_t*>(dst + static_cast<long long>(r) * ld)[lane] =
         reinterpret_cast<const uint32_t*>(&tile[r / D][r % D][0])[lane];
-}
-
-// Pair bias [4 * n_j][n_k] -> bf16 rows of pitch ld.
-template <typename T>
-__global__ void bias_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int n_k, int ld) {
-  const long long total = rows * ld, step = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += step) {
-    const long long r = idx / ld;
-    const int k = static_cast<int>(idx - r * ld);
-    dst[idx] = k < n_k ? __float2bfloat16_rn(static_cast<float>(src[r * n_k + k])) : __float2bfloat16_rn(0.f);
-  }
 }
 
 struct Plan {
@@ -127,37 +136,33 @@ extern "C" int b200tri_attention_core(const b200tri_attention_core_args* a, b200
   const size_t bias_elems = static_cast<size_t>(HEADS) * a->n_j * a->n_k;
   const CoreStrides strides = {D, static_cast<long long>(a->n_j) * D, static_cast<long long>(a->n_k) * D,
                                static_cast<long long>(a->n_j) * D * HEADS, static_cast<long long>(a->n_k) * D * HEADS};
+  const long long bias_rows = bias_in_place ? 0 : static_cast<long long>(HEADS) * a->n_j;
+  const long long grid_blocks = blocks + (bias_rows + 7) / 8;
+  B200_REQUIRE(grid_blocks < (1ll << 31), B200TRI_ERR_UNSUPPORTED, "attention core: too many rows times keys for one launch");
+  // Programmatic launches from the kernel before to the core, where no SM has two blocks of the preparation: the core's
+  // CTA has room beside one (48 / 60 / 64 tokens 8.3 / 8.8 / 8.4 us without, 6.8 / 7.8 / 7.5 with; beside two it has not,
+  // 77 / 88 / 100 tokens 9.8 / 10.6 / 10.7 and 10.0 / 12.7 / 13.6).
+  const bool chained = grid_blocks <= sm_count();
   for (int b = 0; b < a->batch; ++b) {
     const float* mask = a->mask_bias + static_cast<size_t>(b) * a->n_i * a->n_k;
-    const dim3 grid(static_cast<unsigned>(blocks)), block(256);
+    const uint8_t* bias = static_cast<const uint8_t*>(a->bias) + b * bias_elems * (a->bias_f32 ? 4 : 2);
+    __nv_bfloat16* copy = reinterpret_cast<__nv_bfloat16*>(ws + pl.bias);
+    const BiasCopy rows = {bias, copy, bias_rows};
+    auto go = [&](auto kernel, auto* values) {
+      return launch(kernel, dim3(static_cast<unsigned>(grid_blocks)), dim3(256), 0, stream, chained, values + b * tok_k, mask, vt, mb,
+                    a->n_k, ld, static_cast<unsigned>(blocks), rows, chained);
+    };
+    const auto* v32 = static_cast<const float*>(a->v);
+    const auto* v16 = static_cast<const __nv_bfloat16*>(a->v);
     int rc;
     if (a->v_f32)
-      rc = launch(prepare_kernel<float>, grid, block, 0, stream, false, static_cast<const float*>(a->v) + b * tok_k, mask, vt,
-                  mb, a->n_k, ld);
+      rc = a->bias_f32 ? go(prepare_kernel<float, float>, v32) : go(prepare_kernel<float, __nv_bfloat16>, v32);
     else
-      rc = launch(prepare_kernel<__nv_bfloat16>, grid, block, 0, stream, false,
-                  static_cast<const __nv_bfloat16*>(a->v) + b * tok_k, mask, vt, mb, a->n_k, ld);
+      rc = a->bias_f32 ? go(prepare_kernel<__nv_bfloat16, float>, v16) : go(prepare_kernel<__nv_bfloat16, __nv_bfloat16>, v16);
     if (rc) return rc;
-    const uint8_t* bias = static_cast<const uint8_t*>(a->bias) + b * bias_elems * (a->bias_f32 ? 4 : 2);
     b200tri_triatt_core_args ca = {};
-    ca.bias = bias;
-    ca.bias_ld = a->n_k;
-    if (!bias_in_place) {
-      __nv_bfloat16* copy = reinterpret_cast<__nv_bfloat16*>(ws + pl.bias);
-      const long long rows = static_cast<long long>(HEADS) * a->n_j;
-      const long long want = (rows * ld + 255) / 256;
-      const long long most = 16ll * sm_count();
-      const dim3 bias_grid(static_cast<unsigned>(want < most ? want : most));
-      if (a->bias_f32)
-        rc = launch(bias_kernel<float>, bias_grid, block, 0, stream, false, reinterpret_cast<const float*>(bias), copy, rows,
-                    a->n_k, ld);
-      else
-        rc = launch(bias_kernel<__nv_bfloat16>, bias_grid, block, 0, stream, false,
-                    reinterpret_cast<const __nv_bfloat16*>(bias), copy, rows, a->n_k, ld);
-      if (rc) return rc;
-      ca.bias = copy;
-      ca.bias_ld = ld;
-    }
+    ca.bias = bias_in_place ? static_cast<const void*>(bias) : copy;
+    ca.bias_ld = bias_in_place ? a->n_k : ld;
     ca.bias_head_stride = ca.bias_ld * a->n_j;
     ca.n_i = a->n_i;
     ca.n_j = a->n_j;
