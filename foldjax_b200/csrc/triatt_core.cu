@@ -570,6 +570,7 @@ att_core_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         step(std::integral_constant<int, LAST>{}, whole);
         ++g;
       }
+      if (LAST == KT && !alive) break;  // (the wait below would tell; 2400 tokens take 0.7 % more without)
       // ---- item epilogue: O / l -> bf16 -> o[i][j][h*32 ..]
       alive = alive && mbar_wait(&sm.pv_done[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_SOFTMAX);
       if (!__all_sync(0xffffffffu, alive)) break;
