@@ -151,7 +151,7 @@ struct SideStream {
   cudaStream_t main, stream = nullptr;
   cudaEvent_t to_side = nullptr, to_main = nullptr, early = nullptr;
   bool joined = true;
-  SideStream(cudaStream_t main, bool want);
+  explicit SideStream(cudaStream_t main);
   ~SideStream();  // joins if need be
   SideStream(const SideStream&) = delete;
   SideStream& operator=(const SideStream&) = delete;

@@ -92,8 +92,7 @@ void destroy_side(const SideEntry& e) {
 }
 }  // namespace
 
-SideStream::SideStream(cudaStream_t main_, bool want) : main(main_) {
-  if (!want) return;
+SideStream::SideStream(cudaStream_t main_) : main(main_) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(main, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
   std::vector<SideEntry>& pool = g_side[current_device_slot()];
