@@ -33,9 +33,10 @@ namespace {
 
 constexpr int KT = 64;
 
-template <int HDP, bool TOKEN>
+// NWG: softmax warpgroups, each with a row, or (TOKEN) with 128 queries, of its own.
+template <int HDP, bool TOKEN, int NWG_>
 struct Cfg {
-  static constexpr int NWG = HDP == 32 ? 2 : 1;
+  static constexpr int NWG = NWG_;
   static constexpr int KV = TOKEN ? 1 : NWG;  // rows whose keys a step loads
   static constexpr int NB = TOKEN ? NWG : 1;  // bias tiles of a step
   static constexpr int STAGES = 2;
@@ -47,9 +48,9 @@ struct Cfg {
   static constexpr uint32_t STAGE_TX = KV * 3 * (K_BYTES + V_BYTES) + NB * BIAS_BYTES + KV * KT * 4;
 };
 
-template <int HDP, bool TOKEN>
+template <int HDP, bool TOKEN, int NWG>
 struct Smem {
-  using C = Cfg<HDP, TOKEN>;
+  using C = Cfg<HDP, TOKEN, NWG>;
   uint8_t q[C::NWG][3][C::Q_BYTES];
   uint8_t k[C::STAGES][C::KV][3][C::K_BYTES];
   uint8_t v[C::STAGES][C::KV][3][C::V_BYTES];
@@ -82,16 +83,16 @@ __device__ __forceinline__ float2 exp_below(float2 s, float2 minus_m) {
   return make_float2(fast_exp2(t.x), fast_exp2(t.y));
 }
 
-template <int HDP, bool TOKEN, int LAST>
-__global__ void __launch_bounds__(Cfg<HDP, TOKEN>::THREADS, 1)
+template <int HDP, bool TOKEN, int NWG, int LAST>
+__global__ void __launch_bounds__(Cfg<HDP, TOKEN, NWG>::THREADS, 1)
 att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
-  using C = Cfg<HDP, TOKEN>;
+  using C = Cfg<HDP, TOKEN, NWG>;
   using TQ = Terms<3, 3>;  // q . k
   using TP = Terms<3, 3>;  // P . v
-  constexpr int NWG = C::NWG, STAGES = C::STAGES;
-  static_assert(sizeof(Smem<HDP, TOKEN>) <= 232448, "shared memory budget");
+  constexpr int STAGES = C::STAGES;
+  static_assert(sizeof(Smem<HDP, TOKEN, NWG>) <= 232448, "shared memory budget");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  Smem<HDP, TOKEN>& sm = *reinterpret_cast<Smem<HDP, TOKEN>*>(smem_raw);
+  Smem<HDP, TOKEN, NWG>& sm = *reinterpret_cast<Smem<HDP, TOKEN, NWG>*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((smem_u32(smem_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
@@ -442,9 +443,9 @@ int with_last_columns(const Params& p, const F& go) {
   return go(std::integral_constant<int, KT>{});
 }
 
-template <int HDP, bool TOKEN>
+template <int HDP, bool TOKEN, int NWG>
 int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
-  using C = Cfg<HDP, TOKEN>;
+  using C = Cfg<HDP, TOKEN, NWG>;
   const int tiles = (p.n + 127) / 128;
   p.groups = TOKEN ? 1 : (p.n_i + C::NWG - 1) / C::NWG;
   p.tiles_j = TOKEN ? (tiles + C::NWG - 1) / C::NWG : tiles;
@@ -452,11 +453,11 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "float32 attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
   return with_last_columns(p, [&](auto last) {
-    const auto kernel = att_split_kernel<HDP, TOKEN, decltype(last)::value>;
-    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem<HDP, TOKEN>));
+    const auto kernel = att_split_kernel<HDP, TOKEN, NWG, decltype(last)::value>;
+    const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem<HDP, TOKEN, NWG>));
     if (rc) return rc;
     const unsigned sms = sm_count(), grid = p.total_items < sms ? p.total_items : sms;
-    return launch(kernel, dim3(grid), dim3(C::THREADS), sizeof(Smem<HDP, TOKEN>), stream, pdl, tm, p);
+    return launch(kernel, dim3(grid), dim3(C::THREADS), sizeof(Smem<HDP, TOKEN, NWG>), stream, pdl, tm, p);
   });
 }
 
@@ -973,10 +974,15 @@ int launch_att_split(const AttSplitArgs& a, cudaStream_t stream) {
   p.pieces = a.pieces;
   p.status = device_status_word();
   B200_REQUIRE(p.status != nullptr, B200TRI_ERR_CUDA, "general attention: no current CUDA device");
-  if (token) return launch_cfg<32, true>(tm, p, a.pdl, stream);
+  // One row: tiles of 128 queries in a CTA of their own where the SMs are enough for all. A step is 36 products of the tensor pipe
+  // a tile, and with two tiles to a CTA they queued for each other: 203 / 1024 tokens 18.9 / 56.2 us, 13.9 / 40.5 so (blocks of 128 /
+  // 203 / 300 tokens 157.1 / 260.3 / 473.2 -> 155.0 / 255.6 / 465.6). With more tiles than SMs two share their keys.
+  if (token)
+    return static_cast<long long>(a.heads) * ((a.n + 127) / 128) <= sm_count() ? launch_cfg<32, true, 1>(tm, p, a.pdl, stream)
+                                                                               : launch_cfg<32, true, 2>(tm, p, a.pdl, stream);
   if (a.bf16 && hdp == 16) return launch_bf16_narrow<16>(tm, p, a.pdl, stream);
   if (a.bf16) return hdp == 32 ? launch_bf16_narrow<32>(tm, p, a.pdl, stream) : launch_bf16<64, 2>(tm, p, a.pdl, stream);
-  return hdp == 32 ? launch_cfg<32, false>(tm, p, a.pdl, stream) : launch_cfg<64, false>(tm, p, a.pdl, stream);
+  return hdp == 32 ? launch_cfg<32, false, 2>(tm, p, a.pdl, stream) : launch_cfg<64, false, 1>(tm, p, a.pdl, stream);
 }
 
 }  // namespace b200
