@@ -381,13 +381,14 @@ struct GemmRuns {
   uint32_t units;           // slow-direction tiles x parts
 };
 
-// ONCE: the stages hold the whole streamed operand (the weights), which is loaded for a CTA's first unit and stays, and
-// there are places for several units' k steps.
-template <class P, bool ONCE>
+// KEPT_KB > 0: the stages hold the whole streamed operand (the weights) of so many k steps, which is loaded for a CTA's first
+// unit and stays, and there are places for several units' k steps.
+template <class P, int KEPT_KB>
 __global__ void __launch_bounds__(gemm_threads<P>(), 1)
 piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShape g, const GemmRuns runs,
                            const typename P::Params ep) {
   static_assert(P::CTAS == 1 && (P::M_FAST || P::NSEG == 1), "one operand for all segments");
+  constexpr bool ONCE = KEPT_KB > 0;
   constexpr int RES = gemm_res_bytes<P>(), STREAM = gemm_stream_bytes<P>();
   constexpr int SEG = gemm_acc_count<P>() * P::BN, ACC = P::NSEG * SEG;
   constexpr uint32_t NBUF = 2 * ACC <= 512 ? 2 : 1;
@@ -395,7 +396,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
   static_assert(NBUF * ACC <= 512, "tile does not fit");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int kbs = g.kb[0], slots = ONCE ? runs.slots : kbs, stages = runs.stages;
+  const int kbs = ONCE ? KEPT_KB : g.kb[0], slots = ONCE ? runs.slots : kbs, stages = runs.stages;
   uint8_t* ring = smem + slots * RES;
   __shared__ uint64_t res_full[RES_SLOTS], res_empty[RES_SLOTS], full_bar[RES_SLOTS], empty_bar[RES_SLOTS], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
@@ -509,7 +510,9 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
             break;
           }
           tc_fence_after();
+#pragma unroll
           for (int seg = 0; seg < P::NSEG && alive; ++seg)
+#pragma unroll
             for (int kb = 0; kb < kbs; ++kb) {
               const int slot = place(kept, kb);
               if ((f == f0 && seg == 0 && !mbar_wait(&res_full[slot], round ^ (slot < kept), g.status, ST_TIMEOUT_MMA)) ||
@@ -612,14 +615,15 @@ int launch_piece_gemm_resident(const GemmMaps& maps, GemmShape g, const typename
   if constexpr (P::PA * P::PB == 1) {
     const int all = r.fast * P::NSEG * g.kb[0];
     const int left = (222 * 1024 - all * gemm_stream_bytes<P>()) / gemm_res_bytes<P>();
-    if (r.log_parts == 0 && all <= RES_SLOTS && left >= 2 * g.kb[0]) {
+    if (g.kb[0] <= 2 && r.log_parts == 0 && all <= RES_SLOTS && left >= 2 * g.kb[0]) {
       const int most = 4 * g.kb[0] < RES_SLOTS ? 4 * g.kb[0] : RES_SLOTS;
       r.slots = left < most ? left : most;
       r.stages = all;
-      return go(piece_gemm_resident_kernel<P, true>);
+      if (g.kb[0] == 1) return go(piece_gemm_resident_kernel<P, 1>);
+      return go(piece_gemm_resident_kernel<P, 2>);
     }
   }
-  return go(piece_gemm_resident_kernel<P, false>);
+  return go(piece_gemm_resident_kernel<P, 0>);
 }
 
 // Activations: bf16 pieces [pieces][rows][k], row pitch `pitch` elements (a multiple of 8);
