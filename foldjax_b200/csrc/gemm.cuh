@@ -109,6 +109,7 @@ struct GemmShape {
 // What a policy P provides:
 //   BN, PA, PB, NSEG, NMAIN, A_MN, B_MN, M_FAST   shape constants (M_FAST: successive tiles walk m)
 //   EPI, CTAS                                     epilogue warps, CTAs per SM
+//   TURNS (with an operand resident)              whether the epilogue warps take a tile's columns in turn
 //   struct Params                                 arguments
 //   load_a / load_b(maps, params, seg, k, tile, piece, dst, bar)  one piece of one k step
 //   Pre, prefetch(params, m_tile, n_tile, quarter, col0, col1, lane, pre)   what the epilogue reads from
@@ -549,8 +550,8 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
       }
     }
   } else if (warp >= 4) {
-    const int quarter = warp & 3, part = (warp - 4) >> 2;
-    constexpr int SHARE = P::BN / (P::EPI / 4);
+    const int quarter = warp & 3;
+    constexpr int PARTS = P::EPI / 4, SHARE = P::BN / PARTS;
     uint32_t it = 0;
     bool alive = true;
     for (uint32_t unit = blockIdx.x; unit < runs.units && alive; unit += gridDim.x) {
@@ -559,6 +560,7 @@ piece_gemm_resident_kernel(const __grid_constant__ GemmMaps maps, const GemmShap
       for (int f = f0; f < f1; ++f, ++it) {
         const int m_tile = P::M_FAST ? f : slow, n_tile = P::M_FAST ? slow : f;
         const uint32_t buf = it % NBUF, buf_phase = (it / NBUF) & 1;
+        const int part = static_cast<int>((warp - 4) / 4 + (P::TURNS ? it + it / PARTS : 0)) % PARTS;
         typename P::Pre pre;
         P::prefetch(ep, m_tile, n_tile, quarter, part * SHARE, (part + 1) * SHARE, lane, pre);
         if (!mbar_wait(&acc_full[buf], buf_phase, g.status, ST_TIMEOUT_EPILOGUE)) {

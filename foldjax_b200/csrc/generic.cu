@@ -758,6 +758,7 @@ struct RowTile {
 template <int PIECES, int NM, bool RES = false>
 struct GluPolicy {
   static constexpr int BN = PIECES == 1 ? 128 : 64, PA = PIECES, PB = PIECES, NSEG = 2, NMAIN = NM;
+  static constexpr bool TURNS = false;  // (in turn: 42 us instead of 40 for four 200-token templates)
   static constexpr bool A_MN = true, B_MN = false, M_FAST = true;
   static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   struct Params {
@@ -912,6 +913,7 @@ struct OutGatePolicy {
 template <int PIECES, int NM, int BN_, bool RES = false>
 struct QkvbPolicy : NoPrefetch {
   static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 1, NMAIN = NM;
+  static constexpr bool TURNS = true;  // tiles with the bias end in columns that do not exist: 28.0 -> 25.5 us
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = PIECES == 1 && !RES ? 8 : 16, CTAS = PIECES == 1 && !RES ? 2 : 1;
   static constexpr bool BF = PIECES == 1;
