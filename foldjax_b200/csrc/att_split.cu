@@ -93,7 +93,9 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
   static_assert(sizeof(Smem<HDP, TOKEN, NWG>) <= 232448, "shared memory budget");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem<HDP, TOKEN, NWG>& sm = *reinterpret_cast<Smem<HDP, TOKEN, NWG>*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (through a shuffle, so that the compiler knows it to be the same in all lanes)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   if ((smem_u32(smem_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicCAS(p.status, ST_OK, 900);
     return;
@@ -107,7 +109,7 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
     mbar_init(&sm.q_empty, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sm.st_full[s], 1);
-      mbar_init(&sm.st_empty[s], 1 + NWG * 4);
+      mbar_init(&sm.st_empty[s], NWG + NWG * 4);
     }
     for (int g = 0; g < NWG; ++g) {
       mbar_init(&sm.s_full[g], 1);
@@ -181,25 +183,24 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
       }
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0, item_it = 0, g = 0;
-      bool alive = true;
-      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x, ++item_it) {
-        if (!mbar_wait(&sm.q_full, item_it & 1, p.status, ST_TIMEOUT_MMA)) break;
-        for (int t = 0; t < p.steps && alive; ++t, ++g) {
-          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
-            alive = false;
-            break;
-          }
-          const uint32_t idesc = umma_idesc_bf16(128, LAST < KT && t + 1 == p.steps ? LAST : KT);
-          for (int wg = 0; wg < NWG; ++wg) {
-            if (!mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA)) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t d = tmem_base + wg * C::TM_WG + C::TM_S;
+    // In the issuers all lanes walk the loops and wait, and one of them issues; none leaves early: one whose wait has run out
+    // stops waiting and issuing and walks on. Joins as in triatt_core.cu.
+    const bool leader = elect_one();
+    int stage = 0;
+    uint32_t phase = 0, item_it = 0, g = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x, ++item_it) {
+      alive = alive && mbar_wait(&sm.q_full, item_it & 1, p.status, ST_TIMEOUT_MMA);
+      for (int t = 0; t < p.steps; ++t, ++g) {
+        alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+        const uint32_t idesc = umma_idesc_bf16(128, LAST < KT && t + 1 == p.steps ? LAST : KT);
+#pragma unroll
+        for (int wg = 0; wg < NWG; ++wg) {
+          alive = alive && mbar_wait(&sm.s_free[wg], (g & 1) ^ 1, p.status, ST_TIMEOUT_MMA);
+          __syncwarp();
+          tc_fence_after();
+          const uint32_t d = tmem_base + wg * C::TM_WG + C::TM_S;
+          if (leader && alive) {
 #pragma unroll
             for (int term = 0; term < TQ::N; ++term) {
               const uint64_t adesc = umma_desc_kmajor(smem_u32(sm.q[wg][TQ::a(term)]), HDP * 2);
@@ -211,51 +212,46 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
             }
             umma_commit(&sm.s_full[wg]);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
         }
-        if (alive) umma_commit(&sm.q_empty);
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
+      if (leader && alive) umma_commit(&sm.q_empty);
     }
-  } else if (warp == 2) {
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, HDP);
-      int stage = 0;
-      uint32_t phase = 0, g = 0;
-      bool alive = true;
-      for (uint32_t item = blockIdx.x; item < p.total_items && alive; item += gridDim.x) {
-        for (int t = 0; t < p.steps && alive; ++t, ++g) {
-          if (!mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA)) {
-            alive = false;
-            break;
-          }
-          const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
-          for (int wg = 0; wg < NWG; ++wg) {
-            if (!mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA)) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t base = tmem_base + wg * C::TM_WG;
+  } else if (warp < 2 + NWG) {  // P.V of a row each
+    const bool leader = elect_one();
+    constexpr uint32_t idesc = umma_idesc_bf16(128, HDP);
+    const int wg = warp - 2;
+    int stage = 0;
+    uint32_t phase = 0, g = 0;
+    bool alive = true;
+    for (uint32_t item = blockIdx.x; item < p.total_items; item += gridDim.x) {
+      for (int t = 0; t < p.steps; ++t, ++g) {
+        alive = alive && mbar_wait(&sm.st_full[stage], phase, p.status, ST_TIMEOUT_MMA);
+        alive = alive && mbar_wait(&sm.p_full[wg], g & 1, p.status, ST_TIMEOUT_MMA);
+        __syncwarp();
+        tc_fence_after();
+        const int cols = LAST < KT && t + 1 == p.steps ? LAST : KT;
+        const uint32_t base = tmem_base + wg * C::TM_WG;
+        const uint32_t vbase = smem_u32(sm.v[stage][TOKEN ? 0 : wg][0]);
+        if (leader && alive) {
 #pragma unroll
-            for (int term = 0; term < TP::N; ++term) {
-              const uint64_t vdesc = umma_desc_kmajor(smem_u32(sm.v[stage][TOKEN ? 0 : wg][TP::b(term)]), 128);
+          for (int term = 0; term < TP::N; ++term) {
+            const uint64_t vdesc = umma_desc_kmajor(vbase + TP::b(term) * C::V_BYTES, 128);
 #pragma unroll
-              for (int kk = 0; kk < KT / 16; ++kk)
-                if (kk * 16 < LAST || kk * 16 < cols)
-                  umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
+            for (int kk = 0; kk < KT / 16; ++kk)
+              if (kk * 16 < LAST || kk * 16 < cols)
+                umma_bf16_ts(base + C::TM_O, base + C::TM_P + TP::a(term) * 32 + kk * 8, umma_desc_advance(vdesc, kk * 32),
                              idesc, (term | kk) != 0);
-            }
-            umma_commit(&sm.pv_done[wg]);
           }
-          if (!alive) break;
+          umma_commit(&sm.pv_done[wg]);
           umma_commit(&sm.st_empty[stage]);
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
