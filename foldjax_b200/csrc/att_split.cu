@@ -15,8 +15,8 @@
 // thread, which also makes the rescale a register fma).
 //
 // One CTA per SM, persistent; an item is (head, NWG rows, 128 queries), or with one row (head,
-// NWG tiles of 128 queries), walked in steps of 64 keys:
-//   warp 0      TMA producer       warp 1   S issuer       warp 2   P.V issuer
+// NWG tiles of 128 queries), walked in steps of 64 keys, the last one of as many columns as it needs:
+//   warp 0      TMA producer       warp 1   S issuer       warps 2, 3   P.V issuers, one for each row or tile
 //   warpgroups  softmax, one thread per query
 // Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (counters, 512 tokens, 4 heads x
 // 32, 565 us; a score costs about 2 instructions of exponential, 3.5 of split and 4 others, most of them packed two to an
