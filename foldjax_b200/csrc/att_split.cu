@@ -476,7 +476,7 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
 // score) and products (18 of them, 0.35 us, and the trips between the warps), and the rows in flight hide
 // each other's. Three rows, P.V issued by one warp, padded heads of 16, rounded pieces and pairs unpacked from them
 // took 695 us for the four updates of four 200-token templates, 1 178 for those of a 256-token refiner, 112 and 247 for
-// attention of 200 and 320 tokens with 4 heads x 64; now 615, 1 130, 105 and 219. It issues in 69 % of its slots with 65 % of
+// attention of 200 and 320 tokens with 4 heads x 64; 615, 1 130, 105 and 219 so. It issues in 69 % of its slots with 65 % of
 // the MUFU unit busy (counters, 4 x 400 tokens, 4 heads x 16).
 // HDP: a head's width in the products, rounded up to 16, 32 or 64. Heads of 16 as 32 pay for a product of
 // zeros a step and twice the columns in P.V, and read back twice the result: 2.3 % of the templates' time (the same bits).

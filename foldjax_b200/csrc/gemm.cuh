@@ -361,7 +361,7 @@ int launch_piece_gemm(const GemmMaps& maps, GemmShape g, const typename P::Param
 // otherwise, 512 clocks for 256 of products; so it reads half. The resident k steps have barriers
 // of their own and are refilled one by one behind the last tile's products.
 // Gated projection, 65 536 pairs x 384 -> 768 channels: 104 -> 94 us; 160 000 x 64 -> 256: 72 -> 67;
-// q, k, v and bias, 160 000 x 64: 56 -> 45 (384 channels: 96 -> 107, left streaming).
+// q, k, v and bias, 160 000 x 64: 56 -> 45 (wider ones where there are tiles enough: the rule is in generic.cu).
 constexpr int RES_KB = 8, RES_STAGES = 8, RES_SLOTS = 16;  // most k steps kept, streamed stages, places of either
 template <class P>
 constexpr int gemm_res_bytes() {

@@ -17,8 +17,8 @@
 // and an attention five
 //   layer norm -> q, k, v, bias product -> core -> gate product -> output product
 // (plus one that splits or pads weights where they cannot be read as stored). The layer norms
-// are CUDA-core kernels. The four updates of a 256-token 384-channel refiner block take 1.12 ms and
-// those of four 200-token templates 0.62 (26.2 and 6.9 with the products on the CUDA cores). What the
+// are CUDA-core kernels. The four updates of a 256-token 384-channel refiner block take 1.05 ms and
+// those of four 200-token templates 0.54 (26.2 and 6.9 with the products on the CUDA cores). What the
 // threads of an epilogue move, each along a row of its own, goes 32 bytes at a time: with 16 those
 // stacks took 1.29 and 0.80 ms and a 256-token float32 stack 1.01 instead of 0.91.
 //
@@ -1414,14 +1414,15 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         const int groups_w = (hd + 63) / 64, groups = 3 * groups_w + (heads + 63) / 64;
         const GemmShape g = {m_tiles, (groups + Pol::BN / 64 - 1) / (Pol::BN / 64), 1, {ksteps(c_z), 0}, nullptr};
         const float q_scale = BF ? __bfloat162float(__float2bfloat16_rn(root)) : root;
-        // (Kept / streamed, us of the whole bf16 attention of 256 tokens: 128 channels of 8 x 16 heads
-        // 172 / 184, of 12 x 32 304 / 294; 192 of 6 x 32 213 / 220; 256 of 8 x 32 246 / 252; 320 of 10 x 32
-        // 314 / 311; 384 of 12 x 32 367 / 363. Keeping pays where a weight is few column tiles wide, in
-        // float32 up to 128 channels: 455 / 491 for four 200-token templates, 333 / 313 at 192. The rule
-        // goes by k steps, which is within 4 % of the better side.)
+        // Keeping the rows pays up to two k steps, and in bf16 with more where there are tiles enough for long runs: streamed,
+        // 128 x 128 tiles take 64 bytes a clock and SM, all that L2 gives. Kept / streamed, us: refiner stacks (384 channels, 12 x 32
+        // heads) of 300 / 256 / 200 / 150 / 100 tokens 1683 / 1697, 1053 / 1068, 731 / 732, 472 / 460, 243 / 230 (704 / 512 /
+        // 313 / 176 / 79 tiles of rows); float32 attention of 128 channels, four 200-token templates, 455 / 491, of 192 333 / 313.
+        // (512 channels, 256 tokens: 418 / 412.)
+        const bool keep = ksteps(c_z) <= 2 || (BF && ksteps(c_z) <= 6 && m_tiles >= 3 * sm_count());
         return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, groups_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
                                                 static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
-                                                ws + pl.bias}, ksteps(c_z) <= 2, stream);
+                                                ws + pl.bias}, keep, stream);
       };
       if constexpr (BF)
         rc = go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});

@@ -1,7 +1,8 @@
 """Products of the general bf16 path whose weights stay in shared memory (piece_gemm_resident_kernel, ONCE): one and two
 k steps; fewer, as many and more units of rows than SMs, so that the ring of rows goes round; runs of one tile where all of
 them fit the SMs at once; column groups of two weights in a tile, a last group that no weight has, as many heads as a group of
-columns. And shapes on the other side of the rule: weights that leave no room for two units' rows, three k steps.
+columns. And shapes on the other side of the rule: weights that leave no room for two units' rows, three k steps; of
+those a little fewer and a little more tiles of rows than make keeping the rows pay.
 
 Tolerance: the benchmark's bf16 budget (conftest.assert_parity)."""
 
@@ -34,7 +35,8 @@ def test_gated_projection(cuda_device, batch, n, c_z, c_hidden):
 
 @pytest.mark.parametrize("batch,n,c_z,heads,head_dim", [(1, 5, 64, 4, 16), (1, 97, 64, 4, 16), (1, 98, 64, 8, 8), (3, 100, 64, 4, 16),
                                                         (1, 131, 40, 2, 24), (1, 137, 72, 2, 48), (1, 90, 64, 3, 32), (1, 60, 64, 64, 8),
-                                                        (1, 90, 128, 4, 16), (1, 60, 136, 4, 16)])
+                                                        (1, 90, 128, 4, 16), (1, 60, 136, 4, 16),
+                                                        (1, 237, 136, 4, 16), (1, 240, 136, 4, 16), (2, 171, 136, 4, 16)])
 def test_attention_projection(cuda_device, batch, n, c_z, heads, head_dim):
     from foldjax_b200 import _lib
     from foldjax_b200.triangle_attention import triangle_attention_forward
