@@ -809,7 +809,10 @@ int core_launch(const b200tri_triatt_core_args* tiles, int n_tiles, b200tri_stre
   switch (round_up(a->n_k - KT * (p.steps - 1), 16)) {
     case 16: return go(att_core_kernel<1, 16>, one);
     case 32: return go(att_core_kernel<1, 32>, one);
-    case 48: return go(att_core_kernel<1, 48>, one);
+    case 48:
+      // (48 columns behind a single whole step cost as much as 64, in code of their own that each CTA comes to once: attention of 100 /
+      // 110 tokens 22.3 / 22.4 us with 64, 22.8 / 23.0 with 48; 170 tokens 44.5 and 44.1, operator of 300 73.4 and 71.4)
+      if (p.steps != 2) return go(att_core_kernel<1, 48>, one);
   }
   return go(att_core_kernel<1, KT>, one);
 }
