@@ -843,6 +843,10 @@ struct OutGatePolicy {
   static constexpr bool A_MN = false, B_MN = true, M_FAST = false;
   static constexpr int EPI = PIECES == 1 && BN <= 64 ? 8 : 16, CTAS = PIECES == 1 && BN <= 64 ? 2 : 1;
   static constexpr bool BF = PIECES == 1;
+  // A float32 row beside three leading accumulators is more than the registers hold: asked for ahead of them, 68 bytes of spills and,
+  // with or without a residual, 192 channels of 200 / 256 tokens 93 / 118 and 87 / 110 us, 92 / 119 and 76 / 96 behind them. Beside
+  // one, 128 channels of 256 tokens 39.7 against 43.7, without a residual 36.1 both.
+  static constexpr bool EARLY = BF || NM == 1;
   using O = typename std::conditional<BF, __nv_bfloat16, float>::type;
   struct Params {
     int n, c_z;
@@ -853,7 +857,7 @@ struct OutGatePolicy {
   };
   using Pre = typename std::conditional<BF, RowPrefetch<BN / (EPI / 4)>, RowPrefetchF<BN / (EPI / 4)>>::type;
   static __device__ void prefetch(const Params& p, int m_tile, int n_tile, int quarter, int col0, int, int lane, Pre& pre) {
-    if (!p.res || !p.aligned) return;
+    if (!EARLY || !p.res || !p.aligned) return;
     const RowTile rt(m_tile, p.by_n, p.tiles_j, GEMM_BM);
     const int j = rt.t0 + quarter * 32 + lane, c0 = n_tile * BN + col0;
     pre.load(p.res + ((static_cast<long long>(rt.b) * p.n + rt.o) * p.n + j) * p.c_z + c0, j < p.n ? p.c_z - c0 : 0, p.sectors);
@@ -897,7 +901,7 @@ struct OutGatePolicy {
           continue;
         }
       }
-      const bool there = !BF && p.res && p.aligned;  // the residual has been asked for
+      const bool there = EARLY && !BF && p.res && p.aligned;  // the residual has been asked for
       if constexpr (!BF) {
         if (there)
 #pragma unroll
