@@ -39,3 +39,23 @@ def test_attention_core_operator(cuda_device, b, n_i, n_j, n_k, v_f32, bias_f32,
     _lib.device_status()
     assert got.shape == ref.shape and got.dtype == (f32 if v_f32 else bf)
     assert_parity(ref, got.float().cpu().numpy(), label=f"operator {b}x{n_i}x{n_j}x{n_k}")
+
+
+@pytest.mark.parametrize("n_k", [1, 63, 65, 511, 513, 575, 1025])
+@pytest.mark.parametrize("bias_f32", [False, True])
+def test_copied_bias_rows(cuda_device, n_k, bias_f32):
+    """The bias where the preparation copies it: rows that end anywhere in the 512 elements a warp takes at a time, and a
+    last block of rows that is not full."""
+    from foldjax_b200 import _lib
+    from foldjax_b200.triangle_attention import attention_core
+
+    n_j = 9
+    rng = np.random.default_rng(n_k)
+    draw = lambda *shape, scale=1.0: orc.round_bf16(rng.normal(size=shape, scale=scale).astype(np.float32))
+    q, k, v = draw(1, 2, 4, n_j, 32, scale=0.5), draw(1, 2, 4, n_k, 32, scale=0.5), draw(1, 2, 4, n_k, 32)
+    tb, mb = draw(1, 1, 4, n_j, n_k, scale=2.0), np.zeros((1, 2, 1, 1, n_k), np.float32)
+    ref = orc.attention_core(q, k, v, tb, mb, dtype="bfloat16")
+    t = lambda a, dtype=torch.bfloat16: torch.from_numpy(a).to(cuda_device).to(dtype)
+    got = attention_core(t(q), t(k), t(v), t(tb, torch.float32 if bias_f32 else torch.bfloat16), t(mb, torch.float32))
+    _lib.device_status()
+    assert_parity(ref, got.float().cpu().numpy(), label=f"operator, bias rows of {n_k}")
