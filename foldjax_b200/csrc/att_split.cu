@@ -21,6 +21,7 @@
 // Bound of the float32 kernel: two softmax warpgroups fill 41 % of the issue slots (counters, 512 tokens, 4 heads x
 // 32, 565 us; a score costs about 2 instructions of exponential, 3.5 of split and 4 others, most of them packed two to an
 // instruction; with 4.5 of split it was 41 % and 575); the rest is products (1300 clocks of the tensor pipe for a row's step) and loads, 80 KiB a step and SM.
+#include <climits>
 #include <type_traits>
 
 #include "att_split.cuh"
@@ -429,12 +430,18 @@ att_split_kernel(const __grid_constant__ Maps tm, const Params p) {
 // Calls go with the columns of an item's last step as a constant: 16, 32, 48 or 64, whichever hold the keys that are left.
 // (Templates of 200 tokens 610 -> 590 us, 150-token refiner 499 -> 487, 200-token float32 stack 644 -> 642, blocks of 136 and
 // 203 tokens, single track only, 198.7 -> 197.2 and 262.7 -> 261.6; the same bits.)
-template <class F>
+// STEPS48: most steps of an item whose last one takes 48 columns instead of 64. Us of a core with 64 and with 48, 100 / 170 / 240 tokens:
+// 4 bf16 heads x 16 9.0 / 27.4 / 41.5 and 8.7 / 26.2 / 39.6, 12 x 32 22.1 / 60.3 / 105 and 21.4 / 57.3 / 98.6; float32 4 x 32 26.6 /
+// 57.3 / 96.8 and 26.0 / 58.4 / 98.4; but bf16 4 x 64 20.7 / 44.7 / 70.4 and 21.0 / 45.0 / 72.6, float32 2 x 64 24.8 / 55.5 / 89.9 and
+// 25.3 / 56.3 / 90.4, single track 12.9 / 15.7 / 17.1 and 13.1 / 15.8 / 17.1: none there.
+template <int STEPS48, class F>
 int with_last_columns(const Params& p, const F& go) {
   switch (round_up(p.n - KT * (p.steps - 1), 16)) {
     case 16: return go(std::integral_constant<int, 16>{});
     case 32: return go(std::integral_constant<int, 32>{});
-    case 48: return go(std::integral_constant<int, 48>{});
+    case 48:
+      if constexpr (STEPS48 > 0)
+        if (p.steps <= STEPS48) return go(std::integral_constant<int, 48>{});
   }
   return go(std::integral_constant<int, KT>{});
 }
@@ -448,7 +455,7 @@ int launch_cfg(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "float32 attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
-  return with_last_columns(p, [&](auto last) {
+  return with_last_columns<HDP == 32 && !TOKEN ? 2 : 0>(p, [&](auto last) {
     const auto kernel = att_split_kernel<HDP, TOKEN, NWG, decltype(last)::value>;
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(Smem<HDP, TOKEN, NWG>));
     if (rc) return rc;
@@ -891,7 +898,7 @@ int launch_bf16(const Maps& tm, Params p, bool pdl, cudaStream_t stream) {
   const long long items = static_cast<long long>(p.total_items) * p.groups * p.tiles_j;
   B200_REQUIRE(items < (1ll << 32) - 1024, B200TRI_ERR_UNSUPPORTED, "general attention: too many tiles");
   p.total_items = static_cast<uint32_t>(items);
-  return with_last_columns(p, [&](auto last) {
+  return with_last_columns<HDP <= 32 ? INT_MAX : 0>(p, [&](auto last) {
     const auto kernel = att_bf16_kernel<HDP, NWG, decltype(last)::value>;
     const int rc = ensure_smem_limit(reinterpret_cast<const void*>(kernel), (int)sizeof(BfSmem<HDP, NWG>));
     if (rc) return rc;
