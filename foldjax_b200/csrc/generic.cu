@@ -1421,15 +1421,25 @@ int triatt_generic(const b200tri_triatt_args* a, int c_z, cudaStream_t stream) {
         // Keeping the rows pays up to two k steps, and in bf16 with more where there are tiles enough for long runs: streamed,
         // 128 x 128 tiles take 64 bytes a clock and SM, all that L2 gives. Kept / streamed, us: refiner stacks (384 channels, 12 x 32
         // heads) of 300 / 256 / 200 / 150 / 100 tokens 1683 / 1697, 1053 / 1068, 731 / 732, 472 / 460, 243 / 230 (704 / 512 /
-        // 313 / 176 / 79 tiles of rows); float32 attention of 128 channels, four 200-token templates, 455 / 491, of 192 333 / 313.
-        // (512 channels, 256 tokens: 418 / 412.)
+        // 313 / 176 / 79 tiles of rows); attention of as many channels as heads x 32, 192 / 256 / 320 / 384, at 256 tokens 147 / 154, 187 / 189,
+        // 221 / 221, 281 / 295, the last three at 384 tokens 490 / 508, 610 / 625, 756 / 774; 4 heads x 16 at 256 tokens 109.8 / 110.1,
+        // 114.3 / 114.9, 130.1 / 131.1, 140.2 / 141.5 (512 channels 176.6 / 177.4, left streaming); float32 attention of 128 channels, four
+        // 200-token templates, 455 / 491, of 192 333 / 313.
         const bool keep = ksteps(c_z) <= 2 || (BF && ksteps(c_z) <= 6 && m_tiles >= 3 * sm_count());
-        return launch_either<Pol, decltype(kept)>(proj, g, {n, hd, heads, groups_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
-                                                static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt),
-                                                ws + pl.bias}, keep, stream);
+        const typename Pol::Params params = {n, hd, heads, groups_w, ld, Divisor(n), static_cast<uint32_t>(pairs), q_scale, 1.0f / q_scale, pairs * hd,
+                                             static_cast<long long>(nb) * n * hd * ld, at(pl.q), at(pl.k), at(pl.vt), ws + pl.bias};
+        if constexpr (std::is_same<Pol, decltype(kept)>::value)
+          return launch_piece_gemm<Pol>(proj, g, params, stream, true);
+        else
+          return launch_either<Pol, decltype(kept)>(proj, g, params, keep, stream);
       };
+      // Narrow heads with little more than a tile of rows an SM: 64 columns, streamed, are four tiles to share among the SMs instead of two
+      // (us with them and with 128 columns, 4 heads x 16, tokens: 64 channels of 64 / 100 / 150 4.3 / 5.7 / 9.0 and 5.2 / 6.3 / 10.1, 256
+      // 5.4 / 8.4 / 15.0 and 6.3 / 9.5 / 16.0, 512 6.7 / 12.4 / 19.5 and 8.0 / 13.3 / 21.0; at 200 tokens, 313 tiles of rows, 64 / 192 / 256 /
+      // 384 channels 15.9 / 21.0 / 23.9 / 31.3 and 14.2 / 21.6 / 23.8 / 29.5, at 256 19.9 / 30.4 / 36.4 / 41.3 and 15.6 / 28.5 / 32.6 / 36.5).
       if constexpr (BF)
-        rc = go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
+        rc = hd <= 64 && 4ll * m_tiles <= 5ll * sm_count() ? go(QkvbPolicy<1, 1, 64>{}, QkvbPolicy<1, 1, 64>{})
+                                                           : go(QkvbPolicy<1, 1, 128>{}, QkvbPolicy<1, 1, 128, true>{});
       else
         rc = ksteps(c_z) <= 2 ? go(QkvbPolicy<3, 2, 64>{}, QkvbPolicy<3, 2, 64, true>{}) : go(QkvbPolicy<3, 3, 64>{}, QkvbPolicy<3, 3, 64, true>{});
       if (rc) return rc;
