@@ -682,20 +682,19 @@ int map_rows(CUtensorMap* out, const void* base, int k, int n, long long s_inner
 // waited for. Loaded after them it cost a gate tile two memory latencies, most of its time.
 template <int COLS>
 struct RowPrefetch {
-  uint4 row[COLS > 0 ? COLS / 8 : 1];
+  static_assert(COLS % 16 == 0, "whole sectors");
+  uint4 row[COLS / 8];
   // `left` columns exist. `sectors`: rows start on 32-byte boundaries and have whole runs of 16 columns,
   // which then are one access: half an L2 sector at a time, what 128 rows of a tile cost the load/store
   // unit and L2 was most of a product's epilogue.
   __device__ __forceinline__ void load(const __nv_bfloat16* src, int left, bool sectors) {
-    if constexpr (COLS % 16 == 0) {
-      if (sectors) {
+    if (sectors) {
 #pragma unroll
-        for (int q = 0; q < COLS / 8; q += 2) {
-          row[q] = row[q + 1] = make_uint4(0u, 0u, 0u, 0u);
-          if (8 * q < left) load_sector(src + 8 * q, row[q], row[q + 1]);
-        }
-        return;
+      for (int q = 0; q < COLS / 8; q += 2) {
+        row[q] = row[q + 1] = make_uint4(0u, 0u, 0u, 0u);
+        if (8 * q < left) load_sector(src + 8 * q, row[q], row[q + 1]);
       }
+      return;
     }
 #pragma unroll
     for (int q = 0; q < COLS / 8; ++q)
@@ -835,8 +834,8 @@ struct GluPolicy {
 
 // out = R(R(tn p_out) * R(sigmoid(R(xn g_out)))) (+ residual)
 // Here and in the two products behind the attention core a tile of 128 bf16 columns has an SM with 16 epilogue warps to itself: as two
-// CTAs of eight, and with room for one accumulator each, 384-channel refiners of 64 / 100 / 150 tokens took 167 / 241 / 482 us, 159 /
-// 232 / 466 so; 256 tokens the same.
+// CTAs of eight (in this product without a second pair of accumulators) 384-channel refiners of 64 / 100 / 150 tokens took 167 / 241 /
+// 482 us, 159 / 232 / 466 so; 256 tokens the same.
 template <int PIECES, int NM, int BN_>
 struct OutGatePolicy {
   static constexpr int BN = BN_, PA = PIECES, PB = PIECES, NSEG = 2, NMAIN = NM;
