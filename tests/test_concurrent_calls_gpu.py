@@ -58,13 +58,17 @@ def _inputs(device, sizes):
     return out
 
 
-@pytest.mark.parametrize("name", ["mul", "attn", "attn f32", "transition", "core", "trunk"])
+CALLS = [(name, (200, 136, 264)) for name in ("mul", "attn", "attn f32", "transition", "core", "trunk")]
+CALLS += [("core", (60, 48, 64))]  # (whose first kernel is launched programmatically)
+
+
+@pytest.mark.parametrize("name,sizes", CALLS)
 @pytest.mark.parametrize("threads", [False, True])
-def test_concurrent_calls_equal_calls_one_by_one(cuda_device, name, threads):
+def test_concurrent_calls_equal_calls_one_by_one(cuda_device, name, sizes, threads):
     from foldjax_b200 import _lib
 
     call = _calls(cuda_device)[name]
-    inputs = _inputs(cuda_device, (200, 136))
+    inputs = _inputs(cuda_device, sizes[:2])
     want = [call(z, m) for z, m in inputs]
     torch.cuda.synchronize()
     got = [[] for _ in inputs]
@@ -95,14 +99,14 @@ def test_concurrent_calls_equal_calls_one_by_one(cuda_device, name, threads):
             assert torch.equal(r, w)
 
 
-@pytest.mark.parametrize("name", ["mul", "attn", "attn f32", "transition", "core", "trunk"])
-def test_captured_calls(cuda_device, name):
+@pytest.mark.parametrize("name,sizes", CALLS)
+def test_captured_calls(cuda_device, name, sizes):
     """Two graphs captured on one stream, replayed on two, while eager calls of a larger size run and
     the kept scratch is dropped."""
     from foldjax_b200 import _device as dev, _lib
 
     call = _calls(cuda_device)[name]
-    inputs = _inputs(cuda_device, (200, 136, 264))
+    inputs = _inputs(cuda_device, sizes)
     want = [call(z, m) for z, m in inputs]
     torch.cuda.synchronize()
     capture, graphs = torch.cuda.Stream(), []

@@ -1,6 +1,8 @@
 """The attention cores' last step of keys, of which 16, 32, 48 or all 64 columns are computed: remainders at the edges
-of these widths, as the only step and behind a whole one, with rows that keep no key (whose weights show a column too
-many or too few) and with scores that reach their maximum in the last step.
+of these widths, as the only step, behind a whole one and behind several, with rows that keep no key (whose weights show a column too
+many or too few) and with scores that reach their maximum in the last step. 48 columns are taken by the 128-channel core where there
+is no whole step or more than one, by the float32 core for heads of up to 32 in up to two steps, and by the general
+bf16 core for heads of up to 32; elsewhere those keys take 64. With three SMs a CTA goes on from a short last step to its next items.
 
 Tolerances are those of the other tests of each core: the bf16 budget (conftest.assert_parity); float32 results of
 order one against float64, 1e-4; the single track 2e-4 as in the reference's own test."""
@@ -16,7 +18,7 @@ from oracle import triangle_oracle as orc
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-KEYS = [1, 15, 16, 17, 32, 33, 48, 49, 63, 80, 81, 96, 97, 112, 113, 128]
+KEYS = [1, 15, 16, 17, 32, 33, 48, 49, 63, 80, 81, 96, 97, 112, 113, 128, 129, 144, 145, 160, 161, 176, 177, 192, 225, 240]
 
 
 @pytest.mark.parametrize("n_k", KEYS)
@@ -36,12 +38,18 @@ def test_core(cuda_device, n_k):
     tb = orc.round_bf16(tb)
     ref = orc.attention_core(q, k, v, tb, mb, dtype="bfloat16")
     t = lambda a, dtype=torch.bfloat16: torch.from_numpy(a).to(cuda_device).to(dtype)
-    got = attention_core(t(q), t(k), t(v), t(tb), t(mb, torch.float32))
-    _lib.device_status()
+    args = t(q), t(k), t(v), t(tb), t(mb, torch.float32)
+    got, lib = attention_core(*args), _lib.load()
+    _lib.check(lib.b200tri_set_sm_limit(3))  # (of 16 items)
+    try:
+        assert torch.equal(attention_core(*args), got)
+        _lib.device_status()
+    finally:
+        _lib.check(lib.b200tri_set_sm_limit(0))
     assert_parity(ref, got.float().cpu().numpy(), label=f"core, {n_k} keys")
 
 
-@pytest.mark.parametrize("n", [16, 17, 33, 48, 49, 80, 81, 96, 112, 113])
+@pytest.mark.parametrize("n", [16, 17, 33, 48, 49, 80, 81, 96, 112, 113, 145, 161, 176])
 @pytest.mark.parametrize("heads,head_dim,dtype", [(4, 16, "bfloat16"), (12, 32, "bfloat16"), (2, 64, "bfloat16"), (4, 32, "float32"),
                                                   (2, 64, "float32")])
 def test_general_cores(cuda_device, n, heads, head_dim, dtype):
@@ -70,7 +78,7 @@ def test_general_cores(cuda_device, n, heads, head_dim, dtype):
         assert_parity(ref, got, where=~kept, label=f"n={n} {heads}x{head_dim}, rows without a key")
 
 
-@pytest.mark.parametrize("n", [16, 17, 33, 48, 49, 80, 97, 113])
+@pytest.mark.parametrize("n", [16, 17, 33, 48, 49, 80, 97, 113, 145, 161])
 def test_single_track(cuda_device, n):
     from foldjax_b200 import _lib
     from foldjax_b200.attention import attention_pair_bias_forward

@@ -90,7 +90,8 @@ def test_single_representation_off_the_16_byte_grid(cuda_device, monkeypatch, n,
         assert torch.equal(w, g)
 
 
-def test_results_do_not_depend_on_the_sm_limit(cuda_device):
+@pytest.mark.parametrize("limit", [40, 24])  # (16 heads x 2 tiles of queries: a CTA for each tile, and for two)
+def test_results_do_not_depend_on_the_sm_limit(cuda_device, limit):
     """Fewer SMs, the same K splits and therefore the same bits."""
     from foldjax_b200 import _device as dev, _lib
     from foldjax_b200.pairformer import pairformer_forward
@@ -101,7 +102,7 @@ def test_results_do_not_depend_on_the_sm_limit(cuda_device):
     z = dev.to_device(rng.standard_normal((1, n, n, 128)).astype(np.float32), torch.bfloat16)
     s = torch.from_numpy(rng.standard_normal((1, n, 384)).astype(np.float32)).cuda()
     want = pairformer_forward([pd, pd], s, z, torch.ones(1, n, device="cuda"), None)
-    _lib.check(lib.b200tri_set_sm_limit(40))
+    _lib.check(lib.b200tri_set_sm_limit(limit))
     try:
         got = pairformer_forward([pd, pd], s, z, torch.ones(1, n, device="cuda"), None)
         _lib.device_status()
@@ -109,3 +110,29 @@ def test_results_do_not_depend_on_the_sm_limit(cuda_device):
         _lib.check(lib.b200tri_set_sm_limit(0))
     for w, g in zip(want, got):
         assert torch.equal(w, g)
+
+
+@pytest.mark.parametrize("n", [129, 150, 176, 250, 256, 257, 300, 385])
+def test_two_tiles_of_queries_to_a_cta(cuda_device, n):
+    """The attention's form for more tiles than SMs, at 7 SMs: even and odd numbers of tiles, whose last CTA of a head then has one that does
+    not exist, several items a CTA, last steps of all widths. The bits of the form with a CTA for each tile, which the same
+    call takes with all SMs."""
+    from foldjax_b200 import _device as dev, _lib
+    from foldjax_b200.attention import attention_pair_bias_forward
+
+    rng, lib = np.random.default_rng(n), _lib.load()
+    params = orc.round_params(orc.random_attention_pair_bias_params(rng, c_s=384, heads=16, std=0.05, ln_noise=0.1), "bfloat16")
+    s = rng.standard_normal((1, n, 384)).astype(np.float32)
+    z = orc.round_bf16(rng.standard_normal((1, n, n, 128)).astype(np.float32))
+    mask = (rng.random((1, n)) < 0.85).astype(np.float32)
+    mask[0, -1] = 1.0
+    args = (dev.params_to_device(params), torch.from_numpy(s).cuda(), dev.to_device(z, torch.bfloat16), torch.from_numpy(mask).cuda())
+    want = attention_pair_bias_forward(*args)
+    _lib.check(lib.b200tri_set_sm_limit(7))
+    try:
+        got = attention_pair_bias_forward(*args)
+        _lib.device_status()
+    finally:
+        _lib.check(lib.b200tri_set_sm_limit(0))
+    assert torch.equal(got, want)
+    np.testing.assert_allclose(got.cpu().numpy(), orc.attention_pair_bias(params, s, z, mask, dtype="float64"), rtol=2e-4, atol=2e-4)
