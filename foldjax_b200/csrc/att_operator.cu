@@ -8,9 +8,10 @@
 // to fp16 [row][head * 32 + d][key], and the mask-bias rows. The pair bias is read where it is
 // unless its rows are off the 16-byte grid TMA needs, or float32.
 //
-// Bound of the preparation: memory, 2 + 2 bytes per element of V. 4 heads x 384 x 384 x 32: 99 us
-// with the core; relayout copies of all five operands alone are 250. Small operators are launches: with the bias
-// rows in one of their own 60 / 100 / 203 tokens took 10.1 / 12.2 / 30.6 us, 7.8 / 10.7 / 29.0 so.
+// Bound of the preparation: memory, 2 + 2 bytes per element of V. 4 heads x 384 x 384 x 32: 97 us with the core (this and the
+// next: calls replayed in a row on the same operands); relayout copies of all five operands alone are 250. Small operators are
+// launches: with the bias rows in one of their own 60 / 100 / 203 / 300 tokens took 10.3 / 12.4 / 33.7 / 76.2 us, 7.9 / 10.9 / 28.4 / 70.6 so
+// (the core's last step of its own width among it).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
